@@ -482,7 +482,7 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* xchg_abort = reinterpret_cast<volatile int*>(tmem_slot + 2);  // [4]: a warp of the pair gave up
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // CTA order.  Causal query tiles differ in length (2 ... 2 * q_tiles key tiles); within a chunk of `head_chunk`
   // (sample, head) pairs - sized so that the chunk's K and V stay in L2 - the longest tiles of all its heads are launched
   // first and the shortest last, so that the tail of the launch is made of short CTAs whatever the batch.
@@ -530,85 +530,94 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const uint32_t tmem_o = tmem_base + 3 * AT_BK;  // score / probability tile b lives at tmem_base + b * 64
 
   if (warp == 0) {
-    if (lane == 0) {
-      const int smp = bhi / p.heads, hd_slot = bhi - smp * p.heads;  // 5-D maps: (d, position, sample, head slot, plane)
+    // (whole warps with warp-uniform control flow, one elected lane issues: see elect_one)
+    const bool one = elect_one();
+    const int smp = bhi / p.heads, hd_slot = bhi - smp * p.heads;  // 5-D maps: (d, position, sample, head slot, plane)
+    if (one) {
       mbar_expect_tx(q_full, 2 * AT_Q_BYTES);
       tma_load_5d(sQ, &map_q, q_full, 0, q0, smp, hd_slot, 0);
       tma_load_5d(sQ + AT_Q_BYTES, &map_q, q_full, 0, q0, smp, hd_slot, 1);
-      bool ok = true;
-      auto load_k = [&](int j) {
-        const int st = j & 1;
-        if (!mbar_wait(k_empty + st, (static_cast<uint32_t>(j >> 1) & 1) ^ 1, abort_flag, p.err_word, 31)) { ok = false; return; }
-        mbar_expect_tx(k_full + st, A2_STAGE);
-        tma_load_5d(sK + st * A2_STAGE, &map_k, k_full + st, 0, j * AT_BK, smp, p.heads + hd_slot, 0);
-        tma_load_5d(sK + st * A2_STAGE + A2_TILE, &map_k, k_full + st, 0, j * AT_BK, smp, p.heads + hd_slot, 1);
-      };
-      auto load_v = [&](int j) {
-        const int st = j & 1;
-        if (!mbar_wait(v_empty + st, (static_cast<uint32_t>(j >> 1) & 1) ^ 1, abort_flag, p.err_word, 32)) { ok = false; return; }
-        mbar_expect_tx(v_full + st, A2_STAGE);
-        tma_load_5d(sV + st * A2_STAGE, &map_v, v_full + st, 0, j * AT_BK, smp, 2 * p.heads + hd_slot, 0);
-        tma_load_5d(sV + st * A2_STAGE + A2_TILE, &map_v, v_full + st, 0, j * AT_BK, smp, 2 * p.heads + hd_slot, 1);
-      };
-      // in the order the MMA warp consumes them: K_0, K_1, then V_j, K_{j+2}
-      if (n_tiles > 0) load_k(0);
-      if (ok && n_tiles > 1) load_k(1);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        load_v(j);
-        if (ok && j + 2 < n_tiles) load_k(j + 2);
-      }
     }
+    bool ok = true;
+    auto load_k = [&](int j) {
+      const int st = j & 1;
+      if (!mbar_wait_warp(k_empty + st, (static_cast<uint32_t>(j >> 1) & 1) ^ 1, abort_flag, p.err_word, 31)) { ok = false; return; }
+      if (!one) return;
+      mbar_expect_tx(k_full + st, A2_STAGE);
+      tma_load_5d(sK + st * A2_STAGE, &map_k, k_full + st, 0, j * AT_BK, smp, p.heads + hd_slot, 0);
+      tma_load_5d(sK + st * A2_STAGE + A2_TILE, &map_k, k_full + st, 0, j * AT_BK, smp, p.heads + hd_slot, 1);
+    };
+    auto load_v = [&](int j) {
+      const int st = j & 1;
+      if (!mbar_wait_warp(v_empty + st, (static_cast<uint32_t>(j >> 1) & 1) ^ 1, abort_flag, p.err_word, 32)) { ok = false; return; }
+      if (!one) return;
+      mbar_expect_tx(v_full + st, A2_STAGE);
+      tma_load_5d(sV + st * A2_STAGE, &map_v, v_full + st, 0, j * AT_BK, smp, 2 * p.heads + hd_slot, 0);
+      tma_load_5d(sV + st * A2_STAGE + A2_TILE, &map_v, v_full + st, 0, j * AT_BK, smp, 2 * p.heads + hd_slot, 1);
+    };
+    // in the order the MMA warp consumes them: K_0, K_1, then V_j, K_{j+2}
+    if (n_tiles > 0) load_k(0);
+    if (ok && n_tiles > 1) load_k(1);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      load_v(j);
+      if (ok && j + 2 < n_tiles) load_k(j + 2);
+    }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc(AT_BQ, AT_BK, p.f16);   // S = Q K^T: M = 128 queries, N = 64 keys
-      const uint32_t idesc_pv = idesc_s | (1u << 16);             // O += P V: N = 64 (d), V rows are keys: MN-major B
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.err_word, 33);
-      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
-      auto issue_scores = [&](int j) -> bool {
-        const uint32_t st = static_cast<uint32_t>(j) & 1, b = static_cast<uint32_t>(j % 3);
-        if (!mbar_wait(k_full + st, static_cast<uint32_t>(j >> 1) & 1, abort_flag, p.err_word, 34)) return false;
-        tcgen05_fence_after();
-        const uint32_t kb = aK + st * A2_STAGE;
+    const bool one = elect_one();
+    const uint32_t idesc_s = make_idesc(AT_BQ, AT_BK, p.f16);   // S = Q K^T: M = 128 queries, N = 64 keys
+    const uint32_t idesc_pv = idesc_s | (1u << 16);             // O += P V: N = 64 (d), V rows are keys: MN-major B
+    const bool ok_q = mbar_wait_warp(q_full, 0, abort_flag, p.err_word, 33);
+    bool ok = ok_q;
+    const uint64_t dQh = make_smem_desc(smem_u32(sQ), 128), dQl = dQh + (AT_Q_BYTES >> 4);
+    const uint64_t dK = make_smem_desc(smem_u32(sK), 128), dV = make_smem_desc(smem_u32(sV), 128);
+    auto issue_scores = [&](int j) -> bool {
+      const uint32_t st = static_cast<uint32_t>(j) & 1, b = static_cast<uint32_t>(j % 3);
+      if (!mbar_wait_warp(k_full + st, static_cast<uint32_t>(j >> 1) & 1, abort_flag, p.err_word, 34)) return false;
+      tcgen05_fence_after();
+      const uint64_t kh = dK + st * (A2_STAGE >> 4), kl = kh + (A2_TILE >> 4);
+      if (one) {
 #pragma unroll
-        for (int k = 0; k < AT_HD / 16; ++k) {
-          const uint32_t ko = k * 32;
-          const uint64_t qh = make_smem_desc(aQ + ko, 128), ql = make_smem_desc(aQ + AT_Q_BYTES + ko, 128);
-          const uint64_t kh = make_smem_desc(kb + ko, 128), kl = make_smem_desc(kb + A2_TILE + ko, 128);
-          umma_bf16(tmem_base + b * AT_BK, qh, kh, idesc_s, k != 0 ? 1u : 0u);
-          umma_bf16(tmem_base + b * AT_BK, ql, kh, idesc_s, 1u);
-          umma_bf16(tmem_base + b * AT_BK, qh, kl, idesc_s, 1u);
+        for (int k = 0; k < AT_HD / 16; ++k) {  // 32 bytes along d = 2 in the address field
+          umma_bf16(tmem_base + b * AT_BK, dQh + 2 * k, kh + 2 * k, idesc_s, k != 0 ? 1u : 0u);
+          umma_bf16(tmem_base + b * AT_BK, dQl + 2 * k, kh + 2 * k, idesc_s, 1u);
+          umma_bf16(tmem_base + b * AT_BK, dQh + 2 * k, kl + 2 * k, idesc_s, 1u);
         }
         umma_commit(s_full + b);
         umma_commit(k_empty + st);
-        return true;
-      };
-      if (ok && n_tiles > 0) ok = issue_scores(0);
-      if (ok && n_tiles > 1) ok = issue_scores(1);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const uint32_t st = static_cast<uint32_t>(j) & 1, b = static_cast<uint32_t>(j % 3);
-        if (!mbar_wait(p_full + b, static_cast<uint32_t>(j / 3) & 1, abort_flag, p.err_word, 35)) break;
-        if (!mbar_wait(v_full + st, static_cast<uint32_t>(j >> 1) & 1, abort_flag, p.err_word, 36)) break;
-        tcgen05_fence_after();
-        const uint32_t tp = tmem_base + b * AT_BK;  // hi pairs in columns [0, 32), lo pairs in [32, 64) of the tile
-        const uint32_t vb = aV + st * A2_STAGE;
+      }
+      __syncwarp();
+      return true;
+    };
+    if (ok && n_tiles > 0) ok = issue_scores(0);
+    if (ok && n_tiles > 1) ok = issue_scores(1);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const uint32_t st = static_cast<uint32_t>(j) & 1, b = static_cast<uint32_t>(j % 3);
+      if (!mbar_wait_warp(v_full + st, static_cast<uint32_t>(j >> 1) & 1, abort_flag, p.err_word, 36)) break;
+      if (!mbar_wait_warp(p_full + b, static_cast<uint32_t>(j / 3) & 1, abort_flag, p.err_word, 35)) break;
+      tcgen05_fence_after();
+      const uint32_t tp = tmem_base + b * AT_BK;  // hi pairs in columns [0, 32), lo pairs in [32, 64) of the tile
+      const uint64_t vh = dV + st * (A2_STAGE >> 4), vl = vh + (A2_TILE >> 4);
+      if (one) {
 #pragma unroll
         for (int k = 0; k < AT_BK / 16; ++k) {
-          // 16 keys: eight packed columns of P, two 1024-byte groups of eight 128-byte V rows
-          const uint64_t vh = make_smem_desc(vb + k * 2048u, 128), vl = make_smem_desc(vb + A2_TILE + k * 2048u, 128);
-          umma_f16_ts(tmem_o, tp + k * 8, vh, idesc_pv, (j != 0 || k != 0) ? 1u : 0u);
-          umma_f16_ts(tmem_o, tp + 32 + k * 8, vh, idesc_pv, 1u);
-          umma_f16_ts(tmem_o, tp + k * 8, vl, idesc_pv, 1u);
+          // 16 keys: eight packed columns of P, two 1024-byte groups of eight 128-byte V rows (2048 bytes = 128 in the field)
+          umma_f16_ts(tmem_o, tp + k * 8, vh + 128 * k, idesc_pv, (j != 0 || k != 0) ? 1u : 0u);
+          umma_f16_ts(tmem_o, tp + 32 + k * 8, vh + 128 * k, idesc_pv, 1u);
+          umma_f16_ts(tmem_o, tp + k * 8, vl + 128 * k, idesc_pv, 1u);
         }
         umma_commit(pv_done + b);
         umma_commit(v_empty + st);
-        if (j + 2 < n_tiles) {
-          // S_{j+2} goes into the tile that P_{j-1} V_{j-1} read: that product has long finished (P_j came after it), the
-          // wait only makes the reuse explicit
-          if (j >= 1 && !mbar_wait(pv_done + (j - 1) % 3, static_cast<uint32_t>((j - 1) / 3) & 1, abort_flag, p.err_word, 37)) break;
-          if (!issue_scores(j + 2)) break;
-        }
+      }
+      __syncwarp();
+      if (j + 2 < n_tiles) {
+        // S_{j+2} goes into the tile that P_{j-1} V_{j-1} read: that product has long finished (P_j came after it), the
+        // wait only makes the reuse explicit
+        if (j >= 1 && !mbar_wait_warp(pv_done + (j - 1) % 3, static_cast<uint32_t>((j - 1) / 3) & 1, abort_flag, p.err_word, 37)) break;
+        if (!issue_scores(j + 2)) break;
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------ softmax: two threads per query row ------------------------------
     // Warps 2-5 take the first 32 keys of every tile, warps 6-9 the last 32; the two warps that share a TMEM lane

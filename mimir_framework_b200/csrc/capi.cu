@@ -153,7 +153,7 @@ int linear_exec(const LinearExec& e, cudaStream_t st) {
   g.w = e.w_split;
   g.a_planes = ap;
   g.w_planes = wp;
-  g.w_scale = e.w_scale;
+  g.w_scale = e.w_scale; g.w_ready = e.w_ready;
   g.m = e.rows;
   g.n = e.out_f;
   g.k = e.in_f;
@@ -202,7 +202,7 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
   } else {
     if (!e.x_split) MB_TRY(launch_split(e.x, xs, rows, e.embed, ap, st));
     GemmArgs g;
-    g.a = e.x_split ? e.x_split : xs; g.w = e.wqkv_split; g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale;
+    g.a = e.x_split ? e.x_split : xs; g.w = e.wqkv_split; g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale; g.w_ready = e.w_ready;
     g.m = rows; g.n = 3 * e.embed; g.k = e.embed; g.ldo = 3 * e.embed;
     // the tensor-core attention core takes Q and K straight from hi/lo planes written by this GEMM's epilogue (they
     // occupy the fp32 buffer's place: 2 planes x 2 bytes); a cache fill or decode step needs the fp32 rows
@@ -249,7 +249,7 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
     MB_TRY(launch_split(att, xs, rows, e.embed, ap, st));
   }
   GemmArgs o;
-  o.a = xs; o.w = e.wout_split; o.a_planes = ap; o.w_planes = wp; o.w_scale = e.w_scale;
+  o.a = xs; o.w = e.wout_split; o.a_planes = ap; o.w_planes = wp; o.w_scale = e.w_scale; o.w_ready = e.w_ready;
   o.m = rows; o.n = e.embed; o.k = e.embed; o.out_f32 = e.y; o.ldo = e.embed; o.residual = e.residual;
   return launch_gemm(o, st);
 }
@@ -326,7 +326,7 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     GemmArgs g;
     g.a = static_cast<const __nv_bfloat16*>(e.ws);
     g.w = e.w_split;
-    g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale;
+    g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale; g.w_ready = e.w_ready;
     g.m = static_cast<int>(rows); g.n = e.oc; g.k = k;
     g.activation = e.activation;
     g.out_f32 = e.y;
@@ -350,7 +350,7 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     GemmArgs g;
     g.a = static_cast<const __nv_bfloat16*>(e.ws);
     g.w = e.w_split;
-    g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale;
+    g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale; g.w_ready = e.w_ready;
     g.m = bc * ohw; g.n = e.oc; g.k = k;
     g.activation = e.activation;
     g.out_f32 = e.y + static_cast<size_t>(b0) * e.oc * ohw;

@@ -30,11 +30,11 @@ int cross_attention_exec(const CrossAttentionExec& e, cudaStream_t st) {
   MB_TRY(launch_split(e.q_in, qs, qr, E, ap, st));
   MB_TRY(launch_split(e.kv_in, ks, kr, E, ap, st));
   GemmArgs g;
-  g.a = qs; g.w = e.wq_split; g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale;
+  g.a = qs; g.w = e.wq_split; g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale; g.w_ready = e.w_ready;
   g.m = qr; g.n = E; g.k = E; g.out_f32 = q; g.ldo = E;
   MB_TRY(launch_gemm(g, st));
   GemmArgs h;
-  h.a = ks; h.w = e.wkv_split; h.a_planes = ap; h.w_planes = wp; h.w_scale = e.w_scale;
+  h.a = ks; h.w = e.wkv_split; h.a_planes = ap; h.w_planes = wp; h.w_scale = e.w_scale; h.w_ready = e.w_ready;
   h.m = kr; h.n = 2 * E; h.k = E; h.out_f32 = kv; h.ldo = 2 * E;
   MB_TRY(launch_gemm(h, st));
   AttnView v;
@@ -44,7 +44,7 @@ int cross_attention_exec(const CrossAttentionExec& e, cudaStream_t st) {
   MB_TRY(launch_attention_core_view(v, att, e.batch, E, e.heads, e.causal, st));
   MB_TRY(launch_split(att, qs, qr, E, ap, st));  // the query planes are dead by now
   GemmArgs o;
-  o.a = qs; o.w = e.wout_split; o.a_planes = ap; o.w_planes = wp; o.w_scale = e.w_scale;
+  o.a = qs; o.w = e.wout_split; o.a_planes = ap; o.w_planes = wp; o.w_scale = e.w_scale; o.w_ready = e.w_ready;
   o.m = qr; o.n = E; o.k = E; o.out_f32 = e.y; o.ldo = E; o.residual = e.residual;
   return launch_gemm(o, st);
 }

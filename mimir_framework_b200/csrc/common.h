@@ -160,7 +160,22 @@ struct GemmArgs {
   // 32-channel chunk, for the GroupNorm that reads this output; gemm_gn_part_bytes() of scratch.  gn_cpg in {4, 8, 16, 32}.
   float* gn_part = nullptr;
   int gn_cpg = 0;
+  // The weight planes were complete before the launches of this call began (a planned model's): the kernel may fetch them
+  // before the kernel ahead of it in the stream has finished.
+  bool w_ready = false;
 };
+float gemm_acc_scale(const GemmArgs& g);
+// CUDA events around a GEMM launch while live timing is on (mimir_b200_profile_gemm)
+struct GemmProfile {
+  explicit GemmProfile(cudaStream_t s) : st(s) {}
+  int begin();
+  int end();
+  cudaStream_t st;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+};
+// gemm_split.cu: narrow tiles and split K for launches of few 128 x 256 tiles; wanted when its estimate beats `other_cycles`
+bool gemm_split_wanted(const GemmArgs& g, int bk, double other_cycles, int* bn, int* splits);
+int launch_gemm_split(const GemmArgs& g, int bk, int bn, int splits, cudaStream_t st);
 inline size_t gemm_gn_part_bytes(long long m, int n, int cpg) {
   return static_cast<size_t>((m + 31) / 32) * static_cast<size_t>((n + 31) / 32) * static_cast<size_t>(2 * (1 + 64 / cpg)) * sizeof(float);
 }

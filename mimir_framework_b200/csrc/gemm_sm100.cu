@@ -21,6 +21,9 @@
 #include "common.h"
 #include "planes.cuh"
 #include "sm100_ptx.cuh"
+#include "epilogue.cuh"
+#include "launch.cuh"
+#include "tensor_map.h"
 
 #include <cmath>
 #include <cstring>
@@ -37,30 +40,6 @@ constexpr int TMEM_COLS = 512;
 constexpr int NUM_THREADS = 320;  // 10 warps: TMA, MMA, 8 epilogue
 constexpr int EPI_WARPS = 8;
 constexpr float ACC_TRUNC_PER_MMA = 1.5e-8f;  // mean relative loss of the fp32 accumulator per tcgen05.mma (truncating adds)
-
-// GELU in the reference's tanh form (LayerOps.hpp:556-568), x * 0.5 * (1 + tanh(u)) with u = c * (x + 0.044715 x^3) and
-// c = sqrt(2.0f / 3.14159265359f) evaluated in fp32.  0.5 * (1 + tanh(u)) is the logistic function of 2u, so the value is
-// x / (1 + exp(-2u)): one ex2 and one reciprocal on the special-function unit instead of tanhf's ~30 instructions (the
-// epilogue of a K = 768 layer has only ~12 000 cycles per 128 x 256 tile for 32 768 of these), and without the
-// cancellation of 1 + tanh(u) for negative arguments.  Error: a few ulp of the result (ex2.approx 2 ulp, rcp.approx 1 ulp).
-__device__ __forceinline__ float gelu_ref(float x) {
-  const float c = 0.7978845608f;
-  const float u = c * (x + 0.044715f * x * x * x);
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(u * -2.885390082f));  // exp(-2u) = 2^(-2u log2 e)
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return x * r;
-}
-__device__ __forceinline__ float apply_act(float v, int act) {
-  switch (act) {
-    case MIMIR_B200_ELT_GELU: return gelu_ref(v);
-    case MIMIR_B200_ELT_SILU: return v * (1.0f / (1.0f + expf(-v)));
-    case MIMIR_B200_ELT_RELU: return fmaxf(v, 0.0f);
-    case MIMIR_B200_ELT_TANH: return tanhf(v);
-    case MIMIR_B200_ELT_SIGMOID: return 1.0f / (1.0f + expf(-v));
-    default: return v;
-  }
-}
 
 struct GemmParams {
   int m, n, kblocks;         // kblocks = kp / BK
@@ -175,6 +154,70 @@ __device__ __forceinline__ void gn_emit_chunk(const float (&v)[32], bool pix_ok,
   }
 }
 
+// The MMA role: MP planes on the M side, NP on the N side.  The whole warp runs it and one elected lane issues (elect_one); the
+// next stage's barrier is polled before the current stage's MMAs are issued, so that a K block costs its MMAs and not the
+// latency of a wait on top (see gemm_split.cu).  Measured per 64-wide K block of one MMA per product: 1 100 cycles as a
+// branch on lane 0, about 300 in this form; with two and three MMAs per product the tensor pipe is the limit again.
+template <int BK, int PAIR, int MP, int NP>
+__device__ __forceinline__ void mma_role(const GemmParams& p, uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* acc_full,
+                                         uint64_t* acc_empty, volatile int* abort_flag, uint32_t tmem_base, int t_first, int t_step,
+                                         int num_tiles) {
+  constexpr int SWZ = BK * 2, A_TILE = BM * BK * 2, W_TILE = (PAIR ? BN / 2 : BN) * BK * 2;
+  const bool one = elect_one();
+  const uint32_t idesc = make_idesc(PAIR ? 2 * BM : BM, p.bn, p.f16);
+  const int stages = p.stages, stage_bytes = p.stage_bytes, kblocks = p.kblocks;
+  int stage = 0, acc = 0;
+  uint32_t phase = 0, acc_phase = 0;
+  bool ready = false;
+  for (int t = t_first; t < num_tiles; t += t_step) {
+    if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err_word, 3)) return;
+    tcgen05_fence_after();
+    const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+    for (int kb = 0; kb < kblocks; ++kb) {
+      if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.err_word, 4)) return;
+      tcgen05_fence_after();
+      const uint32_t sa = smem_u32(smem + stage * stage_bytes);
+      const uint64_t da = make_smem_desc(sa, SWZ), dw = make_smem_desc(sa + MP * A_TILE, SWZ);
+      const uint64_t da_lo = da + (A_TILE >> 4), dw_lo = dw + (W_TILE >> 4);
+      uint64_t* done = &empty_bar[stage];
+      if (++stage == stages) { stage = 0; phase ^= 1; }
+      ready = mbar_test(&full_bar[stage], phase);
+      if (one) {
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) {  // 32 bytes further along K = 2 in a descriptor's address field
+          const uint32_t add = (kb | k) != 0 ? 1u : 0u;
+          if (PAIR) {
+            umma_bf16_pair(d_tmem, da + 2 * k, dw + 2 * k, idesc, add);
+            if (MP == 2) umma_bf16_pair(d_tmem, da_lo + 2 * k, dw + 2 * k, idesc, 1u);
+            if (NP == 2) umma_bf16_pair(d_tmem, da + 2 * k, dw_lo + 2 * k, idesc, 1u);
+          } else {
+            umma_bf16(d_tmem, da + 2 * k, dw + 2 * k, idesc, add);
+            if (MP == 2) umma_bf16(d_tmem, da_lo + 2 * k, dw + 2 * k, idesc, 1u);
+            if (NP == 2) umma_bf16(d_tmem, da + 2 * k, dw_lo + 2 * k, idesc, 1u);
+          }
+        }
+        if (PAIR) {  // frees the stage in both CTAs when these MMAs have read it
+          umma_commit_pair(mapa_shared(smem_u32(done), 0));
+          umma_commit_pair(mapa_shared(smem_u32(done), 1));
+        } else {
+          umma_commit(done);
+        }
+      }
+      __syncwarp();
+    }
+    if (one) {
+      if (PAIR) {
+        umma_commit_pair(mapa_shared(smem_u32(&acc_full[acc]), 0));
+        umma_commit_pair(mapa_shared(smem_u32(&acc_full[acc]), 1));
+      } else {
+        umma_commit(&acc_full[acc]);
+      }
+    }
+    __syncwarp();
+    if (++acc == NUM_ACC) { acc = 0; acc_phase ^= 1; }
+  }
+}
+
 // CM = 1 compiles the channel-major forms in (NCHW output, convolution as shifted GEMMs, swapped operands; CM = 2: the same
 // plus GroupNorm partials of the stored values from the epilogue); the plain
 // row-major form (CM = 0: every Linear and attention projection) is built without them, so that the two families
@@ -207,7 +250,7 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + NUM_ACC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n;
 
@@ -248,112 +291,67 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = t_first; t < num_tiles && ok; t += t_step) {
-        int tm, tn;
-        tile_coords(t, p, tm, tn);
-        if (PAIR) tm = tm * 2 + static_cast<int>(crank);  // p.tiles_m counts row PAIRS
-        for (int kb = 0; kb < p.kblocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err_word, 1)) { ok = false; break; }
-          uint8_t* sbase = smem + stage * STAGE_BYTES;
-          int a_col = kb * BK, a_row = tm * BM;
-          if (conv) {
-            const int t = kb / p.conv_cblocks, cb = kb - t * p.conv_cblocks;
-            const int kh = t / p.conv_ks, kw = t - kh * p.conv_ks;
-            a_row += (kh - p.conv_pad) * p.conv_wp + (kw - p.conv_pad);  // may be negative: TMA zero-fills
-            a_col = cb * BK;
-          }
+    // (the whole warp runs the loop, one elected lane issues: see elect_one)
+    const bool one = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = t_first; t < num_tiles && ok; t += t_step) {
+      int tm, tn;
+      tile_coords(t, p, tm, tn);
+      if (PAIR) tm = tm * 2 + static_cast<int>(crank);  // p.tiles_m counts row PAIRS
+      const int w_row = swapped ? tm * BM
+                        : PAIR ? tn * BN + static_cast<int>(crank) * (BN / 2)
+                               : tn * p.bn + (p.a_group_rows > 0 ? (tm * BM / p.a_group_rows) * p.w_group_rows : 0);
+      const int a_row0 = swapped ? tn * BN : tm * BM;  // swapped: 256 activation rows (tile tn) are the N side
+      for (int kb = 0; kb < p.kblocks; ++kb) {
+        if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err_word, 1)) { ok = false; break; }
+        uint8_t* m_base = smem + stage * STAGE_BYTES;
+        uint8_t* n_base = m_base + m_planes * A_TILE;
+        int a_col = kb * BK, a_row = a_row0;
+        if (conv) {
+          const int tap = kb / p.conv_cblocks, cb = kb - tap * p.conv_cblocks;
+          const int kh = tap / p.conv_ks, kw = tap - kh * p.conv_ks;
+          a_row += (kh - p.conv_pad) * p.conv_wp + (kw - p.conv_pad);  // may be negative: TMA zero-fills
+          a_col = cb * BK;
+        }
+        if (one) {
           if (PAIR) {
             // the leader arms its barrier for the bytes of both CTAs; this CTA's bytes are counted there whichever
             // of the two arrives first (the phase cannot complete before the leader's arrive)
             if (crank == 0) mbar_expect_tx(&full_bar[stage], tx_bytes);
             const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
-            for (int pl = 0; pl < p.a_planes; ++pl)
-              tma_load_3d_pair(sbase + pl * A_TILE, &map_a, fb, a_col, a_row, pl);
-            for (int pl = 0; pl < p.w_planes; ++pl)
-              tma_load_3d_pair(sbase + m_planes * A_TILE + pl * W_TILE, &map_w, fb, kb * BK, tn * BN + static_cast<int>(crank) * (BN / 2), pl);
-            if (++stage == STAGES) { stage = 0; phase ^= 1; }
-            continue;
-          }
-          mbar_expect_tx(&full_bar[stage], tx_bytes);
-          if (!swapped) {
-            for (int pl = 0; pl < p.a_planes; ++pl)
-              tma_load_3d(sbase + pl * A_TILE, &map_a, &full_bar[stage], a_col, a_row, pl);
-            for (int pl = 0; pl < p.w_planes; ++pl)
-              tma_load_3d(sbase + m_planes * A_TILE + pl * W_TILE, &map_w, &full_bar[stage], kb * BK,
-                          tn * p.bn + (p.a_group_rows > 0 ? (tm * BM / p.a_group_rows) * p.w_group_rows : 0), pl);
+            tma_load_3d_pair(m_base, &map_a, fb, a_col, a_row, 0);
+            if (m_planes == 2) tma_load_3d_pair(m_base + A_TILE, &map_a, fb, a_col, a_row, 1);
+            tma_load_3d_pair(n_base, &map_w, fb, kb * BK, w_row, 0);
+            if (n_planes == 2) tma_load_3d_pair(n_base + W_TILE, &map_w, fb, kb * BK, w_row, 1);
           } else {
-            // 128 weight rows into the M-side tiles, 256 activation rows (tile tn) into the N-side tiles
-            a_row += tn * BN - tm * BM;
-            for (int pl = 0; pl < p.w_planes; ++pl)
-              tma_load_3d(sbase + pl * A_TILE, &map_w, &full_bar[stage], kb * BK, tm * BM, pl);
-            for (int pl = 0; pl < p.a_planes; ++pl)
-              tma_load_3d(sbase + m_planes * A_TILE + pl * W_TILE, &map_a, &full_bar[stage], a_col, a_row, pl);
+            mbar_expect_tx(&full_bar[stage], tx_bytes);
+            uint8_t* ab = swapped ? n_base : m_base;
+            uint8_t* wb = swapped ? m_base : n_base;
+            tma_load_3d(ab, &map_a, &full_bar[stage], a_col, a_row, 0);
+            if (p.a_planes == 2) tma_load_3d(ab + (swapped ? W_TILE : A_TILE), &map_a, &full_bar[stage], a_col, a_row, 1);
+            tma_load_3d(wb, &map_w, &full_bar[stage], kb * BK, w_row, 0);
+            if (p.w_planes == 2) tma_load_3d(wb + (swapped ? A_TILE : W_TILE), &map_w, &full_bar[stage], kb * BK, w_row, 1);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-      }
-      // Drain: every stage this thread filled must have landed and been consumed (or the abort
-      // flag is up) before the CTA may exit with copies in flight.
-      for (int s = 0; s < STAGES; ++s) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err_word, 2)) break;
+        __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
+    // Drain: every stage this warp filled must have landed and been consumed (or the abort
+    // flag is up) before the CTA may exit with copies in flight.
+    for (int s = 0; s < STAGES; ++s) {
+      if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err_word, 2)) break;
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+    }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------------------
-    if (lane == 0 && crank == 0) {
-      const uint32_t idesc = make_idesc(PAIR ? 2 * BM : BM, p.bn, p.f16);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = t_first; t < num_tiles && ok; t += t_step) {
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err_word, 3)) break;
-        tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = 0; kb < p.kblocks; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.err_word, 4)) { ok = false; break; }
-          tcgen05_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t sw = sa + m_planes * A_TILE;
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint32_t koff = k * UMMA_K * 2;  // bytes along K inside the swizzled row
-            const uint64_t a_hi = make_smem_desc(sa + koff, SWZ);
-            const uint64_t w_hi = make_smem_desc(sw + koff, SWZ);
-            if (PAIR) umma_bf16_pair(d_tmem, a_hi, w_hi, idesc, (kb | k) != 0 ? 1u : 0u);
-            else umma_bf16(d_tmem, a_hi, w_hi, idesc, (kb | k) != 0 ? 1u : 0u);
-            if (m_planes == 2) {
-              const uint64_t a_lo = make_smem_desc(sa + A_TILE + koff, SWZ);
-              if (PAIR) umma_bf16_pair(d_tmem, a_lo, w_hi, idesc, 1u);
-              else umma_bf16(d_tmem, a_lo, w_hi, idesc, 1u);
-            }
-            if (n_planes == 2) {
-              const uint64_t w_lo = make_smem_desc(sw + W_TILE + koff, SWZ);
-              if (PAIR) umma_bf16_pair(d_tmem, a_hi, w_lo, idesc, 1u);
-              else umma_bf16(d_tmem, a_hi, w_lo, idesc, 1u);
-            }
-          }
-          if (PAIR) {  // frees the stage in both CTAs when these MMAs have read it
-            umma_commit_pair(mapa_shared(smem_u32(&empty_bar[stage]), 0));
-            umma_commit_pair(mapa_shared(smem_u32(&empty_bar[stage]), 1));
-          } else
-          umma_commit(&empty_bar[stage]);  // frees the stage when these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        if (PAIR) {
-          umma_commit_pair(mapa_shared(smem_u32(&acc_full[acc]), 0));
-          umma_commit_pair(mapa_shared(smem_u32(&acc_full[acc]), 1));
-        } else
-        umma_commit(&acc_full[acc]);
-        if (++acc == NUM_ACC) { acc = 0; acc_phase ^= 1; }
-      }
+    if (crank == 0) {  // (of a pair: the leader)
+      if (m_planes == 2 && n_planes == 2) mma_role<BK, PAIR, 2, 2>(p, smem, full_bar, empty_bar, acc_full, acc_empty, abort_flag, tmem_base, t_first, t_step, num_tiles);
+      else if (m_planes == 2) mma_role<BK, PAIR, 2, 1>(p, smem, full_bar, empty_bar, acc_full, acc_empty, abort_flag, tmem_base, t_first, t_step, num_tiles);
+      else if (n_planes == 2) mma_role<BK, PAIR, 1, 2>(p, smem, full_bar, empty_bar, acc_full, acc_empty, abort_flag, tmem_base, t_first, t_step, num_tiles);
+      else mma_role<BK, PAIR, 1, 1>(p, smem, full_bar, empty_bar, acc_full, acc_empty, abort_flag, tmem_base, t_first, t_step, num_tiles);
     }
   } else {
     // ------------------------------ epilogue (warps 2..9) ---------------------------------
@@ -441,7 +439,7 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           float v[32];
           tmem_ld_32x32(taddr0 + c0, v);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = v[j] * p.acc_scale;  // [pixel][channel]
+          for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = __fmul_rn(v[j], p.acc_scale);  // [pixel][channel]
           __syncwarp();
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = tbuf[lane * 33 + j];  // lane = pixel r0 + lane, j = channel oc0 + j
@@ -499,22 +497,19 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // one 32-column chunk of this lane's row: scale, bias, activation, residual, stores
       auto process = [&](const int c0, const int col0, float (&v)[32]) {
         (void)c0;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] *= p.acc_scale;
         const bool full_cols = (col0 + 32 <= p.n);
-        // bias: the same 32 values for every lane (broadcast loads)
-        if (p.bias != nullptr) {
-          if (full_cols && ((reinterpret_cast<uintptr_t>(p.bias + col0) & 15) == 0)) {
+        // scale and bias (the same 32 values for every lane: broadcast loads) in one rounding, as in gemm_split.cu: both kernels
+        // give the same bits where they add up K in the same order
+        if (p.bias != nullptr && full_cols && ((reinterpret_cast<uintptr_t>(p.bias + col0) & 15) == 0)) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 b4 = __ldg(reinterpret_cast<const float4*>(p.bias + col0 + j));
-              v[j] += b4.x; v[j + 1] += b4.y; v[j + 2] += b4.z; v[j + 3] += b4.w;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col0 + j < p.n) v[j] += __ldg(p.bias + col0 + j);
+          for (int j = 0; j < 32; j += 4) {
+            const float4 b4 = __ldg(reinterpret_cast<const float4*>(p.bias + col0 + j));
+            v[j] = __fmaf_rn(v[j], p.acc_scale, b4.x); v[j + 1] = __fmaf_rn(v[j + 1], p.acc_scale, b4.y);
+            v[j + 2] = __fmaf_rn(v[j + 2], p.acc_scale, b4.z); v[j + 3] = __fmaf_rn(v[j + 3], p.acc_scale, b4.w);
           }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __fmaf_rn(v[j], p.acc_scale, (p.bias != nullptr && col0 + j < p.n) ? __ldg(p.bias + col0 + j) : 0.0f);
         }
         switch (p.activation) {  // hoisted out of the element loop
           case MIMIR_B200_ELT_GELU:
@@ -653,6 +648,69 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 }  // namespace
 
+namespace {
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  return fn;
+}
+}  // namespace
+
+// 3-D map over bf16 planes [planes][rows][kp]; box = {bk, box_rows, 1}; swizzle span = bk * 2 bytes.
+int make_plane_map(CUtensorMap* map, const void* base, int planes, long long rows, int kp, int bk, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(MIMIR_B200_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return fail(MIMIR_B200_E_INVALID, "GEMM operand not 16-byte aligned");
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(kp), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(planes)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(kp) * 2, static_cast<cuuint64_t>(rows) * kp * 2};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(bk), static_cast<cuuint32_t>(box_rows), 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUtensorMapSwizzle sw = (bk == 64) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(MIMIR_B200_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
+  return MIMIR_B200_OK;
+}
+
+// What an accumulator is multiplied by before bias / activation: the mean loss of the tensor core's truncating adds undone, the
+// weight scale divided out.  Measured on B200 against fp64 products of the same operand planes (random normal operands, K = 256 ...
+// 4096, two and three MMAs per 16-wide K step): the accumulated result is low by 1.47e-8 ... 1.58e-8 of its value per MMA
+// instruction that added into it; all-positive operands lose 2.1e-8 ... 3.6e-8.  Zero-padded K adds exact zeros and loses nothing,
+// so only the real K counts.  Undoing the mean loss halves the accumulation error.
+float gemm_acc_scale(const GemmArgs& g) {
+  const long long ksteps = g.conv_ks > 0 ? static_cast<long long>(g.conv_ks) * g.conv_ks * ((g.conv_c + UMMA_K - 1) / UMMA_K)
+                                         : (g.k + UMMA_K - 1) / UMMA_K;
+  const int products = 1 + (g.a_planes == 2 ? 1 : 0) + (g.w_planes == 2 ? 1 : 0);
+  static const bool comp = [] { const char* e = getenv("MIMIR_B200_ACC_COMP"); return !(e && e[0] == '0'); }();
+  return (comp ? 1.0f + ACC_TRUNC_PER_MMA * static_cast<float>(ksteps * products) : 1.0f) / g.w_scale;
+}
+
+int GemmProfile::begin() {
+  if (!ctx().prof_gemm) return MIMIR_B200_OK;
+  MB_CUDA(cudaEventCreate(&e0));
+  MB_CUDA(cudaEventCreate(&e1));
+  MB_CUDA(cudaEventRecord(e0, st));
+  return MIMIR_B200_OK;
+}
+int GemmProfile::end() {
+  if (!e0) return MIMIR_B200_OK;
+  MB_CUDA(cudaEventRecord(e1, st));
+  ctx().prof_events.push_back(e0);
+  ctx().prof_events.push_back(e1);
+  return MIMIR_B200_OK;
+}
+
 // ------------------------------------------------------------------------------------------
 // fp32 -> bf16 hi/lo planes
 // ------------------------------------------------------------------------------------------
@@ -709,39 +767,6 @@ __global__ void split_transposed_kernel(const float* __restrict__ src, __nv_bflo
       if (planes == 2) d16[plane_stride + static_cast<long long>(nn) * kp + kk] = l;
     }
   }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
-// 3-D map over bf16 planes [planes][rows][kp]; box = {bk, box_rows, 1}; swizzle span = bk * 2 bytes.
-int make_plane_map(CUtensorMap* map, const void* base, int planes, long long rows, int kp, int bk, int box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return fail(MIMIR_B200_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return fail(MIMIR_B200_E_INVALID, "GEMM operand not 16-byte aligned");
-  cuuint64_t dims[3] = {static_cast<cuuint64_t>(kp), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(planes)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(kp) * 2, static_cast<cuuint64_t>(rows) * kp * 2};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(bk), static_cast<cuuint32_t>(box_rows), 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapSwizzle sw = (bk == 64) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(MIMIR_B200_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
-  return MIMIR_B200_OK;
 }
 
 // 2-D map over the fp32 row-major output [rows][ld]; box = 32 x 32, 128-byte swizzle (the epilogue's staging tile)
@@ -849,17 +874,7 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
   }
   p.a_group_rows = g.a_group_rows;
   p.w_group_rows = g.w_group_rows;
-  {
-    // Measured on B200 against fp64 products of the same operand planes (random normal operands, K = 256 ... 4096,
-    // two and three MMAs per 16-wide K step): the accumulated result is low by 1.47e-8 ... 1.58e-8 of its value per
-    // MMA instruction that added into it; all-positive operands lose 2.1e-8 ... 3.6e-8.  Zero-padded K adds exact
-    // zeros and loses nothing, so only the real K counts.  Undoing the mean loss halves the accumulation error.
-    const long long ksteps = conv ? static_cast<long long>(g.conv_ks) * g.conv_ks * ((g.conv_c + UMMA_K - 1) / UMMA_K)
-                                  : (g.k + UMMA_K - 1) / UMMA_K;
-    const int products = 1 + (g.a_planes == 2 ? 1 : 0) + (g.w_planes == 2 ? 1 : 0);
-    static const bool comp = [] { const char* e = getenv("MIMIR_B200_ACC_COMP"); return !(e && e[0] == '0'); }();
-    p.acc_scale = (comp ? 1.0f + ACC_TRUNC_PER_MMA * static_cast<float>(ksteps * products) : 1.0f) / g.w_scale;
-  }
+  p.acc_scale = gemm_acc_scale(g);
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   constexpr int RING_BYTES = 196608;  // 192 KB of operand stages, cut into as many stages as the planes in use allow
   constexpr int SMEM = RING_BYTES + 1024 /*align slack*/ + 512 /*barriers*/ + EPI_WARPS * 32 * 33 * 4 /*swapped-epilogue tiles*/;
@@ -895,12 +910,8 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
     const int pairs = ctx().sm_count / 2;
     grid = 2 * (tiles < pairs ? tiles : pairs);
   }
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  if (ctx().prof_gemm) {
-    MB_CUDA(cudaEventCreate(&e0));
-    MB_CUDA(cudaEventCreate(&e1));
-    MB_CUDA(cudaEventRecord(e0, st));
-  }
+  GemmProfile prof(st);
+  MB_TRY(prof.begin());
   if (pair) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -919,11 +930,7 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
     kern<<<grid, NUM_THREADS, SMEM, st>>>(map_a, map_w, map_o, p);
   }
   MB_CUDA(cudaGetLastError());
-  if (e0) {
-    MB_CUDA(cudaEventRecord(e1, st));
-    ctx().prof_events.push_back(e0);
-    ctx().prof_events.push_back(e1);
-  }
+  MB_TRY(prof.end());
   count_launch();
   return MIMIR_B200_OK;
 }

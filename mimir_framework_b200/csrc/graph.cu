@@ -1201,7 +1201,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         if (L.read_split) e.x_split = splitp(L.in_v[0]); else e.x_f32 = f32p(L.in_v[0]);
         e.w_f32 = L.w_f32;
         e.w_split = L.w_split;
-        e.w_scale = L.w_scale;
+        e.w_scale = L.w_scale; e.w_ready = true;
         e.bias = d.use_bias ? L.w_f32 + static_cast<size_t>(L.in_f) * L.out_f : nullptr;
         e.activation = L.fused_act;
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
@@ -1216,7 +1216,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.batch = batch; e.seq = L.seq; e.embed = L.embed; e.heads = L.heads; e.causal = d.causal;
         e.precision = m->precision;
         if (L.read_split) e.x_split = splitp(L.in_v[0]); else e.x = f32p(L.in_v[0]);
-        e.wqkv_split = L.w_split; e.wout_split = L.w_split2; e.w_scale = L.w_scale; e.y = f32p(L.out_v); e.ws = ws;
+        e.wqkv_split = L.w_split; e.wout_split = L.w_split2; e.w_scale = L.w_scale; e.w_ready = true; e.y = f32p(L.out_v); e.ws = ws;
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
         if (m->is_twin) {
           e.kcache = L.kcache; e.vcache = L.vcache; e.max_seq = m->max_seq; e.decode_pos = m->decode_pos;
@@ -1241,7 +1241,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.batch = batch; e.ic = d.in_channels; e.oc = d.out_channels; e.h = L.h; e.w = L.w; e.ks = d.kernel;
         e.stride = d.stride; e.pad = d.padding; e.precision = m->precision;
         e.activation = d.activation ? MIMIR_B200_ELT_RELU : L.fused_act;
-        e.x = f32p(L.in_v[0]); e.w_split = L.w_split; e.w_f32 = L.w_f32; e.w_scale = L.w_scale; e.y = f32p(L.out_v); e.ws = ws;
+        e.x = f32p(L.in_v[0]); e.w_split = L.w_split; e.w_f32 = L.w_f32; e.w_scale = L.w_scale; e.w_ready = true; e.y = f32p(L.out_v); e.ws = ws;
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
         if (L.pre_norm >= 0) {
           const LayerRT& G = m->layers[L.pre_norm];
@@ -1327,7 +1327,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.batch = batch; e.q_len = L.seq; e.kv_len = L.kv_len; e.embed = L.embed; e.heads = L.heads; e.causal = d.causal;
         e.precision = m->precision;
         e.q_in = f32p(L.in_v[0]); e.kv_in = f32p(L.in_v[1]);
-        e.wq_split = L.w_split; e.wkv_split = L.w_split2; e.wout_split = L.w_split3; e.w_scale = L.w_scale;
+        e.wq_split = L.w_split; e.wkv_split = L.w_split2; e.wout_split = L.w_split3; e.w_scale = L.w_scale; e.w_ready = true;
         e.y = f32p(L.out_v); e.ws = ws;
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
         s = cross_attention_exec(e, st);

@@ -1,0 +1,45 @@
+// launch.cuh — launches with programmatic stream serialization (programmatic dependent launch).
+//
+// A kernel launched through launch_pdl may start while the kernel before it in the stream still runs: it must execute pdl_wait()
+// before it touches anything an earlier kernel writes, and before it writes anything an earlier kernel reads.  pdl_wait()
+// returns when every kernel the launch depends on has completed and its writes are visible; without a programmatic edge
+// (first kernel of a stream, after a copy) it returns at once.  pdl_launch_dependents() lets the next such kernel start.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <utility>
+
+#include "common.h"
+
+namespace mb {
+namespace {
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+int launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  MB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+  return MIMIR_B200_OK;
+}
+
+}  // namespace
+}  // namespace mb
