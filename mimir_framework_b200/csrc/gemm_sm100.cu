@@ -1059,6 +1059,20 @@ int launch_wait_timeout_selftest(unsigned long long limit_ns, cudaStream_t st) {
   return MIMIR_B200_OK;
 }
 
+namespace {
+// Estimated SM cycles of a launch in 128 x 256 tiles (the same model as gemm_split.cu's plan_split: the larger of MMA time and
+// operand loads per tile, whole waves, one exposed epilogue).
+double big_tile_cycles(const GemmArgs& g) {
+  const int products = 1 + (g.a_planes == 2) + (g.w_planes == 2);
+  const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
+  const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
+  const double k = g.conv_ks > 0 ? static_cast<double>(g.k) : static_cast<double>(round_up(g.k, 64));
+  const double mma = k / UMMA_K * products * 128.0, load = k * 2.0 * (g.a_planes * BM + g.w_planes * BN) / 40.0;
+  const double tile = (mma > load ? mma : load);
+  return 6000.0 + waves * (tile > 12000.0 ? tile : 12000.0) + (waves > 0 && tile > 12000.0 ? 12000.0 : 0.0);
+}
+}  // namespace
+
 int launch_gemm(const GemmArgs& g, cudaStream_t st) {
   if (g.m <= 0 || g.n <= 0 || g.k <= 0) return fail(MIMIR_B200_E_INVALID, "gemm: empty dimension");
   if (!g.a || !g.w) return fail(MIMIR_B200_E_INVALID, "gemm: null operand");
@@ -1073,6 +1087,14 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
       return fail(MIMIR_B200_E_INVALID, "gemm: bad shifted-convolution arguments");
   }
   const int bk = env_int("MIMIR_B200_GEMM_BK", (g.a_planes + g.w_planes <= 3) ? 64 : 32);
+  // launches that leave SMs without a 128 x 256 tile go to the split-K kernel with narrower tiles (never when the big tiles fill
+  // the GPU more than once over: re-reading the operands for narrow tiles then costs more than an even last wave gives)
+  const int sbk = (g.conv_ks == 0 || g.conv_c % 64 == 0) ? 64 : 32;
+  const long long big_tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
+  int bn = 0, splits = 0;
+  static const bool force_pairs = env_int("MIMIR_B200_GEMM_PAIR", -1) == 1;  // pairs wherever the form allows
+  if (!force_pairs && big_tiles < ctx().sm_count + ctx().sm_count / 2 && gemm_split_wanted(g, sbk, big_tile_cycles(g), &bn, &splits))
+    return launch_gemm_split(g, sbk, bn, splits, st);
   if (bk == 64 && (g.conv_ks == 0 || g.conv_c % 64 == 0)) return launch_gemm_t<64>(g, st);
   return launch_gemm_t<32>(g, st);
 }

@@ -1,0 +1,56 @@
+"""The split-K contraction kernel (csrc/gemm_split.cu) at the sizes where it can go wrong: one row, tile edges in every direction,
+K shorter than a block per split, every width and split count, row-major and channel-major outputs."""
+import numpy as np
+import pytest
+
+from mimir_framework_b200 import abi
+from mimir_framework_b200.abi import make_desc
+from oracle import port
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    from mimir_framework_b200 import runtime
+
+    runtime.init(0)
+    return runtime
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W, abi.PREC_BF16])
+@pytest.mark.parametrize("form,m,n,k", [("16,1", 17, 1, 64), ("16,8", 17, 129, 520), ("32,4", 33, 127, 300), ("48,2", 97, 256, 128), ("64,8", 65, 70, 1000),
+                                        ("96,1", 200, 300, 65), ("128,1", 129, 128, 1), ("128,8", 257, 385, 2048), ("", 40, 1000, 4100), ("", 333, 1000, 1000)])
+def test_linear_against_float64(rt, monkeypatch, precision, form, m, n, k):
+    if form:
+        monkeypatch.setenv("MIMIR_B200_GEMM_SPLIT", form)
+    r = np.random.default_rng(m * 7 + n)
+    x = r.standard_normal((m, k)).astype(np.float32)
+    w = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)
+    if precision != abi.PREC_BF16X2:
+        w = (w.view(np.uint32) & 0xffff0000).view(np.float32)  # exact in one plane
+    b, res = r.standard_normal(n).astype(np.float32), r.standard_normal((m, n)).astype(np.float32)
+    descs = [make_desc("l", "Linear", inputs=["x"], output="h", in_features=k, out_features=n, seq_len=m, use_bias=1, params_count=n * k + n),
+             make_desc("g", "GELU", inputs=["h"], output="a"), make_desc("s", "Add", inputs=["r", "a"], output="x")]
+    mod = rt.GraphModel(descs, precision)
+    mod.upload_weights(0, np.concatenate([w.ravel(), b]))
+    mod.plan({"x": (m * k, False), "r": (m * n, False)}, 1)
+    got = mod.forward({"x": (x.ravel(), False), "r": (res.ravel(), False)}, 1, m * n).reshape(m, n)
+    mod.close()
+    h = x.astype(np.float64) @ w.astype(np.float64).T + b
+    want = h * 0.5 * (1 + np.tanh(0.7978845608 * (h + 0.044715 * h ** 3))) + res
+    tol = 2e-3 if precision == abi.PREC_BF16 else 1e-5
+    assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("form", ["16,1", "48,2", "128,8", ""])
+@pytest.mark.parametrize("batch,ic,oc,h,w,k,stride,pad", [(1, 64, 130, 9, 7, 3, 1, 1), (3, 32, 40, 5, 11, 1, 1, 0), (2, 96, 16, 8, 8, 5, 1, 2), (2, 3, 70, 17, 19, 7, 2, 3)])
+def test_convolution_against_the_port(rt, monkeypatch, form, batch, ic, oc, h, w, k, stride, pad):
+    if form:
+        monkeypatch.setenv("MIMIR_B200_GEMM_SPLIT", form)
+    r = np.random.default_rng(batch * ic + oc)
+    x = r.standard_normal((batch, ic * h * w)).astype(np.float32)
+    wt = (r.standard_normal(oc * ic * k * k) / np.sqrt(ic * k * k)).astype(np.float32)
+    got = rt.conv2d(x, wt, batch, ic, oc, h, w, k, stride, pad).reshape(batch, -1)
+    want = np.stack([port.conv2d(x[i], wt, ic, oc, h, w, k, stride, pad, False).ravel() for i in range(batch)])
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
