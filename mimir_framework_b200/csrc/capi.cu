@@ -69,7 +69,13 @@ int dev_alloc(void** p, size_t bytes, const char* tag) {
     return fail(MIMIR_B200_E_OOM_BUDGET, "HBM budget refused %zu bytes for %s (%s; limit %zu, in use %zu)", bytes, tag,
                 why == 2 ? "allocations are blocked" : why == 3 ? "allocations are frozen" : "over the limit", ctx().guard.limit,
                 ctx().guard.current);
+  if (ctx().temps.bytes && ctx().guard.limit && ctx().guard.current + ctx().temps.bytes > ctx().guard.limit) ctx().temps.trim();
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx().temps.bytes) {
+    cudaGetLastError();
+    ctx().temps.trim();
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     ctx().guard.release(bytes);
     *p = nullptr;
@@ -84,7 +90,49 @@ void dev_free(void* p, size_t bytes) {
   ctx().guard.release(bytes);
 }
 
+void* TempPool::take(size_t* size) {
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = idle.lower_bound(*size);
+  if (it == idle.end() || it->first / 2 > *size) return nullptr;
+  void* p = it->second;
+  *size = it->first;
+  bytes -= it->first;
+  idle.erase(it);
+  return p;
+}
+bool TempPool::put(void* p, size_t size) {
+  std::lock_guard<std::mutex> lk(mu);
+  if (bytes + size > CAP) return false;
+  idle.emplace(size, p);
+  bytes += size;
+  return true;
+}
+void TempPool::trim() {
+  std::lock_guard<std::mutex> lk(mu);
+  for (auto& kv : idle) cudaFree(kv.second);
+  idle.clear();
+  bytes = 0;
+}
+
+int temp_alloc(void** p, size_t* bytes, const char* tag) {
+  *bytes = (*bytes + 511) & ~size_t(511);
+  if (void* q = ctx().initialised ? ctx().temps.take(bytes) : nullptr) {
+    if (ctx().guard.request_why(*bytes) == 0) {
+      *p = q;
+      return MIMIR_B200_OK;
+    }
+    cudaFree(q);  // refused: the ordinary path below words the refusal
+  }
+  return dev_alloc(p, *bytes, tag);
+}
+void temp_free(void* p, size_t bytes, bool idle) {
+  if (p && idle && ctx().temps.put(p, bytes)) ctx().guard.release(bytes);
+  else dev_free(p, bytes);
+}
+
 void release_owned_buffers() {
+  ctx().temps.trim();
+  release_host_copier();
   OwnedBuffers& ob = ctx().owned;
   std::lock_guard<std::mutex> lk(ob.mu);
   for (auto& kv : ob.live) dev_free(kv.first, kv.second.bytes);
@@ -95,9 +143,16 @@ void release_owned_buffers() {
 
 // Reads (and clears) the word that kernels with bounded waits set when a wait gave up.
 int check_device_error_word(cudaStream_t st) {
-  int w = 0;
-  MB_CUDA(cudaMemcpyAsync(&w, ctx().dev_error_word, sizeof(int), cudaMemcpyDeviceToHost, st));
+  MB_TRY(enqueue_error_word(st));
   MB_CUDA(cudaStreamSynchronize(st));
+  return read_error_word(st);
+}
+int enqueue_error_word(cudaStream_t st) {
+  MB_CUDA(cudaMemcpyAsync(ctx().host_error_word, ctx().dev_error_word, sizeof(int), cudaMemcpyDeviceToHost, st));
+  return MIMIR_B200_OK;
+}
+int read_error_word(cudaStream_t st) {
+  const int w = *static_cast<volatile int*>(ctx().host_error_word);
   if (w != 0) {
     cudaMemsetAsync(ctx().dev_error_word, 0, sizeof(int), st);
     cudaStreamSynchronize(st);
@@ -419,6 +474,10 @@ int mimir_b200_init(int device, size_t hbm_budget_bytes) {
   }
   c.dev_error_word = static_cast<int*>(w);
   MB_CUDA(cudaMemset(c.dev_error_word, 0, 256));
+  void* hw = nullptr;
+  MB_CUDA(cudaHostAlloc(&hw, 256, cudaHostAllocPortable));
+  c.host_error_word = static_cast<int*>(hw);
+  *c.host_error_word = 0;
   return MIMIR_B200_OK;
 }
 
@@ -648,7 +707,7 @@ int mimir_b200_linear_forward_ex(const float* input, const float* weights, const
     e.w_split = static_cast<const __nv_bfloat16*>(wsplit);
   }
   MB_TRY(linear_exec(e, nullptr));
-  return finish_download(output, e.y_f32, static_cast<size_t>(batch) * out_f);
+  return finish_download(t, output, e.y_f32, static_cast<size_t>(batch) * out_f);
 }
 
 int mimir_b200_linear_forward(const float* input, const float* weights, const float* bias_or_null, float* output, int batch,
@@ -676,7 +735,7 @@ int mimir_b200_matmul(const float* A, const float* B, float* C, int M, int K, in
   g.w = static_cast<const __nv_bfloat16*>(bs);
   g.m = M; g.n = N; g.k = K; g.out_f32 = c; g.ldo = N;
   MB_TRY(launch_gemm(g, nullptr));
-  return finish_download(C, c, static_cast<size_t>(M) * N);
+  return finish_download(t, C, c, static_cast<size_t>(M) * N);
 }
 
 int mimir_b200_attention(const float* x, const float* wqkv_wout, float* y, int batch, int seq, int embed, int heads,
@@ -703,7 +762,7 @@ int mimir_b200_attention(const float* x, const float* wqkv_wout, float* y, int b
   e.wout_split = static_cast<const __nv_bfloat16*>(wo);
   MB_TRY(t.alloc(&e.ws, attention_ws_bytes(batch, seq, embed, heads, e.precision), "attn.ws"));
   MB_TRY(attention_exec(e, nullptr));
-  return finish_download(y, e.y, rows * E);
+  return finish_download(t, y, e.y, rows * E);
 }
 
 int mimir_b200_conv2d(const float* x, const float* w, float* y, int batch, int ic, int oc, int h, int wd, int k, int stride,
@@ -731,7 +790,7 @@ int mimir_b200_conv2d(const float* x, const float* w, float* y, int batch, int i
   e.w_split = static_cast<const __nv_bfloat16*>(ws);
   MB_TRY(t.alloc(&e.ws, conv_ws_bytes(batch, ic, h, wd, k, stride, pad, e.precision), "conv.ws"));
   MB_TRY(conv_exec(e, nullptr));
-  return finish_download(y, e.y, static_cast<size_t>(batch) * oc * oh * ow);
+  return finish_download(t, y, e.y, static_cast<size_t>(batch) * oc * oh * ow);
 }
 
 int mimir_b200_layernorm(const float* x, const float* gamma, const float* beta, float* y, long long rows, int n, float eps) {
@@ -745,7 +804,7 @@ int mimir_b200_layernorm(const float* x, const float* gamma, const float* beta, 
   if (gamma && beta) MB_TRY(t.upload(&db, beta, n, "ln.b"));
   MB_TRY(t.out(&dy, static_cast<size_t>(rows) * n, "ln.y"));
   MB_TRY(launch_layernorm(dx, dg, db, dy, rows, n, eps, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(rows) * n);
+  return finish_download(t, y, dy, static_cast<size_t>(rows) * n);
 }
 
 int mimir_b200_rmsnorm(const float* x, const float* gamma, long long n_gamma, float* y, int batch, long long n, float eps) {
@@ -758,7 +817,7 @@ int mimir_b200_rmsnorm(const float* x, const float* gamma, long long n_gamma, fl
   if (gamma && n_gamma > 0) MB_TRY(t.upload(&dg, gamma, static_cast<size_t>(n_gamma), "rms.g"));
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * n, "rms.y"));
   MB_TRY(launch_rmsnorm(dx, dg, dg ? n_gamma : 0, dy, batch, n, eps, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(batch) * n);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * n);
 }
 
 int mimir_b200_groupnorm(const float* x, const float* gamma, const float* beta, float* y, int batch, int channels, int h,
@@ -774,7 +833,7 @@ int mimir_b200_groupnorm(const float* x, const float* gamma, const float* beta, 
   if (gamma && beta) MB_TRY(t.upload(&db, beta, channels, "gn.b"));
   MB_TRY(t.out(&dy, n, "gn.y"));
   MB_TRY(launch_groupnorm(dx, dg, db, dy, batch, channels, h * w, groups, eps, act, nullptr, nullptr));
-  return finish_download(y, dy, n);
+  return finish_download(t, y, dy, n);
 }
 
 int mimir_b200_softmax(const float* x, float* y, int batch, long long n, int log_softmax) {
@@ -786,7 +845,7 @@ int mimir_b200_softmax(const float* x, float* y, int batch, long long n, int log
   MB_TRY(t.upload(&dx, x, static_cast<size_t>(batch) * n, "sm.x"));
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * n, "sm.y"));
   MB_TRY(launch_softmax(dx, dy, batch, n, log_softmax, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(batch) * n);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * n);
 }
 
 int mimir_b200_eltwise(int op, const float* a, const float* b, float* y, int batch, long long n, long long nb) {
@@ -799,7 +858,7 @@ int mimir_b200_eltwise(int op, const float* a, const float* b, float* y, int bat
   if (b && nb > 0) MB_TRY(t.upload(&db, b, static_cast<size_t>(batch) * nb, "elt.b"));
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * n, "elt.y"));
   MB_TRY(launch_eltwise(op, da, db, dy, batch, n, nb, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(batch) * n);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * n);
 }
 
 int mimir_b200_embedding(const float* ids_f32, const int32_t* ids_i32, const float* table, float* y, long long n_ids,
@@ -822,7 +881,7 @@ int mimir_b200_embedding(const float* ids_f32, const int32_t* ids_i32, const flo
   }
   MB_TRY(t.out(&dy, static_cast<size_t>(n_ids) * dim, "emb.y"));
   MB_TRY(launch_embedding(df, di, dt, dy, n_ids, vocab, dim, padding_idx, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(n_ids) * dim);
+  return finish_download(t, y, dy, static_cast<size_t>(n_ids) * dim);
 }
 
 int mimir_b200_upsample_nearest(const float* x, float* y, int batch, int channels, int in_h, int in_w, int scale_h,
@@ -836,7 +895,7 @@ int mimir_b200_upsample_nearest(const float* x, float* y, int batch, int channel
   MB_TRY(t.upload(&dx, x, n, "up.x"));
   MB_TRY(t.out(&dy, n * scale_h * scale_w, "up.y"));
   MB_TRY(launch_upsample_nearest(dx, dy, batch, channels, in_h, in_w, scale_h, scale_w, nullptr));
-  return finish_download(y, dy, n * scale_h * scale_w);
+  return finish_download(t, y, dy, n * scale_h * scale_w);
 }
 
 int mimir_b200_permute(const float* x, float* y, int batch, int ndim, const int* shape, const int* dims) {
@@ -852,7 +911,7 @@ int mimir_b200_permute(const float* x, float* y, int batch, int ndim, const int*
   MB_TRY(t.upload(&dx, x, per * batch, "perm.x"));
   MB_TRY(t.out(&dy, per * batch, "perm.y"));
   MB_TRY(launch_permute(dx, dy, batch, ndim, shape, dims, nullptr));
-  return finish_download(y, dy, per * batch);
+  return finish_download(t, y, dy, per * batch);
 }
 
 int mimir_b200_token_mean_pool(const float* x, float* y, int batch, int seq, int dim) {
@@ -865,7 +924,7 @@ int mimir_b200_token_mean_pool(const float* x, float* y, int batch, int seq, int
   MB_TRY(t.upload(&dx, x, static_cast<size_t>(batch) * seq * dim, "tmp.x"));
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * dim, "tmp.y"));
   MB_TRY(launch_token_mean_pool(dx, dy, batch, seq, dim, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(batch) * dim);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * dim);
 }
 
 int mimir_b200_global_avgpool(const float* x, float* y, int batch, int channels, int h, int w) {
@@ -877,7 +936,7 @@ int mimir_b200_global_avgpool(const float* x, float* y, int batch, int channels,
   MB_TRY(t.upload(&dx, x, static_cast<size_t>(batch) * channels * h * w, "gap.x"));
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * channels, "gap.y"));
   MB_TRY(launch_global_avgpool(dx, dy, batch, channels, h * w, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(batch) * channels);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * channels);
 }
 
 // ---- device-pointer forms -------------------------------------------------------------------

@@ -83,7 +83,7 @@ int mimir_b200_cross_attention(const float* query, const float* key_value, const
   e.wout_split = static_cast<const __nv_bfloat16*>(wo);
   MB_TRY(t.alloc(&e.ws, cross_attention_ws_bytes(batch, q_len, kv_len, embed, e.precision), "xattn.ws"));
   MB_TRY(cross_attention_exec(e, nullptr));
-  return finish_download(y, e.y, qr * E);
+  return finish_download(t, y, e.y, qr * E);
 }
 
 int mimir_b200_eltwise_alpha(int op, const float* a, const float* b, float* y, int batch, long long n, long long nb, float alpha) {
@@ -96,7 +96,7 @@ int mimir_b200_eltwise_alpha(int op, const float* a, const float* b, float* y, i
   if (b && nb > 0) MB_TRY(t.upload(&db, b, static_cast<size_t>(batch) * nb, "elt.b"));
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * n, "elt.y"));
   MB_TRY(launch_eltwise(op, da, db, dy, batch, n, nb, nullptr, alpha));
-  return finish_download(y, dy, static_cast<size_t>(batch) * n);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * n);
 }
 
 int mimir_b200_depthwise_conv2d(const float* x, const float* w, const float* bias, float* y, int batch, int channels, int h, int wd,
@@ -116,7 +116,7 @@ int mimir_b200_depthwise_conv2d(const float* x, const float* w, const float* bia
   const size_t ny = static_cast<size_t>(batch) * channels * oh * ow;
   MB_TRY(t.out(&dy, ny, "dw.y"));
   MB_TRY(launch_depthwise_conv2d(dx, dw, db, dy, batch, channels, h, wd, k, stride, pad, static_cast<int64_t>(nw), nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_conv1d(const float* x, const float* w, const float* bias, float* y, int batch, int ic, int oc, int len, int k, int stride,
@@ -136,7 +136,7 @@ int mimir_b200_conv1d(const float* x, const float* w, const float* bias, float* 
   const size_t ny = static_cast<size_t>(batch) * oc * olen;
   MB_TRY(t.out(&dy, ny, "c1.y"));
   MB_TRY(launch_conv1d(dx, dw, db, dy, batch, ic, oc, len, k, stride, pad, static_cast<int64_t>(nw), nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_conv_transpose2d(const float* x, const float* w, float* y, int batch, int ic, int oc, int h, int wd, int k, int stride,
@@ -154,7 +154,7 @@ int mimir_b200_conv_transpose2d(const float* x, const float* w, float* y, int ba
   const size_t ny = static_cast<size_t>(batch) * oc * oh * ow;
   MB_TRY(t.out(&dy, ny, "ct.y"));
   MB_TRY(launch_conv_gather(dx, dw, dy, batch, ic, oc, h, wd, oh, ow, k, stride, pad, relu, nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_conv2d_dilated(const float* x, const float* w, const float* bias, float* y, int batch, int in_c, int out_c, int in_h,
@@ -175,7 +175,7 @@ int mimir_b200_conv2d_dilated(const float* x, const float* w, const float* bias,
   const size_t ny = static_cast<size_t>(batch) * out_c * oh * ow;
   MB_TRY(t.out(&dy, ny, "sconv.y"));
   MB_TRY(launch_conv2d_dilated(dx, dw, db, dy, batch, in_c, out_c, in_h, in_w, kernel, stride, padding, dilation, nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_conv_transpose2d_scatter(const float* x, const float* w, const float* bias, float* y, int batch, int in_c, int out_c,
@@ -194,7 +194,7 @@ int mimir_b200_conv_transpose2d_scatter(const float* x, const float* w, const fl
   const size_t ny = static_cast<size_t>(batch) * out_c * oh * ow;
   MB_TRY(t.out(&dy, ny, "sconvt.y"));
   MB_TRY(launch_conv_transpose2d_scatter(dx, dw, db, dy, batch, in_c, out_c, in_h, in_w, kernel, stride, padding, nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_batchnorm_batchstats(const float* x, const float* gamma, const float* beta, float* y, int batch, int channels,
@@ -211,7 +211,7 @@ int mimir_b200_batchnorm_batchstats(const float* x, const float* gamma, const fl
   MB_TRY(t.upload(&db, beta, static_cast<size_t>(channels), "bnt.b"));
   MB_TRY(t.out(&dy, n, "bnt.y"));
   MB_TRY(launch_batchnorm_batchstats(dx, dg, db, dy, batch, channels, spatial, eps, nullptr));
-  return finish_download(y, dy, n);
+  return finish_download(t, y, dy, n);
 }
 
 int mimir_b200_pool2d(int is_max, const float* x, float* y, int batch, int channels, int h, int wd, int kh, int kw, int stride_h,
@@ -228,7 +228,7 @@ int mimir_b200_pool2d(int is_max, const float* x, float* y, int batch, int chann
   const size_t ny = static_cast<size_t>(batch) * channels * oh * ow;
   MB_TRY(t.out(&dy, ny, "pool.y"));
   MB_TRY(launch_pool2d(is_max, dx, dy, batch, channels, h, wd, kh, kw, stride_h, stride_w, pad_h, pad_w, nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_pad2d(int mode, const float* x, float* y, int batch, int channels, int h, int wd, int pad_h, int pad_w) {
@@ -242,7 +242,7 @@ int mimir_b200_pad2d(int mode, const float* x, float* y, int batch, int channels
   const size_t ny = static_cast<size_t>(batch) * channels * (h + 2 * pad_h) * (wd + 2 * pad_w);
   MB_TRY(t.out(&dy, ny, "pad.y"));
   MB_TRY(launch_pad2d(mode, dx, dy, batch, channels, h, wd, pad_h, pad_w, nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_pixel_shuffle(const float* x, float* y, int batch, int in_channels, int h, int wd, int r) {
@@ -256,7 +256,7 @@ int mimir_b200_pixel_shuffle(const float* x, float* y, int batch, int in_channel
   MB_TRY(t.upload(&dx, x, n, "ps.x"));
   MB_TRY(t.out(&dy, n, "ps.y"));
   MB_TRY(launch_pixel_shuffle(dx, dy, batch, in_channels, h, wd, r, nullptr));
-  return finish_download(y, dy, n);
+  return finish_download(t, y, dy, n);
 }
 
 int mimir_b200_upsample_bilinear(const float* x, float* y, int batch, int channels, int h, int wd, int out_h, int out_w,
@@ -271,7 +271,7 @@ int mimir_b200_upsample_bilinear(const float* x, float* y, int batch, int channe
   const size_t ny = static_cast<size_t>(batch) * channels * out_h * out_w;
   MB_TRY(t.out(&dy, ny, "bil.y"));
   MB_TRY(launch_upsample_bilinear(dx, dy, batch, channels, h, wd, out_h, out_w, half_pixel, nullptr));
-  return finish_download(y, dy, ny);
+  return finish_download(t, y, dy, ny);
 }
 
 int mimir_b200_batch_matmul(const float* A, const float* B, float* C, long long nb, int M, int K, int N) {
@@ -284,7 +284,7 @@ int mimir_b200_batch_matmul(const float* A, const float* B, float* C, long long 
   MB_TRY(t.upload(&db, B, static_cast<size_t>(nb) * K * N, "bmm.b"));
   MB_TRY(t.out(&dc, static_cast<size_t>(nb) * M * N, "bmm.c"));
   MB_TRY(launch_batch_matmul(da, db, dc, nb, M, K, N, nullptr));
-  return finish_download(C, dc, static_cast<size_t>(nb) * M * N);
+  return finish_download(t, C, dc, static_cast<size_t>(nb) * M * N);
 }
 
 int mimir_b200_batchnorm_inference(const float* x, const float* w, long long n_w, float* y, int batch, long long n, float eps) {
@@ -298,7 +298,7 @@ int mimir_b200_batchnorm_inference(const float* x, const float* w, long long n_w
   MB_TRY(t.out(&dy, static_cast<size_t>(batch) * n, "bn.y"));
   MB_TRY(launch_layernorm(dx, nullptr, nullptr, dy, batch, n, eps, nullptr));
   if (dw) MB_TRY(launch_scale_prefix(dy, dw, batch, n, n_w, nullptr));
-  return finish_download(y, dy, static_cast<size_t>(batch) * n);
+  return finish_download(t, y, dy, static_cast<size_t>(batch) * n);
 }
 
 int mimir_b200_batchnorm_running(const float* x, const float* gamma, const float* beta, const float* running_mean,
@@ -317,7 +317,7 @@ int mimir_b200_batchnorm_running(const float* x, const float* gamma, const float
   MB_TRY(t.upload(&dv, running_var, channels, "bn.var"));
   MB_TRY(t.out(&dy, n, "bn.y"));
   MB_TRY(launch_batchnorm_running(dx, dg, db, dm, dv, dy, batch, channels, spatial, eps, nullptr));
-  return finish_download(y, dy, n);
+  return finish_download(t, y, dy, n);
 }
 
 int mimir_b200_attention_qkv(const float* q, const float* k, const float* v, float* y, int batch, int seq, int d_model,
@@ -336,7 +336,7 @@ int mimir_b200_attention_qkv(const float* q, const float* k, const float* v, flo
   MB_TRY(t.out(&dy, n, "attn.y"));
   a.ldq = d_model; a.ldkv = d_model; a.q_len = seq; a.kv_len = seq;
   MB_TRY(launch_attention_core_view(a, dy, batch, d_model, num_heads, 0, nullptr));
-  return finish_download(y, dy, n);
+  return finish_download(t, y, dy, n);
 }
 
 }  // extern "C"

@@ -60,15 +60,34 @@ struct OwnedBuffers {
   size_t total_allocated = 0, num_allocations = 0, local_cap = 0;
 };
 
+// Device buffers of finished host-pointer calls, kept for the next one: cudaMalloc and cudaFree of a call's five or six buffers
+// (each free waits for the device and unmaps) took 2.9 ms of the 3.8 ms that a 512 x 768 x 3072 Linear needed.  Bounded by
+// CAP bytes; not counted by the guard while idle (a reused buffer is requested from it like a new one); given back when the
+// guard's limit or the device runs short and at shutdown.  Buffers enter the pool only after the call has synchronised.
+struct TempPool {
+  static constexpr size_t CAP = size_t(512) << 20;
+  std::mutex mu;
+  std::multimap<size_t, void*> idle;
+  size_t bytes = 0;
+  void* take(size_t* size);        // the smallest idle buffer of at least *size (and at most twice it); *size becomes its size
+  bool put(void* p, size_t size);  // false: no room, the caller frees it
+  void trim();                     // frees every idle buffer
+};
+
+struct HostCopier;  // host_copy.cu
+
 struct Context {
   bool initialised = false;
   int device = 0;
   int sm_count = 148;
   Guard guard;
   OwnedBuffers owned;
+  TempPool temps;
+  HostCopier* copier = nullptr;
   std::atomic<uint64_t> launches{0};
   // One device word that kernels with bounded waits set when a wait gives up.
   int* dev_error_word = nullptr;
+  int* host_error_word = nullptr;  // page-locked copy of it that check_device_error_word reads through
   // Optional live timing of the contraction kernel: pairs of events recorded on the launching
   // stream around every GEMM launch while enabled (read back by mimir_b200_profile_read).
   bool prof_gemm = false;
@@ -112,6 +131,14 @@ int model_device(MimirB200ModelHandle m);
 // Budgeted device allocation: every cudaMalloc of the backend goes through these.
 int dev_alloc(void** p, size_t bytes, const char* tag);
 void dev_free(void* p, size_t bytes);
+// The same through the pool of the current device's idle call buffers; *bytes becomes the buffer's size.
+int temp_alloc(void** p, size_t* bytes, const char* tag);
+void temp_free(void* p, size_t bytes, bool idle);
+// Copies in stream order that may involve pageable host memory (host_copy.cu).  The host side is done with when they return
+// for pageable memory (as with cudaMemcpyAsync); page-locked memory is copied asynchronously.
+int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);
+int copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
+void release_host_copier();
 // Frees every buffer of the RuntimeAllocator verbs on the current device (shutdown).
 void release_owned_buffers();
 

@@ -1653,7 +1653,10 @@ int mimir_b200_model_upload_weights(MimirB200ModelHandle m, int layer_index, con
   if (n != 0 && !host) return fail(MIMIR_B200_E_INVALID, "upload_weights: null host pointer");
   float* dev = nullptr;
   MB_TRY(mimir_b200_model_weights_device(m, layer_index, n, &dev));
-  if (n) MB_CUDA(cudaMemcpy(dev, host, n * 4, cudaMemcpyHostToDevice));
+  if (n) {
+    MB_TRY(copy_to_device(dev, host, n * 4, nullptr));
+    MB_CUDA(cudaStreamSynchronize(nullptr));
+  }
   return MIMIR_B200_OK;
 }
 
@@ -1795,11 +1798,11 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
       float* slot = reinterpret_cast<float*>(arena + t.off_f32);
       if (t.broadcast_input) {
         // every micro-batch: the slot may have been reused after the input's last consumer
-        MB_CUDA(cudaMemcpyAsync(slot, inputs[i].data, static_cast<size_t>(t.n) * 4, cudaMemcpyHostToDevice, m->s_h2d));
+        MB_TRY(copy_to_device(slot, inputs[i].data, static_cast<size_t>(t.n) * 4, m->s_h2d));
         if (micro > 1) MB_TRY(launch_broadcast_rows(slot, slot + t.n, micro - 1, t.n, m->s_h2d));
       } else {
         const float* src = static_cast<const float*>(inputs[i].data) + static_cast<size_t>(c) * micro * t.n;
-        MB_CUDA(cudaMemcpyAsync(slot, src, static_cast<size_t>(t.n) * micro * 4, cudaMemcpyHostToDevice, m->s_h2d));
+        MB_TRY(copy_to_device(slot, src, static_cast<size_t>(t.n) * micro * 4, m->s_h2d));
       }
     }
     MB_CUDA(cudaEventRecord(m->ev_h2d[c], m->s_h2d));
@@ -1809,14 +1812,14 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
     MB_TRY(run_layers_cached(m, micro, b, m->s_comp, arena));
     MB_CUDA(cudaEventRecord(m->ev_comp[c], m->s_comp));
     MB_CUDA(cudaStreamWaitEvent(m->s_d2h, m->ev_comp[c], 0));
-    MB_CUDA(cudaMemcpyAsync(out_host + static_cast<size_t>(c) * micro * ot.n, arena + ot.off_f32, static_cast<size_t>(ot.n) * micro * 4,
-                            cudaMemcpyDeviceToHost, m->s_d2h));
+    MB_TRY(copy_to_host(out_host + static_cast<size_t>(c) * micro * ot.n, arena + ot.off_f32, static_cast<size_t>(ot.n) * micro * 4, m->s_d2h));
     MB_CUDA(cudaEventRecord(m->ev_d2h[c], m->s_d2h));
   }
   MB_CUDA(cudaEventRecord(m->ev1, m->s_comp));
+  MB_TRY(enqueue_error_word(m->s_d2h));  // (the copy-out stream has waited for every micro-batch's compute)
   MB_CUDA(cudaStreamSynchronize(m->s_d2h));
-  MB_CUDA(cudaStreamSynchronize(m->s_comp));
-  MB_TRY(check_device_error_word(m->s_comp));
+  MB_CUDA(cudaEventSynchronize(m->ev1));
+  MB_TRY(read_error_word(m->s_comp));
   cudaEventElapsedTime(&m->last_ms, m->ev0, m->ev1);
   ctx().stats.ms_last_forward = m->last_ms;
   ctx().stats.flops_last_forward = m->flops * P;

@@ -8,21 +8,24 @@
 
 namespace mb {
 
-// Device buffers of one host-pointer call; everything is released when the call returns.
+// Device buffers of one host-pointer call, from the pool of idle buffers; back to it when the call returns (freed, which
+// waits for the device, when the call failed before it had synchronised).
 struct Temps {
   std::vector<std::pair<void*, size_t>> bufs;
+  bool synced = false;
   ~Temps() {
-    for (auto& b : bufs) dev_free(b.first, b.second);
+    for (auto& b : bufs) temp_free(b.first, b.second, synced);
   }
   int alloc(void** p, size_t bytes, const char* tag) {
-    MB_TRY(dev_alloc(p, bytes ? bytes : 4, tag));
-    bufs.emplace_back(*p, bytes ? bytes : 4);
+    size_t got = bytes ? bytes : 4;
+    MB_TRY(temp_alloc(p, &got, tag));
+    bufs.emplace_back(*p, got);
     return MIMIR_B200_OK;
   }
   int upload(const float** dev, const float* host, size_t n, const char* tag) {
     void* p;
     MB_TRY(alloc(&p, n * sizeof(float), tag));
-    MB_CUDA(cudaMemcpy(p, host, n * sizeof(float), cudaMemcpyHostToDevice));
+    MB_TRY(copy_to_device(p, host, n * sizeof(float), nullptr));
     *dev = static_cast<const float*>(p);
     return MIMIR_B200_OK;
   }
@@ -34,10 +37,13 @@ struct Temps {
   }
 };
 
-inline int finish_download(float* host, const float* dev, size_t n) {
-  MB_TRY(check_device_error_word(nullptr));
-  MB_CUDA(cudaMemcpy(host, dev, n * sizeof(float), cudaMemcpyDeviceToHost));
-  return MIMIR_B200_OK;
+// The last step of a call: result to the host, one synchronisation, device error word.
+inline int finish_download(Temps& t, float* host, const float* dev, size_t n) {
+  MB_TRY(enqueue_error_word(nullptr));
+  MB_TRY(copy_to_host(host, dev, n * sizeof(float), nullptr));
+  MB_CUDA(cudaStreamSynchronize(nullptr));
+  t.synced = true;
+  return read_error_word(nullptr);
 }
 
 #define MB_REQUIRE_INIT() \

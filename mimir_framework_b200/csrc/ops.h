@@ -10,7 +10,10 @@ namespace mb {
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 void precision_planes(int precision, int* a_planes, int* w_planes);
 size_t split_bytes(int64_t rows, int k, int planes);
+// reads (and clears) the word that bounded waits set; the two halves let a caller fold the copy into a synchronisation of its own
 int check_device_error_word(cudaStream_t st);
+int enqueue_error_word(cudaStream_t st);
+int read_error_word(cudaStream_t st);
 
 struct LinearExec {
   int rows = 0, in_f = 0, out_f = 0;
