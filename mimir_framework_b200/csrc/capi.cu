@@ -181,6 +181,22 @@ bool linear_uses_skinny(int rows, int precision) {
   return rows <= 16;
 }
 
+bool linear_takes_layernorm(int rows, int in_f, int out_f) { return rows <= 16 && skinny_cluster_supported(rows, in_f, out_f); }
+
+// y = act(norm(x) . w^T + bias) (+ residual) for at most 16 rows: one launch where the weights fit a wave of CTAs, else the
+// streaming kernel and its finishing kernel
+static int skinny_linear(const float* x, const float* w, const float* bias, float* y, int rows, int k, int n, int act, const PreLayerNorm& pre,
+                         bool w_ready, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual) {
+  if (skinny_cluster_supported(rows, k, n) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
+    SkinnyClusterArgs a;
+    a.x = x; a.w = w; a.bias = bias; a.residual = residual; a.y = y; a.m = rows; a.k = k; a.n = n; a.activation = act; a.w_ready = w_ready;
+    a.ln = pre.on; a.gamma = pre.gamma; a.beta = pre.gamma ? pre.beta : nullptr; a.eps = pre.eps;
+    return launch_skinny_cluster(a, st);
+  }
+  if (pre.on) return fail(MIMIR_B200_E_INVALID, "linear: a folded LayerNorm needs the cluster kernel");
+  return launch_skinny_linear(x, w, bias, y, rows, k, n, act, scratch, scratch_bytes, st, residual);
+}
+
 size_t linear_ws_bytes(int rows, int in_f, int out_f, int precision, bool a_presplit) {
   if (linear_uses_skinny(rows, precision)) return align256(skinny_scratch_bytes(rows, in_f, out_f));
   if (a_presplit) return 0;
@@ -192,8 +208,8 @@ size_t linear_ws_bytes(int rows, int in_f, int out_f, int precision, bool a_pres
 int linear_exec(const LinearExec& e, cudaStream_t st) {
   if (linear_uses_skinny(e.rows, e.precision)) {
     if (!e.x_f32 || !e.w_f32 || !e.y_f32) return fail(MIMIR_B200_E_INVALID, "linear: skinny path needs fp32 operands");
-    return launch_skinny_linear(e.x_f32, e.w_f32, e.bias, e.y_f32, e.rows, e.in_f, e.out_f, e.activation, static_cast<float*>(e.ws),
-                                e.ws_bytes, st, e.residual);
+    return skinny_linear(e.x_f32, e.w_f32, e.bias, e.y_f32, e.rows, e.in_f, e.out_f, e.activation, e.pre, e.w_ready,
+                         static_cast<float*>(e.ws), e.ws_bytes, st, e.residual);
   }
   int ap, wp;
   precision_planes(e.precision, &ap, &wp);
@@ -253,7 +269,7 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
   bool qkv_as_planes = false;
   const bool stream_w = e.decode_pos >= 0 && e.wqkv_t_f32 && e.wout_t_f32 && e.x && rows <= 16 && e.skinny_scratch;
   if (stream_w) {
-    MB_TRY(launch_skinny_linear(e.x, e.wqkv_t_f32, nullptr, qkv, rows, e.embed, 3 * e.embed, -1, e.skinny_scratch, e.skinny_scratch_bytes, st));
+    MB_TRY(skinny_linear(e.x, e.wqkv_t_f32, nullptr, qkv, rows, e.embed, 3 * e.embed, -1, e.pre, e.w_ready, e.skinny_scratch, e.skinny_scratch_bytes, st, nullptr));
   } else {
     if (!e.x_split) MB_TRY(launch_split(e.x, xs, rows, e.embed, ap, st));
     GemmArgs g;
@@ -287,8 +303,8 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
     } else
       MB_TRY(launch_attention_core_view(a, att, e.batch, e.embed, e.heads, 0, st));
     if (stream_w) {
-      return launch_skinny_linear(att, e.wout_t_f32, nullptr, e.y, rows, e.embed, e.embed, -1, e.skinny_scratch, e.skinny_scratch_bytes, st,
-                                  e.residual);
+      return skinny_linear(att, e.wout_t_f32, nullptr, e.y, rows, e.embed, e.embed, -1, PreLayerNorm(), e.w_ready, e.skinny_scratch,
+                           e.skinny_scratch_bytes, st, e.residual);
     }
     MB_TRY(launch_split(att, xs, rows, e.embed, ap, st));
   } else

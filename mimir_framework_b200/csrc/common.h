@@ -218,6 +218,18 @@ int launch_wait_timeout_selftest(unsigned long long limit_ns, cudaStream_t st);
 int launch_skinny_linear(const float* x, const float* w, const float* bias, float* y, int m, int k, int n,
                          int activation, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual = nullptr);
 size_t skinny_scratch_bytes(int m, int k, int n);
+// skinny_cluster.cu: the same for weight matrices that fit one wave of CTAs; one launch, no scratch.  ln: x is normalised row by
+// row (mean / variance over k) with gamma and beta before the product.
+struct SkinnyClusterArgs {
+  const float* x = nullptr; const float* w = nullptr; const float* bias = nullptr; const float* residual = nullptr; float* y = nullptr;
+  bool ln = false;
+  const float* gamma = nullptr; const float* beta = nullptr;
+  float eps = 0.0f;
+  int m = 0, k = 0, n = 0, activation = -1;
+  bool w_ready = false;  // as GemmArgs::w_ready
+};
+bool skinny_cluster_supported(int m, int k, int n);
+int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st);
 
 // pointwise.cu ---------------------------------------------------------------------------------
 int launch_eltwise(int op, const float* a, const float* b, float* y, int batch, int64_t n, int64_t nb,

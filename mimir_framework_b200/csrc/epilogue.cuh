@@ -30,5 +30,20 @@ __device__ __forceinline__ float apply_act(float v, int act) {
   }
 }
 
+// The activations of the exact-fp32 kernels for a few rows (tanhf for GELU, as the reference writes it).
+__device__ __forceinline__ float sk_act(float v, int act) {
+  switch (act) {
+    case MIMIR_B200_ELT_GELU: {
+      const float c = 0.7978845608f;
+      return v * (0.5f * (1.0f + tanhf(c * (v + 0.044715f * v * v * v))));
+    }
+    case MIMIR_B200_ELT_SILU: return v * (1.0f / (1.0f + expf(-v)));
+    case MIMIR_B200_ELT_RELU: return fmaxf(0.0f, v);
+    case MIMIR_B200_ELT_TANH: return tanhf(v);
+    case MIMIR_B200_ELT_SIGMOID: return 1.0f / (1.0f + expf(-v));
+    default: return v;
+  }
+}
+
 }  // namespace
 }  // namespace mb

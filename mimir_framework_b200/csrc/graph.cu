@@ -133,6 +133,7 @@ struct LayerRT {
   bool read_split = false;            // Linear reads the producer's planes
   int res_v = -1;                     // residual tensor folded in from a following Add
   int pre_norm = -1;                  // Conv2d: index of the GroupNorm layer applied while its operand planes are laid out
+  int pre_ln = -1;                    // a token-wise LayerNorm folded into this layer (index), see fusion 1f
   bool in_up = false;                 // Conv2d: in_v[0] is the INPUT of a 2 x 2 nearest upsample that the layout pass applies
   int gn_emit_for = -1;               // Conv2d: index of the GroupNorm layer whose statistics this layer's GEMM epilogue emits
   int gn_stats_from = -1;             // GroupNorm: index of the Conv2d layer that emits its statistics
@@ -755,6 +756,11 @@ namespace {
 size_t f32_bytes(const TensorV& t, int batch) { return static_cast<size_t>(batch) * static_cast<size_t>(t.n) * 4; }
 size_t splitv_bytes(const TensorV& t, int batch) { return split_bytes(static_cast<int64_t>(batch) * t.split_rows_ps, t.split_k, 2); }
 
+// A decode step's projections stream fp32 weights (decode_begin keeps output-major copies of them)
+bool attention_streams_weights(const LayerRT& L, int batch) {
+  return batch <= 16 && L.w_f32 && L.w_count >= static_cast<size_t>(4) * L.embed * L.embed;
+}
+
 int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch) {
   if (batch <= 0) return fail(MIMIR_B200_E_INVALID, "plan: batch must be positive");
   if (batch % m->pipeline != 0)
@@ -786,7 +792,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     LayerRT& L = m->layers[li];
     L.in_v.clear();
     L.out_v = -1;
-    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.in_up = false;
+    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false;
     L.ws_off = 0; L.ws_bytes = 0;
     std::vector<std::string> names = L.inputs;
     if (names.empty()) names.push_back("x");
@@ -958,6 +964,32 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       ut.producer = -2;  // dead
       U.skip = true;
     }
+  }
+  // ---- fusion 1f: a token-wise LayerNorm whose only consumer is a Linear of a few rows, or a decode step's attention block:
+  //      the consumer normalises while it stages its rows (skinny_cluster.cu) ----
+  for (int li = 0; li < nl; ++li) {
+    LayerRT& P = m->layers[li];
+    if (P.lt != LT::LayerNorm || P.skip || P.norm_n % 4 != 0) continue;
+    const int pv = P.out_v;
+    TensorV& pt = m->tensors[pv];
+    if (pt.alias_of >= 0 || pv == out_root || total_consumers(pv) != 1 || pt.consumers.size() != 1) continue;
+    const int ci = pt.consumers[0];
+    LayerRT& C = m->layers[ci];
+    if (C.skip || C.in_v[0] != pv || C.res_v == pv) continue;
+    bool ok = false;
+    if (C.lt == LT::Linear) ok = C.in_f == P.norm_n && linear_takes_layernorm(C.rows_ps * batch, C.in_f, C.out_f);
+    else if (C.lt == LT::Attention)
+      ok = m->is_twin && C.embed == P.norm_n && attention_streams_weights(C, batch) && linear_takes_layernorm(batch, C.embed, 3 * C.embed);
+    if (!ok) continue;
+    const int xin = P.in_v[0];
+    C.pre_ln = li;
+    C.in_v[0] = xin;
+    for (int& c : m->tensors[xin].consumers)
+      if (c == li) c = ci;
+    pt.consumers.clear();
+    pt.want_f32 = false;
+    pt.producer = -2;  // dead
+    P.skip = true;
   }
   // ---- fusion 2: hi/lo planes straight from one GEMM epilogue into the next Linear -------------
   for (int li = 0; li < nl; ++li) {
@@ -1179,6 +1211,17 @@ struct Bound {
   float* out_ptr = nullptr;
 };
 
+PreLayerNorm folded_layernorm(const MimirB200Model* m, const LayerRT& L) {
+  PreLayerNorm p;
+  if (L.pre_ln < 0) return p;
+  const LayerRT& N = m->layers[static_cast<size_t>(L.pre_ln)];
+  p.on = true;
+  p.gamma = N.d.affine ? N.w_f32 : nullptr;
+  p.beta = (N.d.affine && N.d.use_bias && N.w_f32) ? N.w_f32 + N.norm_n : nullptr;
+  p.eps = N.d.eps;
+  return p;
+}
+
 int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, uint8_t* arena) {
   auto f32p = [&](int v) -> float* {
     const int r = root_of(m->tensors, v);
@@ -1204,6 +1247,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.w_scale = L.w_scale; e.w_ready = true;
         e.bias = d.use_bias ? L.w_f32 + static_cast<size_t>(L.in_f) * L.out_f : nullptr;
         e.activation = L.fused_act;
+        e.pre = folded_layernorm(m, L);
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
         if (L.emit_f32) e.y_f32 = f32p(L.out_v);
         if (L.emit_split) e.y_split = splitp(L.out_v);
@@ -1215,6 +1259,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         AttentionExec e;
         e.batch = batch; e.seq = L.seq; e.embed = L.embed; e.heads = L.heads; e.causal = d.causal;
         e.precision = m->precision;
+        e.pre = folded_layernorm(m, L);
         if (L.read_split) e.x_split = splitp(L.in_v[0]); else e.x = f32p(L.in_v[0]);
         e.wqkv_split = L.w_split; e.wout_split = L.w_split2; e.w_scale = L.w_scale; e.w_ready = true; e.y = f32p(L.out_v); e.ws = ws;
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
@@ -1895,7 +1940,7 @@ int mimir_b200_model_decode_begin(MimirB200ModelHandle m, const MimirNamedInput*
     if (status == MIMIR_B200_OK) status = dev_alloc(reinterpret_cast<void**>(&L.vcache), L.cache_bytes, "value cache");
     bytes += 2 * L.cache_bytes;
     t->decode_scratch_bytes = std::max(t->decode_scratch_bytes, attention_decode_scratch_bytes(batch, L.heads, L.embed, max_seq));
-    if (status == MIMIR_B200_OK && batch <= 16 && L.w_f32 && L.w_count >= static_cast<size_t>(4) * L.embed * L.embed) {
+    if (status == MIMIR_B200_OK && attention_streams_weights(L, batch)) {
       // Wqkv [E][3E] and Wout [E][E] are stored input-major; the weight-streaming kernel reads W[out][in]
       const int E = L.embed;
       L.w_t_bytes = static_cast<size_t>(4) * E * E * sizeof(float);

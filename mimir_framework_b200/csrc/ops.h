@@ -15,6 +15,14 @@ int check_device_error_word(cudaStream_t st);
 int enqueue_error_word(cudaStream_t st);
 int read_error_word(cudaStream_t st);
 
+// A token-wise LayerNorm folded into the contraction that reads it: x is then the LayerNorm's input.
+struct PreLayerNorm {
+  bool on = false;
+  const float* gamma = nullptr;
+  const float* beta = nullptr;
+  float eps = 0.0f;
+};
+
 struct LinearExec {
   int rows = 0, in_f = 0, out_f = 0;
   int precision = MIMIR_B200_PREC_BF16X2;
@@ -32,7 +40,9 @@ struct LinearExec {
   int out_nchw_hw = 0;
   void* ws = nullptr;
   size_t ws_bytes = 0;
+  PreLayerNorm pre;                         // only where linear_takes_layernorm() holds
 };
+bool linear_takes_layernorm(int rows, int in_f, int out_f);
 bool linear_uses_skinny(int rows, int precision);
 size_t linear_ws_bytes(int rows, int in_f, int out_f, int precision, bool a_presplit);
 int linear_exec(const LinearExec& e, cudaStream_t st);
@@ -62,6 +72,7 @@ struct AttentionExec {
   const float* wqkv_t_f32 = nullptr;
   const float* wout_t_f32 = nullptr;
   float* skinny_scratch = nullptr;
+  PreLayerNorm pre;                 // decode steps of <= 16 samples with streamed weights
   size_t skinny_scratch_bytes = 0;
 };
 size_t attention_ws_bytes(int batch, int seq, int embed, int heads, int precision);

@@ -24,6 +24,8 @@
 #include <cstdlib>
 
 #include "common.h"
+#include "epilogue.cuh"
+#include "launch.cuh"
 
 namespace mb {
 namespace {
@@ -32,20 +34,6 @@ constexpr int SK_THREADS = 256;
 constexpr int SK_WARPS = SK_THREADS / 32;
 constexpr int SK_STEP = 128;   // k covered by one warp step
 constexpr int SK_SLICE = 512;  // k covered by one CTA
-
-__device__ __forceinline__ float sk_act(float v, int act) {
-  switch (act) {
-    case MIMIR_B200_ELT_GELU: {
-      const float c = 0.7978845608f;
-      return v * (0.5f * (1.0f + tanhf(c * (v + 0.044715f * v * v * v))));
-    }
-    case MIMIR_B200_ELT_SILU: return v * (1.0f / (1.0f + expf(-v)));
-    case MIMIR_B200_ELT_RELU: return fmaxf(0.0f, v);
-    case MIMIR_B200_ELT_TANH: return tanhf(v);
-    case MIMIR_B200_ELT_SIGMOID: return 1.0f / (1.0f + expf(-v));
-    default: return v;
-  }
-}
 
 template <int MT, int WR>
 __device__ __forceinline__ void sk_fma_step(float (&acc)[MT * WR], const float4 (&wv)[WR], const float* __restrict__ xs, int c) {
