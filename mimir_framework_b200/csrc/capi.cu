@@ -282,12 +282,16 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
     else g.out_f32 = qkv;
     MB_TRY(launch_gemm(g, st));
   }
-  if (e.kcache)
+  const bool fused_decode = e.decode_pos >= 0 && e.kcache && e.seq == 1 && e.embed % 4 == 0 && attention_decode_fused_supported(e.batch, e.embed, e.heads);
+  if (e.kcache && !fused_decode)
     MB_TRY(launch_kv_cache_write(qkv, e.kcache, e.vcache, e.batch, e.seq, e.embed, e.max_seq, e.decode_pos < 0 ? 0 : e.decode_pos, st,
                                  e.decode_pos >= 0 ? e.pos_dev : nullptr));
   if (e.decode_pos >= 0) {
     // one new token per sample against the cached keys and values (all of them are in its past)
     if (!e.kcache || e.seq != 1) return fail(MIMIR_B200_E_INVALID, "attention: a decode step needs a cache and one token per sample");
+    if (fused_decode) {
+      MB_TRY(launch_attention_decode_fused(qkv, e.kcache, e.vcache, att, e.batch, e.embed, e.heads, e.max_seq, e.decode_pos, e.pos_dev, e.w_ready, st));
+    } else {
     AttnView a;
     a.q = qkv; a.ldq = 3LL * e.embed; a.q_len = 1;
     a.k = e.kcache; a.v = e.vcache; a.ldkv = e.embed; a.kv_len = e.decode_pos + 1;
@@ -302,6 +306,7 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
       return fail(MIMIR_B200_E_UNSUPPORTED, "attention: this head layout cannot take its position from device memory");
     } else
       MB_TRY(launch_attention_core_view(a, att, e.batch, e.embed, e.heads, 0, st));
+    }
     if (stream_w) {
       return skinny_linear(att, e.wout_t_f32, nullptr, e.y, rows, e.embed, e.embed, -1, PreLayerNorm(), e.w_ready, e.skinny_scratch,
                            e.skinny_scratch_bytes, st, e.residual);

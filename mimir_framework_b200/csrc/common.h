@@ -288,6 +288,11 @@ struct AttnView {
 size_t attention_decode_scratch_bytes(int batch, int heads, int embed, int max_seq);
 bool attention_decode_supported(const AttnView& a, int embed, int heads);
 int launch_attention_decode(const AttnView& a, float* out, float* scratch, int batch, int embed, int heads, cudaStream_t st);
+// attention_decode.cu: the whole core of a decode step in one launch - appends K and V of qkv [batch][3E] to the caches at the
+// position and attends to positions 0 .. pos (*pos_dev when given).  cached_ready: the cached rows were complete before this call.
+bool attention_decode_fused_supported(int batch, int embed, int heads);
+int launch_attention_decode_fused(const float* qkv, float* kcache, float* vcache, float* out, int batch, int embed, int heads, int max_seq,
+                                  int pos, const int* pos_dev, bool cached_ready, cudaStream_t st);
 // K and V thirds of qkv [batch*seq][3E] -> cache[b][pos0 + s][E] of caches holding max_seq positions per sample
 int launch_kv_cache_write(const float* qkv, float* kcache, float* vcache, int batch, int seq, int embed, int max_seq, int pos0,
                           cudaStream_t st, const int* pos_dev = nullptr);

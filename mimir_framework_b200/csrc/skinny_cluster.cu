@@ -38,6 +38,12 @@ __device__ __forceinline__ float4 ld_weights(const float* p) {  // read once; vo
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+__device__ __forceinline__ float warp_total(float v) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
 template <int MT, int STEPS>
 __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const SkinnyClusterParams p) {
   constexpr int N = MT * SC_WR, PER = N / 32;
@@ -69,25 +75,36 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
   pdl_wait();
 
   if (p.ln) {
-    // mean and variance of each row (LayerOps.hpp:264-319), two passes over the row (the second from L1)
+    // mean and variance of each row (LayerOps.hpp:264-319), two passes; rows of up to 1024 values stay in registers in between
     for (int r = warp; r < p.m; r += SC_WARPS) {
       const float* row = p.x + static_cast<long long>(r) * p.k;
-      float s = 0.0f;
-      for (int c = lane * 4; c < p.k; c += 128) {
-        const float4 v = *reinterpret_cast<const float4*>(row + c);
-        s += (v.x + v.y) + (v.z + v.w);
-      }
+      float s = 0.0f, q = 0.0f, mean;
+      if (p.k <= 1024) {
+        float4 v[8];
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-      const float mean = s / static_cast<float>(p.k);
-      float q = 0.0f;
-      for (int c = lane * 4; c < p.k; c += 128) {
-        const float4 v = *reinterpret_cast<const float4*>(row + c);
-        const float a = v.x - mean, b = v.y - mean, e = v.z - mean, f = v.w - mean;
-        q += (a * a + b * b) + (e * e + f * f);
-      }
+        for (int j = 0; j < 8; ++j) v[j] = (lane + 32 * j) * 4 < p.k ? *reinterpret_cast<const float4*>(row + (lane + 32 * j) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
+        for (int j = 0; j < 8; ++j) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+        mean = warp_total(s) / static_cast<float>(p.k);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if ((lane + 32 * j) * 4 < p.k) {
+            const float a = v[j].x - mean, b = v[j].y - mean, e = v[j].z - mean, f = v[j].w - mean;
+            q += (a * a + b * b) + (e * e + f * f);
+          }
+      } else {
+        for (int c = lane * 4; c < p.k; c += 128) {
+          const float4 v = *reinterpret_cast<const float4*>(row + c);
+          s += (v.x + v.y) + (v.z + v.w);
+        }
+        mean = warp_total(s) / static_cast<float>(p.k);
+        for (int c = lane * 4; c < p.k; c += 128) {
+          const float4 v = *reinterpret_cast<const float4*>(row + c);
+          const float a = v.x - mean, b = v.y - mean, e = v.z - mean, f = v.w - mean;
+          q += (a * a + b * b) + (e * e + f * f);
+        }
+      }
+      q = warp_total(q);
       if (lane == 0) {
         mean_s[r] = mean;
         rstd_s[r] = 1.0f / sqrtf(q / static_cast<float>(p.k) + p.eps);
