@@ -54,20 +54,20 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
   const float* qrow = p.qkv + static_cast<long long>(b) * 3 * p.embed + h * HD + q4 * 4;
 
   float4 kv[AD_U], vv[AD_U];
-  auto load_old = [&](int g) {  // the cached keys of group g (the new one comes from the projection)
+  auto load_rows = [&](float4 (&r)[AD_U], const float* base, int g) {  // the cached rows of group g (the new one comes from the projection)
 #pragma unroll
     for (int u = 0; u < AD_U; ++u) {
       const int key = g * GROUP + u * KPW + sub;
-      kv[u] = vv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (key < pos) {
-        const long long o = static_cast<long long>(key) * p.embed;
-        asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(kv[u].x), "=f"(kv[u].y), "=f"(kv[u].z), "=f"(kv[u].w) : "l"(kc + o));
-        asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(vv[u].x), "=f"(vv[u].y), "=f"(vv[u].z), "=f"(vv[u].w) : "l"(vc + o));
-      }
+      r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (key < pos)
+        asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r[u].x), "=f"(r[u].y), "=f"(r[u].z), "=f"(r[u].w) : "l"(base + static_cast<long long>(key) * p.embed));
     }
   };
   if (!p.cached_ready) pdl_wait();
-  if (g0 < g1) load_old(g0);
+  if (g0 < g1) {
+    load_rows(kv, kc, g0);
+    load_rows(vv, vc, g0);
+  }
   pdl_launch_dependents();
   pdl_wait();
   const float4 q = *reinterpret_cast<const float4*>(qrow);
@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
     float d[AD_U];
 #pragma unroll
     for (int u = 0; u < AD_U; ++u) d[u] = fmaf(q.w, kv[u].w, fmaf(q.z, kv[u].z, fmaf(q.y, kv[u].y, q.x * kv[u].x)));
+    if (g + 1 < g1) load_rows(kv, kc, g + 1);  // in flight while this group's softmax and P V run
     // sum over the LPK lanes of a key: three rounds halve the eight values, the rest add one value up; the lane's bits LPK/2,
     // LPK/4, LPK/8 name the key of the load it ends with
 #pragma unroll
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
       const float w = __shfl_sync(0xffffffffu, pr, sub * LPK + u * (LPK / 8));
       acc.x = fmaf(w, vv[u].x, acc.x); acc.y = fmaf(w, vv[u].y, acc.y); acc.z = fmaf(w, vv[u].z, acc.z); acc.w = fmaf(w, vv[u].w, acc.w);
     }
-    if (g + 1 < g1) load_old(g + 1);
+    if (g + 1 < g1) load_rows(vv, vc, g + 1);
   }
   // l: LPK / 8 lanes hold the same probabilities; the sum over the warp counts each that often (a power of two, exact)
 #pragma unroll

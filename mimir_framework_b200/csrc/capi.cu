@@ -185,16 +185,16 @@ bool linear_takes_layernorm(int rows, int in_f, int out_f) { return rows <= 16 &
 
 // y = act(norm(x) . w^T + bias) (+ residual) for at most 16 rows: one launch where the weights fit a wave of CTAs, else the
 // streaming kernel and its finishing kernel
-static int skinny_linear(const float* x, const float* w, const float* bias, float* y, int rows, int k, int n, int act, const PreLayerNorm& pre,
+static int skinny_linear(const float* x, const float* w, const uint16_t* w_bf16, const float* bias, float* y, int rows, int k, int n, int act, const PreLayerNorm& pre,
                          bool w_ready, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual) {
-  if (skinny_cluster_supported(rows, k, n) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
+  if (skinny_cluster_supported(rows, k, n) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w_bf16)) & 15) == 0) {
     SkinnyClusterArgs a;
-    a.x = x; a.w = w; a.bias = bias; a.residual = residual; a.y = y; a.m = rows; a.k = k; a.n = n; a.activation = act; a.w_ready = w_ready;
+    a.x = x; a.w = w; a.w_bf16 = w_bf16; a.bias = bias; a.residual = residual; a.y = y; a.m = rows; a.k = k; a.n = n; a.activation = act; a.w_ready = w_ready;
     a.ln = pre.on; a.gamma = pre.gamma; a.beta = pre.gamma ? pre.beta : nullptr; a.eps = pre.eps;
     return launch_skinny_cluster(a, st);
   }
   if (pre.on) return fail(MIMIR_B200_E_INVALID, "linear: a folded LayerNorm needs the cluster kernel");
-  return launch_skinny_linear(x, w, bias, y, rows, k, n, act, scratch, scratch_bytes, st, residual);
+  return launch_skinny_linear(x, w, bias, y, rows, k, n, act, scratch, scratch_bytes, st, residual, w_bf16);
 }
 
 size_t linear_ws_bytes(int rows, int in_f, int out_f, int precision, bool a_presplit) {
@@ -207,8 +207,8 @@ size_t linear_ws_bytes(int rows, int in_f, int out_f, int precision, bool a_pres
 
 int linear_exec(const LinearExec& e, cudaStream_t st) {
   if (linear_uses_skinny(e.rows, e.precision)) {
-    if (!e.x_f32 || !e.w_f32 || !e.y_f32) return fail(MIMIR_B200_E_INVALID, "linear: skinny path needs fp32 operands");
-    return skinny_linear(e.x_f32, e.w_f32, e.bias, e.y_f32, e.rows, e.in_f, e.out_f, e.activation, e.pre, e.w_ready,
+    if (!e.x_f32 || !(e.w_f32 || e.w_bf16) || !e.y_f32) return fail(MIMIR_B200_E_INVALID, "linear: skinny path needs fp32 operands");
+    return skinny_linear(e.x_f32, e.w_f32, e.w_bf16, e.bias, e.y_f32, e.rows, e.in_f, e.out_f, e.activation, e.pre, e.w_ready,
                          static_cast<float*>(e.ws), e.ws_bytes, st, e.residual);
   }
   int ap, wp;
@@ -267,9 +267,9 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
   // a decode step of a few samples: both projections stream fp32 weights (transposed copies, W[out][in]) instead of
   // running 128-row GEMM tiles that are almost empty
   bool qkv_as_planes = false;
-  const bool stream_w = e.decode_pos >= 0 && e.wqkv_t_f32 && e.wout_t_f32 && e.x && rows <= 16 && e.skinny_scratch;
+  const bool stream_w = e.decode_pos >= 0 && ((e.wqkv_t_f32 && e.wout_t_f32) || (e.wqkv_t_bf16 && e.wout_t_bf16)) && e.x && rows <= 16 && e.skinny_scratch;
   if (stream_w) {
-    MB_TRY(skinny_linear(e.x, e.wqkv_t_f32, nullptr, qkv, rows, e.embed, 3 * e.embed, -1, e.pre, e.w_ready, e.skinny_scratch, e.skinny_scratch_bytes, st, nullptr));
+    MB_TRY(skinny_linear(e.x, e.wqkv_t_f32, e.wqkv_t_bf16, nullptr, qkv, rows, e.embed, 3 * e.embed, -1, e.pre, e.w_ready, e.skinny_scratch, e.skinny_scratch_bytes, st, nullptr));
   } else {
     if (!e.x_split) MB_TRY(launch_split(e.x, xs, rows, e.embed, ap, st));
     GemmArgs g;
@@ -308,7 +308,7 @@ int attention_exec(const AttentionExec& e, cudaStream_t st) {
       MB_TRY(launch_attention_core_view(a, att, e.batch, e.embed, e.heads, 0, st));
     }
     if (stream_w) {
-      return skinny_linear(att, e.wout_t_f32, nullptr, e.y, rows, e.embed, e.embed, -1, PreLayerNorm(), e.w_ready, e.skinny_scratch,
+      return skinny_linear(att, e.wout_t_f32, e.wout_t_bf16, nullptr, e.y, rows, e.embed, e.embed, -1, PreLayerNorm(), e.w_ready, e.skinny_scratch,
                            e.skinny_scratch_bytes, st, e.residual);
     }
     MB_TRY(launch_split(att, xs, rows, e.embed, ap, st));

@@ -216,12 +216,14 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st);
 int launch_wait_timeout_selftest(unsigned long long limit_ns, cudaStream_t st);
 // fp32 weight-streaming kernel for very small m (<= 16 rows): y[m,n] = x[m,k] · w[n,k]ᵀ + bias.
 int launch_skinny_linear(const float* x, const float* w, const float* bias, float* y, int m, int k, int n,
-                         int activation, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual = nullptr);
+                         int activation, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual = nullptr,
+                         const uint16_t* w_bf16 = nullptr);
 size_t skinny_scratch_bytes(int m, int k, int n);
 // skinny_cluster.cu: the same for weight matrices that fit one wave of CTAs; one launch, no scratch.  ln: x is normalised row by
 // row (mean / variance over k) with gamma and beta before the product.
 struct SkinnyClusterArgs {
   const float* x = nullptr; const float* w = nullptr; const float* bias = nullptr; const float* residual = nullptr; float* y = nullptr;
+  const uint16_t* w_bf16 = nullptr;  // the same weights as bfloat16, where that is exact (launch_pack_bf16): read instead of w
   bool ln = false;
   const float* gamma = nullptr; const float* beta = nullptr;
   float eps = 0.0f;
@@ -229,6 +231,8 @@ struct SkinnyClusterArgs {
   bool w_ready = false;  // as GemmArgs::w_ready
 };
 bool skinny_cluster_supported(int m, int k, int n);
+// bfloat16 copy of fp32 values; *inexact (device) becomes 1 when one of them is not a bfloat16
+int launch_pack_bf16(const float* src, uint16_t* dst, size_t n, int* inexact, cudaStream_t st);
 int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st);
 
 // pointwise.cu ---------------------------------------------------------------------------------

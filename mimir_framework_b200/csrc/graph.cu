@@ -145,6 +145,8 @@ struct LayerRT {
   size_t cache_bytes = 0;
   float* w_t_f32 = nullptr;           // attention of a twin with <= 16 samples: Wqkv^T [3E][E] then Wout^T [E][E], fp32
   size_t w_t_bytes = 0;
+  uint16_t* w_bf16 = nullptr;         // layers of a twin with <= 16 samples whose weights are exact bfloat16 values: a copy the streaming
+  size_t w_bf16_bytes = 0;            // kernels read instead (attention: of the transposed projections, which are then not kept)
   size_t ws_off = 0, ws_bytes = 0;
   // resolved shapes (per sample)
   int rows_ps = 1, in_f = 0, out_f = 0;       // Linear
@@ -1243,6 +1245,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.rows = batch * L.rows_ps; e.in_f = L.in_f; e.out_f = L.out_f; e.precision = m->precision;
         if (L.read_split) e.x_split = splitp(L.in_v[0]); else e.x_f32 = f32p(L.in_v[0]);
         e.w_f32 = L.w_f32;
+        e.w_bf16 = L.w_bf16;
         e.w_split = L.w_split;
         e.w_scale = L.w_scale; e.w_ready = true;
         e.bias = d.use_bias ? L.w_f32 + static_cast<size_t>(L.in_f) * L.out_f : nullptr;
@@ -1267,9 +1270,10 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
           e.kcache = L.kcache; e.vcache = L.vcache; e.max_seq = m->max_seq; e.decode_pos = m->decode_pos;
           e.decode_scratch = m->decode_scratch;
           e.pos_dev = m->pos_dev;
-          if (L.w_t_f32) {
-            e.wqkv_t_f32 = L.w_t_f32;
-            e.wout_t_f32 = L.w_t_f32 + static_cast<size_t>(3) * L.embed * L.embed;
+          if (L.w_t_f32 || L.w_bf16) {
+            const size_t qkv_n = static_cast<size_t>(3) * L.embed * L.embed;
+            if (L.w_t_f32) { e.wqkv_t_f32 = L.w_t_f32; e.wout_t_f32 = L.w_t_f32 + qkv_n; }
+            if (L.w_bf16) { e.wqkv_t_bf16 = L.w_bf16; e.wout_t_bf16 = L.w_bf16 + qkv_n; }
             e.skinny_scratch = m->skinny_scratch;
             e.skinny_scratch_bytes = m->skinny_scratch_bytes;
           }
@@ -1617,7 +1621,9 @@ static void destroy_model(MimirB200Model* m) {
     if (L.kcache) dev_free(L.kcache, L.cache_bytes);
     if (L.vcache) dev_free(L.vcache, L.cache_bytes);
     if (L.w_t_f32) dev_free(L.w_t_f32, L.w_t_bytes);
+    if (L.w_bf16) dev_free(L.w_bf16, L.w_bf16_bytes);
     L.kcache = L.vcache = L.w_t_f32 = nullptr;
+    L.w_bf16 = nullptr;
   }
   if (m->decode_scratch) dev_free(m->decode_scratch, m->decode_scratch_bytes);
   if (m->skinny_scratch) dev_free(m->skinny_scratch, m->skinny_scratch_bytes);
@@ -1907,6 +1913,47 @@ int mimir_b200_model_decode_end(MimirB200ModelHandle m) {
   return MIMIR_B200_OK;
 }
 
+// A step of a few samples is bound by the weights it streams: where a layer's weights are bfloat16 values (a checkpoint that was
+// rounded to bf16, stored as fp32) a 16-bit copy of them is read instead - half the bytes, the same products.
+static int pack_exact_bf16(MimirB200Model* t, int batch) {
+  if (batch > 16) return MIMIR_B200_OK;
+  std::vector<LayerRT*> packed;
+  for (auto& L : t->layers) {
+    const bool lin = L.lt == LT::Linear && L.w_f32 && L.in_f % 8 == 0 && L.w_count >= static_cast<size_t>(L.in_f) * L.out_f;
+    const bool att = L.lt == LT::Attention && L.w_t_f32 && L.embed % 8 == 0;
+    if (lin || att) packed.push_back(&L);
+  }
+  if (packed.empty()) return MIMIR_B200_OK;
+  int* flags = nullptr;
+  const size_t flag_bytes = packed.size() * sizeof(int);
+  MB_TRY(dev_alloc(reinterpret_cast<void**>(&flags), flag_bytes, "bf16 check"));
+  std::vector<int> inexact(packed.size(), 1);
+  int s = MIMIR_B200_OK;
+  if (cudaMemsetAsync(flags, 0, flag_bytes, nullptr) != cudaSuccess) s = fail(MIMIR_B200_E_CUDA, "decode_begin: clearing flags failed");
+  for (size_t i = 0; i < packed.size() && s == MIMIR_B200_OK; ++i) {
+    LayerRT& L = *packed[i];
+    const size_t n = L.lt == LT::Linear ? static_cast<size_t>(L.in_f) * L.out_f : static_cast<size_t>(4) * L.embed * L.embed;
+    L.w_bf16_bytes = n * sizeof(uint16_t);
+    s = dev_alloc(reinterpret_cast<void**>(&L.w_bf16), L.w_bf16_bytes, "bf16 weights");
+    if (s == MIMIR_B200_OK) s = launch_pack_bf16(L.lt == LT::Linear ? L.w_f32 : L.w_t_f32, L.w_bf16, n, flags + i, nullptr);
+  }
+  if (s == MIMIR_B200_OK && cudaMemcpy(inexact.data(), flags, flag_bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
+    s = fail(MIMIR_B200_E_CUDA, "decode_begin: reading flags failed");
+  dev_free(flags, flag_bytes);
+  if (s != MIMIR_B200_OK) return s;  // (the twin's layers free what was allocated)
+  for (size_t i = 0; i < packed.size(); ++i) {
+    LayerRT& L = *packed[i];
+    if (inexact[i]) {
+      dev_free(L.w_bf16, L.w_bf16_bytes);
+      L.w_bf16 = nullptr;
+    } else if (L.w_t_f32) {
+      dev_free(L.w_t_f32, L.w_t_bytes);
+      L.w_t_f32 = nullptr;
+    }
+  }
+  return MIMIR_B200_OK;
+}
+
 int mimir_b200_model_decode_begin(MimirB200ModelHandle m, const MimirNamedInput* inputs, int n_inputs, int batch, int max_seq,
                                   uint64_t* cache_bytes) {
   DeviceScope dev_scope(m ? m->device : ctx().device);
@@ -1929,6 +1976,7 @@ int mimir_b200_model_decode_begin(MimirB200ModelHandle m, const MimirNamedInput*
     L.borrowed_f32 = true;
     L.borrowed_planes = (L.w_split != nullptr);
     L.kcache = L.vcache = nullptr;
+    L.w_bf16 = nullptr;
     if (L.d.seq_len > 0) L.d.seq_len = 1;  // one token per sample and step
   }
   status = plan_model(t.get(), inputs, n_inputs, batch);
@@ -1952,6 +2000,7 @@ int mimir_b200_model_decode_begin(MimirB200ModelHandle m, const MimirNamedInput*
       t->skinny_scratch_bytes = std::max(t->skinny_scratch_bytes, skinny_scratch_bytes(batch, E, 3 * E));
     }
   }
+  if (status == MIMIR_B200_OK) status = pack_exact_bf16(t.get(), batch);
   bool pos_on_device = (status == MIMIR_B200_OK);
   for (const auto& L : t->layers)
     if (L.lt == LT::Attention) {

@@ -40,6 +40,7 @@ struct LinearExec {
   int out_nchw_hw = 0;
   void* ws = nullptr;
   size_t ws_bytes = 0;
+  const uint16_t* w_bf16 = nullptr;         // exact bfloat16 copy of w_f32 (skinny paths)
   PreLayerNorm pre;                         // only where linear_takes_layernorm() holds
 };
 bool linear_takes_layernorm(int rows, int in_f, int out_f);
@@ -71,6 +72,8 @@ struct AttentionExec {
   // decode steps of <= 16 samples: fp32 copies of the projections as W[out][in] and the weight-streaming kernel's scratch
   const float* wqkv_t_f32 = nullptr;
   const float* wout_t_f32 = nullptr;
+  const uint16_t* wqkv_t_bf16 = nullptr;  // or bfloat16 copies of them, where that is exact
+  const uint16_t* wout_t_bf16 = nullptr;
   float* skinny_scratch = nullptr;
   PreLayerNorm pre;                 // decode steps of <= 16 samples with streamed weights
   size_t skinny_scratch_bytes = 0;

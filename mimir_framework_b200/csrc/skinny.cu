@@ -52,6 +52,10 @@ __device__ __forceinline__ void sk_fma_step(float (&acc)[MT * WR], const float4 
   }
 }
 
+__device__ __forceinline__ float4 bf16_quad(uint32_t a, uint32_t b) {
+  return make_float4(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u), __uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
+}
+
 // MT = rows of x held (m <= MT), WR = rows of W per warp.
 template <int MT, int WR>
 __global__ void __launch_bounds__(SK_THREADS, 2)
@@ -137,7 +141,6 @@ skinny_partial_kernel(const float* __restrict__ x, const float* __restrict__ w, 
 }
 
 constexpr int SK_STAGES = 4;
-constexpr int SK_STEPS = SK_SLICE / SK_STEP;  // steps per item
 
 __device__ __forceinline__ void cp_async16_zfill(void* smem_dst, const void* gsrc, bool valid) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
@@ -167,11 +170,16 @@ struct ItemSplit {
 // output tile, so their partial sums stay in the accumulators and the exchange between lanes and the write of the partials
 // happen once per (CTA, tile) instead of once per item.  Partial p of a tile is the one of the p-th CTA that touched it, in K
 // order: part[(p * m + r) * n + o].
-template <int MT, int WR>
+// BF16: the weights are bfloat16 copies (exact where they are used): 16 bytes per lane and row are then eight consecutive k, a warp
+// step covers 256 k, and x is staged with the two quads of every eight k apart so that its 128-bit reads stay free of conflicts.
+template <int MT, int WR, int BF16>
 __global__ void __launch_bounds__(SK_THREADS, 1)
-skinny_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ part, int m, int k, int n,
+skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any, float* __restrict__ part, int m, int k, int n,
                      int kslices, int items) {
   constexpr int N = MT * WR;
+  constexpr int STEP = BF16 ? 2 * SK_STEP : SK_STEP, STEPS = SK_SLICE / STEP;  // k of a warp step, steps per item
+  constexpr int EB = BF16 ? 2 : 4;                                          // bytes of a weight
+  const char* w = static_cast<const char*>(w_any);
   constexpr int PER = N / 32;
   static_assert(N % 32 == 0 && PER >= 1, "WR x MT must be a multiple of the warp size");
   extern __shared__ __align__(16) float sk_smem[];
@@ -180,7 +188,7 @@ skinny_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, f
   float* ring = sk_smem + 2 * MT * SK_SLICE + warp * (SK_STAGES * WR * SK_STEP);
   const ItemSplit split(items, static_cast<int>(gridDim.x));
   const int my_first = split.first(static_cast<int>(blockIdx.x)), my_items = split.count(static_cast<int>(blockIdx.x));
-  const int total_steps = my_items * SK_STEPS;
+  const int total_steps = my_items * STEPS;
   const long long kk = k;
 
   // Copy group of this CTA's step g (item g / SK_STEPS, step g % SK_STEPS): this warp's WR rows of W, and with the first step
@@ -190,16 +198,16 @@ skinny_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, f
   int i_tile = my_first / kslices, i_ks = my_first - i_tile * kslices;
   auto issue = [&]() {
     if (ig < total_steps) {
-      const int c = i_ks * SK_SLICE + i_st * SK_STEP + lane * 4;
+      const int c = i_ks * SK_SLICE + i_st * STEP + lane * (16 / EB);
       const int o0 = (i_tile * SK_WARPS + warp) * WR;
-      const float* src = w + static_cast<long long>(o0) * kk + c;
+      const char* src = w + (static_cast<long long>(o0) * kk + c) * EB;
       float* dst = ring + (ig % SK_STAGES) * (WR * SK_STEP) + lane * 4;
       const bool col_ok = c < k;
 #pragma unroll
       for (int jj = 0; jj < WR; ++jj) {
         const bool ok = col_ok && (o0 + jj < n);
         cp_async16_zfill(dst + jj * SK_STEP, ok ? src : w, ok);
-        src += kk;
+        src += kk * EB;
       }
       if (i_st == 0) {
         float* xd = xs + (i_j & 1) * (MT * SK_SLICE);
@@ -207,10 +215,11 @@ skinny_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, f
           const int r = i / (SK_SLICE / 4), cc = (i - r * (SK_SLICE / 4)) << 2;
           const int kc = i_ks * SK_SLICE + cc;
           const bool ok = (r < m) && (kc < k);
-          cp_async16_zfill(xd + r * SK_SLICE + cc, ok ? (x + r * kk + kc) : x, ok);
+          const int at = BF16 ? (cc & ~255) + ((cc >> 2) & 1) * 128 + ((cc & 255) >> 3) * 4 : cc;
+          cp_async16_zfill(xd + r * SK_SLICE + at, ok ? (x + r * kk + kc) : x, ok);
         }
       }
-      if (++i_st == SK_STEPS) {
+      if (++i_st == STEPS) {
         i_st = 0;
         ++i_j;
         if (++i_ks == kslices) { i_ks = 0; ++i_tile; }
@@ -229,8 +238,8 @@ skinny_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, f
   for (int j = 0; j < my_items; ++j) {
     const float* xj = xs + (j & 1) * (MT * SK_SLICE);
 #pragma unroll
-    for (int st = 0; st < SK_STEPS; ++st) {
-      const int g = j * SK_STEPS + st;
+    for (int st = 0; st < STEPS; ++st) {
+      const int g = j * STEPS + st;
       if (st == 0) {
         // the group of step g carries this item's x slice: wait for it, then let every thread's share become visible
         // (the next group may overwrite the x buffer of item j - 1: issued after the barrier)
@@ -245,7 +254,17 @@ skinny_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, f
       float4 wv[WR];
 #pragma unroll
       for (int jj = 0; jj < WR; ++jj) wv[jj] = *reinterpret_cast<const float4*>(src + jj * SK_STEP);
-      sk_fma_step<MT, WR>(acc, wv, xj, st * SK_STEP + lane * 4);
+      if (BF16) {
+        float4 half[WR];
+#pragma unroll
+        for (int jj = 0; jj < WR; ++jj) half[jj] = bf16_quad(__float_as_uint(wv[jj].x), __float_as_uint(wv[jj].y));
+        sk_fma_step<MT, WR>(acc, half, xj, st * STEP + lane * 4);
+#pragma unroll
+        for (int jj = 0; jj < WR; ++jj) half[jj] = bf16_quad(__float_as_uint(wv[jj].z), __float_as_uint(wv[jj].w));
+        sk_fma_step<MT, WR>(acc, half, xj, st * STEP + 128 + lane * 4);
+      } else {
+        sk_fma_step<MT, WR>(acc, wv, xj, st * STEP + lane * 4);
+      }
     }
     const bool tile_ends = (ks + 1 == kslices) || (j + 1 == my_items);
     if (tile_ends) {
@@ -309,7 +328,7 @@ __global__ void skinny_finish_kernel(const float* __restrict__ part, const float
 }
 
 template <int MT, int WR>
-int launch_partial(const float* x, const float* w, float* scratch, int m, int k, int n, cudaStream_t st, int* stream_grid, int* stream_items,
+int launch_partial(const float* x, const float* w, const uint16_t* w_bf16, float* scratch, int m, int k, int n, cudaStream_t st, int* stream_grid, int* stream_items,
                    int* tile_cols) {
   const int tiles = (n + SK_WARPS * WR - 1) / (SK_WARPS * WR), kslices = (k + SK_SLICE - 1) / SK_SLICE;
   const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0 && (k & 3) == 0;
@@ -317,16 +336,19 @@ int launch_partial(const float* x, const float* w, float* scratch, int m, int k,
   *stream_grid = 0;
   *stream_items = 0;
   *tile_cols = SK_WARPS * WR;
-  if (vec && !(plain && plain[0] == '1') && static_cast<long long>(tiles) * kslices < (1LL << 30)) {
+  const bool bf16 = w_bf16 != nullptr && (k & 7) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_bf16)) & 15) == 0;
+  if ((vec || bf16) && !(plain && plain[0] == '1') && static_cast<long long>(tiles) * kslices < (1LL << 30)) {
     constexpr int SMEM = (2 * MT * SK_SLICE + SK_WARPS * SK_STAGES * WR * SK_STEP) * 4;
     static PerDeviceOnce attr_once;
     MB_TRY(attr_once.run([&]() -> int {
-      MB_CUDA(cudaFuncSetAttribute(skinny_stream_kernel<MT, WR>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+      MB_CUDA(cudaFuncSetAttribute(skinny_stream_kernel<MT, WR, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+      MB_CUDA(cudaFuncSetAttribute(skinny_stream_kernel<MT, WR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
       return MIMIR_B200_OK;
     }));
     const int items = tiles * kslices;
     const int grid = items < ctx().sm_count ? items : ctx().sm_count;
-    skinny_stream_kernel<MT, WR><<<grid, SK_THREADS, SMEM, st>>>(x, w, scratch, m, k, n, kslices, items);
+    if (bf16) skinny_stream_kernel<MT, WR, 1><<<grid, SK_THREADS, SMEM, st>>>(x, w_bf16, scratch, m, k, n, kslices, items);
+    else skinny_stream_kernel<MT, WR, 0><<<grid, SK_THREADS, SMEM, st>>>(x, w, scratch, m, k, n, kslices, items);
     *stream_grid = grid;
     *stream_items = items;
   } else {
@@ -346,15 +368,15 @@ size_t skinny_scratch_bytes(int m, int k, int n) {
 }
 
 int launch_skinny_linear(const float* x, const float* w, const float* bias, float* y, int m, int k, int n, int activation,
-                         float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual) {
+                         float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual, const uint16_t* w_bf16) {
   if (m <= 0 || m > 16 || k <= 0 || n <= 0) return fail(MIMIR_B200_E_INVALID, "skinny linear: m must be in 1..16");
   if (scratch == nullptr || scratch_bytes < skinny_scratch_bytes(m, k, n))
     return fail(MIMIR_B200_E_INVALID, "skinny linear: scratch too small");
   if ((k + SK_SLICE - 1) / SK_SLICE > 65535) return fail(MIMIR_B200_E_UNSUPPORTED, "skinny linear: in_features %d too large", k);
   int sgrid = 0, sitems = 0, tile_cols = 0;
-  if (m <= 4) MB_TRY((launch_partial<4, 8>(x, w, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
-  else if (m <= 8) MB_TRY((launch_partial<8, 8>(x, w, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
-  else MB_TRY((launch_partial<16, 4>(x, w, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
+  if (m <= 4) MB_TRY((launch_partial<4, 8>(x, w, w_bf16, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
+  else if (m <= 8) MB_TRY((launch_partial<8, 8>(x, w, w_bf16, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
+  else MB_TRY((launch_partial<16, 4>(x, w, w_bf16, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
   const long long total = static_cast<long long>(m) * n;
   int fb = static_cast<int>((total + 255) / 256);
   if (fb > ctx().sm_count * 8) fb = ctx().sm_count * 8;

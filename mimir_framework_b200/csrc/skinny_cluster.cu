@@ -19,22 +19,36 @@ namespace mb {
 namespace {
 
 constexpr int SC_THREADS = 256, SC_WARPS = 8;
-constexpr int SC_WR = 4;                    // weight rows of a warp
-constexpr int SC_ROWS = SC_WARPS * SC_WR;   // output features of a CTA
 constexpr int SC_STEP = 128;                // k of a warp step: 32 lanes x 4
 
 struct SkinnyClusterParams {
-  const float* x; const float* w; const float* bias; const float* residual; float* y;
+  const float* x; const void* w; const float* bias; const float* residual; float* y;
   const float* gamma; const float* beta;  // LayerNorm (ln != 0), either may be null
   float eps;
   int ln, m, k, n, kc, act, w_ready;
 };
 
-__device__ __forceinline__ float4 ld_weights(const float* p) {  // read once; volatile: stays ahead of the dependency wait
+// Four consecutive weights of a row, as fp32 or as bfloat16 (where every weight is one exactly: half the bytes, the same values).
+// Read once; volatile: the loads stay ahead of the dependency wait.
+template <int BF16> struct Quad;
+template <> struct Quad<0> {
   float4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-  return v;
-}
+  __device__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ void load(const void* w, long long i) {
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(static_cast<const float*>(w) + i));
+  }
+  __device__ float4 get() const { return v; }
+};
+template <> struct Quad<1> {
+  uint2 v;
+  __device__ void zero() { v = make_uint2(0u, 0u); }
+  __device__ void load(const void* w, long long i) {
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(static_cast<const uint16_t*>(w) + i));
+  }
+  __device__ float4 get() const {
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+  }
+};
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
@@ -44,9 +58,12 @@ __device__ __forceinline__ float warp_total(float v) {
   return v;
 }
 
-template <int MT, int STEPS>
+// MT rows of x, WR weight rows of a warp, STEPS 128-wide k steps of a CTA.
+template <int MT, int WR, int STEPS, int BF16>
 __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const SkinnyClusterParams p) {
-  constexpr int N = MT * SC_WR, PER = N / 32;
+  constexpr int SC_WR = WR, SC_ROWS = SC_WARPS * WR;  // output features of a CTA
+  constexpr int N = MT * WR;
+  constexpr int R = N % 32 == 0 ? 5 : N % 16 == 0 ? 4 : N % 8 == 0 ? 3 : 2, PER = N >> R;  // halving rounds of the exchange, values left
   constexpr int KC = STEPS * SC_STEP;
   extern __shared__ __align__(16) float sc_smem[];
   float* xs = sc_smem;                       // [MT][KC]
@@ -62,14 +79,14 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
 
   cluster_arrive();  // (waited for before the first write into another CTA)
   if (!p.w_ready) pdl_wait();
-  float4 wv[STEPS][SC_WR];
+  Quad<BF16> wv[STEPS][SC_WR];
 #pragma unroll
   for (int s = 0; s < STEPS; ++s)
 #pragma unroll
     for (int j = 0; j < SC_WR; ++j) {
       const int c = s * SC_STEP + lane * 4;
-      wv[s][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c < klen && o0 + j < p.n) wv[s][j] = ld_weights(p.w + static_cast<long long>(o0 + j) * p.k + k0 + c);
+      wv[s][j].zero();
+      if (c < klen && o0 + j < p.n) wv[s][j].load(p.w, static_cast<long long>(o0 + j) * p.k + k0 + c);
     }
   pdl_launch_dependents();
   pdl_wait();
@@ -135,25 +152,30 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
   for (int i = 0; i < N; ++i) acc[i] = 0.0f;
 #pragma unroll
   for (int s = 0; s < STEPS; ++s) {
+    float4 w[SC_WR];
+#pragma unroll
+    for (int j = 0; j < SC_WR; ++j) w[j] = wv[s][j].get();
 #pragma unroll
     for (int r = 0; r < MT; ++r) {
       const float4 xv = *reinterpret_cast<const float4*>(xs + r * KC + s * SC_STEP + lane * 4);
 #pragma unroll
       for (int j = 0; j < SC_WR; ++j) {
         float a = acc[j * MT + r];
-        a = fmaf(wv[s][j].x, xv.x, a);
-        a = fmaf(wv[s][j].y, xv.y, a);
-        a = fmaf(wv[s][j].z, xv.z, a);
-        a = fmaf(wv[s][j].w, xv.w, a);
+        a = fmaf(w[j].x, xv.x, a);
+        a = fmaf(w[j].y, xv.y, a);
+        a = fmaf(w[j].z, xv.z, a);
+        a = fmaf(w[j].w, xv.w, a);
         acc[j * MT + r] = a;
       }
     }
   }
-  // recursive halving (skinny.cu): a lane ends with the sums of indices lane * PER + t, index = row-of-W * MT + row-of-x
+  // recursive halving (skinny.cu), R rounds, then the lanes that hold the same values add them up: a lane ends with the sums of
+  // indices (lane >> (5 - R)) * PER + t, index = row-of-W * MT + row-of-x
 #pragma unroll
-  for (int half = N / 2, mask = 16; mask >= 1; half >>= 1, mask >>= 1) {
-    const bool upper = (lane & mask) != 0;
-    if (half >= 1) {
+  for (int round = 0; round < 5; ++round) {
+    const int mask = 16 >> round, half = N >> (round + 1);
+    if (round < R) {
+      const bool upper = (lane & mask) != 0;
 #pragma unroll
       for (int i = 0; i < half; ++i) {
         const float send = upper ? acc[i] : acc[i + half];
@@ -161,7 +183,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
         acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
       }
     } else {
-      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], mask);  // fewer values than lanes: the holders of one value add up
+#pragma unroll
+      for (int i = 0; i < PER; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], mask);
     }
   }
   cluster_wait();  // every CTA of the cluster runs: rank 0's shared memory may be written
@@ -172,17 +195,15 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
     const int j = idx / MT, r = idx - j * MT;
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(base + static_cast<uint32_t>((r * SC_ROWS + warp * SC_WR + j) * 4)), "f"(v) : "memory");
   };
-  if (PER >= 1) {
+  if ((lane & ((1 << (5 - R)) - 1)) == 0) {
 #pragma unroll
-    for (int t = 0; t < (PER >= 1 ? PER : 1); ++t) put(lane * PER + t, acc[t]);
-  } else if ((lane & 1) == 0) {
-    put(lane >> 1, acc[0]);  // N = 16: two lanes hold each value
+    for (int t = 0; t < PER; ++t) put((lane >> (5 - R)) * PER + t, acc[t]);
   }
   cluster_arrive();
   cluster_wait();
   if (rank != 0) return;
   for (int i = threadIdx.x; i < p.m * SC_ROWS; i += SC_THREADS) {
-    const int r = i / SC_ROWS, o = tile * SC_ROWS + (i & (SC_ROWS - 1));
+    const int r = i / SC_ROWS, o = tile * SC_ROWS + i % SC_ROWS;
     if (o >= p.n) continue;
     float v = part[i];
     for (uint32_t s = 1; s < size; ++s) v += part[s * (MT * SC_ROWS) + i];
@@ -194,44 +215,92 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
   }
 }
 
-struct ClusterShape { int steps = 0, splits = 0; };
-// The fewest k steps per CTA with which the K ranges fit a cluster and all CTAs are resident at once (two per SM).
-ClusterShape cluster_shape(int k, int n) {
-  const int tiles = (n + SC_ROWS - 1) / SC_ROWS;
-  for (int steps = 1; steps <= 3; ++steps) {
-    const int splits = (k + steps * SC_STEP - 1) / (steps * SC_STEP);
-    if (splits <= 8 && static_cast<long long>(tiles) * splits <= 2 * ctx().sm_count) return {steps, splits};
-  }
-  return {};
+struct ClusterShape { int wr = 0, steps = 0, splits = 0; };
+// Rows per warp, k steps per CTA and K ranges of a launch.  The time of such a launch after its input is ready is the FMAs of the
+// busiest SM plus a latency chain, so: few CTAs per SM (one where possible - the previous kernel's CTAs still hold registers
+// when this one's should start loading), little work in each, a cluster only where K needs it.
+ClusterShape cluster_shape(int m, int k, int n, bool bf16) {
+  const int mt = m <= 4 ? 4 : m <= 8 ? 8 : 16, sms = ctx().sm_count;
+  ClusterShape best;
+  long long best_cost = 0;
+  for (int wr = 2; wr <= 4; ++wr)
+    for (int steps = 2; steps <= 6; steps += bf16 ? 2 : 1) {
+      if (!bf16 && (steps > 3 || wr == 3)) continue;
+      const int splits = (k + steps * SC_STEP - 1) / (steps * SC_STEP);
+      const long long ctas = static_cast<long long>((n + SC_WARPS * wr - 1) / (SC_WARPS * wr)) * splits;
+      if (splits > 8 || ctas > 2 * sms) continue;
+      const long long cost = (ctas + sms - 1) / sms * (steps * wr * mt * 8 + 600) + (splits > 1 ? 300 + 60 * splits : 0);
+      if (best.wr == 0 || cost < best_cost) { best = {wr, steps, splits}; best_cost = cost; }
+    }
+  return best;
 }
 
+template <int MT, int WR, int STEPS, int BF16>
+int launch_shape(const SkinnyClusterParams& p, const ClusterShape& c, cudaStream_t st) {
+  constexpr int ROWS = SC_WARPS * WR;
+  const size_t smem = (static_cast<size_t>(MT) * p.kc + static_cast<size_t>(c.splits) * MT * ROWS) * sizeof(float);
+  static PerDeviceOnce attr_once;
+  MB_TRY(attr_once.run([&]() -> int {
+    MB_CUDA(cudaFuncSetAttribute(skinny_cluster_kernel<MT, WR, STEPS, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (MT * STEPS * SC_STEP + 8 * MT * ROWS) * static_cast<int>(sizeof(float))));
+    return MIMIR_B200_OK;
+  }));
+  return launch_pdl(skinny_cluster_kernel<MT, WR, STEPS, BF16>, dim3(static_cast<unsigned>((p.n + ROWS - 1) / ROWS * c.splits)), dim3(SC_THREADS), smem, st,
+                    c.splits, p);
+}
+template <int MT, int WR>
+int launch_rows(const SkinnyClusterParams& p, const ClusterShape& c, bool bf16, cudaStream_t st) {
+  if (bf16) return c.steps == 2 ? launch_shape<MT, WR, 2, 1>(p, c, st) : c.steps == 4 ? launch_shape<MT, WR, 4, 1>(p, c, st) : launch_shape<MT, WR, 6, 1>(p, c, st);
+  return c.steps == 2 ? launch_shape<MT, WR, 2, 0>(p, c, st) : launch_shape<MT, WR, 3, 0>(p, c, st);
+}
 template <int MT>
-int launch_mt(const SkinnyClusterParams& p, const ClusterShape& c, cudaStream_t st) {
-  const dim3 grid(static_cast<unsigned>((p.n + SC_ROWS - 1) / SC_ROWS * c.splits)), block(SC_THREADS);
-  const size_t smem = (static_cast<size_t>(MT) * p.kc + static_cast<size_t>(c.splits) * MT * SC_ROWS) * sizeof(float);
-  if (c.steps == 1) return launch_pdl(skinny_cluster_kernel<MT, 1>, grid, block, smem, st, c.splits, p);
-  if (c.steps == 2) return launch_pdl(skinny_cluster_kernel<MT, 2>, grid, block, smem, st, c.splits, p);
-  return launch_pdl(skinny_cluster_kernel<MT, 3>, grid, block, smem, st, c.splits, p);
+int launch_mt(const SkinnyClusterParams& p, const ClusterShape& c, bool bf16, cudaStream_t st) {
+  if (c.wr == 2) return launch_rows<MT, 2>(p, c, bf16, st);
+  if (c.wr == 3) return launch_rows<MT, 3>(p, c, true, st);
+  return launch_rows<MT, 4>(p, c, bf16, st);
+}
+
+// dst = the upper halves of src's bit patterns; *inexact becomes 1 when some lower half is not zero
+__global__ void pack_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, size_t n, int* __restrict__ inexact) {
+  bool bad = false;
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    const uint32_t u = __float_as_uint(__ldg(src + i));
+    dst[i] = static_cast<uint16_t>(u >> 16);
+    bad = bad || (u & 0xffffu) != 0;
+  }
+  if (bad) *inexact = 1;
 }
 
 }  // namespace
 
 bool skinny_cluster_supported(int m, int k, int n) {
-  return m >= 1 && m <= 16 && k % 4 == 0 && cluster_shape(k, n).steps > 0;
+  // (with bfloat16 weights every shape that fits as fp32 fits too: the choice of a fused LayerNorm does not depend on them)
+  return m >= 1 && m <= 16 && k % 4 == 0 && cluster_shape(m, k, n, false).wr > 0;
+}
+
+int launch_pack_bf16(const float* src, uint16_t* dst, size_t n, int* inexact, cudaStream_t st) {
+  size_t blocks = (n + 1023) / 1024;
+  if (blocks > static_cast<size_t>(ctx().sm_count) * 8) blocks = static_cast<size_t>(ctx().sm_count) * 8;
+  pack_bf16_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(src, dst, n, inexact);
+  MB_CUDA(cudaGetLastError());
+  count_launch();
+  return MIMIR_B200_OK;
 }
 
 int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st) {
   if (!skinny_cluster_supported(a.m, a.k, a.n)) return fail(MIMIR_B200_E_INVALID, "skinny linear: not a shape of the cluster kernel");
-  const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta);
+  const bool bf16 = a.w_bf16 != nullptr;
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(bf16 ? static_cast<const void*>(a.w_bf16) : a.w) |
+                         reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta);
   if (bits & 15) return fail(MIMIR_B200_E_INVALID, "skinny linear: operands not 16-byte aligned");
-  const ClusterShape c = cluster_shape(a.k, a.n);
+  const ClusterShape c = cluster_shape(a.m, a.k, a.n, bf16);
   SkinnyClusterParams p;
-  p.x = a.x; p.w = a.w; p.bias = a.bias; p.residual = a.residual; p.y = a.y;
+  p.x = a.x; p.w = bf16 ? static_cast<const void*>(a.w_bf16) : a.w; p.bias = a.bias; p.residual = a.residual; p.y = a.y;
   p.gamma = a.gamma; p.beta = a.beta; p.eps = a.eps; p.ln = a.ln ? 1 : 0;
   p.m = a.m; p.k = a.k; p.n = a.n; p.kc = c.steps * SC_STEP; p.act = a.activation; p.w_ready = a.w_ready ? 1 : 0;
-  if (a.m <= 4) MB_TRY(launch_mt<4>(p, c, st));
-  else if (a.m <= 8) MB_TRY(launch_mt<8>(p, c, st));
-  else MB_TRY(launch_mt<16>(p, c, st));
+  if (a.m <= 4) MB_TRY(launch_mt<4>(p, c, bf16, st));
+  else if (a.m <= 8) MB_TRY(launch_mt<8>(p, c, bf16, st));
+  else MB_TRY(launch_mt<16>(p, c, bf16, st));
   count_launch();
   return MIMIR_B200_OK;
 }
