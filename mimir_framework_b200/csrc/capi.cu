@@ -181,13 +181,13 @@ bool linear_uses_skinny(int rows, int precision) {
   return rows <= 16;
 }
 
-bool linear_takes_layernorm(int rows, int in_f, int out_f) { return rows <= 16 && skinny_cluster_supported(rows, in_f, out_f); }
+bool linear_takes_layernorm(int rows, int in_f, int out_f) { return skinny_cluster_supported(rows, in_f, out_f) || skinny_rows_supported(rows, in_f, out_f); }
 
 // y = act(norm(x) . w^T + bias) (+ residual) for at most 16 rows: one launch where the weights fit a wave of CTAs, else the
 // streaming kernel and its finishing kernel
 static int skinny_linear(const float* x, const float* w, const uint16_t* w_bf16, const float* bias, float* y, int rows, int k, int n, int act, const PreLayerNorm& pre,
                          bool w_ready, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual) {
-  if (skinny_cluster_supported(rows, k, n) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w_bf16)) & 15) == 0) {
+  if (linear_takes_layernorm(rows, k, n) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w_bf16)) & 15) == 0) {
     SkinnyClusterArgs a;
     a.x = x; a.w = w; a.w_bf16 = w_bf16; a.bias = bias; a.residual = residual; a.y = y; a.m = rows; a.k = k; a.n = n; a.activation = act; a.w_ready = w_ready;
     a.ln = pre.on; a.gamma = pre.gamma; a.beta = pre.gamma ? pre.beta : nullptr; a.eps = pre.eps;
