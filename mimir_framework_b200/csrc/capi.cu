@@ -181,7 +181,7 @@ bool linear_uses_skinny(int rows, int precision) {
   return rows <= 16;
 }
 
-bool linear_takes_layernorm(int rows, int in_f, int out_f) { return skinny_cluster_supported(rows, in_f, out_f) || skinny_rows_supported(rows, in_f, out_f); }
+bool linear_takes_layernorm(int rows, int in_f, int out_f) { return skinny_cluster_supported(rows, in_f, out_f); }
 
 // y = act(norm(x) . w^T + bias) (+ residual) for at most 16 rows: one launch where the weights fit a wave of CTAs, else the
 // streaming kernel and its finishing kernel

@@ -231,7 +231,6 @@ struct SkinnyClusterArgs {
   bool w_ready = false;  // as GemmArgs::w_ready
 };
 bool skinny_cluster_supported(int m, int k, int n);
-bool skinny_rows_supported(int m, int k, int n);  // its form for any number of weight rows
 // bfloat16 copy of fp32 values; *inexact (device) becomes 1 when one of them is not a bfloat16
 int launch_pack_bf16(const float* src, uint16_t* dst, size_t n, int* inexact, cudaStream_t st);
 int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st);
