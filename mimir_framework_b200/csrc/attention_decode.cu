@@ -17,6 +17,7 @@ namespace mb {
 namespace {
 
 constexpr int AD_THREADS = 128, AD_WARPS = 4;
+constexpr int AD_OCC = 3;  // CTAs per SM
 constexpr int AD_U = 8;  // K rows (and V rows) a lane has in flight
 
 struct AttnDecodeParams {
@@ -30,7 +31,7 @@ struct AttnDecodeParams {
 };
 
 template <int LPK>
-__global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const AttnDecodeParams p) {
+__global__ void __launch_bounds__(AD_THREADS, AD_OCC) attn_decode_fused_kernel(const AttnDecodeParams p) {
   constexpr int HD = LPK * 4, KPW = 32 / LPK;  // head size; keys a warp covers with one load
   constexpr int GROUP = KPW * AD_U;
   __shared__ float s_m[AD_WARPS], s_l[AD_WARPS];
@@ -54,13 +55,22 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
   const float* qrow = p.qkv + static_cast<long long>(b) * 3 * p.embed + h * HD + q4 * 4;
 
   float4 kv[AD_U], vv[AD_U];
-  auto load_rows = [&](float4 (&r)[AD_U], const float* base, int g) {  // the cached rows of group g (the new one comes from the projection)
+  int off[AD_U];  // of a lane's rows within a group
 #pragma unroll
-    for (int u = 0; u < AD_U; ++u) {
-      const int key = g * GROUP + u * KPW + sub;
-      r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (key < pos)
-        asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r[u].x), "=f"(r[u].y), "=f"(r[u].z), "=f"(r[u].w) : "l"(base + static_cast<long long>(key) * p.embed));
+  for (int u = 0; u < AD_U; ++u) off[u] = (u * KPW + sub) * p.embed;
+  auto load_rows = [&](float4 (&r)[AD_U], const float* base, int g) {  // the cached rows of group g (the new one comes from the projection)
+    const float* at = base + static_cast<long long>(g) * (GROUP * p.embed);
+    if ((g + 1) * GROUP <= pos) {  // (warp-uniform) all cached: no predicates
+#pragma unroll
+      for (int u = 0; u < AD_U; ++u)
+        asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r[u].x), "=f"(r[u].y), "=f"(r[u].z), "=f"(r[u].w) : "l"(at + off[u]));
+    } else {
+#pragma unroll
+      for (int u = 0; u < AD_U; ++u) {
+        r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g * GROUP + u * KPW + sub < pos)
+          asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r[u].x), "=f"(r[u].y), "=f"(r[u].z), "=f"(r[u].w) : "l"(at + off[u]));
+      }
     }
   };
   if (!p.cached_ready) pdl_wait();
@@ -103,13 +113,13 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
       }
     }
 #pragma unroll
-    for (int mask = LPK / 16; mask >= 1; mask >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], mask);
-    const int mine = (q4 * 8) / LPK;  // which of the eight
+    for (int mask = LPK / (2 * AD_U); mask >= 1; mask >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], mask);
+    const int mine = (q4 * AD_U) / LPK;  // which of the AD_U
     const bool in = g * GROUP + mine * KPW + sub < nkeys;
     const float s = in ? d[0] * p.scale : -INFINITY;
     float mx = s;
 #pragma unroll
-    for (int mask = 16; mask >= LPK / 8; mask >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, mask));
+    for (int mask = 16; mask >= LPK / AD_U; mask >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, mask));
     const float mn = fmaxf(m, mx), corr = expf(m - mn);
     m = mn;
     const float pr = expf(s - mn);  // exp(-inf) = 0 past the last key
@@ -117,7 +127,7 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
     acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
 #pragma unroll
     for (int u = 0; u < AD_U; ++u) {
-      const float w = __shfl_sync(0xffffffffu, pr, sub * LPK + u * (LPK / 8));
+      const float w = __shfl_sync(0xffffffffu, pr, sub * LPK + u * (LPK / AD_U));
       acc.x = fmaf(w, vv[u].x, acc.x); acc.y = fmaf(w, vv[u].y, acc.y); acc.z = fmaf(w, vv[u].z, acc.z); acc.w = fmaf(w, vv[u].w, acc.w);
     }
     if (g + 1 < g1) load_rows(vv, vc, g + 1);
@@ -125,7 +135,7 @@ __global__ void __launch_bounds__(AD_THREADS, 4) attn_decode_fused_kernel(const 
   // l: LPK / 8 lanes hold the same probabilities; the sum over the warp counts each that often (a power of two, exact)
 #pragma unroll
   for (int mask = 16; mask >= 1; mask >>= 1) l += __shfl_xor_sync(0xffffffffu, l, mask);
-  l *= 8.0f / LPK;
+  l *= static_cast<float>(AD_U) / LPK;
   *reinterpret_cast<float4*>(&s_o[warp * KPW + sub][q4 * 4]) = acc;
   if (lane == 0) { s_m[warp] = m; s_l[warp] = l; }
   __syncthreads();
@@ -184,9 +194,10 @@ int launch_attention_decode_fused(const float* qkv, float* kcache, float* vcache
   p.qkv = qkv; p.kcache = kcache; p.vcache = vcache; p.out = out; p.pos_dev = pos_dev; p.pos = pos; p.heads = heads; p.embed = embed;
   p.max_seq = max_seq; p.cached_ready = cached_ready ? 1 : 0;
   p.scale = 1.0f / sqrtf(static_cast<float>(hd));
-  // as many CTAs per (sample, head) as keep the launch within one wave of four CTAs per SM
-  int c = 4 * ctx().sm_count / bh;
-  c = c < 1 ? 1 : (c > 8 ? 8 : c);
+  // as many CTAs per (sample, head) as keep the launch within one wave, in powers of two (clusters of three left SMs empty:
+  // 16 samples x 12 heads, 992 keys: 25 us; of two, 17.3 us = 5.6 TB/s)
+  const int fit = AD_OCC * ctx().sm_count / bh;
+  const int c = fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
   const dim3 grid(static_cast<unsigned>(bh) * static_cast<unsigned>(c)), block(AD_THREADS);
   if (hd == 32) MB_TRY(launch_pdl(attn_decode_fused_kernel<8>, grid, block, 0, st, c, p));
   else if (hd == 64) MB_TRY(launch_pdl(attn_decode_fused_kernel<16>, grid, block, 0, st, c, p));

@@ -1863,11 +1863,11 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
     MB_TRY(run_layers_cached(m, micro, b, m->s_comp, arena));
     MB_CUDA(cudaEventRecord(m->ev_comp[c], m->s_comp));
     MB_CUDA(cudaStreamWaitEvent(m->s_d2h, m->ev_comp[c], 0));
+    if (c + 1 == P) MB_TRY(enqueue_error_word(m->s_d2h));  // (this stream has waited for every micro-batch's compute)
     MB_TRY(copy_to_host(out_host + static_cast<size_t>(c) * micro * ot.n, arena + ot.off_f32, static_cast<size_t>(ot.n) * micro * 4, m->s_d2h));
     MB_CUDA(cudaEventRecord(m->ev_d2h[c], m->s_d2h));
   }
   MB_CUDA(cudaEventRecord(m->ev1, m->s_comp));
-  MB_TRY(enqueue_error_word(m->s_d2h));  // (the copy-out stream has waited for every micro-batch's compute)
   MB_CUDA(cudaStreamSynchronize(m->s_d2h));
   MB_CUDA(cudaEventSynchronize(m->ev1));
   MB_TRY(read_error_word(m->s_comp));

@@ -1,0 +1,67 @@
+"""Linear layers of at most 16 rows (csrc/skinny_cluster.cu) and the fused decode attention (csrc/attention_decode.cu) at the edges of
+their tiles: one row, odd feature counts, K below and across a step, K ranges over a cluster, folded LayerNorm, exact bfloat16
+weights; cache positions around a group of keys and head sizes 32, 64 and 128."""
+import numpy as np
+import pytest
+
+from mimir_framework_b200 import abi, configs
+from mimir_framework_b200.abi import make_desc
+from oracle import port
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    from mimir_framework_b200 import runtime
+
+    runtime.init(0)
+    return runtime
+
+
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (3, 33, 128), (4, 31, 132), (5, 100, 768), (8, 4737, 300), (9, 768, 3072), (16, 2304, 768), (16, 65, 4096), (2, 40, 1028)])
+def test_few_rows_against_float64(rt, norm, m, n, k):
+    r = np.random.default_rng(m * 31 + n)
+    x = r.standard_normal((m, k)).astype(np.float32)
+    w, b = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32), r.standard_normal(n).astype(np.float32)
+    g, be = (1 + 0.1 * r.standard_normal(k)).astype(np.float32), r.standard_normal(k).astype(np.float32)
+    lin = make_desc("l", "Linear", inputs=["h" if norm else "x"], output="y", in_features=k, out_features=n, seq_len=m, use_bias=1, params_count=n * k + n)
+    descs = ([make_desc("n", "LayerNorm", inputs=["x"], output="h", in_features=k, affine=1, use_bias=1, eps=1e-5, params_count=2 * k)] if norm else []) + [
+        lin, make_desc("s", "SiLU", inputs=["y"], output="x")]
+    weights = ([np.concatenate([g, be])] if norm else []) + [np.concatenate([w.ravel(), b]), None]
+    mod = rt.GraphModel(descs)
+    for i, t in enumerate(weights):
+        mod.upload_weights(i, t)
+    mod.plan({"x": (m * k, False)}, 1)
+    got = mod.forward({"x": (x.ravel(), False)}, 1, m * n).reshape(m, n)
+    mod.close()
+    h = x.astype(np.float64)
+    if norm:
+        h = (h - h.mean(1, keepdims=True)) / np.sqrt(h.var(1, keepdims=True) + 1e-5) * g + be
+    y = h @ w.astype(np.float64).T + b
+    want = y / (1 + np.exp(-y))
+    assert np.linalg.norm(got - want) <= 2e-6 * np.linalg.norm(want) + 1e-7
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("batch,heads,hd,prefix", [(1, 3, 64, 15), (2, 4, 32, 31), (3, 2, 128, 7), (16, 4, 64, 16), (1, 1, 64, 1)])
+def test_decode_steps_against_the_full_forward(rt, bf16, batch, heads, hd, prefix):
+    """Two steps behind a prefix; each row must be the last row of the full causal forward."""
+    E, V, steps = heads * hd, 77, 2
+    ids = np.random.default_rng(5).integers(0, V, (batch, prefix + steps)).astype(np.float32)
+    cfg = dict(layers=2, d_model=E, heads=heads, ffn=4 * E, vocab=V, norm="layer")
+    weights = configs.seeded_weights(configs.gpt_decoder(seq=prefix, **cfg), seed=2, std=0.05, bf16=bf16)
+    m = rt.GraphModel(configs.gpt_decoder(seq=prefix, **cfg), abi.PREC_BF16W if bf16 else abi.PREC_BF16X2)
+    for i, w in enumerate(weights):
+        m.upload_weights(i, w)
+    m.plan({"x": (prefix, False)}, batch)
+    m.decode_begin({"x": (1, False)}, batch, prefix + steps)
+    m.forward({"x": (ids[:, :prefix].copy().ravel(), False)}, batch, prefix * V)
+    for t in range(prefix, prefix + steps):
+        got = m.decode_step({"x": (ids[:, t].copy(), False)}, batch, t, V).reshape(batch, V)
+        descs = configs.gpt_decoder(seq=t + 1, **cfg)
+        for b in range(batch):
+            want = port.run_graph(descs, weights, {"x": ids[b, : t + 1]}).reshape(t + 1, V)[-1]
+            assert np.linalg.norm(got[b] - want) <= 2e-5 * np.linalg.norm(want)
+    m.close()
