@@ -9,7 +9,6 @@
 // on the CUDA cores; K and Q tiles are held d-major in shared memory so that the 4x4 register
 // blocks read them as conflict-free 128-bit vectors.
 #include "common.h"
-#include "launch.cuh"
 
 namespace mb {
 namespace {
@@ -19,8 +18,6 @@ constexpr int BQ = 64, BKV = 64, LDT = 68;  // LDT: padded leading dimension of 
 template <int HD>
 __global__ void __launch_bounds__(256)
 flash_attn_fp32_kernel(const AttnView a, float* __restrict__ out, int embed, int heads, int causal, float scale) {
-  pdl_launch_dependents();
-  pdl_wait();
   constexpr int CPT = HD / 16;  // output columns per thread
   extern __shared__ __align__(16) float sm[];
   float* Qt = sm;                 // [HD][LDT]   Qt[d][row]
@@ -159,8 +156,6 @@ flash_attn_fp32_kernel(const AttnView a, float* __restrict__ out, int embed, int
 constexpr int AR = 8;
 
 __global__ void attn_row_kernel(const AttnView a, float* __restrict__ out, int embed, int heads, int hd, int causal, float scale) {
-  pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   float* q = sm;               // [AR][hd]
   float* p = sm + AR * hd;     // [AR][kv_len]
@@ -321,7 +316,7 @@ int launch_flash(const AttnView& a, float* out, int batch, int embed, int heads,
     return MIMIR_B200_OK;
   }));
   dim3 grid((a.q_len + BQ - 1) / BQ, heads, batch);
-  MB_TRY(launch_pdl(flash_attn_fp32_kernel<HD>, dim3(grid), dim3(256), SMEM, st, 1, a, out, embed, heads, causal, scale));
+  flash_attn_fp32_kernel<HD><<<grid, 256, SMEM, st>>>(a, out, embed, heads, causal, scale);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -352,7 +347,7 @@ int launch_attention_core_view(const AttnView& a, float* out, int batch, int emb
     return MIMIR_B200_OK;
   }));
   dim3 grid((a.q_len + AR - 1) / AR, heads, batch);
-  MB_TRY(launch_pdl(attn_row_kernel, dim3(grid), dim3(256), smem, st, 1, a, out, embed, heads, hd, causal, scale));
+  attn_row_kernel<<<grid, 256, smem, st>>>(a, out, embed, heads, hd, causal, scale);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

@@ -9,7 +9,6 @@
 // Every operand travels as hi + lo 16-bit planes and every product is taken with three MMAs (both sides are data, nothing
 // is exact in one plane), so the result sits inside the same tolerance as the fp32 row kernel it replaces.
 #include "common.h"
-#include "launch.cuh"
 #include "ops.h"
 #include "planes.cuh"
 
@@ -19,8 +18,6 @@ namespace {
 // Q and K planes [rows][E] out of the fp32 QKV rows [rows][3E]; one thread per 16-byte chunk (8 values) of Q or K
 __global__ void attn_qk_planes_kernel(const float* __restrict__ qkv, __nv_bfloat16* __restrict__ qp, __nv_bfloat16* __restrict__ kp,
                                       long long rows, int E, int f16) {
-  pdl_launch_dependents();
-  pdl_wait();
   const int chunks = E >> 3;
   const long long total = rows * chunks * 2;
   const long long plane_stride = rows * static_cast<long long>(E);
@@ -45,8 +42,6 @@ __global__ void attn_qk_planes_kernel(const float* __restrict__ qkv, __nv_bfloat
 
 // V^T planes [B*E][S]: row b*E + e holds V[b*S + s][e] over s.  32 x 32 tiles through shared memory.
 __global__ void attn_vt_planes_kernel(const float* __restrict__ qkv, __nv_bfloat16* __restrict__ vt, int batch, int S, int E, int f16) {
-  pdl_launch_dependents();
-  pdl_wait();
   __shared__ float tile[32][33];
   const int s0 = blockIdx.x * 32, e0 = blockIdx.y * 32, b = blockIdx.z;
   for (int i = threadIdx.y; i < 32; i += blockDim.y)
@@ -66,8 +61,6 @@ __global__ void attn_vt_planes_kernel(const float* __restrict__ qkv, __nv_bfloat
 // One warp per score row: the reference's softmax (LayerOps.hpp:1052-1080) and the hi / lo planes of the probabilities.
 __global__ void attn_softmax_planes_kernel(const float* __restrict__ scores, __nv_bfloat16* __restrict__ p, long long rows, int S,
                                            int causal, float scale, int f16) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -142,9 +135,9 @@ int launch_attention_core_gemm(const float* qkv, int batch, int seq, int embed, 
   {
     const long long total = rows * (embed >> 3) * 2;
     const long long blocks = std::min<long long>((total + 255) / 256, static_cast<long long>(ctx().sm_count) * 16);
-    MB_TRY(launch_pdl(attn_qk_planes_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, qkv, qp, kp, rows, embed, f16));
+    attn_qk_planes_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(qkv, qp, kp, rows, embed, f16);
     MB_CUDA(cudaGetLastError());
-    MB_TRY(launch_pdl(attn_vt_planes_kernel, dim3(dim3(seq / 32, embed / 32, batch)), dim3(dim3(32, 8)), 0, st, 1, qkv, vt, batch, seq, embed, f16));
+    attn_vt_planes_kernel<<<dim3(seq / 32, embed / 32, batch), dim3(32, 8), 0, st>>>(qkv, vt, batch, seq, embed, f16);
     MB_CUDA(cudaGetLastError());
     count_launch(2);
   }
@@ -156,8 +149,8 @@ int launch_attention_core_gemm(const float* qkv, int batch, int seq, int embed, 
   MB_TRY(launch_gemm(s, st));
   {
     const long long blocks = std::min<long long>((rows * 32 + 255) / 256, static_cast<long long>(ctx().sm_count) * 16);
-    MB_TRY(launch_pdl(attn_softmax_planes_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, scores, pp, rows, seq, causal,
-                                                                             1.0f / sqrtf(static_cast<float>(embed)), f16));
+    attn_softmax_planes_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(scores, pp, rows, seq, causal,
+                                                                             1.0f / sqrtf(static_cast<float>(embed)), f16);
     MB_CUDA(cudaGetLastError());
     count_launch();
   }

@@ -27,7 +27,6 @@
 // Every mbarrier wait is bounded; on expiry the CTA raises its abort flag, sets the device error word,
 // leaves all loops and frees its TMEM.
 #include "common.h"
-#include "launch.cuh"
 #include "planes.cuh"
 #include "sm100_ptx.cuh"
 
@@ -528,8 +527,6 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_launch_dependents();
-  pdl_wait();
   const uint32_t tmem_o = tmem_base + 3 * AT_BK;  // score / probability tile b lives at tmem_base + b * 64
 
   if (warp == 0) {
@@ -909,7 +906,8 @@ int launch_attention_core_tc(const float* qkv, float* out, int batch, int seq, i
       MB_CUDA(cudaFuncSetAttribute(flash_attn_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, A2_SMEM));
       return MIMIR_B200_OK;
     }));
-    MB_TRY(launch_pdl(flash_attn_tc2_kernel, grid, dim3(A2_THREADS), static_cast<size_t>(A2_SMEM), st, 1, mq, mk, mv, p));
+    flash_attn_tc2_kernel<<<grid, A2_THREADS, A2_SMEM, st>>>(mq, mk, mv, p);
+    MB_CUDA(cudaGetLastError());
     count_launch(1);
     return MIMIR_B200_OK;
   }

@@ -5,7 +5,6 @@
 // bf16 hi/lo planes the GEMM consumes (one pass over the input, no fp32 column matrix), the OIHW
 // weight block already is the K-major [oc][ic*k*k] operand, and the GEMM epilogue writes NCHW.
 #include "common.h"
-#include "launch.cuh"
 #include "planes.cuh"
 
 namespace mb {
@@ -14,8 +13,6 @@ namespace {
 // One thread produces 8 consecutive K entries of one output pixel.
 __global__ void im2col_split_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst, long long rows, int ic, int h,
                                     int w, int ks, int stride, int pad, int oh, int ow, int k, int kp, int planes, int f16) {
-  pdl_launch_dependents();
-  pdl_wait();
   const int chunks = kp >> 3;
   const long long total = rows * chunks;
   const long long plane_stride = rows * static_cast<long long>(kp);
@@ -65,8 +62,6 @@ constexpr int I2C_TPX = 32;
 __global__ void __launch_bounds__(256) im2col_tile_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst, long long rows,
                                                           int ic, int h, int w, int ks, int stride, int pad, int oh, int ow, int k,
                                                           int kp, int planes, int f16, int cb, int nblocks) {
-  pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ float patch[];  // [cbn][ks][pw]
   const int ox0 = blockIdx.x * I2C_TPX, oy = blockIdx.y;
   const int smp = blockIdx.z / nblocks, blk = blockIdx.z - smp * nblocks;
@@ -126,8 +121,8 @@ int launch_im2col_split(const float* x, __nv_bfloat16* dst, int batch, int ic, i
     const int nblocks = cb > 0 ? (ic + cb - 1) / cb : 0;
     if (!off && cb > 0 && static_cast<long long>(batch) * nblocks <= 65535 && oh <= 65535) {
       dim3 grid((ow + I2C_TPX - 1) / I2C_TPX, oh, batch * nblocks);
-      MB_TRY(launch_pdl(im2col_tile_kernel, dim3(grid), dim3(256), static_cast<size_t>(cb) * per_ch, st, 1, x, dst, rows, ic, h, w, ks, stride, pad, oh, ow, k, kp, planes,
-                                                                              plane_format() == PLANES_F16, cb, nblocks));
+      im2col_tile_kernel<<<grid, 256, static_cast<size_t>(cb) * per_ch, st>>>(x, dst, rows, ic, h, w, ks, stride, pad, oh, ow, k, kp, planes,
+                                                                              plane_format() == PLANES_F16, cb, nblocks);
       MB_CUDA(cudaGetLastError());
       count_launch();
       return MIMIR_B200_OK;
@@ -137,7 +132,7 @@ int launch_im2col_split(const float* x, __nv_bfloat16* dst, int batch, int ic, i
   long long blocks = (total + 255) / 256;
   const long long cap = static_cast<long long>(ctx().sm_count) * 32;
   if (blocks > cap) blocks = cap;
-  MB_TRY(launch_pdl(im2col_split_kernel, dim3(static_cast<int>(blocks)), dim3(256), 0, st, 1, x, dst, rows, ic, h, w, ks, stride, pad, oh, ow, k, kp, planes, plane_format() == PLANES_F16));
+  im2col_split_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(x, dst, rows, ic, h, w, ks, stride, pad, oh, ow, k, kp, planes, plane_format() == PLANES_F16);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -169,8 +164,6 @@ __device__ __forceinline__ void cp_async16_zfill(void* smem_dst, const void* gme
 __global__ void __launch_bounds__(256, 3) nchw_to_padded_nhwc_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst,
                                                                   int c, int h, int w, int pad, int planes, long long plane_stride,
                                                                   const PreNorm pre, int f16, int up) {
-  pdl_launch_dependents();
-  pdl_wait();
   __shared__ float tile[TP_C][TP_X + 1];
   const int hp = h + 2 * pad, wp = w + 2 * pad;
   const int cb = blockIdx.x * TP_C;
@@ -263,8 +256,6 @@ __global__ void __launch_bounds__(256, 3) nchw_to_padded_nhwc_kernel(const float
 __global__ void __launch_bounds__(256) nchw_to_padded_nhwc_vec_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst,
                                                                       int c, int h, int w, int pad, int planes, long long plane_stride,
                                                                       const PreNorm pre, int f16, int up) {
-  pdl_launch_dependents();
-  pdl_wait();
   __shared__ float tile[TP_C][TP_X + 1];
   __shared__ float2 s_aff[TP_C];
   const int hp = h + 2 * pad, wp = w + 2 * pad;
@@ -378,8 +369,6 @@ template <int UP>
 __global__ void __launch_bounds__(256, 5) nchw_to_padded_nhwc_stream_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst,
                                                                            int c, int h, int w, int pad, int planes,
                                                                            long long plane_stride, const PreNorm pre, int f16) {
-  pdl_launch_dependents();
-  pdl_wait();
   __shared__ __align__(16) float tile[2][TP_C][LR_TS];
   const int hp = h + 2 * pad, wp = w + 2 * pad;
   const int cb = blockIdx.x * TP_C, n = blockIdx.z;
@@ -519,12 +508,12 @@ int launch_nchw_to_padded_nhwc_split(const float* x, __nv_bfloat16* dst, int bat
   if (vec && !no_stream && (!up || ((w >> 1) & 3) == 0) && (hp + LR_ROWS - 1) / LR_ROWS <= 65535) {
     dim3 sgrid((c + TP_C - 1) / TP_C, (hp + LR_ROWS - 1) / LR_ROWS, batch);
     const int f16 = plane_format() == PLANES_F16;
-    if (up) MB_TRY(launch_pdl(nchw_to_padded_nhwc_stream_kernel<1>, dim3(sgrid), dim3(256), 0, st, 1, x, dst, c, h, w, pad, planes, plane_stride, pre, f16));
-    else MB_TRY(launch_pdl(nchw_to_padded_nhwc_stream_kernel<0>, dim3(sgrid), dim3(256), 0, st, 1, x, dst, c, h, w, pad, planes, plane_stride, pre, f16));
+    if (up) nchw_to_padded_nhwc_stream_kernel<1><<<sgrid, 256, 0, st>>>(x, dst, c, h, w, pad, planes, plane_stride, pre, f16);
+    else nchw_to_padded_nhwc_stream_kernel<0><<<sgrid, 256, 0, st>>>(x, dst, c, h, w, pad, planes, plane_stride, pre, f16);
   } else if (vec)
-    MB_TRY(launch_pdl(nchw_to_padded_nhwc_vec_kernel, dim3(grid), dim3(256), 0, st, 1, x, dst, c, h, w, pad, planes, plane_stride, pre, plane_format() == PLANES_F16, up));
+    nchw_to_padded_nhwc_vec_kernel<<<grid, 256, 0, st>>>(x, dst, c, h, w, pad, planes, plane_stride, pre, plane_format() == PLANES_F16, up);
   else
-    MB_TRY(launch_pdl(nchw_to_padded_nhwc_kernel, dim3(grid), dim3(256), 0, st, 1, x, dst, c, h, w, pad, planes, plane_stride, pre, plane_format() == PLANES_F16, up));
+    nchw_to_padded_nhwc_kernel<<<grid, 256, 0, st>>>(x, dst, c, h, w, pad, planes, plane_stride, pre, plane_format() == PLANES_F16, up);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -585,8 +574,6 @@ template <int OC, int KS, int R, int VEC>
 __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                        float* __restrict__ y, const float* __restrict__ residual, int ic,
                                                                        int h, int wd, int act) {
-  pdl_launch_dependents();
-  pdl_wait();
   using G = SmallOcGeom<KS, R, VEC>;
   constexpr int PAD = G::PAD, TW = G::TW, TH = G::TH, TWP = G::TWP, TILE = G::TILE, SEG = G::SEG, KK = KS * KS;
   constexpr int WROW = (KS * OC + 3) & ~3;  // the weights of one (channel, kernel row) as [kw][o], padded to whole float4s
@@ -739,7 +726,7 @@ int launch_small_oc_v(const float* x, const float* w, float* y, const float* res
     return MIMIR_B200_OK;
   }));
   dim3 grid((wd + SO_TX * SO_PX - 1) / (SO_TX * SO_PX), (h + SO_TY * R - 1) / (SO_TY * R), batch);
-  MB_TRY(launch_pdl(conv_small_oc_kernel<OC, KS, R, VEC>, dim3(grid), dim3(SO_TX * SO_TY), SMEM, st, 1, x, w, y, residual, ic, h, wd, act));
+  conv_small_oc_kernel<OC, KS, R, VEC><<<grid, SO_TX * SO_TY, SMEM, st>>>(x, w, y, residual, ic, h, wd, act);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

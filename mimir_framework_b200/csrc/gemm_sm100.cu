@@ -280,8 +280,6 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   __syncthreads();
   if (PAIR) cluster_sync_all();  // the peer's barriers exist before anything arrives on them
   tcgen05_fence_after();
-  pdl_launch_dependents();
-  pdl_wait();  // (all of the above ran under the previous kernel)
   const uint32_t tmem_base = *tmem_slot;
 
   // planes on the M side (128-row tiles) and on the N side (256-row tiles) of the MMA
@@ -721,8 +719,6 @@ namespace {
 // One thread per 8 consecutive K elements of one row; the padded tail kp > k is written as zero.
 __global__ void split_rows_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int k,
                                   int kp, int planes, int f16, float scale) {
-  pdl_launch_dependents();
-  pdl_wait();
   const int chunks = kp >> 3;
   const long long total = rows * chunks;
   const long long plane_stride = rows * static_cast<long long>(kp);
@@ -916,7 +912,24 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
   }
   GemmProfile prof(st);
   MB_TRY(prof.begin());
-  MB_TRY(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(NUM_THREADS), static_cast<size_t>(SMEM), st, pair ? 2 : 1, map_a, map_w, map_o, p));
+  if (pair) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    MB_CUDA(cudaLaunchKernelEx(&cfg, kern, map_a, map_w, map_o, p));
+  } else {
+    kern<<<grid, NUM_THREADS, SMEM, st>>>(map_a, map_w, map_o, p);
+  }
+  MB_CUDA(cudaGetLastError());
   MB_TRY(prof.end());
   count_launch();
   return MIMIR_B200_OK;
@@ -981,7 +994,7 @@ int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int 
   long long blocks = (total + threads - 1) / threads;
   const long long cap = static_cast<long long>(ctx().sm_count) * 16;
   if (blocks > cap) blocks = cap;
-  MB_TRY(launch_pdl(split_rows_kernel, dim3(static_cast<int>(blocks)), dim3(threads), 0, st, 1, src, dst, rows, k, kp, planes, plane_format() == PLANES_F16, scale));
+  split_rows_kernel<<<static_cast<int>(blocks), threads, 0, st>>>(src, dst, rows, k, kp, planes, plane_format() == PLANES_F16, scale);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

@@ -18,7 +18,6 @@
 #include <utility>
 
 #include "common.h"
-#include "launch.cuh"
 #include "planes.cuh"
 #include "sm100_ptx.cuh"
 
@@ -742,8 +741,6 @@ constexpr int CLUSTER_SLICE_MAX = 12288;  // floats of shared memory per CTA (48
 
 __global__ void __launch_bounds__(256) meanvar_cluster_kernel(const float* __restrict__ x, float* __restrict__ y, long long len,
                                                               int slice, float eps, Affine a) {
-  pdl_launch_dependents();
-  pdl_wait();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) float sx[];
@@ -824,8 +821,6 @@ __global__ void __launch_bounds__(256) meanvar_cluster_kernel(const float* __res
 
 template <int FAM, int THREADS>
 __global__ void __launch_bounds__(THREADS, (THREADS <= 512) ? 2 : 1) sweep_row_kernel(RowParams p) {
-  pdl_launch_dependents();
-  pdl_wait();
   __shared__ float red[33];
   const long long n = p.len;
   for (long long row = blockIdx.x; row < p.rows; row += gridDim.x) {
@@ -927,13 +922,13 @@ int launch_sweep_rows(const RowParams& p, cudaStream_t st) {
   const bool big = p.len * 4 * 2 * sms > (40ll << 20);
   if (big) {
     long long blocks = sms < p.rows ? sms : p.rows;
-    MB_TRY(launch_pdl(sweep_row_kernel<FAM, 1024>, dim3(static_cast<int>(blocks)), dim3(1024), 0, st, 1, p));
+    sweep_row_kernel<FAM, 1024><<<static_cast<int>(blocks), 1024, 0, st>>>(p);
   } else {
     int threads = 512;
     while (threads > 128 && static_cast<long long>(threads) * 16 > p.len) threads >>= 1;  // >= 4 vectors per thread
     long long blocks = sms * (1024 / threads) * 2;
     if (blocks > p.rows) blocks = p.rows;
-    MB_TRY(launch_pdl(sweep_row_kernel<FAM, 512>, dim3(static_cast<int>(blocks)), dim3(threads), 0, st, 1, p));
+    sweep_row_kernel<FAM, 512><<<static_cast<int>(blocks), threads, 0, st>>>(p);
   }
   MB_CUDA(cudaGetLastError());
   count_launch();
@@ -960,8 +955,6 @@ constexpr int WARP_ROW_MAX = 1024;  // floats
 template <int NV>  // 128-bit vectors per lane
 __global__ void __launch_bounds__(256) meanvar_warp_kernel(const float* __restrict__ x, float* __restrict__ y, long long rows,
                                                            int len, float eps, Affine a) {
-  pdl_launch_dependents();
-  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -1023,7 +1016,7 @@ int launch_warp_rows(const float* x, float* y, long long rows, int len, float ep
   long long blocks = (rows + 7) / 8;
   const long long cap = static_cast<long long>(ctx().sm_count) * 8;
   if (blocks > cap) blocks = cap;
-  MB_TRY(launch_pdl(meanvar_warp_kernel<NV>, dim3(static_cast<int>(blocks)), dim3(256), 0, st, 1, x, y, rows, len, eps, a));
+  meanvar_warp_kernel<NV><<<static_cast<int>(blocks), 256, 0, st>>>(x, y, rows, len, eps, a);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -1103,8 +1096,19 @@ int meanvar_dispatch(const float* x, float* y, long long rows, long long len, fl
       MB_CUDA(cudaFuncSetAttribute(meanvar_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CLUSTER_SLICE_MAX * 4));
       return MIMIR_B200_OK;
     }));
-    MB_TRY(launch_pdl(meanvar_cluster_kernel, dim3(static_cast<unsigned>(rows * ncl)), dim3(256), static_cast<size_t>(slice) * sizeof(float), st, ncl, x, y,
-                      static_cast<long long>(len), slice, eps, a));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(rows * ncl));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = static_cast<size_t>(slice) * sizeof(float);
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ncl);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    MB_CUDA(cudaLaunchKernelEx(&cfg, meanvar_cluster_kernel, x, y, len, slice, eps, a));
     count_launch();
     return MIMIR_B200_OK;
   }

@@ -7,7 +7,6 @@
 //   permute            : LayerOps::permute_forward (LayerOps.hpp:880-945)
 //   token_mean_pool    : Model.cpp:5571-5589;  global_avgpool : LayerOps.hpp:459-482
 #include "common.h"
-#include "launch.cuh"
 
 namespace mb {
 namespace {
@@ -35,8 +34,6 @@ __device__ __forceinline__ float act_apply(int op, float v, float alpha = 0.0f) 
 
 template <int OP>
 __global__ void unary_kernel(const float* __restrict__ a, float* __restrict__ y, long long total, float alpha) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
@@ -68,8 +65,6 @@ __device__ __forceinline__ float bin_apply(float u, float w) {
 template <int BOP>
 __global__ void binary_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y,
                               long long batch, long long n, long long nb) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long total = batch * n;
@@ -97,8 +92,6 @@ __global__ void binary_kernel(const float* __restrict__ a, const float* __restri
 __global__ void embedding_kernel(const float* __restrict__ ids_f, const int32_t* __restrict__ ids_i,
                                  const float* __restrict__ table, float* __restrict__ y, long long n_ids, int vocab,
                                  int dim, int padding_idx) {
-  pdl_launch_dependents();
-  pdl_wait();
   // one warp per id row
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -122,8 +115,6 @@ __global__ void embedding_kernel(const float* __restrict__ ids_f, const int32_t*
 
 __global__ void upsample_nearest_kernel(const float* __restrict__ x, float* __restrict__ y, long long planes, int in_h,
                                         int in_w, int sh, int sw) {
-  pdl_launch_dependents();
-  pdl_wait();
   const int oh = in_h * sh, ow = in_w * sw;
   const long long total = planes * oh * ow;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -139,8 +130,6 @@ __global__ void upsample_nearest_kernel(const float* __restrict__ x, float* __re
 // 2 x 2 nearest upsample of rows with an even width: a thread reads two neighbouring input pixels (64 bits)
 // and writes the same four values (128 bits) into two output rows; all index math in 32 bits per plane row.
 __global__ void upsample_nearest_2x2_kernel(const float* __restrict__ x, float* __restrict__ y, long long plane_rows, int in_w) {
-  pdl_launch_dependents();
-  pdl_wait();
   const int half_w = in_w >> 1;
   const long long total = plane_rows * half_w;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -163,8 +152,6 @@ struct PermuteDesc {
 };
 
 __global__ void permute_kernel(const float* __restrict__ x, float* __restrict__ y, PermuteDesc d, long long batch) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long all = batch * d.total;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < all; i += stride) {
@@ -181,8 +168,6 @@ __global__ void permute_kernel(const float* __restrict__ x, float* __restrict__ 
 
 // y[s, d] = (sum_t x[s, t, d]) * (1/seq): sequential in t like the reference
 __global__ void token_mean_pool_kernel(const float* __restrict__ x, float* __restrict__ y, int batch, int seq, int dim) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long total = static_cast<long long>(batch) * dim;
   const float inv = 1.0f / static_cast<float>(seq);
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -197,8 +182,6 @@ __global__ void token_mean_pool_kernel(const float* __restrict__ x, float* __res
 
 // one warp per (sample, channel) plane
 __global__ void global_avgpool_kernel(const float* __restrict__ x, float* __restrict__ y, long long planes, int hw) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -237,8 +220,6 @@ __global__ void argmax_rows_kernel(const float* __restrict__ x, int32_t* __restr
 
 __global__ void copy_strided_kernel(const float* __restrict__ src, float* __restrict__ dst, long long batch, long long n,
                                     long long total, long long off, long long src_stride) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long all = batch * n;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < all;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -270,28 +251,28 @@ int launch_eltwise(int op, const float* a, const float* b, float* y, int batch, 
       if (op == MIMIR_B200_ELT_MULTIPLY && nb != n) return fail(MIMIR_B200_E_INVALID, "Multiply: input sizes must match");
       if (nb != n && nb != 1 && (n % nb) != 0)
         return fail(MIMIR_B200_E_INVALID, "Add: input sizes must match or be broadcastable");
-      if (op == MIMIR_B200_ELT_ADD) MB_TRY(launch_pdl(binary_kernel<0>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
-      else MB_TRY(launch_pdl(binary_kernel<1>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
+      if (op == MIMIR_B200_ELT_ADD) binary_kernel<0><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
+      else binary_kernel<1><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
       break;
     case MIMIR_B200_ELT_SUBTRACT:
     case MIMIR_B200_ELT_DIVIDE:
       if (!b || nb != n)
         return fail(MIMIR_B200_E_INVALID, "%s: size mismatch: %lld vs %lld", op == MIMIR_B200_ELT_SUBTRACT ? "Subtract" : "Divide",
                     static_cast<long long>(n), static_cast<long long>(nb));
-      if (op == MIMIR_B200_ELT_SUBTRACT) MB_TRY(launch_pdl(binary_kernel<2>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
-      else MB_TRY(launch_pdl(binary_kernel<3>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
+      if (op == MIMIR_B200_ELT_SUBTRACT) binary_kernel<2><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
+      else binary_kernel<3><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
       break;
-    case MIMIR_B200_ELT_GELU: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_GELU>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_SILU: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_SILU>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_RELU: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_RELU>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_TANH: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_TANH>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_SIGMOID: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_SIGMOID>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_LEAKY_RELU: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_LEAKY_RELU>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_ELU: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_ELU>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_SOFTPLUS: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_SOFTPLUS>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_MISH: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_MISH>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_HARD_SIGMOID: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_HARD_SIGMOID>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
-    case MIMIR_B200_ELT_HARD_SWISH: MB_TRY(launch_pdl(unary_kernel<MIMIR_B200_ELT_HARD_SWISH>, dim3(grid), dim3(threads), 0, st, 1, a, y, total, alpha)); break;
+    case MIMIR_B200_ELT_GELU: unary_kernel<MIMIR_B200_ELT_GELU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_SILU: unary_kernel<MIMIR_B200_ELT_SILU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_RELU: unary_kernel<MIMIR_B200_ELT_RELU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_TANH: unary_kernel<MIMIR_B200_ELT_TANH><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_SIGMOID: unary_kernel<MIMIR_B200_ELT_SIGMOID><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_LEAKY_RELU: unary_kernel<MIMIR_B200_ELT_LEAKY_RELU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_ELU: unary_kernel<MIMIR_B200_ELT_ELU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_SOFTPLUS: unary_kernel<MIMIR_B200_ELT_SOFTPLUS><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_MISH: unary_kernel<MIMIR_B200_ELT_MISH><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_HARD_SIGMOID: unary_kernel<MIMIR_B200_ELT_HARD_SIGMOID><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
+    case MIMIR_B200_ELT_HARD_SWISH: unary_kernel<MIMIR_B200_ELT_HARD_SWISH><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
     default: return fail(MIMIR_B200_E_INVALID, "eltwise: unknown op %d", op);
   }
   MB_CUDA(cudaGetLastError());
@@ -304,7 +285,7 @@ int launch_embedding(const float* ids_f32, const int32_t* ids_i32, const float* 
   if (n_ids <= 0) return MIMIR_B200_OK;
   if ((ids_f32 == nullptr) == (ids_i32 == nullptr)) return fail(MIMIR_B200_E_INVALID, "embedding: give exactly one id array");
   const int threads = 256;
-  MB_TRY(launch_pdl(embedding_kernel, dim3(grid_for(n_ids * 32, threads)), dim3(threads), 0, st, 1, ids_f32, ids_i32, table, y, n_ids, vocab, dim, padding_idx));
+  embedding_kernel<<<grid_for(n_ids * 32, threads), threads, 0, st>>>(ids_f32, ids_i32, table, y, n_ids, vocab, dim, padding_idx);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -317,12 +298,12 @@ int launch_upsample_nearest(const float* x, float* y, int batch, int ch, int in_
   const long long total = planes * in_h * sh * in_w * sw;
   if (sh == 2 && sw == 2 && (in_w & 1) == 0 && ((reinterpret_cast<uintptr_t>(x) & 7) | (reinterpret_cast<uintptr_t>(y) & 15)) == 0) {
     const long long items = planes * in_h * (in_w >> 1);
-    MB_TRY(launch_pdl(upsample_nearest_2x2_kernel, dim3(grid_for(items, 256)), dim3(256), 0, st, 1, x, y, planes * in_h, in_w));
+    upsample_nearest_2x2_kernel<<<grid_for(items, 256), 256, 0, st>>>(x, y, planes * in_h, in_w);
     MB_CUDA(cudaGetLastError());
     count_launch();
     return MIMIR_B200_OK;
   }
-  MB_TRY(launch_pdl(upsample_nearest_kernel, dim3(grid_for(total, 256)), dim3(256), 0, st, 1, x, y, planes, in_h, in_w, sh, sw));
+  upsample_nearest_kernel<<<grid_for(total, 256), 256, 0, st>>>(x, y, planes, in_h, in_w, sh, sw);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -345,7 +326,7 @@ int launch_permute(const float* x, float* y, int batch, int nd, const int* shape
     d.total *= shape[i];
   }
   if (seen != (1u << nd) - 1) return fail(MIMIR_B200_E_INVALID, "Permute: dims is not a permutation");
-  MB_TRY(launch_pdl(permute_kernel, dim3(grid_for(d.total * batch, 256)), dim3(256), 0, st, 1, x, y, d, batch));
+  permute_kernel<<<grid_for(d.total * batch, 256), 256, 0, st>>>(x, y, d, batch);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -353,7 +334,7 @@ int launch_permute(const float* x, float* y, int batch, int nd, const int* shape
 
 int launch_token_mean_pool(const float* x, float* y, int batch, int seq, int dim, cudaStream_t st) {
   if (seq <= 0 || dim <= 0) return fail(MIMIR_B200_E_INVALID, "TokenMeanPool: seq_len and embed_dim must be set");
-  MB_TRY(launch_pdl(token_mean_pool_kernel, dim3(grid_for(static_cast<long long>(batch) * dim, 128)), dim3(128), 0, st, 1, x, y, batch, seq, dim));
+  token_mean_pool_kernel<<<grid_for(static_cast<long long>(batch) * dim, 128), 128, 0, st>>>(x, y, batch, seq, dim);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -361,7 +342,7 @@ int launch_token_mean_pool(const float* x, float* y, int batch, int seq, int dim
 
 int launch_global_avgpool(const float* x, float* y, int batch, int ch, int hw, cudaStream_t st) {
   const long long planes = static_cast<long long>(batch) * ch;
-  MB_TRY(launch_pdl(global_avgpool_kernel, dim3(grid_for(planes * 32, 256)), dim3(256), 0, st, 1, x, y, planes, hw));
+  global_avgpool_kernel<<<grid_for(planes * 32, 256), 256, 0, st>>>(x, y, planes, hw);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -378,8 +359,8 @@ int launch_argmax_rows(const float* x, int32_t* ids, int64_t rows, int n, cudaSt
 int launch_copy_strided(const float* src, float* dst, int batch, int64_t n, int64_t total, int64_t off, cudaStream_t st,
                         int64_t src_stride) {
   if (batch <= 0 || n <= 0) return MIMIR_B200_OK;
-  MB_TRY(launch_pdl(copy_strided_kernel, dim3(grid_for(static_cast<long long>(batch) * n, 256)), dim3(256), 0, st, 1, src, dst, batch, n, total, off,
-                                                                                        src_stride > 0 ? src_stride : n));
+  copy_strided_kernel<<<grid_for(static_cast<long long>(batch) * n, 256), 256, 0, st>>>(src, dst, batch, n, total, off,
+                                                                                        src_stride > 0 ? src_stride : n);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
@@ -387,7 +368,7 @@ int launch_copy_strided(const float* src, float* dst, int batch, int64_t n, int6
 
 int launch_broadcast_rows(const float* src, float* dst, int batch, int64_t n, cudaStream_t st) {
   if (batch <= 0 || n <= 0) return MIMIR_B200_OK;
-  MB_TRY(launch_pdl(copy_strided_kernel, dim3(grid_for(static_cast<long long>(batch) * n, 256)), dim3(256), 0, st, 1, src, dst, batch, n, n, 0, 0));
+  copy_strided_kernel<<<grid_for(static_cast<long long>(batch) * n, 256), 256, 0, st>>>(src, dst, batch, n, n, 0, 0);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

@@ -176,8 +176,6 @@ template <int MT, int WR, int BF16>
 __global__ void __launch_bounds__(SK_THREADS, 1)
 skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any, float* __restrict__ part, int m, int k, int n,
                      int kslices, int items) {
-  pdl_launch_dependents();
-  pdl_wait();
   constexpr int N = MT * WR;
   constexpr int STEP = BF16 ? 2 * SK_STEP : SK_STEP, STEPS = SK_SLICE / STEP;  // k of a warp step, steps per item
   constexpr int EB = BF16 ? 2 : 4;                                          // bytes of a weight
@@ -300,8 +298,6 @@ skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any
 // streaming kernel launched with that many CTAs (one partial per CTA that touched the tile); grid == 0: one partial per K slice.
 __global__ void skinny_finish_kernel(const float* __restrict__ part, const float* __restrict__ bias, const float* __restrict__ residual,
                                      float* __restrict__ y, int m, int n, int kslices, int act, int grid, int items, int tile_cols) {
-  pdl_launch_dependents();
-  pdl_wait();
   const long long total = static_cast<long long>(m) * n;
   const ItemSplit split(grid > 0 ? items : 1, grid > 0 ? grid : 1);
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -351,8 +347,8 @@ int launch_partial(const float* x, const float* w, const uint16_t* w_bf16, float
     }));
     const int items = tiles * kslices;
     const int grid = items < ctx().sm_count ? items : ctx().sm_count;
-    if (bf16) MB_TRY(launch_pdl(skinny_stream_kernel<MT, WR, 1>, dim3(grid), dim3(SK_THREADS), SMEM, st, 1, x, w_bf16, scratch, m, k, n, kslices, items));
-    else MB_TRY(launch_pdl(skinny_stream_kernel<MT, WR, 0>, dim3(grid), dim3(SK_THREADS), SMEM, st, 1, x, w, scratch, m, k, n, kslices, items));
+    if (bf16) skinny_stream_kernel<MT, WR, 1><<<grid, SK_THREADS, SMEM, st>>>(x, w_bf16, scratch, m, k, n, kslices, items);
+    else skinny_stream_kernel<MT, WR, 0><<<grid, SK_THREADS, SMEM, st>>>(x, w, scratch, m, k, n, kslices, items);
     *stream_grid = grid;
     *stream_items = items;
   } else {
@@ -384,8 +380,8 @@ int launch_skinny_linear(const float* x, const float* w, const float* bias, floa
   const long long total = static_cast<long long>(m) * n;
   int fb = static_cast<int>((total + 255) / 256);
   if (fb > ctx().sm_count * 8) fb = ctx().sm_count * 8;
-  MB_TRY(launch_pdl(skinny_finish_kernel, dim3(fb), dim3(256), 0, st, 1, scratch, bias, residual, y, m, n, (k + SK_SLICE - 1) / SK_SLICE, activation, sgrid, sitems,
-                                           tile_cols));
+  skinny_finish_kernel<<<fb, 256, 0, st>>>(scratch, bias, residual, y, m, n, (k + SK_SLICE - 1) / SK_SLICE, activation, sgrid, sitems,
+                                           tile_cols);
   MB_CUDA(cudaGetLastError());
   count_launch(2);
   return MIMIR_B200_OK;
