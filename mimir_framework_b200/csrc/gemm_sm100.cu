@@ -1067,9 +1067,9 @@ double big_tile_cycles(const GemmArgs& g) {
   const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
   const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
   const double k = g.conv_ks > 0 ? static_cast<double>(g.k) : static_cast<double>(round_up(g.k, 64));
-  const double mma = k / UMMA_K * products * 128.0, load = k * 2.0 * (g.a_planes * BM + g.w_planes * BN) / 40.0;
+  const double mma = k / UMMA_K * products * 128.0, load = k * 2.0 * (g.a_planes * BM + g.w_planes * BN) / 51.6;
   const double tile = (mma > load ? mma : load);
-  return 6000.0 + waves * (tile > 12000.0 ? tile : 12000.0) + (waves > 0 && tile > 12000.0 ? 12000.0 : 0.0);
+  return 15100.0 + waves * (tile > 12000.0 ? tile : 12000.0);  // (a tile's epilogue takes about 12 000 cycles beside the next main loop)
 }
 }  // namespace
 

@@ -30,12 +30,16 @@ constexpr int SG_M = 128;            // weight rows of a tile
 constexpr int SG_MAX_BN = 128;
 constexpr int SG_MAX_STAGES = 8;
 constexpr int SG_RING_LIMIT = 212992;  // 208 KB of operand stages; the partial tiles reuse them
+constexpr int SG_RING_TWO = 106496;    // 104 KB: two CTAs to an SM
+constexpr int SG_MAX_SPLITS = 16;      // (above eight: the non-portable cluster size)
 
-// Cost model (SM cycles), fitted to a sweep of shapes on B200: see plan_split.
-constexpr double SG_FIXED = 6000.0;        // launch, barriers, first loads, drain
-constexpr double SG_TAIL_PER_COL = 15.0;   // accumulators -> shared memory -> output, per column of the tile
-constexpr double SG_SPLIT = 1500.0, SG_SPLIT_PER_COL = 15.0;  // cluster barriers and the partial tiles through distributed shared memory
-constexpr double SG_LOAD_ALL = 40.0, SG_LOAD_MAX = 70.0;      // operand bytes per cycle an SM gets with all / few SMs loading
+// Cost model (SM cycles): constants fitted to 20 shapes x 30 (width, split) pairs on B200, cold L2 (K = 256 ... 32768, 24 ... 5120 rows);
+// over those the chosen launch is within 1 % of the best one in the geometric mean.
+constexpr double SG_PER_BLOCK = 175.0;     // issue of a k-block beyond its MMAs
+constexpr double SG_FIXED = 10600.0;       // launch, barriers, first loads, drain
+constexpr double SG_TAIL_PER_COL = 70.0;   // accumulators -> shared memory -> output, per column of the tile
+constexpr double SG_SPLIT = 970.0, SG_SPLIT_PER_COL = 30.0;  // cluster barriers and the partial tiles through distributed shared memory
+constexpr double SG_LOAD_ALL = 51.6, SG_LOAD_MAX = 68.8;     // operand bytes per cycle an SM gets with all / few SMs loading
 
 constexpr float SHRINK_PER_MMA = 3.1e-8f;
 
@@ -72,7 +76,7 @@ __device__ __forceinline__ float split_weight(const SplitGemmParams& p, int s) {
 }
 
 template <int BK, int AP, int WP>  // AP, WP: operand planes of the activations and the weights
-__global__ void __launch_bounds__(SG_THREADS, 1)
+__global__ void __launch_bounds__(SG_THREADS, 2)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const SplitGemmParams p) {
   constexpr int SWZ = BK * 2;
   constexpr int W_TILE = SG_M * BK * 2;
@@ -324,16 +328,21 @@ SplitPlan plan_split(const GemmArgs& g, int bk, int kblocks) {
     if (bn > 16 && bn >= g.m + 32) break;
     const long long tiles = static_cast<long long>(tiles_o) * ((g.m + bn - 1) / bn);
     const int stage = (g.w_planes * SG_M + g.a_planes * bn) * bk * 2;
-    for (int splits = 1; splits <= 8; splits *= 2) {
-      if (bn % splits != 0 || splits > kblocks) break;
+    for (int splits = 1; splits <= SG_MAX_SPLITS; splits *= 2) {
+      // (clusters of sixteen: one GPC each, and not every GPC has sixteen SMs free - eight of them took 57 us where sixteen-SM
+      // work in clusters of eight took 46)
+      if (bn % splits != 0 || splits > kblocks || (splits > 8 && tiles > 4)) break;
       const long long ctas = tiles * splits;
-      const long long waves = (ctas + sms - 1) / sms;
+      // CTAs that share an SM overlap one's loads and stores with the other's MMAs: whole rounds of two per SM
+      const bool two = ctas > sms && 2 * stage <= SG_RING_TWO && bn * (SG_M + 1) * 4 <= SG_RING_TWO;
+      const long long rounds = two ? (ctas + 2 * sms - 1) / (2 * sms) : (ctas + sms - 1) / sms;
       const int kb = (kblocks + splits - 1) / splits;
-      const double mma = static_cast<double>(kb) * (bk / 16) * products * (bn > 92 ? bn * 0.5 : 46.0);
+      const double share = two ? static_cast<double>(ctas < 2 * sms ? (ctas + sms - 1) / sms : 2) : 1.0;
+      const double mma = share * kb * ((bk / 16) * products * (bn > 92 ? bn * 0.5 : 46.0) + SG_PER_BLOCK);
       const double busy = static_cast<double>(ctas < sms ? ctas : sms) / sms;
-      const double load = static_cast<double>(kb) * stage / (SG_LOAD_MAX - (SG_LOAD_MAX - SG_LOAD_ALL) * busy);
+      const double load = share * kb * stage / (SG_LOAD_MAX - (SG_LOAD_MAX - SG_LOAD_ALL) * busy);
       const double tail = SG_FIXED + bn * SG_TAIL_PER_COL + (splits > 1 ? SG_SPLIT + bn * SG_SPLIT_PER_COL : 0.0);
-      const double t = static_cast<double>(waves) * ((mma > load ? mma : load) + tail);
+      const double t = static_cast<double>(rounds) * ((mma > load ? mma : load) + tail);
       if (t < best.cycles) { best.bn = bn; best.splits = splits; best.cycles = t; }
     }
   }
@@ -363,7 +372,9 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
   p.err_word = ctx().dev_error_word;
   p.stage_bytes = (WP * SG_M + AP * p.bn) * BK * 2;
   const int per_split = (p.kblocks + p.splits - 1) / p.splits;
-  p.stages = SG_RING_LIMIT / p.stage_bytes;
+  const long long ctas = static_cast<long long>(p.tiles_o) * ((g.m + p.bn - 1) / p.bn) * p.splits;
+  const bool two = ctas > ctx().sm_count && 2 * p.stage_bytes <= SG_RING_TWO && p.bn * (SG_M + 1) * 4 <= SG_RING_TWO;
+  p.stages = (two ? SG_RING_TWO : SG_RING_LIMIT) / p.stage_bytes;
   if (p.stages > SG_MAX_STAGES) p.stages = SG_MAX_STAGES;
   if (p.stages > per_split) p.stages = per_split;
   const int staging = p.bn * (SG_M + 1) * 4, ring = p.stages * p.stage_bytes;
@@ -371,9 +382,9 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
   static PerDeviceOnce attr_once;
   MB_TRY(attr_once.run([&]() -> int {
     MB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BK, AP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_RING_LIMIT + 1024));
+    MB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BK, AP, WP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return MIMIR_B200_OK;
   }));
-  const long long ctas = static_cast<long long>(p.tiles_o) * ((g.m + p.bn - 1) / p.bn) * p.splits;
   GemmProfile prof(st);
   MB_TRY(prof.begin());
   MB_TRY(launch_pdl(gemm_split_kernel<BK, AP, WP>, dim3(static_cast<unsigned>(ctas)), dim3(SG_THREADS), static_cast<size_t>(smem), st, p.splits, map_a, map_w, p));
@@ -392,7 +403,7 @@ bool gemm_split_wanted(const GemmArgs& g, int bk, double other_cycles, int* bn, 
   int fb = 0, fs = 0;
   if (e && sscanf(e, "%d,%d", &fb, &fs) == 2) {
     *bn = fb; *splits = fs;
-    return fb >= 16 && fb <= SG_MAX_BN && fb % 16 == 0 && fs >= 1 && fs <= 8 && fb % fs == 0 && fs <= kblocks;
+    return fb >= 16 && fb <= SG_MAX_BN && fb % 16 == 0 && fs >= 1 && fs <= SG_MAX_SPLITS && fb % fs == 0 && fs <= kblocks;
   }
   const SplitPlan plan = plan_split(g, bk, kblocks);
   *bn = plan.bn; *splits = plan.splits;
