@@ -196,7 +196,7 @@ static int skinny_linear(const float* x, const float* w, const uint16_t* w_bf16,
     return launch_skinny_cluster(a, st);
   }
   if (pre.on) return fail(MIMIR_B200_E_INVALID, "linear: a folded LayerNorm needs the cluster kernel");
-  return launch_skinny_linear(x, w, bias, y, rows, k, n, act, scratch, scratch_bytes, st, residual, w_bf16);
+  return launch_skinny_linear(x, w, bias, y, rows, k, n, act, scratch, scratch_bytes, st, residual, w_bf16, w_ready);
 }
 
 size_t linear_ws_bytes(int rows, int in_f, int out_f, int precision, bool a_presplit) {

@@ -217,7 +217,7 @@ int launch_wait_timeout_selftest(unsigned long long limit_ns, cudaStream_t st);
 // fp32 weight-streaming kernel for very small m (<= 16 rows): y[m,n] = x[m,k] · w[n,k]ᵀ + bias.
 int launch_skinny_linear(const float* x, const float* w, const float* bias, float* y, int m, int k, int n,
                          int activation, float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual = nullptr,
-                         const uint16_t* w_bf16 = nullptr);
+                         const uint16_t* w_bf16 = nullptr, bool w_ready = false);
 size_t skinny_scratch_bytes(int m, int k, int n);
 // skinny_cluster.cu: the same for weight matrices that fit one wave of CTAs; one launch, no scratch.  ln: x is normalised row by
 // row (mean / variance over k) with gamma and beta before the product.
@@ -238,8 +238,15 @@ int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st);
 // pointwise.cu ---------------------------------------------------------------------------------
 int launch_eltwise(int op, const float* a, const float* b, float* y, int batch, int64_t n, int64_t nb,
                    cudaStream_t st, float alpha = 0.0f);
+// Up to two vectors added to the gathered rows: element i of a sample gets p[k][sample * stride[k] + i % n[k]].
+struct EmbeddingAdds {
+  int count = 0;
+  const float* p[2] = {nullptr, nullptr};
+  long long n[2] = {1, 1}, stride[2] = {0, 0};
+  long long ids_ps = 1;  // ids per sample
+};
 int launch_embedding(const float* ids_f32, const int32_t* ids_i32, const float* table, float* y, int64_t n_ids,
-                     int vocab, int dim, int padding_idx, cudaStream_t st);
+                     int vocab, int dim, int padding_idx, cudaStream_t st, const EmbeddingAdds& adds = EmbeddingAdds());
 int launch_upsample_nearest(const float* x, float* y, int batch, int ch, int in_h, int in_w, int sh, int sw,
                             cudaStream_t st);
 int launch_permute(const float* x, float* y, int batch, int nd, const int* shape, const int* dims, cudaStream_t st);

@@ -719,6 +719,8 @@ namespace {
 // One thread per 8 consecutive K elements of one row; the padded tail kp > k is written as zero.
 __global__ void split_rows_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int k,
                                   int kp, int planes, int f16, float scale) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int chunks = kp >> 3;
   const long long total = rows * chunks;
   const long long plane_stride = rows * static_cast<long long>(kp);
@@ -994,7 +996,7 @@ int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int 
   long long blocks = (total + threads - 1) / threads;
   const long long cap = static_cast<long long>(ctx().sm_count) * 16;
   if (blocks > cap) blocks = cap;
-  split_rows_kernel<<<static_cast<int>(blocks), threads, 0, st>>>(src, dst, rows, k, kp, planes, plane_format() == PLANES_F16, scale);
+  MB_TRY(launch_pdl(split_rows_kernel, dim3(static_cast<int>(blocks)), dim3(threads), 0, st, 1, src, dst, rows, k, kp, planes, plane_format() == PLANES_F16, scale));
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

@@ -133,6 +133,7 @@ struct LayerRT {
   bool read_split = false;            // Linear reads the producer's planes
   int res_v = -1;                     // residual tensor folded in from a following Add
   int pre_norm = -1;                  // Conv2d: index of the GroupNorm layer applied while its operand planes are laid out
+  std::vector<int> add_v;             // Embedding: tensors of the Adds folded into it (graph inputs), in layer order
   int pre_ln = -1;                    // a token-wise LayerNorm folded into this layer (index), see fusion 1f
   bool in_up = false;                 // Conv2d: in_v[0] is the INPUT of a 2 x 2 nearest upsample that the layout pass applies
   int gn_emit_for = -1;               // Conv2d: index of the GroupNorm layer whose statistics this layer's GEMM epilogue emits
@@ -166,6 +167,7 @@ struct TensorV {
   std::vector<int> consumers;
   int alias_of = -1;
   bool broadcast_input = false;
+  bool one_copy = false;  // broadcast input whose only readers index one copy of it: not repeated per sample
   bool want_f32 = true, want_split = false;
   int64_t split_rows_ps = 0;
   int split_k = 0;
@@ -794,7 +796,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     LayerRT& L = m->layers[li];
     L.in_v.clear();
     L.out_v = -1;
-    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false;
+    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false; L.add_v.clear();
     L.ws_off = 0; L.ws_bytes = 0;
     std::vector<std::string> names = L.inputs;
     if (names.empty()) names.push_back("x");
@@ -845,6 +847,45 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     return c;
   };
 
+  // ---- fusion 0: Adds of graph inputs (a broadcast vector per model, as the registry's encoder has two) into the Embedding that
+  //      feeds them: one launch instead of one per Add, and an input that only they read is not repeated for every sample ----
+  for (int li = 0; li < nl; ++li) {
+    LayerRT& E = m->layers[li];
+    if (E.lt != LT::Embedding) continue;
+    while (E.add_v.size() < 2) {
+      const int v = E.out_v;
+      if (m->tensors[v].alias_of >= 0 || v == out_root || total_consumers(v) != 1 || m->tensors[v].consumers.size() != 1) break;
+      const int ai = m->tensors[v].consumers[0];
+      LayerRT& A = m->layers[ai];
+      if (A.lt != LT::Add || A.skip || A.in_v.size() != 2 || A.in_v[0] == A.in_v[1]) break;
+      const int o = A.in_v[0] == v ? A.in_v[1] : A.in_v[0];
+      const TensorV& ot = m->tensors[o];
+      if (m->tensors[root_of(m->tensors, o)].producer != -1 || ot.n > m->tensors[v].n || m->tensors[v].n % ot.n != 0) break;
+      E.add_v.push_back(o);
+      E.out_v = A.out_v;
+      m->tensors[A.out_v].producer = li;
+      for (int& c : m->tensors[o].consumers)
+        if (c == ai) c = li;
+      m->tensors[v].consumers.clear();
+      m->tensors[v].want_f32 = false;
+      m->tensors[v].producer = -2;  // dead
+      A.skip = true;
+    }
+  }
+  for (size_t v = 0; v < m->tensors.size(); ++v) {
+    TensorV& t = m->tensors[v];
+    if (!t.broadcast_input || static_cast<int>(v) == out_root) continue;
+    bool only = true;
+    for (size_t a = 0; a < m->tensors.size(); ++a) {
+      if (root_of(m->tensors, static_cast<int>(a)) != static_cast<int>(v)) continue;
+      for (int c : m->tensors[a].consumers) {
+        const LayerRT& C = m->layers[c];
+        only = only && (C.lt == LT::Alias || (C.lt == LT::Embedding && C.in_v[0] != static_cast<int>(a) &&
+                                              std::find(C.add_v.begin(), C.add_v.end(), static_cast<int>(a)) != C.add_v.end()));
+      }
+    }
+    t.one_copy = only;
+  }
   // ---- fusion 1: activation into the producing GEMM / GroupNorm ---------------------------------
   for (int li = 0; li < nl; ++li) {
     LayerRT& A = m->layers[li];
@@ -1351,10 +1392,19 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
                            m->tensors[a].n, m->tensors[b].n, st);
         break;
       }
-      case LT::Embedding:
+      case LT::Embedding: {
+        EmbeddingAdds adds;
+        adds.ids_ps = m->tensors[L.in_v[0]].n;
+        for (int v : L.add_v) {
+          const TensorV& rt = m->tensors[root_of(m->tensors, v)];
+          adds.p[adds.count] = f32p(v);
+          adds.n[adds.count] = m->tensors[v].n;
+          adds.stride[adds.count++] = rt.one_copy ? 0 : m->tensors[v].n;
+        }
         s = launch_embedding(f32p(L.in_v[0]), nullptr, L.w_f32, f32p(L.out_v), static_cast<int64_t>(batch) * m->tensors[L.in_v[0]].n,
-                             std::max(1, d.vocab_size), std::max(1, d.embed_dim), d.padding_idx, st);
+                             std::max(1, d.vocab_size), std::max(1, d.embed_dim), d.padding_idx, st, adds);
         break;
+      }
       case LT::UpsampleNearest:
         s = launch_upsample_nearest(f32p(L.in_v[0]), f32p(L.out_v), batch, L.ch, L.h, L.w, L.oh / L.h, L.ow / L.w, st);
         break;
@@ -1778,7 +1828,9 @@ int mimir_b200_model_forward_device(MimirB200ModelHandle m, const MimirNamedInpu
     b.in_ptr.assign(m->tensors.size(), nullptr);
     for (int i = 0; i < n_inputs; ++i) {
       const TensorV& t = m->tensors[vs[i]];
-      if (t.broadcast_input) {
+      if (t.broadcast_input && t.one_copy) {
+        b.in_ptr[vs[i]] = static_cast<const float*>(inputs[i].data);
+      } else if (t.broadcast_input) {
         // staged again for every micro-batch: the planner may hand the slot to a later tensor once
         // the input's last consumer has run
         float* slot = reinterpret_cast<float*>(m->arena + t.off_f32);
@@ -1850,7 +1902,7 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
       if (t.broadcast_input) {
         // every micro-batch: the slot may have been reused after the input's last consumer
         MB_TRY(copy_to_device(slot, inputs[i].data, static_cast<size_t>(t.n) * 4, m->s_h2d));
-        if (micro > 1) MB_TRY(launch_broadcast_rows(slot, slot + t.n, micro - 1, t.n, m->s_h2d));
+        if (micro > 1 && !t.one_copy) MB_TRY(launch_broadcast_rows(slot, slot + t.n, micro - 1, t.n, m->s_h2d));
       } else {
         const float* src = static_cast<const float*>(inputs[i].data) + static_cast<size_t>(c) * micro * t.n;
         MB_TRY(copy_to_device(slot, src, static_cast<size_t>(t.n) * micro * 4, m->s_h2d));

@@ -3,7 +3,10 @@
 // A kernel launched through launch_pdl may start while the kernel before it in the stream still runs: it must execute pdl_wait()
 // before it touches anything an earlier kernel writes, and before it writes anything an earlier kernel reads.  pdl_wait()
 // returns when every kernel the launch depends on has completed and its writes are visible; without a programmatic edge
-// (first kernel of a stream, after a copy) it returns at once.  pdl_launch_dependents() lets the next such kernel start.
+// (first kernel of a stream, after a copy) it returns at once.  pdl_launch_dependents() lets the next such kernel start: called
+// early only by short kernels that leave room on the SMs.  With it at the start of the large ones too (tensor-core tiles, attention,
+// row sweeps, layout passes) the waiting CTAs took registers and shared memory from the running ones and cost more than the launch
+// latency they hid (UNet 5.27 -> 5.46 ms, decoder with one prompt 1.66 -> 1.73 ms).
 #pragma once
 
 #include <cuda_runtime.h>

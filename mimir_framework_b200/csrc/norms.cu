@@ -18,6 +18,7 @@
 #include <utility>
 
 #include "common.h"
+#include "launch.cuh"
 #include "planes.cuh"
 #include "sm100_ptx.cuh"
 
@@ -741,6 +742,8 @@ constexpr int CLUSTER_SLICE_MAX = 12288;  // floats of shared memory per CTA (48
 
 __global__ void __launch_bounds__(256) meanvar_cluster_kernel(const float* __restrict__ x, float* __restrict__ y, long long len,
                                                               int slice, float eps, Affine a) {
+  pdl_launch_dependents();
+  pdl_wait();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) float sx[];
@@ -1096,19 +1099,8 @@ int meanvar_dispatch(const float* x, float* y, long long rows, long long len, fl
       MB_CUDA(cudaFuncSetAttribute(meanvar_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CLUSTER_SLICE_MAX * 4));
       return MIMIR_B200_OK;
     }));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(rows * ncl));
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = static_cast<size_t>(slice) * sizeof(float);
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(ncl);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    MB_CUDA(cudaLaunchKernelEx(&cfg, meanvar_cluster_kernel, x, y, len, slice, eps, a));
+    MB_TRY(launch_pdl(meanvar_cluster_kernel, dim3(static_cast<unsigned>(rows * ncl)), dim3(256), static_cast<size_t>(slice) * sizeof(float), st, ncl, x, y,
+                      static_cast<long long>(len), slice, eps, a));
     count_launch();
     return MIMIR_B200_OK;
   }

@@ -7,6 +7,7 @@
 //   permute            : LayerOps::permute_forward (LayerOps.hpp:880-945)
 //   token_mean_pool    : Model.cpp:5571-5589;  global_avgpool : LayerOps.hpp:459-482
 #include "common.h"
+#include "launch.cuh"
 
 namespace mb {
 namespace {
@@ -65,6 +66,8 @@ __device__ __forceinline__ float bin_apply(float u, float w) {
 template <int BOP>
 __global__ void binary_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y,
                               long long batch, long long n, long long nb) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long total = batch * n;
@@ -91,12 +94,16 @@ __global__ void binary_kernel(const float* __restrict__ a, const float* __restri
 
 __global__ void embedding_kernel(const float* __restrict__ ids_f, const int32_t* __restrict__ ids_i,
                                  const float* __restrict__ table, float* __restrict__ y, long long n_ids, int vocab,
-                                 int dim, int padding_idx) {
+                                 int dim, int padding_idx, const EmbeddingAdds adds) {
+  pdl_launch_dependents();
+  pdl_wait();
   // one warp per id row
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  const bool vec = ((dim & 3) == 0) && (((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(y)) & 15) == 0);
+  bool vec = ((dim & 3) == 0) && (((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(y)) & 15) == 0);
+  for (int k = 0; k < adds.count; ++k)
+    vec = vec && ((adds.n[k] | adds.stride[k]) & 3) == 0 && (reinterpret_cast<uintptr_t>(adds.p[k]) & 15) == 0;
   for (long long t = warp; t < n_ids; t += nwarps) {
     long long id;
     if (ids_f != nullptr) id = llround(static_cast<double>(ids_f[t]));  // Model.cpp:5322
@@ -104,11 +111,23 @@ __global__ void embedding_kernel(const float* __restrict__ ids_f, const int32_t*
     const bool zero = (padding_idx >= 0 && id == padding_idx) || id < 0 || id >= vocab;
     float* out = y + t * dim;
     const float* row = table + (zero ? 0 : id) * static_cast<long long>(dim);
+    // the folded Adds (add_forward's `i % small_n` broadcast, LayerOps.hpp:165-190), in the order of the layers
+    const long long smp = adds.count ? t / adds.ids_ps : 0, first = adds.count ? (t - smp * adds.ids_ps) * dim : 0;
     if (vec) {
-      for (int d = lane; d < (dim >> 2); d += 32)
-        reinterpret_cast<float4*>(out)[d] = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(reinterpret_cast<const float4*>(row) + d);
+      for (int d = lane; d < (dim >> 2); d += 32) {
+        float4 v = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(reinterpret_cast<const float4*>(row) + d);
+        for (int k = 0; k < adds.count; ++k) {
+          const float4 q = __ldg(reinterpret_cast<const float4*>(adds.p[k] + smp * adds.stride[k] + (first + 4 * d) % adds.n[k]));
+          v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+        }
+        reinterpret_cast<float4*>(out)[d] = v;
+      }
     } else {
-      for (int d = lane; d < dim; d += 32) out[d] = zero ? 0.0f : __ldg(row + d);
+      for (int d = lane; d < dim; d += 32) {
+        float v = zero ? 0.0f : __ldg(row + d);
+        for (int k = 0; k < adds.count; ++k) v += __ldg(adds.p[k] + smp * adds.stride[k] + (first + d) % adds.n[k]);
+        out[d] = v;
+      }
     }
   }
 }
@@ -251,16 +270,16 @@ int launch_eltwise(int op, const float* a, const float* b, float* y, int batch, 
       if (op == MIMIR_B200_ELT_MULTIPLY && nb != n) return fail(MIMIR_B200_E_INVALID, "Multiply: input sizes must match");
       if (nb != n && nb != 1 && (n % nb) != 0)
         return fail(MIMIR_B200_E_INVALID, "Add: input sizes must match or be broadcastable");
-      if (op == MIMIR_B200_ELT_ADD) binary_kernel<0><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
-      else binary_kernel<1><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
+      if (op == MIMIR_B200_ELT_ADD) MB_TRY(launch_pdl(binary_kernel<0>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
+      else MB_TRY(launch_pdl(binary_kernel<1>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
       break;
     case MIMIR_B200_ELT_SUBTRACT:
     case MIMIR_B200_ELT_DIVIDE:
       if (!b || nb != n)
         return fail(MIMIR_B200_E_INVALID, "%s: size mismatch: %lld vs %lld", op == MIMIR_B200_ELT_SUBTRACT ? "Subtract" : "Divide",
                     static_cast<long long>(n), static_cast<long long>(nb));
-      if (op == MIMIR_B200_ELT_SUBTRACT) binary_kernel<2><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
-      else binary_kernel<3><<<grid, threads, 0, st>>>(a, b, y, batch, n, nb);
+      if (op == MIMIR_B200_ELT_SUBTRACT) MB_TRY(launch_pdl(binary_kernel<2>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
+      else MB_TRY(launch_pdl(binary_kernel<3>, dim3(grid), dim3(threads), 0, st, 1, a, b, y, batch, n, nb));
       break;
     case MIMIR_B200_ELT_GELU: unary_kernel<MIMIR_B200_ELT_GELU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
     case MIMIR_B200_ELT_SILU: unary_kernel<MIMIR_B200_ELT_SILU><<<grid, threads, 0, st>>>(a, y, total, alpha); break;
@@ -281,11 +300,11 @@ int launch_eltwise(int op, const float* a, const float* b, float* y, int batch, 
 }
 
 int launch_embedding(const float* ids_f32, const int32_t* ids_i32, const float* table, float* y, int64_t n_ids, int vocab,
-                     int dim, int padding_idx, cudaStream_t st) {
+                     int dim, int padding_idx, cudaStream_t st, const EmbeddingAdds& adds) {
   if (n_ids <= 0) return MIMIR_B200_OK;
   if ((ids_f32 == nullptr) == (ids_i32 == nullptr)) return fail(MIMIR_B200_E_INVALID, "embedding: give exactly one id array");
   const int threads = 256;
-  embedding_kernel<<<grid_for(n_ids * 32, threads), threads, 0, st>>>(ids_f32, ids_i32, table, y, n_ids, vocab, dim, padding_idx);
+  MB_TRY(launch_pdl(embedding_kernel, dim3(grid_for(n_ids * 32, threads)), dim3(threads), 0, st, 1, ids_f32, ids_i32, table, y, n_ids, vocab, dim, padding_idx, adds));
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

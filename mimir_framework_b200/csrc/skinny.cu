@@ -175,7 +175,7 @@ struct ItemSplit {
 template <int MT, int WR, int BF16>
 __global__ void __launch_bounds__(SK_THREADS, 1)
 skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any, float* __restrict__ part, int m, int k, int n,
-                     int kslices, int items) {
+                     int kslices, int items, int w_ready) {
   constexpr int N = MT * WR;
   constexpr int STEP = BF16 ? 2 * SK_STEP : SK_STEP, STEPS = SK_SLICE / STEP;  // k of a warp step, steps per item
   constexpr int EB = BF16 ? 2 : 4;                                          // bytes of a weight
@@ -194,21 +194,25 @@ skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any
   // Copy group of this CTA's step g (item g / SK_STEPS, step g % SK_STEPS): this warp's WR rows of W, and with the first step
   // of an item every thread's share of that item's x slice.  The groups are issued in order, so (tile, ks, step) of the next
   // group and the address of its first row advance incrementally.
+  // one warp's WR rows of a step into ring slot g % SK_STAGES
+  auto copy_w = [&](int g, int t, int k2, int st) {
+    const int c = k2 * SK_SLICE + st * STEP + lane * (16 / EB);
+    const int o0 = (t * SK_WARPS + warp) * WR;
+    const char* src = w + (static_cast<long long>(o0) * kk + c) * EB;
+    float* dst = ring + (g % SK_STAGES) * (WR * SK_STEP) + lane * 4;
+    const bool col_ok = c < k;
+#pragma unroll
+    for (int jj = 0; jj < WR; ++jj) {
+      const bool ok = col_ok && (o0 + jj < n);
+      cp_async16_zfill(dst + jj * SK_STEP, ok ? src : w, ok);
+      src += kk * EB;
+    }
+  };
   int ig = 0, i_st = 0, i_j = 0;
   int i_tile = my_first / kslices, i_ks = my_first - i_tile * kslices;
-  auto issue = [&]() {
+  auto issue = [&](bool with_w) {
     if (ig < total_steps) {
-      const int c = i_ks * SK_SLICE + i_st * STEP + lane * (16 / EB);
-      const int o0 = (i_tile * SK_WARPS + warp) * WR;
-      const char* src = w + (static_cast<long long>(o0) * kk + c) * EB;
-      float* dst = ring + (ig % SK_STAGES) * (WR * SK_STEP) + lane * 4;
-      const bool col_ok = c < k;
-#pragma unroll
-      for (int jj = 0; jj < WR; ++jj) {
-        const bool ok = col_ok && (o0 + jj < n);
-        cp_async16_zfill(dst + jj * SK_STEP, ok ? src : w, ok);
-        src += kk * EB;
-      }
+      if (with_w) copy_w(ig, i_tile, i_ks, i_st);
       if (i_st == 0) {
         float* xd = xs + (i_j & 1) * (MT * SK_SLICE);
         for (int i = threadIdx.x; i < MT * (SK_SLICE / 4); i += SK_THREADS) {
@@ -228,8 +232,18 @@ skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any
     ++ig;
     cp_async_commit();  // one group per step, empty past the end, so that the wait count stays fixed
   };
+  // the first stages' weights do not depend on the kernel before this one
+  if (!w_ready) pdl_wait();
+  for (int u = 0, t = i_tile, k2 = i_ks, st2 = 0; u < SK_STAGES - 1 && u < total_steps; ++u) {
+    copy_w(u, t, k2, st2);
+    if (++st2 == STEPS) {
+      st2 = 0;
+      if (++k2 == kslices) { k2 = 0; ++t; }
+    }
+  }
+  pdl_wait();
 #pragma unroll
-  for (int i = 0; i < SK_STAGES - 1; ++i) issue();
+  for (int i = 0; i < SK_STAGES - 1; ++i) issue(false);
 
   float acc[N];
 #pragma unroll
@@ -245,9 +259,9 @@ skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any
         // (the next group may overwrite the x buffer of item j - 1: issued after the barrier)
         cp_async_wait<SK_STAGES - 2>();
         __syncthreads();
-        issue();
+        issue(true);
       } else {
-        issue();
+        issue(true);
         cp_async_wait<SK_STAGES - 1>();
       }
       const float* src = ring + (g % SK_STAGES) * (WR * SK_STEP) + lane * 4;
@@ -292,12 +306,15 @@ skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any
     if (++ks == kslices) { ks = 0; ++tile; }
   }
   cp_async_wait<0>();
+  pdl_launch_dependents();
 }
 
 // y = sum of a tile's partials in K order (+ bias, activation, folded residual).  grid > 0: the partials come from the
 // streaming kernel launched with that many CTAs (one partial per CTA that touched the tile); grid == 0: one partial per K slice.
 __global__ void skinny_finish_kernel(const float* __restrict__ part, const float* __restrict__ bias, const float* __restrict__ residual,
                                      float* __restrict__ y, int m, int n, int kslices, int act, int grid, int items, int tile_cols) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long total = static_cast<long long>(m) * n;
   const ItemSplit split(grid > 0 ? items : 1, grid > 0 ? grid : 1);
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -328,7 +345,7 @@ __global__ void skinny_finish_kernel(const float* __restrict__ part, const float
 }
 
 template <int MT, int WR>
-int launch_partial(const float* x, const float* w, const uint16_t* w_bf16, float* scratch, int m, int k, int n, cudaStream_t st, int* stream_grid, int* stream_items,
+int launch_partial(const float* x, const float* w, const uint16_t* w_bf16, bool w_ready, float* scratch, int m, int k, int n, cudaStream_t st, int* stream_grid, int* stream_items,
                    int* tile_cols) {
   const int tiles = (n + SK_WARPS * WR - 1) / (SK_WARPS * WR), kslices = (k + SK_SLICE - 1) / SK_SLICE;
   const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0 && (k & 3) == 0;
@@ -347,8 +364,8 @@ int launch_partial(const float* x, const float* w, const uint16_t* w_bf16, float
     }));
     const int items = tiles * kslices;
     const int grid = items < ctx().sm_count ? items : ctx().sm_count;
-    if (bf16) skinny_stream_kernel<MT, WR, 1><<<grid, SK_THREADS, SMEM, st>>>(x, w_bf16, scratch, m, k, n, kslices, items);
-    else skinny_stream_kernel<MT, WR, 0><<<grid, SK_THREADS, SMEM, st>>>(x, w, scratch, m, k, n, kslices, items);
+    if (bf16) MB_TRY(launch_pdl(skinny_stream_kernel<MT, WR, 1>, dim3(grid), dim3(SK_THREADS), SMEM, st, 1, x, w_bf16, scratch, m, k, n, kslices, items, w_ready ? 1 : 0));
+    else MB_TRY(launch_pdl(skinny_stream_kernel<MT, WR, 0>, dim3(grid), dim3(SK_THREADS), SMEM, st, 1, x, w, scratch, m, k, n, kslices, items, w_ready ? 1 : 0));
     *stream_grid = grid;
     *stream_items = items;
   } else {
@@ -368,20 +385,20 @@ size_t skinny_scratch_bytes(int m, int k, int n) {
 }
 
 int launch_skinny_linear(const float* x, const float* w, const float* bias, float* y, int m, int k, int n, int activation,
-                         float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual, const uint16_t* w_bf16) {
+                         float* scratch, size_t scratch_bytes, cudaStream_t st, const float* residual, const uint16_t* w_bf16, bool w_ready) {
   if (m <= 0 || m > 16 || k <= 0 || n <= 0) return fail(MIMIR_B200_E_INVALID, "skinny linear: m must be in 1..16");
   if (scratch == nullptr || scratch_bytes < skinny_scratch_bytes(m, k, n))
     return fail(MIMIR_B200_E_INVALID, "skinny linear: scratch too small");
   if ((k + SK_SLICE - 1) / SK_SLICE > 65535) return fail(MIMIR_B200_E_UNSUPPORTED, "skinny linear: in_features %d too large", k);
   int sgrid = 0, sitems = 0, tile_cols = 0;
-  if (m <= 4) MB_TRY((launch_partial<4, 8>(x, w, w_bf16, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
-  else if (m <= 8) MB_TRY((launch_partial<8, 8>(x, w, w_bf16, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
-  else MB_TRY((launch_partial<16, 4>(x, w, w_bf16, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
+  if (m <= 4) MB_TRY((launch_partial<4, 8>(x, w, w_bf16, w_ready, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
+  else if (m <= 8) MB_TRY((launch_partial<8, 8>(x, w, w_bf16, w_ready, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
+  else MB_TRY((launch_partial<16, 4>(x, w, w_bf16, w_ready, scratch, m, k, n, st, &sgrid, &sitems, &tile_cols)));
   const long long total = static_cast<long long>(m) * n;
   int fb = static_cast<int>((total + 255) / 256);
   if (fb > ctx().sm_count * 8) fb = ctx().sm_count * 8;
-  skinny_finish_kernel<<<fb, 256, 0, st>>>(scratch, bias, residual, y, m, n, (k + SK_SLICE - 1) / SK_SLICE, activation, sgrid, sitems,
-                                           tile_cols);
+  MB_TRY(launch_pdl(skinny_finish_kernel, dim3(fb), dim3(256), 0, st, 1, scratch, bias, residual, y, m, n, (k + SK_SLICE - 1) / SK_SLICE, activation, sgrid, sitems,
+                                           tile_cols));
   MB_CUDA(cudaGetLastError());
   count_launch(2);
   return MIMIR_B200_OK;
