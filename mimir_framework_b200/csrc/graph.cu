@@ -1012,7 +1012,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
   //      the consumer normalises while it stages its rows (skinny_cluster.cu) ----
   for (int li = 0; li < nl; ++li) {
     LayerRT& P = m->layers[li];
-    if (P.lt != LT::LayerNorm || P.skip || P.norm_n % 4 != 0) continue;
+    if (P.lt != LT::LayerNorm || P.skip || P.d.in_features <= 0 || P.norm_n % 4 != 0) continue;
     const int pv = P.out_v;
     TensorV& pt = m->tensors[pv];
     if (pt.alias_of >= 0 || pv == out_root || total_consumers(pv) != 1 || pt.consumers.size() != 1) continue;
