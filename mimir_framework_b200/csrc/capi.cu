@@ -156,6 +156,7 @@ int read_error_word(cudaStream_t st) {
   if (w != 0) {
     cudaMemsetAsync(ctx().dev_error_word, 0, sizeof(int), st);
     cudaStreamSynchronize(st);
+    norm_scratch_clear();
     return fail(MIMIR_B200_E_TIMEOUT, "a device-side wait gave up (site %d)", w);
   }
   return MIMIR_B200_OK;

@@ -328,7 +328,9 @@ struct RmsOnePass {
   long long plane_stride;   // elements between the hi and the lo plane
   int planes;
   int f16;                  // the planes hold IEEE half instead of bfloat16
-  unsigned* ticket;         // [0] ticket counter, [1] abort flag
+  unsigned* ticket;         // [0] ticket counter, [1] abort flag, [2] rows finished
+  unsigned* row_done;       // per row: CTAs that have read everything they need
+  int rows;
   unsigned long long* sum_slots;
   unsigned long long* err_slots;
   long long len;
@@ -350,7 +352,7 @@ __device__ __forceinline__ bool slot_wait(const unsigned long long* slot, volati
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
     unsigned spins = 0;
     while (((v = *p) >> 32) == 0) {
-      __nanosleep(64);
+      __nanosleep(32);
       if ((++spins & 0xFF) == 0) {
         if (*abort_flag) return false;
         uint64_t t1;
@@ -383,10 +385,11 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   extern __shared__ __align__(128) float sx[];  // the chunk, zero beyond its end
   __shared__ __align__(8) uint64_t bar;
   __shared__ unsigned s_id;
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_last;
   __shared__ float redf[33];
   __shared__ double red[8];
   const int tid = threadIdx.x;
+  pdl_wait();
   if (tid == 0) {
     s_id = atomicAdd(p.ticket, 1u);
     s_abort = 0;
@@ -475,6 +478,23 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   if (__syncthreads_or(!ok)) {  // a wait gave up: the error word is set, nothing is written
     if (tid == 0) *abort_flag = 1u;
     return;
+  }
+  // The row's last CTA leaves its slots zero for the next launch, the last row the ticket counter: no clearing between launches
+  // (a memset ahead of every launch and the gaps around it took 5 us of a one-prompt decoder's 18 us per norm).
+  if (tid == 0) s_last = atomicAdd(p.row_done + row, 1u) == static_cast<unsigned>(p.chunks) - 1u;
+  __syncthreads();
+  if (s_last) {
+    for (int j = tid; j < p.chunks; j += 256) {
+      p.sum_slots[slot0 + j] = 0ull;
+      p.err_slots[slot0 + j] = 0ull;
+    }
+    if (tid == 0) {
+      p.row_done[row] = 0u;
+      if (atomicAdd(p.ticket + 2, 1u) == static_cast<unsigned>(p.rows) - 1u) {
+        p.ticket[0] = 0u;
+        p.ticket[2] = 0u;
+      }
+    }
   }
   const float rms = sqrtf(static_cast<float>(sd) / static_cast<float>(p.len) + p.eps);
   const float inv_rms = 1.0f / rms;
@@ -1054,13 +1074,18 @@ int norm_scratch(cudaStream_t st, float** out, bool pin = false) {
         if (jt->second.pinned) { ++jt; continue; }
         MB_CUDA(cudaSetDevice(jt->first.first));
         MB_CUDA(cudaDeviceSynchronize());
-        dev_free(jt->second.p, NORM_SCRATCH_BYTES);
+        dev_free(jt->second.p, 2 * NORM_SCRATCH_BYTES);
         jt = g_norm_scratch.erase(jt);
       }
       MB_CUDA(cudaSetDevice(dev));
     }
     NormScratch ns;
-    MB_TRY(dev_alloc(reinterpret_cast<void**>(&ns.p), NORM_SCRATCH_BYTES, "norm_scratch"));
+    MB_TRY(dev_alloc(reinterpret_cast<void**>(&ns.p), 2 * NORM_SCRATCH_BYTES, "norm_scratch"));
+    // the second half belongs to the one-pass RMSNorm, which expects it zero and leaves it zero
+    if (cudaMemset(reinterpret_cast<uint8_t*>(ns.p) + NORM_SCRATCH_BYTES, 0, NORM_SCRATCH_BYTES) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+      dev_free(ns.p, 2 * NORM_SCRATCH_BYTES);
+      return fail(MIMIR_B200_E_CUDA, "norm_scratch: clearing failed");
+    }
     it = g_norm_scratch.emplace(key, ns).first;
   }
   if (pin) it->second.pinned = true;
@@ -1142,8 +1167,17 @@ void norm_scratch_release(cudaStream_t st) {
   if (cudaGetDevice(&dev) != cudaSuccess) return;
   auto it = g_norm_scratch.find(std::make_pair(dev, st));
   if (it == g_norm_scratch.end()) return;
-  dev_free(it->second.p, NORM_SCRATCH_BYTES);
+  dev_free(it->second.p, 2 * NORM_SCRATCH_BYTES);
   g_norm_scratch.erase(it);
+}
+
+void norm_scratch_clear() {
+  std::lock_guard<std::mutex> lk(g_norm_mu);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return;
+  for (auto& kv : g_norm_scratch)
+    if (kv.first.first == dev) cudaMemset(reinterpret_cast<uint8_t*>(kv.second.p) + NORM_SCRATCH_BYTES, 0, NORM_SCRATCH_BYTES);
+  cudaDeviceSynchronize();
 }
 
 int launch_layernorm(const float* x, const float* gamma, const float* beta, float* y, int64_t rows, int64_t n, float eps,
@@ -1259,7 +1293,7 @@ bool rmsnorm_onepass_ok(int batch, int64_t n) {
   }
   const int64_t chunks = (n + CHUNK - 1) / CHUNK;
   if (chunks > static_cast<int64_t>(per_sm) * ctx().sm_count) return false;
-  return static_cast<uint64_t>(batch) * chunks * 16 + 256 <= NORM_SCRATCH_BYTES && static_cast<uint64_t>(batch) * chunks < 0x7fffffffull;
+  return static_cast<uint64_t>(batch) * chunks * 16 + static_cast<uint64_t>(batch) * 4 + 512 <= NORM_SCRATCH_BYTES && static_cast<uint64_t>(batch) * chunks < 0x7fffffffull;
 }
 
 int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y, int batch, int64_t n, float eps,
@@ -1271,17 +1305,19 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
     MB_TRY(norm_scratch(st, &scratch));
     const int chunks = static_cast<int>((n + CHUNK - 1) / CHUNK);
     const size_t slots = static_cast<size_t>(batch) * chunks;
-    MB_CUDA(cudaMemsetAsync(scratch, 0, 256 + slots * 16, st));
     RmsOnePass p{};
     p.x = x; p.gamma = gamma; p.n_gamma = gamma ? n_gamma : 0; p.y = y; p.y_split = y_split; p.plane_stride = plane_stride;
     p.planes = planes;
     p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
-    p.ticket = reinterpret_cast<unsigned*>(scratch);
-    p.sum_slots = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(scratch) + 256);
+    // the one-pass kernel's own half of the scratch: 256 bytes of counters, row counters, slots
+    uint8_t* op = reinterpret_cast<uint8_t*>(scratch) + NORM_SCRATCH_BYTES;
+    p.ticket = reinterpret_cast<unsigned*>(op);
+    p.row_done = reinterpret_cast<unsigned*>(op + 256);
+    p.rows = batch;
+    p.sum_slots = reinterpret_cast<unsigned long long*>(op + 256 + (static_cast<size_t>(batch) * 4 + 255) / 256 * 256);
     p.err_slots = p.sum_slots + slots;
     p.len = n; p.chunks = chunks; p.eps = eps; p.err_word = ctx().dev_error_word;
-    rms_onepass_kernel<<<static_cast<unsigned>(slots), 256, CHUNK * sizeof(float), st>>>(p);
-    MB_CUDA(cudaGetLastError());
+    MB_TRY(launch_pdl(rms_onepass_kernel, dim3(static_cast<unsigned>(slots)), dim3(256), CHUNK * sizeof(float), st, 1, p));
     count_launch();
     return MIMIR_B200_OK;
   }
