@@ -1,0 +1,323 @@
+// conv_gemm.cu — stride-1 "same" convolutions with ks >= 3 on large images, as an implicit GEMM over spatial tiles
+// (the inline Conv2d case, Model.cpp:4897-5089).  Same operands (zero-padded NHWC planes, (tap, channel) weight planes), same
+// products and epilogue as the shifted-GEMM form of gemm_sm100.cu.
+//
+// That form is bound by what an SM can take from L2: a tile of 256 pixels reads its activation block once per tap, nine times for
+// a 3 x 3 kernel (80 bytes per cycle and SM on a 128 -> 128 layer in the two-MMA mode, where about 50 arrive; the tensor pipe
+// was 48 to 54 % busy).  Here a tile is 16 x 16 pixels of one sample, and a K block of 32 channels brings the tile with its rows of halo,
+// 16 x (16 + ks - 1) pixels, ONCE per kernel column: a vertical shift by one row is 16 pixels further into the same
+// shared-memory tile, 16 x 64 bytes, a whole number of swizzle atoms, so the ks taps of a column are the same copy under ks
+// descriptors.  Activation bytes from L2 fall to (16 + ks - 1) / (16 ks) of before (0.375 for 3 x 3).
+//
+//   warp 0     : TMA producer of activation tiles   (ring of A_STAGES, one per (32 channels, kernel column))
+//   warp 1     : MMA issuer: weights are the M side (128 output channels), 256 pixels the N side; two accumulators in TMEM
+//   warps 2..9 : epilogue: 32 x 32 chunks turned around in shared memory so that a lane owns a pixel; NCHW stores
+//   warp 10    : TMA producer of weight tiles       (ring of W_STAGES, one per tap)
+// Every wait is bounded, as in gemm_sm100.cu.
+#include "common.h"
+#include "epilogue.cuh"
+#include "launch.cuh"
+#include "planes.cuh"
+#include "sm100_ptx.cuh"
+#include "tensor_map.h"
+
+#include <cstdlib>
+
+namespace mb {
+namespace {
+
+constexpr int CG_THREADS = 352;
+constexpr int CG_SIDE = 16;                    // a tile is 16 x 16 pixels
+constexpr int CG_N = CG_SIDE * CG_SIDE;
+constexpr int CG_M = 128;                      // output channels of a tile
+constexpr int CG_BK = 32;                      // channels of a K block: 64-byte swizzle rows
+constexpr int CG_W_TILE = CG_M * CG_BK * 2;
+constexpr int CG_EPI = 8 * 32 * 33 * 4;
+constexpr int CG_MAX_RING = 8;
+constexpr int CG_SMEM_MAX = 232448;
+
+struct ConvGemmParams {
+  int batch, oc, h, w, ks, cblocks;            // cblocks = channels / 32
+  int tiles_x, tiles_y, tiles_o, num_tiles;
+  int a_stages, a_stage_bytes, w_stages;
+  const float* residual;
+  float* out;
+  int activation;
+  float acc_scale;
+  int f16;
+  int* err_word;
+};
+
+struct ConvTile { int oc0, n, y0, x0; };
+__device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) {  // output-channel tiles fastest: they share activations in L2
+  ConvTile c;
+  c.oc0 = (t % p.tiles_o) * CG_M;
+  int s = t / p.tiles_o;
+  c.x0 = (s % p.tiles_x) * CG_SIDE;
+  s /= p.tiles_x;
+  c.y0 = (s % p.tiles_y) * CG_SIDE;
+  c.n = s / p.tiles_y;
+  return c;
+}
+
+template <int AP, int WP>
+__global__ void __launch_bounds__(CG_THREADS, 1)
+conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const ConvGemmParams p) {
+  extern __shared__ __align__(1024) uint8_t cg_smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(cg_smem_raw) + 1023) & ~uintptr_t(1023));
+  const int a_plane = p.a_stage_bytes / AP;                                   // halo tile of one plane
+  uint8_t* a_ring = smem;
+  uint8_t* w_ring = smem + p.a_stages * p.a_stage_bytes;
+  float* epi = reinterpret_cast<float*>(w_ring + p.w_stages * WP * CG_W_TILE);
+  __shared__ uint64_t a_full[CG_MAX_RING], a_empty[CG_MAX_RING], w_full[CG_MAX_RING], w_empty[CG_MAX_RING], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.a_stages; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
+    for (int s = 0; s < p.w_stages; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 8); }
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = tmem_slot;
+  pdl_wait();
+
+  if (warp == 0) {
+    const bool one = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = static_cast<int>(blockIdx.x); t < p.num_tiles && ok; t += static_cast<int>(gridDim.x)) {
+      const ConvTile c = conv_tile(p, t);
+      for (int cb = 0; cb < p.cblocks && ok; ++cb)
+        for (int kw = 0; kw < p.ks; ++kw) {
+          if (!mbar_wait_warp(&a_empty[stage], phase ^ 1, &abort_flag, p.err_word, 51)) { ok = false; break; }
+          if (one) {
+            uint8_t* dst = a_ring + stage * p.a_stage_bytes;
+            mbar_expect_tx(&a_full[stage], static_cast<uint32_t>(p.a_stage_bytes));
+            tma_load_5d(dst, &map_a, &a_full[stage], cb * CG_BK, c.x0 + kw, c.y0, c.n, 0);  // (padded coordinates: the halo starts at y0)
+            if (AP == 2) tma_load_5d(dst + a_plane, &map_a, &a_full[stage], cb * CG_BK, c.x0 + kw, c.y0, c.n, 1);
+          }
+          __syncwarp();
+          if (++stage == p.a_stages) { stage = 0; phase ^= 1; }
+        }
+    }
+    for (int s = 0; s < p.a_stages; ++s) {  // drain: no copy may be in flight when the CTA exits
+      if (!mbar_wait_warp(&a_empty[stage], phase ^ 1, &abort_flag, p.err_word, 52)) break;
+      if (++stage == p.a_stages) { stage = 0; phase ^= 1; }
+    }
+  } else if (warp == 10) {
+    const bool one = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = static_cast<int>(blockIdx.x); t < p.num_tiles && ok; t += static_cast<int>(gridDim.x)) {
+      const int oc0 = (t % p.tiles_o) * CG_M;
+      for (int cb = 0; cb < p.cblocks && ok; ++cb)
+        for (int kw = 0; kw < p.ks && ok; ++kw)
+          for (int kh = 0; kh < p.ks; ++kh) {
+            if (!mbar_wait_warp(&w_empty[stage], phase ^ 1, &abort_flag, p.err_word, 53)) { ok = false; break; }
+            if (one) {
+              uint8_t* dst = w_ring + stage * (WP * CG_W_TILE);
+              const int col = ((kh * p.ks + kw) * p.cblocks + cb) * CG_BK;
+              mbar_expect_tx(&w_full[stage], WP * CG_W_TILE);
+              tma_load_3d(dst, &map_w, &w_full[stage], col, oc0, 0);
+              if (WP == 2) tma_load_3d(dst + CG_W_TILE, &map_w, &w_full[stage], col, oc0, 1);
+            }
+            __syncwarp();
+            if (++stage == p.w_stages) { stage = 0; phase ^= 1; }
+          }
+    }
+    for (int s = 0; s < p.w_stages; ++s) {
+      if (!mbar_wait_warp(&w_empty[stage], phase ^ 1, &abort_flag, p.err_word, 54)) break;
+      if (++stage == p.w_stages) { stage = 0; phase ^= 1; }
+    }
+  } else if (warp == 1) {
+    const bool one = elect_one();
+    const uint32_t idesc = make_idesc(CG_M, CG_N, p.f16);
+    int as = 0, ws = 0, acc = 0;
+    uint32_t aph = 0, wph = 0, acc_phase = 0;
+    bool ok = true, w_ready = false;
+    for (int t = static_cast<int>(blockIdx.x); t < p.num_tiles && ok; t += static_cast<int>(gridDim.x)) {
+      if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, &abort_flag, p.err_word, 55)) break;
+      tcgen05_fence_after();
+      const uint32_t d = tmem + static_cast<uint32_t>(acc * CG_N);
+      bool first = true;
+      for (int b = 0; b < p.cblocks * p.ks && ok; ++b) {  // (32 channels, kernel column)
+        if (!mbar_wait_warp(&a_full[as], aph, &abort_flag, p.err_word, 56)) { ok = false; break; }
+        const uint64_t da0 = make_smem_desc(smem_u32(a_ring + as * p.a_stage_bytes), 64);
+        for (int kh = 0; kh < p.ks; ++kh) {
+          if (!__all_sync(0xffffffffu, w_ready) && !mbar_wait_warp(&w_full[ws], wph, &abort_flag, p.err_word, 57)) { ok = false; break; }
+          tcgen05_fence_after();
+          // kh rows further down: 16 pixels x 64 bytes = 1024 = 64 in the descriptor's address field
+          const uint64_t da = da0 + static_cast<uint64_t>(kh * 64), da_lo = da + static_cast<uint64_t>(a_plane >> 4);
+          const uint64_t dw = make_smem_desc(smem_u32(w_ring + ws * (WP * CG_W_TILE)), 64), dw_lo = dw + (CG_W_TILE >> 4);
+          uint64_t* w_done = &w_empty[ws];
+          if (++ws == p.w_stages) { ws = 0; wph ^= 1; }
+          w_ready = mbar_test(&w_full[ws], wph);
+          if (one) {
+#pragma unroll
+            for (int k = 0; k < CG_BK / 16; ++k) {
+              umma_bf16(d, dw + 2 * k, da + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+              if (AP == 2) umma_bf16(d, dw + 2 * k, da_lo + 2 * k, idesc, 1u);
+              if (WP == 2) umma_bf16(d, dw_lo + 2 * k, da + 2 * k, idesc, 1u);
+            }
+            umma_commit(w_done);
+            if (kh + 1 == p.ks) umma_commit(&a_empty[as]);
+          }
+          first = false;
+          __syncwarp();
+        }
+        if (++as == p.a_stages) { as = 0; aph ^= 1; }
+      }
+      if (!ok) break;
+      if (one) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+    }
+  } else {
+    // epilogue: TMEM lane = output channel, column = pixel (16 to a row)
+    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+    float* tbuf = epi + ew * (32 * 33);
+    const long long hw = static_cast<long long>(p.h) * p.w;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = static_cast<int>(blockIdx.x); t < p.num_tiles; t += static_cast<int>(gridDim.x)) {
+      const ConvTile c = conv_tile(p, t);
+      int ok = 1;
+      if (lane == 0) ok = mbar_wait(&acc_full[acc], acc_phase, &abort_flag, p.err_word, 58) ? 1 : 0;
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) break;
+      while (!mbar_try_wait(&acc_full[acc], acc_phase)) {}  // completes at once: lane 0 saw the phase
+      tcgen05_fence_after();
+      const int oc0 = c.oc0 + quad * 32, nch = p.oc - oc0;
+      const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * CG_N);
+      if (nch > 0) {
+#pragma unroll 1
+        for (int ci = 0; ci < 4; ++ci) {
+          const int c0 = (half * 4 + ci) * 32;  // 32 pixels: two rows of the tile
+          const int y = c.y0 + c0 / CG_SIDE + (lane >> 4), x = c.x0 + (lane & 15);
+          if (c.y0 + c0 / CG_SIDE >= p.h) break;  // warp-uniform
+          const bool in = y < p.h && x < p.w;
+          const long long o0 = (static_cast<long long>(c.n) * p.oc + oc0) * hw + static_cast<long long>(y) * p.w + x;
+          float q[32];
+          if (p.residual != nullptr && in) {  // requested before the accumulators are read
+#pragma unroll
+            for (int j = 0; j < 32; ++j) q[j] = j < nch ? __ldg(p.residual + o0 + j * hw) : 0.0f;
+          }
+          float v[32];
+          tmem_ld_32x32(taddr + c0, v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = __fmul_rn(v[j], p.acc_scale);  // [pixel][channel]
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = tbuf[lane * 33 + j];
+          __syncwarp();
+          if (p.activation != -1) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.activation);
+          }
+          if (in) {
+            if (p.residual != nullptr) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += q[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < nch) p.out[o0 + j * hw] = v[j];
+          }
+        }
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+    }
+  }
+
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+template <int AP, int WP>
+int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
+  const int ks = g.conv_ks, pad = g.conv_pad, hp = g.conv_h + 2 * pad, wp = g.conv_w + 2 * pad;
+  ConvGemmParams p;
+  p.batch = g.m / (hp * wp);
+  p.oc = g.n; p.h = g.conv_h; p.w = g.conv_w; p.ks = ks; p.cblocks = g.conv_c / CG_BK;
+  p.tiles_x = (p.w + CG_SIDE - 1) / CG_SIDE;
+  p.tiles_y = (p.h + CG_SIDE - 1) / CG_SIDE;
+  p.tiles_o = (p.oc + CG_M - 1) / CG_M;
+  p.num_tiles = p.batch * p.tiles_y * p.tiles_x * p.tiles_o;
+  const int rows = CG_SIDE + ks - 1;
+  p.a_stage_bytes = AP * CG_SIDE * rows * CG_BK * 2;
+  const int ring = CG_SMEM_MAX - CG_EPI - 1024 - 1024;  // (less the barriers)
+  p.a_stages = 3;
+  p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (WP * CG_W_TILE);
+  if (p.w_stages < 3) {
+    p.a_stages = 2;
+    p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (WP * CG_W_TILE);
+  }
+  if (p.w_stages > CG_MAX_RING) p.w_stages = CG_MAX_RING;
+  p.residual = g.residual; p.out = g.out_f32; p.activation = g.activation;
+  p.acc_scale = gemm_acc_scale(g);
+  p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
+  p.err_word = ctx().dev_error_word;
+  CUtensorMap map_a, map_w;
+  MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, CG_BK, CG_SIDE, rows));
+  MB_TRY(make_plane_map(&map_w, g.w, WP, g.n, round_up(g.k, 64), CG_BK, CG_M));
+  const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * WP * CG_W_TILE + CG_EPI + 1024;
+  static PerDeviceOnce attr_once;
+  MB_TRY(attr_once.run([&]() -> int {
+    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
+    return MIMIR_B200_OK;
+  }));
+  const int sms = ctx().sm_count;
+  GemmProfile prof(st);
+  MB_TRY(prof.begin());
+  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p));
+  MB_TRY(prof.end());
+  count_launch();
+  return MIMIR_B200_OK;
+}
+
+}  // namespace
+
+bool conv_gemm_wanted(const GemmArgs& g) {
+  const char* e = getenv("MIMIR_B200_CONV_SPATIAL");  // "0": never, "1": wherever the form allows
+  if (e && e[0] == '0') return false;
+  if (g.conv_ks < 3 || g.conv_ks > 7 || g.conv_c % CG_BK != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
+    return false;
+  if (!(g.a_planes == 2 || g.w_planes == 1)) return false;
+  if (e && e[0] == '1') return true;
+  // 16 x 16 tiles must be mostly image, and there must be one for every SM: below that the narrow tiles of gemm_split.cu win
+  const long long ty = (g.conv_h + CG_SIDE - 1) / CG_SIDE, tx = (g.conv_w + CG_SIDE - 1) / CG_SIDE;
+  const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
+  const long long tiles = g.m / per * ty * tx * ((g.n + CG_M - 1) / CG_M);
+  return static_cast<double>(g.conv_h) * g.conv_w >= 0.7 * static_cast<double>(ty * tx * CG_N) && tiles >= ctx().sm_count;
+}
+
+int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {
+  if (g.a_planes == 2 && g.w_planes == 2) return launch_conv_t<2, 2>(g, st);
+  if (g.a_planes == 2 && g.w_planes == 1) return launch_conv_t<2, 1>(g, st);
+  if (g.a_planes == 1 && g.w_planes == 1) return launch_conv_t<1, 1>(g, st);
+  return fail(MIMIR_B200_E_INVALID, "conv: %d activation and %d weight planes", g.a_planes, g.w_planes);
+}
+
+}  // namespace mb

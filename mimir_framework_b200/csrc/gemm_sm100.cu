@@ -683,6 +683,23 @@ int make_plane_map(CUtensorMap* map, const void* base, int planes, long long row
   return MIMIR_B200_OK;
 }
 
+// 5-D map over zero-padded NHWC planes [planes][n][hp][wp][c]; box = {bc, bx, by, 1, 1}; swizzle span = bc * 2 bytes.
+int make_image_map(CUtensorMap* map, const void* base, int planes, int n, int hp, int wp, int c, int bc, int bx, int by) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(MIMIR_B200_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (bc != 32 && bc != 64) || c % bc != 0) return fail(MIMIR_B200_E_INVALID, "conv operand layout");
+  const cuuint64_t row = static_cast<cuuint64_t>(c) * 2, line = row * wp, image = line * hp;
+  cuuint64_t dims[5] = {static_cast<cuuint64_t>(c), static_cast<cuuint64_t>(wp), static_cast<cuuint64_t>(hp), static_cast<cuuint64_t>(n), static_cast<cuuint64_t>(planes)};
+  cuuint64_t strides[4] = {row, line, image, image * n};
+  cuuint32_t box[5] = {static_cast<cuuint32_t>(bc), static_cast<cuuint32_t>(bx), static_cast<cuuint32_t>(by), 1, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUtensorMapSwizzle sw = (bc == 64) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(MIMIR_B200_E_CUDA, "cuTensorMapEncodeTiled (image) failed (%d)", static_cast<int>(r));
+  return MIMIR_B200_OK;
+}
+
 // What an accumulator is multiplied by before bias / activation: the mean loss of the tensor core's truncating adds undone, the
 // weight scale divided out.  Measured on B200 against fp64 products of the same operand planes (random normal operands, K = 256 ...
 // 4096, two and three MMAs per 16-wide K step): the accumulated result is low by 1.47e-8 ... 1.58e-8 of its value per MMA
@@ -1089,6 +1106,8 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
       return fail(MIMIR_B200_E_INVALID, "gemm: bad shifted-convolution arguments");
   }
   const int bk = env_int("MIMIR_B200_GEMM_BK", (g.a_planes + g.w_planes <= 3) ? 64 : 32);
+  // large images with ks >= 3: tiles of 16 x 16 pixels that fetch their halo once per kernel column
+  if (g.conv_ks > 0 && conv_gemm_wanted(g)) return launch_conv_gemm(g, st);
   // launches that leave SMs without a 128 x 256 tile go to the split-K kernel with narrower tiles (never when the big tiles fill
   // the GPU more than once over: re-reading the operands for narrow tiles then costs more than an even last wave gives)
   const int sbk = (g.conv_ks == 0 || g.conv_c % 64 == 0) ? 64 : 32;
