@@ -302,7 +302,7 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
 bool conv_gemm_wanted(const GemmArgs& g) {
   const char* e = getenv("MIMIR_B200_CONV_SPATIAL");  // "0": never, "1": wherever the form allows
   if (e && e[0] == '0') return false;
-  if (g.conv_ks < 3 || g.conv_ks > 7 || g.conv_c % CG_BK != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
+  if (g.conv_ks < 1 || g.conv_ks > 7 || g.conv_c % CG_BK != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
     return false;
   if (!(g.a_planes == 2 || g.w_planes == 1)) return false;
   if (e && e[0] == '1') return true;

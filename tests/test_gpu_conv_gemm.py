@@ -20,7 +20,7 @@ def rt():
 
 @pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W, abi.PREC_BF16])
 @pytest.mark.parametrize("batch,ic,oc,h,w,k", [(1, 32, 16, 16, 16, 3), (2, 64, 130, 17, 33, 3), (3, 96, 40, 31, 15, 5), (1, 32, 260, 5, 48, 7), (2, 256, 128, 32, 32, 3),
-                                               (5, 32, 33, 1, 1, 3)])
+                                               (5, 32, 33, 1, 1, 3), (2, 64, 128, 20, 40, 1)])
 def test_forced_spatial_tiles_against_the_port(rt, monkeypatch, precision, batch, ic, oc, h, w, k):
     monkeypatch.setenv("MIMIR_B200_CONV_SPATIAL", "1")
     r = np.random.default_rng(batch * ic + oc + k)
