@@ -27,8 +27,7 @@ namespace mb {
 namespace {
 
 constexpr int CG_THREADS = 352;
-constexpr int CG_SIDE = 16;                    // a tile is 16 x 16 pixels
-constexpr int CG_N = CG_SIDE * CG_SIDE;
+constexpr int CG_N = 256;                      // pixels of a tile: 16 x 16 or, for 1 x 1 kernels, 256 of the flattened image
 constexpr int CG_M = 128;                      // output channels of a tile
 constexpr int CG_BK = 32;                      // channels of a K block: 64-byte swizzle rows
 constexpr int CG_W_TILE = CG_M * CG_BK * 2;
@@ -38,7 +37,7 @@ constexpr int CG_SMEM_MAX = 232448;
 
 struct ConvGemmParams {
   int batch, oc, h, w, ks, cblocks;            // cblocks = channels / 32
-  int tiles_x, tiles_y, tiles_o, num_tiles;
+  int tw_log, tiles_x, tiles_y, tiles_o, num_tiles;  // a tile is 1 << tw_log pixels wide
   int a_stages, a_stage_bytes, w_stages;
   const float* residual;
   float* out;
@@ -53,9 +52,9 @@ __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) { 
   ConvTile c;
   c.oc0 = (t % p.tiles_o) * CG_M;
   int s = t / p.tiles_o;
-  c.x0 = (s % p.tiles_x) * CG_SIDE;
+  c.x0 = (s % p.tiles_x) << p.tw_log;
   s /= p.tiles_x;
-  c.y0 = (s % p.tiles_y) * CG_SIDE;
+  c.y0 = (s % p.tiles_y) * (CG_N >> p.tw_log);
   c.n = s / p.tiles_y;
   return c;
 }
@@ -159,8 +158,8 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         for (int kh = 0; kh < p.ks; ++kh) {
           if (!__all_sync(0xffffffffu, w_ready) && !mbar_wait_warp(&w_full[ws], wph, &abort_flag, p.err_word, 57)) { ok = false; break; }
           tcgen05_fence_after();
-          // kh rows further down: 16 pixels x 64 bytes = 1024 = 64 in the descriptor's address field
-          const uint64_t da = da0 + static_cast<uint64_t>(kh * 64), da_lo = da + static_cast<uint64_t>(a_plane >> 4);
+          // kh rows further down: tile width x 64 bytes, in the descriptor's address field (16 bytes)
+          const uint64_t da = da0 + static_cast<uint64_t>(kh << (p.tw_log + 2)), da_lo = da + static_cast<uint64_t>(a_plane >> 4);
           const uint64_t dw = make_smem_desc(smem_u32(w_ring + ws * (WP * CG_W_TILE)), 64), dw_lo = dw + (CG_W_TILE >> 4);
           uint64_t* w_done = &w_empty[ws];
           if (++ws == p.w_stages) { ws = 0; wph ^= 1; }
@@ -195,29 +194,42 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     uint32_t acc_phase = 0;
     for (int t = static_cast<int>(blockIdx.x); t < p.num_tiles; t += static_cast<int>(gridDim.x)) {
       const ConvTile c = conv_tile(p, t);
+      const int oc0 = c.oc0 + quad * 32, nch = p.oc - oc0;
+      // chunk ci of this warp: 32 consecutive pixels of the tile
+      auto place = [&](int ci, bool& in, long long& o0) {
+        const int px = (half * 4 + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
+        in = y < p.h && x < p.w;
+        o0 = (static_cast<long long>(c.n) * p.oc + oc0) * hw + static_cast<long long>(y) * p.w + x;
+      };
+      // The residual of a chunk is requested one chunk ahead, the first one's before the accumulators are waited for: a 1 x 1 skip
+      // layer reads and writes more than it multiplies, and its loads would each wait a full memory latency.
+      float q[32];
+      auto request = [&](int ci) {
+        bool in;
+        long long o0;
+        place(ci, in, o0);
+        if (in) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) q[j] = j < nch ? __ldg(p.residual + o0 + j * hw) : 0.0f;
+        }
+      };
+      if (p.residual != nullptr && nch > 0) request(0);
       int ok = 1;
       if (lane == 0) ok = mbar_wait(&acc_full[acc], acc_phase, &abort_flag, p.err_word, 58) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       while (!mbar_try_wait(&acc_full[acc], acc_phase)) {}  // completes at once: lane 0 saw the phase
       tcgen05_fence_after();
-      const int oc0 = c.oc0 + quad * 32, nch = p.oc - oc0;
       const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * CG_N);
       if (nch > 0) {
 #pragma unroll 1
         for (int ci = 0; ci < 4; ++ci) {
-          const int c0 = (half * 4 + ci) * 32;  // 32 pixels: two rows of the tile
-          const int y = c.y0 + c0 / CG_SIDE + (lane >> 4), x = c.x0 + (lane & 15);
-          if (c.y0 + c0 / CG_SIDE >= p.h) break;  // warp-uniform
-          const bool in = y < p.h && x < p.w;
-          const long long o0 = (static_cast<long long>(c.n) * p.oc + oc0) * hw + static_cast<long long>(y) * p.w + x;
-          float q[32];
-          if (p.residual != nullptr && in) {  // requested before the accumulators are read
-#pragma unroll
-            for (int j = 0; j < 32; ++j) q[j] = j < nch ? __ldg(p.residual + o0 + j * hw) : 0.0f;
-          }
+          if (c.y0 + (((half * 4 + ci) * 32) >> p.tw_log) >= p.h) break;  // warp-uniform
+          bool in;
+          long long o0;
+          place(ci, in, o0);
           float v[32];
-          tmem_ld_32x32(taddr + c0, v);
+          tmem_ld_32x32(taddr + (half * 4 + ci) * 32, v);
 #pragma unroll
           for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = __fmul_rn(v[j], p.acc_scale);  // [pixel][channel]
           __syncwarp();
@@ -228,11 +240,12 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.activation);
           }
-          if (in) {
-            if (p.residual != nullptr) {
+          if (p.residual != nullptr) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += q[j];
-            }
+            for (int j = 0; j < 32; ++j) v[j] += q[j];
+            if (ci < 3) request(ci + 1);
+          }
+          if (in) {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < nch) p.out[o0 + j * hw] = v[j];
@@ -255,18 +268,33 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
 }
 
+// Image and tile shape of a launch.  A 1 x 1 kernel sees the image as one line (tiles of 256 consecutive pixels, whole 128-byte
+// lines in every channel plane: with 16-pixel rows its scattered 64-byte stores held DRAM at 4 TB/s).  Otherwise 16 x 16 (32 x 8 where
+// the width allows whole lines measured the same: there the MMAs, not the stores, set the pace).
+struct ConvShape { int h, w, tw_log, tiles_x, tiles_y; };
+ConvShape conv_shape(const GemmArgs& g) {
+  ConvShape s{g.conv_h, g.conv_w, 4, 0, 0};
+  if (g.conv_ks == 1) { s.w = g.conv_h * g.conv_w; s.h = 1; s.tw_log = 8; }
+  const int tw = 1 << s.tw_log, th = CG_N >> s.tw_log;
+  s.tiles_x = (s.w + tw - 1) / tw;
+  s.tiles_y = (s.h + th - 1) / th;
+  return s;
+}
+
 template <int AP, int WP>
 int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
-  const int ks = g.conv_ks, pad = g.conv_pad, hp = g.conv_h + 2 * pad, wp = g.conv_w + 2 * pad;
+  const int ks = g.conv_ks, pad = g.conv_pad;
   ConvGemmParams p;
-  p.batch = g.m / (hp * wp);
-  p.oc = g.n; p.h = g.conv_h; p.w = g.conv_w; p.ks = ks; p.cblocks = g.conv_c / CG_BK;
-  p.tiles_x = (p.w + CG_SIDE - 1) / CG_SIDE;
-  p.tiles_y = (p.h + CG_SIDE - 1) / CG_SIDE;
+  p.batch = g.m / ((g.conv_h + 2 * pad) * (g.conv_w + 2 * pad));
+  const ConvShape sh = conv_shape(g);
+  const int hp = sh.h + 2 * pad, wp = sh.w + 2 * pad, tw = 1 << sh.tw_log, th = CG_N >> sh.tw_log;
+  p.oc = g.n; p.h = sh.h; p.w = sh.w; p.ks = ks; p.cblocks = g.conv_c / CG_BK;
+  p.tw_log = sh.tw_log;
+  p.tiles_x = sh.tiles_x; p.tiles_y = sh.tiles_y;
   p.tiles_o = (p.oc + CG_M - 1) / CG_M;
   p.num_tiles = p.batch * p.tiles_y * p.tiles_x * p.tiles_o;
-  const int rows = CG_SIDE + ks - 1;
-  p.a_stage_bytes = AP * CG_SIDE * rows * CG_BK * 2;
+  const int rows = th + ks - 1;
+  p.a_stage_bytes = AP * tw * rows * CG_BK * 2;
   const int ring = CG_SMEM_MAX - CG_EPI - 1024 - 1024;  // (less the barriers)
   p.a_stages = 3;
   p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (WP * CG_W_TILE);
@@ -280,7 +308,7 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   p.err_word = ctx().dev_error_word;
   CUtensorMap map_a, map_w;
-  MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, CG_BK, CG_SIDE, rows));
+  MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, CG_BK, tw, rows));
   MB_TRY(make_plane_map(&map_w, g.w, WP, g.n, round_up(g.k, 64), CG_BK, CG_M));
   const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * WP * CG_W_TILE + CG_EPI + 1024;
   static PerDeviceOnce attr_once;
@@ -306,11 +334,14 @@ bool conv_gemm_wanted(const GemmArgs& g) {
     return false;
   if (!(g.a_planes == 2 || g.w_planes == 1)) return false;
   if (e && e[0] == '1') return true;
-  // 16 x 16 tiles must be mostly image, and there must be one for every SM: below that the narrow tiles of gemm_split.cu win
-  const long long ty = (g.conv_h + CG_SIDE - 1) / CG_SIDE, tx = (g.conv_w + CG_SIDE - 1) / CG_SIDE;
+  // 1 x 1 (and im2col rows): nothing to share between taps; long K is better off in CTA pairs (K = 4608, 512 channels: 170 against
+  // 111 us), short K is bound by its stores (K = 192, 64 channels: 139 against 247 us)
+  if (g.conv_ks == 1 && g.conv_c > 1024) return false;
+  // the tiles must be mostly image, and there must be one for every SM: below that the narrow tiles of gemm_split.cu win
+  const ConvShape sh = conv_shape(g);
   const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
-  const long long tiles = g.m / per * ty * tx * ((g.n + CG_M - 1) / CG_M);
-  return static_cast<double>(g.conv_h) * g.conv_w >= 0.7 * static_cast<double>(ty * tx * CG_N) && tiles >= ctx().sm_count;
+  const long long tiles = g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
+  return static_cast<double>(g.conv_h) * g.conv_w >= 0.7 * static_cast<double>(sh.tiles_y) * sh.tiles_x * CG_N && tiles >= ctx().sm_count;
 }
 
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {

@@ -706,7 +706,7 @@ int make_image_map(CUtensorMap* map, const void* base, int planes, int n, int hp
 // instruction that added into it; all-positive operands lose 2.1e-8 ... 3.6e-8.  Zero-padded K adds exact zeros and loses nothing,
 // so only the real K counts.  Undoing the mean loss halves the accumulation error.
 float gemm_acc_scale(const GemmArgs& g) {
-  const long long ksteps = g.conv_ks > 0 ? static_cast<long long>(g.conv_ks) * g.conv_ks * ((g.conv_c + UMMA_K - 1) / UMMA_K)
+  const long long ksteps = g.conv_ks > 1 ? static_cast<long long>(g.conv_ks) * g.conv_ks * ((g.conv_c + UMMA_K - 1) / UMMA_K)
                                          : (g.k + UMMA_K - 1) / UMMA_K;
   const int products = 1 + (g.a_planes == 2 ? 1 : 0) + (g.w_planes == 2 ? 1 : 0);
   static const bool comp = [] { const char* e = getenv("MIMIR_B200_ACC_COMP"); return !(e && e[0] == '0'); }();

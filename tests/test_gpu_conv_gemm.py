@@ -20,7 +20,7 @@ def rt():
 
 @pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W, abi.PREC_BF16])
 @pytest.mark.parametrize("batch,ic,oc,h,w,k", [(1, 32, 16, 16, 16, 3), (2, 64, 130, 17, 33, 3), (3, 96, 40, 31, 15, 5), (1, 32, 260, 5, 48, 7), (2, 256, 128, 32, 32, 3),
-                                               (5, 32, 33, 1, 1, 3), (2, 64, 128, 20, 40, 1)])
+                                               (5, 32, 33, 1, 1, 3), (2, 64, 128, 20, 40, 1), (2, 32, 64, 9, 64, 5)])
 def test_forced_spatial_tiles_against_the_port(rt, monkeypatch, precision, batch, ic, oc, h, w, k):
     monkeypatch.setenv("MIMIR_B200_CONV_SPATIAL", "1")
     r = np.random.default_rng(batch * ic + oc + k)
@@ -39,6 +39,17 @@ def test_forced_spatial_tiles_against_the_port(rt, monkeypatch, precision, batch
     want = np.stack([port.conv2d(x[i], wt, ic, oc, h, w, k, 1, k // 2, False).ravel() for i in range(batch)]) + res
     tol = 2e-3 if precision == abi.PREC_BF16 else 1e-5
     assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("batch,ic,oc,h,k,stride,pad", [(2, 3, 64, 37, 7, 2, 3), (1, 40, 130, 20, 3, 2, 1), (3, 4, 70, 18, 3, 1, 1)])
+def test_im2col_rows_as_pixels(rt, monkeypatch, batch, ic, oc, h, k, stride, pad):
+    monkeypatch.setenv("MIMIR_B200_CONV_SPATIAL", "1")
+    r = np.random.default_rng(ic)
+    x = r.standard_normal((batch, ic * h * h)).astype(np.float32)
+    wt = (r.standard_normal(oc * ic * k * k) / np.sqrt(ic * k * k)).astype(np.float32)
+    got = rt.conv2d(x, wt, batch, ic, oc, h, h, k, stride, pad).reshape(batch, -1)
+    want = np.stack([port.conv2d(x[i], wt, ic, oc, h, h, k, stride, pad, False).ravel() for i in range(batch)])
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
 
 
 def test_relu_and_many_tiles(rt):
