@@ -435,13 +435,6 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     g.out_f32 = e.y + static_cast<size_t>(b0) * e.oc * ohw;
     g.residual = e.residual ? e.residual + static_cast<size_t>(b0) * e.oc * ohw : nullptr;
     g.ldo = e.oc;
-    // the im2col rows as the pixels of an image with kp channels: a 1 x 1 convolution in tiles of 256 pixels
-    GemmArgs c = g;
-    c.conv_ks = 1; c.conv_c = round_up(k, 64); c.conv_pad = 0; c.conv_h = oh; c.conv_w = ow;
-    if (conv_gemm_wanted(c)) {
-      MB_TRY(launch_conv_gemm(c, st));
-      continue;
-    }
     g.out_nchw_hw = ohw;
     MB_TRY(launch_gemm(g, st));
   }

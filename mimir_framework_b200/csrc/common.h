@@ -200,11 +200,12 @@ struct GemmProfile {
   cudaStream_t st;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
 };
-// gemm_split.cu: narrow tiles and split K for launches of few 128 x 256 tiles; wanted when its estimate beats `other_cycles`
-bool gemm_split_wanted(const GemmArgs& g, int bk, double other_cycles, int* bn, int* splits);
+// Estimated SM cycles of a launch in each form (1e30: not possible); launch_gemm takes the smallest.
+// gemm_split.cu: narrow tiles and split K for launches of few 128 x 256 tiles
+double gemm_split_cycles(const GemmArgs& g, int bk, int* bn, int* splits);
 int launch_gemm_split(const GemmArgs& g, int bk, int bn, int splits, cudaStream_t st);
-// conv_gemm.cu: shifted-GEMM convolutions (conv_ks >= 3) in 16 x 16 pixel tiles
-bool conv_gemm_wanted(const GemmArgs& g);
+// conv_gemm.cu: shifted-GEMM convolutions in tiles of 256 pixels
+double conv_gemm_cycles(const GemmArgs& g);
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st);
 inline size_t gemm_gn_part_bytes(long long m, int n, int cpg) {
   return static_cast<size_t>((m + 31) / 32) * static_cast<size_t>((n + 31) / 32) * static_cast<size_t>(2 * (1 + 64 / cpg)) * sizeof(float);

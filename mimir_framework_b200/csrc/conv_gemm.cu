@@ -327,21 +327,23 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
 
 }  // namespace
 
-bool conv_gemm_wanted(const GemmArgs& g) {
+double conv_gemm_cycles(const GemmArgs& g) {
+  constexpr double never = 1e30;
   const char* e = getenv("MIMIR_B200_CONV_SPATIAL");  // "0": never, "1": wherever the form allows
-  if (e && e[0] == '0') return false;
+  if (e && e[0] == '0') return never;
   if (g.conv_ks < 1 || g.conv_ks > 7 || g.conv_c % CG_BK != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
-    return false;
-  if (!(g.a_planes == 2 || g.w_planes == 1)) return false;
-  if (e && e[0] == '1') return true;
+    return never;
+  if (!(g.a_planes == 2 || g.w_planes == 1)) return never;
+  if (e && e[0] == '1') return 0.0;
   // 1 x 1 (and im2col rows): nothing to share between taps; long K is better off in CTA pairs (K = 4608, 512 channels: 170 against
   // 111 us), short K is bound by its stores (K = 192, 64 channels: 139 against 247 us)
-  if (g.conv_ks == 1 && g.conv_c > 1024) return false;
-  // the tiles must be mostly image, and there must be one for every SM: below that the narrow tiles of gemm_split.cu win
+  if (g.conv_ks == 1 && g.conv_c > 1024) return never;
   const ConvShape sh = conv_shape(g);
   const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
   const long long tiles = g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
-  return static_cast<double>(g.conv_h) * g.conv_w >= 0.7 * static_cast<double>(sh.tiles_y) * sh.tiles_x * CG_N && tiles >= ctx().sm_count;
+  const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
+  const double mma = 1.15 * g.k / 16.0 * (g.a_planes + g.w_planes - 1) * 128.0;
+  return 17400.0 + waves * (mma > 4500.0 ? mma : 4500.0);  // (within 5 % of 50 measured launches, K = 64 ... 4608)
 }
 
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {

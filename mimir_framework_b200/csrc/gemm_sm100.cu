@@ -1083,10 +1083,14 @@ namespace {
 // operand loads per tile, whole waves, one exposed epilogue).
 double big_tile_cycles(const GemmArgs& g) {
   const int products = 1 + (g.a_planes == 2) + (g.w_planes == 2);
-  const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
-  const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
   const double k = g.conv_ks > 0 ? static_cast<double>(g.k) : static_cast<double>(round_up(g.k, 64));
   const double mma = k / UMMA_K * products * 128.0, load = k * 2.0 * (g.a_planes * BM + g.w_planes * BN) / 51.6;
+  if (g.conv_ks > 0 || g.out_nchw_hw > 0) {  // 256 pixels x 128 channels either way round; the epilogue's scattered stores bound short K
+    const long long tiles = static_cast<long long>((g.m + BN - 1) / BN) * ((g.n + BM - 1) / BM), waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
+    return 19000.0 + waves * (1.2 * mma > 12000.0 ? 1.2 * mma : 12000.0);
+  }
+  const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
+  const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
   const double tile = (mma > load ? mma : load);
   return 15100.0 + waves * (tile > 12000.0 ? tile : 12000.0);  // (a tile's epilogue takes about 12 000 cycles beside the next main loop)
 }
@@ -1106,16 +1110,24 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
       return fail(MIMIR_B200_E_INVALID, "gemm: bad shifted-convolution arguments");
   }
   const int bk = env_int("MIMIR_B200_GEMM_BK", (g.a_planes + g.w_planes <= 3) ? 64 : 32);
-  // large images with ks >= 3: tiles of 16 x 16 pixels that fetch their halo once per kernel column
-  if (g.conv_ks > 0 && conv_gemm_wanted(g)) return launch_conv_gemm(g, st);
-  // launches that leave SMs without a 128 x 256 tile go to the split-K kernel with narrower tiles (never when the big tiles fill
-  // the GPU more than once over: re-reading the operands for narrow tiles then costs more than an even last wave gives)
+  // Three forms: 128 x 256 tiles here, narrow tiles with split K (only where the big tiles fill the GPU less than one and a half times:
+  // beyond that re-reading the operands costs more than an even last wave gives), and for convolutions tiles of 256 pixels.
   const int sbk = (g.conv_ks == 0 || g.conv_c % 64 == 0) ? 64 : 32;
   const long long big_tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
-  int bn = 0, splits = 0;
   static const bool force_pairs = env_int("MIMIR_B200_GEMM_PAIR", -1) == 1;  // pairs wherever the form allows
-  if (!force_pairs && big_tiles < ctx().sm_count + ctx().sm_count / 2 && gemm_split_wanted(g, sbk, big_tile_cycles(g), &bn, &splits))
-    return launch_gemm_split(g, sbk, bn, splits, st);
+  if (!force_pairs) {
+    const double big = big_tile_cycles(g);
+    int bn = 0, splits = 0;
+    const double split = big_tiles < ctx().sm_count + ctx().sm_count / 2 ? gemm_split_cycles(g, sbk, &bn, &splits) : 1e30;
+    GemmArgs c = g;
+    if (g.conv_ks == 0 && g.out_nchw_hw > 0) {  // im2col rows are the pixels of an image with round_up(k, 64) channels
+      c.conv_ks = 1; c.conv_c = round_up(g.k, 64); c.conv_pad = 0; c.conv_h = 1; c.conv_w = g.out_nchw_hw;
+      c.out_nchw_hw = 0;
+    }
+    const double spatial = c.conv_ks > 0 ? conv_gemm_cycles(c) : 1e30;
+    if (spatial < 1e30 && spatial <= split && spatial <= big) return launch_conv_gemm(c, st);
+    if (split < big) return launch_gemm_split(g, sbk, bn, splits, st);
+  }
   if (bk == 64 && (g.conv_ks == 0 || g.conv_c % 64 == 0)) return launch_gemm_t<64>(g, st);
   return launch_gemm_t<32>(g, st);
 }
