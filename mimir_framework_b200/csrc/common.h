@@ -264,6 +264,26 @@ int launch_copy_strided(const float* src, float* dst, int batch, int64_t n, int6
                         cudaStream_t st, int64_t src_stride = 0);
 int launch_broadcast_rows(const float* src, float* dst, int batch, int64_t n, cudaStream_t st);
 
+// norm_rows.cu: rows that fit in registers
+enum : int { ROWS_MEANVAR = 0, ROWS_RMS = 1, ROWS_SOFTMAX = 2 };
+struct RowNormArgs {
+  int family = ROWS_MEANVAR;
+  const float* x = nullptr;
+  float* y = nullptr;
+  long long rows = 0, len = 0;
+  float eps = 0.0f;
+  const float* gamma = nullptr;      // may be null; beta only with gamma
+  const float* beta = nullptr;
+  int per_channel = 0;               // 0: gamma[i]; 1: gamma[(row % groups) * cpg + i / hw]
+  int groups = 1, cpg = 1, hw = 1;
+  int act = -1;                      // -1 or MIMIR_B200_ELT_SILU
+  const float* residual = nullptr;   // added last
+  long long n_gamma = 0;             // RMS: gamma applies to i < n_gamma
+  int log_softmax = 0;
+};
+bool norm_rows_supported(long long rows, long long len);
+int launch_norm_rows(const RowNormArgs& a, cudaStream_t st);
+
 // norms.cu -------------------------------------------------------------------------------------
 int launch_layernorm(const float* x, const float* gamma, const float* beta, float* y, int64_t rows, int64_t n,
                      float eps, cudaStream_t st);

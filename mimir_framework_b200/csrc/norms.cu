@@ -753,95 +753,6 @@ __global__ void meanvar_chunk_apply_kernel(const float* __restrict__ x, float* _
   meanvar_write_row(g, o, cn, vec, mean, inv, row + row0, base, al, off);
 }
 
-// ---- a few rows of up to ~100 000 elements: one thread-block cluster per row -----------------------
-// Each CTA of the cluster keeps a slice of the row in shared memory; the partial sums meet through
-// distributed shared memory (every CTA reads all partials in the same order, so all agree bit for bit):
-// first the sum for the mean, then the centred second moment, as the reference's two loops do
-// (LayerOps.hpp:287-300).  One launch, one read and one write of the row, no global scratch.
-constexpr int CLUSTER_SLICE_MAX = 12288;  // floats of shared memory per CTA (48 KB)
-
-__global__ void __launch_bounds__(256) meanvar_cluster_kernel(const float* __restrict__ x, float* __restrict__ y, long long len,
-                                                              int slice, float eps, Affine a) {
-  pdl_launch_dependents();
-  pdl_wait();
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ __align__(16) float sx[];
-  __shared__ float red[33];
-  __shared__ float part[2];
-  const unsigned ncl = cl.num_blocks(), rank = cl.block_rank();
-  const long long row = blockIdx.x / ncl;
-  const long long off = static_cast<long long>(rank) * slice;
-  const int n = static_cast<int>(max(0ll, min(static_cast<long long>(slice), len - off)));
-  const long long base = row * len;
-  const float acc = stage_and_sum(x + base + off, sx, n);
-  const float s = block_sum(acc, red);
-  if (threadIdx.x == 0) part[0] = s;
-  cl.sync();
-  float total = 0.0f;
-  for (unsigned k = 0; k < ncl; ++k) total += *cl.map_shared_rank(&part[0], k);
-  const float mean = total / static_cast<float>(len);
-  float q = 0.0f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const float d = sx[i] - mean;
-    q = fmaf(d, d, q);
-  }
-  const float m2 = block_sum(q, red);
-  if (threadIdx.x == 0) part[1] = m2;
-  cl.sync();
-  float var = 0.0f;
-  for (unsigned k = 0; k < ncl; ++k) var += *cl.map_shared_rank(&part[1], k);
-  const float inv = 1.0f / sqrtf(var / static_cast<float>(len) + eps);
-  float* o = y + base + off;
-  // 16-byte path: four neighbours share a channel when the plane size is a multiple of 4 (slices start on multiples of 4)
-  const bool vec = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(o) & 15) == 0 &&
-                   (a.residual == nullptr || (reinterpret_cast<uintptr_t>(a.residual + base + off) & 15) == 0) &&
-                   (a.per_channel ? (a.hw & 3) == 0
-                                  : ((a.gamma == nullptr || (reinterpret_cast<uintptr_t>(a.gamma + off) & 15) == 0) &&
-                                     (a.beta == nullptr || (reinterpret_cast<uintptr_t>(a.beta + off) & 15) == 0)));
-  if (vec) {
-    const float4* s4 = reinterpret_cast<const float4*>(sx);
-    const float4* g4 = (a.gamma && !a.per_channel) ? reinterpret_cast<const float4*>(a.gamma + off) : nullptr;
-    const float4* b4 = (a.beta && !a.per_channel) ? reinterpret_cast<const float4*>(a.beta + off) : nullptr;
-    const float4* r4 = a.residual ? reinterpret_cast<const float4*>(a.residual + base + off) : nullptr;
-    const int ch0 = a.per_channel ? static_cast<int>(row % a.groups) * a.cpg : 0;
-    const unsigned off_u = static_cast<unsigned>(off);
-    for (int i = threadIdx.x; i < (n >> 2); i += blockDim.x) {
-      const float4 v = s4[i];
-      float4 r = make_float4((v.x - mean) * inv, (v.y - mean) * inv, (v.z - mean) * inv, (v.w - mean) * inv);
-      if (a.per_channel) {
-        if (a.gamma != nullptr) {
-          const int gi = ch0 + static_cast<int>((off_u + 4u * static_cast<unsigned>(i)) / static_cast<unsigned>(a.hw));
-          const float w = __ldg(a.gamma + gi);
-          r.x *= w; r.y *= w; r.z *= w; r.w *= w;
-          if (a.beta != nullptr) {
-            const float b = __ldg(a.beta + gi);
-            r.x += b; r.y += b; r.z += b; r.w += b;
-          }
-        }
-      } else if (g4 != nullptr) {
-        const float4 w = __ldg(g4 + i);
-        r.x *= w.x; r.y *= w.y; r.z *= w.z; r.w *= w.w;
-        if (b4 != nullptr) {
-          const float4 b = __ldg(b4 + i);
-          r.x += b.x; r.y += b.y; r.z += b.z; r.w += b.w;
-        }
-      }
-      if (a.act == MIMIR_B200_ELT_SILU) {
-        r.x = silu(r.x); r.y = silu(r.y); r.z = silu(r.z); r.w = silu(r.w);
-      }
-      if (r4 != nullptr) {
-        const float4 t = __ldg(r4 + i);
-        r.x += t.x; r.y += t.y; r.z += t.z; r.w += t.w;
-      }
-      __stcs(reinterpret_cast<float4*>(o) + i, r);
-    }
-  } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = finish((sx[i] - mean) * inv, off + i, row, base, a);
-  }
-  cl.sync();  // nobody leaves while a neighbour may still read its partial sums
-}
-
 template <int FAM, int THREADS>
 __global__ void __launch_bounds__(THREADS, (THREADS <= 512) ? 2 : 1) sweep_row_kernel(RowParams p) {
   __shared__ float red[33];
@@ -963,6 +874,11 @@ int launch_sweep_rows(const RowParams& p, cudaStream_t st) {
 // 4 x 256 x 256 slabs, 148 MB in flight) they still beat the chunk path's many short launches, so only
 // very long rows go to the chunk path (L2-sized row groups).
 // MIMIR_B200_NORM_PATH=sweep|chunk overrides the choice (measurement aid).
+// (MIMIR_B200_NORM_PATH=s / c force the sweep / chunk kernels)
+inline bool norm_rows_on() {
+  const char* v = getenv("MIMIR_B200_NORM_PATH");
+  return !(v && (v[0] == 's' || v[0] == 'c'));
+}
 inline bool use_sweeps(long long rows, long long len) {
   const char* v = getenv("MIMIR_B200_NORM_PATH");
   if (v && v[0] == 's') return true;
@@ -972,78 +888,6 @@ inline bool use_sweeps(long long rows, long long len) {
   return rows >= sms && in_flight <= (1024ll << 20);
 }
 
-// ---- warp-per-row LayerNorm for short rows (token-wise norms): no block barrier at all --------
-constexpr int WARP_ROW_MAX = 1024;  // floats
-
-template <int NV>  // 128-bit vectors per lane
-__global__ void __launch_bounds__(256) meanvar_warp_kernel(const float* __restrict__ x, float* __restrict__ y, long long rows,
-                                                           int len, float eps, Affine a) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  const int n4 = len >> 2;  // len is a multiple of 4 on this path
-  const bool gvec = a.gamma == nullptr || ((reinterpret_cast<uintptr_t>(a.gamma) & 15) == 0 &&
-                                           (a.beta == nullptr || (reinterpret_cast<uintptr_t>(a.beta) & 15) == 0));
-  for (long long row = warp; row < rows; row += nwarps) {
-    const long long base = row * len;
-    const float4* g4 = reinterpret_cast<const float4*>(x + base);
-    float4 v[NV];
-    float s = 0.0f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int i = lane + 32 * j;
-      v[j] = (i < n4) ? __ldg(g4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
-    }
-    const float mean = warp_sum(s) / static_cast<float>(len);
-    float q = 0.0f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      if (lane + 32 * j < n4) {
-        const float dx = v[j].x - mean, dy = v[j].y - mean, dz = v[j].z - mean, dw = v[j].w - mean;
-        q += (dx * dx + dy * dy) + (dz * dz + dw * dw);
-      }
-    }
-    const float inv = 1.0f / sqrtf(warp_sum(q) / static_cast<float>(len) + eps);
-    float4* o4 = reinterpret_cast<float4*>(y + base);
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int i = lane + 32 * j;
-      if (i < n4) {
-        float4 r;
-        if (!a.per_channel && gvec && a.act < 0 && a.residual == nullptr) {
-          r = make_float4((v[j].x - mean) * inv, (v[j].y - mean) * inv, (v[j].z - mean) * inv, (v[j].w - mean) * inv);
-          if (a.gamma != nullptr) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(a.gamma) + i);
-            r.x *= w.x; r.y *= w.y; r.z *= w.z; r.w *= w.w;
-            if (a.beta != nullptr) {
-              const float4 b = __ldg(reinterpret_cast<const float4*>(a.beta) + i);
-              r.x += b.x; r.y += b.y; r.z += b.z; r.w += b.w;
-            }
-          }
-        } else {
-          const long long e = static_cast<long long>(i) << 2;
-          r.x = finish((v[j].x - mean) * inv, e, row, base, a);
-          r.y = finish((v[j].y - mean) * inv, e + 1, row, base, a);
-          r.z = finish((v[j].z - mean) * inv, e + 2, row, base, a);
-          r.w = finish((v[j].w - mean) * inv, e + 3, row, base, a);
-        }
-        o4[i] = r;
-      }
-    }
-  }
-}
-
-template <int NV>
-int launch_warp_rows(const float* x, float* y, long long rows, int len, float eps, const Affine& a, cudaStream_t st) {
-  long long blocks = (rows + 7) / 8;
-  const long long cap = static_cast<long long>(ctx().sm_count) * 8;
-  if (blocks > cap) blocks = cap;
-  meanvar_warp_kernel<NV><<<static_cast<int>(blocks), 256, 0, st>>>(x, y, rows, len, eps, a);
-  MB_CUDA(cudaGetLastError());
-  count_launch();
-  return MIMIR_B200_OK;
-}
 
 // ---- scratch for the chunk kernels -------------------------------------------------------------
 // Partial statistics, and the ticket / slot words of the one-pass RMSNorm, live in an 8 MB buffer PER (device,
@@ -1099,35 +943,16 @@ constexpr long long L2_GROUP_BYTES = 104ll << 20;
 
 int meanvar_dispatch(const float* x, float* y, long long rows, long long len, float eps, const Affine& a, cudaStream_t st) {
   if (rows <= 0 || len <= 0) return fail(MIMIR_B200_E_INVALID, "norm: empty input");
-  const bool al16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
-                    (a.residual == nullptr || (reinterpret_cast<uintptr_t>(a.residual) & 15) == 0);
-  if (len <= WARP_ROW_MAX && (len & 3) == 0 && al16 && rows >= 64) {
-    const int nv = static_cast<int>((len / 4 + 31) / 32);
-    const int l = static_cast<int>(len);
-    if (nv <= 2) return launch_warp_rows<2>(x, y, rows, l, eps, a, st);
-    if (nv <= 4) return launch_warp_rows<4>(x, y, rows, l, eps, a, st);
-    if (nv <= 6) return launch_warp_rows<6>(x, y, rows, l, eps, a, st);
-    return launch_warp_rows<8>(x, y, rows, l, eps, a, st);
+  if (norm_rows_on() && norm_rows_supported(rows, len)) {
+    RowNormArgs r;
+    r.x = x; r.y = y; r.rows = rows; r.len = len; r.eps = eps; r.gamma = a.gamma; r.beta = a.beta; r.per_channel = a.per_channel;
+    r.groups = a.groups; r.cpg = a.cpg; r.hw = a.hw; r.act = a.act; r.residual = a.residual;
+    return launch_norm_rows(r, st);
   }
   if (use_sweeps(rows, len)) {
     RowParams p{};
     p.x = x; p.y = y; p.rows = rows; p.len = len; p.eps = eps; p.aff = a;
     return launch_sweep_rows<FAM_MEANVAR>(p, st);
-  }
-  static const bool no_cluster = [] { const char* e = getenv("MIMIR_B200_NORM_CLUSTER"); return e && e[0] == '0'; }();
-  if (!no_cluster && len <= 8ll * CLUSTER_SLICE_MAX && rows * 8 < 0x7fffffffLL) {
-    int ncl = 1;
-    while (ncl < 8 && (len + ncl - 1) / ncl > 4096) ncl *= 2;  // ~16 KB per CTA, at most the portable cluster size
-    const int slice = static_cast<int>(((len + ncl - 1) / ncl + 3) & ~3ll);
-    static PerDeviceOnce attr_once;  // static + dynamic shared memory of the largest slice is just above the 48 KB default
-    MB_TRY(attr_once.run([&]() -> int {
-      MB_CUDA(cudaFuncSetAttribute(meanvar_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CLUSTER_SLICE_MAX * 4));
-      return MIMIR_B200_OK;
-    }));
-    MB_TRY(launch_pdl(meanvar_cluster_kernel, dim3(static_cast<unsigned>(rows * ncl)), dim3(256), static_cast<size_t>(slice) * sizeof(float), st, ncl, x, y,
-                      static_cast<long long>(len), slice, eps, a));
-    count_launch();
-    return MIMIR_B200_OK;
   }
   const int chunks = static_cast<int>((len + CHUNK - 1) / CHUNK);
   std::lock_guard<std::mutex> scratch_lock(g_norm_mu);
@@ -1326,6 +1151,11 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
   // Below this length the sequential chain's rounding loss is < 1e-6 of the sum and any summation order
   // agrees with the reference; above it the chain is reproduced (rms_seq_err_kernel).
   constexpr long long FAITHFUL_FROM = 16384;
+  if (n <= FAITHFUL_FROM && norm_rows_on() && norm_rows_supported(batch, n)) {
+    RowNormArgs r;
+    r.family = ROWS_RMS; r.x = x; r.y = y; r.rows = batch; r.len = n; r.eps = eps; r.gamma = gamma; r.n_gamma = gamma ? n_gamma : 0;
+    return launch_norm_rows(r, st);
+  }
   if (n <= FAITHFUL_FROM && use_sweeps(batch, n)) {
     RowParams p{};
     p.x = x; p.y = y; p.rows = batch; p.len = n; p.eps = eps; p.gamma = gamma; p.n_gamma = gamma ? n_gamma : 0;
@@ -1366,6 +1196,11 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
 
 int launch_softmax(const float* x, float* y, int batch, int64_t n, int log_softmax, cudaStream_t st) {
   if (batch <= 0 || n <= 0) return fail(MIMIR_B200_E_INVALID, "Softmax: empty input");
+  if (norm_rows_on() && norm_rows_supported(batch, n)) {
+    RowNormArgs r;
+    r.family = ROWS_SOFTMAX; r.x = x; r.y = y; r.rows = batch; r.len = n; r.log_softmax = log_softmax;
+    return launch_norm_rows(r, st);
+  }
   if (use_sweeps(batch, n)) {
     RowParams p{};
     p.x = x; p.y = y; p.rows = batch; p.len = n; p.log_softmax = log_softmax;
