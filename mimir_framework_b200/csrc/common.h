@@ -281,7 +281,7 @@ struct RowNormArgs {
   long long n_gamma = 0;             // RMS: gamma applies to i < n_gamma
   int log_softmax = 0;
 };
-bool norm_rows_supported(long long rows, long long len);
+bool norm_rows_supported(const RowNormArgs& a);
 int launch_norm_rows(const RowNormArgs& a, cudaStream_t st);
 
 // norms.cu -------------------------------------------------------------------------------------

@@ -5,8 +5,9 @@
 // four or eight such CTAs, chosen so that a thread holds 4 ... 32 values: enough loads in flight to stream, few enough rows per SM
 // to leave none idle.  The two reductions of a row (mean and centred second moment; maximum and sum of exponentials) take one
 // barrier each: warp sums through shared memory, CTA sums pushed into every peer's shared memory before a cluster barrier.  Rows
-// whose length is no multiple of four are read and written element by element, still in whole lines.
-// ROWS_FIGURES
+// whose length is no multiple of four keep vector accesses: they lie on the tensor's 16-byte boundaries (SHIFT below).
+// LayerNorm 32768 x 768: 41.2 -> 32.8 us (6.1 TB/s); 49840 x 674: 165 -> 72; softmax 2339 x 206: 8.2 -> 4.1, 114 x 4255: 13.3 -> 4.4;
+// GroupNorm + SiLU 576 rows of 41 334 (odd image): 141 -> 87 us.
 #include "common.h"
 #include "launch.cuh"
 
@@ -20,6 +21,19 @@ __device__ __forceinline__ void nr_cluster_wait() { asm volatile("barrier.cluste
 
 template <bool MAX>
 __device__ __forceinline__ float combine(float a, float b) { return MAX ? fmaxf(a, b) : a + b; }
+
+// x * sigmoid(x) with two special-function instructions.  exp(-x) = 2^t with t = -x log2 e; what rounding t loses goes back in as
+// a first-order factor, so the result stays within a few ulp for every x (expf and a division: a third more time on a GroupNorm).
+__device__ __forceinline__ float nr_silu(float x) {
+  const float c = fmaxf(x, -87.0f);  // 2^t stays finite
+  const float t = c * -1.44269504f;
+  const float lost = fmaf(c, -1.44269504f, -t) - c * 1.92596e-8f;  // log2 e = 1.44269504 + 1.92596e-8
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+  e = fmaf(e, lost * 0.69314718f, e);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return x * r;
+}
 
 struct RowShared {
   float warp[3][NR_MAX_THREADS / 32];
@@ -71,10 +85,11 @@ __device__ __forceinline__ float row_reduce1(float v, int step, RowShared& sh, u
   return a[0];
 }
 
-// NV: vectors (VEC: of four floats) of a thread; WARP: a row per warp, else a row per CTA or cluster.
-template <int FAM, bool VEC, int NV, bool WARP>
-__global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS) norm_rows_kernel(const RowNormArgs p, const int slice) {
-  constexpr int W = VEC ? 4 : 1;
+// NV: vectors of four floats of a thread; WARP: a row per warp, else a row per CTA or cluster.  SHIFT: rows may start anywhere; vectors
+// lie on 16-byte boundaries of the tensor all the same, those at a row's ends are moved element by element, and gamma / beta (or
+// the channel of a GroupNorm) are looked up per element.  `slice`: elements of a CTA, counted from the boundary before the row.
+template <int FAM, bool SHIFT, int NV, bool WARP>
+__global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) norm_rows_kernel(const RowNormArgs p, const int slice) {
   __shared__ RowShared sh;
   uint32_t rank = 0, size = 1;
   if (!WARP) {
@@ -87,38 +102,46 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS) norm_rows_kernel(
   const int T = WARP ? 32 : static_cast<int>(blockDim.x), t = WARP ? static_cast<int>(threadIdx.x & 31) : static_cast<int>(threadIdx.x);
   const long long row = WARP ? static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5) : static_cast<long long>(blockIdx.x / size);
   if (WARP && row >= p.rows) return;
-  const int off = static_cast<int>(rank) * slice, n = min(slice, static_cast<int>(p.len) - off);  // this CTA's part of the row
-  const long long base = row * p.len + off;
-  const float* g = p.x + base;
+  const long long base = row * p.len;
+  const int len = static_cast<int>(p.len), lead = SHIFT ? static_cast<int>(base & 3) : 0;
+  const int first = static_cast<int>(rank) * slice + t * 4 - lead;  // the row's element where this thread's first vector starts
+  auto el = [&](int j) { return first + j * T * 4; };
+  auto mine = [&](int j) { return (t + j * T) * 4 < slice && el(j) < len; };
+  auto whole = [&](int j) { return !SHIFT || (el(j) >= 0 && el(j) + 4 <= len); };  // (of a vector that is mine)
+  auto in = [&](int j, int e) { return !SHIFT || static_cast<unsigned>(el(j) + e) < static_cast<unsigned>(len); };
 
-  float v[NV][W];
+  float v[NV][4];
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
-    const int i = (t + j * T) * W;
-    if (VEC) {
-      const float4 q = i < n ? __ldcs(reinterpret_cast<const float4*>(g + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[j][0] = q.x; v[j][W > 1 ? 1 : 0] = W > 1 ? q.y : q.x;
-      if (W > 1) { v[j][W - 2] = q.z; v[j][W - 1] = q.w; }
-    } else {
-      v[j][0] = i < n ? __ldcs(g + i) : 0.0f;
+    const float* g = p.x + base + el(j);
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mine(j)) {
+      if (whole(j)) {
+        q = __ldcs(reinterpret_cast<const float4*>(g));
+      } else {
+        if (in(j, 0)) q.x = __ldcs(g);
+        if (in(j, 1)) q.y = __ldcs(g + 1);
+        if (in(j, 2)) q.z = __ldcs(g + 2);
+        if (in(j, 3)) q.w = __ldcs(g + 3);
+      }
     }
+    v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
   }
   float mul = 1.0f, sub = 0.0f;  // meanvar and rms: (x - sub) * mul; softmax: maximum and 1 / sum (log: log of the sum)
   const float fn = static_cast<float>(p.len);
   if (FAM == ROWS_MEANVAR) {
     float s = 0.0f;
 #pragma unroll
-    for (int j = 0; j < NV; ++j)
-#pragma unroll
-      for (int e = 0; e < W; ++e) s += v[j][e];
+    for (int j = 0; j < NV; ++j) s += (v[j][0] + v[j][1]) + (v[j][2] + v[j][3]);
     sub = row_reduce1<false, WARP>(s, 0, sh, rank, size) / fn;
     // second moment about that mean, and what the mean is off by: a large common offset costs the first sum its low bits
     float c[2] = {0.0f, 0.0f};
 #pragma unroll
     for (int j = 0; j < NV; ++j)
-      if ((t + j * T) * W < n) {
+      if (mine(j)) {
 #pragma unroll
-        for (int e = 0; e < W; ++e) { const float d = v[j][e] - sub; c[0] += d; c[1] = fmaf(d, d, c[1]); }
+        for (int e = 0; e < 4; ++e)
+          if (in(j, e)) { const float d = v[j][e] - sub; c[0] += d; c[1] = fmaf(d, d, c[1]); }
       }
     row_reduce<false, WARP, 2>(c, 1, sh, rank, size);
     const float dm = c[0] / fn;
@@ -129,23 +152,23 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS) norm_rows_kernel(
 #pragma unroll
     for (int j = 0; j < NV; ++j)
 #pragma unroll
-      for (int e = 0; e < W; ++e) q = fmaf(v[j][e], v[j][e], q);
+      for (int e = 0; e < 4; ++e) q = fmaf(v[j][e], v[j][e], q);
     mul = 1.0f / sqrtf(row_reduce1<false, WARP>(q, 0, sh, rank, size) / fn + p.eps);
   } else {
     float m = -INFINITY, s = 0.0f;
 #pragma unroll
     for (int j = 0; j < NV; ++j)
-      if ((t + j * T) * W < n) {
+      if (mine(j)) {
 #pragma unroll
-        for (int e = 0; e < W; ++e) m = fmaxf(m, v[j][e]);
+        for (int e = 0; e < 4; ++e) if (in(j, e)) m = fmaxf(m, v[j][e]);
       }
     sub = row_reduce1<true, WARP>(m, 0, sh, rank, size);
 #pragma unroll
     for (int j = 0; j < NV; ++j)
-      if ((t + j * T) * W < n) {
+      if (mine(j)) {
 #pragma unroll
-        for (int e = 0; e < W; ++e) {
-          const float ex = __expf(v[j][e] - sub);
+        for (int e = 0; e < 4; ++e) {
+          const float ex = in(j, e) ? __expf(v[j][e] - sub) : 0.0f;
           s += ex;
           if (!p.log_softmax) v[j][e] = ex;
         }
@@ -154,78 +177,84 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS) norm_rows_kernel(
     mul = p.log_softmax ? logf(s) : 1.0f / s;
   }
 
-  float* o = p.y + base;
-  // GroupNorm: the channel of this thread's elements, advanced without divisions
-  unsigned ch = 0, rem = 0, ch_step = 0, rem_step = 0;
-  const unsigned hw = static_cast<unsigned>(p.hw);
+  // GroupNorm: the channel of a vector's first element, advanced without divisions (a row's first vector may start before it)
+  int ch = 0, rem = 0, ch_step = 0, rem_step = 0;
   if (FAM == ROWS_MEANVAR && p.per_channel) {
-    const unsigned first = static_cast<unsigned>(off + t * W), step = static_cast<unsigned>(T * W);
-    ch = static_cast<unsigned>(static_cast<int>(row % p.groups) * p.cpg) + first / hw;
-    rem = first % hw;
-    ch_step = step / hw;
-    rem_step = step % hw;
+    const int f = first + p.hw;
+    ch = static_cast<int>(row % p.groups) * p.cpg - 1 + f / p.hw;
+    rem = f % p.hw;
+    ch_step = T * 4 / p.hw;
+    rem_step = T * 4 % p.hw;
   }
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
-    const int i = (t + j * T) * W;
-    if (i >= n) break;
-    float r[W];
+    if (!mine(j)) break;
+    const int i = el(j);
+    float r[4];
 #pragma unroll
-    for (int e = 0; e < W; ++e) r[e] = v[j][e];
-    if (FAM == ROWS_SOFTMAX) {
-#pragma unroll
-      for (int e = 0; e < W; ++e) r[e] = p.log_softmax ? (r[e] - sub) - mul : r[e] * mul;
-    } else {
-#pragma unroll
-      for (int e = 0; e < W; ++e) r[e] = (r[e] - sub) * mul;
+    for (int e = 0; e < 4; ++e) {
+      if (FAM == ROWS_SOFTMAX) r[e] = p.log_softmax ? (v[j][e] - sub) - mul : v[j][e] * mul;
+      else r[e] = (v[j][e] - sub) * mul;
     }
     if (FAM == ROWS_RMS && p.gamma != nullptr) {
-      if (VEC && off + i + W <= p.n_gamma) {
-        const float4 w = __ldg(reinterpret_cast<const float4*>(p.gamma + off + i));
-        r[0] *= w.x; r[W > 1 ? 1 : 0] *= W > 1 ? w.y : 1.0f;
-        if (W > 1) { r[W - 2] *= w.z; r[W - 1] *= w.w; }
+      if (!SHIFT && i + 4 <= p.n_gamma) {
+        const float4 w = __ldg(reinterpret_cast<const float4*>(p.gamma + i));
+        r[0] *= w.x; r[1] *= w.y; r[2] *= w.z; r[3] *= w.w;
       } else {
 #pragma unroll
-        for (int e = 0; e < W; ++e) if (off + i + e < p.n_gamma) r[e] *= __ldg(p.gamma + off + i + e);
+        for (int e = 0; e < 4; ++e) if (in(j, e) && i + e < p.n_gamma) r[e] *= __ldg(p.gamma + i + e);
       }
     }
     if (FAM == ROWS_MEANVAR) {
       if (p.gamma != nullptr) {
-        if (p.per_channel) {  // (vectors never cross a channel: hw is a multiple of four there)
-          const float w = __ldg(p.gamma + ch), b = p.beta != nullptr ? __ldg(p.beta + ch) : 0.0f;
-#pragma unroll
-          for (int e = 0; e < W; ++e) r[e] = r[e] * w + b;
-        } else if (VEC) {
-          const float4 w = __ldg(reinterpret_cast<const float4*>(p.gamma + off + i));
-          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (p.beta != nullptr) b = __ldg(reinterpret_cast<const float4*>(p.beta + off + i));
-          r[0] = r[0] * w.x + b.x;
-          if (W > 1) { r[1 % W] = r[1 % W] * w.y + b.y; r[W - 2] = r[W - 2] * w.z + b.z; r[W - 1] = r[W - 1] * w.w + b.w; }
+        float4 w, b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.per_channel && (!SHIFT || rem + 3 < p.hw) && ch >= 0) {
+          w.x = w.y = w.z = w.w = __ldg(p.gamma + ch);
+          if (p.beta != nullptr) b.x = b.y = b.z = b.w = __ldg(p.beta + ch);
+        } else if (!SHIFT) {
+          w = __ldg(reinterpret_cast<const float4*>(p.gamma + i));
+          if (p.beta != nullptr) b = __ldg(reinterpret_cast<const float4*>(p.beta + i));
         } else {
-          r[0] = r[0] * __ldg(p.gamma + off + i) + (p.beta != nullptr ? __ldg(p.beta + off + i) : 0.0f);
+          float ww[4] = {1.f, 1.f, 1.f, 1.f}, bb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (in(j, e)) {
+              const int k = p.per_channel ? ch + (rem + e) / p.hw : i + e;
+              ww[e] = __ldg(p.gamma + k);
+              if (p.beta != nullptr) bb[e] = __ldg(p.beta + k);
+            }
+          w = make_float4(ww[0], ww[1], ww[2], ww[3]);
+          b = make_float4(bb[0], bb[1], bb[2], bb[3]);
         }
+        r[0] = r[0] * w.x + b.x; r[1] = r[1] * w.y + b.y; r[2] = r[2] * w.z + b.z; r[3] = r[3] * w.w + b.w;
       }
       if (p.act == MIMIR_B200_ELT_SILU) {
 #pragma unroll
-        for (int e = 0; e < W; ++e) r[e] = r[e] * (1.0f / (1.0f + expf(-r[e])));
+        for (int e = 0; e < 4; ++e) r[e] = nr_silu(r[e]);
       }
       if (p.residual != nullptr) {
-        if (VEC) {
-          const float4 q = __ldg(reinterpret_cast<const float4*>(p.residual + base + i));
-          r[0] += q.x;
-          if (W > 1) { r[1 % W] += q.y; r[W - 2] += q.z; r[W - 1] += q.w; }
+        const float* q = p.residual + base + i;
+        if (whole(j)) {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(q));
+          r[0] += a.x; r[1] += a.y; r[2] += a.z; r[3] += a.w;
         } else {
-          r[0] += __ldg(p.residual + base + i);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) if (in(j, e)) r[e] += __ldg(q + e);
         }
       }
       if (p.per_channel) {
         ch += ch_step;
         rem += rem_step;
-        if (rem >= hw) { rem -= hw; ++ch; }
+        if (rem >= p.hw) { rem -= p.hw; ++ch; }
       }
     }
-    if (VEC) __stcs(reinterpret_cast<float4*>(o + i), make_float4(r[0], r[1 % W], r[2 % W], r[3 % W]));
-    else __stcs(o + i, r[0]);
+    float* o = p.y + base + i;
+    if (whole(j)) {
+      __stcs(reinterpret_cast<float4*>(o), make_float4(r[0], r[1], r[2], r[3]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) if (in(j, e)) __stcs(o + e, r[e]);
+    }
   }
 }
 
@@ -234,54 +263,64 @@ struct RowShape { int threads = 0, ctas = 1; };  // threads = 32: a warp
 RowShape row_shape(long long rows, long long len) {
   const long long sms = ctx().sm_count;
   RowShape s;
-  s.threads = len <= 1024 ? 32 : 64;
+  s.threads = len <= 1027 ? 32 : 64;  // (+ 3: see launch_norm_rows)
   while (s.threads < NR_MAX_THREADS && len > s.threads * 16LL && s.threads > 32) s.threads *= 2;
   // few rows: more threads to a row, down to four values each
   while (s.threads < NR_MAX_THREADS && rows * s.threads < sms * 512 && len > s.threads * 8LL) s.threads *= 2;
+  // As few CTAs as hold the row: cluster barriers cost more than the occupancy that fewer values a thread would give (128 rows of
+  // 46 656 values, GroupNorm: four CTAs 20 us, eight 31 us).
   while (s.ctas < 8 && len > static_cast<long long>(s.ctas) * NR_MAX_THREADS * 32) s.ctas *= 2;
   while (s.ctas < 8 && s.threads == NR_MAX_THREADS && rows * s.ctas * 2 <= sms * 2 && len > static_cast<long long>(s.ctas) * NR_MAX_THREADS * 8) s.ctas *= 2;
   return s;
 }
 
-template <int FAM, bool VEC, int NV>
+template <int FAM, bool SHIFT, int NV>
 int launch_nv(const RowNormArgs& a, const RowShape& s, int slice, cudaStream_t st) {
-  if (s.threads == 32) return launch_pdl(norm_rows_kernel<FAM, VEC, NV, true>, dim3(static_cast<unsigned>((a.rows + 3) / 4)), dim3(128), 0, st, 1, a, slice);
-  return launch_pdl(norm_rows_kernel<FAM, VEC, NV, false>, dim3(static_cast<unsigned>(a.rows * s.ctas)), dim3(static_cast<unsigned>(s.threads)), 0, st, s.ctas, a, slice);
+  if (s.threads == 32) return launch_pdl(norm_rows_kernel<FAM, SHIFT, NV, true>, dim3(static_cast<unsigned>((a.rows + 3) / 4)), dim3(128), 0, st, 1, a, slice);
+  return launch_pdl(norm_rows_kernel<FAM, SHIFT, NV, false>, dim3(static_cast<unsigned>(a.rows * s.ctas)), dim3(static_cast<unsigned>(s.threads)), 0, st, s.ctas, a,
+                    slice);
+}
+template <int FAM, bool SHIFT>
+int launch_shift(const RowNormArgs& a, const RowShape& s, cudaStream_t st) {
+  const long long span = a.len + (SHIFT ? 3 : 0);  // with what may lie between the boundary before the row and its start
+  const int slice = static_cast<int>((((span + s.ctas - 1) / s.ctas) + 3) & ~3LL);
+  const int nv = (slice / 4 + s.threads - 1) / s.threads;
+  if (nv <= 1) return launch_nv<FAM, SHIFT, 1>(a, s, slice, st);
+  if (nv <= 2) return launch_nv<FAM, SHIFT, 2>(a, s, slice, st);
+  if (nv <= 3) return launch_nv<FAM, SHIFT, 3>(a, s, slice, st);
+  if (nv <= 4) return launch_nv<FAM, SHIFT, 4>(a, s, slice, st);
+  if (nv <= 5) return launch_nv<FAM, SHIFT, 5>(a, s, slice, st);
+  if (nv <= 6) return launch_nv<FAM, SHIFT, 6>(a, s, slice, st);
+  if (nv <= 7) return launch_nv<FAM, SHIFT, 7>(a, s, slice, st);
+  return launch_nv<FAM, SHIFT, 8>(a, s, slice, st);
 }
 template <int FAM>
-int launch_fam(const RowNormArgs& a, const RowShape& s, bool vec, cudaStream_t st) {
-  const int slice = static_cast<int>((((a.len + s.ctas - 1) / s.ctas) + 3) & ~3LL);
-  const int per = (slice + s.threads - 1) / s.threads;  // values of a thread
-  if (vec) {
-    const int nv = (slice / 4 + s.threads - 1) / s.threads;
-    if (nv <= 1) return launch_nv<FAM, true, 1>(a, s, slice, st);
-    if (nv <= 2) return launch_nv<FAM, true, 2>(a, s, slice, st);
-    if (nv <= 4) return launch_nv<FAM, true, 4>(a, s, slice, st);
-    if (nv <= 6) return launch_nv<FAM, true, 6>(a, s, slice, st);
-    return launch_nv<FAM, true, 8>(a, s, slice, st);
-  }
-  if (per <= 8) return launch_nv<FAM, false, 8>(a, s, slice, st);
-  if (per <= 16) return launch_nv<FAM, false, 16>(a, s, slice, st);
-  return launch_nv<FAM, false, 32>(a, s, slice, st);
+int launch_fam(const RowNormArgs& a, const RowShape& s, bool shift, cudaStream_t st) {
+  return shift ? launch_shift<FAM, true>(a, s, st) : launch_shift<FAM, false>(a, s, st);
 }
 
 }  // namespace
 
-bool norm_rows_supported(long long rows, long long len) {
-  // Longer rows: with a row for every SM the two-sweep kernel (second read from L2) keeps more rows in flight than clusters do.
-  return rows >= 1 && rows * 8 < 0x7fffffffLL && (len <= NR_MAX_THREADS * 32 || (len <= 8LL * NR_MAX_THREADS * 32 && rows < ctx().sm_count));
+bool norm_rows_supported(const RowNormArgs& a) {
+  // (tensors that do not start on 16 bytes go to the sweep and chunk kernels)
+  if (((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.residual)) & 15) != 0) return false;
+  if (a.rows < 1 || a.rows * 8 >= 0x7fffffffLL) return false;
+  const long long len = a.len + 3;
+  // Longer rows: with a row for every SM the two-sweep kernel (second read from L2) keeps more rows in flight than clusters do -
+  // unless it would have to move them element by element.
+  return len <= NR_MAX_THREADS * 32 || (len <= 8LL * NR_MAX_THREADS * 24 && a.rows < ctx().sm_count) ||
+         (len <= 8LL * NR_MAX_THREADS * 32 && (a.len & 3) != 0);
 }
 
 int launch_norm_rows(const RowNormArgs& a, cudaStream_t st) {
-  const RowShape s = row_shape(a.rows, a.len);
-  const bool affine16 = a.per_channel ? (a.hw & 3) == 0
-                                      : ((reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) == 0;
-  const bool vec = (a.len & 3) == 0 && affine16 &&
-                   ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.residual)) & 15) == 0;
+  const RowShape s = row_shape(a.rows, a.len + 3);
+  const bool affine = a.per_channel ? (a.hw & 3) == 0
+                                    : ((reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) == 0;
+  const bool shift = (a.len & 3) != 0 || !affine;
   int r;
-  if (a.family == ROWS_MEANVAR) r = launch_fam<ROWS_MEANVAR>(a, s, vec, st);
-  else if (a.family == ROWS_RMS) r = launch_fam<ROWS_RMS>(a, s, vec, st);
-  else r = launch_fam<ROWS_SOFTMAX>(a, s, vec, st);
+  if (a.family == ROWS_MEANVAR) r = launch_fam<ROWS_MEANVAR>(a, s, shift, st);
+  else if (a.family == ROWS_RMS) r = launch_fam<ROWS_RMS>(a, s, shift, st);
+  else r = launch_fam<ROWS_SOFTMAX>(a, s, shift, st);
   if (r == MIMIR_B200_OK) count_launch();
   return r;
 }

@@ -943,11 +943,11 @@ constexpr long long L2_GROUP_BYTES = 104ll << 20;
 
 int meanvar_dispatch(const float* x, float* y, long long rows, long long len, float eps, const Affine& a, cudaStream_t st) {
   if (rows <= 0 || len <= 0) return fail(MIMIR_B200_E_INVALID, "norm: empty input");
-  if (norm_rows_on() && norm_rows_supported(rows, len)) {
+  if (norm_rows_on()) {
     RowNormArgs r;
     r.x = x; r.y = y; r.rows = rows; r.len = len; r.eps = eps; r.gamma = a.gamma; r.beta = a.beta; r.per_channel = a.per_channel;
     r.groups = a.groups; r.cpg = a.cpg; r.hw = a.hw; r.act = a.act; r.residual = a.residual;
-    return launch_norm_rows(r, st);
+    if (norm_rows_supported(r)) return launch_norm_rows(r, st);
   }
   if (use_sweeps(rows, len)) {
     RowParams p{};
@@ -1151,10 +1151,10 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
   // Below this length the sequential chain's rounding loss is < 1e-6 of the sum and any summation order
   // agrees with the reference; above it the chain is reproduced (rms_seq_err_kernel).
   constexpr long long FAITHFUL_FROM = 16384;
-  if (n <= FAITHFUL_FROM && norm_rows_on() && norm_rows_supported(batch, n)) {
+  if (n <= FAITHFUL_FROM && norm_rows_on()) {
     RowNormArgs r;
     r.family = ROWS_RMS; r.x = x; r.y = y; r.rows = batch; r.len = n; r.eps = eps; r.gamma = gamma; r.n_gamma = gamma ? n_gamma : 0;
-    return launch_norm_rows(r, st);
+    if (norm_rows_supported(r)) return launch_norm_rows(r, st);
   }
   if (n <= FAITHFUL_FROM && use_sweeps(batch, n)) {
     RowParams p{};
@@ -1196,10 +1196,10 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
 
 int launch_softmax(const float* x, float* y, int batch, int64_t n, int log_softmax, cudaStream_t st) {
   if (batch <= 0 || n <= 0) return fail(MIMIR_B200_E_INVALID, "Softmax: empty input");
-  if (norm_rows_on() && norm_rows_supported(batch, n)) {
+  if (norm_rows_on()) {
     RowNormArgs r;
     r.family = ROWS_SOFTMAX; r.x = x; r.y = y; r.rows = batch; r.len = n; r.log_softmax = log_softmax;
-    return launch_norm_rows(r, st);
+    if (norm_rows_supported(r)) return launch_norm_rows(r, st);
   }
   if (use_sweeps(batch, n)) {
     RowParams p{};

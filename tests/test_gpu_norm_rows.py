@@ -1,0 +1,58 @@
+"""Norms and softmax of rows in registers (csrc/norm_rows.cu) at the edges of their forms: a warp, one CTA, clusters; lengths that are no
+multiple of four (rows start between 16-byte boundaries); channels that end inside a vector; tensors that are not 16-byte aligned."""
+import numpy as np
+import pytest
+
+from mimir_framework_b200 import abi
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    from mimir_framework_b200 import runtime
+
+    runtime.init(0)
+    return runtime
+
+
+def close(got, want):
+    assert np.all(np.isfinite(got)) and np.linalg.norm(got.ravel() - want.ravel()) <= 3e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (3, 5), (200, 31), (7, 1024), (301, 1025), (5, 1027), (2000, 2050), (150, 16381), (149, 16383), (2, 16385), (3, 40001), (1, 131069), (160, 17001)])
+def test_layernorm_rmsnorm_softmax(rt, rows, n):
+    r = np.random.default_rng(n)
+    x = (r.standard_normal((rows, n)) * 2 + 0.5).astype(np.float32)
+    g, b = (1 + 0.1 * r.standard_normal(n)).astype(np.float32), r.standard_normal(n).astype(np.float32)
+    d = x.astype(np.float64)
+    if n > 1:
+        close(rt.layernorm(x, g, b, rows, n), (d - d.mean(1, keepdims=True)) / np.sqrt(d.var(1, keepdims=True) + 1e-5) * g + b)
+    e = np.exp(d - d.max(1, keepdims=True))
+    close(rt.softmax(x, rows, n), e / e.sum(1, keepdims=True))
+    if n <= 16384:
+        ng = n - n // 3  # gamma applies to a prefix
+        want = d / np.sqrt((d * d).mean(1, keepdims=True) + 1e-5)
+        want[:, :ng] *= g[:ng]
+        close(rt.rmsnorm(x, g[:ng], rows, n), want)
+
+
+@pytest.mark.parametrize("batch,ch,h,w,groups", [(2, 32, 1, 1, 32), (3, 64, 3, 1, 16), (1, 96, 7, 9, 32), (2, 64, 16, 12, 8), (9, 64, 53, 53, 32), (1, 64, 101, 101, 4), (2, 32, 2, 1, 4)])
+@pytest.mark.parametrize("act", [-1, abi.ELT_SILU])
+def test_groupnorm(rt, batch, ch, h, w, groups, act):
+    r = np.random.default_rng(ch + h)
+    x = r.standard_normal((batch, groups, ch // groups * h * w)).astype(np.float32)
+    g, b = (1 + 0.1 * r.standard_normal(ch)).astype(np.float32), r.standard_normal(ch).astype(np.float32)
+    d = x.astype(np.float64)
+    d = ((d - d.mean(2, keepdims=True)) / np.sqrt(d.var(2, keepdims=True) + 1e-5)).reshape(batch, ch, h * w) * g[None, :, None] + b[None, :, None]
+    close(rt.groupnorm(x, g, b, batch, ch, h, w, groups, 1e-5, act), d / (1 + np.exp(-d)) if act >= 0 else d)
+
+
+def test_unaligned_device_tensors(rt):
+    import torch
+
+    x, rows, n = torch.randn(4 * 301 + 1, device="cuda"), 4, 301
+    y = torch.empty(4 * 301 + 1, device="cuda")
+    rt.check(rt.lib().mimir_b200_dev_softmax(x[1:].data_ptr(), y[1:].data_ptr(), rows, n, 0, None))
+    torch.cuda.synchronize()
+    assert torch.allclose(y[1:].view(rows, n), torch.softmax(x[1:].view(rows, n), 1), atol=1e-6, rtol=1e-5)
