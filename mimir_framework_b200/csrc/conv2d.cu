@@ -10,6 +10,19 @@
 namespace mb {
 namespace {
 
+__device__ __forceinline__ void cp_async16_zfill(void* smem_dst, const void* gmem_src, bool valid) {
+  // 16 bytes, or 16 zero bytes when !valid (source size 0: nothing is read)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
+               "l"(gmem_src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+
+__device__ __forceinline__ void cp_async4_zfill(void* smem_dst, const void* gmem_src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
+               "l"(gmem_src), "r"(valid ? 4 : 0)
+               : "memory");
+}
+
 // One thread produces 8 consecutive K entries of one output pixel.
 __global__ void im2col_split_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst, long long rows, int ic, int h,
                                     int w, int ks, int stride, int pad, int oh, int ow, int k, int kp, int planes, int f16) {
@@ -52,54 +65,64 @@ __global__ void im2col_split_kernel(const float* __restrict__ x, __nv_bfloat16* 
   }
 }
 
-// The same rows from a staged input patch: a CTA owns I2C_TPX consecutive output pixels of one output row and a block of
-// `cb` input channels (a multiple of 8, or all of them), loads the patch those pixels read - cb x ks rows of
-// (I2C_TPX - 1) * stride + ks input pixels, coalesced - into shared memory once, and assembles the 16-byte chunks of its K
-// range from there (consecutive threads: consecutive chunks of one pixel, i.e. contiguous stores).  The input is read
-// once per channel block instead of once per K entry through the caches, and the index arithmetic is per chunk.
-constexpr int I2C_TPX = 32;
-
+// The same rows from a staged input patch: a CTA owns `tpx` consecutive output pixels of one output row and a block of `cb` input
+// channels (a multiple of 8, or all of them), loads the patch those pixels read - cb x ks rows of (tpx - 1) * stride + ks input
+// pixels, coalesced, a warp per row - into shared memory once, and assembles the 16-byte chunks of its K range from there.  A thread
+// keeps one chunk of the K range and walks the pixels, so the eight places of the patch a chunk reads are worked out once; consecutive
+// threads hold consecutive chunks of one pixel, i.e. contiguous stores.
+// (With the index arithmetic done per chunk and pixel the kernel was bound by it: 16 x 512 x 64^2, 3 x 3 stride 2: 208 us for 302 MB
+// written; now 118 us.  64 x 3 x 224^2, 7 x 7 stride 2: 310 us, now 129 us.)
+// KS: the kernel size, 0 = any (then `ks_any`).
+template <int KS>
 __global__ void __launch_bounds__(256) im2col_tile_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ dst, long long rows,
-                                                          int ic, int h, int w, int ks, int stride, int pad, int oh, int ow, int k,
-                                                          int kp, int planes, int f16, int cb, int nblocks) {
-  extern __shared__ float patch[];  // [cbn][ks][pw]
-  const int ox0 = blockIdx.x * I2C_TPX, oy = blockIdx.y;
+                                                          int ic, int h, int w, int ks_any, int stride, int pad, int oh, int ow, int kp,
+                                                          int planes, int f16, int cb, int nblocks, int tpx) {
+  extern __shared__ float patch[];  // [cbn][ks][pw], then one zero
+  const int ks = KS ? KS : ks_any, kk = ks * ks;
+  const int ox0 = blockIdx.x * tpx, oy = blockIdx.y;
   const int smp = blockIdx.z / nblocks, blk = blockIdx.z - smp * nblocks;
   const int c0 = blk * cb, cbn = min(cb, ic - c0);
-  const int kk = ks * ks, pw = (I2C_TPX - 1) * stride + ks;
+  const int pw = (tpx - 1) * stride + ks;
   const int iy0 = oy * stride - pad, ix0 = ox0 * stride - pad;
   const float* xs = x + (static_cast<long long>(smp) * ic + c0) * h * w;
-  for (int i = threadIdx.x; i < cbn * ks * pw; i += 256) {
-    const int c = i / (ks * pw), r = i - c * (ks * pw);
-    const int ky = r / pw, px = r - ky * pw;
-    const int iy = iy0 + ky, ix = ix0 + px;
-    patch[i] = (iy >= 0 && iy < h && ix >= 0 && ix < w) ? __ldg(xs + (static_cast<long long>(c) * h + iy) * w + ix) : 0.0f;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < cbn * ks; r += 8) {
+    const int c = r / ks, iy = iy0 + r - c * ks;
+    const float* line = xs + (static_cast<long long>(c) * h + iy) * w;
+    const bool row_in = iy >= 0 && iy < h;
+    for (int px = lane; px < pw; px += 32) {
+      const int ix = ix0 + px;
+      const bool ok = row_in && ix >= 0 && ix < w;  // (asynchronous: a warp's rows are all in flight at once)
+      cp_async4_zfill(&patch[r * pw + px], ok ? line + ix : x, ok);
+    }
   }
+  if (threadIdx.x == 0) patch[cbn * ks * pw] = 0.0f;
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   // this block's chunks of a row: its channels' K range; the last block also writes the zero padding up to kp
   const int ch_lo = (c0 * kk) >> 3, ch_hi = (blk == nblocks - 1) ? (kp >> 3) : (((c0 + cbn) * kk) >> 3);
-  const int nch = ch_hi - ch_lo, npx = min(I2C_TPX, ow - ox0);
+  const int nch = ch_hi - ch_lo, npx = min(tpx, ow - ox0);
+  const int groups = nch < 256 ? 256 / nch : 1;  // pixels the CTA works on at once
+  const int g = nch < 256 ? static_cast<int>(threadIdx.x) / nch : 0;
   const long long plane_stride = rows * static_cast<long long>(kp);
   const long long row0 = (static_cast<long long>(smp) * oh + oy) * ow + ox0;
-  for (int item = threadIdx.x; item < npx * nch; item += 256) {
-    const int p = item / nch, chunk = ch_lo + (item - p * nch);
-    const int kidx0 = chunk * 8 - c0 * kk;  // relative to this block's first channel
-    int ci = kidx0 / kk, t = kidx0 - ci * kk;
-    int ky = t / ks, kx = t - ky * ks;
-    __align__(16) uint16_t hi[8];
-    __align__(16) uint16_t lo[8];
+  if (g >= groups) return;
+  for (int chunk = static_cast<int>(threadIdx.x) - g * nch; chunk < nch; chunk += 256) {
+    int off[8], step[8];  // where the chunk's elements of pixel 0 are, and how far the next pixel's (0: the zero past the last channel)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float v = (ci < cbn) ? patch[(ci * ks + ky) * pw + p * stride + kx] : 0.0f;  // past the last channel: K padding
-      split_one(v, f16, hi[j], lo[j]);
-      if (++kx == ks) {
-        kx = 0;
-        if (++ky == ks) { ky = 0; ++ci; }
-      }
+      const int kidx = (ch_lo + chunk) * 8 + j - c0 * kk, ci = kidx / kk, t = kidx - ci * kk, ky = t / ks;
+      off[j] = ci < cbn ? (ci * ks + ky) * pw + t - ky * ks : cbn * ks * pw;
+      step[j] = ci < cbn ? stride : 0;
     }
-    __nv_bfloat16* d = dst + (row0 + p) * kp + chunk * 8;
-    *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(hi);
-    if (planes == 2) *reinterpret_cast<uint4*>(d + plane_stride) = *reinterpret_cast<const uint4*>(lo);
+    for (int p = g; p < npx; p += groups) {
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) split_pair(patch[off[j] + p * step[j]], patch[off[j + 1] + p * step[j + 1]], f16, hi[j >> 1], lo[j >> 1]);
+      __nv_bfloat16* d = dst + (row0 + p) * kp + (ch_lo + chunk) * 8;
+      *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      if (planes == 2) *reinterpret_cast<uint4*>(d + plane_stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
   }
 }
 
@@ -114,15 +137,20 @@ int launch_im2col_split(const float* x, __nv_bfloat16* dst, int batch, int ic, i
   {
     // the staged form: channel blocks of a multiple of 8 (so that every block starts on a chunk boundary) within 48 KB
     static const bool off = [] { const char* e = getenv("MIMIR_B200_IM2COL_TILED"); return e && e[0] == '0'; }();
-    const int pw = (I2C_TPX - 1) * stride + ks;
+    // about 64 pixels of a row, evenly cut; patches of 28 KB: several CTAs to an SM, one's loads beside another's stores
+    const int cuts = (ow + 63) / 64, tpx = (ow + cuts - 1) / cuts;
+    const int pw = (tpx - 1) * stride + ks;
     const long long per_ch = static_cast<long long>(ks) * pw * 4;
-    int cb = static_cast<int>(std::min<long long>(ic, (48 * 1024) / per_ch));
+    int cb = static_cast<int>(std::min<long long>(ic, (28 * 1024) / per_ch));
+    if (cb < ic) cb &= ~7;
+    if (cb == 0) cb = static_cast<int>(std::min<long long>(ic, (47 * 1024) / per_ch));
     if (cb < ic) cb &= ~7;
     const int nblocks = cb > 0 ? (ic + cb - 1) / cb : 0;
     if (!off && cb > 0 && static_cast<long long>(batch) * nblocks <= 65535 && oh <= 65535) {
-      dim3 grid((ow + I2C_TPX - 1) / I2C_TPX, oh, batch * nblocks);
-      im2col_tile_kernel<<<grid, 256, static_cast<size_t>(cb) * per_ch, st>>>(x, dst, rows, ic, h, w, ks, stride, pad, oh, ow, k, kp, planes,
-                                                                              plane_format() == PLANES_F16, cb, nblocks);
+      const dim3 grid(cuts, oh, batch * nblocks);
+      auto kern = ks == 3 ? im2col_tile_kernel<3> : ks == 7 ? im2col_tile_kernel<7> : im2col_tile_kernel<0>;
+      kern<<<grid, 256, static_cast<size_t>(cb) * per_ch + 4, st>>>(x, dst, rows, ic, h, w, ks, stride, pad, oh, ow, kp, planes, plane_format() == PLANES_F16, cb,
+                                                                    nblocks, tpx);
       MB_CUDA(cudaGetLastError());
       count_launch();
       return MIMIR_B200_OK;
@@ -149,19 +177,6 @@ namespace mb {
 namespace {
 
 constexpr int TP_C = 64, TP_X = 64;
-
-__device__ __forceinline__ void cp_async16_zfill(void* smem_dst, const void* gmem_src, bool valid) {
-  // 16 bytes, or 16 zero bytes when !valid (source size 0: nothing is read)
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
-               "l"(gmem_src), "r"(valid ? 16 : 0)
-               : "memory");
-}
-
-__device__ __forceinline__ void cp_async4_zfill(void* smem_dst, const void* gmem_src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
-               "l"(gmem_src), "r"(valid ? 4 : 0)
-               : "memory");
-}
 
 // NCHW fp32 -> zero-padded NHWC planes.  A channel plane is read as one line of h * w pixels, so that no tile (64 channels x 64
 // pixels) is cut short at the end of an image row; a CTA owns `tiles_per_cta` consecutive tiles of one sample and 64 channels, and the
