@@ -68,8 +68,9 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
 // Weight of split s's partial sum.  The tensor core adds with truncation, so in ONE accumulator over all of K the contribution of an
 // early range would have shrunk a little with every MMA that came after it.  The weights apply that shrinkage to the ranges that
 // were summed apart, and the result is then scaled as the unsplit kernel's is: a row gives the same answer in a small batch
-// (here) and in a large one (gemm_sm100.cu).  Relative difference of the two kernels at K = 32768, 40 x 1024 outputs, eight
-// splits: 5.8e-5 unweighted, SG_AGREE weighted; at K = 1024 it is below 2e-6 either way.
+// (here) and in a large one (gemm_sm100.cu).  Relative difference of the two kernels' results, 40 x 1024 outputs, eight splits,
+// three MMAs per product: K = 32768 1.0e-4 unweighted, 1e-5 weighted (each is 5.3e-5 from the fp64 product); K = 2048 6.5e-6 and
+// 9e-7.  Fitted: 3e-8 ... 3.2e-8 per MMA at every K and product count.
 __device__ __forceinline__ float split_weight(const SplitGemmParams& p, int s) {
   const int end = static_cast<int>(static_cast<long long>(p.kblocks) * (s + 1) / p.splits);
   return 1.0f - p.shrink * static_cast<float>(p.kblocks - end);
