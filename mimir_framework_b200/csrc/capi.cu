@@ -377,6 +377,22 @@ size_t conv_ws_bytes(int batch, int ic, int h, int w, int ks, int stride, int pa
   return align256(split_bytes(static_cast<int64_t>(conv_chunk_samples(batch, oh * ow, k, precision)) * oh * ow, k, ap));
 }
 
+// A residual that is the 2 x 2 upsample of a smaller image can be read there by the 256-pixel-tile kernel's epilogue.  Only where
+// that kernel has a tile for every SM: below that another form of the convolution may be the faster one by more than the upsample
+// kernel and its tensor cost (a few microseconds at such sizes).
+bool conv_takes_residual_up(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
+  if (!conv_uses_shifted(ic, ks, stride, pad) || ks < 3 || (h | w) % 2 != 0 || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
+  const long long rows = static_cast<long long>(batch) * (h + 2 * pad) * (w + 2 * pad);
+  if (rows > 0x7fffffffLL) return false;
+  GemmArgs g;
+  precision_planes(precision, &g.a_planes, &g.w_planes);
+  float out = 0.0f;
+  g.m = static_cast<int>(rows); g.n = oc; g.k = ic * ks * ks;
+  g.out_f32 = &out;  // (only asked whether there is one)
+  g.conv_ks = ks; g.conv_c = ic; g.conv_pad = pad; g.conv_h = h; g.conv_w = w;
+  return conv_gemm_cycles(g) < 1e30 && conv_gemm_tiles(g) >= ctx().sm_count;
+}
+
 int conv_exec(const ConvExec& e, cudaStream_t st) {
   int ap, wp;
   precision_planes(e.precision, &ap, &wp);
@@ -384,8 +400,9 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
   const int ow = (e.w + 2 * e.pad - e.ks) / e.stride + 1;
   if (oh <= 0 || ow <= 0) return fail(MIMIR_B200_E_INVALID, "Conv2d: empty output");
   const int ohw = oh * ow, k = e.ic * e.ks * e.ks;
+  if (e.residual_up && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: an upsampled residual needs the shifted-GEMM path");
   if (e.in_up && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: an upsampled input needs the shifted-GEMM path");
-  if (e.w_f32 != nullptr && e.pre_groups == 0 && !e.in_up && conv_small_oc_supported(e.oc, e.ks, e.stride, e.pad, e.h, e.w, e.batch, e.activation))
+  if (e.w_f32 != nullptr && e.pre_groups == 0 && !e.in_up && !e.residual_up && conv_small_oc_supported(e.oc, e.ks, e.stride, e.pad, e.h, e.w, e.batch, e.activation))
     return launch_conv_small_oc(e.x, e.w_f32, e.y, e.residual, e.batch, e.ic, e.oc, e.h, e.w, e.ks, e.pad, e.activation, st);
   if (conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) {
     // NCHW fp32 -> zero-padded NHWC planes, then one GEMM that walks the taps as shifted row offsets
@@ -410,6 +427,7 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     g.activation = e.activation;
     g.out_f32 = e.y;
     g.residual = e.residual;
+    g.residual_up = e.residual_up;
     g.ldo = e.oc;
     g.conv_ks = e.ks; g.conv_c = e.ic; g.conv_pad = e.pad; g.conv_h = e.h; g.conv_w = e.w;
     if (e.gn_stats_out != nullptr) {

@@ -170,6 +170,7 @@ struct GemmArgs {
   int m = 0, n = 0, k = 0;           // logical sizes; kp = round_up(k, 64)
   const float* bias = nullptr;       // [n] or null
   const float* residual = nullptr;   // fp32 [m, n] added after the activation, or null
+  bool residual_up = false;          // shifted convolutions (conv_gemm.cu only): the residual is an image of half the size, each value for 2 x 2 pixels
   int activation = -1;
   float* out_f32 = nullptr;          // fp32 [m, ldo] or null
   int64_t ldo = 0;
@@ -206,6 +207,7 @@ double gemm_split_cycles(const GemmArgs& g, int bk, int* bn, int* splits);
 int launch_gemm_split(const GemmArgs& g, int bk, int bn, int splits, cudaStream_t st);
 // conv_gemm.cu: shifted-GEMM convolutions in tiles of 256 pixels
 double conv_gemm_cycles(const GemmArgs& g);
+long long conv_gemm_tiles(const GemmArgs& g);
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st);
 inline size_t gemm_gn_part_bytes(long long m, int n, int cpg) {
   return static_cast<size_t>((m + 31) / 32) * static_cast<size_t>((n + 31) / 32) * static_cast<size_t>(2 * (1 + 64 / cpg)) * sizeof(float);

@@ -40,6 +40,7 @@ struct ConvGemmParams {
   int tw_log, tiles_x, tiles_y, tiles_o, num_tiles;  // a tile is 1 << tw_log pixels wide
   int a_stages, a_stage_bytes, w_stages;
   const float* residual;
+  int res_up;                                  // 1: the residual is [oc][h/2][w/2], a value for 2 x 2 pixels
   float* out;
   int activation;
   float acc_scale;
@@ -206,11 +207,17 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       float q[32];
       auto request = [&](int ci) {
         bool in;
-        long long o0;
+        long long o0, step = hw;
         place(ci, in, o0);
+        // an upsampled residual: the two rows of a chunk read eight neighbours each, one sector, of the half-size image
+        if (p.res_up) {
+          const int px = (half * 4 + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
+          step = hw >> 2;
+          o0 = (static_cast<long long>(c.n) * p.oc + oc0) * step + static_cast<long long>(y >> 1) * (p.w >> 1) + (x >> 1);
+        }
         if (in) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) q[j] = j < nch ? __ldg(p.residual + o0 + j * hw) : 0.0f;
+          for (int j = 0; j < 32; ++j) q[j] = j < nch ? __ldg(p.residual + o0 + j * step) : 0.0f;
         }
       };
       if (p.residual != nullptr && nch > 0) request(0);
@@ -303,7 +310,7 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
     p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (WP * CG_W_TILE);
   }
   if (p.w_stages > CG_MAX_RING) p.w_stages = CG_MAX_RING;
-  p.residual = g.residual; p.out = g.out_f32; p.activation = g.activation;
+  p.residual = g.residual; p.res_up = g.residual != nullptr && g.residual_up ? 1 : 0; p.out = g.out_f32; p.activation = g.activation;
   p.acc_scale = gemm_acc_scale(g);
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   p.err_word = ctx().dev_error_word;
@@ -327,6 +334,12 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
 
 }  // namespace
 
+long long conv_gemm_tiles(const GemmArgs& g) {
+  const ConvShape sh = conv_shape(g);
+  const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
+  return g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
+}
+
 double conv_gemm_cycles(const GemmArgs& g) {
   constexpr double never = 1e30;
   const char* e = getenv("MIMIR_B200_CONV_SPATIAL");  // "0": never, "1": wherever the form allows
@@ -338,10 +351,7 @@ double conv_gemm_cycles(const GemmArgs& g) {
   // 1 x 1 (and im2col rows): nothing to share between taps; long K is better off in CTA pairs (K = 4608, 512 channels: 170 against
   // 111 us), short K is bound by its stores (K = 192, 64 channels: 139 against 247 us)
   if (g.conv_ks == 1 && g.conv_c > 1024) return never;
-  const ConvShape sh = conv_shape(g);
-  const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
-  const long long tiles = g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
-  const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
+  const long long waves = (conv_gemm_tiles(g) + ctx().sm_count - 1) / ctx().sm_count;
   const double mma = 1.15 * g.k / 16.0 * (g.a_planes + g.w_planes - 1) * 128.0;
   return 17400.0 + waves * (mma > 4500.0 ? mma : 4500.0);  // (within 5 % of 50 measured launches, K = 64 ... 4608)
 }

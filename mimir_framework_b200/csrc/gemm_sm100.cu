@@ -1115,6 +1115,10 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
   const int sbk = (g.conv_ks == 0 || g.conv_c % 64 == 0) ? 64 : 32;
   const long long big_tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
   static const bool force_pairs = env_int("MIMIR_B200_GEMM_PAIR", -1) == 1;  // pairs wherever the form allows
+  if (g.residual_up) {  // planned for this kernel (conv_takes_residual_up); the others read a residual of the output's own shape
+    if (conv_gemm_cycles(g) >= 1e30) return fail(MIMIR_B200_E_INVALID, "gemm: an upsampled residual needs the spatial-tile kernel");
+    return launch_conv_gemm(g, st);
+  }
   if (!force_pairs) {
     const double big = big_tile_cycles(g);
     int bn = 0, splits = 0;

@@ -10,7 +10,7 @@
 //                  the producing GEMM / GroupNorm, hi/lo planes straight from one GEMM to the next),
 //                  computes liveness and assigns arena offsets that are reused after the last
 //                  consumer, and checks the arena peak against the HBM budget before any launch.
-//   forward        stages the inputs, runs the layers in index order on one stream, returns "x".
+//   forward        stages the inputs, runs the layers in index order (but see fusion 1a) on one stream, returns "x".
 #include "ops.h"
 
 #include <algorithm>
@@ -133,6 +133,7 @@ struct LayerRT {
   bool read_split = false;            // Linear reads the producer's planes
   int res_v = -1;                     // residual tensor folded in from a following Add
   int pre_norm = -1;                  // Conv2d: index of the GroupNorm layer applied while its operand planes are laid out
+  bool res_up = false;                // Conv2d: res_v is the INPUT of a 2 x 2 nearest upsample that the epilogue applies
   std::vector<int> add_v;             // Embedding: tensors of the Adds folded into it (graph inputs), in layer order
   int pre_ln = -1;                    // a token-wise LayerNorm folded into this layer (index), see fusion 1f
   bool in_up = false;                 // Conv2d: in_v[0] is the INPUT of a 2 x 2 nearest upsample that the layout pass applies
@@ -228,6 +229,7 @@ struct ArenaSim {
 
 struct MimirB200Model {
   std::vector<mb::LayerRT> layers;
+  std::vector<int> order;   // layer indices in the order of execution (see fusion 1a)
   std::vector<mb::TensorV> tensors;
   std::map<std::string, int> input_v;  // graph input name -> tensor version
   int precision = MIMIR_B200_PREC_BF16X2;
@@ -796,7 +798,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     LayerRT& L = m->layers[li];
     L.in_v.clear();
     L.out_v = -1;
-    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false; L.add_v.clear();
+    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false; L.res_up = false; L.add_v.clear();
     L.ws_off = 0; L.ws_bytes = 0;
     std::vector<std::string> names = L.inputs;
     if (names.empty()) names.push_back("x");
@@ -906,6 +908,59 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     pt.producer = -2;  // dead
     A.skip = true;
   }
+  // ---- fusion 1a: the 1 x 1 convolution of a 2 x 2 nearest upsample, added to another convolution's result (a residual block that
+  //      changes its channels): the 1 x 1 convolution runs on the image before the upsample - a quarter of the pixels, each of which
+  //      gives the values of four - and the other convolution's epilogue adds its result upsampled.  It may stand later in the
+  //      graph: m->order runs it first. ----
+  m->order.resize(static_cast<size_t>(nl));
+  for (int li = 0; li < nl; ++li) m->order[li] = li;
+  static const bool fuse_up = [] { const char* e = getenv("MIMIR_B200_FUSE_UPSAMPLE"); return !(e && e[0] == '0'); }();
+  auto takes_up = [&](const LayerRT& C) {
+    return C.lt == LT::Conv2d && !C.skip && conv_takes_residual_up(batch, C.d.in_channels, C.d.out_channels, C.h, C.w, C.d.kernel, C.d.stride, C.d.padding,
+                                                                   m->precision, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act);
+  };
+  // a tensor that only layers read: no alias of it, not the model's output
+  auto plain = [&](int v) {
+    for (const TensorV& t : m->tensors)
+      if (t.alias_of == v) return false;
+    return m->tensors[v].alias_of < 0 && v != out_root;
+  };
+  for (int si = 0; si < nl && fuse_up; ++si) {
+    LayerRT& S = m->layers[si];
+    if (S.lt != LT::Conv2d || S.skip || S.res_v >= 0 || S.d.kernel != 1 || S.d.stride != 1 || S.d.padding != 0) continue;
+    const int uv = S.in_v[0], tv = S.out_v, ui = m->tensors[uv].producer;
+    if (ui < 0 || !plain(uv) || !plain(tv) || m->tensors[tv].consumers.size() != 1) continue;
+    LayerRT& U = m->layers[ui];
+    if (U.lt != LT::UpsampleNearest || U.skip || U.oh != 2 * U.h || U.ow != 2 * U.w || S.h != U.oh || S.w != U.ow) continue;
+    const int sv = root_of(m->tensors, U.in_v[0]);
+    const int ai = m->tensors[tv].consumers[0];
+    LayerRT& A = m->layers[ai];
+    if (A.lt != LT::Add || A.skip || A.in_v.size() != 2 || A.in_v[0] == A.in_v[1]) continue;
+    const int ov = A.in_v[0] == tv ? A.in_v[1] : A.in_v[0];
+    const int ci = m->tensors[ov].producer;
+    if (ci <= ui || ci == si || !plain(ov) || total_consumers(ov) != 1 || m->tensors[ov].n != m->tensors[tv].n) continue;
+    LayerRT& C = m->layers[ci];
+    if (C.out_v != ov || C.res_v >= 0 || !takes_up(C)) continue;
+    for (int& c : m->tensors[uv].consumers)
+      if (c == si) { m->tensors[uv].consumers.erase(m->tensors[uv].consumers.begin() + (&c - m->tensors[uv].consumers.data())); break; }
+    m->tensors[sv].consumers.push_back(si);
+    S.in_v[0] = sv;
+    S.h = U.h; S.w = U.w;
+    m->tensors[tv].n /= 4;
+    m->tensors[tv].consumers[0] = ci;
+    C.res_v = tv;
+    C.res_up = true;
+    C.out_v = A.out_v;
+    m->tensors[A.out_v].producer = ci;
+    m->tensors[ov].consumers.clear();
+    m->tensors[ov].want_f32 = false;
+    m->tensors[ov].producer = -2;  // dead
+    A.skip = true;
+    if (si > ci) {
+      m->order.erase(std::find(m->order.begin(), m->order.end(), si));
+      m->order.insert(std::find(m->order.begin(), m->order.end(), ci), si);
+    }
+  }
   // ---- fusion 1b: a residual Add into the epilogue of the layer that produces one of its operands -------
   for (int li = 0; li < nl; ++li) {
     LayerRT& A = m->layers[li];
@@ -969,9 +1024,8 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     P.skip = true;
   }
   // ---- fusion 1d: a 2 x 2 nearest upsample read by shifted-GEMM convolutions: their layout pass gathers from the
-  //      half-size source (and a folded GroupNorm takes its statistics there: the same values, each four times), so the
-  //      upsampled tensor is read by nobody but residual adds - and is not produced at all when there are none ----
-  static const bool fuse_up = [] { const char* e = getenv("MIMIR_B200_FUSE_UPSAMPLE"); return !(e && e[0] == '0'); }();
+  //      half-size source (and a folded GroupNorm takes its statistics there: the same values, each four times), and so does
+  //      the epilogue of a convolution that adds it as a residual; with no other reader the upsampled tensor never exists ----
   for (int li = 0; li < nl && fuse_up; ++li) {
     LayerRT& U = m->layers[li];
     if (U.lt != LT::UpsampleNearest || U.skip || U.oh != 2 * U.h || U.ow != 2 * U.w) continue;
@@ -984,6 +1038,12 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     std::vector<int> keep;
     for (int ci : ut.consumers) {
       LayerRT& C = m->layers[ci];
+      if (C.res_v == uv && !C.res_up && C.in_v[0] != uv && takes_up(C)) {
+        C.res_up = true;
+        C.res_v = sv;
+        m->tensors[sv].consumers.push_back(ci);
+        continue;
+      }
       const bool conv_in = C.lt == LT::Conv2d && !C.skip && !C.in_up && C.in_v[0] == uv && C.res_v != uv && C.d.in_channels == U.ch &&
                            C.h == U.oh && C.w == U.ow && conv_uses_shifted(C.d.in_channels, C.d.kernel, C.d.stride, C.d.padding) &&
                            (C.pre_norm >= 0 || !conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch,
@@ -1086,17 +1146,19 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
 
   // ---- liveness ------------------------------------------------------------------------------------
   const int nt = static_cast<int>(m->tensors.size());
+  std::vector<int> pos(static_cast<size_t>(nl));  // first / last are places in the order of execution
+  for (int p = 0; p < nl; ++p) pos[m->order[p]] = p;
   for (int v = 0; v < nt; ++v) {
     TensorV& t = m->tensors[v];
-    t.first = (t.producer >= 0) ? t.producer : -1;
+    t.first = (t.producer >= 0) ? pos[t.producer] : -1;
     t.last = t.first;
   }
   for (int v = 0; v < nt; ++v) {
     const int r = root_of(m->tensors, v);
     TensorV& rt = m->tensors[r];
     for (int c : m->tensors[v].consumers)
-      if (!m->layers[c].skip) rt.last = std::max(rt.last, c);
-    if (m->tensors[v].alias_of >= 0) rt.last = std::max(rt.last, m->tensors[v].producer);
+      if (!m->layers[c].skip) rt.last = std::max(rt.last, pos[c]);
+    if (m->tensors[v].alias_of >= 0) rt.last = std::max(rt.last, pos[m->tensors[v].producer]);
   }
   m->tensors[out_root].last = nl;
 
@@ -1121,7 +1183,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     const TensorV& xt = m->tensors[xr];
     if (xt.producer < 0) continue;
     LayerRT& P = m->layers[xt.producer];
-    if (P.lt != LT::Conv2d || P.skip || P.gn_emit_for >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
+    if (P.lt != LT::Conv2d || P.skip || P.res_up || P.gn_emit_for >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
     if (!conv_can_emit_gn(batch, P.d.in_channels, P.d.out_channels, P.h, P.w, P.d.kernel, P.d.stride, P.d.padding, G.d.num_groups,
                           P.d.activation ? MIMIR_B200_ELT_RELU : P.fused_act))
       continue;
@@ -1146,7 +1208,8 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
   for (int v = 0; v < nt; ++v)
     if (m->tensors[v].producer == -1 && m->tensors[v].last == -1 && root_of(m->tensors, v) != out_root) drop(v);
   uint64_t flops = 0, hbm = 0;
-  for (int li = 0; li < nl; ++li) {
+  for (int p = 0; p < nl; ++p) {
+    const int li = m->order[p];
     LayerRT& L = m->layers[li];
     if (!L.skip && L.lt != LT::Alias) {
       place(L.out_v);
@@ -1195,7 +1258,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       // In a pipelined plan the slots of the graph inputs are never handed on: the copy-in of micro-batch c + 2 may then
       // run while micro-batch c is still being copied out of the same arena buffer (nothing else lives in an input slot).
       if (m->pipeline > 1 && t.producer == -1) continue;
-      if (t.alias_of < 0 && t.producer != -2 && t.last == li) drop(v);
+      if (t.alias_of < 0 && t.producer != -2 && t.last == p) drop(v);
     }
   }
   // Does the output share bytes with a graph input's slot (possible only in un-pipelined plans, or when the graph returns
@@ -1273,8 +1336,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
     return reinterpret_cast<float*>(arena + m->tensors[r].off_f32);
   };
   auto splitp = [&](int v) -> __nv_bfloat16* { return reinterpret_cast<__nv_bfloat16*>(arena + m->tensors[v].off_split); };
-  const int nl = static_cast<int>(m->layers.size());
-  for (int li = 0; li < nl; ++li) {
+  for (int li : m->order) {
     LayerRT& L = m->layers[li];
     if (L.skip || L.lt == LT::Alias) continue;
     const MimirLayerDesc& d = L.d;
@@ -1333,6 +1395,7 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.activation = d.activation ? MIMIR_B200_ELT_RELU : L.fused_act;
         e.x = f32p(L.in_v[0]); e.w_split = L.w_split; e.w_f32 = L.w_f32; e.w_scale = L.w_scale; e.w_ready = true; e.y = f32p(L.out_v); e.ws = ws;
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
+        e.residual_up = L.res_up;
         if (L.pre_norm >= 0) {
           const LayerRT& G = m->layers[L.pre_norm];
           e.pre_groups = G.d.num_groups;

@@ -109,6 +109,7 @@ struct ConvExec {
   bool w_ready = false;                        // see LinearExec
   float w_scale = 1.0f;                        // the planes hold W * w_scale
   const float* residual = nullptr;             // NCHW, same shape as y
+  bool residual_up = false;                    // the residual is [oc][h/2][w/2] and stands for its 2 x 2 nearest-neighbour upsample
   float* y = nullptr;
   void* ws = nullptr;
   // GroupNorm (+ SiLU) of the producing layer, applied while the operand planes are laid out (shifted path only):
@@ -138,6 +139,7 @@ bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int strid
 // padded NHWC activation; everything else goes through im2col planes.  The two paths want different
 // weight-plane orders ((kh, kw, ic) vs (ic, kh, kw)).
 bool conv_uses_shifted(int ic, int ks, int stride, int pad);
+bool conv_takes_residual_up(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act);
 size_t conv_ws_bytes(int batch, int ic, int h, int w, int ks, int stride, int pad, int precision);
 int conv_exec(const ConvExec& e, cudaStream_t st);
 

@@ -61,3 +61,33 @@ def test_relu_and_many_tiles(rt):
     got = rt.conv2d(x, wt, batch, ic, oc, h, h, 3, 1, 1, relu=True).reshape(batch, -1)
     want = np.stack([port.conv2d(x[i], wt, ic, oc, h, h, 3, 1, 1, True).ravel() for i in range(batch)])
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("skip_conv", [False, True])
+@pytest.mark.parametrize("batch,ic,oc,h,w", [(40, 32, 130, 12, 10), (10, 64, 64, 34, 18), (150, 32, 32, 1, 1), (2, 32, 32, 8, 8)])
+def test_residual_block_behind_an_upsample(rt, batch, ic, oc, h, w, skip_conv):
+    """Up -> conv -> conv, plus the upsampled image itself or a 1 x 1 convolution of it, which stands after the other two."""
+    oc = oc if skip_conv else ic
+    r = np.random.default_rng(batch + oc)
+    x = r.standard_normal((batch, ic * h * w)).astype(np.float32)
+    shapes = [(oc, ic, 3), (oc, oc, 3), (oc, ic, 1)]
+    ws = [(r.standard_normal(o * i * k * k) / np.sqrt(i * k * k)).astype(np.float32) for o, i, k in shapes]
+    conv = lambda name, a, b, j: make_desc(name, "Conv2d", inputs=[a], output=b, in_channels=shapes[j][1], out_channels=oc, input_height=2 * h,  # noqa: E731
+                                           input_width=2 * w, kernel=shapes[j][2], stride=1, padding=shapes[j][2] // 2, params_count=ws[j].size)
+    descs = [make_desc("u", "UpsampleNearest", inputs=["x"], output="u", in_channels=ic, out_h=h, out_w=w, scale_h=2, scale_w=2),
+             conv("c1", "u", "t", 0), conv("c2", "t", "y", 1)]
+    if skip_conv:
+        descs.append(conv("c3", "u", "s", 2))
+    descs.append(make_desc("a", "Add", inputs=["y", "s" if skip_conv else "u"], output="x"))
+    m = rt.GraphModel(descs, abi.PREC_BF16X2)
+    for j in range(3 if skip_conv else 2):
+        m.upload_weights(1 + j, ws[j])
+    m.plan({"x": (ic * h * w, False)}, batch)
+    got = m.forward({"x": (x, False)}, batch, oc * 4 * h * w)
+    m.close()
+    for i in range(0, batch, 3):
+        u = x[i].reshape(ic, h, w).repeat(2, 1).repeat(2, 2).ravel()
+        t = port.conv2d(u, ws[0], ic, oc, 2 * h, 2 * w, 3, 1, 1, False).ravel()
+        want = port.conv2d(t, ws[1], oc, oc, 2 * h, 2 * w, 3, 1, 1, False).ravel()
+        want = want + (port.conv2d(u, ws[2], ic, oc, 2 * h, 2 * w, 1, 1, 0, False).ravel() if skip_conv else u)
+        assert np.linalg.norm(got[i] - want) <= 2e-5 * np.linalg.norm(want)
