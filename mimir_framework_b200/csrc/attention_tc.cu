@@ -27,6 +27,7 @@
 // Every mbarrier wait is bounded; on expiry the CTA raises its abort flag, sets the device error word,
 // leaves all loops and frees its TMEM.
 #include "common.h"
+#include "launch.cuh"
 #include "planes.cuh"
 #include "sm100_ptx.cuh"
 
@@ -57,6 +58,7 @@ struct AttnParams {
   int qk_from_planes;  // Q and K tiles come straight from the QKV GEMM's output planes [2][batch*seq][3E] (5-D maps)
   int v_mn_major;      // ... and so do the V tiles, as [key][d] rows read by the MMA as an MN-major B operand
   int f16;             // operand planes hold IEEE half instead of bfloat16
+  int splits;          // CTAs (a cluster) that share a query tile's keys in the second kernel form
   int head_chunk;      // (sample, head) pairs per scheduling chunk of the second kernel form
   float acc_comp;      // relative loss of the truncating fp32 accumulation per MMA (0 = no compensation)
   int* err_word;
@@ -450,11 +452,27 @@ flash_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 // Shared memory: Q 32 KB + 2 x 16 KB K + 2 x 16 KB V = 96 KB; 256 TMEM columns (3 x 64 scores + 64 for O): two CTAs
 // per SM as before.  A tile's barriers live per score tile / per stage, so that no waiter is ever more than one phase
 // behind the barrier it waits on.
+//   * A key tile takes about 1.4 us, whatever else the SM does: with fewer query tiles than SMs the longest chain of tiles is the
+// time of the launch.  A cluster of two or four CTAs then shares the keys of a query tile; each leaves its maximum, sum and
+// unnormalised O rows in its shared memory and merges a part of the rows.
+constexpr int A2_OPITCH = AT_HD + 4;  // floats per O row there, a whole number of 16-byte words that spreads rows over the banks
 constexpr int A2_TILE = AT_BK * AT_HD * 2;        // one plane of a 64-key K or V tile
 constexpr int A2_STAGE = 2 * A2_TILE;             // hi and lo plane
 constexpr int A2_THREADS = 320;                    // TMA warp, MMA warp, 8 softmax warps (two threads per query row)
 constexpr int A2_XCHG = 4 * AT_BQ * 4;             // row maxima / sums exchanged between the two threads of a row
 constexpr int A2_SMEM = 2 * AT_Q_BYTES + 2 * A2_STAGE + 2 * A2_STAGE + A2_XCHG + 256;
+
+static_assert(AT_BQ * (A2_OPITCH + 2) * 4 <= 2 * AT_Q_BYTES + 2 * A2_STAGE, "O rows, maxima and sums over Q and K");
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -487,9 +505,11 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   // (sample, head) pairs - sized so that the chunk's K and V stay in L2 - the longest tiles of all its heads are launched
   // first and the shortest last, so that the tail of the launch is made of short CTAs whatever the batch.
   int qt, bhi;
+  pdl_wait();
+  const int split = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   {
     const int q_tiles = (p.seq + AT_BQ - 1) / AT_BQ;
-    const int bid = static_cast<int>(blockIdx.x);
+    const int bid = static_cast<int>(blockIdx.x) / p.splits;
     const int c = bid / (q_tiles * p.head_chunk);
     const int rem = bid - c * q_tiles * p.head_chunk;
     const int hcnt = min(p.head_chunk, p.bh - c * p.head_chunk);
@@ -500,6 +520,8 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int q0 = qt * AT_BQ;
   int n_tiles = (p.seq + AT_BK - 1) / AT_BK;
   if (p.causal) n_tiles = min(n_tiles, (min(p.seq, q0 + AT_BQ) + AT_BK - 1) / AT_BK);
+  const int all_tiles = n_tiles, tile0 = all_tiles * split / p.splits;  // this CTA's key tiles
+  n_tiles = all_tiles * (split + 1) / p.splits - tile0;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -544,16 +566,16 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       if (!mbar_wait_warp(k_empty + st, (static_cast<uint32_t>(j >> 1) & 1) ^ 1, abort_flag, p.err_word, 31)) { ok = false; return; }
       if (!one) return;
       mbar_expect_tx(k_full + st, A2_STAGE);
-      tma_load_5d(sK + st * A2_STAGE, &map_k, k_full + st, 0, j * AT_BK, smp, p.heads + hd_slot, 0);
-      tma_load_5d(sK + st * A2_STAGE + A2_TILE, &map_k, k_full + st, 0, j * AT_BK, smp, p.heads + hd_slot, 1);
+      tma_load_5d(sK + st * A2_STAGE, &map_k, k_full + st, 0, (tile0 + j) * AT_BK, smp, p.heads + hd_slot, 0);
+      tma_load_5d(sK + st * A2_STAGE + A2_TILE, &map_k, k_full + st, 0, (tile0 + j) * AT_BK, smp, p.heads + hd_slot, 1);
     };
     auto load_v = [&](int j) {
       const int st = j & 1;
       if (!mbar_wait_warp(v_empty + st, (static_cast<uint32_t>(j >> 1) & 1) ^ 1, abort_flag, p.err_word, 32)) { ok = false; return; }
       if (!one) return;
       mbar_expect_tx(v_full + st, A2_STAGE);
-      tma_load_5d(sV + st * A2_STAGE, &map_v, v_full + st, 0, j * AT_BK, smp, 2 * p.heads + hd_slot, 0);
-      tma_load_5d(sV + st * A2_STAGE + A2_TILE, &map_v, v_full + st, 0, j * AT_BK, smp, 2 * p.heads + hd_slot, 1);
+      tma_load_5d(sV + st * A2_STAGE, &map_v, v_full + st, 0, (tile0 + j) * AT_BK, smp, 2 * p.heads + hd_slot, 0);
+      tma_load_5d(sV + st * A2_STAGE + A2_TILE, &map_v, v_full + st, 0, (tile0 + j) * AT_BK, smp, 2 * p.heads + hd_slot, 1);
     };
     // in the order the MMA warp consumes them: K_0, K_1, then V_j, K_{j+2}
     if (n_tiles > 0) load_k(0);
@@ -647,7 +669,7 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       int ok_tile = 0;
       if (alive) ok_tile = warp_wait(s_full + b, static_cast<uint32_t>(j / 3) & 1, 38) ? 1 : 0;
       tcgen05_fence_after();
-      const int key0 = j * AT_BK + grp * 32;
+      const int key0 = (tile0 + j) * AT_BK + grp * 32;
       uint32_t sc[32];
       const uint32_t tmem_s = tmem_base + b * AT_BK + lane_base;
       if (ok_tile) {
@@ -734,7 +756,25 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (!alive) xchg_abort[quad] = 1;
     pair_sync();
     if (xchg_abort[quad]) alive = false;
-    if (alive) {
+    if (p.splits > 1) {
+      float* orow = reinterpret_cast<float*>(sQ) + r_local * A2_OPITCH + grp * 32;  // (Q, K and V have been consumed)
+      float* ml = reinterpret_cast<float*>(sQ) + AT_BQ * A2_OPITCH;
+      const bool any = alive && n_tiles > 0;
+      l_run = any ? l_run + xchg[(last + (grp ^ 1)) * AT_BQ + r_local] : 0.0f;
+      if (any) {
+        tcgen05_fence_after();
+        uint32_t v[32];
+        tmem_ld_32x32_nowait(tmem_o + lane_base + grp * 32, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; c += 4)
+          *reinterpret_cast<uint4*>(orow + c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      }
+      if (grp == 0) {
+        ml[r_local] = m_run;
+        ml[AT_BQ + r_local] = l_run;  // 0: nothing to add (no tiles, all keys masked, or a wait gave up)
+      }
+    } else if (alive) {
       l_run += xchg[(last + (grp ^ 1)) * AT_BQ + r_local];
       tcgen05_fence_after();
       const int keys_seen = p.causal ? min(p.seq, row + 1) : p.seq;
@@ -774,6 +814,57 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, AT_TMEM_COLS);
   }
+  if (p.splits == 1) return;
+
+  // ---- the cluster's parts of each row: this CTA merges 128 / splits of the rows ----
+  __syncwarp();
+  cluster_sync_all();
+  if (warp >= 2) {
+    const int t = static_cast<int>(threadIdx.x) - 64, per_row = 2 * p.splits, cols = AT_HD / per_row;  // 256 threads: 16 or 8 columns each
+    const int r_local = split * (AT_BQ / p.splits) + t / per_row, c0 = (t % per_row) * cols, row = q0 + r_local;
+    if (row < p.seq) {
+      const uint32_t o_addr = smem_u32(sQ) + (r_local * A2_OPITCH + c0) * 4, ml_addr = smem_u32(sQ) + (AT_BQ * A2_OPITCH + r_local) * 4;
+      constexpr float LOG2E = 1.4426950408889634f;
+      float m = -1e30f, l = 0.0f, o[16];
+      for (int s = 0; s < p.splits; ++s) m = fmaxf(m, ld_cluster_f32(mapa_shared(ml_addr, s)));
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i] = 0.0f;
+      const int keys_seen = p.causal ? min(p.seq, row + 1) : p.seq;
+      for (int s = 0; s < p.splits; ++s) {
+        const float ls = ld_cluster_f32(mapa_shared(ml_addr + AT_BQ * 4, s));
+        if (!(ls > 0.0f)) continue;
+        const float w = fast_exp2((ld_cluster_f32(mapa_shared(ml_addr, s)) - m) * LOG2E);
+        l += w * ls;
+        const int k0 = all_tiles * s / p.splits * AT_BK, k1 = min(all_tiles * (s + 1) / p.splits * AT_BK, keys_seen);
+        const float wo = w * (1.0f + p.acc_comp * static_cast<float>(3 * ((max(k1 - k0, 0) + 15) / 16)));
+        const uint32_t a = mapa_shared(o_addr, s);
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          if (i >= cols) break;
+          const float4 q = ld_cluster_f32x4(a + i * 4);
+          o[i] += wo * q.x; o[i + 1] += wo * q.y; o[i + 2] += wo * q.z; o[i + 3] += wo * q.w;
+        }
+      }
+      const float inv = 1.0f / (l + 1e-9f);
+      const int bb = bhi / p.heads, h = bhi - bb * p.heads;
+      const long long o_off = (static_cast<long long>(bb) * p.seq + row) * p.embed + h * AT_HD + c0;
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        if (i >= cols) break;
+        const float f[4] = {o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv};
+        if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + o_off + i) = make_float4(f[0], f[1], f[2], f[3]);
+        if (p.out_split != nullptr) {
+          uint32_t h2[2], l2[2];
+          split_pair(f[0], f[1], p.f16, h2[0], l2[0]);
+          split_pair(f[2], f[3], p.f16, h2[1], l2[1]);
+          *reinterpret_cast<uint2*>(p.out_split + o_off + i) = make_uint2(h2[0], h2[1]);
+          if (p.planes == 2) *reinterpret_cast<uint2*>(p.out_split + p.plane_stride + o_off + i) = make_uint2(l2[0], l2[1]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // a peer may still be reading this CTA's rows
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -895,6 +986,7 @@ int launch_attention_core_tc(const float* qkv, float* out, int batch, int seq, i
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   dim3 grid((seq + AT_BQ - 1) / AT_BQ, bh);
   p.head_chunk = 1;
+  p.splits = 1;
   if (v2) {
     // heads whose K and V planes (seq x 64 x 2 planes x 2 bytes, twice) fill about 48 MB of L2
     const long long per_head = static_cast<long long>(seq) * AT_HD * 2 * 2 * 2;
@@ -906,8 +998,11 @@ int launch_attention_core_tc(const float* qkv, float* out, int batch, int seq, i
       MB_CUDA(cudaFuncSetAttribute(flash_attn_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, A2_SMEM));
       return MIMIR_B200_OK;
     }));
-    flash_attn_tc2_kernel<<<grid, A2_THREADS, A2_SMEM, st>>>(mq, mk, mv, p);
-    MB_CUDA(cudaGetLastError());
+    // All CTAs of a split launch are resident together (two per SM); a part of fewer than two key tiles is not worth the merge.
+    const int max_tiles = (seq + AT_BK - 1) / AT_BK, fit = 2 * ctx().sm_count / static_cast<int>(grid.x);
+    p.splits = fit >= 4 && max_tiles >= 8 ? 4 : fit >= 2 && max_tiles >= 4 ? 2 : 1;
+    grid.x *= static_cast<unsigned>(p.splits);
+    MB_TRY(launch_pdl(flash_attn_tc2_kernel, grid, dim3(A2_THREADS), A2_SMEM, st, p.splits, mq, mk, mv, p));
     count_launch(1);
     return MIMIR_B200_OK;
   }
