@@ -11,6 +11,7 @@
 //   * "chunk" kernels when there are only a few (long) rows: pass 1 reduces 8192-element chunks to
 //     partial statistics in a small global scratch, pass 2 combines the partials of its row and
 //     writes the result; rows are processed in groups that fit in L2 so that pass 2 reads from L2.
+#include <type_traits>
 #include <cooperative_groups.h>
 
 #include <map>
@@ -331,6 +332,7 @@ struct RmsOnePass {
   unsigned* ticket;         // [0] ticket counter, [1] abort flag, [2] rows finished
   unsigned* row_done;       // per row: CTAs that have read everything they need
   int rows;
+  int stage_gamma;          // gamma goes through shared memory as well (launches of few CTAs)
   unsigned long long* sum_slots;
   unsigned long long* err_slots;
   long long len;
@@ -348,15 +350,15 @@ __device__ __forceinline__ bool slot_wait(const unsigned long long* slot, volati
   const volatile unsigned long long* p = slot;
   unsigned long long v = *p;
   if ((v >> 32) == 0) {
-    uint64_t t0;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    uint64_t t0 = 0;
     unsigned spins = 0;
     while (((v = *p) >> 32) == 0) {
-      __nanosleep(32);
-      if ((++spins & 0xFF) == 0) {
+      if (++spins > 16) __nanosleep(32);
+      if ((spins & 0xFF) == 0) {
         if (*abort_flag) return false;
         uint64_t t1;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+        if (t0 == 0) t0 = t1;
         if (t1 - t0 > 2000000000ull) {
           *abort_flag = 1u;
           atomicExch(err_word, site);
@@ -383,30 +385,43 @@ __device__ __forceinline__ double block_sum_f64(double v, double* red) {
 
 __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p) {
   extern __shared__ __align__(128) float sx[];  // the chunk, zero beyond its end
-  __shared__ __align__(8) uint64_t bar;
+  float* sg = sx + CHUNK;                       // stage_gamma: its chunk of gamma
+  __shared__ __align__(8) uint64_t bar, gamma_bar;
   __shared__ unsigned s_id;
   __shared__ int s_abort, s_last;
   __shared__ float redf[33];
   __shared__ double red[8];
   const int tid = threadIdx.x;
-  pdl_wait();
   if (tid == 0) {
-    s_id = atomicAdd(p.ticket, 1u);
     s_abort = 0;
     mbar_init(&bar, 1);
+    mbar_init(&gamma_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // gamma has as many elements as a row: fetched into L2 while the sums travel (with one row, before the kernel ahead has finished),
+  // and on into shared memory where there is room.  Loaded by the last loop it cost that loop 5 of a one-prompt norm's 13 us
+  // (1 x 768 000 elements into planes: 14.7 us and a 3.7 us memset at first, 8.9 us now).
+  auto prefetch_gamma = [&](long long o) {
+    if (p.gamma != nullptr && o + tid * 32 < p.n_gamma) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gamma + o + tid * 32));
+  };
+  if (p.rows == 1) prefetch_gamma(static_cast<long long>(blockIdx.x) * CHUNK);
+  pdl_wait();
+  // (one row needs no order among its CTAs, which are resident together: it saves the round trip to the counter)
+  if (tid == 0) s_id = p.rows == 1 ? blockIdx.x : atomicAdd(p.ticket, 1u);
   __syncthreads();
   const long long row = s_id / static_cast<unsigned>(p.chunks);
   const int c = static_cast<int>(s_id % static_cast<unsigned>(p.chunks));
   const long long off = static_cast<long long>(c) * CHUNK;
   const int n = static_cast<int>(min(static_cast<long long>(CHUNK), p.len - off));
   const float* g = p.x + row * p.len + off;
+  if (p.rows > 1) prefetch_gamma(off);
   volatile unsigned* abort_flag = p.ticket + 1;
 
   // ---- the chunk into shared memory: bulk copies when source and size allow, plain loads otherwise ----
   const bool bulk = (reinterpret_cast<uintptr_t>(g) & 15) == 0 && (n & 3) == 0;
   bool ok = true;
+  const bool vec_gamma = p.gamma != nullptr && (reinterpret_cast<uintptr_t>(p.gamma + off) & 15) == 0 && (n & 3) == 0 && off + n <= p.n_gamma;
+  const bool staged = p.stage_gamma && vec_gamma;
   if (bulk) {
     if (tid == 0) {
       mbar_expect_tx(&bar, static_cast<uint32_t>(n) * 4u);
@@ -418,10 +433,15 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
     for (int i = tid; i < CHUNK; i += 256) sx[i] = (i < n) ? __ldg(g + i) : 0.0f;
   }
   __syncthreads();
+  if (staged && tid == 0) {
+    mbar_expect_tx(&gamma_bar, static_cast<uint32_t>(n) * 4u);
+    for (int b0 = 0; b0 < n; b0 += 2048) bulk_load_1d(sg + b0, p.gamma + off + b0, static_cast<uint32_t>(min(2048, n - b0)) * 4u, &gamma_bar);
+  }
   const float4* s4 = reinterpret_cast<const float4*>(sx);
+  // (The loops over the chunk are unrolled no further than they gain by: the code comes from L2 at every launch.)
   // ---- the chunk's sum of squares ----
   float acc = 0.0f;
-#pragma unroll
+#pragma unroll 2
   for (int i = 0; i < OP_VEC; ++i) {
     const float4 v = s4[i * 256 + tid];
     acc += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
@@ -431,22 +451,22 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   if (tid == 0) atomicExch(p.sum_slots + slot0 + c, slot_pack(run));
 
   // ---- sum of the chunks before this one (only its binade matters) ----
-  double before = 0.0;
+  float before = 0.0f;
   for (int j = tid; j < c; j += 256) {
     float t = 0.0f;
     ok = ok && slot_wait(p.sum_slots + slot0 + j, abort_flag, p.err_word, 21, &t);
-    before += static_cast<double>(t);
+    before += t;
   }
-  const double prefix = block_sum_f64(before, red);
+  const float prefix = block_sum(before, redf);
 
   // ---- replay the reference's chain s = fma(x, x, s) over this thread's elements and collect the
   //      rounding error of every step with error-free transformations (see rms_seq_err_kernel) ----
   float err = 0.0f;
-#pragma unroll
+#pragma unroll 2
   for (int i = 0; i < OP_VEC; ++i) {
     // Where the chain stood before this float4: only the binade of that value enters the rounding of a step,
     // so inside the chunk (1 % of a long sample) the running sum is taken as growing evenly.
-    float sf = static_cast<float>(prefix) + run * (static_cast<float>((i * 256 + tid) * 4) * (1.0f / CHUNK));
+    float sf = prefix + run * (static_cast<float>((i * 256 + tid) * 4) * (1.0f / CHUNK));
     const float4 v = s4[i * 256 + tid];
     const float e4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -463,8 +483,8 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
       sf = nf;
     }
   }
-  const double chunk_err = block_sum_f64(static_cast<double>(err), red);
-  if (tid == 0) atomicExch(p.err_slots + slot0 + c, slot_pack(static_cast<float>(chunk_err)));
+  const float chunk_err = block_sum(err, redf);  // (a correction of some 1e-5 of the sum)
+  if (tid == 0) atomicExch(p.err_slots + slot0 + c, slot_pack(chunk_err));
 
   // ---- the sample's total: every chunk's sum and chain error ----
   double mine = 0.0;
@@ -475,12 +495,97 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
     mine += static_cast<double>(s) + static_cast<double>(e);
   }
   const double sd = block_sum_f64(mine, red);
+  if (staged && !mbar_wait(&gamma_bar, 0, &s_abort, p.err_word, 24)) ok = false;  // (asked for before the sums were; nobody leaves before it lands)
   if (__syncthreads_or(!ok)) {  // a wait gave up: the error word is set, nothing is written
     if (tid == 0) *abort_flag = 1u;
     return;
   }
+  const float rms = sqrtf(static_cast<float>(sd) / static_cast<float>(p.len) + p.eps);
+  const float inv_rms = 1.0f / rms;
+
+  // ---- apply and store ----
+  const long long base = row * p.len + off;
+  const bool vec_out = (n & 3) == 0 && (p.y == nullptr || (reinterpret_cast<uintptr_t>(p.y + base) & 15) == 0) &&
+                       (p.y_split == nullptr || ((reinterpret_cast<uintptr_t>(p.y_split + base) & 7) == 0 && (p.plane_stride & 3) == 0));
+  // x / rms as one multiply by the reciprocal plus one correction step (P. Markstein, IBM J. Res. Dev. 34, 1990: with the correctly
+  // rounded reciprocal and the exact remainder of a fused multiply-add the corrected quotient of two normal numbers is the correctly
+  // rounded one)
+  auto quotients = [&](float (&o)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float q0 = o[j] * inv_rms;
+      o[j] = fmaf(fmaf(-q0, rms, o[j]), inv_rms, q0);
+    }
+  };
+  // A whole chunk into two planes: four float4 per thread side by side, no branch between them (the general loop's iterations follow
+  // one another, 550 cycles each with eight warps on the SM: 2.5 us of a one-prompt norm)
+  auto planes_fast = [&](auto half) {
+    for (int i0 = 0; i0 < OP_VEC; i0 += 4) {
+      float o[4][4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e0 = ((i0 + k) * 256 + tid) * 4;
+        const float4 v = s4[(i0 + k) * 256 + tid], gm = staged ? *reinterpret_cast<const float4*>(sg + e0) : __ldg(reinterpret_cast<const float4*>(p.gamma + off + e0));
+        o[k][0] = v.x; o[k][1] = v.y; o[k][2] = v.z; o[k][3] = v.w;
+        quotients(o[k]);
+        o[k][0] *= gm.x; o[k][1] *= gm.y; o[k][2] *= gm.z; o[k][3] *= gm.w;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t h01, h23, l01, l23;
+        split_pair(o[k][0], o[k][1], decltype(half)::value, h01, l01);
+        split_pair(o[k][2], o[k][3], decltype(half)::value, h23, l23);
+        __nv_bfloat16* y = p.y_split + base + ((i0 + k) * 256 + tid) * 4;
+        *reinterpret_cast<uint2*>(y) = make_uint2(h01, h23);
+        *reinterpret_cast<uint2*>(y + p.plane_stride) = make_uint2(l01, l23);
+      }
+    }
+  };
+  if (n == CHUNK && vec_out && vec_gamma && p.y == nullptr && p.planes == 2) {
+    if (p.f16) planes_fast(std::true_type{}); else planes_fast(std::false_type{});
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < OP_VEC; ++i) {
+      const int e0 = (i * 256 + tid) * 4;
+      if (e0 >= n) break;
+      const float4 v = s4[i * 256 + tid];
+      float o[4] = {v.x, v.y, v.z, v.w};
+      quotients(o);
+      if (vec_gamma) {
+        const float4 gm = staged ? *reinterpret_cast<const float4*>(sg + e0) : __ldg(reinterpret_cast<const float4*>(p.gamma + off + e0));
+        o[0] *= gm.x; o[1] *= gm.y; o[2] *= gm.z; o[3] *= gm.w;
+      } else if (p.gamma != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (off + e0 + j < p.n_gamma) o[j] *= __ldg(p.gamma + off + e0 + j);
+      }
+      if (vec_out) {
+        if (p.y != nullptr) __stcs(reinterpret_cast<float4*>(p.y + base + e0), make_float4(o[0], o[1], o[2], o[3]));
+        if (p.y_split != nullptr) {
+          uint32_t h01, h23, l01, l23;
+          split_pair(o[0], o[1], p.f16, h01, l01);
+          split_pair(o[2], o[3], p.f16, h23, l23);
+          *reinterpret_cast<uint2*>(p.y_split + base + e0) = make_uint2(h01, h23);
+          if (p.planes == 2) *reinterpret_cast<uint2*>(p.y_split + p.plane_stride + base + e0) = make_uint2(l01, l23);
+        }
+      } else {
+        for (int j = 0; j < 4 && e0 + j < n; ++j) {
+          if (p.y != nullptr) p.y[base + e0 + j] = o[j];
+          if (p.y_split != nullptr) {
+            uint16_t h, l;
+            split_one(o[j], p.f16, h, l);
+            uint16_t* y16 = reinterpret_cast<uint16_t*>(p.y_split);
+            y16[base + e0 + j] = h;
+            if (p.planes == 2) y16[p.plane_stride + base + e0 + j] = l;
+          }
+        }
+      }
+    }
+  }
+
   // The row's last CTA leaves its slots zero for the next launch, the last row the ticket counter: no clearing between launches
-  // (a memset ahead of every launch and the gaps around it took 5 us of a one-prompt decoder's 18 us per norm).
+  // (a memset ahead of every launch and the gaps around it took 5 us of a one-prompt decoder's 18 us per norm), and
+  // after the stores, because nobody waits for it.
   if (tid == 0) s_last = atomicAdd(p.row_done + row, 1u) == static_cast<unsigned>(p.chunks) - 1u;
   __syncthreads();
   if (s_last) {
@@ -493,57 +598,6 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
       if (atomicAdd(p.ticket + 2, 1u) == static_cast<unsigned>(p.rows) - 1u) {
         p.ticket[0] = 0u;
         p.ticket[2] = 0u;
-      }
-    }
-  }
-  const float rms = sqrtf(static_cast<float>(sd) / static_cast<float>(p.len) + p.eps);
-  const float inv_rms = 1.0f / rms;
-
-  // ---- apply and store ----
-  const long long base = row * p.len + off;
-  const bool vec_out = (n & 3) == 0 && (p.y == nullptr || (reinterpret_cast<uintptr_t>(p.y + base) & 15) == 0) &&
-                       (p.y_split == nullptr || ((reinterpret_cast<uintptr_t>(p.y_split + base) & 7) == 0 && (p.plane_stride & 3) == 0));
-  const bool vec_gamma = p.gamma != nullptr && (reinterpret_cast<uintptr_t>(p.gamma + off) & 15) == 0 && off + n <= p.n_gamma;
-#pragma unroll 2
-  for (int i = 0; i < OP_VEC; ++i) {
-    const int e0 = (i * 256 + tid) * 4;
-    if (e0 >= n) break;
-    const float4 v = s4[i * 256 + tid];
-    // x / rms as one multiply by the reciprocal plus one correction step (what the division routine itself does,
-    // minus its special-case handling: the quotient of two normal numbers comes out correctly rounded)
-    float o[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float q0 = o[j] * inv_rms;
-      o[j] = fmaf(fmaf(-q0, rms, o[j]), inv_rms, q0);
-    }
-    if (vec_gamma) {
-      const float4 gm = __ldg(reinterpret_cast<const float4*>(p.gamma + off + e0));
-      o[0] *= gm.x; o[1] *= gm.y; o[2] *= gm.z; o[3] *= gm.w;
-    } else if (p.gamma != nullptr) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (off + e0 + j < p.n_gamma) o[j] *= __ldg(p.gamma + off + e0 + j);
-    }
-    if (vec_out) {
-      if (p.y != nullptr) __stcs(reinterpret_cast<float4*>(p.y + base + e0), make_float4(o[0], o[1], o[2], o[3]));
-      if (p.y_split != nullptr) {
-        uint32_t h01, h23, l01, l23;
-        split_pair(o[0], o[1], p.f16, h01, l01);
-        split_pair(o[2], o[3], p.f16, h23, l23);
-        *reinterpret_cast<uint2*>(p.y_split + base + e0) = make_uint2(h01, h23);
-        if (p.planes == 2) *reinterpret_cast<uint2*>(p.y_split + p.plane_stride + base + e0) = make_uint2(l01, l23);
-      }
-    } else {
-      for (int j = 0; j < 4 && e0 + j < n; ++j) {
-        if (p.y != nullptr) p.y[base + e0 + j] = o[j];
-        if (p.y_split != nullptr) {
-          uint16_t h, l;
-          split_one(o[j], p.f16, h, l);
-          uint16_t* y16 = reinterpret_cast<uint16_t*>(p.y_split);
-          y16[base + e0 + j] = h;
-          if (p.planes == 2) y16[p.plane_stride + base + e0 + j] = l;
-        }
       }
     }
   }
@@ -1142,7 +1196,14 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
     p.sum_slots = reinterpret_cast<unsigned long long*>(op + 256 + (static_cast<size_t>(batch) * 4 + 255) / 256 * 256);
     p.err_slots = p.sum_slots + slots;
     p.len = n; p.chunks = chunks; p.eps = eps; p.err_word = ctx().dev_error_word;
-    MB_TRY(launch_pdl(rms_onepass_kernel, dim3(static_cast<unsigned>(slots)), dim3(256), CHUNK * sizeof(float), st, 1, p));
+    // up to three CTAs per SM have room for gamma's chunk beside their own; a larger launch keeps six per SM and finds gamma in L2
+    p.stage_gamma = slots <= static_cast<size_t>(3) * ctx().sm_count ? 1 : 0;
+    static PerDeviceOnce attr_once;
+    MB_TRY(attr_once.run([&]() -> int {
+      MB_CUDA(cudaFuncSetAttribute(rms_onepass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CHUNK * sizeof(float)));
+      return MIMIR_B200_OK;
+    }));
+    MB_TRY(launch_pdl(rms_onepass_kernel, dim3(static_cast<unsigned>(slots)), dim3(256), CHUNK * sizeof(float) * (p.stage_gamma ? 2 : 1), st, 1, p));
     count_launch();
     return MIMIR_B200_OK;
   }

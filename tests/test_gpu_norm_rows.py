@@ -1,9 +1,12 @@
 """Norms and softmax of rows in registers (csrc/norm_rows.cu) at the edges of their forms: a warp, one CTA, clusters; lengths that are no
-multiple of four (rows start between 16-byte boundaries); channels that end inside a vector; tensors that are not 16-byte aligned."""
+multiple of four (rows start between 16-byte boundaries); channels that end inside a vector; tensors that are not 16-byte aligned; and the
+one-pass RMSNorm of longer rows (csrc/norms.cu)."""
 import numpy as np
 import pytest
 
 from mimir_framework_b200 import abi
+from mimir_framework_b200.abi import make_desc
+from oracle import port
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +59,34 @@ def test_unaligned_device_tensors(rt):
     rt.check(rt.lib().mimir_b200_dev_softmax(x[1:].data_ptr(), y[1:].data_ptr(), rows, n, 0, None))
     torch.cuda.synchronize()
     assert torch.allclose(y[1:].view(rows, n), torch.softmax(x[1:].view(rows, n), 1), atol=1e-6, rtol=1e-5)
+
+
+@pytest.mark.parametrize("rows,n,ng", [(1, 16388, 16388), (1, 24576, 24576), (2, 16386, 16386), (3, 24580, 24576), (1, 24577, 24577), (148, 24576, 24576), (149, 24576, 24576), (5, 32768, 7)])
+def test_one_pass_rmsnorm_gamma(rt, rows, n, ng):
+    """Gamma through shared memory (up to three chunks per SM) and from L2, whole and ragged last chunks, gamma shorter than the row."""
+    r = np.random.default_rng(rows + n)
+    x, g = r.standard_normal((rows, n)).astype(np.float32), r.standard_normal(ng).astype(np.float32)
+    got = np.asarray(rt.rmsnorm(x.ravel(), g, rows, n)).reshape(rows, n)
+    for i in sorted({0, rows // 2, rows - 1}):
+        want = port.rmsnorm(x[i], g, 1e-5)
+        assert np.abs(got[i] - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("batch,seq", [(1, 256), (1, 300), (3, 257), (40, 300)])
+def test_one_pass_rmsnorm_into_planes(rt, batch, seq):
+    """The next Linear's operand planes written by the norm: whole chunks, a ragged last one, few and many CTAs."""
+    E, out = 128, 8
+    r = np.random.default_rng(seq)
+    x = r.standard_normal((batch, seq * E)).astype(np.float32)
+    g, w = r.standard_normal(seq * E).astype(np.float32), (r.standard_normal(out * E) / np.sqrt(E)).astype(np.float32)
+    descs = [make_desc("n", "RMSNorm", inputs=["x"], output="t", params_count=g.size),
+             make_desc("l", "Linear", inputs=["t"], output="x", in_features=E, out_features=out, seq_len=seq, use_bias=False, params_count=w.size)]
+    m = rt.GraphModel(descs, abi.PREC_BF16X2)
+    m.upload_weights(0, g)
+    m.upload_weights(1, w)
+    m.plan({"x": (seq * E, False)}, batch)
+    got = m.forward({"x": (x, False)}, batch, seq * out)
+    m.close()
+    for i in sorted({0, batch // 2, batch - 1}):
+        want = port.rmsnorm(x[i], g, float(descs[0].eps)).reshape(seq, E).astype(np.float64) @ w.reshape(out, E).T.astype(np.float64)
+        assert np.linalg.norm(got[i] - want.ravel()) <= 1e-5 * np.linalg.norm(want)
