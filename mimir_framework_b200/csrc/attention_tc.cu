@@ -832,7 +832,7 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const int keys_seen = p.causal ? min(p.seq, row + 1) : p.seq;
       for (int s = 0; s < p.splits; ++s) {
         const float ls = ld_cluster_f32(mapa_shared(ml_addr + AT_BQ * 4, s));
-        if (!(ls > 0.0f)) continue;
+        if (ls == 0.0f) continue;  // no key of this part is visible to the row (a NaN sum is an overflow and has to reach the result)
         const float w = fast_exp2((ld_cluster_f32(mapa_shared(ml_addr, s)) - m) * LOG2E);
         l += w * ls;
         const int k0 = all_tiles * s / p.splits * AT_BK, k1 = min(all_tiles * (s + 1) / p.splits * AT_BK, keys_seen);
