@@ -465,6 +465,10 @@ int mimir_b200_check_device(void* stream);
  * mimir_b200_check_device returns E_TIMEOUT ("site 90"); calls after that work as usual.  Nothing faults or hangs.
  * No counterpart in the reference. */
 int mimir_b200_selftest_wait_timeout(unsigned long long limit_ns, void* stream);
+/* Leaves the counters of the long-sample RMSNorm of `stream` as a launch whose wait gave up leaves them: `tickets` chunks
+ * drawn and, with `flag`, the mark that it gave up.  Until the next mimir_b200_check_device that reports it, RMSNorms of
+ * samples above 16 384 elements on that stream write nothing and report E_TIMEOUT.  No counterpart in the reference. */
+int mimir_b200_selftest_norm_gave_up(unsigned tickets, int flag, void* stream);
 /* Live timing of the contraction (GEMM) kernel: while enabled, every launch is bracketed by CUDA
  * events on the launching stream; profile_read synchronises, returns the summed duration and the
  * number of launches, and clears the record.  No counterpart in the reference. */

@@ -299,8 +299,11 @@ bool rmsnorm_onepass_ok(int batch, int64_t n);
 // capturing) and keeps it, at a fixed address, until norm_scratch_release: call on the stream's device.
 int norm_scratch_reserve(cudaStream_t st);
 void norm_scratch_release(cudaStream_t st);
-// After a bounded wait gave up: the one-pass RMSNorm's counters and slots of the current device back to zero.
+// After a bounded wait gave up: the one-pass RMSNorm's counters and slots of the current device back to zero, of the streams where a
+// launch of it left its flag.
 void norm_scratch_clear();
+// Leaves the counters of `st` as a launch that gave up leaves them: `tickets` drawn, and the flag up or not.
+int norm_scratch_selftest_gave_up(unsigned tickets, int flag, cudaStream_t st);
 int launch_groupnorm(const float* x, const float* gamma, const float* beta, float* y, int batch, int ch, int hw,
                      int groups, float eps, int act, const float* residual, cudaStream_t st);
 int launch_softmax(const float* x, float* y, int batch, int64_t n, int log_softmax, cudaStream_t st);

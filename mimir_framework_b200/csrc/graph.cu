@@ -2186,6 +2186,11 @@ int mimir_b200_selftest_wait_timeout(unsigned long long limit_ns, void* stream) 
   return launch_wait_timeout_selftest(limit_ns, static_cast<cudaStream_t>(stream));
 }
 
+int mimir_b200_selftest_norm_gave_up(unsigned tickets, int flag, void* stream) {
+  if (!ctx().initialised) return fail(MIMIR_B200_E_NOT_INIT, "mimir_b200_init has not been called");
+  return norm_scratch_selftest_gave_up(tickets, flag, static_cast<cudaStream_t>(stream));
+}
+
 int mimir_b200_profile_gemm(int enable) {
   if (!ctx().initialised) return fail(MIMIR_B200_E_NOT_INIT, "mimir_b200_init has not been called");
   ctx().prof_gemm = enable != 0;

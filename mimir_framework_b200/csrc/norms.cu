@@ -406,16 +406,34 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   };
   if (p.rows == 1) prefetch_gamma(static_cast<long long>(blockIdx.x) * CHUNK);
   pdl_wait();
-  // (one row needs no order among its CTAs, which are resident together: it saves the round trip to the counter)
-  if (tid == 0) s_id = p.rows == 1 ? blockIdx.x : atomicAdd(p.ticket, 1u);
+  // Counters and slots hold nothing of use after a wait gave up, until the host clears them: the launches in between write nothing and
+  // report it again (the host may have read the word already).  (One row needs no order among its CTAs, which are resident
+  // together: it saves the round trip to the counter, and the flag is looked at when it is there.)
+  volatile unsigned* abort_flag = p.ticket + 1;
+  unsigned gave_up = 0u;
+  if (tid == 0) {
+    gave_up = *abort_flag;
+    unsigned id = blockIdx.x;
+    if (p.rows > 1) {
+      id = atomicAdd(p.ticket, 1u);
+      if (gave_up) id = 0xffffffffu;
+    }
+    s_id = id;
+  }
   __syncthreads();
   const long long row = s_id / static_cast<unsigned>(p.chunks);
+  if (row >= p.rows) {  // given up, or a counter that did not start from zero: no row to work on
+    if (tid == 0) {
+      *abort_flag = 1u;
+      atomicCAS(p.err_word, 0, 25);
+    }
+    return;
+  }
   const int c = static_cast<int>(s_id % static_cast<unsigned>(p.chunks));
   const long long off = static_cast<long long>(c) * CHUNK;
   const int n = static_cast<int>(min(static_cast<long long>(CHUNK), p.len - off));
   const float* g = p.x + row * p.len + off;
   if (p.rows > 1) prefetch_gamma(off);
-  volatile unsigned* abort_flag = p.ticket + 1;
 
   // ---- the chunk into shared memory: bulk copies when source and size allow, plain loads otherwise ----
   const bool bulk = (reinterpret_cast<uintptr_t>(g) & 15) == 0 && (n & 3) == 0;
@@ -496,8 +514,11 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   }
   const double sd = block_sum_f64(mine, red);
   if (staged && !mbar_wait(&gamma_bar, 0, &s_abort, p.err_word, 24)) ok = false;  // (asked for before the sums were; nobody leaves before it lands)
-  if (__syncthreads_or(!ok)) {  // a wait gave up: the error word is set, nothing is written
-    if (tid == 0) *abort_flag = 1u;
+  if (__syncthreads_or(!ok || gave_up)) {  // a wait gave up: nothing is written
+    if (tid == 0) {
+      *abort_flag = 1u;
+      atomicCAS(p.err_word, 0, 25);
+    }
     return;
   }
   const float rms = sqrtf(static_cast<float>(sd) / static_cast<float>(p.len) + p.eps);
@@ -1056,9 +1077,24 @@ void norm_scratch_clear() {
   std::lock_guard<std::mutex> lk(g_norm_mu);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return;
-  for (auto& kv : g_norm_scratch)
-    if (kv.first.first == dev) cudaMemset(reinterpret_cast<uint8_t*>(kv.second.p) + NORM_SCRATCH_BYTES, 0, NORM_SCRATCH_BYTES);
+  for (auto& kv : g_norm_scratch) {
+    if (kv.first.first != dev) continue;
+    // only where a launch gave up: the other streams' launches may be running
+    uint8_t* op = reinterpret_cast<uint8_t*>(kv.second.p) + NORM_SCRATCH_BYTES;
+    unsigned gave_up = 0;
+    if (cudaMemcpy(&gave_up, op + sizeof(unsigned), sizeof(unsigned), cudaMemcpyDeviceToHost) == cudaSuccess && gave_up) cudaMemset(op, 0, NORM_SCRATCH_BYTES);
+  }
   cudaDeviceSynchronize();
+}
+
+int norm_scratch_selftest_gave_up(unsigned tickets, int flag, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_norm_mu);
+  float* p = nullptr;
+  MB_TRY(norm_scratch(st, &p));
+  const unsigned words[2] = {tickets, flag ? 1u : 0u};
+  MB_CUDA(cudaMemcpyAsync(reinterpret_cast<uint8_t*>(p) + NORM_SCRATCH_BYTES, words, sizeof(words), cudaMemcpyHostToDevice, st));
+  MB_CUDA(cudaStreamSynchronize(st));
+  return MIMIR_B200_OK;
 }
 
 int launch_layernorm(const float* x, const float* gamma, const float* beta, float* y, int64_t rows, int64_t n, float eps,

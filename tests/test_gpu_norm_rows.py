@@ -90,3 +90,28 @@ def test_one_pass_rmsnorm_into_planes(rt, batch, seq):
     for i in sorted({0, batch // 2, batch - 1}):
         want = port.rmsnorm(x[i], g, float(descs[0].eps)).reshape(seq, E).astype(np.float64) @ w.reshape(out, E).T.astype(np.float64)
         assert np.linalg.norm(got[i] - want.ravel()) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("rows,n,tickets,flag", [(1, 24576, 0, 1), (3, 24577, 12, 1), (3, 24577, 12, 0), (3, 24577, 5, 1), (40, 40960, 2**31 - 1, 1), (40, 40960, 2**31 - 1, 0)])
+def test_rmsnorms_behind_one_that_gave_up_write_nothing(rt, rows, n, tickets, flag):
+    """After a bounded wait of the one-pass RMSNorm ran out its ticket counter stands where the launch left it.  The norms queued behind
+    it have no row to work on: they leave their output alone and report the timeout, and the first norm after the report is right."""
+    import torch
+
+    lib = rt.lib()
+    rt.check(lib.mimir_b200_check_device(None))
+    x = torch.randn(rows, n, device="cuda")
+    y = torch.full((rows, n), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    run = lambda: rt.check(lib.mimir_b200_dev_rmsnorm(x.data_ptr(), None, 0, y.data_ptr(), rows, n, 1e-5, None))
+    rt.check(lib.mimir_b200_selftest_norm_gave_up(tickets, flag, None))
+    run()
+    run()
+    assert lib.mimir_b200_check_device(None) == abi.E_TIMEOUT
+    assert bool((y == 7.0).all())
+    assert lib.mimir_b200_check_device(None) == abi.OK
+    run()
+    rt.check(lib.mimir_b200_check_device(None))
+    want = x.double() / torch.sqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-5)
+    # (the reference's sequential fp32 sum, which the kernel follows, is off by up to n roundings of 2^-24 of the sum of squares)
+    assert float((y - want).abs().max()) <= (1e-6 + n * 2.0**-25) * float(want.abs().max())
