@@ -136,6 +136,7 @@ struct LayerRT {
   bool res_up = false;                // Conv2d: res_v is the INPUT of a 2 x 2 nearest upsample that the epilogue applies
   std::vector<int> add_v;             // Embedding: tensors of the Adds folded into it (graph inputs), in layer order
   int pre_ln = -1;                    // a token-wise LayerNorm folded into this layer (index), see fusion 1f
+  size_t ln_off = 0;                  // of its result in the workspace, where the norm may have to run on its own (0: never)
   bool in_up = false;                 // Conv2d: in_v[0] is the INPUT of a 2 x 2 nearest upsample that the layout pass applies
   int gn_emit_for = -1;               // Conv2d: index of the GroupNorm layer whose statistics this layer's GEMM epilogue emits
   int gn_stats_from = -1;             // GroupNorm: index of the Conv2d layer that emits its statistics
@@ -1218,6 +1219,15 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       switch (L.lt) {
         case LT::Linear:
           L.ws_bytes = linear_ws_bytes(static_cast<int>(rows), L.in_f, L.out_f, m->precision, L.read_split);
+          L.ln_off = 0;
+          if (L.pre_ln >= 0) {
+            // a caller's own buffer (a graph input, the output) need not start on the 16 bytes that the folded form reads by
+            const int r = root_of(m->tensors, L.in_v[0]);
+            if (m->tensors[r].producer == -1 || r == out_root) {
+              L.ln_off = align256(L.ws_bytes > 0 ? L.ws_bytes : 1);
+              L.ws_bytes = L.ln_off + align256(static_cast<size_t>(rows) * L.in_f * sizeof(float));
+            }
+          }
           flops += 2ull * rows * L.in_f * L.out_f;
           break;
         case LT::Attention: {
@@ -1358,6 +1368,14 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         if (L.emit_f32) e.y_f32 = f32p(L.out_v);
         if (L.emit_split) e.y_split = splitp(L.out_v);
         e.ws = ws; e.ws_bytes = L.ws_bytes;
+        if (L.ln_off && (reinterpret_cast<uintptr_t>(e.x_f32) & 15) != 0) {
+          float* normed = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + L.ln_off);
+          e.ws_bytes = L.ln_off;
+          s = launch_layernorm(e.x_f32, e.pre.gamma, e.pre.beta, normed, e.rows, L.in_f, e.pre.eps, st);
+          if (s != MIMIR_B200_OK) break;
+          e.x_f32 = normed;
+          e.pre.on = false;
+        }
         s = linear_exec(e, st);
         break;
       }

@@ -44,6 +44,37 @@ def test_few_rows_against_float64(rt, norm, m, n, k):
     assert np.linalg.norm(got - want) <= 2e-6 * np.linalg.norm(want) + 1e-7
 
 
+@pytest.mark.parametrize("shift", [0, 1, 2])
+@pytest.mark.parametrize("m,n,k,micro", [(1, 1, 4, 1), (5, 100, 768, 1), (16, 65, 4096, 1), (2, 40, 1028, 1), (3, 33, 12, 3)])
+def test_folded_layernorm_of_a_device_input_at_any_address(rt, m, n, k, micro, shift):
+    """The norm of a graph input (here behind an alias) is folded at plan time; the caller's buffer, and each micro-batch in it, may
+    start anywhere."""
+    import torch
+
+    r = np.random.default_rng(m + n)
+    x = r.standard_normal((micro, m, k)).astype(np.float32)
+    w, b = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32), r.standard_normal(n).astype(np.float32)
+    g, be = (1 + 0.1 * r.standard_normal(k)).astype(np.float32), r.standard_normal(k).astype(np.float32)
+    descs = [make_desc("i", "Identity", inputs=["x"], output="a"),
+             make_desc("n", "LayerNorm", inputs=["a"], output="h", in_features=k, affine=1, use_bias=1, eps=1e-5, params_count=2 * k),
+             make_desc("l", "Linear", inputs=["h"], output="x", in_features=k, out_features=n, seq_len=m, use_bias=1, params_count=n * k + n)]
+    mod = rt.GraphModel(descs, pipeline=micro)
+    mod.upload_weights(1, np.concatenate([g, be]))
+    mod.upload_weights(2, np.concatenate([w.ravel(), b]))
+    mod.plan({"x": (m * k, False)}, micro)
+    buf = torch.zeros(micro * m * k + 4, device="cuda")
+    buf[shift:shift + x.size] = torch.from_numpy(x.ravel())
+    out = torch.empty(micro * m * n, device="cuda")
+    h = x.astype(np.float64)
+    want = (((h - h.mean(-1, keepdims=True)) / np.sqrt(h.var(-1, keepdims=True) + 1e-5) * g + be) @ w.astype(np.float64).T + b).ravel()
+    for _ in range(3):  # layer by layer, captured, replayed
+        out.zero_()
+        mod.forward_device({"x": (buf[shift:].data_ptr(), m * k, False)}, micro, out.data_ptr(), out.numel(), torch.cuda.current_stream().cuda_stream)
+        got = out.cpu().numpy()
+        assert np.linalg.norm(got - want) <= 2e-6 * np.linalg.norm(want) + 1e-7
+    mod.close()
+
+
 @pytest.mark.parametrize("bf16", [False, True])
 @pytest.mark.parametrize("batch,heads,hd,prefix", [(1, 3, 64, 15), (2, 4, 32, 31), (3, 2, 128, 7), (16, 4, 64, 16), (1, 1, 64, 1)])
 def test_decode_steps_against_the_full_forward(rt, bf16, batch, heads, hd, prefix):
