@@ -141,25 +141,43 @@ void release_owned_buffers() {
   ob.pool.clear();
 }
 
-// Reads (and clears) the word that kernels with bounded waits set when a wait gave up.
-int check_device_error_word(cudaStream_t st) {
-  MB_TRY(enqueue_error_word(st));
-  MB_CUDA(cudaStreamSynchronize(st));
-  return read_error_word(st);
+ErrorWatch::ErrorWatch() : c_(ctx()), clears_(c_.error_clears.load()) {}
+ErrorWatch::~ErrorWatch() {
+  if (in_flight_) cudaStreamSynchronize(st_);  // (the call failed behind the copy, which may not land in the next call's word)
+  if (word_ && word_ != &own_) {
+    std::lock_guard<std::mutex> lk(c_.error_mu);
+    c_.error_words.push_back(word_);
+  }
 }
-int enqueue_error_word(cudaStream_t st) {
-  MB_CUDA(cudaMemcpyAsync(ctx().host_error_word, ctx().dev_error_word, sizeof(int), cudaMemcpyDeviceToHost, st));
+int ErrorWatch::enqueue(cudaStream_t st) {
+  if (!word_) {
+    std::lock_guard<std::mutex> lk(c_.error_mu);
+    if (c_.error_words.empty()) {
+      word_ = &own_;
+    } else {
+      word_ = c_.error_words.back();
+      c_.error_words.pop_back();
+    }
+  }
+  st_ = st;
+  in_flight_ = true;
+  MB_CUDA(cudaMemcpyAsync(word_, c_.dev_error_word, sizeof(int), cudaMemcpyDeviceToHost, st));
   return MIMIR_B200_OK;
 }
-int read_error_word(cudaStream_t st) {
-  const int w = *static_cast<volatile int*>(ctx().host_error_word);
+int ErrorWatch::read(cudaStream_t st) {
+  in_flight_ = false;
+  const int w = *static_cast<volatile int*>(word_);
+  std::lock_guard<std::mutex> lk(c_.error_mu);  // (waits for a clear that is under way, which the copy may have come behind)
   if (w != 0) {
-    cudaMemsetAsync(ctx().dev_error_word, 0, sizeof(int), st);
+    cudaMemsetAsync(c_.dev_error_word, 0, sizeof(int), st);
     cudaStreamSynchronize(st);
     norm_scratch_clear();
-    return fail(MIMIR_B200_E_TIMEOUT, "a device-side wait gave up (site %d)", w);
+    c_.last_error_site = w;
+    c_.error_clears.fetch_add(1);
+  } else if (c_.error_clears.load() == clears_) {
+    return MIMIR_B200_OK;
   }
-  return MIMIR_B200_OK;
+  return fail(MIMIR_B200_E_TIMEOUT, "a device-side wait gave up (site %d)", c_.last_error_site);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -516,10 +534,11 @@ int mimir_b200_init(int device, size_t hbm_budget_bytes) {
   }
   c.dev_error_word = static_cast<int*>(w);
   MB_CUDA(cudaMemset(c.dev_error_word, 0, 256));
+  constexpr int CALLS = 64;  // at a time with a page-locked word each
   void* hw = nullptr;
-  MB_CUDA(cudaHostAlloc(&hw, 256, cudaHostAllocPortable));
-  c.host_error_word = static_cast<int*>(hw);
-  *c.host_error_word = 0;
+  MB_CUDA(cudaHostAlloc(&hw, CALLS * sizeof(int), cudaHostAllocPortable));
+  std::lock_guard<std::mutex> el(c.error_mu);
+  for (int i = 0; i < CALLS; ++i) c.error_words.push_back(static_cast<int*>(hw) + i);
   return MIMIR_B200_OK;
 }
 

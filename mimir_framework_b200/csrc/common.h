@@ -85,9 +85,12 @@ struct Context {
   TempPool temps;
   HostCopier* copier = nullptr;
   std::atomic<uint64_t> launches{0};
-  // One device word that kernels with bounded waits set when a wait gives up.
+  // One device word that kernels with bounded waits set when a wait gives up, read by the calls through an ErrorWatch (ops.h).
   int* dev_error_word = nullptr;
-  int* host_error_word = nullptr;  // page-locked copy of it that check_device_error_word reads through
+  std::mutex error_mu;                     // held while the word is looked at on the host and cleared
+  std::vector<int*> error_words;           // page-locked words that no call uses at the moment
+  std::atomic<uint64_t> error_clears{0};
+  int last_error_site = 0;
   // Optional live timing of the contraction kernel: pairs of events recorded on the launching
   // stream around every GEMM launch while enabled (read back by mimir_b200_profile_read).
   bool prof_gemm = false;

@@ -1964,6 +1964,7 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
     MB_CUDA(cudaEventCreate(&m->ev1));
   }
   MB_TRY(ensure_pipeline_objects(m));
+  ErrorWatch errors;
   const int micro = m->planned_micro, P = m->pipeline;
   uint8_t* bufs[2] = {m->arena, m->arena2 ? m->arena2 : m->arena};
   MB_CUDA(cudaEventRecord(m->ev0, m->s_comp));
@@ -1996,14 +1997,14 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
     MB_TRY(run_layers_cached(m, micro, b, m->s_comp, arena));
     MB_CUDA(cudaEventRecord(m->ev_comp[c], m->s_comp));
     MB_CUDA(cudaStreamWaitEvent(m->s_d2h, m->ev_comp[c], 0));
-    if (c + 1 == P) MB_TRY(enqueue_error_word(m->s_d2h));  // (this stream has waited for every micro-batch's compute)
+    if (c + 1 == P) MB_TRY(errors.enqueue(m->s_d2h));  // (this stream has waited for every micro-batch's compute)
     MB_TRY(copy_to_host(out_host + static_cast<size_t>(c) * micro * ot.n, arena + ot.off_f32, static_cast<size_t>(ot.n) * micro * 4, m->s_d2h));
     MB_CUDA(cudaEventRecord(m->ev_d2h[c], m->s_d2h));
   }
   MB_CUDA(cudaEventRecord(m->ev1, m->s_comp));
   MB_CUDA(cudaStreamSynchronize(m->s_d2h));
   MB_CUDA(cudaEventSynchronize(m->ev1));
-  MB_TRY(read_error_word(m->s_comp));
+  MB_TRY(errors.read(m->s_comp));
   cudaEventElapsedTime(&m->last_ms, m->ev0, m->ev1);
   ctx().stats.ms_last_forward = m->last_ms;
   ctx().stats.flops_last_forward = m->flops * P;
@@ -2195,7 +2196,11 @@ int mimir_b200_get_stats(MimirB200Stats* out) {
 // Reads the device error word that bounded waits set; OK when no wait gave up.
 int mimir_b200_check_device(void* stream) {
   if (!ctx().initialised) return fail(MIMIR_B200_E_NOT_INIT, "mimir_b200_init has not been called");
-  return check_device_error_word(static_cast<cudaStream_t>(stream));
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  ErrorWatch errors;
+  MB_TRY(errors.enqueue(st));
+  MB_CUDA(cudaStreamSynchronize(st));
+  return errors.read(st);
 }
 
 // Live timing of the contraction kernel with CUDA events on the launching stream.

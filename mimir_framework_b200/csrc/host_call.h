@@ -12,6 +12,7 @@ namespace mb {
 // waits for the device, when the call failed before it had synchronised).
 struct Temps {
   std::vector<std::pair<void*, size_t>> bufs;
+  ErrorWatch errors;
   bool synced = false;
   ~Temps() {
     for (auto& b : bufs) temp_free(b.first, b.second, synced);
@@ -39,11 +40,11 @@ struct Temps {
 
 // The last step of a call: result to the host, one synchronisation, device error word.
 inline int finish_download(Temps& t, float* host, const float* dev, size_t n) {
-  MB_TRY(enqueue_error_word(nullptr));
+  MB_TRY(t.errors.enqueue(nullptr));
   MB_TRY(copy_to_host(host, dev, n * sizeof(float), nullptr));
   MB_CUDA(cudaStreamSynchronize(nullptr));
   t.synced = true;
-  return read_error_word(nullptr);
+  return t.errors.read(nullptr);
 }
 
 #define MB_REQUIRE_INIT() \

@@ -10,10 +10,26 @@ namespace mb {
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 void precision_planes(int precision, int* a_planes, int* w_planes);
 size_t split_bytes(int64_t rows, int k, int planes);
-// reads (and clears) the word that bounded waits set; the two halves let a caller fold the copy into a synchronisation of its own
-int check_device_error_word(cudaStream_t st);
-int enqueue_error_word(cudaStream_t st);
-int read_error_word(cudaStream_t st);
+// The device's error word as one call sees it, from the call's first launch (construction) to its last synchronisation.  The word is
+// shared by every call on the device, and whoever finds it set clears it: so each call copies it into a page-locked word of its
+// own, and a call during which another one cleared it reports the error as well (it may have been this call's).
+class ErrorWatch {
+ public:
+  ErrorWatch();
+  ~ErrorWatch();
+  ErrorWatch(const ErrorWatch&) = delete;
+  ErrorWatch& operator=(const ErrorWatch&) = delete;
+  int enqueue(cudaStream_t st);  // copies the word in stream order
+  int read(cudaStream_t st);     // after a synchronisation of the stream that carried the copy; clears on `st`
+
+ private:
+  Context& c_;
+  uint64_t clears_;
+  int* word_ = nullptr;
+  int own_ = 0;  // where no page-locked word is left
+  bool in_flight_ = false;
+  cudaStream_t st_ = nullptr;
+};
 
 // A token-wise LayerNorm folded into the contraction that reads it: x is then the LayerNorm's input.
 struct PreLayerNorm {

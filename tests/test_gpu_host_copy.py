@@ -49,3 +49,39 @@ def test_idle_call_buffers_are_not_counted(rt):
     before = rt.guard_stats()["current"]
     rt.eltwise(abi.ELT_RELU, np.ones(1 << 20, np.float32))
     assert rt.guard_stats()["current"] == before
+
+
+@pytest.mark.parametrize("large", ["input", "output"])
+def test_a_call_reports_its_own_wait_that_gave_up(rt, large):
+    """Two threads on one device.  A wait runs out during the large call; the other thread's small calls see the device's error word
+    as well and clear it while the large call still copies.  The large call has to report it all the same."""
+    lib = rt.lib()
+    rt.check(lib.mimir_b200_check_device(None))
+    x = np.ones(16 << 20, np.float32)
+    a, w = np.ones((4096, 4), np.float32), np.ones((4096, 4), np.float32)
+    call = {"input": lambda: rt.eltwise(abi.ELT_RELU, x), "output": lambda: rt.linear_forward(a, w, None, 4096, 4, 4096)}[large]
+    small = np.ones(64, np.float32)
+    call()
+    done = threading.Event()
+
+    def others():
+        rt.init(0)
+        done.wait(0.02)  # the large call has begun
+        while not done.is_set():
+            try:
+                rt.eltwise(abi.ELT_RELU, small)
+            except rt.MimirB200Error as e:
+                assert e.status == abi.E_TIMEOUT
+
+    t = threading.Thread(target=others)
+    rt.check(lib.mimir_b200_selftest_wait_timeout(90_000_000, None))  # ahead of the calls in the stream; gives up after 90 ms
+    t.start()
+    try:
+        with pytest.raises(rt.MimirB200Error) as e:
+            call()
+    finally:
+        done.set()
+        t.join()
+    assert e.value.status == abi.E_TIMEOUT
+    rt.check(lib.mimir_b200_check_device(None))
+    call()
