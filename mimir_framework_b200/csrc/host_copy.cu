@@ -71,8 +71,8 @@ struct Job {
 
 }  // namespace
 
-// The helpers and the ring of one device.  One job at a time (`call` is held for the whole copy); a helper that wakes late
-// finds no piece left.  `active` counts the helpers that may still touch the current job.
+// The helpers and the ring of one device.  One job at a time (`call` is held for the whole copy, waits for the caller's own stream
+// included, so nobody queues for it); a helper that wakes late finds no piece left.  `active` counts the helpers that may still touch the current job.
 struct HostCopier {
   std::mutex call, mu;
   std::condition_variable cv;
@@ -84,6 +84,7 @@ struct HostCopier {
   uint8_t* ring = nullptr;
   cudaEvent_t ev[RING] = {};
   bool in_flight[RING] = {};
+  cudaStream_t on[RING] = {};  // the stream of a slot's copy in flight
 
   int init() {
     if (ring) return MIMIR_B200_OK;
@@ -156,12 +157,13 @@ struct HostCopier {
         e = cudaMemcpyAsync(j.dev + s * j.segment, ring + (s % RING) * SEGMENT, j.seg_bytes(s), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(ev[s % RING], st);
         in_flight[s % RING] = true;
+        on[s % RING] = st;
         if (s + RING < j.segments && e == cudaSuccess) free_slot(s + RING);
       }
       return e;
     }
     auto fetch = [&](size_t s) {
-      if (in_flight[s % RING] && e == cudaSuccess) e = cudaEventSynchronize(ev[s % RING]);  // an earlier job's, on another stream
+      if (in_flight[s % RING] && e == cudaSuccess) e = cudaEventSynchronize(ev[s % RING]);  // an earlier job's
       in_flight[s % RING] = false;
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(ring + (s % RING) * SEGMENT, j.dev + s * j.segment, j.seg_bytes(s), cudaMemcpyDeviceToHost, st);
@@ -183,14 +185,32 @@ struct HostCopier {
     return e;
   }
 
-  int copy(Job& j, cudaStream_t st) {
-    std::lock_guard<std::mutex> one(call);
+  // Does a copy of another stream, which may stand behind that stream's kernels, hold one of the first slots?
+  bool held_by_others(const Job& j, cudaStream_t st) {
+    for (size_t s = 0; s < j.segments && s < RING; ++s)
+      if (in_flight[s] && on[s] != st) {
+        if (cudaEventQuery(ev[s]) != cudaSuccess) return true;
+        in_flight[s] = false;
+      }
+    return false;
+  }
+
+  // *taken = false: the ring is another call's at the moment, nothing was done.  Its copies may stand behind kernels, for
+  // which a call of another thread must not wait; the caller copies without the ring.
+  int copy(Job& j, cudaStream_t st, bool* taken) {
+    std::unique_lock<std::mutex> one(call, std::try_to_lock);
+    *taken = one.owns_lock();
+    if (!*taken) return MIMIR_B200_OK;
     MB_TRY(init());
     // about four segments, so that the first DMA starts early; whole pieces; at most a ring slot
     const size_t quarter = (j.bytes / 4 + PIECE - 1) / PIECE * PIECE;
     j.segment = quarter < SEGMENT ? quarter : SEGMENT;
     j.segments = (j.bytes + j.segment - 1) / j.segment;
     j.pieces = (j.bytes + PIECE - 1) / PIECE;
+    if (held_by_others(j, st)) {
+      *taken = false;
+      return MIMIR_B200_OK;
+    }
     if (j.pieces > 1) {  // (a single piece is the caller's own)
       {
         std::lock_guard<std::mutex> lk(mu);
@@ -233,23 +253,27 @@ bool pageable(const void* p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 int copy(bool to_device, void* dev, void* host, size_t bytes, cudaStream_t st) {
-  if (bytes < COPY_MIN || !pageable(host)) {
-    MB_CUDA(cudaMemcpyAsync(to_device ? dev : host, to_device ? host : dev, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st));
-    return MIMIR_B200_OK;
+  if (bytes >= COPY_MIN && pageable(host)) {
+    HostCopier* c;
+    {
+      static std::mutex mu;
+      std::lock_guard<std::mutex> lk(mu);
+      if (!ctx().copier) ctx().copier = new HostCopier();  // (never destroyed at exit: a helper may be waiting in it)
+      c = ctx().copier;
+    }
+    Job j;
+    j.to_device = to_device;
+    j.dev = static_cast<uint8_t*>(dev);
+    j.host = static_cast<uint8_t*>(host);
+    j.bytes = bytes;
+    bool taken = false;
+    MB_TRY(c->copy(j, st, &taken));
+    if (taken) return MIMIR_B200_OK;
+    // (the driver has locks of its own: while one thread's copy of pageable memory stands behind a kernel the others' wait)
+    MB_CUDA(cudaStreamSynchronize(st));
   }
-  HostCopier* c;
-  {
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!ctx().copier) ctx().copier = new HostCopier();  // (never destroyed at exit: a helper may be waiting in it)
-    c = ctx().copier;
-  }
-  Job j;
-  j.to_device = to_device;
-  j.dev = static_cast<uint8_t*>(dev);
-  j.host = static_cast<uint8_t*>(host);
-  j.bytes = bytes;
-  return c->copy(j, st);
+  MB_CUDA(cudaMemcpyAsync(to_device ? dev : host, to_device ? host : dev, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st));
+  return MIMIR_B200_OK;
 }
 }  // namespace
 

@@ -1,6 +1,7 @@
 """Copies between pageable host memory and the device (csrc/host_copy.cu) at the sizes where they change form - one piece, one
 segment, a full ring, and one element on either side - bit for bit, and from several threads at once."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -85,3 +86,51 @@ def test_a_call_reports_its_own_wait_that_gave_up(rt, large):
     assert e.value.status == abi.E_TIMEOUT
     rt.check(lib.mimir_b200_check_device(None))
     call()
+
+
+@pytest.mark.parametrize("waits_with", ["its copy in", "its copy out", "copies in flight", "its copy out, and a second call without the ring"])
+def test_a_copy_does_not_wait_for_another_call_s_kernels(rt, waits_with):
+    """A per-op call stands behind a 90 ms kernel on the default stream.  A model on its own streams copies in, runs and copies out
+    meanwhile, whatever the waiting call holds of the page-locked ring: all of it, for a copy in larger than the ring or for a copy
+    out, or the slots of a copy in that it has left behind (its result is small and page-locked: inside a small copy to pageable memory
+    the driver itself makes other threads' copies wait)."""
+    import torch
+
+    from mimir_framework_b200.abi import make_desc
+
+    lib = rt.lib()
+    rt.check(lib.mimir_b200_check_device(None))
+    n = 1 << 20
+    x = np.random.default_rng(0).standard_normal(n).astype(np.float32)
+    m = rt.GraphModel([make_desc("r", "ReLU", inputs=["x"], output="x")])
+    m.plan({"x": (n, False)}, 1)
+    big = np.ones((48 if waits_with == "its copy in" else 4) << 18, np.float32)
+    mean = torch.empty(1).pin_memory()
+    pool = lambda: rt.check(lib.mimir_b200_global_avgpool(big.ctypes.data, mean.data_ptr(), 1, 1, 1024, 1024))
+    waiting = pool if waits_with == "copies in flight" else lambda: rt.eltwise(abi.ELT_RELU, big)
+    for _ in range(3):
+        m.forward({"x": (x, False)}, 1, n)
+        waiting()
+    done = threading.Event()
+
+    def blocked():
+        rt.init(0)
+        try:
+            waiting()
+        except rt.MimirB200Error as e:
+            assert e.status == abi.E_TIMEOUT  # (the 90 ms are a wait that gives up)
+        done.set()
+
+    ts = [threading.Thread(target=blocked) for _ in range(2 if "second" in waits_with else 1)]
+    rt.check(lib.mimir_b200_selftest_wait_timeout(90_000_000, None))
+    for t in ts:
+        t.start()
+    time.sleep(0.02)
+    got = m.forward({"x": (x, False)}, 1, n)
+    overtook = not done.is_set()
+    for t in ts:
+        t.join()
+    lib.mimir_b200_check_device(None)
+    m.close()
+    assert np.array_equal(got.ravel(), np.maximum(x, 0))
+    assert overtook
