@@ -90,44 +90,58 @@ void dev_free(void* p, size_t bytes) {
   ctx().guard.release(bytes);
 }
 
-void* TempPool::take(size_t* size) {
+void* TempPool::take(size_t asked, size_t* size) {
   std::lock_guard<std::mutex> lk(mu);
-  auto it = idle.lower_bound(*size);
-  if (it == idle.end() || it->first / 2 > *size) return nullptr;
+  auto it = idle.lower_bound(asked);
+  if (it == idle.end() || it->first / 2 > asked) return nullptr;
   void* p = it->second;
   *size = it->first;
-  bytes -= it->first;
+  bytes -= asked;
   idle.erase(it);
   return p;
 }
-bool TempPool::put(void* p, size_t size) {
+bool TempPool::put(void* p, size_t asked, size_t size) {
   std::lock_guard<std::mutex> lk(mu);
-  if (bytes + size > CAP) return false;
+  if (bytes + asked > CAP) return false;
   idle.emplace(size, p);
-  bytes += size;
+  bytes += asked;
   return true;
+}
+void TempPool::drop(size_t asked, size_t size) {
+  std::lock_guard<std::mutex> lk(mu);
+  bytes -= size - asked;
 }
 void TempPool::trim() {
   std::lock_guard<std::mutex> lk(mu);
-  for (auto& kv : idle) cudaFree(kv.second);
+  for (auto& kv : idle) {
+    cudaFree(kv.second);
+    bytes -= kv.first;
+  }
   idle.clear();
-  bytes = 0;
 }
 
-int temp_alloc(void** p, size_t* bytes, const char* tag) {
-  *bytes = (*bytes + 511) & ~size_t(511);
-  if (void* q = ctx().initialised ? ctx().temps.take(bytes) : nullptr) {
-    if (ctx().guard.request_why(*bytes) == 0) {
-      *p = q;
+int temp_alloc(TempBuffer* b, size_t bytes, const char* tag) {
+  *b = TempBuffer();
+  b->asked = b->size = (bytes + 511) & ~size_t(511);
+  if (void* q = ctx().initialised ? ctx().temps.take(b->asked, &b->size) : nullptr) {
+    if (ctx().guard.request_why(b->asked) == 0) {
+      b->p = q;
       return MIMIR_B200_OK;
     }
     cudaFree(q);  // refused: the ordinary path below words the refusal
+    ctx().temps.drop(b->asked, b->size);
+    b->size = b->asked;
   }
-  return dev_alloc(p, *bytes, tag);
+  return dev_alloc(&b->p, b->asked, tag);
 }
-void temp_free(void* p, size_t bytes, bool idle) {
-  if (p && idle && ctx().temps.put(p, bytes)) ctx().guard.release(bytes);
-  else dev_free(p, bytes);
+void temp_free(const TempBuffer& b, bool idle) {
+  if (!b.p) return;
+  if (idle && ctx().temps.put(b.p, b.asked, b.size)) {
+    ctx().guard.release(b.asked);
+    return;
+  }
+  dev_free(b.p, b.asked);
+  ctx().temps.drop(b.asked, b.size);
 }
 
 void release_owned_buffers() {

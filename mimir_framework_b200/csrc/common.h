@@ -62,16 +62,18 @@ struct OwnedBuffers {
 
 // Device buffers of finished host-pointer calls, kept for the next one: cudaMalloc and cudaFree of a call's five or six buffers
 // (each free waits for the device and unmaps) took 2.9 ms of the 3.8 ms that a 512 x 768 x 3072 Linear needed.  Bounded by
-// CAP bytes; not counted by the guard while idle (a reused buffer is requested from it like a new one); given back when the
-// guard's limit or the device runs short and at shutdown.  Buffers enter the pool only after the call has synchronised.
+// CAP bytes; given back when the guard's limit or the device runs short and at shutdown.  Buffers enter the pool only after the call
+// has synchronised.  The guard counts what a call asks for, reused buffer or new: whether a call fits does not depend on the
+// calls before it.  Idle buffers and the surplus of a larger buffer in use are `bytes`.
 struct TempPool {
   static constexpr size_t CAP = size_t(512) << 20;
   std::mutex mu;
   std::multimap<size_t, void*> idle;
   size_t bytes = 0;
-  void* take(size_t* size);        // the smallest idle buffer of at least *size (and at most twice it); *size becomes its size
-  bool put(void* p, size_t size);  // false: no room, the caller frees it
-  void trim();                     // frees every idle buffer
+  void* take(size_t asked, size_t* size);        // the smallest idle buffer of at least `asked` bytes (and at most twice that), of *size
+  bool put(void* p, size_t asked, size_t size);  // false: no room, the caller frees it
+  void drop(size_t asked, size_t size);          // a taken buffer has been freed instead
+  void trim();                                   // frees every idle buffer
 };
 
 struct HostCopier;  // host_copy.cu
@@ -134,9 +136,10 @@ int model_device(MimirB200ModelHandle m);
 // Budgeted device allocation: every cudaMalloc of the backend goes through these.
 int dev_alloc(void** p, size_t bytes, const char* tag);
 void dev_free(void* p, size_t bytes);
-// The same through the pool of the current device's idle call buffers; *bytes becomes the buffer's size.
-int temp_alloc(void** p, size_t* bytes, const char* tag);
-void temp_free(void* p, size_t bytes, bool idle);
+// The same through the pool of the current device's idle call buffers.
+struct TempBuffer { void* p = nullptr; size_t asked = 0, size = 0; };
+int temp_alloc(TempBuffer* b, size_t bytes, const char* tag);
+void temp_free(const TempBuffer& b, bool idle);
 // Copies in stream order that may involve pageable host memory (host_copy.cu).  The host side is done with when they return
 // for pageable memory (as with cudaMemcpyAsync); page-locked memory is copied asynchronously.
 int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);

@@ -1,7 +1,6 @@
 // host_call.h — helpers of the synchronous host-pointer entry points (copy in, run, copy out).
 #pragma once
 
-#include <utility>
 #include <vector>
 
 #include "ops.h"
@@ -11,16 +10,17 @@ namespace mb {
 // Device buffers of one host-pointer call, from the pool of idle buffers; back to it when the call returns (freed, which
 // waits for the device, when the call failed before it had synchronised).
 struct Temps {
-  std::vector<std::pair<void*, size_t>> bufs;
+  std::vector<TempBuffer> bufs;
   ErrorWatch errors;
   bool synced = false;
   ~Temps() {
-    for (auto& b : bufs) temp_free(b.first, b.second, synced);
+    for (auto& b : bufs) temp_free(b, synced);
   }
   int alloc(void** p, size_t bytes, const char* tag) {
-    size_t got = bytes ? bytes : 4;
-    MB_TRY(temp_alloc(p, &got, tag));
-    bufs.emplace_back(*p, got);
+    TempBuffer b;
+    MB_TRY(temp_alloc(&b, bytes ? bytes : 4, tag));
+    *p = b.p;
+    bufs.push_back(b);
     return MIMIR_B200_OK;
   }
   int upload(const float** dev, const float* host, size_t n, const char* tag) {

@@ -131,3 +131,23 @@ def test_check_no_leaks_follows_the_ten_megabyte_rule(backend):
     assert backend.allocator_check_no_leaks() is False
     backend.buffer_free(p)
     assert backend.allocator_check_no_leaks() == (cur // (1 << 20) < 10)
+
+
+@pytest.mark.parametrize("larger", [1, 1.5, 1.9, 3])
+def test_a_call_that_fits_the_budget_is_granted_whatever_ran_before(backend, larger):
+    """Host-pointer calls reuse the buffers of earlier ones, of up to twice the size asked for; the budget counts what the call asks for."""
+    lib, n = backend.lib(), 1 << 20  # (a multiple of the pool's 512 bytes)
+    base = backend.guard_stats()
+    x = np.random.default_rng(1).standard_normal(int(n * larger)).astype(np.float32)
+    backend.eltwise(abi.ELT_RELU, x)  # leaves two buffers of n * larger floats behind
+    try:
+        backend.check(lib.mimir_b200_guard_set_limit(base["current"] + 8 * n))
+        np.testing.assert_array_equal(backend.eltwise(abi.ELT_RELU, x[:n]), np.maximum(x[:n], 0))
+        backend.check(lib.mimir_b200_guard_set_limit(base["current"] + 8 * n - 512))
+        with pytest.raises(backend.MimirB200Error) as e:
+            backend.eltwise(abi.ELT_RELU, x[:n])
+        assert e.value.status == abi.E_OOM_BUDGET
+    finally:
+        backend.check(lib.mimir_b200_guard_set_limit(base["limit"]))
+    assert backend.guard_stats()["current"] == base["current"]
+    np.testing.assert_array_equal(backend.eltwise(abi.ELT_RELU, x), np.maximum(x, 0))
