@@ -469,6 +469,10 @@ int mimir_b200_selftest_wait_timeout(unsigned long long limit_ns, void* stream);
  * drawn and, with `flag`, the mark that it gave up.  Until the next mimir_b200_check_device that reports it, RMSNorms of
  * samples above 16 384 elements on that stream write nothing and report E_TIMEOUT.  No counterpart in the reference. */
 int mimir_b200_selftest_norm_gave_up(unsigned tickets, int flag, void* stream);
+/* Copies n floats from src to the device and back to dst, through page-locked staging of its own that meets a failure on the
+ * host: inject = 0 none, 1 no page-locked memory, 2 no second helper thread, 3 both.  *ring_copies: how many of the two copies
+ * were staged (0 in a call without page-locked memory, which copies directly).  No counterpart in the reference. */
+int mimir_b200_selftest_host_copy(int inject, const float* src, float* dst, size_t n, int* ring_copies);
 /* Live timing of the contraction (GEMM) kernel: while enabled, every launch is bracketed by CUDA
  * events on the launching stream; profile_read synchronises, returns the summed duration and the
  * number of launches, and clears the record.  No counterpart in the reference. */

@@ -145,6 +145,9 @@ void temp_free(const TempBuffer& b, bool idle);
 int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);
 int copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
 void release_host_copier();
+// src -> device -> dst through a copier of its own that meets failures on the host: `inject` 1 page-locked memory, 2 a second thread,
+// are not to be had
+int host_copy_selftest(int inject, const float* src, float* dst, size_t n, int* ring_copies);
 // Frees every buffer of the RuntimeAllocator verbs on the current device (shutdown).
 void release_owned_buffers();
 

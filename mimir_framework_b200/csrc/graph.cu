@@ -2209,6 +2209,12 @@ int mimir_b200_selftest_wait_timeout(unsigned long long limit_ns, void* stream) 
   return launch_wait_timeout_selftest(limit_ns, static_cast<cudaStream_t>(stream));
 }
 
+int mimir_b200_selftest_host_copy(int inject, const float* src, float* dst, size_t n, int* ring_copies) {
+  if (!ctx().initialised) return fail(MIMIR_B200_E_NOT_INIT, "mimir_b200_init has not been called");
+  if (!src || !dst || n == 0) return fail(MIMIR_B200_E_INVALID, "selftest: bad arguments");
+  return host_copy_selftest(inject, src, dst, n, ring_copies);
+}
+
 int mimir_b200_selftest_norm_gave_up(unsigned tickets, int flag, void* stream) {
   if (!ctx().initialised) return fail(MIMIR_B200_E_NOT_INIT, "mimir_b200_init has not been called");
   return norm_scratch_selftest_gave_up(tickets, flag, static_cast<cudaStream_t>(stream));

@@ -12,6 +12,8 @@
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
+#include <new>
+#include <system_error>
 #include <thread>
 
 #include "ops.h"
@@ -80,22 +82,43 @@ struct HostCopier {
   Job* job = nullptr;
   std::atomic<uint64_t> epoch{0};
   int active = 0;
-  bool stop = false;
+  bool stop = false, no_ring = false;
+  int inject = 0;  // host_copy_selftest: 1 no page-locked memory, 2 no second thread
   uint8_t* ring = nullptr;
   cudaEvent_t ev[RING] = {};
   bool in_flight[RING] = {};
   cudaStream_t on[RING] = {};  // the stream of a slot's copy in flight
 
-  int init() {
-    if (ring) return MIMIR_B200_OK;
-    for (auto& e : ev) MB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // The ring, and as many helpers as the machine starts; false: no ring to be had (asked for once), copies go without
+  bool init() {
+    if (ring) return true;
+    if (no_ring) return false;
+    void* p = nullptr;
+    cudaError_t e = inject & 1 ? cudaErrorMemoryAllocation : cudaHostAlloc(&p, RING * SEGMENT, cudaHostAllocPortable);
+    for (auto& v : ev)
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // (not an error of the copy's)
+      for (auto& v : ev) {
+        if (v) cudaEventDestroy(v);
+        v = nullptr;
+      }
+      if (p) cudaFreeHost(p);
+      no_ring = true;
+      return false;
+    }
+    ring = static_cast<uint8_t*>(p);
     const unsigned cores = std::thread::hardware_concurrency();
     const int helpers = cores >= 4 ? static_cast<int>(cores / 2 < MAX_HELPERS ? cores / 2 : MAX_HELPERS) : 0;
-    void* p = nullptr;
-    MB_CUDA(cudaHostAlloc(&p, RING * SEGMENT, cudaHostAllocPortable));
-    ring = static_cast<uint8_t*>(p);
-    for (int i = 0; i < helpers; ++i) threads.emplace_back([this] { loop(); });
-    return MIMIR_B200_OK;
+    try {
+      for (int i = 0; i < helpers; ++i) {
+        if ((inject & 2) && i > 0) throw std::system_error(std::make_error_code(std::errc::resource_unavailable_try_again));
+        threads.emplace_back([this] { loop(); });
+      }
+    } catch (...) {
+      // no more threads, or no memory: the caller moves what the ones that run do not
+    }
+    return true;
   }
 
   void loop() {
@@ -195,13 +218,12 @@ struct HostCopier {
     return false;
   }
 
-  // *taken = false: the ring is another call's at the moment, nothing was done.  Its copies may stand behind kernels, for
-  // which a call of another thread must not wait; the caller copies without the ring.
+  // *taken = false: there is no ring, or it is another call's at the moment; nothing was done.  Its copies may stand behind
+  // kernels, for which a call of another thread must not wait; the caller copies without the ring.
   int copy(Job& j, cudaStream_t st, bool* taken) {
     std::unique_lock<std::mutex> one(call, std::try_to_lock);
-    *taken = one.owns_lock();
+    *taken = one.owns_lock() && init();
     if (!*taken) return MIMIR_B200_OK;
-    MB_TRY(init());
     // about four segments, so that the first DMA starts early; whole pieces; at most a ring slot
     const size_t quarter = (j.bytes / 4 + PIECE - 1) / PIECE * PIECE;
     j.segment = quarter < SEGMENT ? quarter : SEGMENT;
@@ -252,23 +274,22 @@ bool pageable(const void* p) {
   }
   return a.type == cudaMemoryTypeUnregistered;
 }
-int copy(bool to_device, void* dev, void* host, size_t bytes, cudaStream_t st) {
+HostCopier* copier() {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!ctx().copier) ctx().copier = new (std::nothrow) HostCopier();  // (never destroyed at exit: a helper may be waiting in it)
+  return ctx().copier;
+}
+int copy(HostCopier* c, bool to_device, void* dev, void* host, size_t bytes, cudaStream_t st, bool* taken) {
+  *taken = false;
   if (bytes >= COPY_MIN && pageable(host)) {
-    HostCopier* c;
-    {
-      static std::mutex mu;
-      std::lock_guard<std::mutex> lk(mu);
-      if (!ctx().copier) ctx().copier = new HostCopier();  // (never destroyed at exit: a helper may be waiting in it)
-      c = ctx().copier;
-    }
     Job j;
     j.to_device = to_device;
     j.dev = static_cast<uint8_t*>(dev);
     j.host = static_cast<uint8_t*>(host);
     j.bytes = bytes;
-    bool taken = false;
-    MB_TRY(c->copy(j, st, &taken));
-    if (taken) return MIMIR_B200_OK;
+    if (c) MB_TRY(c->copy(j, st, taken));
+    if (*taken) return MIMIR_B200_OK;
     // (the driver has locks of its own: while one thread's copy of pageable memory stands behind a kernel the others' wait)
     MB_CUDA(cudaStreamSynchronize(st));
   }
@@ -277,8 +298,29 @@ int copy(bool to_device, void* dev, void* host, size_t bytes, cudaStream_t st) {
 }
 }  // namespace
 
-int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st) { return copy(true, dev, const_cast<void*>(host), bytes, st); }
-int copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st) { return copy(false, const_cast<void*>(dev), host, bytes, st); }
+int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st) {
+  bool taken;
+  return copy(bytes >= COPY_MIN ? copier() : nullptr, true, dev, const_cast<void*>(host), bytes, st, &taken);
+}
+int copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st) {
+  bool taken;
+  return copy(bytes >= COPY_MIN ? copier() : nullptr, false, const_cast<void*>(dev), host, bytes, st, &taken);
+}
+int host_copy_selftest(int inject, const float* src, float* dst, size_t n, int* ring_copies) {
+  HostCopier* c = new (std::nothrow) HostCopier();
+  if (!c) return fail(MIMIR_B200_E_INVALID, "selftest: no memory");
+  c->inject = inject;
+  void* dev = nullptr;
+  int s = dev_alloc(&dev, n * sizeof(float), "host copy selftest");
+  bool in = false, out = false;
+  if (s == MIMIR_B200_OK) s = copy(c, true, dev, const_cast<float*>(src), n * sizeof(float), nullptr, &in);
+  if (s == MIMIR_B200_OK) s = copy(c, false, dev, dst, n * sizeof(float), nullptr, &out);
+  if (s == MIMIR_B200_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) s = fail(MIMIR_B200_E_CUDA, "selftest: synchronisation failed");
+  dev_free(dev, n * sizeof(float));
+  delete c;
+  if (ring_copies) *ring_copies = static_cast<int>(in) + static_cast<int>(out);
+  return s;
+}
 void release_host_copier() {
   delete ctx().copier;
   ctx().copier = nullptr;

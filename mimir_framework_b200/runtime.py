@@ -108,6 +108,7 @@ _SIGS = {
     "mimir_b200_get_stats": [_P],
     "mimir_b200_check_device": [_P],
     "mimir_b200_selftest_wait_timeout": [C.c_ulonglong, _P],
+    "mimir_b200_selftest_host_copy": [C.c_int, _P, _P, C.c_size_t, _P],
     "mimir_b200_selftest_norm_gave_up": [C.c_uint, C.c_int, _P],
     "mimir_b200_profile_gemm": [C.c_int],
     "mimir_b200_profile_read": [_P, _P],

@@ -134,3 +134,15 @@ def test_a_copy_does_not_wait_for_another_call_s_kernels(rt, waits_with):
     m.close()
     assert np.array_equal(got.ravel(), np.maximum(x, 0))
     assert overtook
+
+
+@pytest.mark.parametrize("n", [100, 16 << 10, 1 << 20, (9 << 20) + 3])
+@pytest.mark.parametrize("inject", [0, 1, 2, 3])
+def test_copies_without_page_locked_memory_or_threads(rt, inject, n):
+    """No room for the ring, or no more threads: the copy is done all the same, and nothing is thrown through the C interface."""
+    import ctypes
+
+    src, dst, staged = np.random.default_rng(n).standard_normal(n).astype(np.float32), np.zeros(n, np.float32), ctypes.c_int(-1)
+    rt.check(rt.lib().mimir_b200_selftest_host_copy(inject, src.ctypes.data, dst.ctypes.data, n, ctypes.addressof(staged)))
+    assert np.array_equal(src, dst)
+    assert staged.value == (0 if inject & 1 or n < 16 << 10 else 2)
