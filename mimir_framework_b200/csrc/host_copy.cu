@@ -124,8 +124,9 @@ struct HostCopier {
   void loop() {
     uint64_t seen = 0;
     for (;;) {
-      // the copies of one call follow each other closely: stay awake for a moment before sleeping
-      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(100);
+      // the copies of one call follow each other closely: stay awake for a moment before sleeping (512 x 768 x 3072 from host memory:
+      // 540 us without, 528 with 10, 30 or 100 us; more than that only burns the cores, 0.5 ms of CPU time a call at 100 us)
+      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(20);
       while (epoch.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until) cpu_relax();
       Job* j;
       {
