@@ -51,6 +51,26 @@ def test_groupnorm(rt, batch, ch, h, w, groups, act):
     close(rt.groupnorm(x, g, b, batch, ch, h, w, groups, 1e-5, act), d / (1 + np.exp(-d)) if act >= 0 else d)
 
 
+@pytest.mark.parametrize("hw", [(2, 2), (3, 1)])
+def test_silu_over_its_whole_range(rt, hw):
+    """gamma = 0 and beta = v make every value of a channel silu(v): dense around zero, both ends of the exponential's range, the
+    largest floats and the infinities.  Two special-function instructions of 2^-22 each and a few roundings: 2^-21 relative; where
+    the reciprocal is flushed the true value is below 1.2e-36."""
+    v = np.concatenate([np.linspace(-100, 100, 7993), [0.0, -0.0, 1e-30, -1e-30, 1e-40, -87.3, -87.4, -88.0, -88.8, -1e4, -1e35, -3.4e38, 88.8, 1e35, 2.4e38, 3.4e38,
+                        np.inf, 64.0, 64.1]]).astype(np.float32)
+    v = np.append(v, np.zeros(-len(v) % 32, np.float32))
+    x = np.random.default_rng(0).standard_normal((1, v.size, *hw)).astype(np.float32)
+    got = np.asarray(rt.groupnorm(x, np.zeros(v.size, np.float32), v, 1, v.size, *hw, 32, 1e-5, abi.ELT_SILU)).reshape(v.size, -1)
+    d = v.astype(np.float64)[:, None]
+    with np.errstate(over="ignore"):
+        want = np.broadcast_to(d / (1 + np.exp(-d)), got.shape)
+    far = np.isinf(want)
+    assert np.array_equal(got[far], want[far])
+    assert (np.abs(got[~far] - want[~far]) <= 2.0**-21 * np.abs(want[~far]) + 1.2e-36).all()
+    v[:] = -np.inf
+    assert np.isnan(rt.groupnorm(x, np.zeros(v.size, np.float32), v, 1, v.size, *hw, 32, 1e-5, abi.ELT_SILU)).all()
+
+
 def test_unaligned_device_tensors(rt):
     import torch
 
