@@ -97,7 +97,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int kb1 = static_cast<int>(static_cast<long long>(p.kblocks) * (split + 1) / p.splits);
   const uint32_t tmem_cols = p.bn <= 32 ? 32u : (p.bn <= 64 ? 64u : 128u);
 
-  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -115,6 +114,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  // (behind the allocation: a kernel that starts now may take all of an SM's tensor memory and then wait for this one)
+  pdl_launch_dependents();
   const uint32_t tmem = tmem_slot;
   const bool conv = p.conv_ks > 0;
 

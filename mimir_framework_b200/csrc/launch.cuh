@@ -7,6 +7,8 @@
 // early only by short kernels that leave room on the SMs.  With it at the start of the large ones too (tensor-core tiles, attention,
 // row sweeps, layout passes) the waiting CTAs took registers and shared memory from the running ones and cost more than the launch
 // latency they hid (UNet 5.27 -> 5.46 ms, decoder with one prompt 1.66 -> 1.73 ms).
+// A kernel that allocates tensor memory calls it behind the allocation and a barrier: some kernels allocate ahead of their pdl_wait(),
+// and one that held an SM's columns while a CTA of the kernel it waits for still asked for them would wait for good.
 #pragma once
 
 #include <cuda_runtime.h>

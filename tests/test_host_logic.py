@@ -152,3 +152,24 @@ def test_selected_without_a_gpu_is_an_error_not_a_fallback(monkeypatch):
     monkeypatch.setenv("MIMIR_B200", "1")
     on = C.c_int(7)
     assert rt.lib().mimir_b200_init_from_env(C.byref(on)) == abi.E_CUDA and on.value == 0
+
+
+def test_dependents_start_behind_the_tensor_memory_allocation():
+    """A kernel that starts early may allocate an SM's tensor memory and then wait for the kernel ahead of it (launch.cuh): that one must
+    have allocated its own, in every thread's view, before it lets its dependents start."""
+    import glob
+    import os
+    import re
+
+    import mimir_framework_b200
+
+    csrc = os.path.join(os.path.dirname(mimir_framework_b200.__file__), "csrc")
+    checked = 0
+    for path in sorted(glob.glob(os.path.join(csrc, "*.cu"))):
+        for kernel in re.sub(r"//[^\n]*", "", open(path).read()).split("__global__")[1:]:
+            if "tmem_alloc" not in kernel or "pdl_launch_dependents()" not in kernel:
+                continue
+            alloc, trigger = kernel.index("tmem_alloc"), kernel.index("pdl_launch_dependents()")
+            assert "__syncthreads()" in kernel[alloc:trigger], os.path.basename(path)
+            checked += 1
+    assert checked >= 1
