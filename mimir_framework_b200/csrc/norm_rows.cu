@@ -150,7 +150,8 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
     row_reduce<false, WARP, 2>(c, 1, sh, rank, size);
     const float dm = c[0] / fn;
     sub += dm;
-    mul = 1.0f / sqrtf(fmaxf(c[1] - c[0] * dm, 0.0f) / fn + p.eps);
+    // (a second moment beyond fp32 makes the row zero, as the reference's does; c[0] * dm may then be infinite as well)
+    mul = 1.0f / sqrtf((c[1] < INFINITY ? fmaxf(c[1] - c[0] * dm, 0.0f) : c[1]) / fn + p.eps);
   } else if (FAM == ROWS_RMS) {
     float q = 0.0f;
 #pragma unroll

@@ -856,12 +856,12 @@ __global__ void __launch_bounds__(THREADS, (THREADS <= 512) ? 2 : 1) sweep_row_k
       const float fn = static_cast<float>(n);
       const float mean = shift + s1 / fn;
       float m2 = s2 - s1 * (s1 / fn);
-      if (s1 * (s1 / fn) > 0.75f * s2) {  // block-uniform
+      if (s1 * (s1 / fn) > 0.75f * s2 || m2 != m2) {  // block-uniform (the sums may have overflowed where the centred one does not)
         float qc = 0.0f;
         sweep_read(g, n, vec, [&](float v) { const float d = v - mean; qc = fmaf(d, d, qc); });
         m2 = block_sum(qc, red);
       }
-      const float inv = 1.0f / sqrtf(fmaxf(m2, 0.0f) / fn + p.eps);
+      const float inv = 1.0f / sqrtf((m2 < 0.0f ? 0.0f : m2) / fn + p.eps);
       if (p.stats_out != nullptr) {
         if (threadIdx.x == 0) {
           p.stats_out[2 * row] = mean;

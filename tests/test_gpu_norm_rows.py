@@ -51,6 +51,21 @@ def test_groupnorm(rt, batch, ch, h, w, groups, act):
     close(rt.groupnorm(x, g, b, batch, ch, h, w, groups, 1e-5, act), d / (1 + np.exp(-d)) if act >= 0 else d)
 
 
+@pytest.mark.parametrize("rows,n", [(3, 5), (7, 768), (5, 1027), (9, 4096), (3, 16381), (2, 40001), (160, 20004)])
+@pytest.mark.parametrize("scale", [1e15, 3e19, 3e28])
+def test_variances_at_and_beyond_the_largest_float(rt, rows, n, scale):
+    """The reference's variance overflows to infinity there and its rows become beta; so do rows in registers and swept rows."""
+    r = np.random.default_rng(n)
+    x = (r.standard_normal((rows, n)) * scale).astype(np.float32)
+    b = r.standard_normal(n).astype(np.float32)
+    got = np.asarray(rt.layernorm(x, np.ones(n, np.float32), b, rows, n)).reshape(rows, n)
+    if scale < 1e18:
+        d = x.astype(np.float64)
+        close(got, (d - d.mean(1, keepdims=True)) / d.std(1, keepdims=True) + b)
+    else:
+        assert np.abs(got - b).max() <= 1e-6 * np.abs(b).max()
+
+
 @pytest.mark.parametrize("hw", [(2, 2), (3, 1)])
 def test_silu_over_its_whole_range(rt, hw):
     """gamma = 0 and beta = v make every value of a channel silu(v): dense around zero, both ends of the exponential's range, the
