@@ -4,18 +4,16 @@
 //   RMSNorm   : LayerOpsExt::rms_norm_forward (LayerOpsExt.hpp:345-378) row = the whole sample
 //   Softmax   : LayerOps::softmax_forward    (LayerOps.hpp:325-361)  row = the whole sample
 //
-// Three shapes of kernel:
-//   * warp-per-row (LayerNorm rows <= 1024): the row lives in registers, shuffles only;
+// Rows that fit the registers of the threads that share them are norm_rows.cu's.  Here are the others:
 //   * CTA-per-row streaming sweeps (at least one row per SM): first sweep from HBM, later sweeps from
 //     L2, one HBM read and one HBM write per element;
+//   * the one-pass RMSNorm of long samples, whose sum of squares follows the reference's sequential fp32 chain;
 //   * "chunk" kernels when there are only a few (long) rows: pass 1 reduces 8192-element chunks to
 //     partial statistics in a small global scratch, pass 2 combines the partials of its row and
 //     writes the result; rows are processed in groups that fit in L2 so that pass 2 reads from L2.
-#include <type_traits>
-#include <cooperative_groups.h>
-
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "common.h"
