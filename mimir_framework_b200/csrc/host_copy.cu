@@ -87,7 +87,7 @@ struct HostCopier {
   uint8_t* ring = nullptr;
   cudaEvent_t ev[RING] = {};
   bool in_flight[RING] = {};
-  cudaStream_t on[RING] = {};  // the stream of a slot's copy in flight
+  std::thread::id by[RING] = {};  // whose copy is in flight in a slot
 
   // The ring, and as many helpers as the machine starts; false: no ring to be had (asked for once), copies go without
   bool init() {
@@ -182,7 +182,7 @@ struct HostCopier {
         e = cudaMemcpyAsync(j.dev + s * j.segment, ring + (s % RING) * SEGMENT, j.seg_bytes(s), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(ev[s % RING], st);
         in_flight[s % RING] = true;
-        on[s % RING] = st;
+        by[s % RING] = std::this_thread::get_id();
         if (s + RING < j.segments && e == cudaSuccess) free_slot(s + RING);
       }
       return e;
@@ -210,10 +210,11 @@ struct HostCopier {
     return e;
   }
 
-  // Does a copy of another stream, which may stand behind that stream's kernels, hold one of the first slots?
-  bool held_by_others(const Job& j, cudaStream_t st) {
+  // Does another thread's copy, which may stand behind its kernels, hold one of the first slots?  (A thread's own earlier copies are
+  // of the same call, or done: its copy in and its copy out are on different streams.)
+  bool held_by_others(const Job& j) {
     for (size_t s = 0; s < j.segments && s < RING; ++s)
-      if (in_flight[s] && on[s] != st) {
+      if (in_flight[s] && by[s] != std::this_thread::get_id()) {
         if (cudaEventQuery(ev[s]) != cudaSuccess) return true;
         in_flight[s] = false;
       }
@@ -231,7 +232,7 @@ struct HostCopier {
     j.segment = quarter < SEGMENT ? quarter : SEGMENT;
     j.segments = (j.bytes + j.segment - 1) / j.segment;
     j.pieces = (j.bytes + PIECE - 1) / PIECE;
-    if (held_by_others(j, st)) {
+    if (held_by_others(j)) {
       *taken = false;
       return MIMIR_B200_OK;
     }
@@ -315,9 +316,19 @@ int host_copy_selftest(int inject, const float* src, float* dst, size_t n, int* 
   void* dev = nullptr;
   int s = dev_alloc(&dev, n * sizeof(float), "host copy selftest");
   bool in = false, out = false;
-  if (s == MIMIR_B200_OK) s = copy(c, true, dev, const_cast<float*>(src), n * sizeof(float), nullptr, &in);
-  if (s == MIMIR_B200_OK) s = copy(c, false, dev, dst, n * sizeof(float), nullptr, &out);
-  if (s == MIMIR_B200_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) s = fail(MIMIR_B200_E_CUDA, "selftest: synchronisation failed");
+  cudaStream_t st[2] = {};  // in and out on streams of their own, as a model copies
+  cudaEvent_t done = nullptr;
+  if (s == MIMIR_B200_OK && (cudaStreamCreateWithFlags(&st[0], cudaStreamNonBlocking) != cudaSuccess || cudaStreamCreateWithFlags(&st[1], cudaStreamNonBlocking) != cudaSuccess ||
+                             cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess))
+    s = fail(MIMIR_B200_E_CUDA, "selftest: no streams");
+  if (s == MIMIR_B200_OK) s = copy(c, true, dev, const_cast<float*>(src), n * sizeof(float), st[0], &in);
+  if (s == MIMIR_B200_OK && (cudaEventRecord(done, st[0]) != cudaSuccess || cudaStreamWaitEvent(st[1], done, 0) != cudaSuccess)) s = fail(MIMIR_B200_E_CUDA, "selftest: ordering failed");
+  if (s == MIMIR_B200_OK) s = copy(c, false, dev, dst, n * sizeof(float), st[1], &out);
+  for (auto v : st) {
+    if (v && cudaStreamSynchronize(v) != cudaSuccess && s == MIMIR_B200_OK) s = fail(MIMIR_B200_E_CUDA, "selftest: synchronisation failed");
+    if (v) cudaStreamDestroy(v);
+  }
+  if (done) cudaEventDestroy(done);
   dev_free(dev, n * sizeof(float));
   delete c;
   if (ring_copies) *ring_copies = static_cast<int>(in) + static_cast<int>(out);

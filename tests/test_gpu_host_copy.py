@@ -139,7 +139,8 @@ def test_a_copy_does_not_wait_for_another_call_s_kernels(rt, waits_with):
 @pytest.mark.parametrize("n", [100, 16 << 10, 1 << 20, (9 << 20) + 3])
 @pytest.mark.parametrize("inject", [0, 1, 2, 3])
 def test_copies_without_page_locked_memory_or_threads(rt, inject, n):
-    """No room for the ring, or no more threads: the copy is done all the same, and nothing is thrown through the C interface."""
+    """No room for the ring, or no more threads: the copy is done all the same, and nothing is thrown through the C interface.  With the
+    ring both copies of a call take it, although the copy out finds slots in flight on the copy-in stream."""
     import ctypes
 
     src, dst, staged = np.random.default_rng(n).standard_normal(n).astype(np.float32), np.zeros(n, np.float32), ctypes.c_int(-1)
