@@ -1091,7 +1091,7 @@ double big_tile_cycles(const GemmArgs& g) {
   }
   const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
   const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
-  const double tile = (mma > load ? mma : load);
+  const double tile = 1.25 * (mma > load ? mma : load);  // (one tile to an SM starts cold: 1.15 to 1.3 times the estimate in 12 shapes)
   return 15100.0 + waves * (tile > 12000.0 ? tile : 12000.0);  // (a tile's epilogue takes about 12 000 cycles beside the next main loop)
 }
 }  // namespace
@@ -1130,7 +1130,10 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
     }
     const double spatial = c.conv_ks > 0 ? conv_gemm_cycles(c) : 1e30;
     if (spatial < 1e30 && spatial <= split && spatial <= big) return launch_conv_gemm(c, st);
-    if (split < big) return launch_gemm_split(g, sbk, bn, splits, st);
+    // (4096 rows and more may come in micro-batches, which should then give the bits of a single pass: from 64 big tiles on those give
+    // way only to a launch of half the cost - 4096 x 512 x 512 stays, at 0.55)
+    const bool whole = g.conv_ks == 0 && g.out_nchw_hw == 0 && g.m >= 4096 && big_tiles >= 64;
+    if (split < (whole ? 0.5 : 1.0) * big) return launch_gemm_split(g, sbk, bn, splits, st);
   }
   if (bk == 64 && (g.conv_ks == 0 || g.conv_c % 64 == 0)) return launch_gemm_t<64>(g, st);
   return launch_gemm_t<32>(g, st);

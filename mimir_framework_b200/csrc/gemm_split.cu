@@ -4,12 +4,17 @@
 //   Y[m, n] = act( sum_k A[m, k] * W[n, k] + bias[n] ) (+ residual[m, n])          (LayerOps.hpp:24-111)
 //
 // What bounds such a launch is not the tensor pipe but how many SMs take part and how long the chain of one tile is.  So:
-//   * the weights are the M side of the MMA (TMEM lane = output feature) and `bn` activation rows (16 ... 128) its N side: a tile
-//     of 40 rows costs a 48-column instruction, not a 256-column one, and each k-step still consumes 128 rows of weights;
+//   * the weights are the M side of the MMA (TMEM lane = output feature) and `bn` activation rows (16 ... 128) its N side, their two
+//     planes behind one another as ONE operand of 2 bn columns: an instruction of up to 92 columns costs the same 46 cycles, so
+//     hi and lo together cost little more than hi alone, and the sums of the small products get columns of their own;
 //   * K is cut into `splits` ranges that the CTAs of one thread-block cluster take; their partial tiles meet through distributed
 //     shared memory (CTA j sums column slice j of all partials, in split order: deterministic) and each CTA finishes its slice;
-//   * one tile per CTA, no persistent loop; the accumulators leave through shared memory, so that row-major results are stored
-//     with a lane per output feature and channel-major ones with a lane per pixel, both coalesced;
+//   * one tile per CTA, no persistent loop.  Row-major results leave from the registers that read tensor memory (a lane per output
+//     feature, swapped with its neighbour for 8-byte accesses), channel-major ones through shared memory with a lane per pixel;
+//   * sixteen warps finish a tile.  The tail was half of such a launch: eight warps took 0.5 to 1 us for each eight columns, a chain
+//     of dependent instructions (index divisions, a branch per element, a residual load waited for on the spot) at two warps
+//     to an issue slot.  333 x 1000 x 1000 by CTA stamps, from the input's arrival to the last store: 9.5 -> 5.9 us (accumulators
+//     4.4 -> 3.6, exchange 2.2 -> 1.5, stores 2.9 -> 0.8); 1000 x 2304 x 768 10.6 -> 8, 1000 x 768 x 768 with a residual 9.5 -> 4.7;
 //   * launched with programmatic stream serialization: barriers, tensor memory and the first stages of WEIGHTS are set up while
 //     the producing kernel still runs; only the activation loads and everything after wait for it.
 // The tile width and the split count come from a small cost model (plan_split) whose constants were fitted to measurements.
@@ -25,23 +30,26 @@
 namespace mb {
 namespace {
 
-constexpr int SG_THREADS = 256;
+constexpr int SG_THREADS = 512;
+constexpr int SG_GROUPS = SG_THREADS / 128;  // column groups of the epilogue: four warps, one per tensor-memory lane quadrant, to a group
 constexpr int SG_M = 128;            // weight rows of a tile
 constexpr int SG_MAX_BN = 128;
 constexpr int SG_MAX_STAGES = 8;
-constexpr int SG_RING_LIMIT = 212992;  // 208 KB of operand stages; the partial tiles reuse them
+constexpr int SG_RING_LIMIT = 212992;  // 208 KB: operand stages and, where three stages remain, the partial tiles behind them (else in their place)
 constexpr int SG_RING_TWO = 106496;    // 104 KB: two CTAs to an SM
 constexpr int SG_MAX_SPLITS = 16;      // (above eight: the non-portable cluster size)
 
-// Cost model (SM cycles): constants fitted to 20 shapes x 30 (width, split) pairs on B200, cold L2 (K = 256 ... 32768, 24 ... 5120 rows);
-// over those the chosen launch is within 1 % of the best one in the geometric mean.
-constexpr double SG_PER_BLOCK = 175.0;     // issue of a k-block beyond its MMAs
-constexpr double SG_FIXED = 10600.0;       // launch, barriers, first loads, drain
-constexpr double SG_TAIL_PER_COL = 70.0;   // accumulators -> shared memory -> output, per column of the tile
-constexpr double SG_SPLIT = 970.0, SG_SPLIT_PER_COL = 30.0;  // cluster barriers and the partial tiles through distributed shared memory
-constexpr double SG_LOAD_ALL = 51.6, SG_LOAD_MAX = 68.8;     // operand bytes per cycle an SM gets with all / few SMs loading
-
-constexpr float SHRINK_PER_MMA = 3.1e-8f;
+// Cost model (SM cycles): constants fitted to 25 shapes x 20 to 35 (width, split) pairs on B200, weights of 160 MB walked through
+// (K = 256 ... 32768, 17 ... 5120 rows); over those the chosen launch is within 1 % of the best one in the geometric mean, 9 % at worst.
+// A k-block costs what its operands take to arrive, or its MMAs where those are more; issuing them costs nothing beside that.
+constexpr double SG_FIXED = 5100.0;        // launch, barriers, first loads, drain
+constexpr double SG_TAIL_PER_COL = 36.0;   // accumulators -> output, per column that a CTA finishes
+constexpr double SG_SPLIT = 1550.0, SG_SPLIT_PER_COL = 60.0;  // cluster barriers and the partial tiles through distributed shared memory
+constexpr double SG_LOAD_ALL = 56.9, SG_LOAD_MAX = 62.9;      // operand bytes per cycle an SM gets with all / few SMs loading
+// Channel-major results (30 convolutions, 32 ... 512 channels on 7^2 ... 112^2 pixels: within 1 % of the best of every form and the spatial
+// tiles): taps find their operands in L2, scattered stores cost more.
+constexpr double SG_CM_BLOCK = 0.9, SG_CM_FIXED = 7700.0, SG_CM_TAIL_PER_COL = 181.0;
+constexpr double SG_TWO_TAIL = 1.27;       // a tail beside another CTA's main loop on the same SM
 
 struct SplitGemmParams {
   int m, n, kblocks;
@@ -56,8 +64,9 @@ struct SplitGemmParams {
   int ohw;
   int conv_ks, conv_cblocks, conv_pad, conv_hp, conv_wp, conv_h, conv_w;
   float acc_scale;
-  float shrink;  // what a partial sum would have lost per k-block that follows its range (see split_weight)
   int f16, stages, stage_bytes, w_ready;
+  float weight[SG_MAX_SPLITS];  // of the ranges' partial sums (split_weights)
+  int stg_off;  // the staging tile: behind the operand ring, or in its place (0)
   int* err_word;
 };
 
@@ -65,15 +74,45 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
-// Weight of split s's partial sum.  The tensor core adds with truncation, so in ONE accumulator over all of K the contribution of an
-// early range would have shrunk a little with every MMA that came after it.  The weights apply that shrinkage to the ranges that
-// were summed apart, and the result is then scaled as the unsplit kernel's is: a row gives the same answer in a small batch
-// (here) and in a large one (gemm_sm100.cu).  Relative difference of the two kernels' results, 40 x 1024 outputs, eight splits,
-// three MMAs per product: K = 32768 1.0e-4 unweighted, 1e-5 weighted (each is 5.3e-5 from the fp64 product); K = 2048 6.5e-6 and
-// 9e-7.  Fitted: 3e-8 ... 3.2e-8 per MMA at every K and product count.
-__device__ __forceinline__ float split_weight(const SplitGemmParams& p, int s) {
-  const int end = static_cast<int>(static_cast<long long>(p.kblocks) * (s + 1) / p.splits);
-  return 1.0f - p.shrink * static_cast<float>(p.kblocks - end);
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Accesses under a predicate and not behind a branch, so that those of a chunk interleave.
+__device__ __forceinline__ float2 ld_if(bool on, const float* p) {
+  float2 v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t@q ld.global.nc.v2.f32 {%0, %1}, [%3];\n\t}"
+               : "=&f"(v.x), "=&f"(v.y) : "r"(static_cast<int>(on)), "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st_if(bool on, float* p, float2 v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t@q st.global.v2.f32 [%1], {%2, %3};\n\t}" ::"r"(static_cast<int>(on)), "l"(p), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_if(bool on, __nv_bfloat16* p, uint32_t v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t@q st.global.b32 [%1], %2;\n\t}" ::"r"(static_cast<int>(on)), "l"(p), "r"(v) : "memory");
+}
+
+// N accumulator columns of this lane's output feature; with two activation planes the products of the lo plane (and of the weights'
+// lo plane) are in columns of their own, `bn` further on: far smaller sums, which the tensor core's truncating adds cannot cost
+// what they cost the main one.
+template <int N, int AP>
+__device__ __forceinline__ void load_acc(uint32_t taddr, int bn, float (&v)[N]) {
+  if (N == 16) {
+    tmem_ld_32x16(taddr, *reinterpret_cast<float (*)[16]>(v));
+    if (AP == 2) {
+      float w[16];
+      tmem_ld_32x16(taddr + bn, w);
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] += w[j];
+    }
+  } else {
+    tmem_ld_32x8(taddr, *reinterpret_cast<float (*)[8]>(v));
+    if (AP == 2) {
+      float w[8];
+      tmem_ld_32x8(taddr + bn, w);
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] += w[j];
+    }
+  }
 }
 
 template <int BK, int AP, int WP>  // AP, WP: operand planes of the activations and the weights
@@ -95,7 +134,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int to = tile % p.tiles_o, tr = tile / p.tiles_o;
   const int kb0 = static_cast<int>(static_cast<long long>(p.kblocks) * split / p.splits);
   const int kb1 = static_cast<int>(static_cast<long long>(p.kblocks) * (split + 1) / p.splits);
-  const uint32_t tmem_cols = p.bn <= 32 ? 32u : (p.bn <= 64 ? 64u : 128u);
+  const uint32_t tmem_cols = AP * p.bn <= 32 ? 32u : (AP * p.bn <= 64 ? 64u : (AP * p.bn <= 128 ? 128u : 256u));
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -114,6 +153,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  if (p.splits > 1 && p.stg_off > 0) cluster_arrive();  // (waited for ahead of the first store into another CTA)
   // (behind the allocation: a kernel that starts now may take all of an SM's tensor memory and then wait for this one)
   pdl_launch_dependents();
   const uint32_t tmem = tmem_slot;
@@ -143,6 +183,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     };
     // the weights of the first stages do not depend on the kernel before this one
     const int pre = min(p.stages, kb1 - kb0);
+    if (one) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     if (!p.w_ready) pdl_wait();
     for (int i = 0; i < pre; ++i) load_w(kb0 + i, i);
     pdl_wait();
@@ -158,7 +199,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     const bool one = elect_one();
-    const uint32_t idesc = make_idesc(SG_M, p.bn, p.f16);
+    const uint32_t idesc = make_idesc(SG_M, AP * p.bn, p.f16), idesc_lo = make_idesc(SG_M, p.bn, p.f16);
     int stage = 0;
     uint32_t phase = 0;
     bool ready = false;
@@ -167,16 +208,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       tcgen05_fence_after();
       const uint32_t sw = smem_u32(smem + stage * p.stage_bytes), sa = sw + WP * W_TILE;
       const uint64_t dw = make_smem_desc(sw, SWZ), da = make_smem_desc(sa, SWZ);
-      const uint64_t dw_lo = dw + (W_TILE >> 4), da_lo = da + (A_TILE >> 4);
+      const uint64_t dw_lo = dw + (W_TILE >> 4);
       uint64_t* done = &empty_bar[stage];
       if (++stage == p.stages) { stage = 0; phase ^= 1; }
       ready = mbar_test(&full_bar[stage], phase);
       if (one) {
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {  // 32 bytes further along K = 2 in the descriptor's address field
+          // (the lo plane of the activations lies behind the hi plane: one instruction covers both)
           umma_bf16(tmem, dw + 2 * k, da + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          if (AP == 2) umma_bf16(tmem, dw + 2 * k, da_lo + 2 * k, idesc, 1u);
-          if (WP == 2) umma_bf16(tmem, dw_lo + 2 * k, da + 2 * k, idesc, 1u);
+          if (WP == 2) umma_bf16(tmem + (AP == 2 ? p.bn : 0), dw_lo + 2 * k, da + 2 * k, idesc_lo, 1u);
         }
         umma_commit(done);
       }
@@ -189,23 +230,53 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // every thread below reads or writes memory that the previous kernels of the stream may still be using
   pdl_wait();
   const bool chan_major = conv || p.ohw > 0;
-  if (threadIdx.x < p.bn) {
-    const int row = tr * p.bn + static_cast<int>(threadIdx.x);
-    long long off = -1;
-    if (row < p.m) {
-      if (conv) {
-        const int per = p.conv_hp * p.conv_wp, smp = row / per, rem = row - smp * per, yq = rem / p.conv_wp;
-        const int yy = yq - p.conv_pad, xx = rem - yq * p.conv_wp - p.conv_pad;
-        if (yy >= 0 && yy < p.conv_h && xx >= 0 && xx < p.conv_w)
-          off = (static_cast<long long>(smp) * p.n * p.conv_h + yy) * p.conv_w + xx;
-      } else if (p.ohw > 0) {
-        const int smp = row / p.ohw;
-        off = static_cast<long long>(smp) * p.n * p.ohw + (row - smp * p.ohw);
-      } else {
-        off = row;
+  const int slice = p.bn / p.splits;           // columns this CTA finishes
+  const int oc0 = to * SG_M, row0 = tr * p.bn + split * slice;
+  const int quad = warp & 3, group = warp >> 2;
+  // Row-major results: a lane holds one output feature of eight columns (rows of Y) and swaps with its neighbour, so that it ends
+  // with two consecutive features of four columns, c0 + 2 i + (lane & 1): 8-byte accesses, two rows to a warp instruction.
+  const int odd = lane & 1, fe = oc0 + quad * 32 + (lane & ~1), first_row = row0 + odd;
+  const int ldo = static_cast<int>(p.ldo), live = min(slice, p.m - row0) - odd;  // (column c0 + 2 i is written where c0 + 2 i < live)
+  const bool vec = ((ldo & 1) == 0) && fe + 2 <= p.n && ((reinterpret_cast<uintptr_t>(p.out_f32) | reinterpret_cast<uintptr_t>(p.residual)) & 7) == 0;
+  const bool one_by_one = !vec && fe < p.n;
+  const bool has_res = p.residual != nullptr;
+  float2 b2 = make_float2(0.f, 0.f), res[4];
+  auto load_res = [&](int c0) {  // the residual of chunk c0: asked for one chunk ahead of its use
+    const float* src = p.residual + static_cast<long long>(first_row + c0) * ldo + fe;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) res[i] = ld_if(vec && c0 + 2 * i < live, src + static_cast<long long>(2 * i) * ldo);
+    if (one_by_one) {
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        if (c0 + 2 * i >= live) break;
+        const float x = __ldg(src + static_cast<long long>(2 * i) * ldo), y = fe + 1 < p.n ? __ldg(src + static_cast<long long>(2 * i) * ldo + 1) : 0.0f;
+        if (i == 0) res[0] = make_float2(x, y); else if (i == 1) res[1] = make_float2(x, y); else if (i == 2) res[2] = make_float2(x, y); else res[3] = make_float2(x, y);
       }
     }
-    col_off[threadIdx.x] = off;
+  };
+  if (chan_major) {
+    if (threadIdx.x < p.bn) {
+      const int row = tr * p.bn + static_cast<int>(threadIdx.x);
+      long long off = -1;
+      if (row < p.m) {
+        if (conv) {
+          const int per = p.conv_hp * p.conv_wp, smp = row / per, rem = row - smp * per, yq = rem / p.conv_wp;
+          const int yy = yq - p.conv_pad, xx = rem - yq * p.conv_wp - p.conv_pad;
+          if (yy >= 0 && yy < p.conv_h && xx >= 0 && xx < p.conv_w)
+            off = (static_cast<long long>(smp) * p.n * p.conv_h + yy) * p.conv_w + xx;
+        } else {
+          const int smp = row / p.ohw;
+          off = static_cast<long long>(smp) * p.n * p.ohw + (row - smp * p.ohw);
+        }
+      }
+      col_off[threadIdx.x] = off;
+    }
+  } else {
+    if (p.bias != nullptr) {
+      if (fe < p.n) b2.x = __ldg(p.bias + fe);
+      if (fe + 1 < p.n) b2.y = __ldg(p.bias + fe + 1);
+    }
+    if (has_res) load_res(group * 8);
   }
   {
     int ok = 1;
@@ -214,107 +285,196 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if (ok) while (!mbar_try_wait(&acc_bar, 0)) {}  // completes at once: lane 0 saw the phase
   }
   tcgen05_fence_after();
-  // The ring is free now (all MMAs have read it); with several CTAs to a tile, in every one of them.
-  if (p.splits > 1) cluster_sync_all(); else __syncthreads();
-
-  // accumulators -> staging tile of the CTA that finishes their columns: [split][column of the slice][pitch] floats
-  float* stg = reinterpret_cast<float*>(smem);
-  const int slice = p.bn / p.splits;
-  const int pitch = chan_major ? SG_M + 1 : SG_M;  // channel-major tiles are read with a lane per column
-  const int quad = warp & 3;
   const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-  for (int c0 = (warp >> 2) * 16; c0 < p.bn; c0 += 32) {
-    float v[16];
-    tmem_ld_32x16(taddr + c0, v);
-    if (p.splits == 1) {
+  float* stg = reinterpret_cast<float*>(smem + p.stg_off);
+  const int pitch = chan_major ? SG_M + 1 : SG_M;  // channel-major tiles are read with a lane per column
+  if (p.splits > 1 || chan_major) {
+    // accumulators -> staging tile of the CTA that finishes their columns: [split][column of the slice][pitch] floats.  Where
+    // it has the ring's place, every CTA of the cluster must have read its operands; else they need only have started.
+    if (p.splits > 1) {
+      if (p.stg_off == 0) cluster_sync_all(); else cluster_wait();
+    }
+    for (int c0 = group * 16; c0 < p.bn; c0 += 16 * SG_GROUPS) {
+      float v[16];
+      load_acc<16, AP>(taddr + c0, p.bn, v);
+      int owner = p.splits > 1 ? c0 / slice : 0, cl = c0 - owner * slice;
+      if (p.splits == 1) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) stg[(c0 + j) * pitch + quad * 32 + lane] = v[j];
-    } else {
+        for (int j = 0; j < 16; ++j) stg[(c0 + j) * pitch + quad * 32 + lane] = v[j];
+      } else {
+        const uint32_t mine = smem_u32(stg + split * slice * pitch + quad * 32 + lane);
+        uint32_t at = mapa_shared(mine, owner) + cl * pitch * 4;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int owner = (c0 + j) / slice, cl = c0 + j - owner * slice;
-        st_cluster_f32(mapa_shared(smem_u32(stg + (split * slice + cl) * pitch + quad * 32 + lane), owner), v[j]);
+        for (int j = 0; j < 16; ++j) {
+          st_cluster_f32(at, v[j]);
+          at += pitch * 4;
+          if (++cl == slice && j < 15) { cl = 0; at = mapa_shared(mine, ++owner); }
+        }
       }
     }
-  }
-  tcgen05_fence_before();
-  if (p.splits > 1) cluster_sync_all(); else __syncthreads();
-  if (warp == 1) {
-    tcgen05_fence_after();
-    tmem_dealloc(tmem, tmem_cols);
+    tcgen05_fence_before();
+    if (p.splits > 1) cluster_sync_all(); else __syncthreads();
   }
 
-  const int oc0 = to * SG_M, col_base = split * slice;
   if (!chan_major) {
-    // a warp takes a row, a lane four consecutive output features
-    const int oc = oc0 + lane * 4;
-    const bool vec = ((p.ldo & 3) == 0) && oc + 4 <= p.n &&
-                     ((reinterpret_cast<uintptr_t>(p.out_f32) | reinterpret_cast<uintptr_t>(p.residual)) & 15) == 0;
-    float b[4] = {0.f, 0.f, 0.f, 0.f};
-    if (p.bias != nullptr) {
+    for (int c0 = group * 8; c0 < slice; c0 += 8 * SG_GROUPS) {  // (warp-uniform)
+      float v[8];
+      if (p.splits == 1) {
+        load_acc<8, AP>(taddr + c0, p.bn, v);
+      } else {
+        const float* src = stg + c0 * pitch + quad * 32 + lane;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) if (oc + e < p.n) b[e] = __ldg(p.bias + oc + e);
-    }
-    for (int cl = warp; cl < slice; cl += SG_THREADS / 32) {
-      const long long row = col_off[col_base + cl];
-      if (row < 0) continue;  // warp-uniform
-      const float* src = stg + cl * pitch + lane * 4;
-      float4 a = *reinterpret_cast<const float4*>(src + (p.splits - 1) * slice * pitch);  // (the last range's weight is 1)
-      for (int s = p.splits - 2; s >= 0; --s) {
-        const float4 q = *reinterpret_cast<const float4*>(src + s * slice * pitch);
-        const float w = split_weight(p, s);
-        a.x = fmaf(q.x, w, a.x); a.y = fmaf(q.y, w, a.y); a.z = fmaf(q.z, w, a.z); a.w = fmaf(q.w, w, a.w);
-      }
-      float v[4] = {a.x, a.y, a.z, a.w};
+        for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+        for (int s = 0; s < p.splits; ++s) {  // in split order
+          const float w = p.weight[s];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = apply_act(__fmaf_rn(v[e], p.acc_scale, b[e]), p.activation);
-      const long long o = row * p.ldo + oc;
-      if (p.residual != nullptr) {
-        if (vec) {
-          const float4 r = __ldg(reinterpret_cast<const float4*>(p.residual + o));
-          v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) if (oc + e < p.n) v[e] += __ldg(p.residual + o + e);
+          for (int j = 0; j < 8; ++j) if (c0 + j < slice) v[j] = fmaf(src[j * pitch], w, v[j]);
+          src += slice * pitch;
         }
+      }
+      float2 u[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
+        u[i] = odd ? make_float2(other, v[2 * i + 1]) : make_float2(v[2 * i], other);
+        u[i].x = __fmaf_rn(u[i].x, p.acc_scale, b2.x);
+        u[i].y = __fmaf_rn(u[i].y, p.acc_scale, b2.y);
+      }
+      if (p.activation == MIMIR_B200_ELT_GELU) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { u[i].x = gelu_ref(u[i].x); u[i].y = gelu_ref(u[i].y); }
+      } else if (p.activation >= 0) {
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+          float2 t = i == 0 ? u[0] : i == 1 ? u[1] : i == 2 ? u[2] : u[3];
+          t.x = apply_act(t.x, p.activation); t.y = apply_act(t.y, p.activation);
+          if (i == 0) u[0] = t; else if (i == 1) u[1] = t; else if (i == 2) u[2] = t; else u[3] = t;
+        }
+      }
+      if (has_res) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { u[i].x += res[i].x; u[i].y += res[i].y; }
+        load_res(c0 + 8 * SG_GROUPS);
       }
       if (p.out_f32 != nullptr) {
-        if (vec) *reinterpret_cast<float4*>(p.out_f32 + o) = make_float4(v[0], v[1], v[2], v[3]);
-        else {
+        float* dst = p.out_f32 + static_cast<long long>(first_row + c0) * ldo + fe;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) if (oc + e < p.n) p.out_f32[o + e] = v[e];
+        for (int i = 0; i < 4; ++i) st_if(vec && c0 + 2 * i < live, dst + static_cast<long long>(2 * i) * ldo, u[i]);
+        if (one_by_one) {
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            if (c0 + 2 * i >= live) break;
+            const float2 t = i == 0 ? u[0] : i == 1 ? u[1] : i == 2 ? u[2] : u[3];
+            dst[static_cast<long long>(2 * i) * ldo] = t.x;
+            if (fe + 1 < p.n) dst[static_cast<long long>(2 * i) * ldo + 1] = t.y;
+          }
         }
       }
-      if (p.out_split != nullptr && oc < p.np) {
+      if (p.out_split != nullptr) {
         // columns n .. np - 1 are written as zero (the consumer's padded K)
-        uint32_t h[2], l[2];
+        const int np = static_cast<int>(p.np);
+        __nv_bfloat16* dst = p.out_split + static_cast<long long>(first_row + c0) * np + fe;
+        const long long plane = static_cast<long long>(p.m) * np;
+        uint32_t h[4], l[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = oc + e < p.n ? v[e] : 0.0f;
-        split_pair(v[0], v[1], p.f16, h[0], l[0]);
-        split_pair(v[2], v[3], p.f16, h[1], l[1]);
-        __nv_bfloat16* oh = p.out_split + row * p.np + oc;
-        *reinterpret_cast<uint2*>(oh) = make_uint2(h[0], h[1]);
-        *reinterpret_cast<uint2*>(oh + static_cast<long long>(p.m) * p.np) = make_uint2(l[0], l[1]);
+        for (int i = 0; i < 4; ++i) split_pair(fe < p.n ? u[i].x : 0.0f, fe + 1 < p.n ? u[i].y : 0.0f, p.f16, h[i], l[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          __nv_bfloat16* at = dst + static_cast<long long>(2 * i) * np;
+          const bool in = fe < np && c0 + 2 * i < live;
+          st_if(in, at, h[i]);
+          st_if(in, at + plane, l[i]);
+        }
       }
     }
   } else {
     // a lane takes a pixel; consecutive lanes run over the slice's pixels first
     const long long hw = conv ? static_cast<long long>(p.conv_h) * p.conv_w : static_cast<long long>(p.ohw);
-    const int nch = min(SG_M, p.n - oc0);
-    for (int i = threadIdx.x; i < slice * nch; i += SG_THREADS) {
-      const int ch = i / slice, cl = i - ch * slice;
-      const long long off = col_off[col_base + cl];
-      if (off < 0) continue;
-      const float* src = stg + cl * pitch + ch;
-      float a = src[(p.splits - 1) * slice * pitch];
-      for (int s = p.splits - 2; s >= 0; --s) a = fmaf(src[s * slice * pitch], split_weight(p, s), a);
-      a = __fmaf_rn(a, p.acc_scale, p.bias != nullptr ? __ldg(p.bias + oc0 + ch) : 0.0f);
-      a = apply_act(a, p.activation);
-      const long long o = off + static_cast<long long>(oc0 + ch) * hw;
-      if (p.residual != nullptr) a += __ldg(p.residual + o);
-      p.out_f32[o] = a;
+    const int nch = min(SG_M, p.n - oc0), total = slice * nch;
+    const int step_ch = SG_THREADS / slice, step_cl = SG_THREADS - step_ch * slice;
+    int ch = static_cast<int>(threadIdx.x) / slice, cl = static_cast<int>(threadIdx.x) - ch * slice;
+    for (int i = threadIdx.x; i < total; i += 4 * SG_THREADS) {
+      float a[4], r[4];
+      long long o[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = i + u * SG_THREADS < total;
+        const long long off = in ? col_off[split * slice + cl] : -1;
+        o[u] = off < 0 ? -1 : off + static_cast<long long>(oc0 + ch) * hw;
+        r[u] = has_res && o[u] >= 0 ? __ldg(p.residual + o[u]) : 0.0f;
+        a[u] = 0.0f;
+        if (in) {
+          const float* src = stg + cl * pitch + ch;
+          for (int s = 0; s < p.splits; ++s) a[u] = fmaf(src[s * slice * pitch], p.weight[s], a[u]);
+          a[u] = __fmaf_rn(a[u], p.acc_scale, p.bias != nullptr ? __ldg(p.bias + oc0 + ch) : 0.0f);
+        }
+        ch += step_ch;
+        cl += step_cl;
+        if (cl >= slice) { cl -= slice; ++ch; }
+      }
+      if (p.activation >= 0) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = apply_act(a[u], p.activation);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) if (o[u] >= 0) p.out_f32[o[u]] = has_res ? a[u] + r[u] : a[u];
     }
   }
+  tcgen05_fence_before();
+  __syncthreads();  // every warp has read the accumulators
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem, tmem_cols);
+  }
+}
+
+template <int BK, int AP, int WP>
+int prepare_split_kernel() {
+  static PerDeviceOnce attr_once;
+  return attr_once.run([&]() -> int {
+    MB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BK, AP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_RING_LIMIT + 1024));
+    MB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BK, AP, WP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return MIMIR_B200_OK;
+  });
+}
+
+// Stands for the kernel where the runtime is asked how many clusters fit: for kernels that allocate tensor memory it says one CTA per SM
+// whatever they take of it.
+__global__ void __launch_bounds__(SG_THREADS, 2) split_footprint_kernel() {}
+
+constexpr int SG_SPLITS[] = {1, 2, 3, 4, 6, 8, 16};
+
+// Clusters of SG_SPLITS[i] CTAs that run at the same time, one or two CTAs to an SM.  A cluster lives in one GPC, whose SM count is no
+// multiple of it: of the 148 SMs clusters of four use 132, of eight 120, of sixteen 112 (128 CTAs in clusters of eight: 12.9 us, two
+// rounds, where 64 in clusters of four take 8.0).
+int active_clusters(int i, bool two) {
+  struct Table { int n[2][sizeof(SG_SPLITS) / sizeof(int)]; };
+  static PerDeviceOnce once;
+  static Table table[64];  // (PerDeviceOnce counts as many devices)
+  Table& t = table[ctx().device];
+  const int rc = once.run([&]() -> int {
+    MB_CUDA(cudaFuncSetAttribute(split_footprint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_RING_LIMIT + 4096));
+    MB_CUDA(cudaFuncSetAttribute(split_footprint_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int j = 0; j < static_cast<int>(sizeof(SG_SPLITS) / sizeof(int)); ++j)
+      for (int w = 0; w < 2; ++w) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(SG_SPLITS[j] * 512));
+        cfg.blockDim = dim3(SG_THREADS);
+        cfg.dynamicSmemBytes = (w ? SG_RING_TWO : SG_RING_LIMIT) + 4096;  // (with the kernel's static part)
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(SG_SPLITS[j]);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        MB_CUDA(cudaOccupancyMaxActiveClusters(&n, split_footprint_kernel, &cfg));
+        t.n[w][j] = n;
+      }
+    return MIMIR_B200_OK;
+  });
+  return rc == MIMIR_B200_OK ? t.n[two ? 1 : 0][i] : 0;
 }
 
 // Tile width and split count of one launch and its estimated time in SM cycles.
@@ -322,33 +482,53 @@ struct SplitPlan { int bn = 0, splits = 0; double cycles = 1e30; };
 
 SplitPlan plan_split(const GemmArgs& g, int bk, int kblocks) {
   const int sms = ctx().sm_count;
-  const int products = 1 + (g.a_planes == 2) + (g.w_planes == 2);
   const int tiles_o = (g.n + SG_M - 1) / SG_M;
+  const bool cm = g.conv_ks > 0 || g.out_nchw_hw > 0;
+  auto mma = [](int n) { return n > 92 ? n * 0.5 : 46.0; };  // an instruction of 128 x n x 16
   SplitPlan best;
   static const int widths[] = {16, 32, 48, 64, 96, 128};
   for (int bn : widths) {
     if (bn > 16 && bn >= g.m + 32) break;
     const long long tiles = static_cast<long long>(tiles_o) * ((g.m + bn - 1) / bn);
     const int stage = (g.w_planes * SG_M + g.a_planes * bn) * bk * 2;
-    for (int splits = 1; splits <= SG_MAX_SPLITS; splits *= 2) {
-      // (clusters of sixteen: one GPC each, and not every GPC has sixteen SMs free - eight of them took 57 us where sixteen-SM
-      // work in clusters of eight took 46)
-      if (bn % splits != 0 || splits > kblocks || (splits > 8 && tiles > 4)) break;
+    for (int i = 0; i < static_cast<int>(sizeof(SG_SPLITS) / sizeof(int)); ++i) {
+      const int splits = SG_SPLITS[i];
+      if (splits > kblocks) break;
+      if (bn % splits != 0) continue;
       const long long ctas = tiles * splits;
       // CTAs that share an SM overlap one's loads and stores with the other's MMAs: whole rounds of two per SM
       const bool two = ctas > sms && 2 * stage <= SG_RING_TWO && bn * (SG_M + 1) * 4 <= SG_RING_TWO;
-      const long long rounds = two ? (ctas + 2 * sms - 1) / (2 * sms) : (ctas + sms - 1) / sms;
-      const int kb = (kblocks + splits - 1) / splits;
-      const double share = two ? static_cast<double>(ctas < 2 * sms ? (ctas + sms - 1) / sms : 2) : 1.0;
-      const double mma = share * kb * ((bk / 16) * products * (bn > 92 ? bn * 0.5 : 46.0) + SG_PER_BLOCK);
+      const int active = active_clusters(i, two);
+      if (active <= 0) continue;
+      const long long rounds = (tiles + active - 1) / active;
       const double busy = static_cast<double>(ctas < sms ? ctas : sms) / sms;
-      const double load = share * kb * stage / (SG_LOAD_MAX - (SG_LOAD_MAX - SG_LOAD_ALL) * busy);
-      const double tail = SG_FIXED + bn * SG_TAIL_PER_COL + (splits > 1 ? SG_SPLIT + bn * SG_SPLIT_PER_COL : 0.0);
-      const double t = static_cast<double>(rounds) * ((mma > load ? mma : load) + tail);
+      const double load = stage / (SG_LOAD_MAX - (SG_LOAD_MAX - SG_LOAD_ALL) * busy);
+      const double block = (bk / 16) * (mma(g.a_planes * bn) + (g.w_planes == 2 ? mma(bn) : 0.0));
+      const double main = (two ? 2.0 : 1.0) * ((kblocks + splits - 1) / splits) * (block > load ? block : load) * (cm ? SG_CM_BLOCK : 1.0);
+      const double tail = (cm ? SG_CM_FIXED : SG_FIXED) + bn * (cm ? SG_CM_TAIL_PER_COL : SG_TAIL_PER_COL) / splits + (splits > 1 ? SG_SPLIT + bn * SG_SPLIT_PER_COL : 0.0);
+      const double t = static_cast<double>(rounds) * (main + (two ? SG_TWO_TAIL : 1.0) * tail);
       if (t < best.cycles) { best.bn = bn; best.splits = splits; best.cycles = t; }
     }
   }
   return best;
+}
+
+// The tensor core adds with truncation, so in ONE accumulator over all of K (gemm_sm100.cu: `products` instructions per 16 of K) the
+// contribution of an early range shrinks a little with every instruction that comes after it, 3.1e-8 of its value (fitted: 3e-8 ... 3.2e-8
+// at every K and product count), and half as much for those of its own range.  The ranges summed apart here do not lose that, and in
+// one instruction per 16 of K less than they would have.  The weights put it back, and the result is then scaled as the unsplit
+// kernel's is: a row gives the same answer in a small batch and in a large one.  Relative difference of the two, 40 x 1024 outputs,
+// K = 32768, three MMAs per product: 1e-4 without the weights, 1e-5 with them.
+void split_weights(SplitGemmParams& p, long long ksteps, int steps_per_block, int products) {
+  auto at = [&](int s) {  // (zero-padded K adds exact zeros and loses nothing)
+    const long long step = static_cast<long long>(p.kblocks) * s / p.splits * steps_per_block;
+    return step < ksteps ? step : ksteps;
+  };
+  for (int s = 0; s < p.splits; ++s) {
+    const double after = p.splits > 1 ? 3.1e-8 * products * static_cast<double>(ksteps - at(s + 1)) : 0.0;
+    p.weight[s] = static_cast<float>(1.0 - after - 1.5e-8 * (products - 1) * static_cast<double>(at(s + 1) - at(s)));
+  }
+  if (p.splits == 1) p.acc_scale *= p.weight[0];
 }
 
 template <int BK, int AP, int WP>
@@ -368,7 +548,7 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
   p.conv_ks = g.conv_ks; p.conv_cblocks = conv ? g.conv_c / BK : 1; p.conv_pad = g.conv_pad;
   p.conv_hp = g.conv_h + 2 * g.conv_pad; p.conv_wp = g.conv_w + 2 * g.conv_pad; p.conv_h = g.conv_h; p.conv_w = g.conv_w;
   p.acc_scale = gemm_acc_scale(g);
-  p.shrink = SHRINK_PER_MMA * (BK / 16) * (AP + WP - 1);
+  split_weights(p, conv ? static_cast<long long>(p.kblocks) * (BK / 16) : (g.k + 15) / 16, BK / 16, AP + WP - 1);
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   p.w_ready = g.w_ready ? 1 : 0;
   p.err_word = ctx().dev_error_word;
@@ -379,14 +559,17 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
   p.stages = (two ? SG_RING_TWO : SG_RING_LIMIT) / p.stage_bytes;
   if (p.stages > SG_MAX_STAGES) p.stages = SG_MAX_STAGES;
   if (p.stages > per_split) p.stages = per_split;
-  const int staging = p.bn * (SG_M + 1) * 4, ring = p.stages * p.stage_bytes;
-  const int smem = (ring > staging ? ring : staging) + 1024;
-  static PerDeviceOnce attr_once;
-  MB_TRY(attr_once.run([&]() -> int {
-    MB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BK, AP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_RING_LIMIT + 1024));
-    MB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BK, AP, WP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    return MIMIR_B200_OK;
-  }));
+  // the staging tile gets a place of its own where that leaves three stages (or all there are)
+  const int staging = p.bn * (SG_M + 1) * 4, limit = two ? SG_RING_TWO : SG_RING_LIMIT;
+  const int fit = (limit - staging) / p.stage_bytes;
+  p.stg_off = 0;
+  if (p.splits > 1 && (fit >= p.stages || fit >= 3)) {
+    if (p.stages > fit) p.stages = fit;
+    p.stg_off = p.stages * p.stage_bytes;
+  }
+  const int ring = p.stages * p.stage_bytes;
+  const int smem = (p.stg_off > 0 ? ring + staging : ring > staging ? ring : staging) + 1024;
+  MB_TRY((prepare_split_kernel<BK, AP, WP>()));
   GemmProfile prof(st);
   MB_TRY(prof.begin());
   MB_TRY(launch_pdl(gemm_split_kernel<BK, AP, WP>, dim3(static_cast<unsigned>(ctas)), dim3(SG_THREADS), static_cast<size_t>(smem), st, p.splits, map_a, map_w, p));
@@ -410,8 +593,7 @@ double gemm_split_cycles(const GemmArgs& g, int bk, int* bn, int* splits) {
   }
   const SplitPlan plan = plan_split(g, bk, kblocks);
   *bn = plan.bn; *splits = plan.splits;
-  // (convolutions: shifted row blocks and channel-major stores, 1.3 to 1.4 times the estimate in 25 shapes)
-  return plan.cycles * (g.conv_ks > 0 || g.out_nchw_hw > 0 ? 1.35 : 1.0);
+  return plan.cycles;
 }
 
 int launch_gemm_split(const GemmArgs& g, int bk, int bn, int splits, cudaStream_t st) {

@@ -54,3 +54,30 @@ def test_convolution_against_the_port(rt, monkeypatch, form, batch, ic, oc, h, w
     got = rt.conv2d(x, wt, batch, ic, oc, h, w, k, stride, pad).reshape(batch, -1)
     want = np.stack([port.conv2d(x[i], wt, ic, oc, h, w, k, stride, pad, False).ravel() for i in range(batch)])
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("form", ["16,1", "48,3", "48,6", "96,6", "128,2", ""])
+@pytest.mark.parametrize("m,k,n", [(1, 40, 33), (50, 70, 131), (97, 200, 255), (130, 129, 64)])
+def test_chain_through_operand_planes(rt, monkeypatch, form, m, k, n):
+    """Linear -> GELU -> Linear: the first layer writes the second one's operand planes (zero up to a multiple of 64 columns), odd row
+    lengths go element by element, cluster sizes that are no power of two included."""
+    if form:
+        monkeypatch.setenv("MIMIR_B200_GEMM_SPLIT", form)
+    r = np.random.default_rng(m + n)
+    x = r.standard_normal((m, k)).astype(np.float32)
+    w = [(r.standard_normal((o, i)) / np.sqrt(i)).astype(np.float32) for i, o in ((k, n), (n, n))]
+    b = [r.standard_normal(n).astype(np.float32) for _ in range(2)]
+    descs = [make_desc("l", "Linear", inputs=["x"], output="h", in_features=k, out_features=n, seq_len=m, use_bias=1, params_count=n * k + n),
+             make_desc("g", "GELU", inputs=["h"], output="a"),
+             make_desc("m", "Linear", inputs=["a"], output="x", in_features=n, out_features=n, seq_len=m, use_bias=1, params_count=n * n + n)]
+    mod = rt.GraphModel(descs)
+    for layer, i in ((0, 0), (2, 1)):
+        mod.upload_weights(layer, np.concatenate([w[i].ravel(), b[i]]))
+    mod.plan({"x": (m * k, False)}, 1)
+    got = mod.forward({"x": (x.ravel(), False)}, 1, m * n).reshape(m, n)
+    mod.close()
+    h = x.astype(np.float64) @ w[0].astype(np.float64).T + b[0]
+    a = h * 0.5 * (1 + np.tanh(0.7978845608 * (h + 0.044715 * h ** 3)))
+    want = a @ w[1].astype(np.float64).T + b[1]
+    # two contractions of at most 255 products, a few 1e-6 each (operand planes and accumulation)
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
