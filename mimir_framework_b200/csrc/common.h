@@ -249,6 +249,9 @@ bool skinny_cluster_supported(int m, int k, int n);
 // bfloat16 copy of fp32 values; *inexact (device) becomes 1 when one of them is not a bfloat16
 int launch_pack_bf16(const float* src, uint16_t* dst, size_t n, int* inexact, cudaStream_t st);
 int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st);
+// skinny_mma.cu: the same for weights that are bfloat16 values (k a multiple of eight)
+bool skinny_mma_supported(int m, int k, int n);
+int launch_skinny_mma(const SkinnyClusterArgs& a, cudaStream_t st);
 
 // pointwise.cu ---------------------------------------------------------------------------------
 int launch_eltwise(int op, const float* a, const float* b, float* y, int batch, int64_t n, int64_t nb,

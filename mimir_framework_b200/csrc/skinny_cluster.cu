@@ -13,7 +13,7 @@
 //   * with many tiles (a vocabulary projection) one CTA per SM keeps its x in shared memory and walks its tiles;
 //   * a LayerNorm that feeds only this layer is applied while x is staged: every CTA takes the row statistics itself (16 rows of
 //     768 values are 48 KB from L2), which saves a launch of 4 us;
-//   * weights that are bfloat16 values are read from 16-bit copies (launch_pack_bf16): half the bytes, the same products;
+//   * (weights that are bfloat16 values take skinny_mma.cu, with 16-bit copies of them: launch_pack_bf16);
 //   * the step loop is rolled and small.  With weights held in registers and every step unrolled, instruction fetch was the top
 //     stall (no_instruction 1.7 per issue on the vocabulary projection, 38 us).
 #include "common.h"
@@ -29,26 +29,17 @@ constexpr int SC_ROWS = SC_WARPS * SC_WR;   // output features of a tile
 constexpr int SC_STEP = 128;                // k of a warp step: 32 lanes x 4
 
 struct SkinnyClusterParams {
-  const float* x; const void* w; const float* bias; const float* residual; float* y;
+  const float* x; const float* w; const float* bias; const float* residual; float* y;
   const float* gamma; const float* beta;  // LayerNorm (ln != 0), either may be null
   float eps;
   int ln, m, k, n, kc, act, w_ready;
 };
 
-// Four consecutive weights of a row: 16 bytes as fp32, 8 as bfloat16.
-template <int BF16>
-__device__ __forceinline__ void copy_quad(uint32_t dst, const void* w, long long i, bool valid) {
-  constexpr int B = BF16 ? 8 : 16;
-  const char* src = static_cast<const char*>(w) + (valid ? i * (B / 4) : 0);
-  const int n = valid ? B : 0;  // source size 0: zero-fill
-  if (BF16) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
-  else asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
-}
-template <int BF16>
-__device__ __forceinline__ float4 read_quad(const uint8_t* src) {
-  if (!BF16) return *reinterpret_cast<const float4*>(src);
-  const uint2 v = *reinterpret_cast<const uint2*>(src);
-  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+// Four consecutive weights of a row.
+__device__ __forceinline__ void copy_quad(uint32_t dst, const float* w, long long i, bool valid) {
+  const float* src = w + (valid ? i : 0);
+  const int n = valid ? 16 : 0;  // source size 0: zero-fill
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -196,12 +187,12 @@ __device__ __forceinline__ void lane_exchange(float (&acc)[N], int lane) {
 }
 
 // MT rows of x.  grid = tiles * cluster size, or (cluster size 1) any number of CTAs that walk the tiles.
-template <int MT, int BF16>
+template <int MT>
 __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const SkinnyClusterParams p) {
   constexpr int N = MT * SC_WR;
   constexpr int R = N % 32 == 0 ? 5 : 4, PER = N >> R;  // halving rounds of the exchange, values left
-  constexpr int QB = BF16 ? 8 : 16;                     // bytes of a lane's four weights
-  constexpr int STAGE = SC_WR * 32 * QB, STAGES = BF16 ? 8 : 6;
+  constexpr int QB = 16;                                // bytes of a lane's four weights
+  constexpr int STAGE = SC_WR * 32 * QB, STAGES = 6;
   extern __shared__ __align__(16) float sc_smem[];
   float* xs = sc_smem;                       // [MT][kc]
   float* gb = sc_smem + MT * p.kc;           // [2][kc]: the LayerNorm's gamma and beta
@@ -226,7 +217,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
       const uint32_t dst = ring_addr + f_slot * STAGE;
       const long long at = static_cast<long long>(f_o) * p.k + k0 + c;
 #pragma unroll
-      for (int j = 0; j < SC_WR; ++j) copy_quad<BF16>(dst + j * 32 * QB, p.w, at + static_cast<long long>(j) * p.k, c < klen && f_o + j < p.n);
+      for (int j = 0; j < SC_WR; ++j) copy_quad(dst + j * 32 * QB, p.w, at + static_cast<long long>(j) * p.k, c < klen && f_o + j < p.n);
       if (++f_ks == nsteps) { f_ks = 0; f_o += tile_step * SC_ROWS; }
       if (++f_slot == STAGES) f_slot = 0;
       --f_left;
@@ -250,7 +241,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) skinny_cluster_kernel(const Ski
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     float4 w[SC_WR];
 #pragma unroll
-    for (int j = 0; j < SC_WR; ++j) w[j] = read_quad<BF16>(ring + slot * STAGE + j * 32 * QB);
+    for (int j = 0; j < SC_WR; ++j) w[j] = *reinterpret_cast<const float4*>(ring + slot * STAGE + j * 32 * QB);
     fetch();  // (into the slot read one step ago)
     const float* xr = xs + ks * SC_STEP + lane * 4;
 #pragma unroll
@@ -313,11 +304,11 @@ struct ClusterShape { int splits = 0, kc = 0, ctas = 0; size_t smem = 0; };
 // (8 warps x steps x MT x 4 cycles; the FMAs are no more) plus a latency chain: few CTAs per SM (one where possible - the
 // previous kernel's CTAs still hold resources when this one's should start loading), little work in each, a cluster only where
 // K ranges are needed to occupy the SMs.  Chosen for 16 rows whatever m is: a sample gives the same bits in every batch size.
-ClusterShape cluster_shape(int k, int n, bool bf16) {
+ClusterShape cluster_shape(int k, int n) {
   constexpr int mt = 16;
   const int sms = ctx().sm_count, tiles = (n + SC_ROWS - 1) / SC_ROWS;
   const int all = (k + SC_STEP - 1) / SC_STEP;
-  const size_t ring = static_cast<size_t>(SC_WARPS) * (bf16 ? 8 * 8 : 6 * 16) * SC_WR * 32;
+  const size_t ring = static_cast<size_t>(SC_WARPS) * (6 * 16) * SC_WR * 32;
   ClusterShape best;
   long long best_cost = 0;
   for (int splits = 1; splits <= 8; ++splits) {
@@ -337,23 +328,23 @@ ClusterShape cluster_shape(int k, int n, bool bf16) {
 }
 
 template <int MT>
-int launch_mt(const SkinnyClusterParams& p, const ClusterShape& c, bool bf16, cudaStream_t st) {
+int launch_mt(const SkinnyClusterParams& p, const ClusterShape& c, cudaStream_t st) {
   static PerDeviceOnce attr_once;
   MB_TRY(attr_once.run([&]() -> int {
-    MB_CUDA(cudaFuncSetAttribute(skinny_cluster_kernel<MT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SC_SMEM_MAX)));
-    MB_CUDA(cudaFuncSetAttribute(skinny_cluster_kernel<MT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SC_SMEM_MAX)));
+    MB_CUDA(cudaFuncSetAttribute(skinny_cluster_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SC_SMEM_MAX)));
     return MIMIR_B200_OK;
   }));
-  return launch_pdl(bf16 ? skinny_cluster_kernel<MT, 1> : skinny_cluster_kernel<MT, 0>, dim3(static_cast<unsigned>(c.ctas)), dim3(SC_THREADS), c.smem, st, c.splits, p);
+  return launch_pdl(skinny_cluster_kernel<MT>, dim3(static_cast<unsigned>(c.ctas)), dim3(SC_THREADS), c.smem, st, c.splits, p);
 }
 
-// dst = the upper halves of src's bit patterns; *inexact becomes 1 when some lower half is not zero
+// dst = the upper halves of src's bit patterns; *inexact becomes 1 when some lower half is not zero or a value is not finite (cut
+// into planes, x would meet an infinite weight with zeros)
 __global__ void pack_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, size_t n, int* __restrict__ inexact) {
   bool bad = false;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const uint32_t u = __float_as_uint(__ldg(src + i));
     dst[i] = static_cast<uint16_t>(u >> 16);
-    bad = bad || (u & 0xffffu) != 0;
+    bad = bad || (u & 0xffffu) != 0 || (u & 0x7f800000u) == 0x7f800000u;
   }
   if (bad) *inexact = 1;
 }
@@ -361,8 +352,7 @@ __global__ void pack_bf16_kernel(const float* __restrict__ src, uint16_t* __rest
 }  // namespace
 
 bool skinny_cluster_supported(int m, int k, int n) {
-  // (a shape that fits with fp32 weights fits with bfloat16 ones too)
-  return m >= 1 && m <= 16 && k % 4 == 0 && k <= SC_MAX_K && cluster_shape(k, n, false).splits > 0;
+  return m >= 1 && m <= 16 && k % 4 == 0 && k <= SC_MAX_K && cluster_shape(k, n).splits > 0;
 }
 
 int launch_pack_bf16(const float* src, uint16_t* dst, size_t n, int* inexact, cudaStream_t st) {
@@ -375,19 +365,18 @@ int launch_pack_bf16(const float* src, uint16_t* dst, size_t n, int* inexact, cu
 }
 
 int launch_skinny_cluster(const SkinnyClusterArgs& a, cudaStream_t st) {
+  if (a.w_bf16 != nullptr) return launch_skinny_mma(a, st);
   if (!skinny_cluster_supported(a.m, a.k, a.n)) return fail(MIMIR_B200_E_INVALID, "skinny linear: not a shape of the cluster kernel");
-  const bool bf16 = a.w_bf16 != nullptr;
-  const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(bf16 ? static_cast<const void*>(a.w_bf16) : a.w) |
-                         reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta);
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta);
   if (bits & 15) return fail(MIMIR_B200_E_INVALID, "skinny linear: operands not 16-byte aligned");
-  const ClusterShape c = cluster_shape(a.k, a.n, bf16);
+  const ClusterShape c = cluster_shape(a.k, a.n);
   SkinnyClusterParams p;
-  p.x = a.x; p.w = bf16 ? static_cast<const void*>(a.w_bf16) : a.w; p.bias = a.bias; p.residual = a.residual; p.y = a.y;
+  p.x = a.x; p.w = a.w; p.bias = a.bias; p.residual = a.residual; p.y = a.y;
   p.gamma = a.gamma; p.beta = a.beta; p.eps = a.eps; p.ln = a.ln ? 1 : 0;
   p.m = a.m; p.k = a.k; p.n = a.n; p.kc = c.kc; p.act = a.activation; p.w_ready = a.w_ready ? 1 : 0;
-  if (a.m <= 4) MB_TRY(launch_mt<4>(p, c, bf16, st));
-  else if (a.m <= 8) MB_TRY(launch_mt<8>(p, c, bf16, st));
-  else MB_TRY(launch_mt<16>(p, c, bf16, st));
+  if (a.m <= 4) MB_TRY(launch_mt<4>(p, c, st));
+  else if (a.m <= 8) MB_TRY(launch_mt<8>(p, c, st));
+  else MB_TRY(launch_mt<16>(p, c, st));
   count_launch();
   return MIMIR_B200_OK;
 }

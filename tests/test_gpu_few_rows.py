@@ -96,3 +96,39 @@ def test_decode_steps_against_the_full_forward(rt, bf16, batch, heads, hd, prefi
             want = port.run_graph(descs, weights, {"x": ids[b, : t + 1]}).reshape(t + 1, V)[-1]
             assert np.linalg.norm(got[b] - want) <= 2e-5 * np.linalg.norm(want)
     m.close()
+
+
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 8), (3, 33, 128), (8, 17, 40), (9, 31, 1032), (16, 768, 3072), (16, 65, 4096), (5, 4737, 768), (16, 4752, 1024), (7, 100, 264)])
+def test_exact_bfloat16_weights_against_float64(rt, norm, m, n, k):
+    """A step of a token-wise layer whose weights are bfloat16 values (csrc/skinny_mma.cu): one tile and a walk over many, K below a unit, over
+    all warps and over a cluster; every warp's accumulators are exact products summed in fp32, as in the fp32 kernel above."""
+    r = np.random.default_rng(m * 31 + n)
+    x = (r.standard_normal((m, k)) + 1).astype(np.float32)
+    w = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)
+    w, b = (w.view(np.uint32) & 0xffff0000).view(np.float32), r.standard_normal(n).astype(np.float32)
+    g, be = (1 + 0.1 * r.standard_normal(k)).astype(np.float32), r.standard_normal(k).astype(np.float32)
+    lin = make_desc("l", "Linear", inputs=["h" if norm else "x"], output="y", in_features=k, out_features=n, seq_len=1, use_bias=1, params_count=n * k + n)
+    descs = ([make_desc("n", "LayerNorm", inputs=["x"], output="h", in_features=k, affine=1, use_bias=1, eps=1e-5, params_count=2 * k)] if norm else []) + [
+        lin, make_desc("s", "SiLU", inputs=["y"], output="x")]
+    mod = rt.GraphModel(descs, abi.PREC_BF16W)
+    for i, t in enumerate(([np.concatenate([g, be])] if norm else []) + [np.concatenate([w.ravel(), b]), None]):
+        mod.upload_weights(i, t)
+    mod.plan({"x": (k, False)}, m)
+    mod.decode_begin({"x": (k, False)}, m, 2)
+    h = x.astype(np.float64)
+    if norm:
+        h = (h - h.mean(1, keepdims=True)) / np.sqrt(h.var(1, keepdims=True) + 1e-5) * g + be
+    y = h @ w.astype(np.float64).T + b
+    want = y / (1 + np.exp(-y))
+    got = mod.decode_step({"x": (x, False)}, m, 0, n).reshape(m, n)
+    assert np.linalg.norm(got - want) <= 2e-6 * np.linalg.norm(want) + 1e-7
+    x[0, 0] = np.inf  # stays what it is: infinite where the weight is not zero, and the other rows keep their bits
+    again = mod.decode_step({"x": (x, False)}, m, 0, n).reshape(m, n)
+    mod.close()
+    assert np.array_equal(again[1:], got[1:])
+    if not norm:
+        with np.errstate(invalid="ignore", over="ignore"):
+            y = x[:1] @ w.T + b
+            want = y / (1 + np.exp(-y))
+        assert np.array_equal(np.isnan(again[0]), np.isnan(want[0])) and np.array_equal(np.isposinf(again[0]), np.isposinf(want[0]))
