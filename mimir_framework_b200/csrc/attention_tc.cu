@@ -548,6 +548,7 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  pdl_early_if_small();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_o = tmem_base + 3 * AT_BK;  // score / probability tile b lives at tmem_base + b * 64
 

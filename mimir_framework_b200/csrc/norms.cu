@@ -316,7 +316,6 @@ __global__ void rms_chunk_apply_kernel(const float* __restrict__ x, const float*
 // before it or belong to its own sample; the launcher only uses this kernel when a whole sample's
 // CTAs are resident at once.  Every wait is bounded: after ~2 s (or when another CTA gave up) the
 // CTA reports through the device error word and leaves without writing.
-constexpr int OP_VEC = CHUNK / (256 * 4);  // float4 per thread
 
 struct RmsOnePass {
   const float* x;
@@ -368,6 +367,7 @@ __device__ __forceinline__ bool slot_wait(const unsigned long long* slot, volati
   *out = __uint_as_float(static_cast<unsigned>(v & 0xffffffffull));
   return true;
 }
+template <int WARPS>
 __device__ __forceinline__ double block_sum_f64(double v, double* red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -377,18 +377,20 @@ __device__ __forceinline__ double block_sum_f64(double v, double* red) {
   __syncthreads();
   double t = 0.0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) t += red[k];
+  for (int k = 0; k < WARPS; ++k) t += red[k];
   return t;
 }
 
-__global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p) {
+template <int T>  // threads
+__global__ void __launch_bounds__(T, T == 256 ? 6 : 2) rms_onepass_kernel(const RmsOnePass p) {
   extern __shared__ __align__(128) float sx[];  // the chunk, zero beyond its end
   float* sg = sx + CHUNK;                       // stage_gamma: its chunk of gamma
   __shared__ __align__(8) uint64_t bar, gamma_bar;
   __shared__ unsigned s_id;
   __shared__ int s_abort, s_last;
   __shared__ float redf[33];
-  __shared__ double red[8];
+  __shared__ double red[T / 32];
+  constexpr int VEC = CHUNK / (T * 4), STEP = VEC < 4 ? VEC : 4;  // float4 of a thread, side by side in the last loop
   const int tid = threadIdx.x;
   if (tid == 0) {
     s_abort = 0;
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
     if (p.gamma != nullptr && o + tid * 32 < p.n_gamma) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gamma + o + tid * 32));
   };
   if (p.rows == 1) prefetch_gamma(static_cast<long long>(blockIdx.x) * CHUNK);
+  pdl_early_if_small();
   pdl_wait();
   // Counters and slots hold nothing of use after a wait gave up, until the host clears them: the launches in between write nothing and
   // report it again (the host may have read the word already).  (One row needs no order among its CTAs, which are resident
@@ -444,10 +447,10 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
       mbar_expect_tx(&bar, static_cast<uint32_t>(n) * 4u);
       for (int b0 = 0; b0 < n; b0 += 2048) bulk_load_1d(sx + b0, g + b0, static_cast<uint32_t>(min(2048, n - b0)) * 4u, &bar);
     }
-    for (int i = n + tid; i < CHUNK; i += 256) sx[i] = 0.0f;
+    for (int i = n + tid; i < CHUNK; i += T) sx[i] = 0.0f;
     if (!mbar_wait(&bar, 0, &s_abort, p.err_word, 20)) ok = false;
   } else {
-    for (int i = tid; i < CHUNK; i += 256) sx[i] = (i < n) ? __ldg(g + i) : 0.0f;
+    for (int i = tid; i < CHUNK; i += T) sx[i] = (i < n) ? __ldg(g + i) : 0.0f;
   }
   __syncthreads();
   if (staged && tid == 0) {
@@ -459,8 +462,8 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   // ---- the chunk's sum of squares ----
   float acc = 0.0f;
 #pragma unroll 2
-  for (int i = 0; i < OP_VEC; ++i) {
-    const float4 v = s4[i * 256 + tid];
+  for (int i = 0; i < VEC; ++i) {
+    const float4 v = s4[i * T + tid];
     acc += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
   }
   const float run = block_sum(acc, redf);
@@ -469,7 +472,7 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
 
   // ---- sum of the chunks before this one (only its binade matters) ----
   float before = 0.0f;
-  for (int j = tid; j < c; j += 256) {
+  for (int j = tid; j < c; j += T) {
     float t = 0.0f;
     ok = ok && slot_wait(p.sum_slots + slot0 + j, abort_flag, p.err_word, 21, &t);
     before += t;
@@ -480,11 +483,11 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   //      rounding error of every step with error-free transformations (see rms_seq_err_kernel) ----
   float err = 0.0f;
 #pragma unroll 2
-  for (int i = 0; i < OP_VEC; ++i) {
+  for (int i = 0; i < VEC; ++i) {
     // Where the chain stood before this float4: only the binade of that value enters the rounding of a step,
     // so inside the chunk (1 % of a long sample) the running sum is taken as growing evenly.
-    float sf = prefix + run * (static_cast<float>((i * 256 + tid) * 4) * (1.0f / CHUNK));
-    const float4 v = s4[i * 256 + tid];
+    float sf = prefix + run * (static_cast<float>((i * T + tid) * 4) * (1.0f / CHUNK));
+    const float4 v = s4[i * T + tid];
     const float e4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {  // the zero tail adds nothing and rounds nothing
@@ -505,13 +508,13 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
 
   // ---- the sample's total: every chunk's sum and chain error ----
   double mine = 0.0;
-  for (int j = tid; j < p.chunks; j += 256) {
+  for (int j = tid; j < p.chunks; j += T) {
     float e = 0.0f, s = 0.0f;
     ok = ok && slot_wait(p.err_slots + slot0 + j, abort_flag, p.err_word, 22, &e);
     ok = ok && slot_wait(p.sum_slots + slot0 + j, abort_flag, p.err_word, 23, &s);
     mine += static_cast<double>(s) + static_cast<double>(e);
   }
-  const double sd = block_sum_f64(mine, red);
+  const double sd = block_sum_f64<T / 32>(mine, red);
   if (staged && !mbar_wait(&gamma_bar, 0, &s_abort, p.err_word, 24)) ok = false;  // (asked for before the sums were; nobody leaves before it lands)
   if (__syncthreads_or(!ok || gave_up)) {  // a wait gave up: nothing is written
     if (tid == 0) {
@@ -540,22 +543,22 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   // A whole chunk into two planes: four float4 per thread side by side, no branch between them (the general loop's iterations follow
   // one another, 550 cycles each with eight warps on the SM: 2.5 us of a one-prompt norm)
   auto planes_fast = [&](auto half) {
-    for (int i0 = 0; i0 < OP_VEC; i0 += 4) {
-      float o[4][4];
+    for (int i0 = 0; i0 < VEC; i0 += STEP) {
+      float o[STEP][4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int e0 = ((i0 + k) * 256 + tid) * 4;
-        const float4 v = s4[(i0 + k) * 256 + tid], gm = staged ? *reinterpret_cast<const float4*>(sg + e0) : __ldg(reinterpret_cast<const float4*>(p.gamma + off + e0));
+      for (int k = 0; k < STEP; ++k) {
+        const int e0 = ((i0 + k) * T + tid) * 4;
+        const float4 v = s4[(i0 + k) * T + tid], gm = staged ? *reinterpret_cast<const float4*>(sg + e0) : __ldg(reinterpret_cast<const float4*>(p.gamma + off + e0));
         o[k][0] = v.x; o[k][1] = v.y; o[k][2] = v.z; o[k][3] = v.w;
         quotients(o[k]);
         o[k][0] *= gm.x; o[k][1] *= gm.y; o[k][2] *= gm.z; o[k][3] *= gm.w;
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < STEP; ++k) {
         uint32_t h01, h23, l01, l23;
         split_pair(o[k][0], o[k][1], decltype(half)::value, h01, l01);
         split_pair(o[k][2], o[k][3], decltype(half)::value, h23, l23);
-        __nv_bfloat16* y = p.y_split + base + ((i0 + k) * 256 + tid) * 4;
+        __nv_bfloat16* y = p.y_split + base + ((i0 + k) * T + tid) * 4;
         *reinterpret_cast<uint2*>(y) = make_uint2(h01, h23);
         *reinterpret_cast<uint2*>(y + p.plane_stride) = make_uint2(l01, l23);
       }
@@ -565,10 +568,10 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
     if (p.f16) planes_fast(std::true_type{}); else planes_fast(std::false_type{});
   } else {
 #pragma unroll 1
-    for (int i = 0; i < OP_VEC; ++i) {
-      const int e0 = (i * 256 + tid) * 4;
+    for (int i = 0; i < VEC; ++i) {
+      const int e0 = (i * T + tid) * 4;
       if (e0 >= n) break;
-      const float4 v = s4[i * 256 + tid];
+      const float4 v = s4[i * T + tid];
       float o[4] = {v.x, v.y, v.z, v.w};
       quotients(o);
       if (vec_gamma) {
@@ -609,7 +612,7 @@ __global__ void __launch_bounds__(256, 6) rms_onepass_kernel(const RmsOnePass p)
   if (tid == 0) s_last = atomicAdd(p.row_done + row, 1u) == static_cast<unsigned>(p.chunks) - 1u;
   __syncthreads();
   if (s_last) {
-    for (int j = tid; j < p.chunks; j += 256) {
+    for (int j = tid; j < p.chunks; j += T) {
       p.sum_slots[slot0 + j] = 0ull;
       p.err_slots[slot0 + j] = 0ull;
     }
@@ -1201,8 +1204,8 @@ bool rmsnorm_onepass_ok(int batch, int64_t n) {
     int& slot = per_sm_dev[ctx().device];
     if (slot == 0) {
       int v = 0;
-      cudaFuncSetAttribute(rms_onepass_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, rms_onepass_kernel, 256, CHUNK * sizeof(float)) != cudaSuccess) v = 0;
+      cudaFuncSetAttribute(rms_onepass_kernel<256>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, rms_onepass_kernel<256>, 256, CHUNK * sizeof(float)) != cudaSuccess) v = 0;
       slot = v > 0 ? v : -1;
     }
     per_sm = slot > 0 ? slot : 0;
@@ -1237,10 +1240,15 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
     p.stage_gamma = slots <= static_cast<size_t>(3) * ctx().sm_count ? 1 : 0;
     static PerDeviceOnce attr_once;
     MB_TRY(attr_once.run([&]() -> int {
-      MB_CUDA(cudaFuncSetAttribute(rms_onepass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CHUNK * sizeof(float)));
+      MB_CUDA(cudaFuncSetAttribute(rms_onepass_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CHUNK * sizeof(float)));
+      MB_CUDA(cudaFuncSetAttribute(rms_onepass_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CHUNK * sizeof(float)));
       return MIMIR_B200_OK;
     }));
-    MB_TRY(launch_pdl(rms_onepass_kernel, dim3(static_cast<unsigned>(slots)), dim3(256), CHUNK * sizeof(float) * (p.stage_gamma ? 2 : 1), st, 1, p));
+    // With a chunk to an SM at most, twice the threads halve the stretches between the exchanges (one prompt of 1000 tokens, 25 norms:
+    // 1041 -> 1033 us).
+    const size_t smem = CHUNK * sizeof(float) * (p.stage_gamma ? 2 : 1);
+    if (slots <= static_cast<size_t>(ctx().sm_count)) MB_TRY(launch_pdl(rms_onepass_kernel<512>, dim3(static_cast<unsigned>(slots)), dim3(512), smem, st, 1, p));
+    else MB_TRY(launch_pdl(rms_onepass_kernel<256>, dim3(static_cast<unsigned>(slots)), dim3(256), smem, st, 1, p));
     count_launch();
     return MIMIR_B200_OK;
   }
