@@ -25,6 +25,7 @@
 #include "launch.cuh"
 #include "tensor_map.h"
 
+#include <climits>
 #include <cmath>
 #include <cstring>
 
@@ -73,6 +74,8 @@ struct GemmParams {
   // weight plane at BK = 32), so the same shared memory gives six stages instead of four - the K = 768 layers were
   // starved of operands with four (the MMA thread spent a quarter of every tile waiting on a full barrier).
   int stages, stage_bytes;
+  // Tiles from this one on run as two of 128 columns each: the last wave's, where it would leave half of the CTAs idle.
+  int full_tiles;
   int* err_word;
   // grouped form: W rows of tile (tm, tn) start at (tm * BM / a_group_rows) * w_group_rows + tn * bn (0 = one group)
   int a_group_rows, w_group_rows;
@@ -93,6 +96,17 @@ __device__ __forceinline__ void tile_coords(int t, const GemmParams& p, int& tm,
   const int gw = min(p.group_n, p.tiles_n - gn0);
   tn = gn0 + r % gw;
   tm = r / gw;
+}
+
+// The tile of work item t and, of a tile that is cut in two, which half of its columns (else -1).
+__device__ __forceinline__ int work_coords(int t, const GemmParams& p, int& tm, int& tn) {
+  int half = -1;
+  if (t >= p.full_tiles) {
+    half = (t - p.full_tiles) & 1;
+    t = p.full_tiles + ((t - p.full_tiles) >> 1);
+  }
+  tile_coords(t, p, tm, tn);
+  return half;
 }
 
 template <int BK>
@@ -164,7 +178,7 @@ __device__ __forceinline__ void mma_role(const GemmParams& p, uint8_t* smem, uin
                                          int num_tiles) {
   constexpr int SWZ = BK * 2, A_TILE = BM * BK * 2, W_TILE = (PAIR ? BN / 2 : BN) * BK * 2;
   const bool one = elect_one();
-  const uint32_t idesc = make_idesc(PAIR ? 2 * BM : BM, p.bn, p.f16);
+  const uint32_t idesc_full = make_idesc(PAIR ? 2 * BM : BM, p.bn, p.f16), idesc_half = make_idesc(PAIR ? 2 * BM : BM, BN / 2, p.f16);
   const int stages = p.stages, stage_bytes = p.stage_bytes, kblocks = p.kblocks;
   int stage = 0, acc = 0;
   uint32_t phase = 0, acc_phase = 0;
@@ -173,6 +187,7 @@ __device__ __forceinline__ void mma_role(const GemmParams& p, uint8_t* smem, uin
     if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.err_word, 3)) return;
     tcgen05_fence_after();
     const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+    const uint32_t idesc = t >= p.full_tiles ? idesc_half : idesc_full;
     for (int kb = 0; kb < kblocks; ++kb) {
       if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.err_word, 4)) return;
       tcgen05_fence_after();
@@ -252,7 +267,8 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  const int num_tiles = p.tiles_m * p.tiles_n;
+  const int all_tiles = p.tiles_m * p.tiles_n;
+  const int num_tiles = CM == 0 && p.full_tiles < all_tiles ? 2 * all_tiles - p.full_tiles : all_tiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -297,10 +313,14 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint32_t phase = 0;
     bool ok = true;
     for (int t = t_first; t < num_tiles && ok; t += t_step) {
-      int tm, tn;
-      tile_coords(t, p, tm, tn);
+      int tm, tn, cut = -1;
+      if (CM == 0) cut = work_coords(t, p, tm, tn); else tile_coords(t, p, tm, tn);
       if (PAIR) tm = tm * 2 + static_cast<int>(crank);  // p.tiles_m counts row PAIRS
+      // (of a tile that is cut in two: 128 columns, 64 of them in each CTA of a pair)
+      const CUtensorMap* const wmap = cut >= 0 ? &map_o : &map_w;
+      const uint32_t tx = cut >= 0 ? static_cast<uint32_t>((PAIR ? 2 : 1) * (m_planes * A_TILE + n_planes * (W_TILE / 2))) : tx_bytes;
       const int w_row = swapped ? tm * BM
+                        : cut >= 0 ? tn * BN + cut * (BN / 2) + (PAIR ? static_cast<int>(crank) * (BN / 4) : 0)
                         : PAIR ? tn * BN + static_cast<int>(crank) * (BN / 2)
                                : tn * p.bn + (p.a_group_rows > 0 ? (tm * BM / p.a_group_rows) * p.w_group_rows : 0);
       const int a_row0 = swapped ? tn * BN : tm * BM;  // swapped: 256 activation rows (tile tn) are the N side
@@ -319,20 +339,20 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           if (PAIR) {
             // the leader arms its barrier for the bytes of both CTAs; this CTA's bytes are counted there whichever
             // of the two arrives first (the phase cannot complete before the leader's arrive)
-            if (crank == 0) mbar_expect_tx(&full_bar[stage], tx_bytes);
+            if (crank == 0) mbar_expect_tx(&full_bar[stage], tx);
             const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
             tma_load_3d_pair(m_base, &map_a, fb, a_col, a_row, 0);
             if (m_planes == 2) tma_load_3d_pair(m_base + A_TILE, &map_a, fb, a_col, a_row, 1);
-            tma_load_3d_pair(n_base, &map_w, fb, kb * BK, w_row, 0);
-            if (n_planes == 2) tma_load_3d_pair(n_base + W_TILE, &map_w, fb, kb * BK, w_row, 1);
+            tma_load_3d_pair(n_base, wmap, fb, kb * BK, w_row, 0);
+            if (n_planes == 2) tma_load_3d_pair(n_base + W_TILE, wmap, fb, kb * BK, w_row, 1);
           } else {
-            mbar_expect_tx(&full_bar[stage], tx_bytes);
+            mbar_expect_tx(&full_bar[stage], tx);
             uint8_t* ab = swapped ? n_base : m_base;
             uint8_t* wb = swapped ? m_base : n_base;
             tma_load_3d(ab, &map_a, &full_bar[stage], a_col, a_row, 0);
             if (p.a_planes == 2) tma_load_3d(ab + (swapped ? W_TILE : A_TILE), &map_a, &full_bar[stage], a_col, a_row, 1);
-            tma_load_3d(wb, &map_w, &full_bar[stage], kb * BK, w_row, 0);
-            if (p.w_planes == 2) tma_load_3d(wb + (swapped ? A_TILE : W_TILE), &map_w, &full_bar[stage], kb * BK, w_row, 1);
+            tma_load_3d(wb, wmap, &full_bar[stage], kb * BK, w_row, 0);
+            if (p.w_planes == 2) tma_load_3d(wb + (swapped ? A_TILE : W_TILE), wmap, &full_bar[stage], kb * BK, w_row, 1);
           }
         }
         __syncwarp();
@@ -365,8 +385,8 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = t_first; t < num_tiles; t += t_step) {
-      int tm, tn;
-      tile_coords(t, p, tm, tn);
+      int tm, tn, cut = -1;
+      if (CM == 0) cut = work_coords(t, p, tm, tn); else tile_coords(t, p, tm, tn);
       if (PAIR) tm = tm * 2 + static_cast<int>(crank);
       // lane 0 does the bounded wait; the verdict is made warp-uniform because tcgen05.ld below
       // is a warp-collective instruction
@@ -615,11 +635,11 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // (Tried: the next chunk's tensor-memory load in flight while this one is processed - two register sets, the
       // plain form has the room.  Measured neutral to 7 % slower on the K = 768 layers: the load's latency is not what
       // the short-K tiles wait for; operand and store bytes per MMA cycle are.)
-      const int nch = (p.bn / 32) / 2;
+      const int bn = cut >= 0 ? BN / 2 : p.bn, nch = (bn / 32) / 2;
 #pragma unroll 1
       for (int ci = 0; ci < nch; ++ci) {
-        const int c0 = (half * (p.bn / 64) + ci) * 32;
-        const int col0 = tn * p.bn + c0;
+        const int c0 = (half * (bn / 64) + ci) * 32;
+        const int col0 = tn * p.bn + (cut > 0 ? BN / 2 : 0) + c0;
         if (col0 >= col_limit) break;  // warp-uniform
         float v[32];
         tmem_ld_32x32(taddr0 + c0, v);
@@ -929,6 +949,16 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
     const int pairs = ctx().sm_count / 2;
     grid = 2 * (tiles < pairs ? tiles : pairs);
   }
+  // The last wave's tiles as halves where it has at most half as many tiles as there are CTAs (pairs): the same sums in the same order, bit
+  // for bit.  A half takes 0.53 of a tile with three MMAs per product, 0.67 with two (the activations are loaded whole).
+  p.full_tiles = INT_MAX;
+  const int workers = pair ? ctx().sm_count / 2 : ctx().sm_count, rest = tiles % workers;
+  static const bool halves = env_int("MIMIR_B200_GEMM_HALVES", 1) != 0;
+  if (halves && !cm && !tma_store && p.bn == BN && g.a_group_rows <= 0 && g.a_planes + g.w_planes >= 3 && rest > 0 && 2 * rest <= workers) {
+    p.full_tiles = tiles - rest;
+    MB_TRY(make_plane_map(&map_o, g.w, g.w_planes, g.n, kp, BK, pair ? BN / 4 : BN / 2));
+    if (tiles < workers) grid = (pair ? 2 : 1) * 2 * rest;
+  }
   GemmProfile prof(st);
   MB_TRY(prof.begin());
   if (pair) {
@@ -1091,7 +1121,8 @@ double big_tile_cycles(const GemmArgs& g) {
   }
   const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
   const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
-  const double tile = 1.25 * (mma > load ? mma : load);  // (one tile to an SM starts cold: 1.15 to 1.3 times the estimate in 12 shapes)
+  // (one tile to an SM starts cold: 1.15 to 1.3 times the estimate in 12 shapes; two waves, 1440 x 3784 x 3784, are as estimated)
+  const double tile = (waves == 1 ? 1.25 : 1.0) * (mma > load ? mma : load);
   return 15100.0 + waves * (tile > 12000.0 ? tile : 12000.0);  // (a tile's epilogue takes about 12 000 cycles beside the next main loop)
 }
 }  // namespace

@@ -62,3 +62,33 @@ def test_forced_cta_pairs_on_ragged_shapes():
     out = subprocess.run([sys.executable, "-c", "ROOT = %r\n" % ROOT + CHILD], env=env, capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stdout[-2000:] + out.stderr[-4000:]
     assert "PAIR_CASES_OK 13" in out.stdout, out.stdout[-2000:]
+
+
+@pytest.mark.parametrize("precision", ["x2", "w"])
+@pytest.mark.parametrize("whole,cut,n,k", [(9472, 9600, 1024, 256), (12800, 8192, 256, 616), (9472, 9500, 1000, 1032)])
+def test_tiles_cut_in_two_keep_their_bits(precision, whole, cut, n, k):
+    """The last wave's tiles run as two of 128 columns where it would leave half of the CTAs idle (`cut` rows: 4 of 74 pair tiles, and 64 of
+    148 single ones) and whole elsewhere (`whole` rows): the rows the two launches share have the same bits."""
+    import numpy as np
+    from mimir_framework_b200 import abi, configs, runtime as rt
+
+    rt.init(0)
+    r = np.random.default_rng(n)
+    w = (r.standard_normal(n * k + n) * 0.05).astype(np.float32)
+    if precision == "w":
+        w = configs.round_to_bf16(w)
+    x = r.standard_normal((max(whole, cut), k)).astype(np.float32)
+    got = []
+    for rows in (whole, cut):
+        m = rt.GraphModel([abi.make_desc("l", "Linear", in_features=k, out_features=n, seq_len=rows, use_bias=1, params_count=w.size),
+                           abi.make_desc("g", "GELU", inputs=["x"], output="x")], abi.PREC_BF16X2 if precision == "x2" else abi.PREC_BF16W)
+        m.upload_weights(0, w)
+        m.plan({"x": (rows * k, False)}, 1)
+        got.append(m.forward({"x": (x[:rows].ravel(), False)}, 1, rows * n).reshape(rows, n))
+        m.close()
+    both = min(whole, cut)
+    assert np.array_equal(got[0][:both], got[1][:both])
+    want = x[-40:].astype(np.float64) @ w[: n * k].reshape(n, k).T.astype(np.float64) + w[n * k:]
+    want = want * 0.5 * (1 + np.tanh(0.7978845608 * (want + 0.044715 * want ** 3)))
+    big = got[0] if whole > cut else got[1]
+    assert np.linalg.norm(big[-40:] - want) <= 1e-5 * np.linalg.norm(want)
