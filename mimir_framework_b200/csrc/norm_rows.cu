@@ -4,10 +4,11 @@
 // What bounds it: HBM for many rows, latency for few.  A row belongs to a warp, to a CTA of 64 ... 512 threads or to a cluster of two,
 // four or eight such CTAs, chosen so that a thread holds 4 ... 32 values: enough loads in flight to stream, few enough rows per SM
 // to leave none idle.  The two reductions of a row (mean and centred second moment; maximum and sum of exponentials) take one
-// barrier each: warp sums through shared memory, CTA sums pushed into every peer's shared memory before a cluster barrier.  Rows
+// barrier each: warp sums through shared memory; over a cluster, CTA results pushed into every peer's shared memory before a cluster barrier.  Rows
 // whose length is no multiple of four keep vector accesses: they lie on the tensor's 16-byte boundaries (SHIFT below).
 // LayerNorm 32768 x 768: 41.2 -> 32.8 us (6.1 TB/s); 49840 x 674: 165 -> 72; softmax 2339 x 206: 8.2 -> 4.1, 114 x 4255: 13.3 -> 4.4;
-// GroupNorm + SiLU 576 rows of 41 334 (odd image): 141 -> 87 us.
+// GroupNorm + SiLU 576 rows of 41 334 (odd image): 141 -> 87 us.  Eight rows of 32 768 in clusters of eight, one exchange instead of two and gamma
+// asked for ahead of the wait: the registry transformer at batch 8 192.0 -> 189.9 us (four norms), at batch 1 from host arrays 235 -> 228 us.
 #include "common.h"
 #include "launch.cuh"
 
@@ -15,6 +16,7 @@ namespace mb {
 namespace {
 
 constexpr int NR_MAX_THREADS = 512;
+constexpr long long NR_FEW_ROWS = 64;
 
 __device__ __forceinline__ void nr_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void nr_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -102,6 +104,13 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
     if (size > 1) nr_cluster_arrive();
   }
   pdl_launch_dependents();
+  if (!WARP && FAM == ROWS_MEANVAR && !p.per_channel && p.gamma != nullptr && p.rows <= NR_FEW_ROWS) {
+    // few long rows: gamma and beta, as long as the row, come from memory where a streaming layer has passed since (weights: no wait)
+    for (int i = static_cast<int>(rank) * slice + static_cast<int>(threadIdx.x) * 32; i < min(static_cast<int>(p.len), (static_cast<int>(rank) + 1) * slice); i += static_cast<int>(blockDim.x) * 32) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gamma + i));
+      if (p.beta != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.beta + i));
+    }
+  }
   pdl_wait();
   const int T = WARP ? 32 : static_cast<int>(blockDim.x), t = WARP ? static_cast<int>(threadIdx.x & 31) : static_cast<int>(threadIdx.x);
   const long long row = WARP ? static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5) : static_cast<long long>(blockIdx.x / size);
@@ -137,7 +146,12 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
     float s = 0.0f;
 #pragma unroll
     for (int j = 0; j < NV; ++j) s += (v[j][0] + v[j][1]) + (v[j][2] + v[j][3]);
-    sub = row_reduce1<false, WARP>(s, 0, sh, rank, size) / fn;
+    // (over a cluster: each CTA's own mean and second moment first, which then meet in ONE exchange - T. F. Chan, G. H. Golub, R. J. LeVeque
+    // 1979 - with a cluster barrier fewer than exchanging the mean before the second moment)
+    const bool parts = !WARP && size > 1;
+    auto count = [&](int r) { return max(min((r + 1) * slice - lead, len) - max(r * slice - lead, 0), 0); };  // a CTA's elements of the row
+    const float n_own = parts ? static_cast<float>(max(count(static_cast<int>(rank)), 1)) : fn;
+    sub = row_reduce1<false, WARP>(s, 0, sh, 0, 1) / n_own;
     // second moment about that mean, and what the mean is off by: a large common offset costs the first sum its low bits
     float c[2] = {0.0f, 0.0f};
 #pragma unroll
@@ -147,11 +161,32 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
         for (int e = 0; e < 4; ++e)
           if (in(j, e)) { const float d = v[j][e] - sub; c[0] += d; c[1] = fmaf(d, d, c[1]); }
       }
-    row_reduce<false, WARP, 2>(c, 1, sh, rank, size);
-    const float dm = c[0] / fn;
+    row_reduce<false, WARP, 2>(c, 1, sh, 0, 1);
+    const float dm = c[0] / n_own;
     sub += dm;
     // (a second moment beyond fp32 makes the row zero, as the reference's does; c[0] * dm may then be infinite as well)
-    mul = 1.0f / sqrtf((c[1] < INFINITY ? fmaxf(c[1] - c[0] * dm, 0.0f) : c[1]) / fn + p.eps);
+    float m2 = c[1] < INFINITY ? fmaxf(c[1] - c[0] * dm, 0.0f) : c[1];
+    if (parts) {
+      nr_cluster_wait();  // every CTA of the cluster runs (the arrive is at the kernel's start)
+      if (threadIdx.x < size) {
+        uint32_t at;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&sh.cta[0][rank]))), "r"(threadIdx.x));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(sub) : "memory");
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at + static_cast<uint32_t>(sizeof(sh.cta[0]))), "f"(m2) : "memory");
+      }
+      nr_cluster_arrive();
+      nr_cluster_wait();
+      const float ref = sh.cta[0][0];
+      float off = 0.0f;
+      for (int r = 1; r < static_cast<int>(size); ++r) off = fmaf(static_cast<float>(count(r)), sh.cta[0][r] - ref, off);
+      sub = ref + off / fn;
+      m2 = 0.0f;
+      for (int r = 0; r < static_cast<int>(size); ++r) {
+        const float d = sh.cta[0][r] - sub;
+        if (count(r) > 0) m2 += fmaf(static_cast<float>(count(r)) * d, d, sh.cta[1][r]);
+      }
+    }
+    mul = 1.0f / sqrtf(m2 / fn + p.eps);
   } else if (FAM == ROWS_RMS) {
     float q = 0.0f;
 #pragma unroll
