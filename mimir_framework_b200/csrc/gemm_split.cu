@@ -230,13 +230,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // every thread below reads or writes memory that the previous kernels of the stream may still be using
   pdl_wait();
   const bool chan_major = conv || p.ohw > 0;
-  const int slice = p.bn / p.splits;           // columns this CTA finishes
+  const int slice = (p.bn + p.splits - 1) / p.splits;  // columns a CTA finishes; the last ones fewer, or none
   const int oc0 = to * SG_M, row0 = tr * p.bn + split * slice;
   const int quad = warp & 3, group = warp >> 2;
   // Row-major results: a lane holds one output feature of eight columns (rows of Y) and swaps with its neighbour, so that it ends
   // with two consecutive features of four columns, c0 + 2 i + (lane & 1): 8-byte accesses, two rows to a warp instruction.
   const int odd = lane & 1, fe = oc0 + quad * 32 + (lane & ~1), first_row = row0 + odd;
-  const int ldo = static_cast<int>(p.ldo), live = min(slice, p.m - row0) - odd;  // (column c0 + 2 i is written where c0 + 2 i < live)
+  const int ldo = static_cast<int>(p.ldo), mine = min(slice, p.bn - split * slice), live = min(mine, p.m - row0) - odd;  // (column c0 + 2 i is written where c0 + 2 i < live)
   const bool vec = ((ldo & 1) == 0) && fe + 2 <= p.n && ((reinterpret_cast<uintptr_t>(p.out_f32) | reinterpret_cast<uintptr_t>(p.residual)) & 7) == 0;
   const bool one_by_one = !vec && fe < p.n;
   const bool has_res = p.residual != nullptr;
@@ -302,13 +302,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 16; ++j) stg[(c0 + j) * pitch + quad * 32 + lane] = v[j];
       } else {
-        const uint32_t mine = smem_u32(stg + split * slice * pitch + quad * 32 + lane);
-        uint32_t at = mapa_shared(mine, owner) + cl * pitch * 4;
+        const uint32_t own = smem_u32(stg + split * slice * pitch + quad * 32 + lane);
+        uint32_t at = mapa_shared(own, owner) + cl * pitch * 4;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           st_cluster_f32(at, v[j]);
           at += pitch * 4;
-          if (++cl == slice && j < 15) { cl = 0; at = mapa_shared(mine, ++owner); }
+          if (++cl == slice && j < 15) { cl = 0; at = mapa_shared(own, ++owner); }
         }
       }
     }
@@ -317,7 +317,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 
   if (!chan_major) {
-    for (int c0 = group * 8; c0 < slice; c0 += 8 * SG_GROUPS) {  // (warp-uniform)
+    for (int c0 = group * 8; c0 < mine; c0 += 8 * SG_GROUPS) {  // (warp-uniform)
       float v[8];
       if (p.splits == 1) {
         load_acc<8, AP>(taddr + c0, p.bn, v);
@@ -390,9 +390,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   } else {
     // a lane takes a pixel; consecutive lanes run over the slice's pixels first
     const long long hw = conv ? static_cast<long long>(p.conv_h) * p.conv_w : static_cast<long long>(p.ohw);
-    const int nch = min(SG_M, p.n - oc0), total = slice * nch;
-    const int step_ch = SG_THREADS / slice, step_cl = SG_THREADS - step_ch * slice;
-    int ch = static_cast<int>(threadIdx.x) / slice, cl = static_cast<int>(threadIdx.x) - ch * slice;
+    const int nch = min(SG_M, p.n - oc0), total = max(mine, 0) * nch, width = max(mine, 1);
+    const int step_ch = SG_THREADS / width, step_cl = SG_THREADS - step_ch * width;
+    int ch = static_cast<int>(threadIdx.x) / width, cl = static_cast<int>(threadIdx.x) - ch * width;
     for (int i = threadIdx.x; i < total; i += 4 * SG_THREADS) {
       float a[4], r[4];
       long long o[4];
@@ -410,7 +410,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
         ch += step_ch;
         cl += step_cl;
-        if (cl >= slice) { cl -= slice; ++ch; }
+        if (cl >= width) { cl -= width; ++ch; }
       }
       if (p.activation >= 0) {
 #pragma unroll
@@ -442,7 +442,9 @@ int prepare_split_kernel() {
 // whatever they take of it.
 __global__ void __launch_bounds__(SG_THREADS, 2) split_footprint_kernel() {}
 
-constexpr int SG_SPLITS[] = {1, 2, 3, 4, 6, 8, 16};
+// (any number of CTAs may share a tile; seven and nine fit the GPCs no better than eight and ten: 40 x 1024 x 32768 in ten 31.1 us, nine 33.4,
+// eight 35.1, as more SMs have weights on the way)
+constexpr int SG_SPLITS[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
 
 // Clusters of SG_SPLITS[i] CTAs that run at the same time, one or two CTAs to an SM.  A cluster lives in one GPC, whose SM count is no
 // multiple of it: of the 148 SMs clusters of four use 132, of eight 120, of sixteen 112 (128 CTAs in clusters of eight: 12.9 us, two
@@ -493,11 +495,10 @@ SplitPlan plan_split(const GemmArgs& g, int bk, int kblocks) {
     const int stage = (g.w_planes * SG_M + g.a_planes * bn) * bk * 2;
     for (int i = 0; i < static_cast<int>(sizeof(SG_SPLITS) / sizeof(int)); ++i) {
       const int splits = SG_SPLITS[i];
-      if (splits > kblocks) break;
-      if (bn % splits != 0) continue;
+      if (splits > kblocks || splits > bn) break;
       const long long ctas = tiles * splits;
       // CTAs that share an SM overlap one's loads and stores with the other's MMAs: whole rounds of two per SM
-      const bool two = ctas > sms && 2 * stage <= SG_RING_TWO && bn * (SG_M + 1) * 4 <= SG_RING_TWO;
+      const bool two = ctas > sms && 2 * stage <= SG_RING_TWO && (bn + splits - 1) * (SG_M + 1) * 4 <= SG_RING_TWO;
       const int active = active_clusters(i, two);
       if (active <= 0) continue;
       const long long rounds = (tiles + active - 1) / active;
@@ -555,12 +556,12 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
   p.stage_bytes = (WP * SG_M + AP * p.bn) * BK * 2;
   const int per_split = (p.kblocks + p.splits - 1) / p.splits;
   const long long ctas = static_cast<long long>(p.tiles_o) * ((g.m + p.bn - 1) / p.bn) * p.splits;
-  const bool two = ctas > ctx().sm_count && 2 * p.stage_bytes <= SG_RING_TWO && p.bn * (SG_M + 1) * 4 <= SG_RING_TWO;
+  const bool two = ctas > ctx().sm_count && 2 * p.stage_bytes <= SG_RING_TWO && (p.bn + p.splits - 1) * (SG_M + 1) * 4 <= SG_RING_TWO;
   p.stages = (two ? SG_RING_TWO : SG_RING_LIMIT) / p.stage_bytes;
   if (p.stages > SG_MAX_STAGES) p.stages = SG_MAX_STAGES;
   if (p.stages > per_split) p.stages = per_split;
   // the staging tile gets a place of its own where that leaves three stages (or all there are)
-  const int staging = p.bn * (SG_M + 1) * 4, limit = two ? SG_RING_TWO : SG_RING_LIMIT;
+  const int staging = p.splits * ((p.bn + p.splits - 1) / p.splits) * (SG_M + 1) * 4, limit = two ? SG_RING_TWO : SG_RING_LIMIT;
   const int fit = (limit - staging) / p.stage_bytes;
   p.stg_off = 0;
   if (p.splits > 1 && (fit >= p.stages || fit >= 3)) {
@@ -589,7 +590,7 @@ double gemm_split_cycles(const GemmArgs& g, int bk, int* bn, int* splits) {
   int fb = 0, fs = 0;
   if (e && sscanf(e, "%d,%d", &fb, &fs) == 2) {
     *bn = fb; *splits = fs;
-    return fb >= 16 && fb <= SG_MAX_BN && fb % 16 == 0 && fs >= 1 && fs <= SG_MAX_SPLITS && fb % fs == 0 && fs <= kblocks ? 0.0 : never;
+    return fb >= 16 && fb <= SG_MAX_BN && fb % 16 == 0 && fs >= 1 && fs <= SG_MAX_SPLITS && fs <= fb && fs <= kblocks ? 0.0 : never;
   }
   const SplitPlan plan = plan_split(g, bk, kblocks);
   *bn = plan.bn; *splits = plan.splits;

@@ -20,7 +20,7 @@ def rt():
 
 @pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W, abi.PREC_BF16])
 @pytest.mark.parametrize("form,m,n,k", [("16,1", 17, 1, 64), ("16,8", 17, 129, 520), ("32,4", 33, 127, 300), ("48,2", 97, 256, 128), ("64,8", 65, 70, 1000),
-                                        ("96,1", 200, 300, 65), ("128,1", 129, 128, 1), ("128,8", 257, 385, 2048), ("", 40, 1000, 4100), ("", 333, 1000, 1000)])
+                                        ("96,1", 200, 300, 65), ("48,10", 50, 131, 700), ("32,12", 33, 70, 1000), ("64,5", 100, 129, 520), ("128,1", 129, 128, 1), ("128,8", 257, 385, 2048), ("", 40, 1000, 4100), ("", 333, 1000, 1000)])
 def test_linear_against_float64(rt, monkeypatch, precision, form, m, n, k):
     if form:
         monkeypatch.setenv("MIMIR_B200_GEMM_SPLIT", form)
@@ -43,7 +43,7 @@ def test_linear_against_float64(rt, monkeypatch, precision, form, m, n, k):
     assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
 
 
-@pytest.mark.parametrize("form", ["16,1", "48,2", "128,8", ""])
+@pytest.mark.parametrize("form", ["16,1", "48,2", "48,5", "128,8", ""])
 @pytest.mark.parametrize("batch,ic,oc,h,w,k,stride,pad", [(1, 64, 130, 9, 7, 3, 1, 1), (3, 32, 40, 5, 11, 1, 1, 0), (2, 96, 16, 8, 8, 5, 1, 2), (2, 3, 70, 17, 19, 7, 2, 3)])
 def test_convolution_against_the_port(rt, monkeypatch, form, batch, ic, oc, h, w, k, stride, pad):
     if form:
@@ -56,7 +56,7 @@ def test_convolution_against_the_port(rt, monkeypatch, form, batch, ic, oc, h, w
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
 
 
-@pytest.mark.parametrize("form", ["16,1", "48,3", "48,6", "96,6", "128,2", ""])
+@pytest.mark.parametrize("form", ["16,1", "16,5", "48,3", "48,10", "96,6", "128,2", ""])
 @pytest.mark.parametrize("m,k,n", [(1, 40, 33), (50, 70, 131), (97, 200, 255), (130, 129, 64)])
 def test_chain_through_operand_planes(rt, monkeypatch, form, m, k, n):
     """Linear -> GELU -> Linear: the first layer writes the second one's operand planes (zero up to a multiple of 64 columns), odd row
