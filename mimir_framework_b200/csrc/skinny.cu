@@ -314,17 +314,27 @@ skinny_stream_kernel(const float* __restrict__ x, const void* __restrict__ w_any
 __global__ void skinny_finish_kernel(const float* __restrict__ part, const float* __restrict__ bias, const float* __restrict__ residual,
                                      float* __restrict__ y, int m, int n, int kslices, int act, int grid, int items, int tile_cols) {
   pdl_launch_dependents();
-  pdl_wait();
-  const long long total = static_cast<long long>(m) * n;
+  const long long total = static_cast<long long>(m) * n, step = static_cast<long long>(gridDim.x) * blockDim.x;
   const ItemSplit split(grid > 0 ? items : 1, grid > 0 ? grid : 1);
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int o = static_cast<int>(i % n);
-    int np = kslices;
+  // What does not come from the streaming kernel is fetched ahead of the wait for it (the residual was complete before that kernel passed
+  // its own wait): registry transformer, five such launches, 190.5 -> 189.2 us at batch 8, 230 -> 224.6 at batch 1 from host arrays.
+  long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  int o = 0, np = 0;
+  float b = 0.0f, r = 0.0f;
+  auto ahead = [&]() {
+    if (i >= total) return;
+    o = static_cast<int>(i % n);
+    np = kslices;
     if (grid > 0) {
       const int tile = o / tile_cols;
       np = split.owner((tile + 1) * kslices - 1) - split.owner(tile * kslices) + 1;
     }
+    if (bias != nullptr) b = __ldg(bias + o);
+    if (residual != nullptr) r = __ldg(residual + i);  // a residual Add folded into this layer
+  };
+  ahead();
+  pdl_wait();
+  for (; i < total; i += step, ahead()) {
     // the partials are added in K order; eight loads are issued before the first add so that a long chain does not pay
     // the memory latency once per partial
     float s = 0.0f;
@@ -332,14 +342,14 @@ __global__ void skinny_finish_kernel(const float* __restrict__ part, const float
     for (; ks + 8 <= np; ks += 8) {
       float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = __ldcs(part + static_cast<long long>(ks + u) * total + i);
+      for (int u = 0; u < 8; ++u) v[u] = __ldcs(part + (ks + u) * total + i);
 #pragma unroll
       for (int u = 0; u < 8; ++u) s += v[u];
     }
-    for (; ks < np; ++ks) s += __ldcs(part + static_cast<long long>(ks) * total + i);
-    if (bias != nullptr) s += __ldg(bias + o);
+    for (; ks < np; ++ks) s += __ldcs(part + ks * total + i);
+    if (bias != nullptr) s += b;
     s = sk_act(s, act);
-    if (residual != nullptr) s += __ldg(residual + i);  // a residual Add folded into this layer
+    if (residual != nullptr) s += r;
     y[i] = s;
   }
 }
