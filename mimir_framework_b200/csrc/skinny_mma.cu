@@ -18,6 +18,8 @@
 // Within a step of 16 samples (12 layers of 768, vocabulary 32000), by CTA stamps from the input's arrival to the last store:
 // 768 -> 2304 with LayerNorm 8.0 -> 5.0 us, 768 -> 768 5.4 -> 2.9, 768 -> 3072 with LayerNorm 7.3 -> 5.6, 3072 -> 768 8.5 -> 4.2.  What is left of a
 // LayerNorm form: x 0.6, statistics and planes 2.3, products 1.5 (the instruction issues every 32 cycles), sums and store 0.6.
+#include <type_traits>
+
 #include "common.h"
 #include "epilogue.cuh"
 #include "launch.cuh"
@@ -44,13 +46,17 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// x0, x1 as pairs of bfloat16: hi + mid + lo is x exactly (each cut off after eight significant bits); infinities stay in hi
+// x0, x1 as pairs of bfloat16: hi + mid + lo is x exactly (each cut off after eight significant bits); INF: infinities stay in hi (what a
+// LayerNorm makes of a row with one is NaN anyway; a step of 16 samples 624.5 -> 620 us)
+template <bool INF>
 __device__ __forceinline__ void planes3(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const uint32_t u0 = __float_as_uint(x0), u1 = __float_as_uint(x1);
   hi = __byte_perm(u0, u1, 0x7632);
   float r0 = x0 - __uint_as_float(u0 & 0xffff0000u), r1 = x1 - __uint_as_float(u1 & 0xffff0000u);
-  r0 = fabsf(x0) == INFINITY ? 0.0f : r0;
-  r1 = fabsf(x1) == INFINITY ? 0.0f : r1;
+  if (INF) {
+    r0 = fabsf(x0) == INFINITY ? 0.0f : r0;
+    r1 = fabsf(x1) == INFINITY ? 0.0f : r1;
+  }
   const uint32_t v0 = __float_as_uint(r0), v1 = __float_as_uint(r1);
   mid = __byte_perm(v0, v1, 0x7632);
   lo = __byte_perm(__float_as_uint(r0 - __uint_as_float(v0 & 0xffff0000u)), __float_as_uint(r1 - __uint_as_float(v1 & 0xffff0000u)), 0x7632);
@@ -209,15 +215,18 @@ __global__ void __launch_bounds__(SM_THREADS, LOOP ? 1 : 2) skinny_mma_kernel(co
   }
   // (rows past m hold what the LayerNorm makes of zeros: their products are never written)
   uint32_t hi[U][NT][4], mid[U][NT][4], lo[U][NT][4];
+  auto cut = [&](auto inf) {
 #pragma unroll
-  for (int u = 0; u < U; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
+      for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        planes3(v[u][j][h].x, v[u][j][h].y, hi[u][j][2 * h], mid[u][j][2 * h], lo[u][j][2 * h]);
-        planes3(v[u][j][h].z, v[u][j][h].w, hi[u][j][2 * h + 1], mid[u][j][2 * h + 1], lo[u][j][2 * h + 1]);
-      }
+        for (int h = 0; h < 2; ++h) {
+          planes3<decltype(inf)::value>(v[u][j][h].x, v[u][j][h].y, hi[u][j][2 * h], mid[u][j][2 * h], lo[u][j][2 * h]);
+          planes3<decltype(inf)::value>(v[u][j][h].z, v[u][j][h].w, hi[u][j][2 * h + 1], mid[u][j][2 * h + 1], lo[u][j][2 * h + 1]);
+        }
+  };
+  if (p.ln) cut(std::false_type{}); else cut(std::true_type{});
 
   int buf = 0;
 #pragma unroll 1
