@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 6 : 2) rms_onepass_kernel(const 
   __shared__ float redf[33];
   __shared__ double red[T / 32];
   constexpr int VEC = CHUNK / (T * 4), STEP = VEC < 4 ? VEC : 4;  // float4 of a thread, side by side in the last loop
+  static_assert(CHUNK % (T * 4) == 0 && VEC % STEP == 0, "whole float4, in whole steps");
   const int tid = threadIdx.x;
   if (tid == 0) {
     s_abort = 0;
