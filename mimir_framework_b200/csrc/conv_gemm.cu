@@ -10,7 +10,7 @@
 // descriptors.  Activation bytes from L2 fall to (16 + ks - 1) / (16 ks) of before (0.375 for 3 x 3).
 //
 //   warp 0     : TMA producer of activation tiles   (ring of A_STAGES, one per (32 channels, kernel column))
-//   warp 1     : MMA issuer: weights are the M side (128 output channels), 256 pixels the N side; two accumulators in TMEM
+//   warp 1     : MMA issuer: weights are the M side (128 output channels), 256 pixels (or 128) the N side; two accumulators in TMEM
 //   warps 2..9 : epilogue: 32 x 32 chunks turned around in shared memory so that a lane owns a pixel; NCHW stores
 //   warp 10    : TMA producer of weight tiles       (ring of W_STAGES, one per tap)
 // Every wait is bounded, as in gemm_sm100.cu.
@@ -27,7 +27,7 @@ namespace mb {
 namespace {
 
 constexpr int CG_THREADS = 352;
-constexpr int CG_N = 256;                      // pixels of a tile: 16 x 16 or, for 1 x 1 kernels, 256 of the flattened image
+constexpr int CG_N = 256;                      // pixels of a tile: 16 x 16 or, for 1 x 1 kernels, 256 of the flattened image; or half of that
 constexpr int CG_M = 128;                      // output channels of a tile
 constexpr int CG_BK = 32;                      // channels of a K block: 64-byte swizzle rows
 constexpr int CG_W_TILE = CG_M * CG_BK * 2;
@@ -37,7 +37,7 @@ constexpr int CG_SMEM_MAX = 232448;
 
 struct ConvGemmParams {
   int batch, oc, h, w, ks, cblocks;            // cblocks = channels / 32
-  int tw_log, tiles_x, tiles_y, tiles_o, num_tiles;  // a tile is 1 << tw_log pixels wide
+  int px, tw_log, tiles_x, tiles_y, tiles_o, num_tiles;  // a tile has px pixels (256 or 128) and is 1 << tw_log of them wide
   int a_stages, a_stage_bytes, w_stages;
   const float* residual;
   int res_up;                                  // 1: the residual is [oc][h/2][w/2], a value for 2 x 2 pixels
@@ -55,7 +55,7 @@ __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) { 
   int s = t / p.tiles_o;
   c.x0 = (s % p.tiles_x) << p.tw_log;
   s /= p.tiles_x;
-  c.y0 = (s % p.tiles_y) * (CG_N >> p.tw_log);
+  c.y0 = (s % p.tiles_y) * (p.px >> p.tw_log);
   c.n = s / p.tiles_y;
   return c;
 }
@@ -144,7 +144,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   } else if (warp == 1) {
     const bool one = elect_one();
-    const uint32_t idesc = make_idesc(CG_M, CG_N, p.f16);
+    const uint32_t idesc = make_idesc(CG_M, p.px, p.f16);
     int as = 0, ws = 0, acc = 0;
     uint32_t aph = 0, wph = 0, acc_phase = 0;
     bool ok = true, w_ready = false;
@@ -190,6 +190,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // epilogue: TMEM lane = output channel, column = pixel (16 to a row)
     const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
     float* tbuf = epi + ew * (32 * 33);
+    const int chunks = p.px / 64;  // of 32 pixels, in each half of the tile
     const long long hw = static_cast<long long>(p.h) * p.w;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -198,7 +199,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const int oc0 = c.oc0 + quad * 32, nch = p.oc - oc0;
       // chunk ci of this warp: 32 consecutive pixels of the tile
       auto place = [&](int ci, bool& in, long long& o0) {
-        const int px = (half * 4 + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
+        const int px = (half * chunks + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
         in = y < p.h && x < p.w;
         o0 = (static_cast<long long>(c.n) * p.oc + oc0) * hw + static_cast<long long>(y) * p.w + x;
       };
@@ -211,7 +212,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         place(ci, in, o0);
         // an upsampled residual: the two rows of a chunk read eight neighbours each, one sector, of the half-size image
         if (p.res_up) {
-          const int px = (half * 4 + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
+          const int px = (half * chunks + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
           step = hw >> 2;
           o0 = (static_cast<long long>(c.n) * p.oc + oc0) * step + static_cast<long long>(y >> 1) * (p.w >> 1) + (x >> 1);
         }
@@ -230,13 +231,13 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * CG_N);
       if (nch > 0) {
 #pragma unroll 1
-        for (int ci = 0; ci < 4; ++ci) {
-          if (c.y0 + (((half * 4 + ci) * 32) >> p.tw_log) >= p.h) break;  // warp-uniform
+        for (int ci = 0; ci < chunks; ++ci) {
+          if (c.y0 + (((half * chunks + ci) * 32) >> p.tw_log) >= p.h) break;  // warp-uniform
           bool in;
           long long o0;
           place(ci, in, o0);
           float v[32];
-          tmem_ld_32x32(taddr + (half * 4 + ci) * 32, v);
+          tmem_ld_32x32(taddr + (half * chunks + ci) * 32, v);
 #pragma unroll
           for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = __fmul_rn(v[j], p.acc_scale);  // [pixel][channel]
           __syncwarp();
@@ -250,7 +251,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (p.residual != nullptr) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] += q[j];
-            if (ci < 3) request(ci + 1);
+            if (ci + 1 < chunks) request(ci + 1);
           }
           if (in) {
 #pragma unroll
@@ -279,13 +280,33 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // lines in every channel plane: with 16-pixel rows its scattered 64-byte stores held DRAM at 4 TB/s).  Otherwise 16 x 16 (32 x 8 where
 // the width allows whole lines measured the same: there the MMAs, not the stores, set the pace).
 struct ConvShape { int h, w, tw_log, tiles_x, tiles_y; };
-ConvShape conv_shape(const GemmArgs& g) {
+ConvShape conv_shape(const GemmArgs& g, int px) {
   ConvShape s{g.conv_h, g.conv_w, 4, 0, 0};
-  if (g.conv_ks == 1) { s.w = g.conv_h * g.conv_w; s.h = 1; s.tw_log = 8; }
-  const int tw = 1 << s.tw_log, th = CG_N >> s.tw_log;
+  if (g.conv_ks == 1) { s.w = g.conv_h * g.conv_w; s.h = 1; s.tw_log = px == CG_N ? 8 : 7; }
+  const int tw = 1 << s.tw_log, th = px >> s.tw_log;
   s.tiles_x = (s.w + tw - 1) / tw;
   s.tiles_y = (s.h + th - 1) / th;
   return s;
+}
+
+long long tiles_of(const GemmArgs& g, int px) {
+  const ConvShape sh = conv_shape(g, px);
+  const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
+  return g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
+}
+
+// Estimated SM cycles of a launch and the tile it takes: within 5 % of 50 measured launches, K = 64 ... 4608.  Tiles of 128 pixels (half of
+// the accumulator's columns: the same sums in the same order, bit for bit) where 256 leave SMs without one: they load the weights whole, so
+// that one takes 0.77 of a tile's MMA time with three MMAs per product and 0.86 with two, and 2800 cycles less beside it.  16 x 512 -> 512 on
+// 16^2, 64 tiles: 78.1 -> 62.4 us; 4 x 128 -> 128 on 63^2, 64 tiles: 30.9 -> 25.4; 3 x 256 -> 256 on 56^2, 96 tiles: stays (45.3, 62.7 in 192).
+double conv_cycles(const GemmArgs& g, int* px) {
+  const int sms = ctx().sm_count, products = g.a_planes + g.w_planes - 1;
+  const double mma = 1.15 * g.k / 16.0 * products * 128.0, part = (products == 3 ? 0.77 : products == 2 ? 0.86 : 0.95) * mma;
+  const double whole = 17400.0 + static_cast<double>((tiles_of(g, CG_N) + sms - 1) / sms) * (mma > 4500.0 ? mma : 4500.0);
+  const double half = 14600.0 + static_cast<double>((tiles_of(g, CG_N / 2) + sms - 1) / sms) * (part > 2800.0 ? part : 2800.0);
+  const char* force = getenv("MIMIR_B200_CONV_PX");  // "128", "256": always
+  *px = force && (atoi(force) == CG_N || atoi(force) == CG_N / 2) ? atoi(force) : half < whole ? CG_N / 2 : CG_N;
+  return *px == CG_N ? whole : half;
 }
 
 template <int AP, int WP>
@@ -293,8 +314,9 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   const int ks = g.conv_ks, pad = g.conv_pad;
   ConvGemmParams p;
   p.batch = g.m / ((g.conv_h + 2 * pad) * (g.conv_w + 2 * pad));
-  const ConvShape sh = conv_shape(g);
-  const int hp = sh.h + 2 * pad, wp = sh.w + 2 * pad, tw = 1 << sh.tw_log, th = CG_N >> sh.tw_log;
+  conv_cycles(g, &p.px);
+  const ConvShape sh = conv_shape(g, p.px);
+  const int hp = sh.h + 2 * pad, wp = sh.w + 2 * pad, tw = 1 << sh.tw_log, th = p.px >> sh.tw_log;
   p.oc = g.n; p.h = sh.h; p.w = sh.w; p.ks = ks; p.cblocks = g.conv_c / CG_BK;
   p.tw_log = sh.tw_log;
   p.tiles_x = sh.tiles_x; p.tiles_y = sh.tiles_y;
@@ -334,11 +356,7 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
 
 }  // namespace
 
-long long conv_gemm_tiles(const GemmArgs& g) {
-  const ConvShape sh = conv_shape(g);
-  const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
-  return g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
-}
+long long conv_gemm_tiles(const GemmArgs& g) { return tiles_of(g, CG_N); }
 
 double conv_gemm_cycles(const GemmArgs& g) {
   constexpr double never = 1e30;
@@ -351,9 +369,8 @@ double conv_gemm_cycles(const GemmArgs& g) {
   // 1 x 1 (and im2col rows): nothing to share between taps; long K is better off in CTA pairs (K = 4608, 512 channels: 170 against
   // 111 us), short K is bound by its stores (K = 192, 64 channels: 139 against 247 us)
   if (g.conv_ks == 1 && g.conv_c > 1024) return never;
-  const long long waves = (conv_gemm_tiles(g) + ctx().sm_count - 1) / ctx().sm_count;
-  const double mma = 1.15 * g.k / 16.0 * (g.a_planes + g.w_planes - 1) * 128.0;
-  return 17400.0 + waves * (mma > 4500.0 ? mma : 4500.0);  // (within 5 % of 50 measured launches, K = 64 ... 4608)
+  int px;
+  return conv_cycles(g, &px);
 }
 
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {

@@ -91,3 +91,37 @@ def test_residual_block_behind_an_upsample(rt, batch, ic, oc, h, w, skip_conv):
         want = port.conv2d(t, ws[1], oc, oc, 2 * h, 2 * w, 3, 1, 1, False).ravel()
         want = want + (port.conv2d(u, ws[2], ic, oc, 2 * h, 2 * w, 1, 1, 0, False).ravel() if skip_conv else u)
         assert np.linalg.norm(got[i] - want) <= 2e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W])
+@pytest.mark.parametrize("batch,ic,oc,h,w,k,up", [(1, 32, 16, 16, 16, 3, 0), (2, 64, 130, 17, 33, 3, 0), (3, 96, 40, 31, 15, 5, 0), (1, 32, 260, 9, 48, 7, 0), (5, 32, 33, 1, 1, 3, 0),
+                                                  (2, 64, 128, 20, 40, 1, 0), (3, 64, 70, 3, 43, 1, 0), (40, 32, 32, 12, 10, 3, 1)])
+def test_tiles_of_128_pixels_keep_the_bits_of_256(rt, monkeypatch, precision, batch, ic, oc, h, w, k, up):
+    """Half of a tile's pixels, the same sums in the same order: 8 rows of 16, or 128 of a line; with a residual, plain or read at half size."""
+    monkeypatch.setenv("MIMIR_B200_CONV_SPATIAL", "1")
+    r = np.random.default_rng(batch * ic + oc + k)
+    wt = (r.standard_normal(oc * ic * k * k) / np.sqrt(ic * k * k)).astype(np.float32)
+    if precision != abi.PREC_BF16X2:
+        wt = (wt.view(np.uint32) & 0xffff0000).view(np.float32)
+    s = 2 if up else 1
+    conv = lambda name, a, b: make_desc(name, "Conv2d", inputs=[a], output=b, in_channels=ic, out_channels=oc, input_height=s * h, input_width=s * w,  # noqa: E731
+                                        kernel=k, stride=1, padding=k // 2, params_count=wt.size)
+    if up:
+        descs = [make_desc("u", "UpsampleNearest", inputs=["x"], output="u", in_channels=ic, out_h=h, out_w=w, scale_h=2, scale_w=2), conv("c", "u", "t"), conv("d", "t", "y"),
+                 make_desc("a", "Add", inputs=["y", "u"], output="x")]
+    else:
+        descs = [conv("c", "x", "y"), make_desc("a", "Add", inputs=["y", "r"], output="x")]
+    ins = {"x": (r.standard_normal((batch, ic * h * w)).astype(np.float32), False)}
+    if not up:
+        ins["r"] = (r.standard_normal((batch, oc * h * w)).astype(np.float32), False)
+    got = []
+    for px in ("256", "128"):
+        monkeypatch.setenv("MIMIR_B200_CONV_PX", px)
+        m = rt.GraphModel(descs, precision)
+        for j, d in enumerate(descs):
+            if d.type == b"Conv2d":
+                m.upload_weights(j, wt)
+        m.plan({n: (a.shape[1], bc) for n, (a, bc) in ins.items()}, batch)
+        got.append(m.forward(ins, batch, oc * s * s * h * w))
+        m.close()
+    assert np.array_equal(got[0], got[1])
