@@ -4,15 +4,15 @@
 //
 // That form is bound by what an SM can take from L2: a tile of 256 pixels reads its activation block once per tap, nine times for
 // a 3 x 3 kernel (80 bytes per cycle and SM on a 128 -> 128 layer in the two-MMA mode, where about 50 arrive; the tensor pipe
-// was 48 to 54 % busy).  Here a tile is 16 x 16 pixels of one sample, and a K block of 32 channels brings the tile with its rows of halo,
-// 16 x (16 + ks - 1) pixels, ONCE per kernel column: a vertical shift by one row is 16 pixels further into the same
-// shared-memory tile, 16 x 64 bytes, a whole number of swizzle atoms, so the ks taps of a column are the same copy under ks
+// was 48 to 54 % busy).  Here a tile is 16 x 16 pixels of one sample, and a K block of 32 or 64 channels brings the tile with its rows of
+// halo, 16 x (16 + ks - 1) pixels, ONCE per kernel column: a vertical shift by one row is 16 pixels further into the same
+// shared-memory tile, 16 x 64 or 128 bytes, a whole number of swizzle atoms, so the ks taps of a column are the same copy under ks
 // descriptors.  Activation bytes from L2 fall to (16 + ks - 1) / (16 ks) of before (0.375 for 3 x 3).
 //
-//   warp 0     : TMA producer of activation tiles   (ring of A_STAGES, one per (32 channels, kernel column))
+//   warp 0     : TMA producer of activation tiles   (ring of A_STAGES, one per (BK channels, kernel column))
 //   warp 1     : MMA issuer: weights are the M side (128 output channels), 256 pixels (or 128) the N side; two accumulators in TMEM
 //   warps 2..9 : epilogue: 32 x 32 chunks turned around in shared memory so that a lane owns a pixel; NCHW stores
-//   warp 10    : TMA producer of weight tiles       (ring of W_STAGES, one per tap)
+//   warp 10    : TMA producer of weight tiles       (ring of W_STAGES, one per tap and plane)
 // Every wait is bounded, as in gemm_sm100.cu.
 #include "common.h"
 #include "epilogue.cuh"
@@ -29,14 +29,12 @@ namespace {
 constexpr int CG_THREADS = 352;
 constexpr int CG_N = 256;                      // pixels of a tile: 16 x 16 or, for 1 x 1 kernels, 256 of the flattened image; or half of that
 constexpr int CG_M = 128;                      // output channels of a tile
-constexpr int CG_BK = 32;                      // channels of a K block: 64-byte swizzle rows
-constexpr int CG_W_TILE = CG_M * CG_BK * 2;
 constexpr int CG_EPI = 8 * 32 * 33 * 4;
-constexpr int CG_MAX_RING = 8;
+constexpr int CG_MAX_RING = 16;
 constexpr int CG_SMEM_MAX = 232448;
 
 struct ConvGemmParams {
-  int batch, oc, h, w, ks, cblocks;            // cblocks = channels / 32
+  int batch, oc, h, w, ks, cblocks;            // cblocks = channels / BK
   int px, tw_log, tiles_x, tiles_y, tiles_o, num_tiles;  // a tile has px pixels (256 or 128) and is 1 << tw_log of them wide
   int a_stages, a_stage_bytes, w_stages;
   const float* residual;
@@ -60,15 +58,17 @@ __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) { 
   return c;
 }
 
-template <int AP, int WP>
+// BK: channels of a K block, 32 (64-byte swizzle rows) or 64 (128-byte rows)
+template <int AP, int WP, int BK>
 __global__ void __launch_bounds__(CG_THREADS, 1)
 conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const ConvGemmParams p) {
+  constexpr int W_TILE = CG_M * BK * 2;
   extern __shared__ __align__(1024) uint8_t cg_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(cg_smem_raw) + 1023) & ~uintptr_t(1023));
   const int a_plane = p.a_stage_bytes / AP;                                   // halo tile of one plane
   uint8_t* a_ring = smem;
   uint8_t* w_ring = smem + p.a_stages * p.a_stage_bytes;
-  float* epi = reinterpret_cast<float*>(w_ring + p.w_stages * WP * CG_W_TILE);
+  float* epi = reinterpret_cast<float*>(w_ring + p.w_stages * W_TILE);
   __shared__ uint64_t a_full[CG_MAX_RING], a_empty[CG_MAX_RING], w_full[CG_MAX_RING], w_empty[CG_MAX_RING], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -105,8 +105,8 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (one) {
             uint8_t* dst = a_ring + stage * p.a_stage_bytes;
             mbar_expect_tx(&a_full[stage], static_cast<uint32_t>(p.a_stage_bytes));
-            tma_load_5d(dst, &map_a, &a_full[stage], cb * CG_BK, c.x0 + kw, c.y0, c.n, 0);  // (padded coordinates: the halo starts at y0)
-            if (AP == 2) tma_load_5d(dst + a_plane, &map_a, &a_full[stage], cb * CG_BK, c.x0 + kw, c.y0, c.n, 1);
+            tma_load_5d(dst, &map_a, &a_full[stage], cb * BK, c.x0 + kw, c.y0, c.n, 0);  // (padded coordinates: the halo starts at y0)
+            if (AP == 2) tma_load_5d(dst + a_plane, &map_a, &a_full[stage], cb * BK, c.x0 + kw, c.y0, c.n, 1);
           }
           __syncwarp();
           if (++stage == p.a_stages) { stage = 0; phase ^= 1; }
@@ -126,16 +126,17 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       for (int cb = 0; cb < p.cblocks && ok; ++cb)
         for (int kw = 0; kw < p.ks && ok; ++kw)
           for (int kh = 0; kh < p.ks; ++kh) {
-            if (!mbar_wait_warp(&w_empty[stage], phase ^ 1, &abort_flag, p.err_word, 53)) { ok = false; break; }
-            if (one) {
-              uint8_t* dst = w_ring + stage * (WP * CG_W_TILE);
-              const int col = ((kh * p.ks + kw) * p.cblocks + cb) * CG_BK;
-              mbar_expect_tx(&w_full[stage], WP * CG_W_TILE);
-              tma_load_3d(dst, &map_w, &w_full[stage], col, oc0, 0);
-              if (WP == 2) tma_load_3d(dst + CG_W_TILE, &map_w, &w_full[stage], col, oc0, 1);
+            const int col = ((kh * p.ks + kw) * p.cblocks + cb) * BK;
+            for (int plane = 0; plane < WP && ok; ++plane) {  // a ring slot per plane
+              if (!mbar_wait_warp(&w_empty[stage], phase ^ 1, &abort_flag, p.err_word, 53)) { ok = false; break; }
+              if (one) {
+                mbar_expect_tx(&w_full[stage], W_TILE);
+                tma_load_3d(w_ring + stage * W_TILE, &map_w, &w_full[stage], col, oc0, plane);
+              }
+              __syncwarp();
+              if (++stage == p.w_stages) { stage = 0; phase ^= 1; }
             }
-            __syncwarp();
-            if (++stage == p.w_stages) { stage = 0; phase ^= 1; }
+            if (!ok) break;
           }
     }
     for (int s = 0; s < p.w_stages; ++s) {
@@ -153,30 +154,32 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       tcgen05_fence_after();
       const uint32_t d = tmem + static_cast<uint32_t>(acc * CG_N);
       bool first = true;
-      for (int b = 0; b < p.cblocks * p.ks && ok; ++b) {  // (32 channels, kernel column)
+      for (int b = 0; b < p.cblocks * p.ks && ok; ++b) {  // (BK channels, kernel column)
         if (!mbar_wait_warp(&a_full[as], aph, &abort_flag, p.err_word, 56)) { ok = false; break; }
-        const uint64_t da0 = make_smem_desc(smem_u32(a_ring + as * p.a_stage_bytes), 64);
-        for (int kh = 0; kh < p.ks; ++kh) {
-          if (!__all_sync(0xffffffffu, w_ready) && !mbar_wait_warp(&w_full[ws], wph, &abort_flag, p.err_word, 57)) { ok = false; break; }
-          tcgen05_fence_after();
-          // kh rows further down: tile width x 64 bytes, in the descriptor's address field (16 bytes)
-          const uint64_t da = da0 + static_cast<uint64_t>(kh << (p.tw_log + 2)), da_lo = da + static_cast<uint64_t>(a_plane >> 4);
-          const uint64_t dw = make_smem_desc(smem_u32(w_ring + ws * (WP * CG_W_TILE)), 64), dw_lo = dw + (CG_W_TILE >> 4);
-          uint64_t* w_done = &w_empty[ws];
-          if (++ws == p.w_stages) { ws = 0; wph ^= 1; }
-          w_ready = mbar_test(&w_full[ws], wph);
-          if (one) {
+        const uint64_t da0 = make_smem_desc(smem_u32(a_ring + as * p.a_stage_bytes), BK * 2);
+        for (int kh = 0; kh < p.ks && ok; ++kh) {
+          // kh rows further down: tile width x 2 BK bytes, in the descriptor's address field (16 bytes)
+          const uint64_t da = da0 + static_cast<uint64_t>((kh << p.tw_log) * (BK / 8)), da_lo = da + static_cast<uint64_t>(a_plane >> 4);
 #pragma unroll
-            for (int k = 0; k < CG_BK / 16; ++k) {
-              umma_bf16(d, dw + 2 * k, da + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
-              if (AP == 2) umma_bf16(d, dw + 2 * k, da_lo + 2 * k, idesc, 1u);
-              if (WP == 2) umma_bf16(d, dw_lo + 2 * k, da + 2 * k, idesc, 1u);
+          for (int plane = 0; plane < WP; ++plane) {  // of the weights; their lo plane meets the activations' hi plane only
+            if (!__all_sync(0xffffffffu, w_ready) && !mbar_wait_warp(&w_full[ws], wph, &abort_flag, p.err_word, 57)) { ok = false; break; }
+            tcgen05_fence_after();
+            const uint64_t dw = make_smem_desc(smem_u32(w_ring + ws * W_TILE), BK * 2);
+            uint64_t* w_done = &w_empty[ws];
+            if (++ws == p.w_stages) { ws = 0; wph ^= 1; }
+            w_ready = mbar_test(&w_full[ws], wph);
+            if (one) {
+#pragma unroll
+              for (int k = 0; k < BK / 16; ++k) {
+                umma_bf16(d, dw + 2 * k, da + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+                if (AP == 2 && plane == 0) umma_bf16(d, dw + 2 * k, da_lo + 2 * k, idesc, 1u);
+              }
+              umma_commit(w_done);
+              if (kh + 1 == p.ks && plane + 1 == WP) umma_commit(&a_empty[as]);
             }
-            umma_commit(w_done);
-            if (kh + 1 == p.ks) umma_commit(&a_empty[as]);
+            first = false;
+            __syncwarp();
           }
-          first = false;
-          __syncwarp();
         }
         if (++as == p.a_stages) { as = 0; aph ^= 1; }
       }
@@ -295,13 +298,28 @@ long long tiles_of(const GemmArgs& g, int px) {
   return g.m / per * sh.tiles_y * sh.tiles_x * ((g.n + CG_M - 1) / CG_M);
 }
 
+// Blocks of 64 channels where two activation tiles and three weight planes of them fit the ring: a 128-byte row costs the copy engine
+// little more than a 64-byte one, and with 448 rows to a tap and 32 channels (3 x 3, four planes) those set the pace: a tile of 128 pixels
+// took 676 cycles for 384 of MMAs.  16 x 512 -> 512 on 16^2: 62.8 -> 53.0 us, with two products 52.2 -> 42.4; 3 x 256 -> 256 on 56^2, tiles
+// of 256 pixels: 45.2 -> 44.3.
+bool conv_wide_blocks(const GemmArgs& g, int px) {
+  const char* e = getenv("MIMIR_B200_CONV_BK");  // "32": never
+  if (g.conv_c % 64 != 0 || (e && atoi(e) == 32)) return false;
+  const ConvShape sh = conv_shape(g, px);
+  const int tw = 1 << sh.tw_log, rows = (px >> sh.tw_log) + g.conv_ks - 1;
+  return 2 * g.a_planes * tw * rows * 128 + 3 * CG_M * 128 <= CG_SMEM_MAX - CG_EPI - 2048;
+}
+
 // Estimated SM cycles of a launch and the tile it takes: within 5 % of 50 measured launches, K = 64 ... 4608.  Tiles of 128 pixels (half of
 // the accumulator's columns: the same sums in the same order, bit for bit) where 256 leave SMs without one: they load the weights whole, so
-// that one takes 0.77 of a tile's MMA time with three MMAs per product and 0.86 with two, and 2800 cycles less beside it.  16 x 512 -> 512 on
-// 16^2, 64 tiles: 78.1 -> 62.4 us; 4 x 128 -> 128 on 63^2, 64 tiles: 30.9 -> 25.4; 3 x 256 -> 256 on 56^2, 96 tiles: stays (45.3, 62.7 in 192).
+// that one takes 0.64 of a tile's MMA time with three MMAs per product and 0.68 with two (0.83 and 0.94 in blocks of 32 channels), and 2800
+// cycles less beside it.  16 x 512 -> 512 on 16^2, 64 tiles: 78.1 -> 53.0 us; 4 x 128 -> 128 on 63^2, 64 tiles: 30.9 -> 23.2; 8 x 64 -> 64
+// on 58^2, 128 tiles: stays (19.0, 22.4 in 256).
 double conv_cycles(const GemmArgs& g, int* px) {
   const int sms = ctx().sm_count, products = g.a_planes + g.w_planes - 1;
-  const double mma = 1.15 * g.k / 16.0 * products * 128.0, part = (products == 3 ? 0.77 : products == 2 ? 0.86 : 0.95) * mma;
+  const bool wide = conv_wide_blocks(g, CG_N / 2);
+  const double mma = 1.15 * g.k / 16.0 * products * 128.0;
+  const double part = (products == 3 ? (wide ? 0.64 : 0.83) : products == 2 ? (wide ? 0.68 : 0.94) : (wide ? 0.8 : 1.0)) * mma;
   const double whole = 17400.0 + static_cast<double>((tiles_of(g, CG_N) + sms - 1) / sms) * (mma > 4500.0 ? mma : 4500.0);
   const double half = 14600.0 + static_cast<double>((tiles_of(g, CG_N / 2) + sms - 1) / sms) * (part > 2800.0 ? part : 2800.0);
   const char* force = getenv("MIMIR_B200_CONV_PX");  // "128", "256": always
@@ -309,7 +327,7 @@ double conv_cycles(const GemmArgs& g, int* px) {
   return *px == CG_N ? whole : half;
 }
 
-template <int AP, int WP>
+template <int AP, int WP, int BK>
 int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   const int ks = g.conv_ks, pad = g.conv_pad;
   ConvGemmParams p;
@@ -317,19 +335,19 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   conv_cycles(g, &p.px);
   const ConvShape sh = conv_shape(g, p.px);
   const int hp = sh.h + 2 * pad, wp = sh.w + 2 * pad, tw = 1 << sh.tw_log, th = p.px >> sh.tw_log;
-  p.oc = g.n; p.h = sh.h; p.w = sh.w; p.ks = ks; p.cblocks = g.conv_c / CG_BK;
+  p.oc = g.n; p.h = sh.h; p.w = sh.w; p.ks = ks; p.cblocks = g.conv_c / BK;
   p.tw_log = sh.tw_log;
   p.tiles_x = sh.tiles_x; p.tiles_y = sh.tiles_y;
   p.tiles_o = (p.oc + CG_M - 1) / CG_M;
   p.num_tiles = p.batch * p.tiles_y * p.tiles_x * p.tiles_o;
   const int rows = th + ks - 1;
-  p.a_stage_bytes = AP * tw * rows * CG_BK * 2;
+  p.a_stage_bytes = AP * tw * rows * BK * 2;
   const int ring = CG_SMEM_MAX - CG_EPI - 1024 - 1024;  // (less the barriers)
   p.a_stages = 3;
-  p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (WP * CG_W_TILE);
-  if (p.w_stages < 3) {
+  p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (CG_M * BK * 2);
+  if (p.w_stages < 3 * WP) {
     p.a_stages = 2;
-    p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (WP * CG_W_TILE);
+    p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (CG_M * BK * 2);
   }
   if (p.w_stages > CG_MAX_RING) p.w_stages = CG_MAX_RING;
   p.residual = g.residual; p.res_up = g.residual != nullptr && g.residual_up ? 1 : 0; p.out = g.out_f32; p.activation = g.activation;
@@ -337,18 +355,18 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   p.err_word = ctx().dev_error_word;
   CUtensorMap map_a, map_w;
-  MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, CG_BK, tw, rows));
-  MB_TRY(make_plane_map(&map_w, g.w, WP, g.n, round_up(g.k, 64), CG_BK, CG_M));
-  const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * WP * CG_W_TILE + CG_EPI + 1024;
+  MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, BK, tw, rows));
+  MB_TRY(make_plane_map(&map_w, g.w, WP, g.n, round_up(g.k, 64), BK, CG_M));
+  const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * (CG_M * BK * 2) + CG_EPI + 1024;
   static PerDeviceOnce attr_once;
   MB_TRY(attr_once.run([&]() -> int {
-    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
+    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
     return MIMIR_B200_OK;
   }));
   const int sms = ctx().sm_count;
   GemmProfile prof(st);
   MB_TRY(prof.begin());
-  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p));
+  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP, BK>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p));
   MB_TRY(prof.end());
   count_launch();
   return MIMIR_B200_OK;
@@ -362,7 +380,7 @@ double conv_gemm_cycles(const GemmArgs& g) {
   constexpr double never = 1e30;
   const char* e = getenv("MIMIR_B200_CONV_SPATIAL");  // "0": never, "1": wherever the form allows
   if (e && e[0] == '0') return never;
-  if (g.conv_ks < 1 || g.conv_ks > 7 || g.conv_c % CG_BK != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
+  if (g.conv_ks < 1 || g.conv_ks > 7 || g.conv_c % 32 != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
     return never;
   if (!(g.a_planes == 2 || g.w_planes == 1)) return never;
   if (e && e[0] == '1') return 0.0;
@@ -374,9 +392,12 @@ double conv_gemm_cycles(const GemmArgs& g) {
 }
 
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {
-  if (g.a_planes == 2 && g.w_planes == 2) return launch_conv_t<2, 2>(g, st);
-  if (g.a_planes == 2 && g.w_planes == 1) return launch_conv_t<2, 1>(g, st);
-  if (g.a_planes == 1 && g.w_planes == 1) return launch_conv_t<1, 1>(g, st);
+  int px;
+  conv_cycles(g, &px);
+  const bool wide = conv_wide_blocks(g, px);
+  if (g.a_planes == 2 && g.w_planes == 2) return wide ? launch_conv_t<2, 2, 64>(g, st) : launch_conv_t<2, 2, 32>(g, st);
+  if (g.a_planes == 2 && g.w_planes == 1) return wide ? launch_conv_t<2, 1, 64>(g, st) : launch_conv_t<2, 1, 32>(g, st);
+  if (g.a_planes == 1 && g.w_planes == 1) return wide ? launch_conv_t<1, 1, 64>(g, st) : launch_conv_t<1, 1, 32>(g, st);
   return fail(MIMIR_B200_E_INVALID, "conv: %d activation and %d weight planes", g.a_planes, g.w_planes);
 }
 
