@@ -828,6 +828,13 @@ int env_int(const char* name, int dflt) {
   return (v && *v) ? atoi(v) : dflt;
 }
 
+// Do the tiles of this launch run in CTA pairs (in the forms that can: see launch_gemm_t)?
+bool takes_pairs(const GemmArgs& g) {
+  static const int pair_env = env_int("MIMIR_B200_GEMM_PAIR", -1);
+  const long long tiles_m = (g.m + BM - 1) / BM, tiles = tiles_m * ((g.n + BN - 1) / BN);
+  return tiles_m >= 2 && g.a_group_rows <= 0 && (pair_env == 1 || (pair_env != 0 && g.a_planes + g.w_planes >= 3 && tiles >= ctx().sm_count));
+}
+
 template <int BK>
 int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
   const int kp = round_up(g.k, 64);
@@ -869,10 +876,7 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
   // step 18.51 -> 18.2 ms).  The one-MMA mode (14.78 -> 14.88 ms) and launches of a few tiles (the registry
   // transformer's 1024-row layers: 0.290 -> 0.295 ms per step) are better off alone.  MIMIR_B200_GEMM_PAIR=0 turns pairs
   // off, =1 takes them wherever the form allows.
-  static const int pair_env = env_int("MIMIR_B200_GEMM_PAIR", -1);
-  const bool pair_can = !swap && !tma_store && p.bn == BN && p.tiles_m >= 2 && g.a_group_rows <= 0;
-  const long long tiles_all = static_cast<long long>(p.tiles_m) * ((g.n + BN - 1) / BN);
-  const bool pair = pair_can && (pair_env == 1 || (pair_env != 0 && g.a_planes + g.w_planes >= 3 && tiles_all >= ctx().sm_count));
+  const bool pair = !swap && !tma_store && p.bn == BN && takes_pairs(g);
   if (g.a_group_rows > 0 && (swap || conv || g.out_nchw_hw > 0 || g.a_group_rows % BM != 0 || g.w_group_rows <= 0 ||
                              g.w_rows_total < static_cast<long long>((g.m + g.a_group_rows - 1) / g.a_group_rows - 1) * g.w_group_rows + g.n))
     return fail(MIMIR_B200_E_INVALID, "gemm: bad grouped-form arguments");
@@ -1134,13 +1138,15 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
   if (g.residual && !g.out_f32) return fail(MIMIR_B200_E_INVALID, "gemm: residual needs the fp32 output stride");
   // K block per stage.  With at most three planes in play (one of the operands single-plane) a 64-wide block still leaves
   // three 64 KB stages, halves the barrier round trips per MMA and uses 128-byte swizzle rows: measured on the decoder's
-  // K = 768 layers 0.77 -> 0.90 of the sustained cuBLAS rate.  With four planes (both operands split) 64-wide blocks would
-  // leave two 96 KB stages, which measured slower than four 48 KB stages of 32.
+  // K = 768 layers 0.77 -> 0.90 of the sustained cuBLAS rate.  With four planes (both operands split) 64-wide blocks leave a CTA on its
+  // own two 96 KB stages, which measured slower than four 48 KB stages of 32, but a CTA of a pair three of 64 KB: the copy engine takes
+  // half as many rows, 4096 x 4096 x 4096 three times 962 -> 939 us, 20000 x 1100 twice 355 -> 333, a 15 x 721 decoder 5.89 -> 5.78 ms.
   if (g.conv_ks > 0) {
     if (g.conv_c <= 0 || g.conv_c % 32 != 0 || g.k != g.conv_ks * g.conv_ks * g.conv_c || g.out_split || !g.out_f32)
       return fail(MIMIR_B200_E_INVALID, "gemm: bad shifted-convolution arguments");
   }
-  const int bk = env_int("MIMIR_B200_GEMM_BK", (g.a_planes + g.w_planes <= 3) ? 64 : 32);
+  const bool pairs = g.conv_ks == 0 && g.out_nchw_hw <= 0 && takes_pairs(g);
+  const int bk = env_int("MIMIR_B200_GEMM_BK", (g.a_planes + g.w_planes <= 3 || pairs) ? 64 : 32);
   // Three forms: 128 x 256 tiles here, narrow tiles with split K (only where the big tiles fill the GPU less than one and a half times:
   // beyond that re-reading the operands costs more than an even last wave gives), and for convolutions tiles of 256 pixels.
   const int sbk = (g.conv_ks == 0 || g.conv_c % 64 == 0) ? 64 : 32;
