@@ -446,14 +446,14 @@ __global__ void __launch_bounds__(SG_THREADS, 2) split_footprint_kernel() {}
 // eight 35.1, as more SMs have weights on the way)
 constexpr int SG_SPLITS[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
 
-// Clusters of SG_SPLITS[i] CTAs that run at the same time, one or two CTAs to an SM.  A cluster lives in one GPC, whose SM count is no
+// n[two][i]: clusters of SG_SPLITS[i] CTAs that run at the same time, one or two CTAs to an SM.  A cluster lives in one GPC, whose SM count is no
 // multiple of it: of the 148 SMs clusters of four use 132, of eight 120, of sixteen 112 (128 CTAs in clusters of eight: 12.9 us, two
 // rounds, where 64 in clusters of four take 8.0).
-int active_clusters(int i, bool two) {
-  struct Table { int n[2][sizeof(SG_SPLITS) / sizeof(int)]; };
+struct ClusterTable { int n[2][sizeof(SG_SPLITS) / sizeof(int)]; };
+const ClusterTable* active_clusters() {
   static PerDeviceOnce once;
-  static Table table[64];  // (PerDeviceOnce counts as many devices)
-  Table& t = table[ctx().device];
+  static ClusterTable table[64];  // (PerDeviceOnce counts as many devices)
+  ClusterTable& t = table[ctx().device];
   const int rc = once.run([&]() -> int {
     MB_CUDA(cudaFuncSetAttribute(split_footprint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_RING_LIMIT + 4096));
     MB_CUDA(cudaFuncSetAttribute(split_footprint_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -476,7 +476,7 @@ int active_clusters(int i, bool two) {
       }
     return MIMIR_B200_OK;
   });
-  return rc == MIMIR_B200_OK ? t.n[two ? 1 : 0][i] : 0;
+  return rc == MIMIR_B200_OK ? &t : nullptr;
 }
 
 // Tile width and split count of one launch and its estimated time in SM cycles.
@@ -488,6 +488,8 @@ SplitPlan plan_split(const GemmArgs& g, int bk, int kblocks) {
   const bool cm = g.conv_ks > 0 || g.out_nchw_hw > 0;
   auto mma = [](int n) { return n > 92 ? n * 0.5 : 46.0; };  // an instruction of 128 x n x 16
   SplitPlan best;
+  const ClusterTable* clusters = active_clusters();
+  if (clusters == nullptr) return best;
   static const int widths[] = {16, 32, 48, 64, 96, 128};
   for (int bn : widths) {
     if (bn > 16 && bn >= g.m + 32) break;
@@ -499,7 +501,7 @@ SplitPlan plan_split(const GemmArgs& g, int bk, int kblocks) {
       const long long ctas = tiles * splits;
       // CTAs that share an SM overlap one's loads and stores with the other's MMAs: whole rounds of two per SM
       const bool two = ctas > sms && 2 * stage <= SG_RING_TWO && (bn + splits - 1) * (SG_M + 1) * 4 <= SG_RING_TWO;
-      const int active = active_clusters(i, two);
+      const int active = clusters->n[two ? 1 : 0][i];
       if (active <= 0) continue;
       const long long rounds = (tiles + active - 1) / active;
       const double busy = static_cast<double>(ctas < sms ? ctas : sms) / sms;
