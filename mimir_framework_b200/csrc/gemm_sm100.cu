@@ -1125,9 +1125,22 @@ double big_tile_cycles(const GemmArgs& g) {
   }
   const long long tiles = static_cast<long long>((g.m + BM - 1) / BM) * ((g.n + BN - 1) / BN);
   const long long waves = (tiles + ctx().sm_count - 1) / ctx().sm_count;
-  // (one tile to an SM starts cold: 1.15 to 1.3 times the estimate in 12 shapes; two waves, 1440 x 3784 x 3784, are as estimated)
-  const double tile = (waves == 1 ? 1.25 : 1.0) * (mma > load ? mma : load);
-  return 15100.0 + waves * (tile > 12000.0 ? tile : 12000.0);  // (a tile's epilogue takes about 12 000 cycles beside the next main loop)
+  const double tile = mma > load ? mma : load;
+  const double even = 15100.0 + waves * (tile > 12000.0 ? tile : 12000.0);  // (a tile's epilogue takes about 12 000 cycles beside the next main loop)
+  // One tile to an SM starts cold: 1.25 tiles where the loop is short, and a long one has that behind it (measured, three MMAs per product,
+  // 128 tiles, K = 1024 / 2048 / 4096: 26.4 / 42.5 / 77 us; this gives 26.5 / 42.4 / 74; 1.25 tiles for any K would give 85, which narrow
+  // tiles beat on paper and miss by 15 % live).  Last waves in halves (launch_gemm_t): 1536 x 4096 x 4096 takes 110 us, here 106.
+  if (waves == 1) {
+    const double brief = 15100.0 + (1.25 * tile > 12000.0 ? 1.25 * tile : 12000.0), lengthy = 21000.0 + 1.02 * tile;
+    return brief < lengthy ? brief : lengthy;
+  }
+  const bool pair = takes_pairs(g);
+  const long long units = pair ? static_cast<long long>((g.m + 2 * BM - 1) / (2 * BM)) * ((g.n + BN - 1) / BN) : tiles;
+  const int workers = pair ? ctx().sm_count / 2 : ctx().sm_count;
+  const long long rest = units % workers;
+  if (g.a_planes + g.w_planes < 3 || rest == 0 || 2 * rest > workers) return even;
+  const double cut = 21000.0 + (static_cast<double>(units / workers) + (products == 3 ? 0.53 : 0.67)) * tile;
+  return cut < even ? cut : even;
 }
 }  // namespace
 

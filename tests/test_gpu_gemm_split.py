@@ -43,6 +43,29 @@ def test_linear_against_float64(rt, monkeypatch, precision, form, m, n, k):
     assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W])
+@pytest.mark.parametrize("m,n,k", [(257, 6000, 2100), (1025, 4100, 2100), (1409, 2700, 2500), (1537, 2304, 1100), (100, 38000, 520)])
+def test_around_one_wave_of_big_tiles(rt, precision, m, n, k):
+    """72, 153, 132, 117 and 149 tiles of 128 x 256, where narrow tiles give way to big ones (cut in two in the last wave, in pairs and alone)."""
+    r = np.random.default_rng(m + n)
+    x = r.standard_normal((m, k)).astype(np.float32)
+    w = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)
+    if precision != abi.PREC_BF16X2:
+        w = (w.view(np.uint32) & 0xffff0000).view(np.float32)
+    b = r.standard_normal(n).astype(np.float32)
+    mod = rt.GraphModel([make_desc("l", "Linear", in_features=k, out_features=n, seq_len=m, use_bias=1, params_count=n * k + n)], precision)
+    mod.upload_weights(0, np.concatenate([w.ravel(), b]))
+    mod.plan({"x": (m * k, False)}, 1)
+    got = mod.forward({"x": (x.ravel(), False)}, 1, m * n).reshape(m, n)
+    mod.close()
+    rows = np.unique(np.concatenate([np.arange(0, m, 37), np.arange(m - 5, m)]))
+    want = x[rows].astype(np.float64) @ w.astype(np.float64).T + b
+    assert np.all(np.isfinite(got)) and np.linalg.norm(got[rows] - want) <= 1e-5 * np.linalg.norm(want)
+    cols = np.unique(np.concatenate([np.arange(0, n, 61), np.arange(n - 5, n)]))
+    want = x.astype(np.float64) @ w[cols].astype(np.float64).T + b[cols]
+    assert np.linalg.norm(got[:, cols] - want) <= 1e-5 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("form", ["16,1", "48,2", "48,5", "128,8", ""])
 @pytest.mark.parametrize("batch,ic,oc,h,w,k,stride,pad", [(1, 64, 130, 9, 7, 3, 1, 1), (3, 32, 40, 5, 11, 1, 1, 0), (2, 96, 16, 8, 8, 5, 1, 2), (2, 3, 70, 17, 19, 7, 2, 3)])
 def test_convolution_against_the_port(rt, monkeypatch, form, batch, ic, oc, h, w, k, stride, pad):
