@@ -531,7 +531,10 @@ void split_weights(SplitGemmParams& p, long long ksteps, int steps_per_block, in
     const double after = p.splits > 1 ? 3.1e-8 * products * static_cast<double>(ksteps - at(s + 1)) : 0.0;
     p.weight[s] = static_cast<float>(1.0 - after - 1.5e-8 * (products - 1) * static_cast<double>(at(s + 1) - at(s)));
   }
-  if (p.splits == 1) p.acc_scale *= p.weight[0];
+  if (p.splits == 1) {  // (a factor of the result: row-major tiles then leave tensor memory without another multiplication)
+    p.acc_scale *= p.weight[0];
+    p.weight[0] = 1.0f;
+  }
 }
 
 template <int BK, int AP, int WP>

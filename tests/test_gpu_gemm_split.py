@@ -104,3 +104,39 @@ def test_chain_through_operand_planes(rt, monkeypatch, form, m, k, n):
     want = a @ w[1].astype(np.float64).T + b[1]
     # two contractions of at most 255 products, a few 1e-6 each (operand planes and accumulation)
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W])
+@pytest.mark.parametrize("form", ["64,1", "128,1", "32,3"])
+@pytest.mark.parametrize("ic,stride", [(512, 1), (512, 2), (1024, 1), (1024, 0)])
+def test_mean_loss_of_the_sums_is_put_back_once(rt, monkeypatch, precision, form, ic, stride):
+    """The tensor core's truncating adds make every sum a little too small, by a share that K fixes; the kernel puts the mean of it back, in
+    channel-major results (3 x 3 convolutions, stride 2 over im2col rows) and row-major ones (stride 0 here: a Linear) alike."""
+    monkeypatch.setenv("MIMIR_B200_GEMM_SPLIT", form)
+    r = np.random.default_rng(ic + stride)
+    oc, k = 130, 9 * ic
+    w = (r.standard_normal((oc, k)) / np.sqrt(k)).astype(np.float32)
+    if precision != abi.PREC_BF16X2:
+        w = (w.view(np.uint32) & 0xffff0000).view(np.float32)
+    if stride:
+        h = 9 if stride == 1 else 18
+        x = r.standard_normal((2, ic, h, h)).astype(np.float32)
+        desc = make_desc("c", "Conv2d", in_channels=ic, out_channels=oc, input_height=h, input_width=h, kernel=3, stride=stride, padding=1, params_count=w.size)
+        taps = np.lib.stride_tricks.sliding_window_view(np.pad(x, ((0, 0), (0, 0), (1, 1), (1, 1))), (3, 3), (2, 3))[:, :, ::stride, ::stride]
+        rows = taps.transpose(0, 2, 3, 1, 4, 5).reshape(2, -1, k)
+        want = (rows.astype(np.float64) @ w.T.astype(np.float64)).transpose(0, 2, 1)
+        batch = 2
+    else:
+        x = r.standard_normal((162, k)).astype(np.float32)
+        desc = make_desc("l", "Linear", in_features=k, out_features=oc, seq_len=162, use_bias=0, params_count=w.size)
+        want = (x.astype(np.float64) @ w.T.astype(np.float64))[None]
+        batch = 1
+    mod = rt.GraphModel([desc], precision)
+    mod.upload_weights(0, w.ravel())
+    mod.plan({"x": (x.size // batch, False)}, batch)
+    got = mod.forward({"x": (x.reshape(batch, -1), False)}, batch, want[0].size).reshape(want.shape)
+    mod.close()
+    # Normal operands lose 1.5e-8 of the sum per instruction, measured to within 1e-9 at every K; a correction that is missing, or there
+    # twice, is 1.5e-8 x one or two of the products per 16 of K.
+    products = 3 if precision == abi.PREC_BF16X2 else 2
+    assert abs(np.vdot(got - want, want) / np.vdot(want, want)) <= 2e-9 * products * k / 16
