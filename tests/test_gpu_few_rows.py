@@ -132,3 +132,42 @@ def test_exact_bfloat16_weights_against_float64(rt, norm, m, n, k):
             y = x[:1] @ w.T + b
             want = y / (1 + np.exp(-y))
         assert np.array_equal(np.isnan(again[0]), np.isnan(want[0])) and np.array_equal(np.isposinf(again[0]), np.isposinf(want[0]))
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_BF16W, abi.PREC_BF16X2])
+@pytest.mark.parametrize("what", ["beta", "-gamma", "overflow"])
+@pytest.mark.parametrize("m,n,k", [(3, 33, 128), (9, 31, 1032), (16, 65, 4096), (5, 4737, 768), (16, 4752, 1024), (7, 100, 264)])
+def test_infinities_that_a_layernorm_makes(rt, precision, what, m, n, k):
+    """An infinite beta or gamma, and a gamma that takes a finite row past fp32: the Linear behind that LayerNorm has infinities where the
+    weight is not zero and NaN where it is, with exact bfloat16 weights as with fp32 ones."""
+    r = np.random.default_rng(m * 31 + n)
+    x = (r.standard_normal((m, k)) + 1).astype(np.float32)
+    w = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)
+    b = r.standard_normal(n).astype(np.float32)
+    if precision == abi.PREC_BF16W:
+        w = (w.view(np.uint32) & 0xffff0000).view(np.float32)
+    at = k - 5
+    w[1::3, at] = 0.0
+    g, be = (1 + 0.1 * r.standard_normal(k)).astype(np.float32), r.standard_normal(k).astype(np.float32)
+    if what == "beta":
+        be[at] = np.inf
+    elif what == "-gamma":
+        g[at] = -np.inf
+    else:
+        g[at] = 3e38
+        x[:, at] = 1 + 4 * (-1.0) ** np.arange(m)  # about four deviations off either way
+    descs = [make_desc("n", "LayerNorm", inputs=["x"], output="h", in_features=k, affine=1, use_bias=1, eps=1e-5, params_count=2 * k),
+             make_desc("l", "Linear", inputs=["h"], output="x", in_features=k, out_features=n, seq_len=1, use_bias=1, params_count=n * k + n)]
+    mod = rt.GraphModel(descs, precision)
+    mod.upload_weights(0, np.concatenate([g, be]))
+    mod.upload_weights(1, np.concatenate([w.ravel(), b]))
+    mod.plan({"x": (k, False)}, m)
+    mod.decode_begin({"x": (k, False)}, m, 2)
+    got = mod.decode_step({"x": (x, False)}, m, 0, n).reshape(m, n)
+    mod.close()
+    with np.errstate(invalid="ignore", over="ignore"):
+        h = x.astype(np.float64)
+        h = ((h - h.mean(1, keepdims=True)) / np.sqrt(h.var(1, keepdims=True) + 1e-5) * g + be).astype(np.float32)
+        want = h[:, at:at + 1] * w[:, at]
+    assert np.all(np.isinf(h[:, at])) and np.isnan(want).any() and np.isinf(want).any()
+    assert np.array_equal(got, want, equal_nan=True)
