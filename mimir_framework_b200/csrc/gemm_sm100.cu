@@ -828,11 +828,53 @@ int env_int(const char* name, int dflt) {
   return (v && *v) ? atoi(v) : dflt;
 }
 
-// Do the tiles of this launch run in CTA pairs (in the forms that can: see launch_gemm_t)?
+// The form of a launch, the same for its choice (big_tile_cycles, the K block in launch_gemm) and for the launch itself.
+
+// narrow channel-major layers run with the operands swapped (see GemmParams::swap); short K keeps the usual
+// form, whose epilogue writes NCHW with coalesced stores
+bool swaps_operands(const GemmArgs& g) {
+  const char* noswap = getenv("MIMIR_B200_GEMM_NOSWAP");
+  const int k = g.conv_ks > 0 ? g.conv_ks * g.conv_ks * g.conv_c : round_up(g.k, 64);
+  return (g.conv_ks > 0 || g.out_nchw_hw > 0) && g.n <= BM && g.bias == nullptr && g.out_split == nullptr && g.out_f32 != nullptr &&
+         g.m >= 4 * BN && k >= 256 && !(noswap && noswap[0] == '1');
+}
+
+// Optional (MIMIR_B200_GEMM_TMA_STORE=1): row-major fp32 outputs leave through TMA stores.  Measured neutral on the
+// decoder's K = 768 layers (1 078 vs 1 100 TFLOP/s issued): what slows those layers is not the shape of the stores but
+// their bytes - the operand loads alone run at ~62 B per cycle and SM, next to what an SM can take from L2, and the
+// same kernel without any output store reaches 1 315.
+bool stores_by_tma(const GemmArgs& g) {
+  static const bool on = [] { const char* e = getenv("MIMIR_B200_GEMM_TMA_STORE"); return e && e[0] == '1'; }();
+  return on && g.conv_ks <= 0 && g.out_nchw_hw <= 0 && g.out_f32 != nullptr && g.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(g.out_f32) & 15) == 0;
+}
+
+// MIMIR_B200_GEMM_BN=192: 192-column tiles.  On paper they shorten launches whose last wave is mostly empty (N = 768
+// over 256 row tiles: 7 waves of 192 columns instead of 6 of 256, 12.5 % less work per SM); measured, the
+// 32768 x 768 x 768 projection takes 0.076 ms either way and the K = 3072 one 0.243 against 0.251: an N = 192
+// instruction costs the tensor pipe about what an N = 256 one does.  Kept as a switch, off by default.
+int tile_columns(const GemmArgs& g) {
+  static const int force = env_int("MIMIR_B200_GEMM_BN", 0);
+  return force == 192 && g.conv_ks <= 0 && !swaps_operands(g) && !stores_by_tma(g) ? 192 : BN;
+}
+
+// CTA pairs: every form but the swapped one, full-width tiles.  Taken by default where they were measured to pay: launches of at least one
+// full wave of tiles in the modes with two or three MMAs per product (same-run A/B: the K = N = 4096 layer 14.9-15.0
+// -> 14.5 ms per three-layer step = 0.333 of the sustained peak, the whole ceiling of the three-MMA scheme; the decoder
+// step 18.51 -> 18.2 ms).  The one-MMA mode (14.78 -> 14.88 ms) and launches of a few tiles (the registry
+// transformer's 1024-row layers: 0.290 -> 0.295 ms per step) are better off alone.  MIMIR_B200_GEMM_PAIR=0 turns pairs
+// off, =1 takes them wherever the form allows.
 bool takes_pairs(const GemmArgs& g) {
   static const int pair_env = env_int("MIMIR_B200_GEMM_PAIR", -1);
   const long long tiles_m = (g.m + BM - 1) / BM, tiles = tiles_m * ((g.n + BN - 1) / BN);
-  return tiles_m >= 2 && g.a_group_rows <= 0 && (pair_env == 1 || (pair_env != 0 && g.a_planes + g.w_planes >= 3 && tiles >= ctx().sm_count));
+  return !swaps_operands(g) && !stores_by_tma(g) && tile_columns(g) == BN && tiles_m >= 2 && g.a_group_rows <= 0 &&
+         (pair_env == 1 || (pair_env != 0 && g.a_planes + g.w_planes >= 3 && tiles >= ctx().sm_count));
+}
+
+// The last wave's tiles as halves where it has at most half as many tiles as there are CTAs (pairs): the same sums in the same order, bit
+// for bit.  A half takes 0.53 of a tile with three MMAs per product, 0.67 with two (the activations are loaded whole).
+bool halves_last_wave(const GemmArgs& g) {
+  static const bool on = env_int("MIMIR_B200_GEMM_HALVES", 1) != 0;
+  return on && g.conv_ks <= 0 && g.out_nchw_hw <= 0 && !stores_by_tma(g) && tile_columns(g) == BN && g.a_group_rows <= 0 && g.a_planes + g.w_planes >= 3;
 }
 
 template <int BK>
@@ -841,42 +883,17 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
   const bool conv = g.conv_ks > 0;
   CUtensorMap map_a, map_w;
   // conv: A rows are `conv_c` channels long and K = taps * conv_c runs over (tap, channel)
-  // narrow channel-major layers run with the operands swapped (see GemmParams::swap); short K keeps the usual
-  // form, whose epilogue writes NCHW with coalesced stores
-  const char* noswap = getenv("MIMIR_B200_GEMM_NOSWAP");
-  const int kblocks_all = conv ? g.conv_ks * g.conv_ks * (g.conv_c / BK) : kp / BK;
-  const bool swap = (conv || g.out_nchw_hw > 0) && g.n <= BM && g.bias == nullptr && g.out_split == nullptr && g.out_f32 != nullptr &&
-                    g.m >= 4 * BN && kblocks_all * BK >= 256 && !(noswap && noswap[0] == '1');
+  const bool swap = swaps_operands(g);
   MB_TRY(make_plane_map(&map_a, g.a, g.a_planes, g.m, conv ? g.conv_c : kp, BK, swap ? BN : BM));
-  // Optional (MIMIR_B200_GEMM_TMA_STORE=1): row-major fp32 outputs leave through TMA stores.  Measured neutral on the
-  // decoder's K = 768 layers (1 078 vs 1 100 TFLOP/s issued): what slows those layers is not the shape of the stores but
-  // their bytes - the operand loads alone run at ~62 B per cycle and SM, next to what an SM can take from L2, and the
-  // same kernel without any output store reaches 1 315.
-  static const bool use_tma_store = [] { const char* e = getenv("MIMIR_B200_GEMM_TMA_STORE"); return e && e[0] == '1'; }();
-  const bool tma_store = use_tma_store && !swap && !conv && g.out_nchw_hw <= 0 && g.out_f32 != nullptr && g.ldo % 4 == 0 &&
-                         (reinterpret_cast<uintptr_t>(g.out_f32) & 15) == 0;
+  const bool tma_store = stores_by_tma(g);
   CUtensorMap map_o = map_a;  // (a valid map when unused)
   if (tma_store) MB_TRY(make_out_map(&map_o, g.out_f32, g.m, g.n, g.ldo));
   GemmParams p;
   p.tma_store = tma_store ? 1 : 0;
   p.swap = swap ? 1 : 0;
   p.tiles_m = swap ? (g.n + BM - 1) / BM : (g.m + BM - 1) / BM;
-  p.bn = BN;
-  if (!swap && !conv && !tma_store) {
-    // MIMIR_B200_GEMM_BN=192: 192-column tiles.  On paper they shorten launches whose last wave is mostly empty (N = 768
-    // over 256 row tiles: 7 waves of 192 columns instead of 6 of 256, 12.5 % less work per SM); measured, the
-    // 32768 x 768 x 768 projection takes 0.076 ms either way and the K = 3072 one 0.243 against 0.251: an N = 192
-    // instruction costs the tensor pipe about what an N = 256 one does.  Kept as a switch, off by default.
-    static const int force = env_int("MIMIR_B200_GEMM_BN", 0);
-    if (force == 192) p.bn = 192;
-  }
-  // CTA pairs: every form but the swapped one, full-width tiles.  Taken by default where they were measured to pay: launches of at least one
-  // full wave of tiles in the modes with two or three MMAs per product (same-run A/B: the K = N = 4096 layer 14.9-15.0
-  // -> 14.5 ms per three-layer step = 0.333 of the sustained peak, the whole ceiling of the three-MMA scheme; the decoder
-  // step 18.51 -> 18.2 ms).  The one-MMA mode (14.78 -> 14.88 ms) and launches of a few tiles (the registry
-  // transformer's 1024-row layers: 0.290 -> 0.295 ms per step) are better off alone.  MIMIR_B200_GEMM_PAIR=0 turns pairs
-  // off, =1 takes them wherever the form allows.
-  const bool pair = !swap && !tma_store && p.bn == BN && takes_pairs(g);
+  p.bn = tile_columns(g);
+  const bool pair = takes_pairs(g);
   if (g.a_group_rows > 0 && (swap || conv || g.out_nchw_hw > 0 || g.a_group_rows % BM != 0 || g.w_group_rows <= 0 ||
                              g.w_rows_total < static_cast<long long>((g.m + g.a_group_rows - 1) / g.a_group_rows - 1) * g.w_group_rows + g.n))
     return fail(MIMIR_B200_E_INVALID, "gemm: bad grouped-form arguments");
@@ -953,12 +970,9 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
     const int pairs = ctx().sm_count / 2;
     grid = 2 * (tiles < pairs ? tiles : pairs);
   }
-  // The last wave's tiles as halves where it has at most half as many tiles as there are CTAs (pairs): the same sums in the same order, bit
-  // for bit.  A half takes 0.53 of a tile with three MMAs per product, 0.67 with two (the activations are loaded whole).
   p.full_tiles = INT_MAX;
   const int workers = pair ? ctx().sm_count / 2 : ctx().sm_count, rest = tiles % workers;
-  static const bool halves = env_int("MIMIR_B200_GEMM_HALVES", 1) != 0;
-  if (halves && !cm && !tma_store && p.bn == BN && g.a_group_rows <= 0 && g.a_planes + g.w_planes >= 3 && rest > 0 && 2 * rest <= workers) {
+  if (halves_last_wave(g) && rest > 0 && 2 * rest <= workers) {
     p.full_tiles = tiles - rest;
     MB_TRY(make_plane_map(&map_o, g.w, g.w_planes, g.n, kp, BK, pair ? BN / 4 : BN / 2));
     if (tiles < workers) grid = (pair ? 2 : 1) * 2 * rest;
@@ -1138,7 +1152,7 @@ double big_tile_cycles(const GemmArgs& g) {
   const long long units = pair ? static_cast<long long>((g.m + 2 * BM - 1) / (2 * BM)) * ((g.n + BN - 1) / BN) : tiles;
   const int workers = pair ? ctx().sm_count / 2 : ctx().sm_count;
   const long long rest = units % workers;
-  if (g.a_planes + g.w_planes < 3 || rest == 0 || 2 * rest > workers) return even;
+  if (!halves_last_wave(g) || rest == 0 || 2 * rest > workers) return even;
   const double cut = 21000.0 + (static_cast<double>(units / workers) + (products == 3 ? 0.53 : 0.67)) * tile;
   return cut < even ? cut : even;
 }
