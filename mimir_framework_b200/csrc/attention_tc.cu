@@ -59,6 +59,7 @@ struct AttnParams {
   int v_mn_major;      // ... and so do the V tiles, as [key][d] rows read by the MMA as an MN-major B operand
   int f16;             // operand planes hold IEEE half instead of bfloat16
   int splits;          // CTAs (a cluster) that share a query tile's keys in the second kernel form
+  int early;           // pdl_small_grid() of the second kernel form's launch
   int head_chunk;      // (sample, head) pairs per scheduling chunk of the second kernel form
   float acc_comp;      // relative loss of the truncating fp32 accumulation per MMA (0 = no compensation)
   int* err_word;
@@ -548,7 +549,7 @@ flash_attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  pdl_early_if_small();
+  pdl_early_if(p.early);
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_o = tmem_base + 3 * AT_BK;  // score / probability tile b lives at tmem_base + b * 64
 
@@ -988,6 +989,7 @@ int launch_attention_core_tc(const float* qkv, float* out, int batch, int seq, i
   dim3 grid((seq + AT_BQ - 1) / AT_BQ, bh);
   p.head_chunk = 1;
   p.splits = 1;
+  p.early = 0;
   if (v2) {
     // heads whose K and V planes (seq x 64 x 2 planes x 2 bytes, twice) fill about 48 MB of L2
     const long long per_head = static_cast<long long>(seq) * AT_HD * 2 * 2 * 2;
@@ -1003,6 +1005,7 @@ int launch_attention_core_tc(const float* qkv, float* out, int batch, int seq, i
     const int max_tiles = (seq + AT_BK - 1) / AT_BK, fit = 2 * ctx().sm_count / static_cast<int>(grid.x);
     p.splits = fit >= 4 && max_tiles >= 8 ? 4 : fit >= 2 && max_tiles >= 4 ? 2 : 1;
     grid.x *= static_cast<unsigned>(p.splits);
+    p.early = pdl_small_grid(grid.x) ? 1 : 0;
     MB_TRY(launch_pdl(flash_attn_tc2_kernel, grid, dim3(A2_THREADS), A2_SMEM, st, p.splits, mq, mk, mv, p));
     count_launch(1);
     return MIMIR_B200_OK;

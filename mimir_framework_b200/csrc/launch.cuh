@@ -28,9 +28,10 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // 269.7 -> 264.5 us.  (Not the convolutions' chain of layout passes, sweeps and tiles: with it and dependency waits throughout the
 // UNet of 3 samples took 613 -> 686 us, the conv stack 7.17 -> 7.38 ms.  Nor with a kernel's set-up moved ahead of its wait: attention
 // of 8 samples x 128 tokens lost 2 us a launch.)
-constexpr unsigned PDL_SMALL_GRID = 296;  // two CTAs per SM
-__device__ __forceinline__ void pdl_early_if_small() {
-  if (gridDim.x * gridDim.y * gridDim.z <= PDL_SMALL_GRID) pdl_launch_dependents();
+// `early` is pdl_small_grid() of the launch: at most two CTAs per SM, which both kernels have room for (their launch bounds and shared memory).
+inline bool pdl_small_grid(unsigned ctas) { return ctas <= 2u * static_cast<unsigned>(ctx().sm_count); }
+__device__ __forceinline__ void pdl_early_if(int early) {
+  if (early) pdl_launch_dependents();
 }
 
 template <class... P, class... A>

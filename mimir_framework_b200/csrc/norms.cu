@@ -330,6 +330,7 @@ struct RmsOnePass {
   unsigned* row_done;       // per row: CTAs that have read everything they need
   int rows;
   int stage_gamma;          // gamma goes through shared memory as well (launches of few CTAs)
+  int early;                // pdl_small_grid() of the launch
   unsigned long long* sum_slots;
   unsigned long long* err_slots;
   long long len;
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 6 : 2) rms_onepass_kernel(const 
     if (p.gamma != nullptr && o + tid * 32 < p.n_gamma) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gamma + o + tid * 32));
   };
   if (p.rows == 1) prefetch_gamma(static_cast<long long>(blockIdx.x) * CHUNK);
-  pdl_early_if_small();
+  pdl_early_if(p.early);
   pdl_wait();
   // Counters and slots hold nothing of use after a wait gave up, until the host clears them: the launches in between write nothing and
   // report it again (the host may have read the word already).  (One row needs no order among its CTAs, which are resident
@@ -1239,6 +1240,7 @@ int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y
     p.len = n; p.chunks = chunks; p.eps = eps; p.err_word = ctx().dev_error_word;
     // up to three CTAs per SM have room for gamma's chunk beside their own; a larger launch keeps six per SM and finds gamma in L2
     p.stage_gamma = slots <= static_cast<size_t>(3) * ctx().sm_count ? 1 : 0;
+    p.early = pdl_small_grid(static_cast<unsigned>(slots)) ? 1 : 0;
     static PerDeviceOnce attr_once;
     MB_TRY(attr_once.run([&]() -> int {
       MB_CUDA(cudaFuncSetAttribute(rms_onepass_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CHUNK * sizeof(float)));
