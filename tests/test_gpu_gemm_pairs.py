@@ -92,3 +92,46 @@ def test_tiles_cut_in_two_keep_their_bits(precision, whole, cut, n, k):
     want = want * 0.5 * (1 + np.tanh(0.7978845608 * (want + 0.044715 * want ** 3)))
     big = got[0] if whole > cut else got[1]
     assert np.linalg.norm(big[-40:] - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("precision", ["x2", "w"])
+@pytest.mark.parametrize("what", ["residual", "planes"])
+@pytest.mark.parametrize("whole,cut,n,k", [(9472, 9600, 1024, 256), (12800, 8192, 256, 616), (9472, 9500, 1000, 1032)])
+def test_cut_tiles_of_every_epilogue_keep_their_bits(precision, what, whole, cut, n, k):
+    """As above, for tiles that add a residual and tiles that write the next layer's operand planes (whose own tiles are cut as well)."""
+    import numpy as np
+    from mimir_framework_b200 import abi, configs, runtime as rt
+
+    rt.init(0)
+    r = np.random.default_rng(n + k)
+    weights = [(r.standard_normal(o * i + o) * 0.05).astype(np.float32) for i, o in ((k, n), (n, n))]
+    if precision == "w":
+        weights = [configs.round_to_bf16(w) for w in weights]
+    x, res = (r.standard_normal((max(whole, cut), c)).astype(np.float32) for c in (k, n))
+    got = []
+    for rows in (whole, cut):
+        descs = [abi.make_desc("l", "Linear", inputs=["x"], output="h", in_features=k, out_features=n, seq_len=rows, use_bias=1, params_count=weights[0].size)]
+        if what == "residual":
+            descs.append(abi.make_desc("s", "Add", inputs=["h", "r"], output="x"))
+        else:
+            descs.append(abi.make_desc("m", "Linear", inputs=["h"], output="x", in_features=n, out_features=n, seq_len=rows, use_bias=1, params_count=weights[1].size))
+        m = rt.GraphModel(descs, abi.PREC_BF16X2 if precision == "x2" else abi.PREC_BF16W)
+        m.upload_weights(0, weights[0])
+        inputs = {"x": (x[:rows].ravel(), False)}
+        if what == "residual":
+            inputs["r"] = (res[:rows].ravel(), False)
+        else:
+            m.upload_weights(1, weights[1])
+        m.plan({name: (v.size, bc) for name, (v, bc) in inputs.items()}, 1)
+        got.append(m.forward(inputs, 1, rows * n).reshape(rows, n))
+        m.close()
+    both = min(whole, cut)
+    assert np.array_equal(got[0][:both], got[1][:both])
+    want = x[-40:].astype(np.float64) @ weights[0][: n * k].reshape(n, k).T.astype(np.float64) + weights[0][n * k:]
+    if what == "residual":
+        want = want + res[-40:]
+    else:
+        want = want @ weights[1][: n * n].reshape(n, n).T.astype(np.float64) + weights[1][n * n:]
+    big = got[0] if whole > cut else got[1]
+    # 1e-5 for each contraction
+    assert np.linalg.norm(big[-40:] - want) <= (1e-5 if what == "residual" else 2e-5) * np.linalg.norm(want)
