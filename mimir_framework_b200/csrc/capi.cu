@@ -409,9 +409,10 @@ size_t conv_ws_bytes(int batch, int ic, int h, int w, int ks, int stride, int pa
   return align256(split_bytes(static_cast<int64_t>(conv_chunk_samples(batch, oh * ow, k, precision)) * oh * ow, k, ap));
 }
 
-// A residual that is the 2 x 2 upsample of a smaller image can be read there by the 256-pixel-tile kernel's epilogue.  Only where
-// that kernel has a tile for every SM: below that another form of the convolution may be the faster one by more than the upsample
-// kernel and its tensor cost (a few microseconds at such sizes).
+// A residual that is the 2 x 2 upsample of a smaller image can be read there by the spatial-tile kernel's epilogue.  Only where
+// that kernel has a tile of 256 pixels for every SM: below that another form of the convolution may be the faster one by more than the
+// upsample kernel and its tensor cost (a few microseconds at such sizes).  The line dates from before tiles of 128 pixels; launches that
+// run in those still read a residual of the output's own size.
 bool conv_takes_residual_up(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
   if (!conv_uses_shifted(ic, ks, stride, pad) || ks < 3 || (h | w) % 2 != 0 || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
   const long long rows = static_cast<long long>(batch) * (h + 2 * pad) * (w + 2 * pad);

@@ -1,5 +1,6 @@
 // gemm_split.cu — the contraction kernel for launches that cannot fill the GPU with 128 x 256 tiles (gemm_sm100.cu): a few rows,
-// short sequences, one sample's low-resolution convolution.  Same operands, same products, same results as launch_gemm's form
+// short sequences, one sample's low-resolution convolution.  Same operands, same products as launch_gemm's form, and results that differ
+// from its by the order of their sums only (split_weights)
 //
 //   Y[m, n] = act( sum_k A[m, k] * W[n, k] + bias[n] ) (+ residual[m, n])          (LayerOps.hpp:24-111)
 //
@@ -521,7 +522,10 @@ SplitPlan plan_split(const GemmArgs& g, int bk, int kblocks) {
 // at every K and product count), and half as much for those of its own range.  The ranges summed apart here do not lose that, and in
 // one instruction per 16 of K less than they would have.  The weights put it back, and the result is then scaled as the unsplit
 // kernel's is: a row gives the same answer in a small batch and in a large one.  Relative difference of the two, 40 x 1024 outputs,
-// K = 32768, three MMAs per product: 1e-4 without the weights, 1e-5 with them.
+// K = 32768, three MMAs per product: 1e-4 without the weights, 1e-5 with them.  What the weights put back is the mean loss, not what each
+// sum lost; the fewer ranges, the more of that differs.  162 x 130 outputs in one / three / eight ranges: K = 4608 5.6e-6 / 2.4e-6 / 1.7e-6,
+// K = 9216 1.1e-5 / 4.4e-6 / 3.0e-6, K = 32768 3.9e-5 / 1.5e-5 / 9.5e-6; one range is the nearest to the products in 64 bits (K = 9216:
+// 5.5e-6 against 1.5e-5 in three).
 void split_weights(SplitGemmParams& p, long long ksteps, int steps_per_block, int products) {
   auto at = [&](int s) {  // (zero-padded K adds exact zeros and loses nothing)
     const long long step = static_cast<long long>(p.kblocks) * s / p.splits * steps_per_block;

@@ -17,7 +17,11 @@
 //     next tile's weights on the way.
 // Within a step of 16 samples (12 layers of 768, vocabulary 32000), by CTA stamps from the input's arrival to the last store:
 // 768 -> 2304 with LayerNorm 8.0 -> 5.0 us, 768 -> 768 5.4 -> 2.9, 768 -> 3072 with LayerNorm 7.3 -> 5.6, 3072 -> 768 8.5 -> 4.2.  What is left of a
-// LayerNorm form: x 0.6, statistics and planes 2.3, products 1.5 (the instruction issues every 32 cycles), sums and store 0.6.
+// LayerNorm form: x 0.6, statistics and planes 2.3, products 1.5 (the instruction issues every 32 cycles), sums and store 0.6.  (The forms
+// without one are half a microsecond shorter since a warp looks for infinities once.)
+// Whole steps, FMAs / now: 16 samples, 12 layers of 768, 814 / 610 us; of 1024 with ffn 4096 892 / 793; 9 samples, six such layers, 326 / 261, of
+// 896 with ffn 3584 (14 samples) 375 / 278.  From K = 769 to a CTA on, 9 to 16 rows take more registers than two CTAs to an SM leave
+// (skinny_mma_kernel<4, 2, false>: 128, and 300 bytes of spills); the gain there is the smaller one.
 #include <type_traits>
 
 #include "common.h"
