@@ -294,13 +294,23 @@ struct RowNormArgs {
   const float* residual = nullptr;   // added last
   long long n_gamma = 0;             // RMS: gamma applies to i < n_gamma
   int log_softmax = 0;
+  // ROWS_MEANVAR without per_channel: the result as a contraction's operand planes (planes.cuh) instead of in y; only where
+  // norm_rows_planes_ok() holds for the contraction's K
+  __nv_bfloat16* y_split = nullptr;
+  int split_planes = 0, f16 = 0;
 };
 bool norm_rows_supported(const RowNormArgs& a);
+bool norm_rows_planes_ok(long long rows, long long len, int k);
 int launch_norm_rows(const RowNormArgs& a, cudaStream_t st);
 
 // norms.cu -------------------------------------------------------------------------------------
 int launch_layernorm(const float* x, const float* gamma, const float* beta, float* y, int64_t rows, int64_t n,
                      float eps, cudaStream_t st);
+// The same into the operand planes [planes][rows * n / k][k] of the contraction that reads it, where layernorm_planes_ok() holds and x
+// starts on 16 bytes
+int launch_layernorm_planes(const float* x, const float* gamma, const float* beta, __nv_bfloat16* y_split, int planes, int64_t rows, int64_t n,
+                            float eps, cudaStream_t st);
+bool layernorm_planes_ok(int64_t rows, int64_t n, int k);
 // y_split (optional): the result as bf16 hi (+ lo) operand planes, `plane_stride` elements apart, written by the
 // one-pass kernel; only where rmsnorm_onepass_ok() holds.  y may then be nullptr.
 int launch_rmsnorm(const float* x, const float* gamma, int64_t n_gamma, float* y, int batch, int64_t n, float eps,

@@ -1162,7 +1162,7 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
   if (g.m <= 0 || g.n <= 0 || g.k <= 0) return fail(MIMIR_B200_E_INVALID, "gemm: empty dimension");
   if (!g.a || !g.w) return fail(MIMIR_B200_E_INVALID, "gemm: null operand");
   if (!g.out_f32 && !g.out_split) return fail(MIMIR_B200_E_INVALID, "gemm: no output");
-  if (g.residual && !g.out_f32) return fail(MIMIR_B200_E_INVALID, "gemm: residual needs the fp32 output stride");
+  if (g.residual && !g.out_f32 && g.ldo < g.n) return fail(MIMIR_B200_E_INVALID, "gemm: residual needs the fp32 output stride");
   // K block per stage.  With at most three planes in play (one of the operands single-plane) a 64-wide block still leaves
   // three 64 KB stages, halves the barrier round trips per MMA and uses 128-byte swizzle rows: measured on the decoder's
   // K = 768 layers 0.77 -> 0.90 of the sustained cuBLAS rate.  With four planes (both operands split) 64-wide blocks leave a CTA on its

@@ -1104,7 +1104,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     TensorV& t = m->tensors[v];
     if (t.alias_of >= 0 || t.producer < 0 || v == out_root || total_consumers(v) != 1) continue;
     LayerRT& P = m->layers[t.producer];
-    if (P.lt != LT::Linear || P.out_v != v || P.out_f != C.in_f || P.rows_ps != C.rows_ps || P.res_v >= 0) continue;
+    if (P.lt != LT::Linear || P.out_v != v || P.out_f != C.in_f || P.rows_ps != C.rows_ps) continue;
     if (linear_uses_skinny(P.rows_ps * batch, m->precision)) continue;
     P.emit_split = true;
     P.emit_f32 = false;
@@ -1136,6 +1136,35 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       continue;
     }
     if (k <= 0 || k % 64 != 0 || rows_ps * k != t.n) continue;
+    P.emit_split = true;
+    P.emit_f32 = false;
+    C.read_split = true;
+    t.want_f32 = false;
+    t.want_split = true;
+    t.split_rows_ps = rows_ps;
+    t.split_k = k;
+  }
+
+  // ---- fusion 2c: the same for a LayerNorm that norm_rows.cu takes (not one that reads a caller's buffer, which need not start on 16 bytes) ----
+  for (int li = 0; li < nl; ++li) {
+    LayerRT& P = m->layers[li];
+    if (P.lt != LT::LayerNorm || P.skip) continue;
+    const int v = P.out_v, xr = root_of(m->tensors, P.in_v[0]);
+    TensorV& t = m->tensors[v];
+    if (t.alias_of >= 0 || v == out_root || total_consumers(v) != 1 || t.consumers.size() != 1) continue;
+    if (m->tensors[xr].producer < 0 || xr == out_root) continue;
+    LayerRT& C = m->layers[t.consumers[0]];
+    if (C.skip || C.in_v[0] != v || C.res_v == v || C.pre_ln >= 0) continue;
+    int k = 0;
+    int64_t rows_ps = 0;
+    if (C.lt == LT::Linear && !linear_uses_skinny(C.rows_ps * batch, m->precision)) {
+      k = C.in_f; rows_ps = C.rows_ps;
+    } else if (C.lt == LT::Attention && !(m->is_twin && attention_streams_weights(C, batch))) {
+      k = C.embed; rows_ps = C.seq;
+    } else {
+      continue;
+    }
+    if (rows_ps * k != t.n || !layernorm_planes_ok(batch * (t.n / P.norm_n), P.norm_n, k)) continue;
     P.emit_split = true;
     P.emit_f32 = false;
     C.read_split = true;
@@ -1436,7 +1465,13 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         const float* g = d.affine ? L.w_f32 : nullptr;
         const float* b = (d.affine && d.use_bias) ? L.w_f32 + L.norm_n : nullptr;
         const int64_t rows = static_cast<int64_t>(batch) * (m->tensors[L.in_v[0]].n / L.norm_n);
-        s = launch_layernorm(f32p(L.in_v[0]), g, b, f32p(L.out_v), rows, L.norm_n, d.eps, st);
+        if (L.emit_split) {
+          int ap, wp;
+          precision_planes(m->precision, &ap, &wp);
+          s = launch_layernorm_planes(f32p(L.in_v[0]), g, b, splitp(L.out_v), ap, rows, L.norm_n, d.eps, st);
+        } else {
+          s = launch_layernorm(f32p(L.in_v[0]), g, b, f32p(L.out_v), rows, L.norm_n, d.eps, st);
+        }
         break;
       }
       case LT::RMSNorm: {

@@ -11,6 +11,7 @@
 // asked for ahead of the wait: the registry transformer at batch 8 192.0 -> 189.9 us (four norms), at batch 1 from host arrays 235 -> 228 us.
 #include "common.h"
 #include "launch.cuh"
+#include "planes.cuh"
 
 namespace mb {
 namespace {
@@ -94,7 +95,10 @@ __device__ __forceinline__ float row_reduce1(float v, int step, RowShared& sh, u
 // NV: vectors of four floats of a thread; WARP: a row per warp, else a row per CTA or cluster.  SHIFT: rows may start anywhere; vectors
 // lie on 16-byte boundaries of the tensor all the same, those at a row's ends are moved element by element, and gamma / beta (or
 // the channel of a GroupNorm) are looked up per element.  `slice`: elements of a CTA, counted from the boundary before the row.
-template <int FAM, bool SHIFT, int NV, bool WARP>
+// PLANES: a LayerNorm that only a contraction reads writes that contraction's operand planes, and the fp32 result and the pass that would
+// cut it never exist (a pass of its own wrote and read them again: 1 to 3 us of a chain of launches; 40 samples x 128 tokens x 256, two
+// layers: 255.6 -> 249.1 us).  Rows of k elements, a multiple of 64: the planes have no padding and the layout of the fp32 result.
+template <int FAM, bool SHIFT, int NV, bool WARP, bool PLANES>
 __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) norm_rows_kernel(const RowNormArgs p, const int slice) {
   __shared__ RowShared sh;
   uint32_t rank = 0, size = 1;
@@ -288,6 +292,14 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
         if (rem >= p.hw) { rem -= p.hw; ++ch; }
       }
     }
+    if (PLANES) {
+      uint2 h, l;
+      split_pair(r[0], r[1], p.f16, h.x, l.x);
+      split_pair(r[2], r[3], p.f16, h.y, l.y);
+      *reinterpret_cast<uint2*>(p.y_split + base + i) = h;
+      if (p.split_planes == 2) *reinterpret_cast<uint2*>(p.y_split + p.rows * p.len + base + i) = l;
+      continue;
+    }
     float* o = p.y + base + i;
     if (whole(j)) {
       __stcs(reinterpret_cast<float4*>(o), make_float4(r[0], r[1], r[2], r[3]));
@@ -314,25 +326,25 @@ RowShape row_shape(long long rows, long long len) {
   return s;
 }
 
-template <int FAM, bool SHIFT, int NV>
+template <int FAM, bool SHIFT, int NV, bool PLANES>
 int launch_nv(const RowNormArgs& a, const RowShape& s, int slice, cudaStream_t st) {
-  if (s.threads == 32) return launch_pdl(norm_rows_kernel<FAM, SHIFT, NV, true>, dim3(static_cast<unsigned>((a.rows + 3) / 4)), dim3(128), 0, st, 1, a, slice);
-  return launch_pdl(norm_rows_kernel<FAM, SHIFT, NV, false>, dim3(static_cast<unsigned>(a.rows * s.ctas)), dim3(static_cast<unsigned>(s.threads)), 0, st, s.ctas, a,
+  if (s.threads == 32) return launch_pdl(norm_rows_kernel<FAM, SHIFT, NV, true, PLANES>, dim3(static_cast<unsigned>((a.rows + 3) / 4)), dim3(128), 0, st, 1, a, slice);
+  return launch_pdl(norm_rows_kernel<FAM, SHIFT, NV, false, PLANES>, dim3(static_cast<unsigned>(a.rows * s.ctas)), dim3(static_cast<unsigned>(s.threads)), 0, st, s.ctas, a,
                     slice);
 }
-template <int FAM, bool SHIFT>
+template <int FAM, bool SHIFT, bool PLANES = false>
 int launch_shift(const RowNormArgs& a, const RowShape& s, cudaStream_t st) {
   const long long span = a.len + (SHIFT ? 3 : 0);  // with what may lie between the boundary before the row and its start
   const int slice = static_cast<int>((((span + s.ctas - 1) / s.ctas) + 3) & ~3LL);
   const int nv = (slice / 4 + s.threads - 1) / s.threads;
-  if (nv <= 1) return launch_nv<FAM, SHIFT, 1>(a, s, slice, st);
-  if (nv <= 2) return launch_nv<FAM, SHIFT, 2>(a, s, slice, st);
-  if (nv <= 3) return launch_nv<FAM, SHIFT, 3>(a, s, slice, st);
-  if (nv <= 4) return launch_nv<FAM, SHIFT, 4>(a, s, slice, st);
-  if (nv <= 5) return launch_nv<FAM, SHIFT, 5>(a, s, slice, st);
-  if (nv <= 6) return launch_nv<FAM, SHIFT, 6>(a, s, slice, st);
-  if (nv <= 7) return launch_nv<FAM, SHIFT, 7>(a, s, slice, st);
-  return launch_nv<FAM, SHIFT, 8>(a, s, slice, st);
+  if (nv <= 1) return launch_nv<FAM, SHIFT, 1, PLANES>(a, s, slice, st);
+  if (nv <= 2) return launch_nv<FAM, SHIFT, 2, PLANES>(a, s, slice, st);
+  if (nv <= 3) return launch_nv<FAM, SHIFT, 3, PLANES>(a, s, slice, st);
+  if (nv <= 4) return launch_nv<FAM, SHIFT, 4, PLANES>(a, s, slice, st);
+  if (nv <= 5) return launch_nv<FAM, SHIFT, 5, PLANES>(a, s, slice, st);
+  if (nv <= 6) return launch_nv<FAM, SHIFT, 6, PLANES>(a, s, slice, st);
+  if (nv <= 7) return launch_nv<FAM, SHIFT, 7, PLANES>(a, s, slice, st);
+  return launch_nv<FAM, SHIFT, 8, PLANES>(a, s, slice, st);
 }
 template <int FAM>
 int launch_fam(const RowNormArgs& a, const RowShape& s, bool shift, cudaStream_t st) {
@@ -352,13 +364,22 @@ bool norm_rows_supported(const RowNormArgs& a) {
          (len <= 8LL * NR_MAX_THREADS * 32 && (a.len & 3) != 0);
 }
 
+bool norm_rows_planes_ok(long long rows, long long len, int k) {
+  RowNormArgs a;
+  a.rows = rows; a.len = len;
+  return k > 0 && k % 64 == 0 && len % k == 0 && norm_rows_supported(a);
+}
+
 int launch_norm_rows(const RowNormArgs& a, cudaStream_t st) {
   const RowShape s = row_shape(a.rows, a.len + 3);
   const bool affine = a.per_channel ? (a.hw & 3) == 0
                                     : ((reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) == 0;
   const bool shift = (a.len & 3) != 0 || !affine;
   int r;
-  if (a.family == ROWS_MEANVAR) r = launch_fam<ROWS_MEANVAR>(a, s, shift, st);
+  if (a.y_split != nullptr) {
+    if (a.family != ROWS_MEANVAR || shift) return fail(MIMIR_B200_E_UNSUPPORTED, "norm: operand planes need aligned rows and parameters");
+    r = launch_shift<ROWS_MEANVAR, false, true>(a, s, st);
+  } else if (a.family == ROWS_MEANVAR) r = launch_fam<ROWS_MEANVAR>(a, s, shift, st);
   else if (a.family == ROWS_RMS) r = launch_fam<ROWS_RMS>(a, s, shift, st);
   else r = launch_fam<ROWS_SOFTMAX>(a, s, shift, st);
   if (r == MIMIR_B200_OK) count_launch();

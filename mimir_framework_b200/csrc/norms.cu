@@ -1107,6 +1107,18 @@ int launch_layernorm(const float* x, const float* gamma, const float* beta, floa
   return meanvar_dispatch(x, y, rows, n, eps, a, st);
 }
 
+bool layernorm_planes_ok(int64_t rows, int64_t n, int k) { return norm_rows_on() && norm_rows_planes_ok(rows, n, k); }
+
+int launch_layernorm_planes(const float* x, const float* gamma, const float* beta, __nv_bfloat16* y_split, int planes, int64_t rows, int64_t n,
+                            float eps, cudaStream_t st) {
+  RowNormArgs r;
+  r.x = x; r.rows = rows; r.len = n; r.eps = eps; r.gamma = gamma; r.beta = gamma ? beta : nullptr;
+  r.y_split = y_split; r.split_planes = planes; r.f16 = plane_format() == PLANES_F16 ? 1 : 0;
+  if (!norm_rows_supported(r))
+    return fail(MIMIR_B200_E_UNSUPPORTED, "LayerNorm: operand planes were requested for a shape or an address that the row kernel does not take");
+  return launch_norm_rows(r, st);
+}
+
 int launch_groupnorm(const float* x, const float* gamma, const float* beta, float* y, int batch, int ch, int hw, int groups,
                      float eps, int act, const float* residual, cudaStream_t st) {
   if (groups <= 0 || ch % groups != 0) return fail(MIMIR_B200_E_INVALID, "GroupNorm: channels must be divisible by num_groups");

@@ -150,3 +150,56 @@ def test_rmsnorms_behind_one_that_gave_up_write_nothing(rt, rows, n, tickets, fl
     want = x.double() / torch.sqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-5)
     # (the reference's sequential fp32 sum, which the kernel follows, is off by up to n roundings of 2^-24 of the sum of squares)
     assert float((y - want).abs().max()) <= (1e-6 + n * 2.0**-25) * float(want.abs().max())
+
+
+def contraction_bound(k):
+    """fp32 inputs and their split to 2e-6; three MMAs per 16 of K, each of which loses 1.5e-8 to 3.6e-8 of the sum by truncation, of which
+    the epilogue puts 1.5e-8 back."""
+    return 2e-6 + 3 * (k + 15) // 16 * 2.1e-8
+
+
+@pytest.mark.parametrize("tokens,d,whole", [(17, 64, False), (200, 128, False), (33, 1088, False), (40, 100, False), (128, 4096, False),
+                                            (20, 64, True), (160, 192, True), (128, 256, True), (333, 1024, True), (20, 100, True)])
+def test_layernorm_into_operand_planes(rt, tokens, d, whole):
+    """A LayerNorm that only a contraction reads writes its operand planes: a row for a warp, a CTA and a cluster, one row of all
+    tokens, one too long for registers, and (100 elements, whose planes are padded) the form that stays apart."""
+    r = np.random.default_rng(tokens + d)
+    n, batch, f = tokens * d, 3, 40
+    x = (r.standard_normal((batch, n)) + 0.5).astype(np.float32)
+    ln = n if whole else d
+    g, be = (1 + 0.1 * r.standard_normal(ln)).astype(np.float32), r.standard_normal(ln).astype(np.float32)
+    w, b = (r.standard_normal((f, d)) / np.sqrt(d)).astype(np.float32), r.standard_normal(f).astype(np.float32)
+    descs = [abi.make_desc("a", "ReLU", inputs=["x"], output="a"),
+             abi.make_desc("n", "LayerNorm", inputs=["a"], output="h", in_features=0 if whole else d, affine=1, use_bias=1, eps=1e-5, params_count=2 * ln),
+             abi.make_desc("l", "Linear", inputs=["h"], output="x", in_features=d, out_features=f, seq_len=tokens, use_bias=1, params_count=f * d + f)]
+    mod = rt.GraphModel(descs)
+    mod.upload_weights(1, np.concatenate([g, be]))
+    mod.upload_weights(2, np.concatenate([w.ravel(), b]))
+    mod.plan({"x": (n, False)}, batch)
+    h = np.maximum(x, 0).astype(np.float64).reshape(batch, -1, ln)
+    h = (h - h.mean(-1, keepdims=True)) / np.sqrt(h.var(-1, keepdims=True) + 1e-5) * g + be
+    want = h.reshape(batch, tokens, d) @ w.astype(np.float64).T + b
+    for _ in range(3):  # layer by layer, captured, replayed
+        got = mod.forward({"x": (x.ravel(), False)}, batch, tokens * f).reshape(want.shape)
+        assert np.linalg.norm(got - want) <= contraction_bound(d) * np.linalg.norm(want)
+    mod.close()
+
+
+@pytest.mark.parametrize("rows,k,n", [(17, 64, 64), (40, 130, 1000), (300, 96, 70), (1000, 256, 768), (20000, 64, 300)])
+def test_linear_with_a_residual_into_operand_planes(rt, rows, k, n):
+    """x = act(a) + lin(act(a)), read by one Linear only: the sum leaves the first Linear as the second one's planes."""
+    r = np.random.default_rng(rows)
+    x = r.standard_normal((rows, k)).astype(np.float32)
+    w0, w1, w2 = ((r.standard_normal(s) / np.sqrt(s[1])).astype(np.float32) for s in ((n, k), (n, n), (64, n)))
+    lin = lambda name, i, o, w: abi.make_desc(name, "Linear", inputs=[i], output=o, in_features=w.shape[1], out_features=w.shape[0], seq_len=rows, use_bias=0,
+                                              params_count=w.size)
+    descs = [lin("l0", "x", "a", w0), lin("l1", "a", "b", w1), abi.make_desc("s", "Add", inputs=["a", "b"], output="c"), lin("l2", "c", "x", w2)]
+    mod = rt.GraphModel(descs)
+    for i, w in ((0, w0), (1, w1), (3, w2)):
+        mod.upload_weights(i, w.ravel())
+    mod.plan({"x": (rows * k, False)}, 1)
+    a = x.astype(np.float64) @ w0.astype(np.float64).T
+    want = (a + a @ w1.astype(np.float64).T) @ w2.astype(np.float64).T
+    got = mod.forward({"x": (x.ravel(), False)}, 1, rows * 64).reshape(want.shape)
+    mod.close()
+    assert np.linalg.norm(got - want) <= (contraction_bound(k) + 2 * contraction_bound(n)) * np.linalg.norm(want)
