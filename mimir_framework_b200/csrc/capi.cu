@@ -4,6 +4,7 @@
 // in graph.cu.  No function here throws; none falls back to the CPU.
 #include "ops.h"
 #include "host_call.h"
+#include "planes.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -163,6 +164,30 @@ ErrorWatch::~ErrorWatch() {
     c_.error_words.push_back(word_);
   }
 }
+StageBlock::StageBlock() : c_(ctx()) {
+  std::lock_guard<std::mutex> lk(c_.error_mu);
+  if (c_.stage_blocks.empty()) return;
+  p = c_.stage_blocks.back();
+  c_.stage_blocks.pop_back();
+}
+StageBlock::~StageBlock() {
+  if (!p) return;
+  if (in_use) cudaStreamSynchronize(in_use);  // (the call failed half-way)
+  std::lock_guard<std::mutex> lk(c_.error_mu);
+  c_.stage_blocks.push_back(p);
+}
+int* ErrorWatch::claim(cudaStream_t st) {
+  if (!word_) {
+    std::lock_guard<std::mutex> lk(c_.error_mu);
+    if (c_.error_words.empty()) return nullptr;
+    word_ = c_.error_words.back();
+    c_.error_words.pop_back();
+  }
+  if (word_ == &own_) return nullptr;
+  st_ = st;
+  in_flight_ = true;
+  return word_;
+}
 int ErrorWatch::enqueue(cudaStream_t st) {
   if (!word_) {
     std::lock_guard<std::mutex> lk(c_.error_mu);
@@ -259,7 +284,7 @@ int linear_exec(const LinearExec& e, cudaStream_t st) {
   g.w = e.w_split;
   g.a_planes = ap;
   g.w_planes = wp;
-  g.w_scale = e.w_scale; g.w_ready = e.w_ready;
+  g.w_scale = e.w_scale; g.w_amax = e.w_amax; g.w_ready = e.w_ready;
   g.m = e.rows;
   g.n = e.out_f;
   g.k = e.in_f;
@@ -549,11 +574,14 @@ int mimir_b200_init(int device, size_t hbm_budget_bytes) {
   }
   c.dev_error_word = static_cast<int*>(w);
   MB_CUDA(cudaMemset(c.dev_error_word, 0, 256));
-  constexpr int CALLS = 64;  // at a time with a page-locked word each
-  void* hw = nullptr;
-  MB_CUDA(cudaHostAlloc(&hw, CALLS * sizeof(int), cudaHostAllocPortable));
+  constexpr int CALLS = 64, BLOCKS = 8;  // at a time with a page-locked word each, with a block each
   std::lock_guard<std::mutex> el(c.error_mu);
-  for (int i = 0; i < CALLS; ++i) c.error_words.push_back(static_cast<int*>(hw) + i);
+  if (c.host_words) return MIMIR_B200_OK;  // (they outlive a shutdown)
+  void* hw = nullptr;
+  MB_CUDA(cudaHostAlloc(&hw, BLOCKS * STAGE_BYTES + CALLS * sizeof(int), cudaHostAllocPortable));
+  c.host_words = true;
+  for (int i = 0; i < BLOCKS; ++i) c.stage_blocks.push_back(static_cast<uint8_t*>(hw) + i * STAGE_BYTES);
+  for (int i = 0; i < CALLS; ++i) c.error_words.push_back(reinterpret_cast<int*>(static_cast<uint8_t*>(hw) + BLOCKS * STAGE_BYTES) + i);
   return MIMIR_B200_OK;
 }
 
@@ -778,8 +806,13 @@ int mimir_b200_linear_forward_ex(const float* input, const float* weights, const
     precision_planes(precision, &ap, &wp);
     void* wsplit;
     MB_TRY(t.alloc(&wsplit, split_bytes(out_f, in_f, wp), "linear.wsplit"));
-    MB_TRY(weight_plane_scale(e.w_f32, static_cast<size_t>(out_f) * in_f, nullptr, &e.w_scale));
-    MB_TRY(launch_split(e.w_f32, static_cast<__nv_bfloat16*>(wsplit), out_f, in_f, wp, nullptr, e.w_scale));
+    if (plane_format() == PLANES_F16) {
+      void* word;
+      MB_TRY(t.alloc(&word, sizeof(unsigned), "linear.wmax"));
+      MB_TRY(launch_absmax(e.w_f32, static_cast<size_t>(out_f) * in_f, static_cast<unsigned*>(word), nullptr));
+      e.w_amax = static_cast<const unsigned*>(word);
+    }
+    MB_TRY(launch_split(e.w_f32, static_cast<__nv_bfloat16*>(wsplit), out_f, in_f, wp, nullptr, 1.0f, e.w_amax));
     e.w_split = static_cast<const __nv_bfloat16*>(wsplit);
   }
   MB_TRY(linear_exec(e, nullptr));

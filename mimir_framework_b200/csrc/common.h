@@ -91,6 +91,8 @@ struct Context {
   int* dev_error_word = nullptr;
   std::mutex error_mu;                     // held while the word is looked at on the host and cleared
   std::vector<int*> error_words;           // page-locked words that no call uses at the moment
+  bool host_words = false;                 // these and the blocks exist
+  std::vector<uint8_t*> stage_blocks;      // page-locked blocks of STAGE_BYTES, likewise (StageBlock, ops.h)
   std::atomic<uint64_t> error_clears{0};
   int last_error_site = 0;
   // Optional live timing of the contraction kernel: pairs of events recorded on the launching
@@ -145,6 +147,18 @@ void temp_free(const TempBuffer& b, bool idle);
 int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);
 int copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
 void release_host_copier();
+bool host_memory(const void* p);  // ordinary or page-locked, and so the caller's to read and write
+// Small tensors of a host-pointer call, by one kernel each way instead of a copy command per tensor (pointwise.cu).
+constexpr int STAGE_ITEMS = 8;
+constexpr size_t STAGE_BYTES = size_t(32) << 10;
+struct StageItems {
+  int count = 0;
+  struct { const uint32_t* src; uint32_t* dst; int words, copies; } item[STAGE_ITEMS];  // `copies` one behind the other at dst
+  void add(const void* src, void* dst, size_t words, int copies = 1) {
+    item[count++] = {static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), static_cast<int>(words), copies};
+  }
+};
+int launch_stage_copy(const StageItems& items, cudaStream_t st);
 // src -> device -> dst through a copier of its own that meets failures on the host: `inject` 1 page-locked memory, 2 a second thread,
 // are not to be had
 int host_copy_selftest(int inject, const float* src, float* dst, size_t n, int* ring_copies);
@@ -166,8 +180,12 @@ int plane_format();
 // Power of two that the weights of one layer are multiplied by before they become half planes (1 for bfloat16
 // planes): brings the largest magnitude near 2^14 so that small weights keep their bits.  Synchronises `st`.
 int weight_plane_scale(const float* w_dev, size_t n, cudaStream_t st, float* scale);
-// fp32 [rows, k] -> planes (hi, and lo when planes == 2) of src * scale
-int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int planes, cudaStream_t st, float scale = 1.0f);
+// The largest finite |w| as its bits, left on the device: for calls that use their weights once, where finding the scale on the host
+// would cost a synchronisation (one call on host arrays, 512 x 768 x 3072: 25 us of 520)
+int launch_absmax(const float* w_dev, size_t n, unsigned* word, cudaStream_t st);
+// fp32 [rows, k] -> planes (hi, and lo when planes == 2) of src * scale (amax: of the scale that belongs to that word instead)
+int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int planes, cudaStream_t st, float scale = 1.0f,
+                 const unsigned* amax = nullptr);
 // fp32 [k, n] (row-major, "input-major") -> planes of its transpose [n, kp], times scale
 int launch_split_transposed(const float* src, __nv_bfloat16* dst, int k, int n, int planes, cudaStream_t st, float scale = 1.0f);
 
@@ -176,6 +194,7 @@ struct GemmArgs {
   const __nv_bfloat16* w = nullptr;  // [w_planes][n][kp]
   int a_planes = 2, w_planes = 2;
   float w_scale = 1.0f;              // the weight planes hold w * w_scale (weight_plane_scale); divided out in the epilogue
+  const unsigned* w_amax = nullptr;  // or w times the scale of this device word (launch_absmax), and w_scale 1; row-major results only
   int m = 0, n = 0, k = 0;           // logical sizes; kp = round_up(k, 64)
   const float* bias = nullptr;       // [n] or null
   const float* residual = nullptr;   // fp32 [m, n] added after the activation, or null

@@ -69,6 +69,7 @@ struct GemmParams {
   // The tensor core adds each MMA's products to the fp32 accumulator with truncation, not round-to-nearest, which
   // shrinks every result by a little less than 2^-26 of its value per instruction (see launch_gemm_t).
   float acc_scale;
+  const unsigned* w_amax;  // see GemmArgs
   int f16;        // operand planes (and out_split) hold IEEE half instead of bfloat16
   // The operand ring: a stage holds only the planes the precision mode uses (32 KB with two activation planes and one
   // weight plane at BK = 32), so the same shared memory gives six stages instead of four - the K = 768 layers were
@@ -382,6 +383,7 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int quad = warp & 3;   // TMEM lane quadrant this warp may read
     const int half = ew >> 2;    // which half of the columns
     const bool chan_major = CM && (p.ohw > 0 || p.conv_ks > 0);
+    const float acc_scale = p.w_amax == nullptr ? p.acc_scale : p.acc_scale * plane_unscale(__ldg(p.w_amax));
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = t_first; t < num_tiles; t += t_step) {
@@ -459,7 +461,7 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           float v[32];
           tmem_ld_32x32(taddr0 + c0, v);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = __fmul_rn(v[j], p.acc_scale);  // [pixel][channel]
+          for (int j = 0; j < 32; ++j) tbuf[j * 33 + lane] = __fmul_rn(v[j], acc_scale);  // [pixel][channel]
           __syncwarp();
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = tbuf[lane * 33 + j];  // lane = pixel r0 + lane, j = channel oc0 + j
@@ -524,12 +526,12 @@ gemm_tn_bf16split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             const float4 b4 = __ldg(reinterpret_cast<const float4*>(p.bias + col0 + j));
-            v[j] = __fmaf_rn(v[j], p.acc_scale, b4.x); v[j + 1] = __fmaf_rn(v[j + 1], p.acc_scale, b4.y);
-            v[j + 2] = __fmaf_rn(v[j + 2], p.acc_scale, b4.z); v[j + 3] = __fmaf_rn(v[j + 3], p.acc_scale, b4.w);
+            v[j] = __fmaf_rn(v[j], acc_scale, b4.x); v[j + 1] = __fmaf_rn(v[j + 1], acc_scale, b4.y);
+            v[j + 2] = __fmaf_rn(v[j + 2], acc_scale, b4.z); v[j + 3] = __fmaf_rn(v[j + 3], acc_scale, b4.w);
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __fmaf_rn(v[j], p.acc_scale, (p.bias != nullptr && col0 + j < p.n) ? __ldg(p.bias + col0 + j) : 0.0f);
+          for (int j = 0; j < 32; ++j) v[j] = __fmaf_rn(v[j], acc_scale, (p.bias != nullptr && col0 + j < p.n) ? __ldg(p.bias + col0 + j) : 0.0f);
         }
         switch (p.activation) {  // hoisted out of the element loop
           case MIMIR_B200_ELT_GELU:
@@ -755,9 +757,10 @@ namespace {
 
 // One thread per 8 consecutive K elements of one row; the padded tail kp > k is written as zero.
 __global__ void split_rows_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int k,
-                                  int kp, int planes, int f16, float scale) {
+                                  int kp, int planes, int f16, float scale, const unsigned* __restrict__ amax) {
   pdl_launch_dependents();
   pdl_wait();
+  if (amax != nullptr) scale = plane_scale(__ldg(amax));
   const int chunks = kp >> 3;
   const long long total = rows * chunks;
   const long long plane_stride = rows * static_cast<long long>(kp);
@@ -935,6 +938,7 @@ int launch_gemm_t(const GemmArgs& g, cudaStream_t st) {
   p.a_group_rows = g.a_group_rows;
   p.w_group_rows = g.w_group_rows;
   p.acc_scale = gemm_acc_scale(g);
+  p.w_amax = g.w_amax;
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   constexpr int RING_BYTES = 196608;  // 192 KB of operand stages, cut into as many stages as the planes in use allow
   constexpr int SMEM = RING_BYTES + 1024 /*align slack*/ + 512 /*barriers*/ + EPI_WARPS * 32 * 33 * 4 /*swapped-epilogue tiles*/;
@@ -1026,34 +1030,31 @@ __global__ void absmax_kernel(const float* __restrict__ w, size_t n, unsigned* _
 }
 }  // namespace
 
-int weight_plane_scale(const float* w_dev, size_t n, cudaStream_t st, float* scale) {
-  *scale = 1.0f;
-  if (plane_format() != PLANES_F16 || n == 0 || w_dev == nullptr) return MIMIR_B200_OK;
-  static std::mutex mu;  // one spare device word is shared by every caller
-  std::lock_guard<std::mutex> lk(mu);
-  unsigned* word = reinterpret_cast<unsigned*>(ctx().dev_error_word) + 8;  // a spare word of the 256-byte error block
+int launch_absmax(const float* w_dev, size_t n, unsigned* word, cudaStream_t st) {
   MB_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned), st));
   const size_t want = (n + 255) / 256;
   const int blocks = static_cast<int>(want < static_cast<size_t>(ctx().sm_count) * 8 ? want : static_cast<size_t>(ctx().sm_count) * 8);
   absmax_kernel<<<blocks, 256, 0, st>>>(w_dev, n, word);
   MB_CUDA(cudaGetLastError());
   count_launch();
-  unsigned bits = 0;
-  MB_CUDA(cudaMemcpyAsync(&bits, word, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-  MB_CUDA(cudaStreamSynchronize(st));
-  float amax;
-  memcpy(&amax, &bits, sizeof(float));
-  if (!(amax > 0.0f)) return MIMIR_B200_OK;
-  int e = 0;
-  frexpf(amax, &e);            // amax = f * 2^e with f in [0.5, 1)
-  int s = 14 - e;              // amax * 2^s in [2^13, 2^14)
-  if (s > 60) s = 60;
-  if (s < -60) s = -60;
-  *scale = ldexpf(1.0f, s);
   return MIMIR_B200_OK;
 }
 
-int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int planes, cudaStream_t st, float scale) {
+int weight_plane_scale(const float* w_dev, size_t n, cudaStream_t st, float* scale) {
+  *scale = 1.0f;
+  if (plane_format() != PLANES_F16 || n == 0 || w_dev == nullptr) return MIMIR_B200_OK;
+  static std::mutex mu;  // one spare device word is shared by every caller
+  std::lock_guard<std::mutex> lk(mu);
+  unsigned* word = reinterpret_cast<unsigned*>(ctx().dev_error_word) + 8;  // a spare word of the 256-byte error block
+  MB_TRY(launch_absmax(w_dev, n, word, st));
+  unsigned bits = 0;
+  MB_CUDA(cudaMemcpyAsync(&bits, word, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  MB_CUDA(cudaStreamSynchronize(st));
+  *scale = ldexpf(1.0f, plane_scale_exponent(bits));
+  return MIMIR_B200_OK;
+}
+
+int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int planes, cudaStream_t st, float scale, const unsigned* amax) {
   if (rows <= 0 || k <= 0) return MIMIR_B200_OK;
   const int kp = round_up(k, 64);
   const long long total = rows * (kp >> 3);
@@ -1061,7 +1062,7 @@ int launch_split(const float* src, __nv_bfloat16* dst, int64_t rows, int k, int 
   long long blocks = (total + threads - 1) / threads;
   const long long cap = static_cast<long long>(ctx().sm_count) * 16;
   if (blocks > cap) blocks = cap;
-  MB_TRY(launch_pdl(split_rows_kernel, dim3(static_cast<int>(blocks)), dim3(threads), 0, st, 1, src, dst, rows, k, kp, planes, plane_format() == PLANES_F16, scale));
+  MB_TRY(launch_pdl(split_rows_kernel, dim3(static_cast<int>(blocks)), dim3(threads), 0, st, 1, src, dst, rows, k, kp, planes, plane_format() == PLANES_F16, scale, amax));
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

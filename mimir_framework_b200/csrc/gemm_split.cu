@@ -65,6 +65,7 @@ struct SplitGemmParams {
   int ohw;
   int conv_ks, conv_cblocks, conv_pad, conv_hp, conv_wp, conv_h, conv_w;
   float acc_scale;
+  const unsigned* w_amax;  // see GemmArgs
   int f16, stages, stage_bytes, w_ready;
   float weight[SG_MAX_SPLITS];  // of the ranges' partial sums (split_weights)
   int stg_off;  // the staging tile: behind the operand ring, or in its place (0)
@@ -231,6 +232,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // every thread below reads or writes memory that the previous kernels of the stream may still be using
   pdl_wait();
   const bool chan_major = conv || p.ohw > 0;
+  const float acc_scale = p.w_amax == nullptr ? p.acc_scale : p.acc_scale * plane_unscale(__ldg(p.w_amax));
   const int slice = (p.bn + p.splits - 1) / p.splits;  // columns a CTA finishes; the last ones fewer, or none
   const int oc0 = to * SG_M, row0 = tr * p.bn + split * slice;
   const int quad = warp & 3, group = warp >> 2;
@@ -338,8 +340,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       for (int i = 0; i < 4; ++i) {
         const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
         u[i] = odd ? make_float2(other, v[2 * i + 1]) : make_float2(v[2 * i], other);
-        u[i].x = __fmaf_rn(u[i].x, p.acc_scale, b2.x);
-        u[i].y = __fmaf_rn(u[i].y, p.acc_scale, b2.y);
+        u[i].x = __fmaf_rn(u[i].x, acc_scale, b2.x);
+        u[i].y = __fmaf_rn(u[i].y, acc_scale, b2.y);
       }
       if (p.activation == MIMIR_B200_ELT_GELU) {
 #pragma unroll
@@ -407,7 +409,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (in) {
           const float* src = stg + cl * pitch + ch;
           for (int s = 0; s < p.splits; ++s) a[u] = fmaf(src[s * slice * pitch], p.weight[s], a[u]);
-          a[u] = __fmaf_rn(a[u], p.acc_scale, p.bias != nullptr ? __ldg(p.bias + oc0 + ch) : 0.0f);
+          a[u] = __fmaf_rn(a[u], acc_scale, p.bias != nullptr ? __ldg(p.bias + oc0 + ch) : 0.0f);
         }
         ch += step_ch;
         cl += step_cl;
@@ -558,6 +560,7 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
   p.conv_ks = g.conv_ks; p.conv_cblocks = conv ? g.conv_c / BK : 1; p.conv_pad = g.conv_pad;
   p.conv_hp = g.conv_h + 2 * g.conv_pad; p.conv_wp = g.conv_w + 2 * g.conv_pad; p.conv_h = g.conv_h; p.conv_w = g.conv_w;
   p.acc_scale = gemm_acc_scale(g);
+  p.w_amax = g.w_amax;
   split_weights(p, conv ? static_cast<long long>(p.kblocks) * (BK / 16) : (g.k + 15) / 16, BK / 16, AP + WP - 1);
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   p.w_ready = g.w_ready ? 1 : 0;

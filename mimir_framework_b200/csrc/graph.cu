@@ -1986,9 +1986,74 @@ static int ensure_pipeline_objects(MimirB200Model* m) {
   return MIMIR_B200_OK;
 }
 
-int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inputs, int n_inputs, int batch, float* out_host,
-                             uint64_t out_capacity, uint64_t* out_len) {
-  DeviceScope dev_scope(m ? m->device : ctx().device);
+// A forward that is not cut into micro-batches: everything on one stream.  Small inputs, a decode step's position, a small result
+// and the error word go through a page-locked block (launch_stage_copy), larger ones through copy commands.
+static int forward_host_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, const std::vector<int>& vs, float* out_host, const int* pos) {
+  const TensorV& ot = m->tensors[root_of(m->tensors, m->out_v)];
+  const int batch = m->planned_micro;
+  const cudaStream_t st = m->s_comp;
+  ErrorWatch errors;
+  StageBlock block;
+  size_t used = 0;
+  StageItems in, out;
+  auto place = [&](size_t bytes) {  // in the block; the item that follows starts on 16 bytes
+    const size_t at = used;
+    used += (bytes + 15) & ~size_t(15);
+    return block.p + at;
+  };
+  auto fits = [&](const StageItems& items, size_t bytes) { return block.p != nullptr && items.count < STAGE_ITEMS && bytes <= STAGE_BYTES - 16 && used <= STAGE_BYTES - 16 - bytes; };
+  MB_CUDA(cudaEventRecord(m->ev0, st));
+  if (pos) {
+    if (fits(in, sizeof(int))) {
+      uint8_t* p = place(sizeof(int));
+      memcpy(p, pos, sizeof(int));
+      in.add(p, m->pos_dev, 1);
+    } else {
+      MB_CUDA(cudaMemcpyAsync(m->pos_dev, pos, sizeof(int), cudaMemcpyHostToDevice, st));
+    }
+  }
+  for (int i = 0; i < n_inputs; ++i) {
+    const TensorV& t = m->tensors[vs[i]];
+    float* slot = reinterpret_cast<float*>(m->arena + t.off_f32);
+    const int copies = t.broadcast_input && !t.one_copy ? batch : 1;
+    const size_t n = static_cast<size_t>(t.n) * (t.broadcast_input ? 1 : batch);
+    if (fits(in, n * 4) && n * copies <= (size_t(1) << 20) && host_memory(inputs[i].data)) {
+      uint8_t* p = place(n * 4);
+      memcpy(p, inputs[i].data, n * 4);
+      in.add(p, slot, n, copies);
+    } else {
+      MB_TRY(copy_to_device(slot, inputs[i].data, n * 4, st));
+      if (copies > 1) MB_TRY(launch_broadcast_rows(slot, slot + t.n, copies - 1, t.n, st));
+    }
+  }
+  if (in.count > 0) block.in_use = st;
+  MB_TRY(launch_stage_copy(in, st));
+  Bound b;
+  MB_TRY(run_layers_cached(m, batch, b, st, m->arena));
+  MB_CUDA(cudaEventRecord(m->ev1, st));
+  const size_t n_out = static_cast<size_t>(ot.n) * batch;
+  const float* result = reinterpret_cast<const float*>(m->arena + ot.off_f32);
+  uint8_t* staged = fits(out, n_out * 4) && host_memory(out_host) ? place(n_out * 4) : nullptr;
+  if (staged) out.add(result, staged, n_out);
+  if (int* word = staged ? errors.claim(st) : nullptr) out.add(ctx().dev_error_word, word, 1);
+  else MB_TRY(errors.enqueue(st));
+  if (staged) block.in_use = st;
+  MB_TRY(launch_stage_copy(out, st));
+  if (!staged) MB_TRY(copy_to_host(out_host, result, n_out * 4, st));
+  MB_CUDA(cudaStreamSynchronize(st));
+  block.in_use = nullptr;
+  if (staged) memcpy(out_host, staged, n_out * 4);
+  MB_TRY(errors.read(st));
+  cudaEventElapsedTime(&m->last_ms, m->ev0, m->ev1);
+  ctx().stats.ms_last_forward = m->last_ms;
+  ctx().stats.flops_last_forward = m->flops;
+  ctx().stats.bytes_last_forward = m->hbm_bytes;
+  return MIMIR_B200_OK;
+}
+
+// pos: a decode step's position, for m->pos_dev
+static int forward_host(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch, float* out_host, uint64_t out_capacity,
+                        uint64_t* out_len, const int* pos) {
   std::vector<int> vs;
   MB_TRY(check_inputs(m, inputs, n_inputs, batch, &vs));
   const TensorV& ot = m->tensors[root_of(m->tensors, m->out_v)];
@@ -1999,8 +2064,10 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
     MB_CUDA(cudaEventCreate(&m->ev1));
   }
   MB_TRY(ensure_pipeline_objects(m));
-  ErrorWatch errors;
   const int micro = m->planned_micro, P = m->pipeline;
+  if (P == 1) return forward_host_once(m, inputs, n_inputs, vs, out_host, pos);
+  ErrorWatch errors;
+  if (pos) MB_CUDA(cudaMemcpyAsync(m->pos_dev, pos, sizeof(int), cudaMemcpyHostToDevice, m->s_comp));
   uint8_t* bufs[2] = {m->arena, m->arena2 ? m->arena2 : m->arena};
   MB_CUDA(cudaEventRecord(m->ev0, m->s_comp));
   // copy-in, compute and copy-out of consecutive micro-batches overlap; buffer c & 1 is reused by
@@ -2045,6 +2112,12 @@ int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inpu
   ctx().stats.flops_last_forward = m->flops * P;
   ctx().stats.bytes_last_forward = m->hbm_bytes * P;
   return MIMIR_B200_OK;
+}
+
+int mimir_b200_model_forward(MimirB200ModelHandle m, const MimirNamedInput* inputs, int n_inputs, int batch, float* out_host,
+                             uint64_t out_capacity, uint64_t* out_len) {
+  DeviceScope dev_scope(m ? m->device : ctx().device);
+  return forward_host(m, inputs, n_inputs, batch, out_host, out_capacity, out_len, nullptr);
 }
 
 // ---- incremental decoding ---------------------------------------------------------------------------
@@ -2202,12 +2275,8 @@ int mimir_b200_model_decode_step(MimirB200ModelHandle m, const MimirNamedInput* 
   if (pos < 0 || pos >= m->decode->max_seq) return fail(MIMIR_B200_E_INVALID, "decode_step: position %d outside the cache of %d", pos, m->decode->max_seq);
   MimirB200Model* t = m->decode;
   t->decode_pos = pos;
-  if (t->pos_dev) {
-    // the previous step has fully drained (forward synchronises), so the word can be rewritten before this one starts
-    MB_TRY(ensure_pipeline_objects(t));
-    MB_CUDA(cudaMemcpyAsync(t->pos_dev, &t->decode_pos, sizeof(int), cudaMemcpyHostToDevice, t->s_comp));
-  }
-  return mimir_b200_model_forward(t, inputs, n_inputs, batch, out_host, out_capacity, out_len);
+  // (the previous step has fully drained - forward synchronises - so the position on the device can be rewritten before this one starts)
+  return forward_host(t, inputs, n_inputs, batch, out_host, out_capacity, out_len, t->pos_dev ? &t->decode_pos : nullptr);
 }
 
 // Cuts the batch of the host-pointer forward into `micro_batches` pieces that overlap their

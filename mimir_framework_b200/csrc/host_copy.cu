@@ -2,9 +2,10 @@
 //
 // cudaMemcpy stages such memory through the driver's own page-locked buffers on the calling thread: 10 to 18 GB/s on the 16-core
 // hosts measured, of the 50 GB/s that the link takes from page-locked memory.  Here a few helper threads and the caller move
-// pieces of 256 KB between the caller's memory and a page-locked ring, while the caller issues the DMA of whole segments of up
-// to 2 MB (a copy command costs about 6 us on these hosts whatever its size, so small segments from several threads gave
-// 15 GB/s).  The helpers make no CUDA calls.  Used from COPY_MIN bytes up, with helpers
+// pieces of 64 KB between the caller's memory and a page-locked ring, while the caller issues the DMA of whole segments of up
+// to 2 MB (a copy command costs about 8 us on these hosts whatever its size, so small segments from several threads gave
+// 15 GB/s, and 2 MB to the host in four of them took 95 us where one takes 46).  To the device the first segments are small, so that the
+// link starts early; to the host the last one is, so that little is left to move when the link is done.  The helpers make no CUDA calls.  Used from COPY_MIN bytes up, with helpers
 // from two pieces up (waking them costs more than one piece), and for pageable memory only; page-locked memory goes straight to cudaMemcpyAsync.
 //   9.4 MB to the device 0.51 -> 0.25 ms, 6.3 MB to the host 0.31 -> 0.20 ms, 64 MB 4.4 -> 1.6 and 1.8 ms (42 and 38 GB/s)
 #include <immintrin.h>
@@ -22,7 +23,7 @@ namespace mb {
 namespace {
 
 constexpr size_t COPY_MIN = size_t(64) << 10;
-constexpr size_t PIECE = size_t(256) << 10;
+constexpr size_t PIECE = size_t(64) << 10;
 constexpr size_t SEGMENT = size_t(2) << 20;
 constexpr int RING = 8;  // segments: 16 MB of page-locked memory per device
 constexpr int MAX_HELPERS = 5;
@@ -53,19 +54,40 @@ struct Job {
   bool to_device = false;
   uint8_t* dev = nullptr;
   uint8_t* host = nullptr;
-  size_t bytes = 0, segment = 0;  // bytes per segment, a multiple of PIECE
-  size_t pieces = 0, segments = 0;
+  size_t bytes = 0, pieces = 0, segments = 0;
+  size_t lead = 0, last = 0;  // to the host: segments of SEGMENT bytes, bytes of the one behind them (all but the last)
   std::atomic<size_t> next{0};   // next piece to move
   std::atomic<size_t> open{0};   // segments whose ring slot may be filled (to the device) / has landed (to the host)
   std::atomic<uint32_t> moved[RING];
   std::atomic<bool> cancel{false};
 
-  size_t seg_of(size_t piece) const { return piece * PIECE / segment; }
+  void cut() {
+    pieces = (bytes + PIECE - 1) / PIECE;
+    if (to_device) {  // 512 KB, 1 MB, then SEGMENT each
+      segments = seg_of(pieces - 1) + 1;
+      return;
+    }
+    size_t rest = bytes;
+    while (rest > SEGMENT + SEGMENT / 2) { rest -= SEGMENT; ++lead; }
+    // (a rest of 512 KB and less goes as one)
+    last = rest <= SEGMENT / 4 ? rest : (rest * 5 / 8 + PIECE - 1) / PIECE * PIECE;
+    if (last > SEGMENT) last = SEGMENT;
+    segments = lead + (rest > last ? 2 : 1);
+  }
+  size_t seg_off(size_t s) const {
+    if (to_device) return s == 0 ? 0 : s == 1 ? SEGMENT / 4 : SEGMENT / 4 * 3 + (s - 2) * SEGMENT;
+    return s <= lead ? s * SEGMENT : lead * SEGMENT + last;
+  }
+  size_t seg_of(size_t piece) const {
+    const size_t off = piece * PIECE;
+    if (to_device) return off < SEGMENT / 4 ? 0 : off < SEGMENT / 4 * 3 ? 1 : 2 + (off - SEGMENT / 4 * 3) / SEGMENT;
+    return off < lead * SEGMENT ? off / SEGMENT : off < lead * SEGMENT + last ? lead : lead + 1;
+  }
   size_t pieces_of(size_t s) const { return (seg_bytes(s) + PIECE - 1) / PIECE; }
-  size_t seg_bytes(size_t s) const { return s + 1 == segments ? bytes - s * segment : segment; }
+  size_t seg_bytes(size_t s) const { return (s + 1 == segments ? bytes : seg_off(s + 1)) - seg_off(s); }
   void move(size_t piece, uint8_t* ring) {
     const size_t off = piece * PIECE, s = seg_of(piece), n = bytes - off < PIECE ? bytes - off : PIECE;
-    uint8_t* slot = ring + (s % RING) * SEGMENT + (off - s * segment);
+    uint8_t* slot = ring + (s % RING) * SEGMENT + (off - seg_off(s));
     if (to_device) copy_into_ring(slot, host + off, n); else memcpy(host + off, slot, n);
     moved[s % RING].fetch_add(1, std::memory_order_release);
   }
@@ -179,7 +201,7 @@ struct HostCopier {
       for (size_t s = 0; s < j.segments && s < RING && e == cudaSuccess; ++s) free_slot(s);
       for (size_t s = 0; s < j.segments && e == cudaSuccess; ++s) {
         wait_moved(j, s);
-        e = cudaMemcpyAsync(j.dev + s * j.segment, ring + (s % RING) * SEGMENT, j.seg_bytes(s), cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync(j.dev + j.seg_off(s), ring + (s % RING) * SEGMENT, j.seg_bytes(s), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(ev[s % RING], st);
         in_flight[s % RING] = true;
         by[s % RING] = std::this_thread::get_id();
@@ -191,7 +213,7 @@ struct HostCopier {
       if (in_flight[s % RING] && e == cudaSuccess) e = cudaEventSynchronize(ev[s % RING]);  // an earlier job's
       in_flight[s % RING] = false;
       if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ring + (s % RING) * SEGMENT, j.dev + s * j.segment, j.seg_bytes(s), cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(ring + (s % RING) * SEGMENT, j.dev + j.seg_off(s), j.seg_bytes(s), cudaMemcpyDeviceToHost, st);
       if (e == cudaSuccess) e = cudaEventRecord(ev[s % RING], st);
     };
     for (size_t s = 0; s < j.segments && s < RING && e == cudaSuccess; ++s) fetch(s);
@@ -227,11 +249,7 @@ struct HostCopier {
     std::unique_lock<std::mutex> one(call, std::try_to_lock);
     *taken = one.owns_lock() && init();
     if (!*taken) return MIMIR_B200_OK;
-    // about four segments, so that the first DMA starts early; whole pieces; at most a ring slot
-    const size_t quarter = (j.bytes / 4 + PIECE - 1) / PIECE * PIECE;
-    j.segment = quarter < SEGMENT ? quarter : SEGMENT;
-    j.segments = (j.bytes + j.segment - 1) / j.segment;
-    j.pieces = (j.bytes + PIECE - 1) / PIECE;
+    j.cut();
     if (held_by_others(j)) {
       *taken = false;
       return MIMIR_B200_OK;
@@ -277,6 +295,16 @@ bool pageable(const void* p) {
   }
   return a.type == cudaMemoryTypeUnregistered;
 }
+}  // namespace
+bool host_memory(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
+}
+namespace {
 HostCopier* copier() {
   static std::mutex mu;
   std::lock_guard<std::mutex> lk(mu);

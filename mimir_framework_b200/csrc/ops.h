@@ -20,6 +20,7 @@ class ErrorWatch {
   ErrorWatch(const ErrorWatch&) = delete;
   ErrorWatch& operator=(const ErrorWatch&) = delete;
   int enqueue(cudaStream_t st);  // copies the word in stream order
+  int* claim(cudaStream_t st);   // the same left to a launch of the caller's: where to (page-locked), or null
   int read(cudaStream_t st);     // after a synchronisation of the stream that carried the copy; clears on `st`
 
  private:
@@ -29,6 +30,20 @@ class ErrorWatch {
   int own_ = 0;  // where no page-locked word is left
   bool in_flight_ = false;
   cudaStream_t st_ = nullptr;
+};
+
+// A page-locked block of STAGE_BYTES for one call; null where none is left.  The stream that reads or writes it has drained when it goes back.
+class StageBlock {
+ public:
+  StageBlock();
+  ~StageBlock();
+  StageBlock(const StageBlock&) = delete;
+  StageBlock& operator=(const StageBlock&) = delete;
+  uint8_t* p = nullptr;
+  cudaStream_t in_use = nullptr;  // set while launches that use it may be in flight
+
+ private:
+  Context& c_;
 };
 
 // A token-wise LayerNorm folded into the contraction that reads it: x is then the LayerNorm's input.
@@ -47,6 +62,7 @@ struct LinearExec {
   const float* w_f32 = nullptr;             // fp32 [out_f, in_f] (skinny path)
   const __nv_bfloat16* w_split = nullptr;   // planes [w_planes][out_f][kp] (tensor-core path)
   float w_scale = 1.0f;                     // the planes hold W * w_scale (weight_plane_scale)
+  const unsigned* w_amax = nullptr;         // see GemmArgs
   bool w_ready = false;                     // the planes were complete before this call's launches (GemmArgs::w_ready)
   const float* bias = nullptr;
   const float* residual = nullptr;          // same layout as y_f32

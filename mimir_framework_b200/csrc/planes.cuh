@@ -23,6 +23,15 @@ enum : int { PLANES_BF16 = 0, PLANES_F16 = 1 };
 
 namespace {
 
+// The power of two that weights of largest magnitude `amax` (the bits of a float; 0: no finite one but zero) are multiplied by, amax * 2^s in
+// [2^13, 2^14) with |s| <= 60, and its reciprocal: weight_plane_scale()'s value, for launches that find amax on the device.
+__host__ __device__ __forceinline__ int plane_scale_exponent(unsigned amax) {
+  const int s = 140 - static_cast<int>(amax >> 23);
+  return amax == 0 ? 0 : s > 60 ? 60 : s < -60 ? -60 : s;
+}
+__device__ __forceinline__ float plane_scale(unsigned amax) { return __uint_as_float(static_cast<unsigned>(127 + plane_scale_exponent(amax)) << 23); }
+__device__ __forceinline__ float plane_unscale(unsigned amax) { return __uint_as_float(static_cast<unsigned>(127 - plane_scale_exponent(amax)) << 23); }
+
 // two values -> two packed pairs (element 0 in the low half)
 __device__ __forceinline__ void split_pair(float x0, float x1, int f16, uint32_t& hi, uint32_t& lo) {
   if (f16) {

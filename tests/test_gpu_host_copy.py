@@ -28,6 +28,50 @@ def test_round_trip_is_exact(rt, bytes_, extra):
     assert np.array_equal(rt.eltwise(abi.ELT_RELU, x), np.maximum(x, 0))
 
 
+@pytest.mark.parametrize("bytes_", [128 << 10, 512 << 10, (512 << 10) + (64 << 10), 3 * (512 << 10), 3 << 20, (3 << 20) + (64 << 10), (3 * 512 << 10) + (16 << 20), 19 << 20])
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+def test_round_trip_at_the_edges_of_uneven_segments(rt, bytes_, extra):
+    x = np.random.default_rng(bytes_ + extra).standard_normal(bytes_ // 4 + extra, dtype=np.float32)
+    assert np.array_equal(rt.eltwise(abi.ELT_RELU, x), np.maximum(x, 0))
+
+
+@pytest.mark.parametrize("batch,n,inputs", [(1, 1, 1), (3, 5, 2), (1, 8188, 1), (1, 8189, 1), (2, 4097, 2), (4, 1025, 7), (2, 33, 9), (1, 4096, 3)])
+def test_small_tensors_through_the_staging_block(rt, batch, n, inputs):
+    """Around the block's 32 KB and eight tensors, each sample's own and broadcast ones (made in a kernel), with results that
+    change from call to call."""
+    descs, names = [], ["x"] + [f"i{k}" for k in range(1, inputs)]
+    for k in range(1, inputs):
+        descs.append(abi.make_desc(f"a{k}", "Add", inputs=["x" if k == 1 else f"s{k - 1}", names[k]], output="x" if k + 1 == inputs else f"s{k}"))
+    if not descs:
+        descs.append(abi.make_desc("r", "ReLU", inputs=["x"], output="x"))
+    mod = rt.GraphModel(descs)
+    mod.plan({m: (n, k % 2 == 1) for k, m in enumerate(names)}, batch)
+    for seed in range(4):
+        r = np.random.default_rng(seed)
+        a = {m: r.standard_normal((1 if k % 2 else batch, n), dtype=np.float32) for k, m in enumerate(names)}
+        want = np.maximum(a["x"], 0) if inputs == 1 else a["x"]
+        for m in names[1:]:
+            want = want + a[m]
+        got = mod.forward({m: (a[m].ravel(), k % 2 == 1) for k, m in enumerate(names)}, batch, n)
+        assert np.array_equal(got.reshape(batch, n), want.reshape(batch, n))
+    mod.close()
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-42, 1e-30, 2.0**-13, 1.0, 3.0, 1e30])
+@pytest.mark.parametrize("rows,k,n", [(17, 64, 40), (600, 100, 1000)])
+def test_weight_scale_found_on_the_device(rt, scale, rows, k, n):
+    """One call on host arrays has the bits of a planned model, whose weight scale is found on the host."""
+    r = np.random.default_rng(k)
+    x, w = r.standard_normal((rows, k), dtype=np.float32), (r.standard_normal((n, k)) * scale).astype(np.float32)
+    b = r.standard_normal(n, dtype=np.float32)
+    mod = rt.GraphModel([abi.make_desc("l", "Linear", inputs=["x"], output="x", in_features=k, out_features=n, seq_len=rows, use_bias=1, params_count=n * k + n)])
+    mod.upload_weights(0, np.concatenate([w.ravel(), b]))
+    mod.plan({"x": (rows * k, False)}, 1)
+    want = mod.forward({"x": (x.ravel(), False)}, 1, rows * n).ravel()
+    mod.close()
+    assert np.array_equal(rt.linear_forward(x.ravel(), w.ravel(), b, rows, k, n), want, equal_nan=True)  # (1e30 leaves the planes' range either way)
+
+
 def test_threads_do_not_mix(rt):
     bad = []
 
