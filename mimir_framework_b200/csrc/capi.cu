@@ -410,18 +410,33 @@ bool conv_uses_shifted(int ic, int ks, int stride, int pad) {
 
 size_t conv_prenorm_bytes(int batch, int groups) { return align256(static_cast<size_t>(batch) * groups * 2 * sizeof(float)); }
 
-size_t conv_gn_emit_bytes(int batch, int oc, int h, int w, int pad, int groups) {
+// The arguments of a shifted convolution's launch, as far as the choice of its form looks at them
+static bool shifted_args(int batch, int ic, int oc, int h, int w, int ks, int pad, int precision, GemmArgs* g) {
   const long long rows = static_cast<long long>(batch) * (h + 2 * pad) * (w + 2 * pad);
-  return align256(gemm_gn_part_bytes(rows, oc, oc / groups));
+  if (rows > 0x7fffffffLL) return false;
+  static float some = 0.0f;  // (only asked whether there is an output)
+  precision_planes(precision, &g->a_planes, &g->w_planes);
+  g->m = static_cast<int>(rows); g->n = oc; g->k = ic * ks * ks;
+  g->out_f32 = &some;
+  g->conv_ks = ks; g->conv_c = ic; g->conv_pad = pad; g->conv_h = h; g->conv_w = w;
+  return true;
 }
 
-bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int groups, int act) {
-  static const bool on = [] { const char* e = getenv("MIMIR_B200_GN_EPILOGUE"); return e && e[0] == '1'; }();
-  if (!on || groups <= 0 || oc % groups != 0) return false;
-  const int cpg = oc / groups;
-  if (!(cpg == 4 || cpg == 8 || cpg == 16 || cpg == 32)) return false;
+size_t conv_gn_emit_bytes(int batch, int ic, int oc, int h, int w, int ks, int pad, int precision) {
+  GemmArgs g;
+  return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) ? align256(conv_gemm_gn_bytes(g)) : 0;
+}
+
+// From a result of 32 MB on, and where the spatial-tile kernel runs the convolution anyway: a smaller one is swept in L2 in the time that
+// merging the moments takes (33 MB: a sweep of 7.1 us against 2.5 here and 2.5 in the convolution; 8 MB: 3.6 us).
+bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int groups, int act, bool res_up) {
+  static const char mode = [] { const char* e = getenv("MIMIR_B200_GN_EPILOGUE"); return e ? e[0] : ' '; }();  // "0": never, "1": wherever it can
+  if (mode == '0' || groups <= 0 || oc % groups != 0 || oc / groups % 4 != 0 || oc % 32 != 0) return false;
   if (!conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
-  return static_cast<long long>(h + 2 * pad) * (w + 2 * pad) >= 64 && batch <= 65535;
+  GemmArgs g;
+  if (!shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) || conv_gemm_cycles(g) >= 1e30) return false;
+  if (mode == '1') return true;
+  return static_cast<long long>(batch) * oc * h * w * 4 >= (32ll << 20) && (res_up || gemm_takes_spatial(g));
 }
 
 size_t conv_ws_bytes(int batch, int ic, int h, int w, int ks, int stride, int pad, int precision) {
@@ -440,14 +455,8 @@ size_t conv_ws_bytes(int batch, int ic, int h, int w, int ks, int stride, int pa
 // run in those still read a residual of the output's own size.
 bool conv_takes_residual_up(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
   if (!conv_uses_shifted(ic, ks, stride, pad) || ks < 3 || (h | w) % 2 != 0 || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
-  const long long rows = static_cast<long long>(batch) * (h + 2 * pad) * (w + 2 * pad);
-  if (rows > 0x7fffffffLL) return false;
   GemmArgs g;
-  precision_planes(precision, &g.a_planes, &g.w_planes);
-  float out = 0.0f;
-  g.m = static_cast<int>(rows); g.n = oc; g.k = ic * ks * ks;
-  g.out_f32 = &out;  // (only asked whether there is one)
-  g.conv_ks = ks; g.conv_c = ic; g.conv_pad = pad; g.conv_h = h; g.conv_w = w;
+  if (!shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g)) return false;
   return conv_gemm_cycles(g) < 1e30 && conv_gemm_tiles(g) >= ctx().sm_count;
 }
 
@@ -489,11 +498,9 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     g.ldo = e.oc;
     g.conv_ks = e.ks; g.conv_c = e.ic; g.conv_pad = e.pad; g.conv_h = e.h; g.conv_w = e.w;
     if (e.gn_stats_out != nullptr) {
-      g.gn_part = reinterpret_cast<float*>(static_cast<uint8_t*>(e.ws) + planes_bytes + (e.pre_groups > 0 ? conv_prenorm_bytes(e.batch, e.pre_groups) : 0));
-      g.gn_cpg = e.oc / e.gn_groups;
+      g.gn_part = reinterpret_cast<float4*>(static_cast<uint8_t*>(e.ws) + planes_bytes + (e.pre_groups > 0 ? conv_prenorm_bytes(e.batch, e.pre_groups) : 0));
       MB_TRY(launch_gemm(g, st));
-      return launch_gn_stats_from_partials(g.gn_part, e.gn_stats_out, e.batch, e.gn_groups, g.gn_cpg, rows, e.oc,
-                                           (e.h + 2 * e.pad) * (e.w + 2 * e.pad), e.gn_eps, st);
+      return launch_conv_gn_stats(g, e.gn_stats_out, e.gn_groups, e.gn_eps, st);
     }
     return launch_gemm(g, st);
   }

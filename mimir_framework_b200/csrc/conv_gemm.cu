@@ -13,6 +13,9 @@
 //   warp 1     : MMA issuer: weights are the M side (128 output channels), 256 pixels (or 128) the N side; two accumulators in TMEM
 //   warps 2..9 : epilogue: 32 x 32 chunks turned around in shared memory so that a lane owns a pixel; NCHW stores
 //   warp 10    : TMA producer of weight tiles       (ring of W_STAGES, one per tap and plane)
+// Where a GroupNorm reads the result the epilogue leaves its moments behind (GN): a sweep over a tensor larger than L2 less, and the
+// warps that take them have the time, as the MMAs of a K of 576 and more outlast the stores: 2 to 3 us of 110 to 450 on a launch, for
+// sweeps of 7 to 89 us (UNet of 16 samples: 4167 -> 3945 us, conv stack 7159 -> 7055).
 // Every wait is bounded, as in gemm_sm100.cu.
 #include "common.h"
 #include "epilogue.cuh"
@@ -43,8 +46,25 @@ struct ConvGemmParams {
   int activation;
   float acc_scale;
   int f16;
+  float4* gn_part;                             // [sample][four channels][spatial tile x 2 halves] (mean, second moment about it, values, -)
   int* err_word;
 };
+
+// Sums over the warp of eight values a lane (recursive halving): lanes 4 g ... 4 g + 3 end with that of value g.
+__device__ __forceinline__ float sum8(float (&a)[8], int lane) {
+  int mask = 16;
+#pragma unroll
+  for (int half = 4; half >= 1; half >>= 1, mask >>= 1) {
+    const bool upper = (lane & mask) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = upper ? a[i] : a[i + half], keep = upper ? a[i + half] : a[i];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+    }
+  }
+  a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+  return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+}
 
 struct ConvTile { int oc0, n, y0, x0; };
 __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) {  // output-channel tiles fastest: they share activations in L2
@@ -59,7 +79,7 @@ __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) { 
 }
 
 // BK: channels of a K block, 32 (64-byte swizzle rows) or 64 (128-byte rows)
-template <int AP, int WP, int BK>
+template <int AP, int WP, int BK, int GN>
 __global__ void __launch_bounds__(CG_THREADS, 1)
 conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const ConvGemmParams p) {
   constexpr int W_TILE = CG_M * BK * 2;
@@ -232,6 +252,13 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       while (!mbar_try_wait(&acc_full[acc], acc_phase)) {}  // completes at once: lane 0 saw the phase
       tcgen05_fence_after();
       const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * CG_N);
+      // A lane's own moments of each four channels: sums about the first value it met, so that a large mean costs nothing
+      float ref[8], s1[8], s2[8];
+      int pixels = 0;
+      if (GN) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g) ref[g] = s1[g] = s2[g] = 0.0f;
+      }
       if (nch > 0) {
 #pragma unroll 1
         for (int ci = 0; ci < chunks; ++ci) {
@@ -260,6 +287,42 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < nch) p.out[o0 + j * hw] = v[j];
+          }
+          if (GN && in) {
+            if (pixels++ == 0) {
+#pragma unroll
+              for (int g = 0; g < 8; ++g) ref[g] = v[4 * g];
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float e = v[j] - ref[j >> 2];
+              s1[j >> 2] += e;
+              s2[j >> 2] = fmaf(e, e, s2[j >> 2]);
+            }
+          }
+        }
+        if (GN) {
+          // the lanes' moments meet (T. F. Chan, G. H. Golub, R. J. LeVeque 1979); a second moment beyond fp32 stays infinite
+          const float n = 4.0f * pixels, inv = pixels > 0 ? 1.0f / n : 0.0f;
+          const float total = 4.0f * __reduce_add_sync(0xffffffffu, pixels), inv_total = total > 0.0f ? 1.0f / total : 0.0f;
+          float a[8];
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const float d = s1[g] * inv;
+            s2[g] = s2[g] < INFINITY ? fmaxf(s2[g] - s1[g] * d, 0.0f) : s2[g];
+            ref[g] += d;  // the lane's mean
+            a[g] = n * ref[g];
+          }
+          const float mean = sum8(a, lane) * inv_total;
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const float d = ref[g] - __shfl_sync(0xffffffffu, mean, 4 * g);
+            a[g] = fmaf(n * d, d, s2[g]);
+          }
+          const float m2 = sum8(a, lane);
+          if ((lane & 3) == 0) {
+            const int spatial = p.tiles_x * p.tiles_y, place = (t / p.tiles_o) % spatial * 2 + half;
+            p.gn_part[(static_cast<long long>(c.n) * (p.oc >> 2) + (oc0 >> 2) + (lane >> 2)) * (2 * spatial) + place] = make_float4(mean, m2, total, 0.0f);
           }
         }
       }
@@ -327,7 +390,39 @@ double conv_cycles(const GemmArgs& g, int* px) {
   return *px == CG_N ? whole : half;
 }
 
-template <int AP, int WP, int BK>
+// (mean, 1 / std) of one (sample, group) from the tiles' moments, a CTA each, in double and in an order that does not change.  (A warp each took
+// 14 us for the 512 x 512 entries of 16 images of 256^2.)
+__global__ void __launch_bounds__(128) conv_gn_stats_kernel(const float4* __restrict__ part, float* __restrict__ stats, int entries, float eps) {
+  __shared__ double sh[4][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double n = 0.0, mean = 0.0, m2 = 0.0;
+  auto merge = [&](double nb, double mb, double m2b) {
+    if (nb <= 0.0) return;
+    const double nt = n + nb, d = mb - mean, f = nb / nt;
+    mean += d * f;
+    m2 += m2b + d * d * n * f;
+    n = nt;
+  };
+  const float4* e = part + static_cast<long long>(blockIdx.x) * entries;
+  for (int i = threadIdx.x; i < entries; i += 128) {
+    const float4 q = __ldg(e + i);
+    merge(q.z, q.x, q.y);
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const double nb = __shfl_down_sync(0xffffffffu, n, d), mb = __shfl_down_sync(0xffffffffu, mean, d), m2b = __shfl_down_sync(0xffffffffu, m2, d);
+    merge(nb, mb, m2b);  // (lanes past the end merge what nobody reads)
+  }
+  if (lane == 0) { sh[warp][0] = n; sh[warp][1] = mean; sh[warp][2] = m2; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 4; ++w) merge(sh[w][0], sh[w][1], sh[w][2]);
+    stats[2 * blockIdx.x] = static_cast<float>(mean);
+    stats[2 * blockIdx.x + 1] = 1.0f / sqrtf(static_cast<float>(n > 0.0 ? m2 / n : 0.0) + eps);
+  }
+}
+
+template <int AP, int WP, int BK, int GN>
 int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   const int ks = g.conv_ks, pad = g.conv_pad;
   ConvGemmParams p;
@@ -353,6 +448,7 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   p.residual = g.residual; p.res_up = g.residual != nullptr && g.residual_up ? 1 : 0; p.out = g.out_f32; p.activation = g.activation;
   p.acc_scale = gemm_acc_scale(g);
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
+  p.gn_part = g.gn_part;
   p.err_word = ctx().dev_error_word;
   CUtensorMap map_a, map_w;
   MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, BK, tw, rows));
@@ -360,13 +456,13 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * (CG_M * BK * 2) + CG_EPI + 1024;
   static PerDeviceOnce attr_once;
   MB_TRY(attr_once.run([&]() -> int {
-    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
+    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP, BK, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
     return MIMIR_B200_OK;
   }));
   const int sms = ctx().sm_count;
   GemmProfile prof(st);
   MB_TRY(prof.begin());
-  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP, BK>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p));
+  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP, BK, GN>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p));
   MB_TRY(prof.end());
   count_launch();
   return MIMIR_B200_OK;
@@ -380,7 +476,7 @@ double conv_gemm_cycles(const GemmArgs& g) {
   constexpr double never = 1e30;
   const char* e = getenv("MIMIR_B200_CONV_SPATIAL");  // "0": never, "1": wherever the form allows
   if (e && e[0] == '0') return never;
-  if (g.conv_ks < 1 || g.conv_ks > 7 || g.conv_c % 32 != 0 || g.gn_part != nullptr || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
+  if (g.conv_ks < 1 || g.conv_ks > 7 || g.conv_c % 32 != 0 || g.bias != nullptr || g.out_f32 == nullptr || g.out_split != nullptr)
     return never;
   if (!(g.a_planes == 2 || g.w_planes == 1)) return never;
   if (e && e[0] == '1') return 0.0;
@@ -391,13 +487,40 @@ double conv_gemm_cycles(const GemmArgs& g) {
   return conv_cycles(g, &px);
 }
 
+size_t conv_gemm_gn_bytes(const GemmArgs& g) {
+  const ConvShape a = conv_shape(g, CG_N), b = conv_shape(g, CG_N / 2);
+  const long long per = static_cast<long long>(g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad);
+  const long long tiles = static_cast<long long>(a.tiles_x) * a.tiles_y, halves = static_cast<long long>(b.tiles_x) * b.tiles_y;
+  return static_cast<size_t>(g.m / per * (g.n / 4) * 2 * (tiles > halves ? tiles : halves)) * sizeof(float4);
+}
+
+int launch_conv_gn_stats(const GemmArgs& g, float* stats, int groups, float eps, cudaStream_t st) {
+  int px;
+  conv_cycles(g, &px);
+  const ConvShape sh = conv_shape(g, px);
+  const int batch = g.m / ((g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad)), slabs = batch * groups;
+  conv_gn_stats_kernel<<<slabs, 128, 0, st>>>(g.gn_part, stats, g.n / groups / 4 * 2 * sh.tiles_x * sh.tiles_y, eps);
+  MB_CUDA(cudaGetLastError());
+  count_launch();
+  return MIMIR_B200_OK;
+}
+
+template <int AP, int WP>
+int launch_conv_planes(const GemmArgs& g, bool wide, cudaStream_t st) {
+  if (g.gn_part != nullptr) {
+    if (g.n % 32 != 0) return fail(MIMIR_B200_E_INVALID, "conv: GroupNorm moments need output channels in whole chunks of 32");
+    return wide ? launch_conv_t<AP, WP, 64, 1>(g, st) : launch_conv_t<AP, WP, 32, 1>(g, st);
+  }
+  return wide ? launch_conv_t<AP, WP, 64, 0>(g, st) : launch_conv_t<AP, WP, 32, 0>(g, st);
+}
+
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {
   int px;
   conv_cycles(g, &px);
   const bool wide = conv_wide_blocks(g, px);
-  if (g.a_planes == 2 && g.w_planes == 2) return wide ? launch_conv_t<2, 2, 64>(g, st) : launch_conv_t<2, 2, 32>(g, st);
-  if (g.a_planes == 2 && g.w_planes == 1) return wide ? launch_conv_t<2, 1, 64>(g, st) : launch_conv_t<2, 1, 32>(g, st);
-  if (g.a_planes == 1 && g.w_planes == 1) return wide ? launch_conv_t<1, 1, 64>(g, st) : launch_conv_t<1, 1, 32>(g, st);
+  if (g.a_planes == 2 && g.w_planes == 2) return launch_conv_planes<2, 2>(g, wide, st);
+  if (g.a_planes == 2 && g.w_planes == 1) return launch_conv_planes<2, 1>(g, wide, st);
+  if (g.a_planes == 1 && g.w_planes == 1) return launch_conv_planes<1, 1>(g, wide, st);
   return fail(MIMIR_B200_E_INVALID, "conv: %d activation and %d weight planes", g.a_planes, g.w_planes);
 }
 

@@ -595,7 +595,7 @@ int launch_split_t(const GemmArgs& g, const SplitPlan& plan, cudaStream_t st) {
 
 double gemm_split_cycles(const GemmArgs& g, int bk, int* bn, int* splits) {
   constexpr double never = 1e30;
-  if (g.a_group_rows > 0 || g.gn_part != nullptr) return never;
+  if (g.a_group_rows > 0) return never;
   const int kblocks = g.conv_ks > 0 ? g.conv_ks * g.conv_ks * (g.conv_c / bk) : round_up(g.k, 64) / bk;
   const char* e = getenv("MIMIR_B200_GEMM_SPLIT");  // "0": never; "<bn>,<splits>": always, in that shape
   if (e && e[0] == '0' && e[1] == '\0') return never;

@@ -1193,10 +1193,10 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
   m->tensors[out_root].last = nl;
 
   // ---- offsets ---------------------------------------------------------------------------------------
-  // ---- fusion 1e: GroupNorm statistics out of the producing convolution's GEMM epilogue (MIMIR_B200_GN_EPILOGUE=1) ----
-  //      A GroupNorm (folded into a convolution's layout pass or running on its own) whose input is the output of a shifted-GEMM
-  //      convolution does not sweep that tensor for its mean and variance: the convolution's epilogue leaves per-block partials
-  //      behind, a small kernel merges them, and the GroupNorm (or the layout pass) reads (mean, 1 / std) from there.
+  // ---- fusion 1e: GroupNorm statistics out of the producing convolution's epilogue ----
+  //      A GroupNorm (folded into a convolution's layout pass or running on its own) whose input is a large result of the spatial-tile
+  //      convolution does not sweep that tensor for its mean and variance: the convolution's epilogue leaves moments behind,
+  //      a small kernel merges them, and the GroupNorm (or the layout pass) reads (mean, 1 / std) from there.
   for (auto& L : m->layers) { L.gn_emit_for = -1; L.gn_stats_from = -1; }
   for (int li = 0; li < nl; ++li) {
     LayerRT& G = m->layers[li];
@@ -1205,7 +1205,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     if (G.skip) {  // folded: the statistics are taken over the consuming convolution's (possibly pre-upsample) input
       for (int ci = 0; ci < nl; ++ci)
         if (m->layers[ci].lt == LT::Conv2d && !m->layers[ci].skip && m->layers[ci].pre_norm == li) xin = m->layers[ci].in_v[0];
-    } else {
+    } else if (groupnorm_takes_stats(batch, G.ch, G.h * G.w, G.d.num_groups)) {
       xin = G.in_v[0];
     }
     if (xin < 0) continue;
@@ -1213,9 +1213,9 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     const TensorV& xt = m->tensors[xr];
     if (xt.producer < 0) continue;
     LayerRT& P = m->layers[xt.producer];
-    if (P.lt != LT::Conv2d || P.skip || P.res_up || P.gn_emit_for >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
-    if (!conv_can_emit_gn(batch, P.d.in_channels, P.d.out_channels, P.h, P.w, P.d.kernel, P.d.stride, P.d.padding, G.d.num_groups,
-                          P.d.activation ? MIMIR_B200_ELT_RELU : P.fused_act))
+    if (P.lt != LT::Conv2d || P.skip || P.gn_emit_for >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
+    if (!conv_can_emit_gn(batch, P.d.in_channels, P.d.out_channels, P.h, P.w, P.d.kernel, P.d.stride, P.d.padding, m->precision, G.d.num_groups,
+                          P.d.activation ? MIMIR_B200_ELT_RELU : P.fused_act, P.res_up))
       continue;
     P.gn_emit_for = li;
     G.gn_stats_from = xt.producer;
@@ -1277,7 +1277,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
           L.ws_bytes = conv_ws_bytes(batch, L.d.in_channels, L.h, L.w, L.d.kernel, L.d.stride, L.d.padding, m->precision);
           if (L.pre_norm >= 0) L.ws_bytes += conv_prenorm_bytes(batch, m->layers[L.pre_norm].d.num_groups);
           if (L.gn_emit_for >= 0)
-            L.ws_bytes += conv_gn_emit_bytes(batch, L.d.out_channels, L.h, L.w, L.d.padding, m->layers[L.gn_emit_for].d.num_groups);
+            L.ws_bytes += conv_gn_emit_bytes(batch, L.d.in_channels, L.d.out_channels, L.h, L.w, L.d.kernel, L.d.padding, m->precision);
           flops += 2ull * batch * L.oh * L.ow * k * L.d.out_channels;
           break;
         }
