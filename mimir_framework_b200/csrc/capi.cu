@@ -439,6 +439,26 @@ bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int strid
   return static_cast<long long>(batch) * oc * h * w * 4 >= (32ll << 20) && (res_up || gemm_takes_spatial(g));
 }
 
+size_t conv_normed_residual_bytes(int batch, int oc, int groups) { return conv_prenorm_bytes(batch, groups) + align256(static_cast<size_t>(batch) * oc * sizeof(float4)); }
+
+// A layout pass over the tensor less; the ring costs a few per cent of the tiles (114^2 for 112^2: 3.5 %, 34^2 for 32^2: 13 %).  64 images
+// of 112^2: 136 us with 128 channels, 70 with 64.
+bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
+  if (ks != 1 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
+  GemmArgs g;
+  return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) && h >= 32 && w >= 32 && gemm_takes_spatial(g);
+}
+
+// The normalised tensor then never exists: where it is larger than L2's reach the epilogue's arithmetic (a skip layer of 1 x 1 waits for
+// memory anyway) costs less than writing it and reading it back.  64 images of 112^2, by launch: a
+// sweep of 281 us and a 1 x 1 convolution 128 -> 256 of 424 -> 625 in all; 64 -> 128 133 + 220 -> 327.
+bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
+  if (oc % 32 != 0 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
+  GemmArgs g;
+  if (!shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g)) return false;
+  return static_cast<long long>(batch) * oc * h * w * 4 >= (32ll << 20) && gemm_takes_spatial(g);
+}
+
 size_t conv_ws_bytes(int batch, int ic, int h, int w, int ks, int stride, int pad, int precision) {
   int ap, wp;
   precision_planes(precision, &ap, &wp);
@@ -468,15 +488,16 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
   if (oh <= 0 || ow <= 0) return fail(MIMIR_B200_E_INVALID, "Conv2d: empty output");
   const int ohw = oh * ow, k = e.ic * e.ks * e.ks;
   if (e.residual_up && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: an upsampled residual needs the shifted-GEMM path");
+  if (e.res_groups > 0 && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: a normalised residual needs the shifted-GEMM path");
   if (e.in_up && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: an upsampled input needs the shifted-GEMM path");
-  if (e.w_f32 != nullptr && e.pre_groups == 0 && !e.in_up && !e.residual_up && conv_small_oc_supported(e.oc, e.ks, e.stride, e.pad, e.h, e.w, e.batch, e.activation))
+  if (e.w_f32 != nullptr && e.pre_groups == 0 && e.res_groups == 0 && !e.in_up && !e.residual_up && conv_small_oc_supported(e.oc, e.ks, e.stride, e.pad, e.h, e.w, e.batch, e.activation))
     return launch_conv_small_oc(e.x, e.w_f32, e.y, e.residual, e.batch, e.ic, e.oc, e.h, e.w, e.ks, e.pad, e.activation, st);
   if (conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) {
     // NCHW fp32 -> zero-padded NHWC planes, then one GEMM that walks the taps as shifted row offsets
     const long long rows = static_cast<long long>(e.batch) * (e.h + 2 * e.pad) * (e.w + 2 * e.pad);
     if (rows > 0x7fffffffLL) return fail(MIMIR_B200_E_UNSUPPORTED, "Conv2d: batch too large for one launch");
     PreNorm pre;
-    const size_t planes_bytes = align256(static_cast<size_t>(ap) * rows * e.ic * sizeof(__nv_bfloat16));
+    const size_t planes_bytes = e.planes != nullptr ? 0 : align256(static_cast<size_t>(ap) * rows * e.ic * sizeof(__nv_bfloat16));
     if (e.pre_groups > 0) {
       // statistics live behind the operand planes in the workspace (unless the producer's epilogue delivered them)
       float* stats = reinterpret_cast<float*>(static_cast<uint8_t*>(e.ws) + planes_bytes);
@@ -485,9 +506,14 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
         MB_TRY(launch_groupnorm_stats(e.x, stats, e.batch, e.ic, e.in_up ? (e.h >> 1) * (e.w >> 1) : e.h * e.w, e.pre_groups, e.pre_eps, st));
       pre.stats = e.pre_stats ? e.pre_stats : stats; pre.gamma = e.pre_gamma; pre.beta = e.pre_gamma ? e.pre_beta : nullptr; pre.groups = e.pre_groups; pre.act = e.pre_act;
     }
-    MB_TRY(launch_nchw_to_padded_nhwc_split(e.x, static_cast<__nv_bfloat16*>(e.ws), e.batch, e.ic, e.h, e.w, e.pad, ap, st, pre, e.in_up));
     GemmArgs g;
-    g.a = static_cast<const __nv_bfloat16*>(e.ws);
+    if (e.planes != nullptr) {
+      g.a = e.planes;
+      g.conv_src_pad = e.planes_pad;
+    } else {
+      MB_TRY(launch_nchw_to_padded_nhwc_split(e.x, static_cast<__nv_bfloat16*>(e.ws), e.batch, e.ic, e.h, e.w, e.pad, ap, st, pre, e.in_up));
+      g.a = static_cast<const __nv_bfloat16*>(e.ws);
+    }
     g.w = e.w_split;
     g.a_planes = ap; g.w_planes = wp; g.w_scale = e.w_scale; g.w_ready = e.w_ready;
     g.m = static_cast<int>(rows); g.n = e.oc; g.k = k;
@@ -497,8 +523,18 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     g.residual_up = e.residual_up;
     g.ldo = e.oc;
     g.conv_ks = e.ks; g.conv_c = e.ic; g.conv_pad = e.pad; g.conv_h = e.h; g.conv_w = e.w;
+    uint8_t* rest = static_cast<uint8_t*>(e.ws) + planes_bytes + (e.pre_groups > 0 ? conv_prenorm_bytes(e.batch, e.pre_groups) : 0);
+    if (e.res_groups > 0) {
+      float* stats = reinterpret_cast<float*>(rest);
+      float4* coef = reinterpret_cast<float4*>(rest + conv_prenorm_bytes(e.batch, e.res_groups));
+      if (e.res_stats == nullptr) MB_TRY(launch_groupnorm_stats(e.residual, stats, e.batch, e.oc, e.h * e.w, e.res_groups, e.res_eps, st));
+      MB_TRY(launch_gn_coefs(e.res_stats ? e.res_stats : stats, e.res_gamma, e.res_beta, coef, e.batch, e.oc, e.res_groups, st));
+      g.res_coef = coef;
+      g.res_act = e.res_act;
+      rest += conv_normed_residual_bytes(e.batch, e.oc, e.res_groups);
+    }
     if (e.gn_stats_out != nullptr) {
-      g.gn_part = reinterpret_cast<float4*>(static_cast<uint8_t*>(e.ws) + planes_bytes + (e.pre_groups > 0 ? conv_prenorm_bytes(e.batch, e.pre_groups) : 0));
+      g.gn_part = reinterpret_cast<float4*>(rest);
       MB_TRY(launch_gemm(g, st));
       return launch_conv_gn_stats(g, e.gn_stats_out, e.gn_groups, e.gn_eps, st);
     }

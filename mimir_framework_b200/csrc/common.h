@@ -207,6 +207,7 @@ struct GemmArgs {
   // Shifted-GEMM convolution (conv_ks > 0): `a` is the zero-padded NHWC activation [samples*(h+2p)*(w+2p)][conv_c],
   // m counts padded-grid rows, k = conv_ks^2 * conv_c ordered (tap, channel), output is NCHW [samples][n][h][w].
   int conv_ks = 0, conv_c = 0, conv_pad = 0, conv_h = 0, conv_w = 0;
+  int conv_src_pad = 0;              // 1 x 1 kernels (conv_gemm.cu only): `a` has a ring of so many pixels all the same (m counts none of it)
   // Grouped form (a_group_rows > 0, plain row-major GEMM only): the rows of `a` come in groups of a_group_rows, and group g
   // multiplies the w rows [g * w_group_rows, g * w_group_rows + n): a block-diagonal batch of small GEMMs in one launch
   // (attention scores Q_b K_b^T and P_b V_b per sample).  `w` then holds w_rows_total rows.
@@ -215,6 +216,10 @@ struct GemmArgs {
   // Shifted convolutions (conv_gemm.cu only): moments of the values stored, for the GroupNorm that reads this output;
   // conv_gemm_gn_bytes() of scratch, merged by launch_conv_gn_stats
   float4* gn_part = nullptr;
+  // Shifted convolutions (conv_gemm.cu only): the residual is a GroupNorm's INPUT, normalised on its way: (mean, gamma / std, beta, -) per
+  // (sample, channel) from launch_gn_coefs, then SiLU where res_act says so
+  const float4* res_coef = nullptr;
+  int res_act = -1;
   // The weight planes were complete before the launches of this call began (a planned model's): the kernel may fetch them
   // before the kernel ahead of it in the stream has finished.
   bool w_ready = false;
@@ -345,6 +350,7 @@ int norm_scratch_selftest_gave_up(unsigned tickets, int flag, cudaStream_t st);
 int launch_groupnorm(const float* x, const float* gamma, const float* beta, float* y, int batch, int ch, int hw,
                      int groups, float eps, int act, const float* residual, cudaStream_t st);
 int launch_softmax(const float* x, float* y, int batch, int64_t n, int log_softmax, cudaStream_t st);
+int launch_gn_coefs(const float* stats, const float* gamma, const float* beta, float4* coef, int batch, int ch, int groups, cudaStream_t st);
 // stats[(sample * groups + g) * 2 + {0, 1}] = mean, 1 / sqrt(var + eps) of each GroupNorm slab
 int launch_groupnorm_stats(const float* x, float* stats, int batch, int ch, int hw, int groups, float eps, cudaStream_t st);
 bool groupnorm_takes_stats(int batch, int ch, int hw, int groups);

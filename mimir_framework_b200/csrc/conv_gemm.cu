@@ -33,6 +33,7 @@ constexpr int CG_THREADS = 352;
 constexpr int CG_N = 256;                      // pixels of a tile: 16 x 16 or, for 1 x 1 kernels, 256 of the flattened image; or half of that
 constexpr int CG_M = 128;                      // output channels of a tile
 constexpr int CG_EPI = 8 * 32 * 33 * 4;
+constexpr int CG_COEF = 8 * 32 * 16;
 constexpr int CG_MAX_RING = 16;
 constexpr int CG_SMEM_MAX = 232448;
 
@@ -66,6 +67,14 @@ __device__ __forceinline__ float sum8(float (&a)[8], int lane) {
   return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
+// What only some forms need: an argument of its own (with these among ConvGemmParams the compiler took 168 registers for every form and the
+// plain one lost 10 % of a 1 x 1 convolution)
+struct ConvFormParams {
+  int flat_pad, flat_w, flat_iw, flat_ih;      // CG_FLAT: the line of padded images flat_w wide, whose inside is flat_ih x flat_iw
+  const float4* res_coef;                      // CG_RN: see GemmArgs
+  int res_silu;
+};
+
 struct ConvTile { int oc0, n, y0, x0; };
 __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) {  // output-channel tiles fastest: they share activations in L2
   ConvTile c;
@@ -79,10 +88,15 @@ __device__ __forceinline__ ConvTile conv_tile(const ConvGemmParams& p, int t) { 
 }
 
 // BK: channels of a K block, 32 (64-byte swizzle rows) or 64 (128-byte rows)
-template <int AP, int WP, int BK, int GN>
+// FORM: what the epilogue does beside, each in a form of its own (the plain one runs in 128 registers, which the others leave)
+enum : int { CG_PLAIN = 0, CG_GN = 1 /* moments of the result for the GroupNorm that reads it */, CG_RN = 2 /* the residual is a GroupNorm's input */,
+             CG_FLAT = 4 /* the line of a padded image */ };
+template <int AP, int WP, int BK, int FORM>
 __global__ void __launch_bounds__(CG_THREADS, 1)
-conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const ConvGemmParams p) {
+conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const ConvGemmParams p,
+                 const ConvFormParams f) {
   constexpr int W_TILE = CG_M * BK * 2;
+  constexpr bool GN = (FORM & CG_GN) != 0, RN = (FORM & CG_RN) != 0, FLAT = (FORM & CG_FLAT) != 0;
   extern __shared__ __align__(1024) uint8_t cg_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(cg_smem_raw) + 1023) & ~uintptr_t(1023));
   const int a_plane = p.a_stage_bytes / AP;                                   // halo tile of one plane
@@ -213,8 +227,9 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // epilogue: TMEM lane = output channel, column = pixel (16 to a row)
     const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
     float* tbuf = epi + ew * (32 * 33);
+    float4* coef = reinterpret_cast<float4*>(epi + CG_EPI / 4) + ew * 32;  // RN: of this warp's 32 channels
     const int chunks = p.px / 64;  // of 32 pixels, in each half of the tile
-    const long long hw = static_cast<long long>(p.h) * p.w;
+    const long long hw = FLAT ? static_cast<long long>(f.flat_ih) * f.flat_iw : static_cast<long long>(p.h) * p.w;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = static_cast<int>(blockIdx.x); t < p.num_tiles; t += static_cast<int>(gridDim.x)) {
@@ -225,6 +240,11 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int px = (half * chunks + ci) * 32 + lane, y = c.y0 + (px >> p.tw_log), x = c.x0 + (px & ((1 << p.tw_log) - 1));
         in = y < p.h && x < p.w;
         o0 = (static_cast<long long>(c.n) * p.oc + oc0) * hw + static_cast<long long>(y) * p.w + x;
+        if (FLAT) {
+          const int iy = x / f.flat_w - f.flat_pad, ix = x % f.flat_w - f.flat_pad;
+          in = static_cast<unsigned>(iy) < static_cast<unsigned>(f.flat_ih) && static_cast<unsigned>(ix) < static_cast<unsigned>(f.flat_iw);
+          o0 = (static_cast<long long>(c.n) * p.oc + oc0) * hw + static_cast<long long>(iy) * f.flat_iw + ix;
+        }
       };
       // The residual of a chunk is requested one chunk ahead, the first one's before the accumulators are waited for: a 1 x 1 skip
       // layer reads and writes more than it multiplies, and its loads would each wait a full memory latency.
@@ -245,6 +265,11 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
       };
       if (p.residual != nullptr && nch > 0) request(0);
+      if (RN && nch > 0) {
+        __syncwarp();
+        coef[lane] = __ldg(f.res_coef + static_cast<long long>(c.n) * p.oc + oc0 + lane);
+        __syncwarp();
+      }
       int ok = 1;
       if (lane == 0) ok = mbar_wait(&acc_full[acc], acc_phase, &abort_flag, p.err_word, 58) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -279,8 +304,23 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.activation);
           }
           if (p.residual != nullptr) {
+            if (RN) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += q[j];
+              for (int j = 0; j < 32; ++j) {
+                const float4 k = coef[j];  // (the same for every lane)
+                q[j] = fmaf(q[j] - k.x, k.y, k.z);
+              }
+              if (f.res_silu) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = fmaf(q[j], logistic(q[j]), v[j]);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] += q[j];
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += q[j];
+            }
             if (ci + 1 < chunks) request(ci + 1);
           }
           if (in) {
@@ -343,12 +383,12 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 }
 
 // Image and tile shape of a launch.  A 1 x 1 kernel sees the image as one line (tiles of 256 consecutive pixels, whole 128-byte
-// lines in every channel plane: with 16-pixel rows its scattered 64-byte stores held DRAM at 4 TB/s).  Otherwise 16 x 16 (32 x 8 where
+// lines in every channel plane; the line of the padded image where that is what the planes hold: with 16-pixel rows its scattered 64-byte stores held DRAM at 4 TB/s).  Otherwise 16 x 16 (32 x 8 where
 // the width allows whole lines measured the same: there the MMAs, not the stores, set the pace).
 struct ConvShape { int h, w, tw_log, tiles_x, tiles_y; };
 ConvShape conv_shape(const GemmArgs& g, int px) {
   ConvShape s{g.conv_h, g.conv_w, 4, 0, 0};
-  if (g.conv_ks == 1) { s.w = g.conv_h * g.conv_w; s.h = 1; s.tw_log = px == CG_N ? 8 : 7; }
+  if (g.conv_ks == 1) { s.w = (g.conv_h + 2 * g.conv_src_pad) * (g.conv_w + 2 * g.conv_src_pad); s.h = 1; s.tw_log = px == CG_N ? 8 : 7; }
   const int tw = 1 << s.tw_log, th = px >> s.tw_log;
   s.tiles_x = (s.w + tw - 1) / tw;
   s.tiles_y = (s.h + th - 1) / th;
@@ -422,7 +462,7 @@ __global__ void __launch_bounds__(128) conv_gn_stats_kernel(const float4* __rest
   }
 }
 
-template <int AP, int WP, int BK, int GN>
+template <int AP, int WP, int BK, int FORM>
 int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   const int ks = g.conv_ks, pad = g.conv_pad;
   ConvGemmParams p;
@@ -437,7 +477,7 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   p.num_tiles = p.batch * p.tiles_y * p.tiles_x * p.tiles_o;
   const int rows = th + ks - 1;
   p.a_stage_bytes = AP * tw * rows * BK * 2;
-  const int ring = CG_SMEM_MAX - CG_EPI - 1024 - 1024;  // (less the barriers)
+  const int ring = CG_SMEM_MAX - CG_EPI - (FORM & CG_RN ? CG_COEF : 0) - 1024 - 1024;  // (less the barriers)
   p.a_stages = 3;
   p.w_stages = (ring - p.a_stages * p.a_stage_bytes) / (CG_M * BK * 2);
   if (p.w_stages < 3 * WP) {
@@ -449,20 +489,21 @@ int launch_conv_t(const GemmArgs& g, cudaStream_t st) {
   p.acc_scale = gemm_acc_scale(g);
   p.f16 = plane_format() == PLANES_F16 ? 1 : 0;
   p.gn_part = g.gn_part;
+  const ConvFormParams f{g.conv_src_pad, g.conv_w + 2 * g.conv_src_pad, g.conv_w, g.conv_h, g.res_coef, g.res_act == MIMIR_B200_ELT_SILU ? 1 : 0};
   p.err_word = ctx().dev_error_word;
   CUtensorMap map_a, map_w;
   MB_TRY(make_image_map(&map_a, g.a, AP, p.batch, hp, wp, g.conv_c, BK, tw, rows));
   MB_TRY(make_plane_map(&map_w, g.w, WP, g.n, round_up(g.k, 64), BK, CG_M));
-  const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * (CG_M * BK * 2) + CG_EPI + 1024;
+  const size_t smem = static_cast<size_t>(p.a_stages) * p.a_stage_bytes + static_cast<size_t>(p.w_stages) * (CG_M * BK * 2) + CG_EPI + (FORM & CG_RN ? CG_COEF : 0) + 1024;
   static PerDeviceOnce attr_once;
   MB_TRY(attr_once.run([&]() -> int {
-    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP, BK, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
+    MB_CUDA(cudaFuncSetAttribute(conv_gemm_kernel<AP, WP, BK, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM_MAX - 1024));
     return MIMIR_B200_OK;
   }));
   const int sms = ctx().sm_count;
   GemmProfile prof(st);
   MB_TRY(prof.begin());
-  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP, BK, GN>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p));
+  MB_TRY(launch_pdl(conv_gemm_kernel<AP, WP, BK, FORM>, dim3(static_cast<unsigned>(p.num_tiles < sms ? p.num_tiles : sms)), dim3(CG_THREADS), smem, st, 1, map_a, map_w, p, f));
   MB_TRY(prof.end());
   count_launch();
   return MIMIR_B200_OK;
@@ -507,11 +548,16 @@ int launch_conv_gn_stats(const GemmArgs& g, float* stats, int groups, float eps,
 
 template <int AP, int WP>
 int launch_conv_planes(const GemmArgs& g, bool wide, cudaStream_t st) {
-  if (g.gn_part != nullptr) {
-    if (g.n % 32 != 0) return fail(MIMIR_B200_E_INVALID, "conv: GroupNorm moments need output channels in whole chunks of 32");
-    return wide ? launch_conv_t<AP, WP, 64, 1>(g, st) : launch_conv_t<AP, WP, 32, 1>(g, st);
+  const int form = (g.gn_part != nullptr ? CG_GN : 0) | (g.res_coef != nullptr ? CG_RN : 0) | (g.conv_src_pad > 0 ? CG_FLAT : 0);
+  if ((form & (CG_GN | CG_RN)) != 0 && g.n % 32 != 0) return fail(MIMIR_B200_E_INVALID, "conv: this form needs output channels in whole chunks of 32");
+  switch (form) {
+    case CG_PLAIN: return wide ? launch_conv_t<AP, WP, 64, CG_PLAIN>(g, st) : launch_conv_t<AP, WP, 32, CG_PLAIN>(g, st);
+    case CG_GN: return wide ? launch_conv_t<AP, WP, 64, CG_GN>(g, st) : launch_conv_t<AP, WP, 32, CG_GN>(g, st);
+    case CG_RN: return wide ? launch_conv_t<AP, WP, 64, CG_RN>(g, st) : launch_conv_t<AP, WP, 32, CG_RN>(g, st);
+    case CG_FLAT: return wide ? launch_conv_t<AP, WP, 64, CG_FLAT>(g, st) : launch_conv_t<AP, WP, 32, CG_FLAT>(g, st);
+    case CG_RN | CG_FLAT: return wide ? launch_conv_t<AP, WP, 64, CG_RN | CG_FLAT>(g, st) : launch_conv_t<AP, WP, 32, CG_RN | CG_FLAT>(g, st);
+    default: return fail(MIMIR_B200_E_INVALID, "conv: no such form of the epilogue");
   }
-  return wide ? launch_conv_t<AP, WP, 64, 0>(g, st) : launch_conv_t<AP, WP, 32, 0>(g, st);
 }
 
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st) {

@@ -20,6 +20,13 @@ __device__ __forceinline__ float gelu_ref(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
   return __fmul_rn(x, r);  // (not contracted with a residual that follows)
 }
+// 1 / (1 + exp(-x)) in four instructions, two of them on the special-function unit: 2^-21 of its value for x above -87, 0 below
+__device__ __forceinline__ float logistic(float x) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.442695041f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return r;
+}
 __device__ __forceinline__ float apply_act(float v, int act) {
   switch (act) {
     case MIMIR_B200_ELT_GELU: return gelu_ref(v);

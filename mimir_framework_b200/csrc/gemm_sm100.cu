@@ -1119,10 +1119,10 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st) {
   }
   const bool pairs = g.conv_ks == 0 && g.out_nchw_hw <= 0 && takes_pairs(g);
   const int bk = env_int("MIMIR_B200_GEMM_BK", (g.a_planes + g.w_planes <= 3 || pairs) ? 64 : 32);
-  // planned for the spatial-tile kernel (conv_takes_residual_up, conv_can_emit_gn): the others read a residual of the output's own
-  // shape and leave no statistics
-  if (g.residual_up || g.gn_part != nullptr) {
-    if (conv_gemm_cycles(g) >= 1e30) return fail(MIMIR_B200_E_INVALID, "gemm: an upsampled residual and GroupNorm statistics need the spatial-tile kernel");
+  // planned for the spatial-tile kernel (conv_takes_residual_up, conv_can_emit_gn, conv_takes_normed_residual, conv_takes_padded_planes): the
+  // others add a residual of the output's own shape as it is, leave no statistics and read planes of their own
+  if (g.residual_up || g.gn_part != nullptr || g.res_coef != nullptr || g.conv_src_pad > 0) {
+    if (conv_gemm_cycles(g) >= 1e30) return fail(MIMIR_B200_E_INVALID, "gemm: this residual, GroupNorm statistics or planes with a ring need the spatial-tile kernel");
     return launch_conv_gemm(g, st);
   }
   const GemmChoice c = choose_form(g);

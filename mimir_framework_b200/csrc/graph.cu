@@ -132,6 +132,9 @@ struct LayerRT {
   bool emit_f32 = true;
   bool read_split = false;            // Linear reads the producer's planes
   int res_v = -1;                     // residual tensor folded in from a following Add
+  int planes_from = -1;               // Conv2d: index of the Conv2d layer whose operand planes (of the same tensor) this one reads
+  int ws_until = -1;                  // Conv2d: the place in the order of execution up to which its workspace is kept for that
+  int res_norm = -1;                  // Conv2d: index of the GroupNorm layer whose INPUT res_v is (the epilogue normalises)
   int pre_norm = -1;                  // Conv2d: index of the GroupNorm layer applied while its operand planes are laid out
   bool res_up = false;                // Conv2d: res_v is the INPUT of a 2 x 2 nearest upsample that the epilogue applies
   std::vector<int> add_v;             // Embedding: tensors of the Adds folded into it (graph inputs), in layer order
@@ -768,7 +771,8 @@ bool attention_streams_weights(const LayerRT& L, int batch) {
   return batch <= 16 && L.w_f32 && L.w_count >= static_cast<size_t>(4) * L.embed * L.embed;
 }
 
-int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch) {
+// keep_planes: convolutions may hold on to their operand planes for a later one of the same tensor
+int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch, bool keep_planes = true) {
   if (batch <= 0) return fail(MIMIR_B200_E_INVALID, "plan: batch must be positive");
   if (batch % m->pipeline != 0)
     return fail(MIMIR_B200_E_INVALID, "plan: batch %d is not a multiple of the %d pipeline micro-batches", batch, m->pipeline);
@@ -799,7 +803,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     LayerRT& L = m->layers[li];
     L.in_v.clear();
     L.out_v = -1;
-    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false; L.res_up = false; L.add_v.clear();
+    L.skip = false; L.fused_act = -1; L.emit_split = false; L.emit_f32 = true; L.read_split = false; L.res_v = -1; L.res_norm = -1; L.planes_from = -1; L.ws_until = -1; L.pre_norm = -1; L.pre_ln = -1; L.in_up = false; L.res_up = false; L.add_v.clear();
     L.ws_off = 0; L.ws_bytes = 0;
     std::vector<std::string> names = L.inputs;
     if (names.empty()) names.push_back("x");
@@ -1069,6 +1073,56 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       U.skip = true;
     }
   }
+  // ---- fusion 1g: a GroupNorm (+ SiLU) that is only added to a convolution's result (a block whose skip connection is a convolution): that
+  //      convolution's epilogue reads the GroupNorm's input and normalises it; the normalised tensor never exists ----
+  for (int li = 0; li < nl && fuse_gn; ++li) {
+    LayerRT& P = m->layers[li];
+    if (P.lt != LT::GroupNorm || P.skip || P.res_v >= 0) continue;
+    if (P.fused_act >= 0 && P.fused_act != MIMIR_B200_ELT_SILU) continue;
+    const int pv = P.out_v, xin = P.in_v[0];
+    TensorV& pt = m->tensors[pv];
+    if (pt.alias_of >= 0 || pv == out_root || total_consumers(pv) != 1 || pt.consumers.size() != 1) continue;
+    const int ci = pt.consumers[0];
+    LayerRT& C = m->layers[ci];
+    if (C.lt != LT::Conv2d || C.skip || C.res_v != pv || C.res_up || C.in_v[0] == pv || C.d.out_channels != P.ch || C.h != P.h || C.w != P.w) continue;
+    if (m->tensors[pv].n != m->tensors[C.out_v].n || m->tensors[xin].n != m->tensors[pv].n) continue;
+    if (!conv_takes_normed_residual(batch, C.d.in_channels, C.d.out_channels, C.h, C.w, C.d.kernel, C.d.stride, C.d.padding, m->precision,
+                                    C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act))
+      continue;
+    C.res_norm = li;
+    C.res_v = xin;
+    for (int& c : m->tensors[xin].consumers)
+      if (c == li) c = ci;
+    pt.consumers.clear();
+    pt.want_f32 = false;
+    pt.producer = -2;  // dead
+    P.skip = true;
+  }
+  // ---- fusion 1h: a 1 x 1 convolution of a tensor that another convolution reads as it is before it (the skip connection of a block): the
+  //      planes that one laid out are kept for it ----
+  bool kept_planes = false;
+  {
+    auto reads_plain = [&](const LayerRT& C) {
+      return C.lt == LT::Conv2d && !C.skip && C.pre_norm < 0 && !C.in_up && conv_uses_shifted(C.d.in_channels, C.d.kernel, C.d.stride, C.d.padding) &&
+             !conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act);
+    };
+    for (int p = 0; p < nl && keep_planes && fuse_gn; ++p) {
+      LayerRT& S = m->layers[m->order[p]];
+      if (!reads_plain(S) || !conv_takes_padded_planes(batch, S.d.in_channels, S.d.out_channels, S.h, S.w, S.d.kernel, S.d.stride, S.d.padding, m->precision,
+                                                       S.d.activation ? MIMIR_B200_ELT_RELU : S.fused_act))
+        continue;
+      for (int q = p - 1; q >= 0; --q) {
+        LayerRT& E = m->layers[m->order[q]];
+        if (!reads_plain(E) || E.planes_from >= 0 || E.d.padding < 1 || E.d.in_channels != S.d.in_channels || E.h != S.h || E.w != S.w ||
+            root_of(m->tensors, E.in_v[0]) != root_of(m->tensors, S.in_v[0]))
+          continue;
+        S.planes_from = m->order[q];
+        E.ws_until = std::max(E.ws_until, p);
+        kept_planes = true;
+        break;
+      }
+    }
+  }
   // ---- fusion 1f: a token-wise LayerNorm whose only consumer is a Linear of a few rows, or a decode step's attention block:
   //      the consumer normalises while it stages its rows (skinny_cluster.cu) ----
   for (int li = 0; li < nl; ++li) {
@@ -1202,9 +1256,10 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     LayerRT& G = m->layers[li];
     if (G.lt != LT::GroupNorm) continue;
     int xin = -1;
-    if (G.skip) {  // folded: the statistics are taken over the consuming convolution's (possibly pre-upsample) input
+    if (G.skip) {  // folded: the statistics are taken over what the convolution reads in its place (its possibly pre-upsample input, its residual)
       for (int ci = 0; ci < nl; ++ci)
         if (m->layers[ci].lt == LT::Conv2d && !m->layers[ci].skip && m->layers[ci].pre_norm == li) xin = m->layers[ci].in_v[0];
+        else if (m->layers[ci].lt == LT::Conv2d && !m->layers[ci].skip && m->layers[ci].res_norm == li) xin = m->layers[ci].res_v;
     } else if (groupnorm_takes_stats(batch, G.ch, G.h * G.w, G.d.num_groups)) {
       xin = G.in_v[0];
     }
@@ -1213,7 +1268,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     const TensorV& xt = m->tensors[xr];
     if (xt.producer < 0) continue;
     LayerRT& P = m->layers[xt.producer];
-    if (P.lt != LT::Conv2d || P.skip || P.gn_emit_for >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
+    if (P.lt != LT::Conv2d || P.skip || P.gn_emit_for >= 0 || P.res_norm >= 0 || P.planes_from >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
     if (!conv_can_emit_gn(batch, P.d.in_channels, P.d.out_channels, P.h, P.w, P.d.kernel, P.d.stride, P.d.padding, m->precision, G.d.num_groups,
                           P.d.activation ? MIMIR_B200_ELT_RELU : P.fused_act, P.res_up))
       continue;
@@ -1275,7 +1330,9 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
         case LT::Conv2d: {
           const int k = L.d.in_channels * L.d.kernel * L.d.kernel;
           L.ws_bytes = conv_ws_bytes(batch, L.d.in_channels, L.h, L.w, L.d.kernel, L.d.stride, L.d.padding, m->precision);
+          if (L.planes_from >= 0) L.ws_bytes = 0;
           if (L.pre_norm >= 0) L.ws_bytes += conv_prenorm_bytes(batch, m->layers[L.pre_norm].d.num_groups);
+          if (L.res_norm >= 0) L.ws_bytes += conv_normed_residual_bytes(batch, L.d.out_channels, m->layers[L.res_norm].d.num_groups);
           if (L.gn_emit_for >= 0)
             L.ws_bytes += conv_gn_emit_bytes(batch, L.d.in_channels, L.d.out_channels, L.h, L.w, L.d.kernel, L.d.padding, m->precision);
           flops += 2ull * batch * L.oh * L.ow * k * L.d.out_channels;
@@ -1289,9 +1346,11 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       }
       if (L.ws_bytes) {
         L.ws_off = sim.alloc(L.ws_bytes);
-        sim.release(L.ws_off, L.ws_bytes);
+        if (L.ws_until <= p) sim.release(L.ws_off, L.ws_bytes);
       }
     }
+    for (LayerRT& E : m->layers)
+      if (E.ws_until == p) sim.release(E.ws_off, E.ws_bytes);
     for (int v = 0; v < nt; ++v) {
       const TensorV& t = m->tensors[v];
       // In a pipelined plan the slots of the graph inputs are never handed on: the copy-in of micro-batch c + 2 may then
@@ -1331,12 +1390,20 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     m->arena = m->arena2 = nullptr;
     m->arena_bytes = 0;
   }
+  // (where the budget has no room for planes that are kept, the plan is made without)
   if (!m->arena) {
-    MB_TRY(dev_alloc(reinterpret_cast<void**>(&m->arena), need, "activation arena"));
+    const int s1 = dev_alloc(reinterpret_cast<void**>(&m->arena), need, "activation arena");
+    if (s1 != MIMIR_B200_OK) return kept_planes ? plan_model(m, inputs, n_inputs, full_batch, false) : s1;
     m->arena_bytes = need;
   }
   if (m->pipeline > 1 && !m->arena2) {
     int s2 = dev_alloc(reinterpret_cast<void**>(&m->arena2), m->arena_bytes, "activation arena (second pipeline buffer)");
+    if (s2 != MIMIR_B200_OK && kept_planes) {
+      dev_free(m->arena, m->arena_bytes);
+      m->arena = nullptr;
+      m->arena_bytes = 0;
+      return plan_model(m, inputs, n_inputs, full_batch, false);
+    }
     if (s2 != MIMIR_B200_OK) return s2;
   }
   if (m->pipeline == 1 && m->arena2) {
@@ -1441,6 +1508,11 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
         e.stride = d.stride; e.pad = d.padding; e.precision = m->precision;
         e.activation = d.activation ? MIMIR_B200_ELT_RELU : L.fused_act;
         e.x = f32p(L.in_v[0]); e.w_split = L.w_split; e.w_f32 = L.w_f32; e.w_scale = L.w_scale; e.w_ready = true; e.y = f32p(L.out_v); e.ws = ws;
+        if (L.planes_from >= 0) {
+          const LayerRT& E = m->layers[L.planes_from];
+          e.planes = reinterpret_cast<const __nv_bfloat16*>(arena + E.ws_off);
+          e.planes_pad = E.d.padding;
+        }
         if (L.res_v >= 0) e.residual = f32p(L.res_v);
         e.residual_up = L.res_up;
         if (L.pre_norm >= 0) {
@@ -1451,6 +1523,15 @@ int run_layers(MimirB200Model* m, int batch, const Bound& bnd, cudaStream_t st, 
           e.pre_eps = G.d.eps;
           e.pre_act = G.fused_act;
           if (G.gn_stats_from >= 0) e.pre_stats = reinterpret_cast<const float*>(arena + m->layers[G.gn_stats_from].gn_stats_off);
+        }
+        if (L.res_norm >= 0) {
+          const LayerRT& G = m->layers[L.res_norm];
+          e.res_groups = G.d.num_groups;
+          e.res_gamma = G.d.affine ? G.w_f32 : nullptr;
+          e.res_beta = (G.d.affine && G.d.use_bias) ? G.w_f32 + G.ch : nullptr;
+          e.res_eps = G.d.eps;
+          e.res_act = G.fused_act;
+          if (G.gn_stats_from >= 0) e.res_stats = reinterpret_cast<const float*>(arena + m->layers[G.gn_stats_from].gn_stats_off);
         }
         e.in_up = L.in_up ? 1 : 0;
         if (L.gn_emit_for >= 0) {

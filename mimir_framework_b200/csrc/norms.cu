@@ -1148,6 +1148,25 @@ int launch_groupnorm_apply(const float* x, const float* stats, const float* gamm
   return launch_sweep_rows<FAM_MEANVAR>(p, st);
 }
 
+namespace {
+__global__ void __launch_bounds__(256) gn_coefs_kernel(const float* __restrict__ stats, const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                       float4* __restrict__ coef, int total, int ch, int cpg) {
+  const int i = static_cast<int>(blockIdx.x) * 256 + static_cast<int>(threadIdx.x);
+  if (i >= total) return;
+  const int c = i % ch;
+  const float* s = stats + 2 * (i / cpg);  // (channels are whole groups: i / cpg counts them over the samples)
+  coef[i] = make_float4(s[0], s[1] * (gamma != nullptr ? __ldg(gamma + c) : 1.0f), beta != nullptr ? __ldg(beta + c) : 0.0f, 0.0f);
+}
+}  // namespace
+int launch_gn_coefs(const float* stats, const float* gamma, const float* beta, float4* coef, int batch, int ch, int groups, cudaStream_t st) {
+  if (groups <= 0 || ch % groups != 0) return fail(MIMIR_B200_E_INVALID, "GroupNorm: channels must be divisible by num_groups");
+  const int total = batch * ch;
+  gn_coefs_kernel<<<(total + 255) / 256, 256, 0, st>>>(stats, gamma, gamma ? beta : nullptr, coef, total, ch, ch / groups);
+  MB_CUDA(cudaGetLastError());
+  count_launch();
+  return MIMIR_B200_OK;
+}
+
 // (mean, 1 / sqrt(var + eps)) of every (sample, group) slab, for consumers that normalise on the fly
 int launch_groupnorm_stats(const float* x, float* stats, int batch, int ch, int hw, int groups, float eps, cudaStream_t st) {
   if (groups <= 0 || ch % groups != 0) return fail(MIMIR_B200_E_INVALID, "GroupNorm: channels must be divisible by num_groups");

@@ -156,6 +156,17 @@ struct ConvExec {
   int in_up = 0;
   // The statistics of the folded GroupNorm already exist (the producer's epilogue emitted them): [batch][pre_groups][2]
   const float* pre_stats = nullptr;
+  // The residual is the INPUT of a GroupNorm (+ SiLU), which the epilogue applies (where conv_takes_normed_residual() holds)
+  int res_groups = 0;                          // > 0 switches it on
+  const float* res_gamma = nullptr;
+  const float* res_beta = nullptr;
+  float res_eps = 1e-5f;
+  int res_act = -1;
+  const float* res_stats = nullptr;            // as pre_stats
+  // The operand planes of x already exist, laid out by an earlier convolution with a ring of `planes_pad` pixels (1 x 1 kernels, where
+  // conv_takes_padded_planes() holds)
+  const __nv_bfloat16* planes = nullptr;
+  int planes_pad = 0;
   // This convolution's output feeds a GroupNorm of gn_groups groups: its epilogue leaves moments behind and
   // (mean, 1 / std) per (sample, group) go to gn_stats_out (where conv_can_emit_gn() holds; the workspace holds the moments)
   float* gn_stats_out = nullptr;
@@ -165,6 +176,11 @@ struct ConvExec {
 size_t conv_prenorm_bytes(int batch, int groups);
 // can this convolution's epilogue emit the statistics of a GroupNorm with `groups` groups over its output, and should it?
 bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int groups, int act, bool res_up);
+// may its residual be a GroupNorm's input?  conv_normed_residual_bytes() of workspace then
+bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act);
+// may it read the padded operand planes of another convolution of the same tensor?
+bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act);
+size_t conv_normed_residual_bytes(int batch, int oc, int groups);
 // scratch of the moments it leaves (behind the planes and the pre-norm statistics)
 size_t conv_gn_emit_bytes(int batch, int ic, int oc, int h, int w, int ks, int pad, int precision);
 // stride-1 "same" convolutions with a channel count that is a multiple of 32 run as shifted GEMMs over the

@@ -125,3 +125,81 @@ def test_tiles_of_128_pixels_keep_the_bits_of_256(rt, monkeypatch, precision, ba
         got.append(m.forward(ins, batch, oc * s * s * h * w))
         m.close()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("form", ["skip", "chain", "plain"])
+@pytest.mark.parametrize("batch,ic,oc,h,w,groups", [(20, 64, 128, 58, 58, 32), (33, 32, 64, 63, 65, 16), (3, 32, 256, 120, 99, 8), (45, 32, 160, 37, 33, 5), (80, 32, 64, 48, 48, 32),
+                                                  (2, 32, 64, 40, 34, 8), (1, 64, 40, 32, 32, 8)])
+def test_groupnorm_statistics_of_a_large_result(rt, form, batch, ic, oc, h, w, groups):
+    """Conv -> GroupNorm -> SiLU on more than 32 MB: the moments come from the convolution's epilogue (four channels and more to a group; the
+    last case, with two, sweeps).  Then a 1 x 1 convolution that the normalised tensor is added to, a convolution that reads it, or
+    nothing.  Tiles cut at the right and the lower edge; values with a mean of several deviations.  In the first form the 1 x 1
+    convolution reads the padded planes that the first one laid out (the two small cases: without the rest)."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(batch + oc)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x = randn(batch, ic, h, w) + 2.0
+    w1 = (randn(oc, ic, 3, 3) + 0.3) / (9 * ic) ** 0.5
+    g, b = 1 + 0.2 * randn(oc), 0.1 * randn(oc)
+    k2 = 1 if form == "skip" else 3
+    w2 = randn(oc, ic if form == "skip" else oc, k2, k2) / (k2 * k2 * oc) ** 0.5
+    conv = lambda name, i, o, c, k: make_desc(name, "Conv2d", inputs=[i], output=o, in_channels=c, out_channels=oc, input_height=h, input_width=w,  # noqa: E731
+                                              kernel=k, stride=1, padding=k // 2, params_count=oc * c * k * k)
+    descs = [conv("c1", "x", "a", ic, 3),
+             make_desc("g", "GroupNorm", inputs=["a"], output="b", in_channels=oc, input_height=h, input_width=w, num_groups=groups, affine=1, use_bias=1, eps=1e-5,
+                       params_count=2 * oc), make_desc("s", "SiLU", inputs=["b"], output="x" if form == "plain" else "c")]
+    if form == "skip":
+        descs += [conv("c2", "x", "d", ic, 1), make_desc("add", "Add", inputs=["c", "d"], output="x")]
+    elif form == "chain":
+        descs += [conv("c2", "c", "x", oc, 3)]
+    m = rt.GraphModel(descs)
+    m.upload_weights(0, w1.cpu().numpy().ravel())
+    m.upload_weights(1, torch.cat([g, b]).cpu().numpy())
+    if form != "plain":
+        m.upload_weights(3, w2.cpu().numpy().ravel())
+    m.plan({"x": (ic * h * w, False)}, batch)
+    got = torch.empty(batch, oc, h, w, device="cuda")
+    d = lambda t: t.double()  # noqa: E731
+    c = torch.nn.functional.silu(torch.nn.functional.group_norm(torch.nn.functional.conv2d(d(x), d(w1), padding=1), groups, d(g), d(b), 1e-5))
+    want = c + torch.nn.functional.conv2d(d(x), d(w2)) if form == "skip" else torch.nn.functional.conv2d(c, d(w2), padding=1) if form == "chain" else c
+    torch.cuda.synchronize()
+    for _ in range(3):  # layer by layer, captured, replayed
+        got.zero_()
+        m.forward_device({"x": (x.data_ptr(), ic * h * w, False)}, batch, got.data_ptr(), got.numel())
+        torch.cuda.synchronize()
+        # two contractions (4e-6 each, of values that the norm then takes a mean of up to five deviations from)
+        assert (got - want).norm() <= 3e-5 * want.norm()
+    m.close()
+
+
+def test_planes_are_not_kept_where_the_budget_has_no_room(rt):
+    """Conv -> conv -> Add with a 1 x 1 convolution of the input, which reads the first one's planes; planned again with a budget that
+    these would exceed, it lays out its own, and gives the same."""
+    batch, c, h = 4, 64, 64
+    r = np.random.default_rng(3)
+    x = r.standard_normal((batch, c * h * h)).astype(np.float32)
+    ws = [(r.standard_normal(c * c * k * k) / np.sqrt(c * k * k)).astype(np.float32) for k in (3, 3, 1)]
+    conv = lambda name, i, o, k: make_desc(name, "Conv2d", inputs=[i], output=o, in_channels=c, out_channels=c, input_height=h, input_width=h, kernel=k,  # noqa: E731
+                                           stride=1, padding=k // 2, params_count=c * c * k * k)
+    descs = [conv("c1", "x", "a", 3), conv("c2", "a", "b", 3), conv("c3", "x", "d", 1), make_desc("add", "Add", inputs=["b", "d"], output="x")]
+
+    def run():
+        m = rt.GraphModel(descs)
+        for i, w in enumerate(ws):
+            m.upload_weights(i, w)
+        m.plan({"x": (c * h * h, False)}, batch)
+        used, arena = rt.guard_stats()["current"], rt.stats()["arena_peak_bytes"]
+        got = m.forward({"x": (x, False)}, batch, c * h * h).copy()
+        m.close()
+        return got, used, arena
+
+    before = rt.guard_stats()["limit"]
+    want, used, arena = run()
+    rt.check(rt.lib().mimir_b200_guard_set_limit(used - (1 << 20)))
+    try:
+        got, _, less = run()
+    finally:
+        rt.check(rt.lib().mimir_b200_guard_set_limit(before))
+    assert less < arena
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
