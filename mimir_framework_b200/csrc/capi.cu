@@ -490,8 +490,17 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
   if (e.residual_up && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: an upsampled residual needs the shifted-GEMM path");
   if (e.res_groups > 0 && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: a normalised residual needs the shifted-GEMM path");
   if (e.in_up && !conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) return fail(MIMIR_B200_E_INVALID, "Conv2d: an upsampled input needs the shifted-GEMM path");
-  if (e.w_f32 != nullptr && e.pre_groups == 0 && e.res_groups == 0 && !e.in_up && !e.residual_up && conv_small_oc_supported(e.oc, e.ks, e.stride, e.pad, e.h, e.w, e.batch, e.activation))
-    return launch_conv_small_oc(e.x, e.w_f32, e.y, e.residual, e.batch, e.ic, e.oc, e.h, e.w, e.ks, e.pad, e.activation, st);
+  if (e.w_f32 != nullptr && e.res_groups == 0 && !e.in_up && !e.residual_up && conv_small_oc_supported(e.oc, e.ks, e.stride, e.pad, e.h, e.w, e.batch, e.activation) &&
+      (e.pre_groups == 0 || conv_small_oc_takes_norm(e.h, e.w))) {
+    float4* coef = nullptr;
+    if (e.pre_groups > 0) {
+      float* stats = static_cast<float*>(e.ws);
+      coef = reinterpret_cast<float4*>(static_cast<uint8_t*>(e.ws) + conv_prenorm_bytes(e.batch, e.pre_groups));
+      if (e.pre_stats == nullptr) MB_TRY(launch_groupnorm_stats(e.x, stats, e.batch, e.ic, e.h * e.w, e.pre_groups, e.pre_eps, st));
+      MB_TRY(launch_gn_coefs(e.pre_stats ? e.pre_stats : stats, e.pre_gamma, e.pre_beta, coef, e.batch, e.ic, e.pre_groups, st));
+    }
+    return launch_conv_small_oc(e.x, e.w_f32, e.y, e.residual, e.batch, e.ic, e.oc, e.h, e.w, e.ks, e.pad, e.activation, st, coef, e.pre_act == MIMIR_B200_ELT_SILU ? 1 : 0);
+  }
   if (conv_uses_shifted(e.ic, e.ks, e.stride, e.pad)) {
     // NCHW fp32 -> zero-padded NHWC planes, then one GEMM that walks the taps as shifted row offsets
     const long long rows = static_cast<long long>(e.batch) * (e.h + 2 * e.pad) * (e.w + 2 * e.pad);

@@ -5,6 +5,7 @@
 // bf16 hi/lo planes the GEMM consumes (one pass over the input, no fp32 column matrix), the OIHW
 // weight block already is the K-major [oc][ic*k*k] operand, and the GEMM epilogue writes NCHW.
 #include "common.h"
+#include "epilogue.cuh"
 #include "planes.cuh"
 
 namespace mb {
@@ -401,10 +402,14 @@ struct SmallOcGeom {
   static constexpr int TILE = SO_CC * TH * TWP, WOFF = (SO_NBUF * TILE + 3) & ~3;
 };
 
-template <int OC, int KS, int R, int VEC>
+// NORM: x is the input of a GroupNorm (+ SiLU), which every thread applies to the chunks it has copied itself, between their arrival and the barrier
+// that lets the others read them; the padding ring stays zero.  A tensor less written and read: 16 x 128 channels at 256^2, GroupNorm's
+// sweep and the convolution to 3 channels 473 -> 391 us.
+template <int OC, int KS, int R, int VEC, int NORM>
 __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                        float* __restrict__ y, const float* __restrict__ residual, int ic,
-                                                                       int h, int wd, int act) {
+                                                                       int h, int wd, int act, const float4* __restrict__ coef, int pre_silu) {
+  static_assert(VEC || !NORM, "whole chunks");
   using G = SmallOcGeom<KS, R, VEC>;
   constexpr int PAD = G::PAD, TW = G::TW, TH = G::TH, TWP = G::TWP, TILE = G::TILE, SEG = G::SEG, KK = KS * KS;
   constexpr int WROW = (KS * OC + 3) & ~3;  // the weights of one (channel, kernel row) as [kw][o], padded to whole float4s
@@ -432,15 +437,30 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
     xdst[k] = xx < TW ? xx + xx / SO_PX : -1;
     xsrc[k] = (xx < TW && gx >= 0 && gx < wd) ? gx : -1;
   }
+  // a thread copies the same chunks of every tile: their places once per thread (VEC)
+  constexpr int CELLS = SO_CC * TH * G::CHUNKS, NC = VEC ? (CELLS + SO_TX * SO_TY - 1) / (SO_TX * SO_TY) : 1;
+  int csrc[NC], cdst[NC];  // csrc: within the first SO_CC channels; < 0: outside the image (a chunk is wholly inside or wholly outside)
+  if (VEC) {
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const int idx = threadIdx.x + k * (SO_TX * SO_TY), row = idx / G::CHUNKS, ch = idx - row * G::CHUNKS;
+      const int c = row / TH, yy = row - c * TH, gy = y0 + yy - PAD, gx = x0 - 4 + 4 * ch;
+      cdst[k] = idx < CELLS ? row * TWP + 4 * ch : -1;
+      csrc[k] = idx < CELLS && gy >= 0 && gy < h && gx >= 0 && gx < wd ? (c * h + gy) * wd + gx : -1;
+    }
+  }
+  const int second = h * wd;  // csrc from here on: the second channel of a chunk of two
+  static_assert(SO_CC == 2, "two channels at a time");
   auto fetch = [&](int c0, int buf) {
     const int cc = min(SO_CC, ic - c0);
     float* tile = so_smem + buf * TILE;
     if (VEC) {
-      for (int idx = threadIdx.x; idx < SO_CC * TH * G::CHUNKS; idx += SO_TX * SO_TY) {
-        const int row = idx / G::CHUNKS, ch = idx - row * G::CHUNKS;
-        const int c = row / TH, yy = row - c * TH, gy = y0 + yy - PAD, gx = x0 - 4 + 4 * ch;
-        const bool ok = c < cc && gy >= 0 && gy < h && gx >= 0 && gx < wd;  // a chunk is wholly inside or wholly outside
-        cp_async16_zfill(tile + row * TWP + 4 * ch, ok ? xs + (static_cast<long long>(c0 + c) * h + gy) * wd + gx : xs, ok);
+      const float* src = xs + static_cast<long long>(c0) * second;
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        if (cdst[k] < 0) continue;
+        const bool ok = csrc[k] >= 0 && (cc == SO_CC || csrc[k] < second);
+        cp_async16_zfill(tile + cdst[k], ok ? src + csrc[k] : xs, ok);
       }
     } else
     for (int row = ty; row < SO_CC * TH; row += SO_TY) {  // one warp per tile row
@@ -463,6 +483,20 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  auto normalise = [&](int c0, int buf) {
+    float* tile = so_smem + buf * TILE;
+    const float4 k0 = __ldg(coef + static_cast<long long>(n) * ic + c0), k1 = __ldg(coef + static_cast<long long>(n) * ic + min(c0 + 1, ic - 1));
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      if (cdst[k] < 0 || csrc[k] < 0) continue;
+      const bool b = csrc[k] >= second;
+      const float m = b ? k1.x : k0.x, a = b ? k1.y : k0.y, o = b ? k1.z : k0.z;
+      float4 v = *reinterpret_cast<const float4*>(tile + cdst[k]);
+      v.x = fmaf(v.x - m, a, o); v.y = fmaf(v.y - m, a, o); v.z = fmaf(v.z - m, a, o); v.w = fmaf(v.w - m, a, o);
+      if (pre_silu) { v.x *= logistic(v.x); v.y *= logistic(v.y); v.z *= logistic(v.z); v.w *= logistic(v.w); }
+      *reinterpret_cast<float4*>(tile + cdst[k]) = v;
+    }
+  };
   // SO_NBUF - 1 chunks in flight; one commit per iteration (an empty group past the end) keeps the wait count uniform
 #pragma unroll
   for (int b = 0; b < SO_NBUF - 1; ++b) {
@@ -473,6 +507,7 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
   for (int c0 = 0; c0 < ic; c0 += SO_CC, cur = cur + 1 == SO_NBUF ? 0 : cur + 1) {
     const int cc = min(SO_CC, ic - c0);
     asm volatile("cp.async.wait_group %0;" ::"n"(SO_NBUF - 2) : "memory");
+    if (NORM) normalise(c0, cur);
     __syncthreads();  // this chunk has landed for every thread, and everyone is done with the buffer refilled next
     if (c0 + (SO_NBUF - 1) * SO_CC < ic) fetch(c0 + (SO_NBUF - 1) * SO_CC, cur == 0 ? SO_NBUF - 1 : cur - 1);
     else asm volatile("cp.async.commit_group;" ::: "memory");
@@ -545,43 +580,51 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
   }
 }
 
-template <int OC, int KS, int VEC>
+template <int OC, int KS, int VEC, int NORM>
 int launch_small_oc_v(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int h, int wd, int act,
-                      cudaStream_t st) {
+                      cudaStream_t st, const float4* coef, int pre_silu) {
   constexpr int R = so_rows(OC);
   using G = SmallOcGeom<KS, R, VEC>;
   constexpr int SMEM = (G::WOFF + SO_NBUF * SO_CC * KS * ((KS * OC + 3) & ~3)) * static_cast<int>(sizeof(float));
   static PerDeviceOnce attr_once;
   MB_TRY(attr_once.run([&]() -> int {
-    MB_CUDA(cudaFuncSetAttribute(conv_small_oc_kernel<OC, KS, R, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    MB_CUDA(cudaFuncSetAttribute(conv_small_oc_kernel<OC, KS, R, VEC, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     return MIMIR_B200_OK;
   }));
   dim3 grid((wd + SO_TX * SO_PX - 1) / (SO_TX * SO_PX), (h + SO_TY * R - 1) / (SO_TY * R), batch);
-  conv_small_oc_kernel<OC, KS, R, VEC><<<grid, SO_TX * SO_TY, SMEM, st>>>(x, w, y, residual, ic, h, wd, act);
+  conv_small_oc_kernel<OC, KS, R, VEC, NORM><<<grid, SO_TX * SO_TY, SMEM, st>>>(x, w, y, residual, ic, h, wd, act, coef, pre_silu);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;
 }
 
+bool small_oc_vec(int h, int wd) {
+  static const bool off = [] { const char* e = getenv("MIMIR_B200_CONV_SMALL_OC_VEC"); return e && e[0] == '0'; }();
+  return !off && (wd & 3) == 0 && static_cast<long long>(h) * wd * SO_CC <= 0x7fffffffLL;
+}
+
 template <int OC, int KS>
 int launch_small_oc_k(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int h, int wd, int act,
-                      cudaStream_t st) {
+                      cudaStream_t st, const float4* coef, int pre_silu) {
   // whole 16-byte chunks per image row and an aligned base: the vector form (MIMIR_B200_CONV_SMALL_OC_VEC=0 turns it off)
-  static const bool vec_off = [] { const char* e = getenv("MIMIR_B200_CONV_SMALL_OC_VEC"); return e && e[0] == '0'; }();
-  if (!vec_off && (wd & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0)
-    return launch_small_oc_v<OC, KS, 1>(x, w, y, residual, batch, ic, h, wd, act, st);
-  return launch_small_oc_v<OC, KS, 0>(x, w, y, residual, batch, ic, h, wd, act, st);
+  const bool vec = small_oc_vec(h, wd) && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  if (coef != nullptr) {
+    if (!vec) return fail(MIMIR_B200_E_INVALID, "conv_small_oc: a normalised input comes in whole aligned chunks");
+    return launch_small_oc_v<OC, KS, 1, 1>(x, w, y, residual, batch, ic, h, wd, act, st, coef, pre_silu);
+  }
+  if (vec) return launch_small_oc_v<OC, KS, 1, 0>(x, w, y, residual, batch, ic, h, wd, act, st, nullptr, 0);
+  return launch_small_oc_v<OC, KS, 0, 0>(x, w, y, residual, batch, ic, h, wd, act, st, nullptr, 0);
 }
 
 template <int OC>
 int launch_small_oc_t(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int h, int wd, int ks, int pad,
-                      int act, cudaStream_t st) {
+                      int act, cudaStream_t st, const float4* coef, int pre_silu) {
   (void)pad;
   switch (ks) {
-    case 1: return launch_small_oc_k<OC, 1>(x, w, y, residual, batch, ic, h, wd, act, st);
-    case 3: return launch_small_oc_k<OC, 3>(x, w, y, residual, batch, ic, h, wd, act, st);
-    case 5: return launch_small_oc_k<OC, 5>(x, w, y, residual, batch, ic, h, wd, act, st);
-    case 7: return launch_small_oc_k<OC, 7>(x, w, y, residual, batch, ic, h, wd, act, st);
+    case 1: return launch_small_oc_k<OC, 1>(x, w, y, residual, batch, ic, h, wd, act, st, coef, pre_silu);
+    case 3: return launch_small_oc_k<OC, 3>(x, w, y, residual, batch, ic, h, wd, act, st, coef, pre_silu);
+    case 5: return launch_small_oc_k<OC, 5>(x, w, y, residual, batch, ic, h, wd, act, st, coef, pre_silu);
+    case 7: return launch_small_oc_k<OC, 7>(x, w, y, residual, batch, ic, h, wd, act, st, coef, pre_silu);
     default: return fail(MIMIR_B200_E_INVALID, "conv_small_oc: kernel size %d", ks);
   }
 }
@@ -595,17 +638,19 @@ bool conv_small_oc_supported(int oc, int ks, int stride, int pad, int h, int wd,
          static_cast<long long>(h) * wd >= 4096;  // small images keep the tensor-core path (too few tiles to fill the SMs)
 }
 
+bool conv_small_oc_takes_norm(int h, int wd) { return small_oc_vec(h, wd); }
+
 int launch_conv_small_oc(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int oc, int h, int wd, int ks,
-                         int pad, int act, cudaStream_t st) {
+                         int pad, int act, cudaStream_t st, const float4* coef, int pre_silu) {
   switch (oc) {
-    case 1: return launch_small_oc_t<1>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 2: return launch_small_oc_t<2>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 3: return launch_small_oc_t<3>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 4: return launch_small_oc_t<4>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 5: return launch_small_oc_t<5>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 6: return launch_small_oc_t<6>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 7: return launch_small_oc_t<7>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
-    case 8: return launch_small_oc_t<8>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st);
+    case 1: return launch_small_oc_t<1>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 2: return launch_small_oc_t<2>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 3: return launch_small_oc_t<3>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 4: return launch_small_oc_t<4>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 5: return launch_small_oc_t<5>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 6: return launch_small_oc_t<6>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 7: return launch_small_oc_t<7>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
+    case 8: return launch_small_oc_t<8>(x, w, y, residual, batch, ic, h, wd, ks, pad, act, st, coef, pre_silu);
     default: return fail(MIMIR_B200_E_INVALID, "conv_small_oc: %d output channels", oc);
   }
 }

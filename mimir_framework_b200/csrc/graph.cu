@@ -1014,10 +1014,12 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     if (C.lt != LT::Conv2d || C.skip || C.pre_norm >= 0 || C.in_v[0] != pv) continue;
     if (!conv_uses_shifted(C.d.in_channels, C.d.kernel, C.d.stride, C.d.padding)) continue;
     if (C.d.in_channels != P.ch || C.h != P.h || C.w != P.w) continue;
-    // a convolution that takes the direct fp32 kernel reads the normalised tensor itself: it has no layout pass to fold into
-    if (conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch,
-                                C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act))
-      continue;
+    // A convolution that takes the direct fp32 kernel normalises what it has copied (not a caller's buffer, which need not start on 16 bytes);
+    // a small tensor is read once by a GroupNorm of its own, and from L2 by the convolution.
+    if (conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act)) {
+      const int r = root_of(m->tensors, P.in_v[0]);
+      if (!conv_small_oc_takes_norm(C.h, C.w) || m->tensors[r].producer < 0 || r == out_root || f32_bytes(m->tensors[r], batch) < (size_t(32) << 20)) continue;
+    }
     const int xin = P.in_v[0];
     C.pre_norm = li;
     C.in_v[0] = xin;
@@ -1051,8 +1053,8 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       }
       const bool conv_in = C.lt == LT::Conv2d && !C.skip && !C.in_up && C.in_v[0] == uv && C.res_v != uv && C.d.in_channels == U.ch &&
                            C.h == U.oh && C.w == U.ow && conv_uses_shifted(C.d.in_channels, C.d.kernel, C.d.stride, C.d.padding) &&
-                           (C.pre_norm >= 0 || !conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch,
-                                                                        C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act));
+                           !conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch,
+                                                    C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act);
       if (!conv_in) {
         keep.push_back(ci);
         continue;
@@ -1332,6 +1334,10 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
           L.ws_bytes = conv_ws_bytes(batch, L.d.in_channels, L.h, L.w, L.d.kernel, L.d.stride, L.d.padding, m->precision);
           if (L.planes_from >= 0) L.ws_bytes = 0;
           if (L.pre_norm >= 0) L.ws_bytes += conv_prenorm_bytes(batch, m->layers[L.pre_norm].d.num_groups);
+          if (L.pre_norm >= 0) {  // (the direct kernel's coefficients: within a larger workspace in any case, but for one channel)
+            const size_t direct = conv_prenorm_bytes(batch, m->layers[L.pre_norm].d.num_groups) + align256(static_cast<size_t>(batch) * L.d.in_channels * sizeof(float4));
+            if (L.ws_bytes < direct) L.ws_bytes = direct;
+          }
           if (L.res_norm >= 0) L.ws_bytes += conv_normed_residual_bytes(batch, L.d.out_channels, m->layers[L.res_norm].d.num_groups);
           if (L.gn_emit_for >= 0)
             L.ws_bytes += conv_gn_emit_bytes(batch, L.d.in_channels, L.d.out_channels, L.h, L.w, L.d.kernel, L.d.padding, m->precision);

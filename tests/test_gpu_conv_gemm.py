@@ -203,3 +203,36 @@ def test_planes_are_not_kept_where_the_budget_has_no_room(rt):
         rt.check(rt.lib().mimir_b200_guard_set_limit(before))
     assert less < arena
     assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("silu", [True, False])
+@pytest.mark.parametrize("batch,ic,oc,h,w,k,groups", [(9, 64, 3, 120, 124, 3, 32), (3, 96, 1, 171, 172, 5, 8), (35, 32, 8, 65, 128, 1, 32), (2, 160, 4, 203, 132, 7, 40)])
+def test_direct_convolution_normalises_its_input(rt, silu, batch, ic, oc, h, w, k, groups):
+    """GroupNorm (+ SiLU) read by a convolution to a handful of channels only, on more than 32 MB: tiles cut at every edge, whose ring stays zero."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(ic + oc)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x = randn(batch, ic, h, w) + 1.0
+    g, b, wt = 1 + 0.2 * randn(ic), 0.5 * randn(ic), randn(oc, ic, k, k) / (ic * k * k) ** 0.5
+    descs = [make_desc("r", "LeakyReLU", inputs=["x"], output="a"),
+             make_desc("g", "GroupNorm", inputs=["a"], output="b", in_channels=ic, input_height=h, input_width=w, num_groups=groups, affine=1, use_bias=1, eps=1e-5,
+                       params_count=2 * ic)]
+    if silu:
+        descs.append(make_desc("s", "SiLU", inputs=["b"], output="c"))
+    descs.append(make_desc("c", "Conv2d", inputs=["c" if silu else "b"], output="x", in_channels=ic, out_channels=oc, input_height=h, input_width=w, kernel=k, stride=1,
+                           padding=k // 2, params_count=wt.numel()))
+    m = rt.GraphModel(descs)
+    m.upload_weights(1, torch.cat([g, b]).cpu().numpy())
+    m.upload_weights(len(descs) - 1, wt.cpu().numpy().ravel())
+    m.plan({"x": (ic * h * w, False)}, batch)
+    got = torch.empty(batch, oc, h, w, device="cuda")
+    n = torch.nn.functional.group_norm(torch.nn.functional.leaky_relu(x.double(), 0.01), groups, g.double(), b.double(), 1e-5)
+    want = torch.nn.functional.conv2d(torch.nn.functional.silu(n) if silu else n, wt.double(), padding=k // 2)
+    torch.cuda.synchronize()
+    for _ in range(3):  # layer by layer, captured, replayed
+        got.zero_()
+        m.forward_device({"x": (x.data_ptr(), ic * h * w, False)}, batch, got.data_ptr(), got.numel())
+        torch.cuda.synchronize()
+        assert (got - want).norm() <= 3e-6 * want.norm()  # fp32 throughout: 2^-21 for SiLU, a few 2^-24 for the norm and the sums
+    m.close()
