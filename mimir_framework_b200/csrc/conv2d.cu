@@ -404,9 +404,10 @@ struct SmallOcGeom {
 
 // NORM: x is the input of a GroupNorm (+ SiLU), which every thread applies to the chunks it has copied itself, between their arrival and the barrier
 // that lets the others read them; the padding ring stays zero.  A tensor less written and read: 16 x 128 channels at 256^2, GroupNorm's
-// sweep and the convolution to 3 channels 473 -> 391 us.
+// sweep and the convolution to 3 channels 473 -> 376 us.
+// (Four CTAs to an SM where the accumulators allow: the UNet's 512 tiles are then one round; at 80 registers they were two, 389 us.)
 template <int OC, int KS, int R, int VEC, int NORM>
-__global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(SO_TX * SO_TY, VEC && OC <= 3 && KS <= 3 ? 4 : 1) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                        float* __restrict__ y, const float* __restrict__ residual, int ic,
                                                                        int h, int wd, int act, const float4* __restrict__ coef, int pre_silu) {
   static_assert(VEC || !NORM, "whole chunks");
@@ -439,13 +440,14 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
   }
   // a thread copies the same chunks of every tile: their places once per thread (VEC)
   constexpr int CELLS = SO_CC * TH * G::CHUNKS, NC = VEC ? (CELLS + SO_TX * SO_TY - 1) / (SO_TX * SO_TY) : 1;
-  int csrc[NC], cdst[NC];  // csrc: within the first SO_CC channels; < 0: outside the image (a chunk is wholly inside or wholly outside)
+  int csrc[NC];  // within the first SO_CC channels; < 0: outside the image (a chunk is wholly inside or wholly outside)
+  auto cell = [&](int k) { return static_cast<int>(threadIdx.x) + k * (SO_TX * SO_TY); };  // chunk `cell` of the tile, which has no padding
+  static_assert(!VEC || TWP == 4 * G::CHUNKS, "chunks side by side");
   if (VEC) {
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      const int idx = threadIdx.x + k * (SO_TX * SO_TY), row = idx / G::CHUNKS, ch = idx - row * G::CHUNKS;
+      const int idx = cell(k), row = idx / G::CHUNKS, ch = idx - row * G::CHUNKS;
       const int c = row / TH, yy = row - c * TH, gy = y0 + yy - PAD, gx = x0 - 4 + 4 * ch;
-      cdst[k] = idx < CELLS ? row * TWP + 4 * ch : -1;
       csrc[k] = idx < CELLS && gy >= 0 && gy < h && gx >= 0 && gx < wd ? (c * h + gy) * wd + gx : -1;
     }
   }
@@ -458,9 +460,9 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
       const float* src = xs + static_cast<long long>(c0) * second;
 #pragma unroll
       for (int k = 0; k < NC; ++k) {
-        if (cdst[k] < 0) continue;
+        if (cell(k) >= CELLS) continue;
         const bool ok = csrc[k] >= 0 && (cc == SO_CC || csrc[k] < second);
-        cp_async16_zfill(tile + cdst[k], ok ? src + csrc[k] : xs, ok);
+        cp_async16_zfill(tile + 4 * cell(k), ok ? src + csrc[k] : xs, ok);
       }
     } else
     for (int row = ty; row < SO_CC * TH; row += SO_TY) {  // one warp per tile row
@@ -488,13 +490,13 @@ __global__ void __launch_bounds__(SO_TX * SO_TY) conv_small_oc_kernel(const floa
     const float4 k0 = __ldg(coef + static_cast<long long>(n) * ic + c0), k1 = __ldg(coef + static_cast<long long>(n) * ic + min(c0 + 1, ic - 1));
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      if (cdst[k] < 0 || csrc[k] < 0) continue;
+      if (csrc[k] < 0) continue;
       const bool b = csrc[k] >= second;
       const float m = b ? k1.x : k0.x, a = b ? k1.y : k0.y, o = b ? k1.z : k0.z;
-      float4 v = *reinterpret_cast<const float4*>(tile + cdst[k]);
+      float4 v = *reinterpret_cast<const float4*>(tile + 4 * cell(k));
       v.x = fmaf(v.x - m, a, o); v.y = fmaf(v.y - m, a, o); v.z = fmaf(v.z - m, a, o); v.w = fmaf(v.w - m, a, o);
       if (pre_silu) { v.x *= logistic(v.x); v.y *= logistic(v.y); v.z *= logistic(v.z); v.w *= logistic(v.w); }
-      *reinterpret_cast<float4*>(tile + cdst[k]) = v;
+      *reinterpret_cast<float4*>(tile + 4 * cell(k)) = v;
     }
   };
   // SO_NBUF - 1 chunks in flight; one commit per iteration (an empty group past the end) keeps the wait count uniform
