@@ -148,15 +148,13 @@ int copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);
 int copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
 void release_host_copier();
 bool host_memory(const void* p);  // ordinary or page-locked, and so the caller's to read and write
-// Small tensors of a host-pointer call, by one kernel each way instead of a copy command per tensor (pointwise.cu).
-constexpr int STAGE_ITEMS = 8;
-constexpr size_t STAGE_BYTES = size_t(32) << 10;
+// The result of a host-pointer call, up to STAGE_BYTES of it, and its error word, by one kernel instead of a copy command each (pointwise.cu).
+constexpr int STAGE_ITEMS = 2;
+constexpr size_t STAGE_BYTES = size_t(256) << 10;
 struct StageItems {
   int count = 0;
-  struct { const uint32_t* src; uint32_t* dst; int words, copies; } item[STAGE_ITEMS];  // `copies` one behind the other at dst
-  void add(const void* src, void* dst, size_t words, int copies = 1) {
-    item[count++] = {static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), static_cast<int>(words), copies};
-  }
+  struct { const uint32_t* src; uint32_t* dst; int words; } item[STAGE_ITEMS];
+  void add(const void* src, void* dst, size_t words) { item[count++] = {static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), static_cast<int>(words)}; }
 };
 int launch_stage_copy(const StageItems& items, cudaStream_t st);
 // src -> device -> dst through a copier of its own that meets failures on the host: `inject` 1 page-locked memory, 2 a second thread,

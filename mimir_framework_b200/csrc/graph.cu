@@ -2073,55 +2073,31 @@ static int ensure_pipeline_objects(MimirB200Model* m) {
   return MIMIR_B200_OK;
 }
 
-// A forward that is not cut into micro-batches: everything on one stream.  Small inputs, a decode step's position, a small result
-// and the error word go through a page-locked block (launch_stage_copy), larger ones through copy commands.
+// A forward that is not cut into micro-batches: everything on one stream.  A result of up to STAGE_BYTES and the error word come back
+// through a page-locked block (launch_stage_copy), a larger one through copy commands.
 static int forward_host_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, const std::vector<int>& vs, float* out_host, const int* pos) {
   const TensorV& ot = m->tensors[root_of(m->tensors, m->out_v)];
   const int batch = m->planned_micro;
   const cudaStream_t st = m->s_comp;
   ErrorWatch errors;
-  StageBlock block;
-  size_t used = 0;
-  StageItems in, out;
-  auto place = [&](size_t bytes) {  // in the block; the item that follows starts on 16 bytes
-    const size_t at = used;
-    used += (bytes + 15) & ~size_t(15);
-    return block.p + at;
-  };
-  auto fits = [&](const StageItems& items, size_t bytes) { return block.p != nullptr && items.count < STAGE_ITEMS && bytes <= STAGE_BYTES - 16 && used <= STAGE_BYTES - 16 - bytes; };
   MB_CUDA(cudaEventRecord(m->ev0, st));
-  if (pos) {
-    if (fits(in, sizeof(int))) {
-      uint8_t* p = place(sizeof(int));
-      memcpy(p, pos, sizeof(int));
-      in.add(p, m->pos_dev, 1);
-    } else {
-      MB_CUDA(cudaMemcpyAsync(m->pos_dev, pos, sizeof(int), cudaMemcpyHostToDevice, st));
-    }
-  }
+  if (pos) MB_CUDA(cudaMemcpyAsync(m->pos_dev, pos, sizeof(int), cudaMemcpyHostToDevice, st));
   for (int i = 0; i < n_inputs; ++i) {
     const TensorV& t = m->tensors[vs[i]];
     float* slot = reinterpret_cast<float*>(m->arena + t.off_f32);
     const int copies = t.broadcast_input && !t.one_copy ? batch : 1;
-    const size_t n = static_cast<size_t>(t.n) * (t.broadcast_input ? 1 : batch);
-    if (fits(in, n * 4) && n * copies <= (size_t(1) << 20) && host_memory(inputs[i].data)) {
-      uint8_t* p = place(n * 4);
-      memcpy(p, inputs[i].data, n * 4);
-      in.add(p, slot, n, copies);
-    } else {
-      MB_TRY(copy_to_device(slot, inputs[i].data, n * 4, st));
-      if (copies > 1) MB_TRY(launch_broadcast_rows(slot, slot + t.n, copies - 1, t.n, st));
-    }
+    MB_TRY(copy_to_device(slot, inputs[i].data, static_cast<size_t>(t.n) * (t.broadcast_input ? 1 : batch) * 4, st));
+    if (copies > 1) MB_TRY(launch_broadcast_rows(slot, slot + t.n, copies - 1, t.n, st));
   }
-  if (in.count > 0) block.in_use = st;
-  MB_TRY(launch_stage_copy(in, st));
   Bound b;
   MB_TRY(run_layers_cached(m, batch, b, st, m->arena));
   MB_CUDA(cudaEventRecord(m->ev1, st));
   const size_t n_out = static_cast<size_t>(ot.n) * batch;
   const float* result = reinterpret_cast<const float*>(m->arena + ot.off_f32);
-  uint8_t* staged = fits(out, n_out * 4) && host_memory(out_host) ? place(n_out * 4) : nullptr;
-  if (staged) out.add(result, staged, n_out);
+  StageBlock block;
+  const uint8_t* staged = block.p != nullptr && n_out * 4 <= STAGE_BYTES && host_memory(out_host) ? block.p : nullptr;
+  StageItems out;
+  if (staged) out.add(result, block.p, n_out);
   if (int* word = staged ? errors.claim(st) : nullptr) out.add(ctx().dev_error_word, word, 1);
   else MB_TRY(errors.enqueue(st));
   if (staged) block.in_use = st;

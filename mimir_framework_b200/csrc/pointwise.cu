@@ -33,24 +33,24 @@ __device__ __forceinline__ float act_apply(int op, float v, float alpha = 0.0f) 
   }
 }
 
-// Tensors of a few KB between a page-locked block and the device, all of a call in one launch: what bounds it is one round trip over the
-// host link (2 us), where a copy command per tensor costs about 4 us each on the stream and a hop to the copy engine and back.  Registry
-// encoder, one sample from host arrays, three tensors in, one and the error word out: 219 -> 204 us.  From about 64 KB on the copy engine is faster:
-// an SM's writes to host memory reached 35 GB/s, and telling the host of each piece costs 8 us.
-constexpr int STAGE_CTAS = 4;
+// A call's result and error word into page-locked memory, both in one launch: what bounds it is the host link's latency (2 us) and the rate of
+// an SM's writes to host memory (35 GB/s over 16 CTAs), where a copy command costs about 4 us on the stream and a hop to the copy engine
+// and back.  Decode step of 12 samples: 36 KB 146.5 us with commands, 135.5 with this; 142 KB 152.6 and 143.0; 240 KB 157.7 and 147.5 (4 CTAs
+// as fast, 32 slower by 2).  Beyond 256 KB the host's own share, one thread against the ring's helpers, would be the longer one.  To the device
+// commands are faster: the driver puts a few KB into the command itself (the same step 3.8 us slower with a kernel that read them from
+// page-locked memory, 0.5 with one that had them as arguments).
+constexpr int STAGE_CTAS = 16;
 __global__ void __launch_bounds__(256) stage_copy_kernel(const StageItems p) {
   const uint32_t* src = p.item[blockIdx.y].src;
   uint32_t* dst = p.item[blockIdx.y].dst;
-  const int n = p.item[blockIdx.y].words, copies = p.item[blockIdx.y].copies, step = STAGE_CTAS * 256;
+  const int n = p.item[blockIdx.y].words, step = static_cast<int>(gridDim.x) * 256;
   for (int i0 = blockIdx.x * 256 + threadIdx.x; i0 < n; i0 += 4 * step) {
     uint32_t v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) v[u] = i0 + u * step < n ? __ldcv(src + i0 + u * step) : 0u;
-    for (long long c = 0; c < copies; ++c) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (i0 + u * step < n) dst[c * n + i0 + u * step] = v[u];
-    }
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * step < n) dst[i0 + u * step] = v[u];
   }
 }
 
@@ -408,7 +408,10 @@ int launch_copy_strided(const float* src, float* dst, int batch, int64_t n, int6
 
 int launch_stage_copy(const StageItems& items, cudaStream_t st) {
   if (items.count == 0) return MIMIR_B200_OK;
-  stage_copy_kernel<<<dim3(STAGE_CTAS, items.count), 256, 0, st>>>(items);
+  int words = 0;
+  for (int i = 0; i < items.count; ++i) words = items.item[i].words > words ? items.item[i].words : words;
+  const int ctas = (words + 1023) / 1024;  // four words a thread
+  stage_copy_kernel<<<dim3(ctas < STAGE_CTAS ? (ctas > 0 ? ctas : 1) : STAGE_CTAS, items.count), 256, 0, st>>>(items);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

@@ -35,10 +35,11 @@ def test_round_trip_at_the_edges_of_uneven_segments(rt, bytes_, extra):
     assert np.array_equal(rt.eltwise(abi.ELT_RELU, x), np.maximum(x, 0))
 
 
-@pytest.mark.parametrize("batch,n,inputs", [(1, 1, 1), (3, 5, 2), (1, 8188, 1), (1, 8189, 1), (2, 4097, 2), (4, 1025, 7), (2, 33, 9), (1, 4096, 3)])
+@pytest.mark.parametrize("batch,n,inputs", [(1, 1, 1), (3, 5, 2), (1, 1023, 1), (1, 1025, 1), (2, 4097, 2), (4, 1025, 7), (2, 33, 9),
+                                            (1, 16385, 3), (1, 65535, 1), (1, 65536, 1), (1, 65537, 1), (8, 8192, 2), (3, 21846, 2)])
 def test_small_tensors_through_the_staging_block(rt, batch, n, inputs):
-    """Around the block's 32 KB and eight tensors, each sample's own and broadcast ones (made in a kernel), with results that
-    change from call to call."""
+    """Results around a CTA's 4 KB, the 64 KB of a launch's CTAs together and the block's 256 KB, of inputs of each sample's own and broadcast ones,
+    which change from call to call."""
     descs, names = [], ["x"] + [f"i{k}" for k in range(1, inputs)]
     for k in range(1, inputs):
         descs.append(abi.make_desc(f"a{k}", "Add", inputs=["x" if k == 1 else f"s{k - 1}", names[k]], output="x" if k + 1 == inputs else f"s{k}"))
