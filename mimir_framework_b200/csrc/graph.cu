@@ -771,8 +771,11 @@ bool attention_streams_weights(const LayerRT& L, int batch) {
   return batch <= 16 && L.w_f32 && L.w_count >= static_cast<size_t>(4) * L.embed * L.embed;
 }
 
-// keep_planes: convolutions may hold on to their operand planes for a later one of the same tensor
-int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch, bool keep_planes = true) {
+// One plan.  `extras`: the forms that take more memory than they save may be chosen (operand planes kept for a later convolution, moments and
+// coefficients of a GroupNorm in a convolution's workspace, a residual Linear's planes, whose rows are padded); *took: one of them was, or
+// the arena of an earlier plan is larger than this one needs.
+int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch, bool extras, bool* took) {
+  *took = false;
   if (batch <= 0) return fail(MIMIR_B200_E_INVALID, "plan: batch must be positive");
   if (batch % m->pipeline != 0)
     return fail(MIMIR_B200_E_INVALID, "plan: batch %d is not a multiple of the %d pipeline micro-batches", batch, m->pipeline);
@@ -1018,7 +1021,8 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     // a small tensor is read once by a GroupNorm of its own, and from L2 by the convolution.
     if (conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act)) {
       const int r = root_of(m->tensors, P.in_v[0]);
-      if (!conv_small_oc_takes_norm(C.h, C.w) || m->tensors[r].producer < 0 || r == out_root || f32_bytes(m->tensors[r], batch) < (size_t(32) << 20)) continue;
+      if (!extras || !conv_small_oc_takes_norm(C.h, C.w) || m->tensors[r].producer < 0 || r == out_root || f32_bytes(m->tensors[r], batch) < (size_t(32) << 20)) continue;
+      *took = true;
     }
     const int xin = P.in_v[0];
     C.pre_norm = li;
@@ -1077,7 +1081,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
   }
   // ---- fusion 1g: a GroupNorm (+ SiLU) that is only added to a convolution's result (a block whose skip connection is a convolution): that
   //      convolution's epilogue reads the GroupNorm's input and normalises it; the normalised tensor never exists ----
-  for (int li = 0; li < nl && fuse_gn; ++li) {
+  for (int li = 0; li < nl && fuse_gn && extras; ++li) {
     LayerRT& P = m->layers[li];
     if (P.lt != LT::GroupNorm || P.skip || P.res_v >= 0) continue;
     if (P.fused_act >= 0 && P.fused_act != MIMIR_B200_ELT_SILU) continue;
@@ -1093,6 +1097,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       continue;
     C.res_norm = li;
     C.res_v = xin;
+    *took = true;
     for (int& c : m->tensors[xin].consumers)
       if (c == li) c = ci;
     pt.consumers.clear();
@@ -1102,13 +1107,12 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
   }
   // ---- fusion 1h: a 1 x 1 convolution of a tensor that another convolution reads as it is before it (the skip connection of a block): the
   //      planes that one laid out are kept for it ----
-  bool kept_planes = false;
   {
     auto reads_plain = [&](const LayerRT& C) {
       return C.lt == LT::Conv2d && !C.skip && C.pre_norm < 0 && !C.in_up && conv_uses_shifted(C.d.in_channels, C.d.kernel, C.d.stride, C.d.padding) &&
              !conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act);
     };
-    for (int p = 0; p < nl && keep_planes && fuse_gn; ++p) {
+    for (int p = 0; p < nl && extras && fuse_gn; ++p) {
       LayerRT& S = m->layers[m->order[p]];
       if (!reads_plain(S) || !conv_takes_padded_planes(batch, S.d.in_channels, S.d.out_channels, S.h, S.w, S.d.kernel, S.d.stride, S.d.padding, m->precision,
                                                        S.d.activation ? MIMIR_B200_ELT_RELU : S.fused_act))
@@ -1120,7 +1124,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
           continue;
         S.planes_from = m->order[q];
         E.ws_until = std::max(E.ws_until, p);
-        kept_planes = true;
+        *took = true;
         break;
       }
     }
@@ -1162,6 +1166,10 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     LayerRT& P = m->layers[t.producer];
     if (P.lt != LT::Linear || P.out_v != v || P.out_f != C.in_f || P.rows_ps != C.rows_ps) continue;
     if (linear_uses_skinny(P.rows_ps * batch, m->precision)) continue;
+    if (P.res_v >= 0 && P.out_f % 64 != 0) {
+      if (!extras) continue;
+      *took = true;
+    }
     P.emit_split = true;
     P.emit_f32 = false;
     C.read_split = true;
@@ -1254,7 +1262,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
   //      convolution does not sweep that tensor for its mean and variance: the convolution's epilogue leaves moments behind,
   //      a small kernel merges them, and the GroupNorm (or the layout pass) reads (mean, 1 / std) from there.
   for (auto& L : m->layers) { L.gn_emit_for = -1; L.gn_stats_from = -1; }
-  for (int li = 0; li < nl; ++li) {
+  for (int li = 0; li < nl && extras; ++li) {
     LayerRT& G = m->layers[li];
     if (G.lt != LT::GroupNorm) continue;
     int xin = -1;
@@ -1276,6 +1284,7 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
       continue;
     P.gn_emit_for = li;
     G.gn_stats_from = xt.producer;
+    *took = true;
   }
   ArenaSim sim;
   auto place = [&](int v) {
@@ -1396,32 +1405,37 @@ int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, i
     m->arena = m->arena2 = nullptr;
     m->arena_bytes = 0;
   }
-  // (where the budget has no room for planes that are kept, the plan is made without)
   if (!m->arena) {
-    const int s1 = dev_alloc(reinterpret_cast<void**>(&m->arena), need, "activation arena");
-    if (s1 != MIMIR_B200_OK) return kept_planes ? plan_model(m, inputs, n_inputs, full_batch, false) : s1;
+    MB_TRY(dev_alloc(reinterpret_cast<void**>(&m->arena), need, "activation arena"));
     m->arena_bytes = need;
   }
-  if (m->pipeline > 1 && !m->arena2) {
-    int s2 = dev_alloc(reinterpret_cast<void**>(&m->arena2), m->arena_bytes, "activation arena (second pipeline buffer)");
-    if (s2 != MIMIR_B200_OK && kept_planes) {
-      dev_free(m->arena, m->arena_bytes);
-      m->arena = nullptr;
-      m->arena_bytes = 0;
-      return plan_model(m, inputs, n_inputs, full_batch, false);
-    }
-    if (s2 != MIMIR_B200_OK) return s2;
-  }
+  *took = *took || m->arena_bytes > need;
+  if (m->pipeline > 1 && !m->arena2) MB_TRY(dev_alloc(reinterpret_cast<void**>(&m->arena2), m->arena_bytes, "activation arena (second pipeline buffer)"));
   if (m->pipeline == 1 && m->arena2) {
     dev_free(m->arena2, m->arena_bytes);
     m->arena2 = nullptr;
   }
-  m->planned_batch = full_batch;
   m->planned_micro = batch;
   for (auto& L : m->layers) MB_TRY(prepare_weight_planes(m, L, nullptr));
   MB_CUDA(cudaStreamSynchronize(nullptr));
+  m->planned_batch = full_batch;  // (last: no forward without all of its planes)
   ctx().stats.arena_peak_bytes = need * (m->pipeline > 1 ? 2 : 1);
   return MIMIR_B200_OK;
+}
+
+// Where the memory does not reach - for the arena or for the weight planes behind it - the plan is made once more without what takes extra.
+int plan_model(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, int batch) {
+  bool took = false;
+  int s = plan_once(m, inputs, n_inputs, batch, true, &took);
+  if (took && (s == MIMIR_B200_E_OOM_BUDGET || s == MIMIR_B200_E_CUDA)) {
+    cudaGetLastError();  // (a refused cudaMalloc leaves its error behind for the next launch's check)
+    if (m->arena) dev_free(m->arena, m->arena_bytes);
+    if (m->arena2) dev_free(m->arena2, m->arena_bytes);
+    m->arena = m->arena2 = nullptr;
+    m->arena_bytes = 0;
+    s = plan_once(m, inputs, n_inputs, batch, false, &took);
+  }
+  return s;
 }
 
 struct Bound {

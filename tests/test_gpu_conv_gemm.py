@@ -236,3 +236,54 @@ def test_direct_convolution_normalises_its_input(rt, silu, batch, ic, oc, h, w, 
         torch.cuda.synchronize()
         assert (got - want).norm() <= 3e-6 * want.norm()  # fp32 throughout: 2^-21 for SiLU, a few 2^-24 for the norm and the sums
     m.close()
+
+
+def skip_block(c, oc, h):
+    """conv -> conv -> Add with a 1 x 1 convolution of the input: operand planes that the first one laid out are read again."""
+    conv = lambda name, i, o, ic, k: make_desc(name, "Conv2d", inputs=[i], output=o, in_channels=ic, out_channels=oc, input_height=h, input_width=h, kernel=k,  # noqa: E731
+                                               stride=1, padding=k // 2, params_count=oc * ic * k * k)
+    descs = [conv("c1", "x", "a", c, 3), conv("c2", "a", "b", oc, 3), conv("c3", "x", "d", c, 1), make_desc("add", "Add", inputs=["b", "d"], output="x")]
+    r = np.random.default_rng(c + oc)
+    return descs, [(r.standard_normal(d.params_count) / np.sqrt(d.in_channels * d.kernel**2)).astype(np.float32) if d.params_count else None for d in descs]
+
+
+def plan_and_run(rt, descs, ws, x, batch, out):
+    """The result, the arena's size and the memory that uploading and planning took."""
+    before = rt.guard_stats()["current"]
+    m = rt.GraphModel(descs)
+    try:
+        for i, w in enumerate(ws):
+            if w is not None:
+                m.upload_weights(i, w)
+        uploaded = rt.guard_stats()["current"]
+        m.plan({"x": (x.shape[1], False)}, batch)
+        used, arena = rt.guard_stats()["current"] - before, rt.stats()["arena_peak_bytes"]
+        got = m.forward({"x": (x, False)}, batch, out).copy()
+    finally:
+        m.close()
+    return got, used, arena, uploaded - before
+
+
+@pytest.mark.parametrize("missing", ["arena", "weights"])
+def test_a_plan_goes_without_kept_planes_where_the_weight_planes_would_not_fit(rt, monkeypatch, missing):
+    """A budget with room for the plan that keeps no planes, to the byte: the larger arena does not fit (16 images of 128^2), or does,
+    and the weight planes behind it do not (few pixels, 512 channels)."""
+    batch, c, oc, h = (16, 64, 64, 128) if missing == "arena" else (2, 512, 512, 32)
+    descs, ws = skip_block(c, oc, h)
+    x = np.random.default_rng(5).standard_normal((batch, c * h * h)).astype(np.float32)
+    want, used, arena, _ = plan_and_run(rt, descs, ws, x, batch, oc * h * h)
+    monkeypatch.setenv("MIMIR_B200_FUSE_GN_CONV", "0")
+    plain, least, least_arena, uploaded = plan_and_run(rt, descs, ws, x, batch, oc * h * h)
+    monkeypatch.delenv("MIMIR_B200_FUSE_GN_CONV")
+    assert least < used, "the kept planes cost memory here, or this test shows nothing"
+    # the weight planes are what does not fit: the larger arena alone does
+    assert (uploaded + arena > least) == (missing == "arena")
+    before, base = rt.guard_stats()["limit"], rt.guard_stats()["current"]
+    rt.check(rt.lib().mimir_b200_guard_set_limit(base + least))
+    try:
+        got, now, got_arena, _ = plan_and_run(rt, descs, ws, x, batch, oc * h * h)
+    finally:
+        rt.check(rt.lib().mimir_b200_guard_set_limit(before))
+    assert (now, got_arena) == (least, least_arena)
+    assert np.array_equal(got, plain)
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
