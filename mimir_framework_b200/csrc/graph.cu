@@ -1017,11 +1017,11 @@ int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, in
     if (C.lt != LT::Conv2d || C.skip || C.pre_norm >= 0 || C.in_v[0] != pv) continue;
     if (!conv_uses_shifted(C.d.in_channels, C.d.kernel, C.d.stride, C.d.padding)) continue;
     if (C.d.in_channels != P.ch || C.h != P.h || C.w != P.w) continue;
-    // A convolution that takes the direct fp32 kernel normalises what it has copied (not a caller's buffer, which need not start on 16 bytes);
-    // a small tensor is read once by a GroupNorm of its own, and from L2 by the convolution.
+    // A convolution that takes the direct fp32 kernel normalises what it has copied (not a caller's buffer, which need not start on 16 bytes; what is
+    // faster apart stays apart).
     if (conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act)) {
       const int r = root_of(m->tensors, P.in_v[0]);
-      if (!extras || !conv_small_oc_takes_norm(C.h, C.w) || m->tensors[r].producer < 0 || r == out_root || f32_bytes(m->tensors[r], batch) < (size_t(32) << 20)) continue;
+      if (!extras || m->tensors[r].producer < 0 || r == out_root || !conv_small_oc_pays_norm(batch, C.d.in_channels, C.d.out_channels, C.h, C.w, C.d.kernel, P.d.num_groups)) continue;
       *took = true;
     }
     const int xin = P.in_v[0];

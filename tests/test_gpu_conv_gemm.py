@@ -287,3 +287,56 @@ def test_a_plan_goes_without_kept_planes_where_the_weight_planes_would_not_fit(r
     assert (now, got_arena) == (least, least_arena)
     assert np.array_equal(got, plain)
     assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
+def head_graph(ic, oc, h, w, k, groups, silu=True):
+    """LeakyReLU -> GroupNorm (-> SiLU) -> convolution to a handful of channels."""
+    d = [make_desc("r", "LeakyReLU", inputs=["x"], output="a"),
+         make_desc("g", "GroupNorm", inputs=["a"], output="b", in_channels=ic, input_height=h, input_width=w, num_groups=groups, affine=1, use_bias=1, eps=1e-5,
+                   params_count=2 * ic)]
+    if silu:
+        d.append(make_desc("s", "SiLU", inputs=["b"], output="c"))
+    return d + [make_desc("c", "Conv2d", inputs=["c" if silu else "b"], output="x", in_channels=ic, out_channels=oc, input_height=h, input_width=w, kernel=k, stride=1,
+                          padding=k // 2, params_count=oc * ic * k * k)]
+
+
+def run_on_device(rt, descs, weights, x, out_shape, passes=1):
+    import torch
+
+    m = rt.GraphModel(descs)
+    for i, wt in weights.items():
+        m.upload_weights(i, wt.cpu().numpy().ravel())
+    per = x[0].numel()
+    m.plan({"x": (per, False)}, x.shape[0])
+    got = torch.empty(out_shape, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(passes):  # layer by layer, captured, replayed
+        got.zero_()
+        m.forward_device({"x": (x.data_ptr(), per, False)}, x.shape[0], got.data_ptr(), got.numel())
+        torch.cuda.synchronize()
+    m.close()
+    return got
+
+
+@pytest.mark.parametrize("batch,ic,oc,h,w,k,groups,folded", [(1, 96, 3, 512, 512, 3, 4, False),      # 96 MB and four rows: the GroupNorm stays apart
+                                                            (9, 64, 3, 120, 124, 3, 32, False),     # a tensor of L2's size
+                                                            (100, 64, 3, 128, 128, 3, 32, False),   # short rows
+                                                            (12, 128, 5, 260, 256, 5, 32, False),   # a large kernel
+                                                            (12, 128, 3, 260, 256, 3, 32, True), (3, 64, 8, 420, 424, 5, 16, True), (25, 64, 1, 260, 260, 5, 8, True)])
+def test_direct_convolution_normalises_where_that_is_faster(rt, monkeypatch, batch, ic, oc, h, w, k, groups, folded):
+    """Which form ran shows in the bits: a GroupNorm that stays apart gives those of a plan without the fold."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(ic + oc)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x = randn(batch, ic, h, w) + 1.0
+    g, b, wt = 1 + 0.2 * randn(ic), 0.5 * randn(ic), randn(oc, ic, k, k) / (ic * k * k) ** 0.5
+    descs, weights = head_graph(ic, oc, h, w, k, groups), {1: torch.cat([g, b]), 3: wt}
+    got = run_on_device(rt, descs, weights, x, (batch, oc, h, w), 3)
+    monkeypatch.setenv("MIMIR_B200_FUSE_GN_CONV", "0")
+    apart = run_on_device(rt, descs, weights, x, (batch, oc, h, w))
+    assert torch.equal(got, apart) != folded
+    for i in range(0, batch, 4):
+        n = torch.nn.functional.group_norm(torch.nn.functional.leaky_relu(x[i:i + 4].double(), 0.01), groups, g.double(), b.double(), 1e-5)
+        want = torch.nn.functional.conv2d(torch.nn.functional.silu(n), wt.double(), padding=k // 2)
+        assert (got[i:i + 4] - want).norm() <= 3e-6 * want.norm()  # fp32 throughout: 2^-21 for SiLU, a few 2^-24 for the norm and the sums
