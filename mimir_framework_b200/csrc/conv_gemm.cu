@@ -404,13 +404,14 @@ long long tiles_of(const GemmArgs& g, int px) {
 // Blocks of 64 channels where two activation tiles and three weight planes of them fit the ring: a 128-byte row costs the copy engine
 // little more than a 64-byte one, and with 448 rows to a tap and 32 channels (3 x 3, four planes) those set the pace: a tile of 128 pixels
 // took 676 cycles for 384 of MMAs.  16 x 512 -> 512 on 16^2: 62.8 -> 53.0 us, with two products 52.2 -> 42.4; 3 x 256 -> 256 on 56^2, tiles
-// of 256 pixels: 45.2 -> 44.3.
+// of 256 pixels: 45.2 -> 44.3.  A normalised residual's coefficients leave the 3 x 3 form of 256 pixels and four planes a slot short, which then takes
+// blocks of 32: 16 x 256 -> 256 on 64^2 with its producer 427 -> 388 us (405 with the GroupNorm apart), 512 -> 256 830 -> 747 (763).
 bool conv_wide_blocks(const GemmArgs& g, int px) {
   const char* e = getenv("MIMIR_B200_CONV_BK");  // "32": never
   if (g.conv_c % 64 != 0 || (e && atoi(e) == 32)) return false;
   const ConvShape sh = conv_shape(g, px);
   const int tw = 1 << sh.tw_log, rows = (px >> sh.tw_log) + g.conv_ks - 1;
-  return 2 * g.a_planes * tw * rows * 128 + 3 * CG_M * 128 <= CG_SMEM_MAX - CG_EPI - 2048;
+  return 2 * g.a_planes * tw * rows * 128 + 3 * CG_M * 128 <= CG_SMEM_MAX - CG_EPI - (g.res_coef != nullptr ? CG_COEF : 0) - 2048;
 }
 
 // Estimated SM cycles of a launch and the tile it takes: within 5 % of 50 measured launches, K = 64 ... 4608.  Tiles of 128 pixels (half of

@@ -340,3 +340,71 @@ def test_direct_convolution_normalises_where_that_is_faster(rt, monkeypatch, bat
         n = torch.nn.functional.group_norm(torch.nn.functional.leaky_relu(x[i:i + 4].double(), 0.01), groups, g.double(), b.double(), 1e-5)
         want = torch.nn.functional.conv2d(torch.nn.functional.silu(n), wt.double(), padding=k // 2)
         assert (got[i:i + 4] - want).norm() <= 3e-6 * want.norm()  # fp32 throughout: 2^-21 for SiLU, a few 2^-24 for the norm and the sums
+
+
+def residual_graph(ic, oc, h, w, k1, k2, groups, silu=True, act=None):
+    """conv -> GroupNorm (-> SiLU) added to another convolution of the input."""
+    conv = lambda name, o, k: make_desc(name, "Conv2d", inputs=["x"], output=o, in_channels=ic, out_channels=oc, input_height=h, input_width=w, kernel=k,  # noqa: E731
+                                        stride=1, padding=k // 2, params_count=oc * ic * k * k)
+    d = [conv("c1", "a", k1), make_desc("g", "GroupNorm", inputs=["a"], output="b", in_channels=oc, input_height=h, input_width=w, num_groups=groups, affine=1, use_bias=1,
+                                        eps=1e-5, params_count=2 * oc)]
+    if silu:
+        d.append(make_desc("s", "SiLU", inputs=["b"], output="c"))
+    return d + [conv("c2", "d", k2), make_desc("add", "Add", inputs=["c" if silu else "b", "d"], output="x")]
+
+
+def residual_case(ic, oc, k1, k2, batch, h, w, seed):
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    half = lambda t: (t.view(torch.int32) & -65536).view(torch.float32)  # noqa: E731  (weights that are bfloat16 values, for every precision)
+    w1, w2 = (half(randn(oc, ic, k, k) / (k * k * ic) ** 0.5) for k in (k1, k2))
+    return randn(batch, ic, h, w) + 0.5, w1, 1 + 0.2 * randn(oc), 0.1 * randn(oc), w2
+
+
+def residual_want(x, w1, g, b, w2, groups, silu=True):
+    import torch
+
+    f = torch.nn.functional
+    n = f.group_norm(f.conv2d(x.double(), w1.double(), padding=w1.shape[2] // 2), groups, g.double(), b.double(), 1e-5)
+    return (f.silu(n) if silu else n) + f.conv2d(x.double(), w2.double(), padding=w2.shape[2] // 2)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W])
+@pytest.mark.parametrize("batch,ic,oc,h,w,k2,groups,silu", [(9, 64, 128, 97, 95, 3, 16, True), (5, 128, 160, 113, 112, 3, 5, True), (10, 32, 96, 96, 96, 5, 32, False)])
+def test_a_normed_residual_leaves_a_3_x_3_convolution_its_weight_slots(rt, monkeypatch, precision, batch, ic, oc, h, w, k2, groups, silu):
+    """The coefficients' 4 KB do not fit beside two activation tiles and three weight planes in blocks of 64 channels (two activation planes, 3 x 3,
+    tiles of 256 pixels): blocks of 32 then, whose sums are in another order, so that the bits show which ran (the first convolution, 5 x 5, takes
+    blocks of 32 in any case).  No planes are kept here: the form that normalises and reads planes of its own."""
+    import torch
+
+    monkeypatch.setenv("MIMIR_B200_CONV_PX", "256")
+    x, w1, g, b, w2 = residual_case(ic, oc, 5, k2, batch, h, w, oc + k2)
+    descs = residual_graph(ic, oc, h, w, 5, k2, groups, silu)
+    weights = {0: w1, 1: torch.cat([g, b]), len(descs) - 2: w2}
+    got = run_residual(rt, descs, weights, x, oc, precision, 3)
+    want = residual_want(x, w1, g, b, w2, groups, silu)
+    assert (got - want).norm() <= 3e-5 * want.norm()  # two contractions (4e-6 each), one of them normalised
+    monkeypatch.setenv("MIMIR_B200_CONV_BK", "32")
+    assert torch.equal(run_residual(rt, descs, weights, x, oc, precision), got)
+    monkeypatch.setenv("MIMIR_B200_FUSE_GN_CONV", "0")
+    assert not torch.equal(run_residual(rt, descs, weights, x, oc, precision), got), "the residual was not normalised by the convolution"
+
+
+def run_residual(rt, descs, weights, x, oc, precision=abi.PREC_BF16X2, passes=1):
+    import torch
+
+    m = rt.GraphModel(descs, precision)
+    for i, wt in weights.items():
+        m.upload_weights(i, wt.cpu().numpy().ravel())
+    per = x[0].numel()
+    m.plan({"x": (per, False)}, x.shape[0])
+    got = torch.empty(x.shape[0], oc, *x.shape[2:], device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(passes):
+        got.zero_()
+        m.forward_device({"x": (x.data_ptr(), per, False)}, x.shape[0], got.data_ptr(), got.numel())
+        torch.cuda.synchronize()
+    m.close()
+    return got
