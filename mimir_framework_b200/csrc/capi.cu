@@ -449,11 +449,13 @@ bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, i
   return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) && h >= 32 && w >= 32 && gemm_takes_spatial(g);
 }
 
-// The normalised tensor then never exists: where it is larger than L2's reach the epilogue's arithmetic (a skip layer of 1 x 1 waits for
-// memory anyway) costs less than writing it and reading it back.  64 images of 112^2, by launch: a
-// sweep of 281 us and a 1 x 1 convolution 128 -> 256 of 424 -> 625 in all; 64 -> 128 133 + 220 -> 327.
+// The normalised tensor then never exists: from 32 MB on the epilogue's arithmetic costs less than writing it and reading it back, for every kernel
+// size and every number of rows (where no moments exist the GroupNorm apart reads its input twice, too), but not with fewer than 96 channels: the
+// epilogue's warps are bound to the channels of a tile of 128, and half of them have nothing to do with 64.  Blocks of two
+// convolutions and a GroupNorm, apart and in here: 64 x 64 -> 128 of 112^2 with 1 x 1 700 and 650 us, 3 x 3 848 and 770, 16 x 256 -> 256 of
+// 64^2 278 and 268, 1 x 64 -> 128 of 256^2 in one group 435 and 368; 64 x 64 -> 96 of 112^2 648 and 594; 64 x 64 -> 64 562 and 585, 32 -> 32 380 and 419.
 bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
-  if (oc % 32 != 0 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
+  if (oc % 32 != 0 || oc < 96 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
   GemmArgs g;
   if (!shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g)) return false;
   return static_cast<long long>(batch) * oc * h * w * 4 >= (32ll << 20) && gemm_takes_spatial(g);

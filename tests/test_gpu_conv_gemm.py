@@ -408,3 +408,17 @@ def run_residual(rt, descs, weights, x, oc, precision=abi.PREC_BF16X2, passes=1)
         torch.cuda.synchronize()
     m.close()
     return got
+
+
+@pytest.mark.parametrize("batch,ic,oc,h,groups,folded", [(20, 32, 64, 87, 16, False), (40, 64, 32, 90, 8, False), (14, 32, 96, 87, 24, True), (3, 64, 256, 111, 2, True)])
+def test_a_residual_of_few_channels_is_normalised_apart(rt, monkeypatch, batch, ic, oc, h, groups, folded):
+    """Fewer than 96 channels: the GroupNorm of its own, whose bits a plan without the fold has."""
+    import torch
+
+    x, w1, g, b, w2 = residual_case(ic, oc, 3, 3, batch, h, h, oc)
+    descs, weights = residual_graph(ic, oc, h, h, 3, 3, groups), {0: w1, 1: torch.cat([g, b]), 3: w2}
+    got = run_residual(rt, descs, weights, x, oc)
+    want = residual_want(x, w1, g, b, w2, groups)
+    assert (got - want).norm() <= 3e-5 * want.norm()
+    monkeypatch.setenv("MIMIR_B200_FUSE_GN_CONV", "0")
+    assert torch.equal(run_residual(rt, descs, weights, x, oc), got) != folded
