@@ -441,12 +441,11 @@ bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int strid
 
 size_t conv_normed_residual_bytes(int batch, int oc, int groups) { return conv_prenorm_bytes(batch, groups) + align256(static_cast<size_t>(batch) * oc * sizeof(float4)); }
 
-// A layout pass over the tensor less; the ring costs a few per cent of the tiles (114^2 for 112^2: 3.5 %, 34^2 for 32^2: 13 %).  64 images
-// of 112^2: 136 us with 128 channels, 70 with 64.
-bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
+// A layout pass over the tensor less (64 images of 112^2: 136 us with 128 channels, 70 with 64), where it outweighs the ring (conv_gemm_ring_pays).
+bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int ring) {
   if (ks != 1 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
   GemmArgs g;
-  return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) && h >= 32 && w >= 32 && gemm_takes_spatial(g);
+  return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) && conv_gemm_ring_pays(g, ring) && gemm_takes_spatial(g);
 }
 
 // The normalised tensor then never exists: from 32 MB on the epilogue's arithmetic costs less than writing it and reading it back, for every kernel

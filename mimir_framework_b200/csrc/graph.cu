@@ -1114,13 +1114,13 @@ int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, in
     };
     for (int p = 0; p < nl && extras && fuse_gn; ++p) {
       LayerRT& S = m->layers[m->order[p]];
-      if (!reads_plain(S) || !conv_takes_padded_planes(batch, S.d.in_channels, S.d.out_channels, S.h, S.w, S.d.kernel, S.d.stride, S.d.padding, m->precision,
-                                                       S.d.activation ? MIMIR_B200_ELT_RELU : S.fused_act))
-        continue;
+      if (!reads_plain(S)) continue;
       for (int q = p - 1; q >= 0; --q) {
         LayerRT& E = m->layers[m->order[q]];
         if (!reads_plain(E) || E.planes_from >= 0 || E.d.padding < 1 || E.d.in_channels != S.d.in_channels || E.h != S.h || E.w != S.w ||
-            root_of(m->tensors, E.in_v[0]) != root_of(m->tensors, S.in_v[0]))
+            root_of(m->tensors, E.in_v[0]) != root_of(m->tensors, S.in_v[0]) ||
+            !conv_takes_padded_planes(batch, S.d.in_channels, S.d.out_channels, S.h, S.w, S.d.kernel, S.d.stride, S.d.padding, m->precision,
+                                      S.d.activation ? MIMIR_B200_ELT_RELU : S.fused_act, E.d.padding))
           continue;
         S.planes_from = m->order[q];
         E.ws_until = std::max(E.ws_until, p);

@@ -267,8 +267,8 @@ def plan_and_run(rt, descs, ws, x, batch, out):
 @pytest.mark.parametrize("missing", ["arena", "weights"])
 def test_a_plan_goes_without_kept_planes_where_the_weight_planes_would_not_fit(rt, monkeypatch, missing):
     """A budget with room for the plan that keeps no planes, to the byte: the larger arena does not fit (16 images of 128^2), or does,
-    and the weight planes behind it do not (few pixels, 512 channels)."""
-    batch, c, oc, h = (16, 64, 64, 128) if missing == "arena" else (2, 512, 512, 32)
+    and the weight planes behind it do not (two of 56^2, 512 channels)."""
+    batch, c, oc, h = (16, 64, 64, 128) if missing == "arena" else (2, 512, 512, 56)
     descs, ws = skip_block(c, oc, h)
     x = np.random.default_rng(5).standard_normal((batch, c * h * h)).astype(np.float32)
     want, used, arena, _ = plan_and_run(rt, descs, ws, x, batch, oc * h * h)
@@ -422,3 +422,21 @@ def test_a_residual_of_few_channels_is_normalised_apart(rt, monkeypatch, batch, 
     assert (got - want).norm() <= 3e-5 * want.norm()
     monkeypatch.setenv("MIMIR_B200_FUSE_GN_CONV", "0")
     assert torch.equal(run_residual(rt, descs, weights, x, oc), got) != folded
+
+
+@pytest.mark.parametrize("batch,c,oc,h,w,k,kept", [(4, 128, 128, 96, 96, 3, False), (4, 64, 256, 64, 64, 3, False), (8, 64, 64, 32, 32, 3, False), (2, 64, 64, 128, 128, 7, False),
+                                                  (3, 64, 100, 61, 67, 3, True), (5, 128, 72, 131, 103, 5, True), (1, 32, 64, 64, 200, 3, True)])
+def test_planes_are_kept_where_their_ring_costs_less_than_laying_them_out(rt, monkeypatch, batch, c, oc, h, w, k, kept):
+    """A second wave of tiles, twice as many outputs as inputs and more, a wide ring: planes of its own.  Whether planes are kept shows in the
+    arena.  The kept ones: ragged lines and channels, rings of one and two pixels, a residual added."""
+    conv = lambda name, i, o, ic, ks: make_desc(name, "Conv2d", inputs=[i], output=o, in_channels=ic, out_channels=oc, input_height=h, input_width=w,  # noqa: E731
+                                                kernel=ks, stride=1, padding=ks // 2, params_count=oc * ic * ks * ks)
+    descs = [conv("c1", "x", "a", c, k), conv("c3", "x", "d", c, 1), make_desc("add", "Add", inputs=["a", "d"], output="x")]
+    r = np.random.default_rng(h + oc)
+    ws = [(r.standard_normal(d.params_count) / np.sqrt(d.in_channels * d.kernel**2)).astype(np.float32) if d.params_count else None for d in descs]
+    x = r.standard_normal((batch, c * h * w)).astype(np.float32)
+    got, _, arena, _ = plan_and_run(rt, descs, ws, x, batch, oc * h * w)
+    monkeypatch.setenv("MIMIR_B200_FUSE_GN_CONV", "0")
+    apart, _, least, _ = plan_and_run(rt, descs, ws, x, batch, oc * h * w)
+    assert (arena > least) == kept
+    assert np.array_equal(got, apart)  # the same sums in the same order
