@@ -20,10 +20,19 @@ __device__ __forceinline__ float gelu_ref(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
   return __fmul_rn(x, r);  // (not contracted with a residual that follows)
 }
-// 1 / (1 + exp(-x)) in four instructions, two of them on the special-function unit: 2^-21 of its value for x above -87, 0 below
+// 1 / (1 + exp(-x)), the factor of SiLU, with two special-function instructions (expf and a division: a third more time on a GroupNorm).
+// exp(-x) = 2^t with t = -x log2 e.  What rounding t loses goes back in as a first-order factor: the constant in two parts (W. J. Cody and
+// W. Waite, Software Manual for the Elementary Functions, 1980), the product's rounding error by fused multiply-add, 2^d = 1 + d ln 2 for
+// |d| < 1.2e-5 (the next term is 4e-11).  With 2^-22 for each of the two instructions x times the result is within 2^-21 of its value for
+// -87.3 <= x, infinity included: above 64 it is x itself (2^t is 0 next to 1; the bound keeps `lost` finite).  Below -87.3 the
+// reciprocal is flushed and the product is -0, off by less than 1.2e-36; -inf gives NaN, as x * (1 / (1 + expf(-x))) does.
 __device__ __forceinline__ float logistic(float x) {
+  const float c = fminf(fmaxf(x, -88.0f), 64.0f);
+  const float t = c * -1.44269504f;
+  const float lost = fmaf(c, -1.44269504f, -t) - c * 1.92596e-8f;  // log2 e = 1.44269502163 + 1.92596e-8
   float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.442695041f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+  e = fmaf(e, lost * 0.69314718f, e);
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
   return r;
 }

@@ -10,6 +10,7 @@
 // GroupNorm + SiLU 576 rows of 41 334 (odd image): 141 -> 87 us.  Eight rows of 32 768 in clusters of eight, one exchange instead of two and gamma
 // asked for ahead of the wait: the registry transformer at batch 8 192.0 -> 189.9 us (four norms), at batch 1 from host arrays 235 -> 228 us.
 #include "common.h"
+#include "epilogue.cuh"
 #include "launch.cuh"
 #include "planes.cuh"
 
@@ -24,23 +25,6 @@ __device__ __forceinline__ void nr_cluster_wait() { asm volatile("barrier.cluste
 
 template <bool MAX>
 __device__ __forceinline__ float combine(float a, float b) { return MAX ? fmaxf(a, b) : a + b; }
-
-// x * sigmoid(x) with two special-function instructions (expf and a division: a third more time on a GroupNorm).  exp(-x) = 2^t with
-// t = -x log2 e.  What rounding t loses goes back in as a first-order factor: the constant in two parts (W. J. Cody and W. Waite,
-// Software Manual for the Elementary Functions, 1980), the product's rounding error by fused multiply-add, 2^d = 1 + d ln 2 for
-// |d| < 1.2e-5 (the next term is 4e-11).  With 2^-22 for each of the two instructions the result is within 2^-21 of its value for
-// -87.3 <= x, infinity included: above 64 it is x itself (2^t is 0 next to 1; the bound keeps `lost` finite).  Below -87.3 the
-// reciprocal is flushed and the result is -0, off by less than 1.2e-36; -inf gives NaN, as x * (1 / (1 + expf(-x))) does.
-__device__ __forceinline__ float nr_silu(float x) {
-  const float c = fminf(fmaxf(x, -88.0f), 64.0f);
-  const float t = c * -1.44269504f;
-  const float lost = fmaf(c, -1.44269504f, -t) - c * 1.92596e-8f;  // log2 e = 1.44269502163 + 1.92596e-8
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
-  e = fmaf(e, lost * 0.69314718f, e);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return x * r;
-}
 
 struct RowShared {
   float warp[3][NR_MAX_THREADS / 32];
@@ -274,7 +258,7 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
       }
       if (p.act == MIMIR_B200_ELT_SILU) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r[e] = nr_silu(r[e]);
+        for (int e = 0; e < 4; ++e) r[e] *= logistic(r[e]);
       }
       if (p.residual != nullptr) {
         const float* q = p.residual + base + i;

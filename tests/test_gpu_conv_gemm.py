@@ -440,3 +440,44 @@ def test_planes_are_kept_where_their_ring_costs_less_than_laying_them_out(rt, mo
     apart, _, least, _ = plan_and_run(rt, descs, ws, x, batch, oc * h * w)
     assert (arena > least) == kept
     assert np.array_equal(got, apart)  # the same sums in the same order
+
+
+def silu_arguments(n):
+    """fp32 values over the range where SiLU is no subnormal, and their SiLU in 64 bits."""
+    import torch
+
+    beta = torch.linspace(-87.0, 70.0, n, device="cuda") + torch.rand(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    return beta, torch.nn.functional.silu(beta.double())
+
+
+# two special-function instructions of 2^-22 each; rounding of the product and, where a sum follows, of the sum
+SILU_BOUND = 2.0**-21 + 2.0**-23
+
+
+def test_silu_of_a_normed_residual_over_the_whole_range(rt):
+    """gamma = 0: the residual is SiLU(beta) of each channel, and the convolution that it is added to adds zeros."""
+    import torch
+
+    batch, ic, oc, h = 5, 32, 160, 120
+    x, w1, _, _, w2 = residual_case(ic, oc, 3, 3, batch, h, h, 1)
+    beta, want = silu_arguments(oc)
+    got = run_residual(rt, residual_graph(ic, oc, h, h, 3, 3, 32), {0: w1, 1: torch.cat([torch.zeros_like(beta), beta]), 3: torch.zeros_like(w2)}, x, oc)
+    want = want.view(1, oc, 1, 1)
+    assert bool(((got - want).abs() <= SILU_BOUND * want.abs()).all())
+
+
+@pytest.mark.parametrize("oc,groups", [(8, 4), (3, 2)])
+def test_silu_of_a_direct_convolution_over_the_whole_range(rt, oc, groups):
+    """gamma = 0, and an output channel takes one input channel with weight one."""
+    import torch
+
+    batch, ic, h, w = 1, 64, 1024, 512  # 128 MB in a few rows: the convolution normalises
+    beta, want = silu_arguments(ic)
+    x = torch.randn(batch, ic, h, w, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    for first in range(0, ic, oc):
+        pick = [min(first + o, ic - 1) for o in range(oc)]
+        wt = torch.zeros(oc, ic, 1, 1, device="cuda")
+        wt[range(oc), pick] = 1.0
+        got = run_on_device(rt, head_graph(ic, oc, h, w, 1, groups), {1: torch.cat([torch.zeros_like(beta), beta]), 3: wt}, x, (batch, oc, h, w))
+        exact = want[pick].view(1, oc, 1, 1)
+        assert bool(((got - exact).abs() <= SILU_BOUND * exact.abs()).all())
