@@ -402,12 +402,22 @@ struct SmallOcGeom {
   static constexpr int TILE = SO_CC * TH * TWP, WOFF = (SO_NBUF * TILE + 3) & ~3;
 };
 
+// CTAs of an SM that the compiler makes room for in registers (0: it chooses).  Four, in 64 registers, where a form of one to three channels then
+// spills next to nothing: the normalising 3 x 3 to 3 channels (12 bytes) takes the UNet's 512 tiles in one round, 376 us against 389 in 80
+// registers; the plain 1 x 1 on 16 x 128 of 256^2 298 against 340.  The plain 3 x 3 to 3 channels loses by it: 16 x 64 of 128^2 82 us
+// against 77 in 93 registers, one image of 256^2 64 against 59.  Element by element with 7 x 7 the compiler's own choice is better for 3, 6 and 7
+// channels (16 x 64 of 128 x 126: 203, 305 and 348 us against 206, 321 and 356), and one is for the rest (8 channels 385 against 411, 5 x 5
+// 234 against 244).
+constexpr int so_ctas(int oc, int ks, int vec, int norm) {
+  if (!vec) return ks == 7 && (oc == 3 || oc == 6 || oc == 7) ? 0 : 1;
+  return oc <= 3 && ks <= 3 && (norm || ks == 1 || oc < 3) ? 4 : 1;
+}
+
 // NORM: x is the input of a GroupNorm (+ SiLU), which every thread applies to the chunks it has copied itself, between their arrival and the barrier
 // that lets the others read them; the padding ring stays zero.  A tensor less written and read: 16 x 128 channels at 256^2, GroupNorm's
 // sweep and the convolution to 3 channels 473 -> 376 us.
-// (Four CTAs to an SM where the accumulators allow: the UNet's 512 tiles are then one round; at 80 registers they were two, 389 us.)
 template <int OC, int KS, int R, int VEC, int NORM>
-__global__ void __launch_bounds__(SO_TX * SO_TY, VEC && OC <= 3 && KS <= 3 ? 4 : 1) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(SO_TX * SO_TY, so_ctas(OC, KS, VEC, NORM)) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                        float* __restrict__ y, const float* __restrict__ residual, int ic,
                                                                        int h, int wd, int act, const float4* __restrict__ coef, int pre_silu) {
   static_assert(VEC || !NORM, "whole chunks");
