@@ -861,11 +861,15 @@ int mimir_b200_linear_forward_ex(const float* input, const float* weights, const
     MB_TRY(t.alloc(&wsplit, split_bytes(out_f, in_f, wp), "linear.wsplit"));
     if (plane_format() == PLANES_F16) {
       void* word;
-      MB_TRY(t.alloc(&word, sizeof(unsigned), "linear.wmax"));
-      MB_TRY(launch_absmax(e.w_f32, static_cast<size_t>(out_f) * in_f, static_cast<unsigned*>(word), nullptr));
-      e.w_amax = static_cast<const unsigned*>(word);
+      if (t.alloc(&word, sizeof(unsigned), "linear.wmax") == MIMIR_B200_OK) {
+        MB_TRY(launch_absmax(e.w_f32, static_cast<size_t>(out_f) * in_f, static_cast<unsigned*>(word), nullptr));
+        e.w_amax = static_cast<const unsigned*>(word);
+      } else {  // a budget that ends here: the host waits for the scale instead
+        cudaGetLastError();
+        MB_TRY(weight_plane_scale(e.w_f32, static_cast<size_t>(out_f) * in_f, nullptr, &e.w_scale));
+      }
     }
-    MB_TRY(launch_split(e.w_f32, static_cast<__nv_bfloat16*>(wsplit), out_f, in_f, wp, nullptr, 1.0f, e.w_amax));
+    MB_TRY(launch_split(e.w_f32, static_cast<__nv_bfloat16*>(wsplit), out_f, in_f, wp, nullptr, e.w_scale, e.w_amax));
     e.w_split = static_cast<const __nv_bfloat16*>(wsplit);
   }
   MB_TRY(linear_exec(e, nullptr));

@@ -171,3 +171,22 @@ def test_infinities_that_a_layernorm_makes(rt, precision, what, m, n, k):
         want = h[:, at:at + 1] * w[:, at]
     assert np.all(np.isinf(h[:, at])) and np.isnan(want).any() and np.isinf(want).any()
     assert np.array_equal(got, want, equal_nan=True)
+
+
+def test_a_linear_on_host_arrays_whose_budget_ends_at_its_planes(rt):
+    """Room for the arrays and the operand planes to the byte, and none for the word of the weights' largest magnitude."""
+    rows, k, n = 256, 256, 256
+    r = np.random.default_rng(7)
+    x, w = (r.standard_normal(s).astype(np.float32) for s in ((rows, k), (n, k)))
+    want = rt.linear_forward(x, w, None, rows, k, n).copy()
+    need = 4 * (rows * k + n * k + rows * n) + 4 * rows * k + 4 * n * k  # two planes of two bytes
+    stats = rt.guard_stats()
+    rt.check(rt.lib().mimir_b200_guard_set_limit(stats["current"] + need))
+    try:
+        got = rt.linear_forward(x, w, None, rows, k, n)
+        rt.check(rt.lib().mimir_b200_guard_set_limit(stats["current"] + need - 1))
+        with pytest.raises(rt.MimirB200Error):
+            rt.linear_forward(x, w, None, rows, k, n)
+    finally:
+        rt.check(rt.lib().mimir_b200_guard_set_limit(stats["limit"]))
+    assert np.array_equal(got, want)
