@@ -481,3 +481,65 @@ def test_silu_of_a_direct_convolution_over_the_whole_range(rt, oc, groups):
         got = run_on_device(rt, head_graph(ic, oc, h, w, 1, groups), {1: torch.cat([torch.zeros_like(beta), beta]), 3: wt}, x, (batch, oc, h, w))
         exact = want[pick].view(1, oc, 1, 1)
         assert bool(((got - exact).abs() <= SILU_BOUND * exact.abs()).all())
+
+
+@pytest.mark.parametrize("form", ["apart", "residual"])
+def test_moments_of_infinities_overflows_and_far_means(rt, form):
+    """conv + r -> GroupNorm -> SiLU on more than 32 MB, of which r gives one group of a sample an infinity or a NaN (the group becomes NaN, and no
+    other changes a bit), values whose squares overflow (beta is left), or a mean of 700 deviations."""
+    import torch
+
+    batch, ic, oc, h, groups = 16, 32, 96, 80, 24
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x, w1, w2 = randn(batch, ic, h, h), randn(oc, ic, 3, 3) / (9 * ic) ** 0.5, randn(oc, ic, 3, 3) / (9 * ic) ** 0.5
+    g, b = 1 + 0.2 * randn(oc), 0.5 * randn(oc)
+    conv = lambda name, i, o: make_desc(name, "Conv2d", inputs=[i], output=o, in_channels=ic, out_channels=oc, input_height=h, input_width=h, kernel=3, stride=1,  # noqa: E731
+                                        padding=1, params_count=w1.numel())
+    sums = [conv("c1", "x", "a"), make_desc("add", "Add", inputs=["a", "r"], output="s")]
+    norm = [make_desc("g", "GroupNorm", inputs=["s"], output="n", in_channels=oc, input_height=h, input_width=h, num_groups=groups, affine=1, use_bias=1, eps=1e-5,
+                      params_count=2 * oc), make_desc("silu", "SiLU", inputs=["n"], output="x" if form == "apart" else "t")]
+    rest = [] if form == "apart" else [conv("c2", "x", "d"), make_desc("add2", "Add", inputs=["t", "d"], output="x")]
+
+    def run(descs, r, launches=None):
+        m = rt.GraphModel(descs)
+        m.upload_weights(0, w1.cpu().numpy().ravel())
+        if len(descs) > 2:
+            m.upload_weights(2, torch.cat([g, b]).cpu().numpy())
+        if len(descs) > 4:
+            m.upload_weights(4, w2.cpu().numpy().ravel())
+        m.plan({"x": (ic * h * h, False), "r": (oc * h * h, False)}, batch)
+        got = torch.empty(batch, oc, h, h, device="cuda")
+        torch.cuda.synchronize()
+        before = rt.stats()["kernels_launched"]
+        m.forward_device({"x": (x.data_ptr(), ic * h * h, False), "r": (r.data_ptr(), oc * h * h, False)}, batch, got.data_ptr(), got.numel())
+        torch.cuda.synchronize()
+        if launches is not None:  # planes, convolution, moments merged, then the GroupNorm or (coefficients, planes, convolution)
+            assert rt.stats()["kernels_launched"] - before == launches
+        m.close()
+        return got
+
+    last = [make_desc("add", "Add", inputs=["a", "r"], output="x")]
+    run_all = lambda r: run(sums + norm + rest, r, 4 if form == "apart" else 6)  # noqa: E731
+    r0 = randn(batch, oc, h, h)
+    clean = run_all(r0)
+    for value in (float("inf"), float("-inf"), float("nan")):
+        r = r0.clone()
+        r[1, 5, h - 1, 17] = value
+        got = run_all(r)
+        assert bool(got[1, 4:8].isnan().all())
+        got[1, 4:8] = clean[1, 4:8]
+        assert torch.equal(got, clean)
+    r = r0.clone()
+    r[2, 8:12] *= 1e22
+    r[3, 12:16] += 700.0
+    got, plain = run_all(r), run([sums[0]] + last, r)
+    other = torch.nn.functional.conv2d(x.double(), w2.double(), padding=1) if rest else torch.zeros_like(got)
+    want = torch.nn.functional.silu(b.double())[8:12].view(4, 1, 1) + other[2, 8:12]
+    assert bool(((got[2, 8:12] - want).abs() <= 2e-6 * (1 + want.abs()) + (4e-5 if rest else 0.0)).all())  # (the second convolution's own error: 4e-6 of its norm)
+    n = torch.nn.functional.group_norm(plain[3:4].double(), groups, g.double(), b.double(), 1e-5)
+    want = torch.nn.functional.silu(n)[0, 12:16] + other[3, 12:16]
+    # the mean, its product with 1 / std and the sum are rounded at 700 deviations each
+    assert bool(((got[3, 12:16] - want).abs() <= 4 * 700 * 2.0**-24 * 1.1 * g[12:16].abs().max() + (4e-5 if rest else 0.0)).all())
+    got[2, 8:12], got[3, 12:16] = clean[2, 8:12], clean[3, 12:16]
+    assert torch.equal(got, clean)

@@ -203,3 +203,33 @@ def test_linear_with_a_residual_into_operand_planes(rt, rows, k, n):
     got = mod.forward({"x": (x.ravel(), False)}, 1, rows * 64).reshape(want.shape)
     mod.close()
     assert np.linalg.norm(got - want) <= (contraction_bound(k) + 2 * contraction_bound(n)) * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("tokens,d", [(40, 64), (200, 128), (33, 1088), (128, 4096)])
+def test_layernorm_into_a_single_operand_plane(rt, tokens, d):
+    """PREC_BF16, one plane: the bits of the LayerNorm and the Linear one after the other."""
+    r = np.random.default_rng(tokens * d)
+    n, batch, f = tokens * d, 2, 72
+    x = (r.standard_normal((batch, n)) + 0.5).astype(np.float32)
+    g, be = (1 + 0.1 * r.standard_normal(d)).astype(np.float32), r.standard_normal(d).astype(np.float32)
+    w, b = (r.standard_normal((f, d)) / np.sqrt(d)).astype(np.float32), r.standard_normal(f).astype(np.float32)
+    lin = lambda i: abi.make_desc("l", "Linear", inputs=[i], output="x", in_features=d, out_features=f, seq_len=tokens, use_bias=1, params_count=f * d + f)  # noqa: E731
+    norm = lambda o: abi.make_desc("n", "LayerNorm", inputs=["a"], output=o, in_features=d, affine=1, use_bias=1, eps=1e-5, params_count=2 * d)  # noqa: E731
+    act = abi.make_desc("a", "ReLU", inputs=["x"], output="a")
+
+    def run(descs, values, per_in, per_out):
+        mod = rt.GraphModel(descs, abi.PREC_BF16)
+        for i, desc in enumerate(descs):
+            if desc.params_count:
+                mod.upload_weights(i, np.concatenate([g, be]) if desc.type == b"LayerNorm" else np.concatenate([w.ravel(), b]))
+        mod.plan({"x": (per_in, False)}, batch)
+        got = mod.forward({"x": (values, False)}, batch, per_out).copy()
+        mod.close()
+        return got
+
+    got = run([act, norm("h"), lin("h")], x.ravel(), n, tokens * f)
+    h = run([act, norm("x")], x.ravel(), n, n)
+    assert np.array_equal(got, run([lin("x")], h.ravel(), n, tokens * f))
+    # what one plane of 8 or 11 bits per operand leaves
+    want = h.reshape(batch, tokens, d).astype(np.float64) @ w.astype(np.float64).T + b
+    assert np.linalg.norm(got.reshape(want.shape) - want) <= 2.0**-7 * np.linalg.norm(want)
