@@ -6,7 +6,7 @@
 // to 2 MB (a copy command costs about 8 us on these hosts whatever its size, so small segments from several threads gave
 // 15 GB/s, and 2 MB to the host in four of them took 95 us where one takes 46).  To the device the first segments are small, so that the
 // link starts early; to the host the last one is, so that little is left to move when the link is done.  The helpers make no CUDA calls.  Used from COPY_MIN bytes up, with helpers
-// from two pieces up (waking them costs more than one piece), and for pageable memory only; page-locked memory goes straight to cudaMemcpyAsync.
+// from HELP_MIN up (waking them costs more than a piece), and for pageable memory only; page-locked memory goes straight to cudaMemcpyAsync.
 //   9.4 MB to the device 0.51 -> 0.25 ms, 6.3 MB to the host 0.31 -> 0.20 ms, 64 MB 4.4 -> 1.6 and 1.8 ms (42 and 38 GB/s)
 #include <immintrin.h>
 
@@ -24,6 +24,7 @@ namespace {
 
 constexpr size_t COPY_MIN = size_t(64) << 10;
 constexpr size_t PIECE = size_t(64) << 10;
+constexpr size_t HELP_MIN = size_t(88) << 10;  // in and out of an element-wise layer: 72 KB 45 us with helpers, 43 without; 88 KB 46 and 47; 128 KB 50 and 66
 constexpr size_t SEGMENT = size_t(2) << 20;
 constexpr int RING = 8;  // segments: 16 MB of page-locked memory per device
 constexpr int MAX_HELPERS = 5;
@@ -254,7 +255,7 @@ struct HostCopier {
       *taken = false;
       return MIMIR_B200_OK;
     }
-    if (j.pieces > 1) {  // (a single piece is the caller's own)
+    if (j.bytes >= HELP_MIN) {  // (the caller moves less by itself)
       {
         std::lock_guard<std::mutex> lk(mu);
         job = &j;
