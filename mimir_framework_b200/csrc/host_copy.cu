@@ -233,8 +233,9 @@ struct HostCopier {
     return e;
   }
 
-  // Does another thread's copy, which may stand behind its kernels, hold one of the first slots?  (A thread's own earlier copies are
-  // of the same call, or done: its copy in and its copy out are on different streams.)
+  // Does another thread's copy, which may stand behind its kernels, hold one of the first slots?  (A thread's own earlier copies are done, or
+  // copies in of the same call.  Waiting for one of these before a slot is used again waits for nothing that this copy does not stand
+  // behind itself: on one stream it is ahead of it, and a copy out on a stream of its own follows the kernels that read what came in.)
   bool held_by_others(const Job& j) {
     for (size_t s = 0; s < j.segments && s < RING; ++s)
       if (in_flight[s] && by[s] != std::this_thread::get_id()) {
