@@ -1280,7 +1280,7 @@ int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, in
     LayerRT& P = m->layers[xt.producer];
     if (P.lt != LT::Conv2d || P.skip || P.gn_emit_for >= 0 || P.res_norm >= 0 || P.planes_from >= 0 || root_of(m->tensors, P.out_v) != xr || P.d.out_channels != G.ch) continue;
     if (!conv_can_emit_gn(batch, P.d.in_channels, P.d.out_channels, P.h, P.w, P.d.kernel, P.d.stride, P.d.padding, m->precision, G.d.num_groups,
-                          P.d.activation ? MIMIR_B200_ELT_RELU : P.fused_act, P.res_up))
+                          P.d.activation ? MIMIR_B200_ELT_RELU : P.fused_act, P.res_up, G.skip))
       continue;
     P.gn_emit_for = li;
     G.gn_stats_from = xt.producer;

@@ -174,8 +174,10 @@ struct ConvExec {
   float gn_eps = 1e-5f;
 };
 size_t conv_prenorm_bytes(int batch, int groups);
-// can this convolution's epilogue emit the statistics of a GroupNorm with `groups` groups over its output, and should it?
-bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int groups, int act, bool res_up);
+// can this convolution's epilogue emit the statistics of a GroupNorm with `groups` groups over its output, and should it?  (folded: into what
+// reads the GroupNorm)
+bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int groups, int act, bool res_up,
+                      bool folded);
 // may its residual be a GroupNorm's input?  conv_normed_residual_bytes() of workspace then
 bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act);
 // may it read the operand planes of another convolution of the same tensor, with their ring of so many pixels, and should it?

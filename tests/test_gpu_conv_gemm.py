@@ -485,11 +485,11 @@ def test_silu_of_a_direct_convolution_over_the_whole_range(rt, oc, groups):
 
 @pytest.mark.parametrize("form", ["apart", "residual"])
 def test_moments_of_infinities_overflows_and_far_means(rt, form):
-    """conv + r -> GroupNorm -> SiLU on more than 32 MB, of which r gives one group of a sample an infinity or a NaN (the group becomes NaN, and no
+    """conv + r -> GroupNorm -> SiLU on more than 96 MB, of which r gives one group of a sample an infinity or a NaN (the group becomes NaN, and no
     other changes a bit), values whose squares overflow (beta is left), or a mean of 700 deviations."""
     import torch
 
-    batch, ic, oc, h, groups = 16, 32, 96, 80, 24
+    batch, ic, oc, h, groups = 42, 32, 96, 80, 24
     gen = torch.Generator(device="cuda").manual_seed(9)
     randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
     x, w1, w2 = randn(batch, ic, h, h), randn(oc, ic, 3, 3) / (9 * ic) ** 0.5, randn(oc, ic, 3, 3) / (9 * ic) ** 0.5
@@ -543,3 +543,28 @@ def test_moments_of_infinities_overflows_and_far_means(rt, form):
     assert bool(((got[3, 12:16] - want).abs() <= 4 * 700 * 2.0**-24 * 1.1 * g[12:16].abs().max() + (4e-5 if rest else 0.0)).all())
     got[2, 8:12], got[3, 12:16] = clean[2, 8:12], clean[3, 12:16]
     assert torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("batch,ic,oc,h,k,groups,emits", [(16, 64, 128, 96, 3, 32, False), (16, 64, 64, 168, 1, 16, False), (22, 64, 96, 112, 1, 24, True), (35, 32, 64, 108, 3, 8, True)])
+def test_moments_are_taken_where_a_sweep_costs_more(rt, batch, ic, oc, h, k, groups, emits):
+    """A convolution and a GroupNorm of its own, by launches: planes, convolution, GroupNorm, and one that merges the moments."""
+    import torch
+
+    x, w1, g, b, _ = residual_case(ic, oc, k, 1, batch, h, h, oc + h)
+    descs = residual_graph(ic, oc, h, h, k, 1, groups)[:3]
+    descs[2] = make_desc("s", "SiLU", inputs=["b"], output="x")
+    m = rt.GraphModel(descs)
+    m.upload_weights(0, w1.cpu().numpy().ravel())
+    m.upload_weights(1, torch.cat([g, b]).cpu().numpy())
+    m.plan({"x": (ic * h * h, False)}, batch)
+    got = torch.empty(batch, oc, h, h, device="cuda")
+    torch.cuda.synchronize()
+    before = rt.stats()["kernels_launched"]
+    m.forward_device({"x": (x.data_ptr(), ic * h * h, False)}, batch, got.data_ptr(), got.numel())
+    torch.cuda.synchronize()
+    assert rt.stats()["kernels_launched"] - before == (4 if emits else 3)
+    m.close()
+    f = torch.nn.functional
+    for i in range(0, batch, 8):
+        want = f.silu(f.group_norm(f.conv2d(x[i:i + 8].double(), w1.double(), padding=k // 2), groups, g.double(), b.double(), 1e-5))
+        assert (got[i:i + 8] - want).norm() <= 3e-5 * want.norm()
