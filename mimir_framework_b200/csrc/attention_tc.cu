@@ -27,6 +27,7 @@
 // Every mbarrier wait is bounded; on expiry the CTA raises its abort flag, sets the device error word,
 // leaves all loops and frees its TMEM.
 #include "common.h"
+#include "epilogue.cuh"
 #include "launch.cuh"
 #include "planes.cuh"
 #include "sm100_ptx.cuh"
@@ -481,23 +482,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Two single-precision operations in one issue slot, and a maximum of three (with a mask that is one comparison per key: 244 -> 240 us)
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-  unsigned long long v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-  return v;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
+// A maximum of three (with a mask that is one comparison per key and two operations in one issue slot: 244 -> 240 us)
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));

@@ -402,20 +402,20 @@ struct SmallOcGeom {
   static constexpr int TILE = SO_CC * TH * TWP, WOFF = (SO_NBUF * TILE + 3) & ~3;
 };
 
-// CTAs of an SM that the compiler makes room for in registers (0: it chooses).  Four, in 64 registers, where a form of one to three channels then
-// spills next to nothing: the normalising 3 x 3 to 3 channels (12 bytes) takes the UNet's 512 tiles in one round, 376 us against 389 in 80
-// registers; the plain 1 x 1 on 16 x 128 of 256^2 298 against 340.  The plain 3 x 3 to 3 channels loses by it: 16 x 64 of 128^2 82 us
-// against 77 in 93 registers, one image of 256^2 64 against 59.  Element by element with 7 x 7 the compiler's own choice is better for 3, 6 and 7
-// channels (16 x 64 of 128 x 126: 203, 305 and 348 us against 206, 321 and 356), and one is for the rest (8 channels 385 against 411, 5 x 5
-// 234 against 244).
+// CTAs of an SM that the compiler makes room for in registers (0: it chooses).  Four, in 64 registers, for forms of one to three channels with few
+// spills, or none: the plain 1 x 1 to 3 channels on 16 x 128 of 256^2 298 us against 340, the normalising ones to 1 and 3 channels, with the
+// statistics, 460 and 510 against 512 and 525 in 80 registers.  The 3 x 3 to 3 channels loses by it: normalising, 16 x 128 of 256^2 669 us against
+// 644 with three, plain, 16 x 64 of 128^2 82 against 77 with one and one image of 256^2 64 against 59.  Element by element with 7 x 7 the
+// compiler's own choice is better for 3, 6 and 7 channels (16 x 64 of 128 x 126: 203, 305 and 348 us against 206, 321 and 356), and one is
+// for the rest (8 channels 385 against 411, 5 x 5 234 against 244).
 constexpr int so_ctas(int oc, int ks, int vec, int norm) {
   if (!vec) return ks == 7 && (oc == 3 || oc == 6 || oc == 7) ? 0 : 1;
-  return oc <= 3 && ks <= 3 && (norm || ks == 1 || oc < 3) ? 4 : 1;
+  if (oc == 3 && ks == 3) return norm ? 3 : 1;
+  return oc <= 3 && ks <= 3 ? 4 : 1;
 }
 
 // NORM: x is the input of a GroupNorm (+ SiLU), which every thread applies to the chunks it has copied itself, between their arrival and the barrier
-// that lets the others read them; the padding ring stays zero.  A tensor less written and read: 16 x 128 channels at 256^2, GroupNorm's
-// sweep and the convolution to 3 channels 473 -> 376 us.
+// that lets the others read them; the padding ring stays zero.  A tensor less written and read (conv_small_oc_pays_norm has the figures).
 template <int OC, int KS, int R, int VEC, int NORM>
 __global__ void __launch_bounds__(SO_TX * SO_TY, so_ctas(OC, KS, VEC, NORM)) conv_small_oc_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                        float* __restrict__ y, const float* __restrict__ residual, int ic,
@@ -504,8 +504,10 @@ __global__ void __launch_bounds__(SO_TX * SO_TY, so_ctas(OC, KS, VEC, NORM)) con
       const bool b = csrc[k] >= second;
       const float m = b ? k1.x : k0.x, a = b ? k1.y : k0.y, o = b ? k1.z : k0.z;
       float4 v = *reinterpret_cast<const float4*>(tile + 4 * cell(k));
-      v.x = fmaf(v.x - m, a, o); v.y = fmaf(v.y - m, a, o); v.z = fmaf(v.z - m, a, o); v.w = fmaf(v.w - m, a, o);
-      if (pre_silu) { v.x *= logistic(v.x); v.y *= logistic(v.y); v.z *= logistic(v.z); v.w *= logistic(v.w); }
+      const unsigned long long m2 = pack2(-m, -m), a2 = pack2(a, a), o2 = pack2(o, o);
+      unpack2(fma2(add2(pack2(v.x, v.y), m2), a2, o2), v.x, v.y);
+      unpack2(fma2(add2(pack2(v.z, v.w), m2), a2, o2), v.z, v.w);
+      if (pre_silu) { silu2(v.x, v.y); silu2(v.z, v.w); }
       *reinterpret_cast<float4*>(tile + 4 * cell(k)) = v;
     }
   };

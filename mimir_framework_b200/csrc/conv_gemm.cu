@@ -312,15 +312,11 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               }
               if (f.res_silu) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = fmaf(q[j], logistic(q[j]), v[j]);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += q[j];
+                for (int j = 0; j < 32; j += 2) silu2(q[j], q[j + 1]);
               }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += q[j];
             }
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += q[j];
             if (ci + 1 < chunks) request(ci + 1);
           }
           if (in) {

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(WARP ? 128 : NR_MAX_THREADS, WARP ? 8 : 2) nor
       }
       if (p.act == MIMIR_B200_ELT_SILU) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r[e] *= logistic(r[e]);
+        for (int e = 0; e < 4; e += 2) silu2(r[e], r[e + 1]);
       }
       if (p.residual != nullptr) {
         const float* q = p.residual + base + i;
