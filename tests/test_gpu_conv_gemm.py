@@ -131,10 +131,9 @@ def test_tiles_of_128_pixels_keep_the_bits_of_256(rt, monkeypatch, precision, ba
 @pytest.mark.parametrize("batch,ic,oc,h,w,groups", [(20, 64, 128, 58, 58, 32), (33, 32, 64, 63, 65, 16), (3, 32, 256, 120, 99, 8), (45, 32, 160, 37, 33, 5), (80, 32, 64, 48, 48, 32),
                                                   (2, 32, 64, 40, 34, 8), (1, 64, 40, 32, 32, 8)])
 def test_groupnorm_statistics_of_a_large_result(rt, form, batch, ic, oc, h, w, groups):
-    """Conv -> GroupNorm -> SiLU on more than 32 MB: the moments come from the convolution's epilogue (four channels and more to a group; the
-    last case, with two, sweeps).  Then a 1 x 1 convolution that the normalised tensor is added to, a convolution that reads it, or
-    nothing.  Tiles cut at the right and the lower edge; values with a mean of several deviations.  In the first form the 1 x 1
-    convolution reads the padded planes that the first one laid out (the two small cases: without the rest)."""
+    """Conv -> GroupNorm -> SiLU on 32 MB and more: the moments come from the convolution's epilogue where a GroupNorm of four channels and more
+    to a group is folded behind few rows or a long sum, else from a sweep.  Then a 1 x 1 convolution that the normalised tensor is
+    added to, a convolution that reads it, or nothing.  Tiles cut at the right and the lower edge; values with a mean of several deviations."""
     import torch
 
     gen = torch.Generator(device="cuda").manual_seed(batch + oc)
@@ -208,7 +207,8 @@ def test_planes_are_not_kept_where_the_budget_has_no_room(rt):
 @pytest.mark.parametrize("silu", [True, False])
 @pytest.mark.parametrize("batch,ic,oc,h,w,k,groups", [(9, 64, 3, 120, 124, 3, 32), (3, 96, 1, 171, 172, 5, 8), (35, 32, 8, 65, 128, 1, 32), (2, 160, 4, 203, 132, 7, 40)])
 def test_direct_convolution_normalises_its_input(rt, silu, batch, ic, oc, h, w, k, groups):
-    """GroupNorm (+ SiLU) read by a convolution to a handful of channels only, on more than 32 MB: tiles cut at every edge, whose ring stays zero."""
+    """GroupNorm (+ SiLU) read by a convolution to a handful of channels only, on more than 32 MB: tiles cut at every edge, whose ring stays zero (in
+    one launch where that is faster, test_direct_convolution_normalises_where_that_is_faster)."""
     import torch
 
     gen = torch.Generator(device="cuda").manual_seed(ic + oc)
@@ -568,3 +568,40 @@ def test_moments_are_taken_where_a_sweep_costs_more(rt, batch, ic, oc, h, k, gro
     for i in range(0, batch, 8):
         want = f.silu(f.group_norm(f.conv2d(x[i:i + 8].double(), w1.double(), padding=k // 2), groups, g.double(), b.double(), 1e-5))
         assert (got[i:i + 8] - want).norm() <= 3e-5 * want.norm()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_BF16X2, abi.PREC_BF16W, abi.PREC_BF16])
+@pytest.mark.parametrize("form,launches", [("apart", 4), ("kept planes", 5), ("own planes", 6)])
+@pytest.mark.parametrize("silu", [True, False])
+def test_moments_and_normed_residuals_of_ragged_images(rt, precision, form, launches, silu):
+    """61 x 67 pixels, cut by every tile, and a mean of half a deviation, by launches: planes, convolution, moments merged, then the GroupNorm, or
+    coefficients and the convolution that normalises its residual, on the planes of the first one or on its own."""
+    import torch
+
+    batch, ic, oc, h, w, groups = 49, 64, 128, 61, 67, 32
+    k2 = 3 if form == "own planes" else 1
+    x, w1, g, b, w2 = residual_case(ic, oc, 3, k2, batch, h, w, 61)
+    descs = residual_graph(ic, oc, h, w, 3, k2, groups, silu)
+    weights = {0: w1, 1: torch.cat([g, b]), len(descs) - 2: w2}
+    if form == "apart":
+        descs = descs[:2 + silu]
+        descs[-1] = make_desc("s", "SiLU", inputs=["b"], output="x") if silu else make_desc(
+            "g", "GroupNorm", inputs=["a"], output="x", in_channels=oc, input_height=h, input_width=w, num_groups=groups, affine=1, use_bias=1, eps=1e-5, params_count=2 * oc)
+        weights = {0: w1, 1: torch.cat([g, b])}
+    m = rt.GraphModel(descs, precision)
+    for i, wt in weights.items():
+        m.upload_weights(i, wt.cpu().numpy().ravel())
+    m.plan({"x": (ic * h * w, False)}, batch)
+    got = torch.empty(batch, oc, h, w, device="cuda")
+    torch.cuda.synchronize()
+    before = rt.stats()["kernels_launched"]
+    m.forward_device({"x": (x.data_ptr(), ic * h * w, False)}, batch, got.data_ptr(), got.numel())
+    torch.cuda.synchronize()
+    assert rt.stats()["kernels_launched"] - before == launches
+    m.close()
+    for i in range(0, batch, 12):
+        want = residual_want(x[i:i + 12], w1, g, b, w2, groups, silu)
+        if form == "apart":
+            want = want - torch.nn.functional.conv2d(x[i:i + 12].double(), w2.double(), padding=k2 // 2)
+        # two contractions of 4e-6, or of one plane of 11 bits per operand (the weights are bfloat16 values)
+        assert (got[i:i + 12] - want).norm() <= (2.0**-9 if precision == abi.PREC_BF16 else 3e-5) * want.norm()

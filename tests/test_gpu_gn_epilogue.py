@@ -1,13 +1,11 @@
-"""GroupNorm statistics out of the producing convolution's GEMM epilogue (MIMIR_B200_GN_EPILOGUE=1, read once per process,
-hence the child process; off by default because it measured slower than the statistics sweep it replaces).
+"""GroupNorm behind convolutions under MIMIR_B200_GN_EPILOGUE=1 (read once per process, hence the child process): the spatial-tile
+convolution's epilogue leaves moments behind wherever it can, not only for the large results that take this form by default.
 
-The convolution's epilogue leaves per-(32-pixel block, 32-channel chunk) sums behind, a small kernel merges them into
-(mean, 1 / std) per (sample, group), and the GroupNorm that follows - on its own, or folded into the next convolution's
-layout pass - reads them instead of sweeping the tensor.  Cases: 4, 8, 16 and 32 channels per group; 128 output channels
-(operands swapped) and 256 (unswapped, CTA pairs where a full wave forms); several samples whose padded grids are not a
-multiple of 32 rows, so that pixel blocks straddle two samples; enough (sample, group) rows for the stand-alone GroupNorm to
-take the statistics it is handed (the row sweeps want one row per SM); a residual Add folded into the convolution; GroupNorm + SiLU
-followed by a convolution (the folded form) and by an Add (the stand-alone form)."""
+The epilogue leaves (mean, second moment, values) per four channels and half tile, a small kernel merges them into (mean, 1 / std) per
+(sample, group), and a GroupNorm that is folded into the next convolution's layout pass reads these instead of sweeping the tensor.  Cases: 4,
+8, 16 and 32 channels per group; images smaller than a tile and cut by one; several samples; a residual Add folded into the
+convolution; GroupNorm + SiLU followed by a convolution (the folded form) and by an Add (a GroupNorm of its own: its rows fit registers
+here and are read once, so that it takes no statistics; test_gpu_conv_gemm.py has the large ones that do)."""
 import os
 import subprocess
 import sys
