@@ -574,13 +574,13 @@ def test_moments_are_taken_where_a_sweep_costs_more(rt, batch, ic, oc, h, k, gro
 @pytest.mark.parametrize("form,launches", [("apart", 4), ("kept planes", 5), ("own planes", 6)])
 @pytest.mark.parametrize("silu", [True, False])
 def test_moments_and_normed_residuals_of_ragged_images(rt, precision, form, launches, silu):
-    """61 x 67 pixels, cut by every tile, and a mean of half a deviation, by launches: planes, convolution, moments merged, then the GroupNorm, or
+    """63 x 78 pixels, cut by every tile, and a mean of half a deviation, by launches: planes, convolution, moments merged, then the GroupNorm, or
     coefficients and the convolution that normalises its residual, on the planes of the first one or on its own."""
     import torch
 
-    batch, ic, oc, h, w, groups = 49, 64, 128, 61, 67, 32
+    batch, ic, oc, h, w, groups = 42, 64, 128, 63, 78, 16
     k2 = 3 if form == "own planes" else 1
-    x, w1, g, b, w2 = residual_case(ic, oc, 3, k2, batch, h, w, 61)
+    x, w1, g, b, w2 = residual_case(ic, oc, 3, k2, batch, h, w, 63)
     descs = residual_graph(ic, oc, h, w, 3, k2, groups, silu)
     weights = {0: w1, 1: torch.cat([g, b]), len(descs) - 2: w2}
     if form == "apart":
