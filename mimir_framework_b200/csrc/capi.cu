@@ -429,10 +429,11 @@ size_t conv_gn_emit_bytes(int batch, int ic, int oc, int h, int w, int ks, int p
 
 // Where the spatial-tile kernel runs the convolution anyway and the sweep that it replaces costs more than taking and merging the moments: the
 // convolution's MMAs have to outlast its stores (not a kernel of 1 x 1 to fewer channels than most of a tile's, whose few epilogue warps
-// set the pace: convolution and GroupNorm, 64 x 64 -> 64 of 88^2 173 -> 181 us), and the result has to be beyond what L2 sweeps: 96 MB for a GroupNorm of its own
-// (16 x 64 -> 128 of 96^2, 75 MB, 77.1 -> 80.3; of 120^2, 118 MB, 131 -> 120), 48 MB for one that is folded (its sweep has a CTA to a row; 16 x 32 -> 64
-// of 96^2, 38 MB, with the convolution behind it 120.2 -> 122.5; 16 x 64 -> 128 of 80^2, 52 MB, with a skip convolution 117.9 -> 112.8), and 32 MB where
-// there are fewer rows than SMs (1 x 64 -> 128 of 256^2 in four groups 192 -> 127).
+// set the pace: convolution and GroupNorm, 64 x 64 -> 64 of 88^2 173 -> 181 us), and the result has to be beyond what L2 sweeps.  A GroupNorm of
+// its own: 96 MB (16 x 64 -> 128 of 96^2 with 1 x 1, 75 MB, 77.1 -> 80.3; of 120^2, 118 MB, 131 -> 120), 56 behind a long sum (with 3 x 3, 75 MB, 106.6 ->
+// 103.8; 16 x 64 -> 64 of 112^2, 51 MB, 113.6 -> 116.6).  One that is folded, whose sweep has a CTA to a row: 48 MB (16 x 32 -> 64 of 96^2, 38 MB, with
+// the convolution behind it 120.2 -> 122.5; 16 x 64 -> 128 of 80^2, 52 MB, with a skip convolution 117.9 -> 112.8), 32 behind a long sum (16 x 128 -> 128
+// of 72^2 182.4 -> 179.2) or with fewer rows than SMs (1 x 64 -> 128 of 256^2 in four groups 192 -> 127).
 bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int groups, int act, bool res_up, bool folded) {
   static const char mode = [] { const char* e = getenv("MIMIR_B200_GN_EPILOGUE"); return e ? e[0] : ' '; }();  // "0": never, "1": wherever it can
   if (mode == '0' || groups <= 0 || oc % groups != 0 || oc / groups % 4 != 0 || oc % 32 != 0) return false;
@@ -440,7 +441,7 @@ bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int strid
   GemmArgs g;
   if (!shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) || conv_gemm_cycles(g) >= 1e30) return false;
   if (mode == '1') return true;
-  const long long from = !folded ? 96 : g.k >= 512 || batch * groups < ctx().sm_count ? 32 : 48;
+  const long long from = !folded ? (g.k >= 512 ? 56 : 96) : g.k >= 512 || batch * groups < ctx().sm_count ? 32 : 48;
   if ((ks == 1 && oc < 96) || static_cast<long long>(batch) * oc * h * w * 4 < (from << 20)) return false;
   return res_up || gemm_takes_spatial(g);
 }
@@ -448,10 +449,11 @@ bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int strid
 size_t conv_normed_residual_bytes(int batch, int oc, int groups) { return conv_prenorm_bytes(batch, groups) + align256(static_cast<size_t>(batch) * oc * sizeof(float4)); }
 
 // A layout pass over the tensor less (64 images of 112^2: 136 us with 128 channels, 70 with 64), where it outweighs the ring (conv_gemm_ring_pays).
-bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int ring) {
+bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int ring,
+                              bool normed_residual) {
   if (ks != 1 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
   GemmArgs g;
-  return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) && conv_gemm_ring_pays(g, ring) && gemm_takes_spatial(g);
+  return shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g) && conv_gemm_ring_pays(g, ring, normed_residual) && gemm_takes_spatial(g);
 }
 
 // The normalised tensor then never exists: from 32 MB on the epilogue's arithmetic costs less than writing it and reading it back, for every kernel

@@ -238,7 +238,7 @@ int launch_gemm_split(const GemmArgs& g, int bk, int bn, int splits, cudaStream_
 // conv_gemm.cu: shifted-GEMM convolutions in tiles of 256 pixels
 double conv_gemm_cycles(const GemmArgs& g);
 long long conv_gemm_tiles(const GemmArgs& g);
-bool conv_gemm_ring_pays(const GemmArgs& g, int ring);
+bool conv_gemm_ring_pays(const GemmArgs& g, int ring, bool normed_residual);
 int launch_conv_gemm(const GemmArgs& g, cudaStream_t st);
 // The scratch of gn_part, and (mean, 1 / sqrt(var + eps)) per (sample, group of a multiple of four channels) from it
 size_t conv_gemm_gn_bytes(const GemmArgs& g);

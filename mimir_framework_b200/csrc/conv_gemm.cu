@@ -527,12 +527,15 @@ double conv_gemm_cycles(const GemmArgs& g) {
 
 // A 1 x 1 convolution on planes that have a ring of `ring` pixels: the layout pass that it saves grows with the input, what the ring costs (tiles
 // of it, stores that cross lines) with the output and the ring.  Two convolutions of one tensor, planes laid out twice and once: 64 x 64 -> 64
-// of 64^2 245 and 231 us, 128 -> 256 of 56^2 627 and 618, 256 -> 256 572 and 548, 64 -> 128 of 112^2 with a normalised residual 682 and 649; but
-// 64 -> 256 of 64^2 555 and 562, 512 -> 1024 of 32^2 (a ring of 13 %) 1809 and 1827, 64 -> 256 of 64^2 with a ring of two (13 %) 802 and 827, and
-// 4 x 128 -> 128 of 96^2, whose 152 tiles are a second wave where 144 were one, 77.6 and 83.3.
-bool conv_gemm_ring_pays(const GemmArgs& g, int ring) {
-  if (g.n > 2 * g.conv_c) return false;
-  if (100ll * (g.conv_h + 2 * ring) * (g.conv_w + 2 * ring) > 108ll * g.conv_h * g.conv_w) return false;
+// of 64^2 245 and 231 us, 128 -> 256 of 56^2 627 and 618, 256 -> 256 572 and 548, 12 x 256 -> 256 of 78^2 372 and 356; but 64 -> 256 of 64^2 555 and
+// 562, 512 -> 1024 of 32^2 (a ring of 13 %) 1809 and 1827, 256 -> 512 of 48^2 (9 %) 322 and 327 (64 -> 64 of 40^2, 10 %, 128 and 125), 64 -> 256 of
+// 64^2 with a ring of two (13 %) 802 and 827, and, where the ring is a third
+// wave of half tiles to two, 4 x 64 -> 128 of 96^2 61.0 and 67.3, a fifth to four 6 x 64 -> 64 of 112^2 84.6 and 86.7.  An epilogue that normalises
+// the residual hides both (6 x 128 -> 128 of 112^2 128 and 118, 4 x 64 -> 128 of 96^2 63.0 and 63.5, 64 x 64 -> 256 of 64^2 398 and 399).
+bool conv_gemm_ring_pays(const GemmArgs& g, int ring, bool normed_residual) {
+  const long long widest = g.n <= 256 ? 111 : 108;  // per cent
+  if (100ll * (g.conv_h + 2 * ring) * (g.conv_w + 2 * ring) > widest * g.conv_h * g.conv_w) return false;
+  if (normed_residual) return true;
   GemmArgs q = g;
   q.conv_src_pad = ring;
   auto waves = [](const GemmArgs& a) {
@@ -540,8 +543,7 @@ bool conv_gemm_ring_pays(const GemmArgs& g, int ring) {
     conv_cycles(a, &px);
     return (tiles_of(a, px) + ctx().sm_count - 1) / ctx().sm_count * (px == CG_N ? 2 : 1);  // of half tiles
   };
-  const long long before = waves(g);
-  return waves(q) <= before || before >= 8;
+  return g.n <= 2 * g.conv_c && 6 * waves(q) <= 7 * waves(g);
 }
 
 size_t conv_gemm_gn_bytes(const GemmArgs& g) {

@@ -1120,7 +1120,7 @@ int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, in
         if (!reads_plain(E) || E.planes_from >= 0 || E.d.padding < 1 || E.d.in_channels != S.d.in_channels || E.h != S.h || E.w != S.w ||
             root_of(m->tensors, E.in_v[0]) != root_of(m->tensors, S.in_v[0]) ||
             !conv_takes_padded_planes(batch, S.d.in_channels, S.d.out_channels, S.h, S.w, S.d.kernel, S.d.stride, S.d.padding, m->precision,
-                                      S.d.activation ? MIMIR_B200_ELT_RELU : S.fused_act, E.d.padding))
+                                      S.d.activation ? MIMIR_B200_ELT_RELU : S.fused_act, E.d.padding, S.res_norm >= 0))
           continue;
         S.planes_from = m->order[q];
         E.ws_until = std::max(E.ws_until, p);

@@ -181,7 +181,8 @@ bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int strid
 // may its residual be a GroupNorm's input?  conv_normed_residual_bytes() of workspace then
 bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act);
 // may it read the operand planes of another convolution of the same tensor, with their ring of so many pixels, and should it?
-bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int ring);
+bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int ring,
+                              bool normed_residual);
 size_t conv_normed_residual_bytes(int batch, int oc, int groups);
 // scratch of the moments it leaves (behind the planes and the pre-norm statistics)
 size_t conv_gn_emit_bytes(int batch, int ic, int oc, int h, int w, int ks, int pad, int precision);

@@ -424,7 +424,7 @@ def test_a_residual_of_few_channels_is_normalised_apart(rt, monkeypatch, batch, 
     assert torch.equal(run_residual(rt, descs, weights, x, oc), got) != folded
 
 
-@pytest.mark.parametrize("batch,c,oc,h,w,k,kept", [(4, 128, 128, 96, 96, 3, False), (4, 64, 256, 64, 64, 3, False), (8, 64, 64, 32, 32, 3, False), (2, 64, 64, 128, 128, 7, False),
+@pytest.mark.parametrize("batch,c,oc,h,w,k,kept", [(4, 128, 128, 96, 96, 3, False), (4, 64, 256, 64, 64, 3, False), (8, 64, 64, 32, 32, 3, False), (2, 64, 64, 96, 96, 7, False), (2, 64, 64, 128, 128, 7, True),
                                                   (3, 64, 100, 61, 67, 3, True), (5, 128, 72, 131, 103, 5, True), (1, 32, 64, 64, 200, 3, True)])
 def test_planes_are_kept_where_their_ring_costs_less_than_laying_them_out(rt, monkeypatch, batch, c, oc, h, w, k, kept):
     """A second wave of tiles, twice as many outputs as inputs and more, a wide ring: planes of its own.  Whether planes are kept shows in the
@@ -545,7 +545,8 @@ def test_moments_of_infinities_overflows_and_far_means(rt, form):
     assert torch.equal(got, clean)
 
 
-@pytest.mark.parametrize("batch,ic,oc,h,k,groups,emits", [(16, 64, 128, 96, 3, 32, False), (16, 64, 64, 168, 1, 16, False), (22, 64, 96, 112, 1, 24, True), (35, 32, 64, 108, 3, 8, True)])
+@pytest.mark.parametrize("batch,ic,oc,h,k,groups,emits", [(16, 32, 128, 96, 3, 32, False), (16, 64, 64, 168, 1, 16, False), (16, 64, 64, 112, 3, 16, False), (22, 64, 96, 112, 1, 24, True), (35, 32, 64, 108, 3, 8, True),
+                                                            (16, 64, 128, 96, 3, 32, True)])
 def test_moments_are_taken_where_a_sweep_costs_more(rt, batch, ic, oc, h, k, groups, emits):
     """A convolution and a GroupNorm of its own, by launches: planes, convolution, GroupNorm, and one that merges the moments."""
     import torch
@@ -605,3 +606,26 @@ def test_moments_and_normed_residuals_of_ragged_images(rt, precision, form, laun
             want = want - torch.nn.functional.conv2d(x[i:i + 12].double(), w2.double(), padding=k2 // 2)
         # two contractions of 4e-6, or of one plane of 11 bits per operand (the weights are bfloat16 values)
         assert (got[i:i + 12] - want).norm() <= (2.0**-9 if precision == abi.PREC_BF16 else 3e-5) * want.norm()
+
+
+@pytest.mark.parametrize("batch,ic,oc,h", [(6, 64, 128, 112), (9, 64, 256, 64)])
+def test_planes_are_kept_for_a_convolution_that_normalises_its_residual(rt, batch, ic, oc, h):
+    """A fifth wave of half tiles to four, four times as many outputs as inputs: by launches, planes, convolution, moments merged, coefficients,
+    convolution."""
+    import torch
+
+    x, w1, g, b, w2 = residual_case(ic, oc, 3, 1, batch, h, h, oc)
+    descs = residual_graph(ic, oc, h, h, 3, 1, 16)
+    m = rt.GraphModel(descs)
+    for i, wt in ((0, w1), (1, torch.cat([g, b])), (3, w2)):
+        m.upload_weights(i, wt.cpu().numpy().ravel())
+    m.plan({"x": (ic * h * h, False)}, batch)
+    got = torch.empty(batch, oc, h, h, device="cuda")
+    torch.cuda.synchronize()
+    before = rt.stats()["kernels_launched"]
+    m.forward_device({"x": (x.data_ptr(), ic * h * h, False)}, batch, got.data_ptr(), got.numel())
+    torch.cuda.synchronize()
+    assert rt.stats()["kernels_launched"] - before == 5
+    m.close()
+    want = residual_want(x, w1, g, b, w2, 16)
+    assert (got - want).norm() <= 3e-5 * want.norm()
