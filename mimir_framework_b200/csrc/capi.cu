@@ -460,9 +460,14 @@ bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, i
 // size and every number of rows (where no moments exist the GroupNorm apart reads its input twice, too), but not with fewer than 96 channels: the
 // epilogue's warps are bound to the channels of a tile of 128, and half of them have nothing to do with 64.  Blocks of two
 // convolutions and a GroupNorm, apart and in here: 64 x 64 -> 128 of 112^2 with 1 x 1 700 and 650 us, 3 x 3 848 and 770, 16 x 256 -> 256 of
-// 64^2 278 and 268, 1 x 64 -> 128 of 256^2 in one group 435 and 368; 64 x 64 -> 96 of 112^2 648 and 594; 64 x 64 -> 64 562 and 585, 32 -> 32 380 and 419.
-bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act) {
-  if (oc % 32 != 0 || oc < 96 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
+// 64^2 278 and 268, 1 x 64 -> 128 of 256^2 in one group 435 and 368; 64 x 64 -> 96 of 112^2 648 and 594; 64 x 64 -> 64 562 and 585, 32 -> 32 380 and 419.  With
+// fewer rows than SMs, and longer than registers, or channels that are no whole vectors, the GroupNorm apart is the slower one all the same (2 x 32 ->
+// 64 of 386^2 in four groups 434 and 353; 64 x 64 -> 64 of 111^2 791 and 583, 64 -> 32 of 113^2 563 and 496).
+bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int groups) {
+  RowNormArgs r;
+  r.rows = static_cast<long long>(batch) * groups; r.len = groups > 0 ? static_cast<long long>(oc / groups) * h * w : 0;
+  if (oc < 96 && h * w % 4 == 0 && (r.rows >= ctx().sm_count || norm_rows_supported(r))) return false;
+  if (groups <= 0 || oc % 32 != 0 || !conv_uses_shifted(ic, ks, stride, pad) || conv_small_oc_supported(oc, ks, stride, pad, h, w, batch, act)) return false;
   GemmArgs g;
   if (!shifted_args(batch, ic, oc, h, w, ks, pad, precision, &g)) return false;
   return static_cast<long long>(batch) * oc * h * w * 4 >= (32ll << 20) && gemm_takes_spatial(g);

@@ -657,7 +657,8 @@ bool conv_small_oc_takes_norm(int h, int wd) { return small_oc_vec(h, wd); }
 // Where that is the faster one.  The normalised tensor is not written and read again, but the convolution, which waits for its own instructions, takes
 // longer: the tensor has to be several times L2 (384 MB), its statistics long rows (a CTA sweeps each), its kernel small.  To 3 channels,
 // 3 x 3, GroupNorm apart and in here: 16 x 128 of 256^2 with 32 groups 703 and 660 us, 8 of them 369 and 363; but 16 x 128 of 128^2 208 and 228,
-// 96 x 64 of 128^2 in rows of two channels 475 and 491, and to 8 channels with 7 x 7 2276 and 2337.  With fewer rows than SMs the GroupNorm that
+// 96 x 64 of 128^2 in rows of two channels 475 and 491, and to 8 channels with 7 x 7 2276 and 2337; to one
+// channel with 1 x 1 256 MB are enough (21 x 96 of 192^2, 297 MB, 657 and 581).  With fewer rows than SMs the GroupNorm that
 // reads and writes is the slower one by far (one that fits registers excepted), and 128 MB are enough: 4 x 64 of 364^2 245 and 199 us, 2 x 128 of
 // 512^2 684 and 411; 3 x 128 of 256^2 (96 MB) 211 and 218.
 bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups) {
@@ -666,7 +667,7 @@ bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, i
   r.rows = static_cast<long long>(batch) * groups; r.len = static_cast<long long>(ic / groups) * h * wd;
   const long long bytes = static_cast<long long>(batch) * ic * h * wd * 4;
   if (r.rows < ctx().sm_count) return bytes >= (128ll << 20) && !norm_rows_supported(r);
-  return bytes >= (384ll << 20) && r.len >= 65536 && oc * ks * ks <= 80;
+  return bytes >= ((oc * ks * ks <= 8 ? 256ll : 384ll) << 20) && r.len >= 65536 && oc * ks * ks <= 80;
 }
 
 int launch_conv_small_oc(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int oc, int h, int wd, int ks,

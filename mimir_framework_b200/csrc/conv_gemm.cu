@@ -531,10 +531,14 @@ double conv_gemm_cycles(const GemmArgs& g) {
 // 562, 512 -> 1024 of 32^2 (a ring of 13 %) 1809 and 1827, 256 -> 512 of 48^2 (9 %) 322 and 327 (64 -> 64 of 40^2, 10 %, 128 and 125), 64 -> 256 of
 // 64^2 with a ring of two (13 %) 802 and 827, and, where the ring is a third
 // wave of half tiles to two, 4 x 64 -> 128 of 96^2 61.0 and 67.3, a fifth to four 6 x 64 -> 64 of 112^2 84.6 and 86.7.  An epilogue that normalises
-// the residual hides both (6 x 128 -> 128 of 112^2 128 and 118, 4 x 64 -> 128 of 96^2 63.0 and 63.5, 64 x 64 -> 256 of 64^2 398 and 399).
+// the residual hides both (6 x 128 -> 128 of 112^2 128 and 118, 4 x 64 -> 128 of 96^2 63.0 and 63.5, 64 x 64 -> 256 of 64^2 398 and 399), and where
+// the image's channel planes do not start on lines the stores cross them in any case and the layout pass is the slower one (64 x 64 -> 256 of 63^2 640
+// and 616, 51 x 256 -> 256 of 33^2, 13 %, 368 and 332, 64 x 128 -> 64 of 37^2 with a ring of two, 23 %, 281 and 265; of 33^2, 25 %, 197 and 203).
 bool conv_gemm_ring_pays(const GemmArgs& g, int ring, bool normed_residual) {
-  const long long widest = g.n <= 256 ? 111 : 108;  // per cent
-  if (100ll * (g.conv_h + 2 * ring) * (g.conv_w + 2 * ring) > widest * g.conv_h * g.conv_w) return false;
+  const long long pixels = static_cast<long long>(g.conv_h) * g.conv_w;
+  const bool crossing = pixels % 32 != 0;
+  const long long widest = crossing ? 123 : normed_residual || g.n <= 256 ? 111 : 108;  // per cent
+  if (100ll * (g.conv_h + 2 * ring) * (g.conv_w + 2 * ring) > widest * pixels) return false;
   if (normed_residual) return true;
   GemmArgs q = g;
   q.conv_src_pad = ring;
@@ -543,7 +547,7 @@ bool conv_gemm_ring_pays(const GemmArgs& g, int ring, bool normed_residual) {
     conv_cycles(a, &px);
     return (tiles_of(a, px) + ctx().sm_count - 1) / ctx().sm_count * (px == CG_N ? 2 : 1);  // of half tiles
   };
-  return g.n <= 2 * g.conv_c && 6 * waves(q) <= 7 * waves(g);
+  return crossing ? 4 * waves(q) <= 5 * waves(g) : g.n <= 2 * g.conv_c && 6 * waves(q) <= 7 * waves(g);
 }
 
 size_t conv_gemm_gn_bytes(const GemmArgs& g) {

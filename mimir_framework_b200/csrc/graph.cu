@@ -1093,7 +1093,7 @@ int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, in
     if (C.lt != LT::Conv2d || C.skip || C.res_v != pv || C.res_up || C.in_v[0] == pv || C.d.out_channels != P.ch || C.h != P.h || C.w != P.w) continue;
     if (m->tensors[pv].n != m->tensors[C.out_v].n || m->tensors[xin].n != m->tensors[pv].n) continue;
     if (!conv_takes_normed_residual(batch, C.d.in_channels, C.d.out_channels, C.h, C.w, C.d.kernel, C.d.stride, C.d.padding, m->precision,
-                                    C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act))
+                                    C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act, P.d.num_groups))
       continue;
     C.res_norm = li;
     C.res_v = xin;

@@ -1127,11 +1127,13 @@ int launch_groupnorm(const float* x, const float* gamma, const float* beta, floa
   return meanvar_dispatch(x, y, static_cast<long long>(batch) * groups, static_cast<long long>(cpg) * hw, eps, a, st);
 }
 
-// Do statistics that already exist save a GroupNorm of its own anything?  Rows that fit registers are read once either way.
+// Do statistics that already exist save a GroupNorm of its own anything?  Rows that fit registers are read once either way, and channels that
+// are no whole vectors leave element by element, one load at a time, which is slower from memory than behind a sweep (14 x 128 of 93^2 with
+// its convolution 236 -> 254 us).
 bool groupnorm_takes_stats(int batch, int ch, int hw, int groups) {
   RowNormArgs r;
   r.rows = static_cast<long long>(batch) * groups; r.len = static_cast<long long>(ch / groups) * hw;
-  return use_sweeps(r.rows, r.len) && !(norm_rows_on() && norm_rows_supported(r));
+  return hw % 4 == 0 && use_sweeps(r.rows, r.len) && !(norm_rows_on() && norm_rows_supported(r));
 }
 
 // GroupNorm whose statistics [batch][groups][2] already exist (they came out of the producing convolution's epilogue): the

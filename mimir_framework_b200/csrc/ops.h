@@ -179,7 +179,7 @@ size_t conv_prenorm_bytes(int batch, int groups);
 bool conv_can_emit_gn(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int groups, int act, bool res_up,
                       bool folded);
 // may its residual be a GroupNorm's input?  conv_normed_residual_bytes() of workspace then
-bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act);
+bool conv_takes_normed_residual(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int groups);
 // may it read the operand planes of another convolution of the same tensor, with their ring of so many pixels, and should it?
 bool conv_takes_padded_planes(int batch, int ic, int oc, int h, int w, int ks, int stride, int pad, int precision, int act, int ring,
                               bool normed_residual);
