@@ -33,7 +33,7 @@ constexpr int CG_THREADS = 352;
 constexpr int CG_N = 256;                      // pixels of a tile: 16 x 16 or, for 1 x 1 kernels, 256 of the flattened image; or half of that
 constexpr int CG_M = 128;                      // output channels of a tile
 constexpr int CG_EPI = 8 * 32 * 33 * 4;
-constexpr int CG_COEF = 8 * 32 * 16;
+constexpr int CG_COEF = 8 * 128 * 4;
 constexpr int CG_MAX_RING = 16;
 constexpr int CG_SMEM_MAX = 232448;
 
@@ -227,7 +227,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // epilogue: TMEM lane = output channel, column = pixel (16 to a row)
     const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
     float* tbuf = epi + ew * (32 * 33);
-    float4* coef = reinterpret_cast<float4*>(epi + CG_EPI / 4) + ew * 32;  // RN: of this warp's 32 channels
+    float* coef = epi + CG_EPI / 4 + ew * 128;  // RN: -mean, gamma / std and beta of this warp's 32 channels, each in a row, for pairs of channels
     const int chunks = p.px / 64;  // of 32 pixels, in each half of the tile
     const long long hw = FLAT ? static_cast<long long>(f.flat_ih) * f.flat_iw : static_cast<long long>(p.h) * p.w;
     int acc = 0;
@@ -266,8 +266,11 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       };
       if (p.residual != nullptr && nch > 0) request(0);
       if (RN && nch > 0) {
+        const float4 k = __ldg(f.res_coef + static_cast<long long>(c.n) * p.oc + oc0 + lane);
         __syncwarp();
-        coef[lane] = __ldg(f.res_coef + static_cast<long long>(c.n) * p.oc + oc0 + lane);
+        coef[lane] = -k.x;
+        coef[32 + lane] = k.y;
+        coef[64 + lane] = k.z;
         __syncwarp();
       }
       int ok = 1;
@@ -306,17 +309,22 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (p.residual != nullptr) {
             if (RN) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const float4 k = coef[j];  // (the same for every lane)
-                q[j] = fmaf(q[j] - k.x, k.y, k.z);
+              for (int j = 0; j < 32; j += 4) {  // (the same for every lane)
+                const float4 m = *reinterpret_cast<const float4*>(coef + j), a = *reinterpret_cast<const float4*>(coef + 32 + j),
+                             o = *reinterpret_cast<const float4*>(coef + 64 + j);
+                unpack2(fma2(add2(pack2(q[j], q[j + 1]), pack2(m.x, m.y)), pack2(a.x, a.y), pack2(o.x, o.y)), q[j], q[j + 1]);
+                unpack2(fma2(add2(pack2(q[j + 2], q[j + 3]), pack2(m.z, m.w)), pack2(a.z, a.w), pack2(o.z, o.w)), q[j + 2], q[j + 3]);
               }
               if (f.res_silu) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) silu2(q[j], q[j + 1]);
               }
-            }
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += q[j];
+              for (int j = 0; j < 32; j += 2) unpack2(add2(pack2(v[j], v[j + 1]), pack2(q[j], q[j + 1])), v[j], v[j + 1]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += q[j];
+            }
             if (ci + 1 < chunks) request(ci + 1);
           }
           if (in) {
