@@ -510,7 +510,7 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     if (e.pre_groups > 0) {
       float* stats = static_cast<float*>(e.ws);
       coef = reinterpret_cast<float4*>(static_cast<uint8_t*>(e.ws) + conv_prenorm_bytes(e.batch, e.pre_groups));
-      if (e.pre_stats == nullptr) MB_TRY(launch_groupnorm_stats(e.x, stats, e.batch, e.ic, e.h * e.w, e.pre_groups, e.pre_eps, st));
+      if (e.pre_stats == nullptr) MB_TRY(launch_groupnorm_stats(e.x, stats, e.batch, e.ic, e.h * e.w, e.pre_groups, e.pre_eps, st, true));
       MB_TRY(launch_gn_coefs(e.pre_stats ? e.pre_stats : stats, e.pre_gamma, e.pre_beta, coef, e.batch, e.ic, e.pre_groups, st));
     }
     return launch_conv_small_oc(e.x, e.w_f32, e.y, e.residual, e.batch, e.ic, e.oc, e.h, e.w, e.ks, e.pad, e.activation, st, coef, e.pre_act == MIMIR_B200_ELT_SILU ? 1 : 0);
@@ -550,7 +550,7 @@ int conv_exec(const ConvExec& e, cudaStream_t st) {
     if (e.res_groups > 0) {
       float* stats = reinterpret_cast<float*>(rest);
       float4* coef = reinterpret_cast<float4*>(rest + conv_prenorm_bytes(e.batch, e.res_groups));
-      if (e.res_stats == nullptr) MB_TRY(launch_groupnorm_stats(e.residual, stats, e.batch, e.oc, e.h * e.w, e.res_groups, e.res_eps, st));
+      if (e.res_stats == nullptr) MB_TRY(launch_groupnorm_stats(e.residual, stats, e.batch, e.oc, e.h * e.w, e.res_groups, e.res_eps, st, true));
       MB_TRY(launch_gn_coefs(e.res_stats ? e.res_stats : stats, e.res_gamma, e.res_beta, coef, e.batch, e.oc, e.res_groups, st));
       g.res_coef = coef;
       g.res_act = e.res_act;

@@ -243,6 +243,8 @@ int launch_conv_gemm(const GemmArgs& g, cudaStream_t st);
 // The scratch of gn_part, and (mean, 1 / sqrt(var + eps)) per (sample, group of a multiple of four channels) from it
 size_t conv_gemm_gn_bytes(const GemmArgs& g);
 int launch_conv_gn_stats(const GemmArgs& g, float* stats, int groups, float eps, cudaStream_t st);
+// stats[2 * row + {0, 1}] = mean, 1 / sqrt(var + eps) from `entries` (mean, second moment about it, values, -) of each row
+int launch_merge_moments(const float4* part, float* stats, int rows, int entries, float eps, cudaStream_t st);
 bool gemm_takes_spatial(const GemmArgs& g);
 // y = act(a · wᵀ + bias) (+ residual); tcgen05 / TMEM / TMA.
 int launch_gemm(const GemmArgs& g, cudaStream_t st);
@@ -351,7 +353,7 @@ int launch_groupnorm(const float* x, const float* gamma, const float* beta, floa
 int launch_softmax(const float* x, float* y, int batch, int64_t n, int log_softmax, cudaStream_t st);
 int launch_gn_coefs(const float* stats, const float* gamma, const float* beta, float4* coef, int batch, int ch, int groups, cudaStream_t st);
 // stats[(sample * groups + g) * 2 + {0, 1}] = mean, 1 / sqrt(var + eps) of each GroupNorm slab
-int launch_groupnorm_stats(const float* x, float* stats, int batch, int ch, int hw, int groups, float eps, cudaStream_t st);
+int launch_groupnorm_stats(const float* x, float* stats, int batch, int ch, int hw, int groups, float eps, cudaStream_t st, bool spread = false);
 bool groupnorm_takes_stats(int batch, int ch, int hw, int groups);
 int launch_groupnorm_apply(const float* x, const float* stats, const float* gamma, const float* beta, float* y, int batch, int ch, int hw,
                            int groups, float eps, int act, const float* residual, cudaStream_t st);
@@ -423,7 +425,7 @@ int launch_conv_weight_planes(const float* w, __nv_bfloat16* dst, int oc, int ic
 bool conv_small_oc_supported(int oc, int ks, int stride, int pad, int h, int wd, int batch, int act);
 // coef (where conv_small_oc_takes_norm() holds and x starts on 16 bytes): x is a GroupNorm's input, from launch_gn_coefs, with SiLU behind it or not
 bool conv_small_oc_takes_norm(int h, int wd);
-bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups);
+bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups, bool moments);
 int launch_conv_small_oc(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int oc, int h, int wd, int ks,
                          int pad, int act, cudaStream_t st, const float4* coef = nullptr, int pre_silu = 0);
 

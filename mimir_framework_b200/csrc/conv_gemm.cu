@@ -538,7 +538,8 @@ double conv_gemm_cycles(const GemmArgs& g) {
 // of 64^2 245 and 231 us, 128 -> 256 of 56^2 627 and 618, 256 -> 256 572 and 548, 12 x 256 -> 256 of 78^2 372 and 356; but 64 -> 256 of 64^2 555 and
 // 562, 512 -> 1024 of 32^2 (a ring of 13 %) 1809 and 1827, 256 -> 512 of 48^2 (9 %) 322 and 327 (64 -> 64 of 40^2, 10 %, 128 and 125), 64 -> 256 of
 // 64^2 with a ring of two (13 %) 802 and 827, and, where the ring is a third
-// wave of half tiles to two, 4 x 64 -> 128 of 96^2 61.0 and 67.3, a fifth to four 6 x 64 -> 64 of 112^2 84.6 and 86.7.  An epilogue that normalises
+// wave of half tiles to two, 4 x 64 -> 128 of 96^2 61.0 and 67.3, a fifth to four 6 x 64 -> 64 of 112^2 84.6 and 86.7 (with half as many
+// outputs as inputs a third more waves pay: 10 x 256 -> 64 of 104^2 542 and 516, 19 x 256 -> 96 of 54^2 200 and 180).  An epilogue that normalises
 // the residual hides both (6 x 128 -> 128 of 112^2 128 and 118, 4 x 64 -> 128 of 96^2 63.0 and 63.5, 64 x 64 -> 256 of 64^2 398 and 399), and where
 // the image's channel planes do not start on lines the stores cross them in any case and the layout pass is the slower one (64 x 64 -> 256 of 63^2 640
 // and 616, 51 x 256 -> 256 of 33^2, 13 %, 368 and 332, 64 x 128 -> 64 of 37^2 with a ring of two, 23 %, 281 and 265; of 33^2, 25 %, 197 and 203).
@@ -555,7 +556,9 @@ bool conv_gemm_ring_pays(const GemmArgs& g, int ring, bool normed_residual) {
     conv_cycles(a, &px);
     return (tiles_of(a, px) + ctx().sm_count - 1) / ctx().sm_count * (px == CG_N ? 2 : 1);  // of half tiles
   };
-  return crossing ? 4 * waves(q) <= 5 * waves(g) : g.n <= 2 * g.conv_c && 6 * waves(q) <= 7 * waves(g);
+  const long long before = waves(g), after = waves(q);
+  if (2 * g.n <= g.conv_c) return 3 * after <= 4 * before;
+  return crossing ? 4 * after <= 5 * before : g.n <= 2 * g.conv_c && 6 * after <= 7 * before;
 }
 
 size_t conv_gemm_gn_bytes(const GemmArgs& g) {
@@ -570,7 +573,11 @@ int launch_conv_gn_stats(const GemmArgs& g, float* stats, int groups, float eps,
   conv_cycles(g, &px);
   const ConvShape sh = conv_shape(g, px);
   const int batch = g.m / ((g.conv_h + 2 * g.conv_pad) * (g.conv_w + 2 * g.conv_pad)), slabs = batch * groups;
-  conv_gn_stats_kernel<<<slabs, 128, 0, st>>>(g.gn_part, stats, g.n / groups / 4 * 2 * sh.tiles_x * sh.tiles_y, eps);
+  return launch_merge_moments(g.gn_part, stats, slabs, g.n / groups / 4 * 2 * sh.tiles_x * sh.tiles_y, eps, st);
+}
+
+int launch_merge_moments(const float4* part, float* stats, int rows, int entries, float eps, cudaStream_t st) {
+  conv_gn_stats_kernel<<<rows, 128, 0, st>>>(part, stats, entries, eps);
   MB_CUDA(cudaGetLastError());
   count_launch();
   return MIMIR_B200_OK;

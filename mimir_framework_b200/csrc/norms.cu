@@ -123,7 +123,8 @@ __device__ __forceinline__ float finish(float xn, long long i, long long row, lo
 }
 
 // ---- chunk kernels (mean / variance) ----------------------------------------------------------
-// pass 1: per chunk (count, mean, M2)
+// pass 1: per chunk (count, mean, M2), or (mean, M2, count, -) for launch_merge_moments
+template <bool MERGED>
 __global__ void meanvar_chunk_stats_kernel(const float* __restrict__ x, float* __restrict__ part, long long len, int chunks,
                                            int chunk_len) {
   extern __shared__ __align__(16) float sch[];
@@ -141,6 +142,10 @@ __global__ void meanvar_chunk_stats_kernel(const float* __restrict__ x, float* _
   }
   const float m2 = block_sum(acc, red);
   if (threadIdx.x == 0) {
+    if (MERGED) {
+      reinterpret_cast<float4*>(part)[row * chunks + c] = make_float4(mean, m2, static_cast<float>(n), 0.0f);
+      return;
+    }
     float* p = part + (row * chunks + c) * 3;
     p[0] = static_cast<float>(n);
     p[1] = mean;
@@ -1050,7 +1055,7 @@ int meanvar_dispatch(const float* x, float* y, long long rows, long long len, fl
     dim3 grid(chunks, static_cast<unsigned>(nr));
     Affine ag = a;
     // the kernels index gamma / residual by absolute row: shift the pointers, keep row numbering
-    meanvar_chunk_stats_kernel<<<grid, 256, CHUNK * 4, st>>>(x + r0 * len, part, len, chunks, CHUNK);
+    meanvar_chunk_stats_kernel<false><<<grid, 256, CHUNK * 4, st>>>(x + r0 * len, part, len, chunks, CHUNK);
     MB_CUDA(cudaGetLastError());
     meanvar_chunk_apply_kernel<<<grid, 256, 0, st>>>(x + r0 * len, y + r0 * len, part, len, chunks, CHUNK, eps, ag, r0);
     MB_CUDA(cudaGetLastError());
@@ -1169,14 +1174,33 @@ int launch_gn_coefs(const float* stats, const float* gamma, const float* beta, f
   return MIMIR_B200_OK;
 }
 
-// (mean, 1 / sqrt(var + eps)) of every (sample, group) slab, for consumers that normalise on the fly
-int launch_groupnorm_stats(const float* x, float* stats, int batch, int ch, int hw, int groups, float eps, cudaStream_t st) {
+// (mean, 1 / sqrt(var + eps)) of every (sample, group) slab, for consumers that normalise on the fly.  `spread`: slabs that are fewer than the SMs
+// and longer than registers go chunk by chunk over all of them, as such a GroupNorm of its own does.  A CTA to a slab reads 70 GB/s, and its
+// threads' long sums were off by 5e-6 of a slab of 32 M values where chunks and their merge in double leave 1e-6 of the result.
+int launch_groupnorm_stats(const float* x, float* stats, int batch, int ch, int hw, int groups, float eps, cudaStream_t st, bool spread) {
   if (groups <= 0 || ch % groups != 0) return fail(MIMIR_B200_E_INVALID, "GroupNorm: channels must be divisible by num_groups");
+  RowNormArgs r;
+  r.rows = static_cast<long long>(batch) * groups; r.len = static_cast<long long>(ch / groups) * hw;
+  const long long chunks = (r.len + CHUNK - 1) / CHUNK, cap_rows = static_cast<long long>(NORM_SCRATCH_BYTES / sizeof(float4)) / (chunks > 0 ? chunks : 1);
+  if (spread && r.rows < ctx().sm_count && r.len > 0 && cap_rows > 0 && !norm_rows_supported(r)) {
+    std::lock_guard<std::mutex> scratch_lock(g_norm_mu);
+    float* part;
+    MB_TRY(norm_scratch(st, &part));
+    for (long long r0 = 0; r0 < r.rows; r0 += cap_rows) {
+      const int nr = static_cast<int>(r.rows - r0 < cap_rows ? r.rows - r0 : cap_rows);
+      meanvar_chunk_stats_kernel<true><<<dim3(static_cast<unsigned>(chunks), static_cast<unsigned>(nr)), 256, CHUNK * 4, st>>>(
+          x + r0 * r.len, part, r.len, static_cast<int>(chunks), CHUNK);
+      MB_CUDA(cudaGetLastError());
+      count_launch();
+      MB_TRY(launch_merge_moments(reinterpret_cast<const float4*>(part), stats + 2 * r0, nr, static_cast<int>(chunks), eps, st));
+    }
+    return MIMIR_B200_OK;
+  }
   RowParams p{};
   p.x = x;
   p.y = const_cast<float*>(x);  // never written on this path
-  p.rows = static_cast<long long>(batch) * groups;
-  p.len = static_cast<long long>(ch / groups) * hw;
+  p.rows = r.rows;
+  p.len = r.len;
   p.eps = eps;
   p.aff = Affine{nullptr, nullptr, 1, groups, ch / groups, hw, -1, nullptr};
   p.stats_out = stats;
