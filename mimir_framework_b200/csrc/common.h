@@ -425,7 +425,7 @@ int launch_conv_weight_planes(const float* w, __nv_bfloat16* dst, int oc, int ic
 bool conv_small_oc_supported(int oc, int ks, int stride, int pad, int h, int wd, int batch, int act);
 // coef (where conv_small_oc_takes_norm() holds and x starts on 16 bytes): x is a GroupNorm's input, from launch_gn_coefs, with SiLU behind it or not
 bool conv_small_oc_takes_norm(int h, int wd);
-bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups, bool moments);
+bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups);
 int launch_conv_small_oc(const float* x, const float* w, float* y, const float* residual, int batch, int ic, int oc, int h, int wd, int ks,
                          int pad, int act, cudaStream_t st, const float4* coef = nullptr, int pre_silu = 0);
 

@@ -658,18 +658,16 @@ bool conv_small_oc_takes_norm(int h, int wd) { return small_oc_vec(h, wd); }
 // longer: the tensor has to be several times L2 (384 MB), its statistics long rows (a CTA sweeps each), its kernel small.  To 3 channels,
 // 3 x 3, GroupNorm apart and in here: 16 x 128 of 256^2 with 32 groups 703 and 660 us, 8 of them 369 and 363; but 16 x 128 of 128^2 208 and 228,
 // 96 x 64 of 128^2 in rows of two channels 475 and 491, and to 8 channels with 7 x 7 2276 and 2337; to one
-// channel with 1 x 1 256 MB are enough (21 x 96 of 192^2, 297 MB, 657 and 581).  With fewer rows than SMs the GroupNorm that
-// reads and writes is the slower one by far (one that fits registers excepted), and 128 MB are enough: 4 x 64 of 364^2 245 and 199 us, 2 x 128 of
-// 512^2 684 and 411; 3 x 128 of 256^2 (96 MB) 211 and 218.
-// With moments out of the convolution ahead rows of 512 K values are long enough, without them of 4 M (1 x 128 of 256^2 in eight groups 239 and 225
-// with, 192 and 208 without; in one group 481 and 452; 2 x 64 of 348^2 in eight, with, 239 and 168; in 32, with, 204 and 220).
-bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups, bool moments) {
+// channel with 1 x 1 256 MB are enough (21 x 96 of 192^2, 297 MB, 657 and 581).  With fewer rows than SMs, longer
+// than registers, the GroupNorm that reads and writes is the slower one by far, and 96 MB or rows of 900 K values are enough: 3 x 128 of 256^2 (96 MB)
+// 198 and 195 us, 4 x 64 of 364^2 237 and 192, 2 x 128 of 512^2 669 and 350, 1 x 128 of 256^2 in eight groups (1 M values) 163 and 155, in one
+// 454 and 159; in 16 141 and 155.
+bool conv_small_oc_pays_norm(int batch, int ic, int oc, int h, int wd, int ks, int groups) {
   if (!conv_small_oc_takes_norm(h, wd) || groups <= 0) return false;
   RowNormArgs r;
   r.rows = static_cast<long long>(batch) * groups; r.len = static_cast<long long>(ic / groups) * h * wd;
   const long long bytes = static_cast<long long>(batch) * ic * h * wd * 4;
-  if (r.rows < ctx().sm_count)
-    return bytes >= (32ll << 20) && !norm_rows_supported(r) && (bytes >= (128ll << 20) || r.len >= (moments ? 1ll << 19 : 1ll << 22));
+  if (r.rows < ctx().sm_count) return bytes >= (32ll << 20) && !norm_rows_supported(r) && (bytes >= (96ll << 20) || r.len >= 900000);
   return bytes >= ((oc * ks * ks <= 8 ? 256ll : 384ll) << 20) && r.len >= 65536 && oc * ks * ks <= 80;
 }
 

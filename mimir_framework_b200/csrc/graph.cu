@@ -1021,11 +1021,7 @@ int plan_once(MimirB200Model* m, const MimirNamedInput* inputs, int n_inputs, in
     // faster apart stays apart).
     if (conv_small_oc_supported(C.d.out_channels, C.d.kernel, C.d.stride, C.d.padding, C.h, C.w, batch, C.d.activation ? MIMIR_B200_ELT_RELU : C.fused_act)) {
       const int r = root_of(m->tensors, P.in_v[0]);
-      if (!extras || m->tensors[r].producer < 0 || r == out_root) continue;
-      const LayerRT& X = m->layers[m->tensors[r].producer];  // (whose epilogue may leave the moments)
-      const bool moments = X.lt == LT::Conv2d && !X.skip && conv_can_emit_gn(batch, X.d.in_channels, X.d.out_channels, X.h, X.w, X.d.kernel, X.d.stride, X.d.padding,
-                                                                           m->precision, P.d.num_groups, X.d.activation ? MIMIR_B200_ELT_RELU : X.fused_act, false, true);
-      if (!conv_small_oc_pays_norm(batch, C.d.in_channels, C.d.out_channels, C.h, C.w, C.d.kernel, P.d.num_groups, moments)) continue;
+      if (!extras || m->tensors[r].producer < 0 || r == out_root || !conv_small_oc_pays_norm(batch, C.d.in_channels, C.d.out_channels, C.h, C.w, C.d.kernel, P.d.num_groups)) continue;
       *took = true;
     }
     const int xin = P.in_v[0];
