@@ -405,11 +405,12 @@ struct SmallOcGeom {
 // CTAs of an SM that the compiler makes room for in registers (0: it chooses).  Four, in 64 registers, for forms of one to three channels with few
 // spills, or none: the plain 1 x 1 to 3 channels on 16 x 128 of 256^2 298 us against 340, the normalising ones to 1 and 3 channels, with the
 // statistics, 460 and 510 against 512 and 525 in 80 registers.  The 3 x 3 to 3 channels loses by it: normalising, 16 x 128 of 256^2 669 us against
-// 644 with three, plain, 16 x 64 of 128^2 82 against 77 with one and one image of 256^2 64 against 59.  Element by element with 7 x 7 the
-// compiler's own choice is better for 3, 6 and 7 channels (16 x 64 of 128 x 126: 203, 305 and 348 us against 206, 321 and 356), and one is
-// for the rest (8 channels 385 against 411, 5 x 5 234 against 244).
+// 644 with three, plain, 16 x 64 of 128^2 82 against 77 with one and one image of 256^2 64 against 59.  Element by element the
+// compiler's own choice is better for 1 x 1 (17 x 64 of 361^2 to 8 channels 443 us against 493, 3 x 32 of 513^2 to one 94 against 97), 3 x 3 to 1, 2
+// and 5 (17 x 64 of 361^2 473, 526 and 738 against 477, 557 and 786), 5 x 5 to one (601 against 613) and 7 x 7 to 3, 6 and 7 (16 x 64 of 128 x 126: 203, 305 and 348 against 206, 321 and 356), and one for the rest (3 x 3 and
+// 7 x 7 to 8 channels 133 and 385 against 142 and 411, 5 x 5 234 against 244).
 constexpr int so_ctas(int oc, int ks, int vec, int norm) {
-  if (!vec) return ks == 7 && (oc == 3 || oc == 6 || oc == 7) ? 0 : 1;
+  if (!vec) return ks == 1 || (ks == 3 && (oc <= 2 || oc == 5)) || (ks == 5 && oc == 1) || (ks == 7 && (oc == 3 || oc == 6 || oc == 7)) ? 0 : 1;
   if (oc == 3 && ks == 3) return norm ? 3 : 1;
   return oc <= 3 && ks <= 3 ? 4 : 1;
 }
